@@ -95,9 +95,8 @@ void        spyb_destroy(spyb_backend *backend);
  * spy_assert/std::terminate error path (util/include/util/log/logger.h:96-150) */
 const char *spyb_last_error(const spyb_backend *backend);
 
-/* Host-only self-check of the library's book-keeping (per-device shared-memory limits of the kernels) and of the e4m3 codes
- * the prompt GEMM feeds the tensor cores (every code decodes to its integer, every 8-bit value is the sum of its two
- * parts); needs no GPU. 0 = passed. No reference counterpart. */
+/* Host-only self-check of the library's book-keeping (per-device shared-memory limits of the kernels); needs no GPU.
+ * 0 = passed. No reference counterpart. */
 int32_t spyb_selftest_host(void);
 
 /* ---- Backend::get_max/avail_memory_capacity (backend.h:46-51) */
@@ -192,8 +191,8 @@ spyb_status spyb_matmul_noalloc(spyb_backend *backend, int32_t weight_type, cons
 /* MatMul(W[Q4_0 | Q8_0], x) for a prompt of n_cols tokens on the tensor cores - the operator the reference evaluates as
  * n_cols x n_rows independent dot products (OperatorMatMul, backend/host/operator/mat.cpp:95-128, Dot<Q4_0,Q8_0> /
  * Dot<Q8_0,Q8_0>, backend/host/include/simd/vec_dot.h:42-115), with the same f32 arithmetic and order, so the result is
- * bit-identical to spyb_submit(MatMul) and to the CPU backend. The integer lane sums of a block come from one
- * tcgen05 MMA per tile of 128 rows x 16 tokens; the f32 chains follow in block order.
+ * bit-identical to spyb_submit(MatMul) and to the CPU backend. The integer lane sums of a block come from tcgen05 MMAs
+ * on tiles of 128 rows x 16 (or 8) tokens; the f32 chains follow in block order.
  *   w_rows_host : n_rows rows of k / 32 blocks in GGUF order (18 or 34 bytes per block), host memory
  *   x_host      : [n_cols][k] f32; norm_w_host (optional, [k]): RMSNorm(x) * norm_w is applied first, as in front of
  *                 the QKV and FFN MatMuls of the graph (eps as in NormRMS)

@@ -162,8 +162,7 @@ using namespace spyb;
 extern "C" {
 
 int32_t spyb_selftest_host(void) {
-    const int a = smem_ledger_selftest();
-    return a != 0 ? a : prefill_e4m3_selftest();
+    return smem_ledger_selftest();
 }
 
 spyb_status spyb_create(const spyb_config *config, spyb_backend **out) {
@@ -423,7 +422,7 @@ spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const voi
         be->set_error("prefill_matmul: needs k a multiple of 32 up to %d, 1..4096 columns", PF_MAX_K); return SPYB_UNSUPPORTED;
     }
     cudaSetDevice(be->config.device_id);
-    const int nb = (int)(k / QK), T = (int)n_cols;
+    const int nb = (int)(k / QK), T = (int)n_cols, tile_tok = prefill_tile_tokens(weight_type, n_rows, T);
     const int64_t rb = kq ? (k / 256) * (weight_type == SPYB_Q4_K ? 144 : 210) : (int64_t)nb * (weight_type == SPYB_Q4_0 ? 18 : 34);
     const size_t wbytes = prefill_weight_bytes(weight_type, n_rows, nb), ybytes = prefill_act_bytes(T, nb);
     uint8_t *raw = nullptr, *w = nullptr, *yq = nullptr; float *x = nullptr, *nw = nullptr, *out = nullptr;
@@ -440,26 +439,12 @@ spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const voi
     if (err == cudaSuccess) { err = cudaMemcpyAsync(x, x_host, (size_t)T * k * 4, cudaMemcpyHostToDevice, be->stream); }
     if (err == cudaSuccess && nw != nullptr) { err = cudaMemcpyAsync(nw, norm_w_host, (size_t)k * 4, cudaMemcpyHostToDevice, be->stream); }
     if (err == cudaSuccess) { err = launch_prefill_retile(weight_type, raw, rb, n_rows, nb, w, 0, be->stream); }
-    if (err == cudaSuccess) { err = launch_prefill_quant(x, k, T, (int)k, nw, eps, yq, be->stream, weight_type); }
+    if (err == cudaSuccess) { err = launch_prefill_quant(x, k, T, (int)k, nw, eps, yq, be->stream, weight_type, tile_tok); }
     if (err == cudaSuccess) {
         PrefillGemm g;
-        g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.T = T; g.out = out; g.out_stride = n_rows;
+        g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.tile_tok = tile_tok; g.T = T; g.out = out; g.out_stride = n_rows;
         g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
-        // profiling aid (SPYB_PF_STAMPS=<file>): clock stamps of the roles of one CTA of a second, warm launch
-        long long *stamps = nullptr;
-        const char *dump = std::getenv("SPYB_PF_STAMPS");
-        const size_t stamp_bytes = 8 * 512 * 4 * sizeof(long long);
         err = launch_prefill_gemm(g, be->stream);
-        if (err == cudaSuccess && dump != nullptr && cudaMalloc(&stamps, stamp_bytes) == cudaSuccess) {
-            cudaMemsetAsync(stamps, 0, stamp_bytes, be->stream);
-            g.stamps = stamps;
-            err = launch_prefill_gemm(g, be->stream);
-            std::vector<long long> h(stamp_bytes / sizeof(long long));
-            cudaStreamSynchronize(be->stream);
-            cudaMemcpy(h.data(), stamps, stamp_bytes, cudaMemcpyDeviceToHost);
-            if (FILE *f = std::fopen(dump, "wb")) { std::fwrite(h.data(), 8, h.size(), f); std::fclose(f); }
-            cudaFree(stamps);
-        }
     }
     if (err == cudaSuccess) { err = cudaMemcpyAsync(out_host, out, (size_t)T * n_rows * 4, cudaMemcpyDeviceToHost, be->stream); }
     if (err == cudaSuccess) { err = cudaStreamSynchronize(be->stream); }
@@ -488,8 +473,8 @@ spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *be, uint64_t limit_
     if (err == cudaSuccess) { err = cudaMemsetAsync(yq, 0, ybytes, be->stream); }
     if (err == cudaSuccess) {
         PrefillGemm g;
-        g.w = w; g.type = SPYB_Q8_0; g.n_rows = PF_ROWS; g.nb = nb; g.yq = yq; g.T = T; g.out = out; g.out_stride = PF_ROWS;
-        g.error_flag = be->d_error_flag; g.wait_limit_ns = limit_ns; g.selftest_skip_batch = 1;
+        g.w = w; g.type = SPYB_Q8_0; g.n_rows = PF_ROWS; g.nb = nb; g.yq = yq; g.tile_tok = prefill_tile_tokens(SPYB_Q8_0, PF_ROWS, T); g.T = T; g.out = out; g.out_stride = PF_ROWS;
+        g.error_flag = be->d_error_flag; g.wait_limit_ns = limit_ns; g.selftest_skip_step = 1;
         err = launch_prefill_gemm(g, be->stream);
     }
     if (err == cudaSuccess) { err = cudaStreamSynchronize(be->stream); }   // returns: the kernel ended by itself
@@ -568,7 +553,7 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
             SPYB_CUDA(be, cudaMalloc(&raw, wbytes));
             be->owned.push_back(raw);
             tiles = static_cast<uint8_t *>(raw);
-            SPYB_CUDA(be, cudaMemsetAsync(tiles, 0, wbytes, be->stream));   // (rows that pad the last tile stay zero)
+            if (n_rows % PF_ROWS != 0) { SPYB_CUDA(be, cudaMemsetAsync(tiles, 0, wbytes, be->stream)); }   // (rows that pad the last tile stay zero)
             SPYB_CUDA(be, launch_prefill_retile(type, static_cast<const uint8_t *>(w.data), rb, n_rows, nb, tiles, 0, be->stream));
             be->pf_tiles[w.data] = tiles;
         }
@@ -581,8 +566,9 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
     for (int64_t t0 = 0; t0 < T; t0 += chunk) {
         const int Tc = (int)std::min(chunk, T - t0);
         SPYB_CUDA(be, cudaMemsetAsync(yq, 0, prefill_act_bytes(Tc, nb), be->stream));
-        SPYB_CUDA(be, launch_prefill_quant(static_cast<const float *>(x.data) + t0 * k, k, Tc, (int)k, nullptr, 0.f, static_cast<uint8_t *>(yq), be->stream, type));
         PrefillGemm g;
+        g.tile_tok = prefill_tile_tokens(type, n_rows, Tc);
+        SPYB_CUDA(be, launch_prefill_quant(static_cast<const float *>(x.data) + t0 * k, k, Tc, (int)k, nullptr, 0.f, static_cast<uint8_t *>(yq), be->stream, type, g.tile_tok));
         g.w = tiles; g.type = type; g.n_rows = n_rows; g.nb = nb; g.yq = static_cast<uint8_t *>(yq); g.T = Tc;
         g.out = static_cast<float *>(out_dev) + t0 * n_rows; g.out_stride = n_rows;
         g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;

@@ -108,10 +108,9 @@ struct MatvecParams {
 };
 
 // Prompt evaluation as a GEMM on the tcgen05 tensor cores (spyb_prefill.cu). Weights in tiles of PF_ROWS rows x 1 block,
-// activations as compact Q8_0 blocks grouped by (tile of PF_TOK tokens, block).
-constexpr int PF_ROWS = 128, PF_TOK = 16;
-constexpr int PF_YQ_BYTES = PF_TOK * 32 + PF_TOK * 4;           // the s8 form (16 x 32 s8, 16 f32 scales; no Q4_0 / Q8_0 kernel uses it any more)
-constexpr int PF_YQ_BYTES_F8 = 2 * PF_TOK * 32 + PF_TOK * 4;    // Q4_0 / Q8_0 weights: the activation bytes split into two e4m3 planes (16 x 32 each), 16 f32 scales
+// activations as compact Q8_0 blocks grouped by (token tile, block).
+constexpr int PF_ROWS = 128, PF_TOK = 16;   // (PF_TOK: fewest tokens worth a pass on this path, and the widest token tile of the Q4_0 / Q8_0 kernel)
+constexpr int PF_WTILE_F16 = 128 * 32 * 2 + 128 * 4;            // Q4_0 / Q8_0: the f16 A operand of a 32-element block (128 rows), then one f32 scale per row
 constexpr int PF_KQ_TOK = 64;                                   // K-quant kernels: 64 tokens per tile, two columns of D per token
 constexpr int PF_KQ_YQ_BYTES = PF_KQ_TOK * 32 + PF_KQ_TOK * 8;   // Q6_K weights: 64 x 32 s8, 64 f32 scales, 64 f32 block sums
 constexpr int PF_KQ_YQ_BYTES_F8 = 2 * PF_KQ_TOK * 32 + PF_KQ_TOK * 8;   // Q4_K weights: two e4m3 planes of 64 x 32, scales, block sums
@@ -122,23 +121,23 @@ struct PrefillGemm {
     int            type = 0;          // 2 = Q4_0, 8 = Q8_0, 12 = Q4_K, 14 = Q6_K
     int64_t        n_rows = 0;        // (the last tile of PF_ROWS rows may be partly padding: zero weights, rows not stored)
     int            nb = 0;            // blocks per row
-    const uint8_t *yq = nullptr;      // [ceil(T / PF_TOK)][nb][PF_YQ_BYTES or PF_YQ_BYTES_F8] (launch_prefill_quant for this weight type)
+    const uint8_t *yq = nullptr;      // [token tiles][nb] blocks of activations (launch_prefill_quant for this weight type and tile_tok)
+    int            tile_tok = 0;      // tokens per tile: prefill_tile_tokens()
     int            T = 0;
     float         *out = nullptr;     // [T][out_stride]
     int64_t        out_stride = 0;
     const float   *resid = nullptr;   // optional [T][out_stride]: out = W x + resid (may alias out)
     int           *error_flag = nullptr;
     uint64_t       wait_limit_ns = 1000000000ull;
-    long long     *stamps = nullptr;  // profiling aid: clock stamps of CTA (0, 0), [8 roles][512 blocks][4]
-    int            selftest_skip_batch = -1;   // failure-path check: the copy thread leaves this batch out, so the waits for it run out
+    int            selftest_skip_step = -1;   // failure-path check: the copy warp leaves this step out, so the waits for it run out
 };
-int         prefill_e4m3_selftest();   // host-only: 0 when the e4m3 codes of the prompt GEMM decode to the integers they stand for
+int         prefill_tile_tokens(int type, int64_t n_rows, int T);   // width of the token tiles for this matrix and number of tokens
 size_t      prefill_weight_bytes(int type, int64_t n_rows, int nb);
 size_t      prefill_act_bytes(int T, int nb);
 cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);
-// weight_type: the type of the matrix the activations will meet (2, 8, 12 or 14): it decides their layout;
+// weight_type, tile_tok: the type of the matrix the activations will meet (2, 8, 12 or 14) and its token tile: they decide the layout;
 // part_len > 0: a row lies in K / part_len parts, part_stride floats apart
-cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type,
+cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type, int tile_tok,
                                  int part_len = 0, int64_t part_stride = 0);
 cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream);   // type 12 = Q4_K, 14 = Q6_K (spyb_prefill_kq.cu)
 cudaError_t launch_prefill_retile_kq(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);

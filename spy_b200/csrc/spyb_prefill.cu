@@ -5,96 +5,88 @@
 // per 32-element block the eight integer "lane sums" (4 products each) are converted to f32 and folded into eight f32
 // accumulators with acc = fma(d_w * d_x, lane_sum, acc), block after block, and the eight accumulators meet in the
 // hsum_float_8 tree at the end of the row. Only the integer lane sums are a contraction; everything after them is
-// order-bound f32 work. So the tensor core computes the lane sums of one block for a tile of 128 rows x 16 tokens:
+// order-bound f32 work. So the tensor core computes the lane sums of a block for 128 rows x TT tokens, half a block at a time:
 //
-//   A (128 x 32)  = the block's weights of 128 rows
-//   B (128 x 32)  = for token t and accumulator n the row 8 t + n holds the four activation bytes of accumulator n
-//                   at their place in the block and zeros elsewhere (block-diagonal per token)
-//   D (128 x 128, tensor memory) = A B^T: D[r][8 t + n] = lane sum n of (row r, token t) of this block
+//   A (128 x 16)   = the half block's weights of 128 rows
+//   B (4 TT x 16)  = for token t and accumulator n (four per half) the row 8 (t / 2) + 2 n + t % 2 holds the four activation values of
+//                    accumulator n at their place and zeros elsewhere
+//   D (128 x 4 TT, tensor memory) = A B^T: one lane sum per row, token and accumulator
 //
-// with e4m3 operands and f32 accumulators (tcgen05.mma kind::f8f6f4), four D buffers in flight. Small integers are exact in
-// e4m3: a Q4_0 weight nibble - 8 directly; an 8-bit value y (an activation byte, a Q8_0 weight) as the sum of two e4m3 values,
-// y - (y mod 16) and y mod 16. So a block takes two MMAs (Q4_0) or four (Q8_0: weights split as well) onto the same buffer,
-// the first with accumulate = 0. Every product and every sum of a lane's four products are integers below 2^17, exact in
-// f32, so D holds (float)lane_sum itself: no conversion, no preset, and a buffer is free for the next MMA as soon as it has
-// been read. (The K-quant kernel of spyb_prefill_kq.cu keeps an s8 / s32 form for Q6_K, whose values do not fit.)
-// The epilogue warps read D back with tcgen05.ld (lane = row) and run the CPU's FMA chains in block order on f32 accumulators
-// held as packed f32x2 pairs. Operands reach shared memory by cp.async.bulk (weights in a 128-row x 1-block tile layout
-// made at upload, activations as compact blocks); an expander warp writes the activations into the canonical K-major
-// no-swizzle operand layout (core matrices of 8 rows x 16 bytes) ahead of the MMA. Every wait is bounded.
+// with f16 operands and f32 accumulators (tcgen05.mma kind::f16, K = 16). Every 8-bit integer is exact in f16, products and sums of four
+// of them are exact in f32: D holds (float)lane_sum itself, for Q4_0 and Q8_0 weights alike. (An earlier form with e4m3 operands, K = 32,
+// had to split every 8-bit value in two and take two MMAs of twice the columns per block for Q4_0 and four for Q8_0.)
+// The epilogue warps read D back with tcgen05.ld (lane = row) and run the CPU's FMA chains in block order on f32 accumulators held as
+// packed f32x2 pairs of neighbouring tokens, whose scales come as pairs from shared memory. Operands reach shared memory by
+// cp.async.bulk (weights in a 128-row x 1-block tile layout made at upload, activations as compact blocks); an expander warp writes the
+// activations into the canonical K-major no-swizzle operand layout (core matrices of 8 rows x 16 bytes). Every wait is bounded.
 #include "spyb_tc.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace spyb {
 
 namespace {
 
-constexpr int PF_N           = 8 * PF_TOK;         // 8 accumulator columns per token
-static_assert(PF_N == PF_NCOL, "16 tokens x 8 accumulators fill the MMA's columns");
 constexpr int PF_QUANT_THREADS = 512;
 constexpr int PF_QUANT_GROUPS  = PF_MAX_K / (4 * PF_QUANT_THREADS);   // float4 groups per thread
 
 // ---------------------------------------------------------------------------------------------
-// the GEMM. grid = (token tiles, row tiles); one CTA per SM (it takes all 512 tensor-memory columns).
+// the GEMM: persistent CTAs (one per SM, all 512 tensor-memory columns), each walking tiles of 128 rows x TT tokens along K in
+// steps of NB = 32 / TT blocks, so that a step is 256 columns of D whatever the tile's width; two D buffers. 20 warps (96 registers):
+//   warps 0-15  epilogue: row = 32 (warp % 4) + lane, a quarter of the tile's tokens; four warps per scheduler hide the latency of tensor
+//               memory and of the hand-offs behind one another's FMAs
+//   warp 16     streams the operands of step after step with cp.async.bulk (weights: A operands as they are; compact activations)
+//   warp 17     expands the compact activations into the B operands
+//   warps 18-19 issue the MMAs of alternate steps and one commit each
+// The pipeline does not drain between tiles: copies, expansion and MMAs run on into the next tile while a tile's rows are stored.
 //
-// 20 warps (96 registers):
-// warps 0-15  epilogue - row = 32 (warp % 4) + lane, tokens 4 (warp / 4) .. + 3 of the tile; four warps per scheduler hide the
-//             latency of tensor memory behind one another's f32 chains
-// warp 16     its first thread streams batches of PF_BATCH blocks with cp.async.bulk: two copies per batch (the weight tiles,
-//             which arrive as A operands, and the compact activations) - issuing a bulk copy costs its thread hundreds of cycles
-// warp 17     expands the compact activations of a batch into the B operands
-// warps 18-19 their first threads issue the MMAs of alternate blocks (MMAs and commit hold the issuing thread for hundreds
-//             of cycles; threads of different warps issue in parallel)
-//
-// Shared memory: rings of NS blocks (NQ batches), one ring per kind so that a batch is one contiguous run:
-//   A ring  [NS][4352 | 8448]   weight tiles (one or two A operands + 128 fp16 scales), written by cp.async.bulk
-//   Y ring  [NS][1088]          compact activations (two e4m3 planes of 16 tokens x 32 codes; 16 f32 scales)
-//   B ring  [NS][8192]          expanded activations (two B operands), written by the expander warp
-template <int WT> struct PfGeom {
-    static constexpr int  NA      = WT == 8 ? 2 : 1;                       // A operands per block: Q8_0 weights are split like the activations
-    static constexpr int  WTILE   = NA * PF_TILE + 256;                    // a weight tile in HBM: the A operand(s) of 128 rows x 32 e4m3 codes, then 128 fp16 block scales
-    static constexpr int  YQ      = PF_YQ_BYTES_F8;                        // a block's compact activations
-    static constexpr int  BT      = 2 * PF_TILE;                           // a block's two B operands
-    static constexpr int  NQ      = WT == 8 ? 3 : PF_RING;                 // batches in the rings (what fits the shared memory)
-    static constexpr int  NS      = NQ * PF_BATCH;                         // blocks in the rings
-    static constexpr int  EPI_W   = PF_EPI_WARPS_F8;
-    static constexpr int  MMA_W   = PF_MMA_WARPS_F8;
-    static constexpr int  THREADS = PF_THREADS_F8;
-    static constexpr size_t SMEM  = (size_t)NS * (WTILE + YQ + BT) + 8 * (3 * NQ + 2 * PF_DBUF) + 16;
+// Bound: issue slots. A step is 32 packed FMAs (two slots each: a packed FMA measures no faster than 2.5 cycles per scheduler) and 4 packed
+// multiplies per epilogue warp, i.e. 290 slots per scheduler, and everything else around them another 165; the loop is written for few
+// instructions (waits of one test and one branch, D buffers as constants of the unrolled code, one arrival per step), and measures 600
+// cycles per step: 4096 x 4096 x 448 tokens 155 us, 22016 rows 690 us (the e4m3 form: 216 and 1017 us). Tiles of 32 tokens halve the
+// weight bytes per FMA but need 110 registers: spills, 265 us. Eight epilogue warps with 216 registers each: 186-208 us.
+template <int TT> struct PfGeom {
+    static constexpr int NB     = 32 / TT;                                // blocks per step
+    static constexpr int YB     = TT * 64 + TT * 4;                       // a block's compact activations: TT x 32 f16, TT f32 scales
+    static constexpr int RAW    = NB * (PF_WTILE_F16 + YB);               // a step as it arrives
+    static constexpr int STAGE  = RAW + 8192;                             // ... and its B operands
+    static constexpr int NS     = TT == 16 ? 6 : 4;                       // steps in the ring (even)
+    static constexpr int PW     = TT / 8;                                 // token pairs per epilogue warp
+    static constexpr int PC     = PW < 2 ? 1 : 2;                         // pairs per chunk of tensor-memory columns (8 columns each)
+    static constexpr int NC     = NB * 2 * (PW / PC);                     // chunks per step and warp
+    static constexpr size_t SMEM = (size_t)NS * STAGE + 8 * (3 * NS + 4) + 16;
 };
 
-template <int WT>
-__global__ void __launch_bounds__(PfGeom<WT>::THREADS, 1) prefill_gemm_kernel(PrefillGemm g) {
-    constexpr int NS = PfGeom<WT>::NS, NQ = PfGeom<WT>::NQ, NA = PfGeom<WT>::NA, PF_WTILE = PfGeom<WT>::WTILE;
-    constexpr int YQ = PfGeom<WT>::YQ, BT = PfGeom<WT>::BT, EPI_W = PfGeom<WT>::EPI_W, MMA_W = PfGeom<WT>::MMA_W, THREADS = PfGeom<WT>::THREADS;
+template <int TT>
+__global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(PrefillGemm g) {
+    using G = PfGeom<TT>;
+    constexpr int NB = G::NB, NS = G::NS, PW = G::PW, PC = G::PC, YB = G::YB;
     extern __shared__ __align__(128) uint8_t smem[];
-    const uint32_t sbase = smem_u32(smem);
-    const uint32_t a_ring = sbase, y_ring = a_ring + NS * PF_WTILE, b_ring = y_ring + NS * YQ;
-    const uint32_t bars  = b_ring + NS * BT;
-    auto raw_full = [&](int q) { return bars + 8u * q; };                        // the batch's weights and activations have landed
-    auto ops_full = [&](int q) { return bars + 8u * (NQ + q); };                 // the batch's B operands are written and fenced
-    auto st_free  = [&](int q) { return bars + 8u * (2 * NQ + q); };             // the batch's stages may be refilled (one arrival per epilogue warp)
-    auto d_full   = [&](int i) { return bars + 8u * (3 * NQ + i); };             // the MMA into buffer i has completed
-    auto d_free   = [&](int i) { return bars + 8u * (3 * NQ + PF_DBUF + i); };   // buffer i has been read (one arrival per epilogue warp)
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + (size_t)NS * (PF_WTILE + YQ + BT) + 8 * (3 * NQ + 2 * PF_DBUF));
+    const uint32_t sbase = smem_u32(smem), bars = sbase + NS * G::STAGE;
+    // a stage: [NB weight tiles][NB compact activation blocks][8192 bytes of B operands]
+    auto raw_full = [&](int s) { return bars + 8u * s; };                       // the step's weights and activations have landed
+    auto ops_full = [&](int s) { return bars + 8u * (NS + s); };                // its B operands are written and fenced
+    auto st_free  = [&](int s) { return bars + 8u * (2 * NS + s); };            // the stage may be refilled: its step's D buffer and scales have been read (arrival by the MMA warp, which waits for that anyway)
+    auto d_full   = [&](int i) { return bars + 8u * (3 * NS + i); };            // the MMAs into buffer i have completed
+    auto d_free   = [&](int i) { return bars + 8u * (3 * NS + 2 + i); };        // buffer i has been read (one arrival per epilogue warp)
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + (size_t)NS * G::STAGE + 8 * (3 * NS + 4));
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nb = g.nb, n_batch = (nb + PF_BATCH - 1) / PF_BATCH;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int nb = g.nb, n_step = (nb + NB - 1) / NB;
+    const int n_tok = (g.T + TT - 1) / TT;
+    const int n_tile = n_tok * (int)((g.n_rows + PF_M - 1) / PF_M);
     const uint64_t limit = g.wait_limit_ns;
-    const int row_tile = blockIdx.y, tok_tile = blockIdx.x;   // CTAs that run together share a weight tile: it crosses HBM once
-    const uint8_t *wsrc = g.w + ((int64_t)row_tile * nb) * PF_WTILE;
-    const uint8_t *ysrc = g.yq + ((int64_t)tok_tile * nb) * YQ;
 
     if (tid == 0) {
-        for (int q = 0; q < NQ; ++q) { mbar_init(raw_full(q), 1); mbar_init(ops_full(q), 1); mbar_init(st_free(q), EPI_W); }
-        for (int i = 0; i < PF_DBUF; ++i) { mbar_init(d_full(i), 1); mbar_init(d_free(i), EPI_W); }
+        for (int s = 0; s < NS; ++s) { mbar_init(raw_full(s), 1); mbar_init(ops_full(s), 1); mbar_init(st_free(s), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(d_full(i), 1); mbar_init(d_free(i), PF_GEMM_EPI_WARPS); }
         mbar_init_fence();
     }
-    // the B tiles are zero except where the expansion writes, and it writes the same places for every block
-    for (int i = tid; i < NS * (BT / 16); i += THREADS) { sts128(b_ring + (uint32_t)i * 16u, make_uint4(0u, 0u, 0u, 0u)); }
+    // the B operands are zero except where the expansion writes, and it writes the same places in every step
+    for (int i = tid; i < NS * 512; i += PF_GEMM_THREADS) { sts128(sbase + (uint32_t)(i >> 9) * G::STAGE + G::RAW + (uint32_t)(i & 511) * 16u, make_uint4(0u, 0u, 0u, 0u)); }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(PF_DBUF * PF_N) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     fence_async_smem();
@@ -103,179 +95,224 @@ __global__ void __launch_bounds__(PfGeom<WT>::THREADS, 1) prefill_gemm_kernel(Pr
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp >= EPI_W + 2) {
-        // ---- MMA warps: the first thread of warp m issues the 128 x 128 x 32 MMAs of blocks m, m + MMA_W, ... onto a buffer
-        // the epilogue has read; MMAs into different buffers do not depend on one another
-        if (lane == 0) {
-            int last = -1;
-            for (int b = warp - (EPI_W + 2); b < nb; b += MMA_W) {
-                const int s = b % NS, q = b / PF_BATCH, buf = b % PF_DBUF;
-                PF_STAMP(2, b, 0);
-                if (!mbar_wait_relaxed(ops_full(q % NQ), (uint32_t)(q / NQ) & 1u, limit)) { pf_report(g.error_flag, 5); break; }
-                PF_STAMP(2, b, 1);
-                if (!mbar_wait_relaxed(d_free(buf), (uint32_t)(b / PF_DBUF) & 1u, limit)) { pf_report(g.error_flag, 5); break; }
-                PF_STAMP(2, b, 2);
-                tc_fence_after();
-                // the e4m3 parts of the activation bytes (and of Q8_0 weights), one product after the other onto the same accumulators
-                const uint32_t d_tmem = tmem + (uint32_t)(buf * PF_N);
-                const uint64_t b_hi = operand_desc(b_ring + (uint32_t)s * BT), b_lo = operand_desc(b_ring + (uint32_t)s * BT + PF_TILE);
-#pragma unroll
-                for (int a = 0; a < NA; ++a) {
-                    const uint64_t a_desc = operand_desc(a_ring + (uint32_t)s * PF_WTILE + (uint32_t)a * PF_TILE);
-                    mma_f8_ss(d_tmem, a_desc, b_hi, a == 0 ? 0u : 1u);
-                    mma_f8_ss(d_tmem, a_desc, b_lo, 1u);
+    // CTAs that run together take neighbouring token tiles of the same rows: a weight tile crosses HBM once
+    if (warp >= PF_GEMM_EPI_WARPS) {
+        uint64_t left_ns = limit;   // (zero once a wait has run out)
+        if (warp == PF_GEMM_EPI_WARPS) {
+            // ---- copies
+            int st = 0, k = 0, issued = 0;
+            uint32_t par = 1;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < n_tile && ok; tile += gridDim.x) {
+                const uint8_t *wsrc = g.w + (int64_t)(tile / n_tok) * nb * PF_WTILE_F16;
+                const uint8_t *ysrc = g.yq + (int64_t)(tile % n_tok) * nb * YB;
+                for (int i = 0; i < n_step; ++i, ++k) {
+                    if (k >= NS) {
+                        ok = __all_sync(0xffffffffu, mbar_wait_relaxed(st_free(st), par, limit));
+                        if (!ok) { break; }
+                    }
+                    const int n = min(NB, nb - i * NB);
+                    if (k != g.selftest_skip_step && elect_one()) {   // (failure-path check: that step never arrives)
+                        const uint32_t dst = sbase + (uint32_t)st * G::STAGE;
+                        mbar_expect_tx(raw_full(st), (uint32_t)(n * (PF_WTILE_F16 + YB)));
+                        bulk_copy_g2s(dst, wsrc, (uint32_t)(n * PF_WTILE_F16), raw_full(st));
+                        bulk_copy_g2s(dst + NB * PF_WTILE_F16, ysrc, (uint32_t)(n * YB), raw_full(st));
+                    }
+                    __syncwarp();
+                    issued = k + 1;
+                    wsrc += NB * PF_WTILE_F16; ysrc += NB * YB;
+                    if (++st == NS) { st = 0; par ^= 1u; }
                 }
-                mma_commit(d_full(buf));
-                PF_STAMP(2, b, 3);
-                last = b;
             }
-            // every MMA has completed (it reads shared memory and writes tensor memory) before the CTA leaves
-            if (last >= 0 && !mbar_wait_relaxed(d_full(last % PF_DBUF), (uint32_t)(last / PF_DBUF) & 1u, limit)) { pf_report(g.error_flag, 5); }
-        }
-    } else if (warp == EPI_W) {
-        // ---- copy warp: one thread requests batch after batch
-        if (lane == 0) {
-            int issued = 0;
-            for (int q = 0; q < n_batch; ++q) {
-                if (q == g.selftest_skip_batch) { issued = q + 1; continue; }   // (failure-path check: this batch never arrives)
-                if (q >= NQ && !mbar_wait_relaxed(st_free(q % NQ), (uint32_t)((q / NQ) - 1) & 1u, limit)) { pf_report(g.error_flag, 4); break; }
-                const int b0 = q * PF_BATCH, n = min(PF_BATCH, nb - b0), s0 = b0 % NS;
-                PF_STAMP(0, b0, 0);
-                mbar_expect_tx(raw_full(q % NQ), (uint32_t)(n * (PF_WTILE + YQ)));
-                bulk_copy_g2s(a_ring + (uint32_t)s0 * PF_WTILE, wsrc + (int64_t)b0 * PF_WTILE, (uint32_t)(n * PF_WTILE), raw_full(q % NQ));
-                bulk_copy_g2s(y_ring + (uint32_t)s0 * YQ, ysrc + (int64_t)b0 * YQ, (uint32_t)(n * YQ), raw_full(q % NQ));
-                issued = q + 1;
-            }
+            if (!ok && lane == 0) { pf_report(g.error_flag, 4); }
             // no copy of this CTA is in flight when it leaves
-            for (int q = max(0, issued - NQ); q < issued; ++q) {
-                if (!mbar_wait_relaxed(raw_full(q % NQ), (uint32_t)(q / NQ) & 1u, limit)) { pf_report(g.error_flag, 4); break; }
+            for (int j = max(0, issued - NS); j < issued; ++j) {
+                if (j != g.selftest_skip_step && !mbar_wait_relaxed(raw_full(j % NS), (uint32_t)(j / NS) & 1u, limit)) { if (lane == 0) { pf_report(g.error_flag, 4); } break; }
             }
-        }
-    } else if (warp == EPI_W + 1) {
-        // ---- expander warp: word w of token tt of the compact activations -> row 8 tt + w of B, at its own place in the
-        // block (the rest of B stays zero); one proxy fence per batch makes the writes visible to the tensor core
-        for (int q = 0; q < n_batch; ++q) {
-            bool ok = mbar_wait_relaxed(raw_full(q % NQ), (uint32_t)(q / NQ) & 1u, limit);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) { if (lane == 0) { pf_report(g.error_flag, 4); } break; }
-            const int b0 = q * PF_BATCH, n = min(PF_BATCH, nb - b0), s0 = b0 % NS;
-            if (lane == 0) { PF_STAMP(1, b0, 0); }
-            for (int j = 0; j < n; ++j) {
-                const uint32_t ysrc_s = y_ring + (uint32_t)(s0 + j) * YQ, bdst = b_ring + (uint32_t)(s0 + j) * BT;
-                constexpr int NW = 2 * PF_TOK * 8 / 32;   // words per lane (the second plane of words goes to the second B operand)
-                uint32_t v[NW];
+        } else if (warp == PF_GEMM_EPI_WARPS + 1) {
+            // ---- expansion. The four values of accumulator n of token t in half h of a block go to row 8 (t / 2) + 2 n + t % 2 of the half's
+            // B operand (4 TT rows x 16), at their place 4 n; the rest of B stays zero. A lane takes 16 bytes (accumulators 2 np and
+            // 2 np + 1) at a time.
+            int st = 0;
+            uint32_t par = 0;
+            const int h = (lane >> 1) & 1, np = lane & 1, t0 = lane >> 2;   // token t0 + 8 k of the step (block (t0 + 8 k) / TT)
+            const uint32_t dst_lane = (uint32_t)(h * 128 * TT + np * (64 * TT + 64) + (t0 >> 1) * 128 + (t0 & 1) * 16);
+            for (int tile = blockIdx.x; tile < n_tile && left_ns != 0; tile += gridDim.x) {
+                for (int i = 0; i < n_step; ++i) {
+                    mbar_wait_lean(raw_full(st), par, left_ns);
+                    if (left_ns == 0) { break; }
+                    const uint32_t base = sbase + (uint32_t)st * G::STAGE, src = base + NB * PF_WTILE_F16 + (uint32_t)lane * 16u, dst = base + G::RAW + dst_lane;
+                    uint4 v[4];
 #pragma unroll
-                for (int k = 0; k < NW; ++k) { v[k] = lds32(ysrc_s + (uint32_t)(lane + 32 * k) * 4u); }   // all loads in flight before the first store
+                    for (int k = 0; k < 4; ++k) { v[k] = lds128(src + (uint32_t)((k * 8 / TT) * YB + (k * 8 % TT) * 64)); }   // all loads in flight before the first store
 #pragma unroll
-                for (int k = 0; k < NW; ++k) {
-                    const int i = lane + 32 * k, plane = i >> 7, tt = (i >> 3) & (PF_TOK - 1), w = i & 7;
-                    sts32(bdst + (uint32_t)plane * PF_TILE + (uint32_t)tt * 256u + (uint32_t)(w >> 2) * 128u + (uint32_t)w * 16u + (uint32_t)(w & 3) * 4u, v[k]);
+                    for (int k = 0; k < 4; ++k) {
+                        const uint32_t d = dst + (uint32_t)((k * 8 / TT) * 256 * TT + (k * 8 % TT) * 64);
+                        sts64(d, v[k].x, v[k].y);
+                        sts64(d + 40u, v[k].z, v[k].w);
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) { mbar_arrive(ops_full(st)); }
+                    if (++st == NS) { st = 0; par ^= 1u; }
                 }
             }
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) { mbar_arrive(ops_full(q % NQ)); PF_STAMP(1, b0, 1); }
+            if (left_ns == 0 && lane == 0) { pf_report(g.error_flag, 4); }
+        } else {
+            // ---- MMAs: per block and half of 16 elements one 128 x 4 TT x 16 product; warp m takes the steps of D buffer m (issuing a step's
+            // MMAs and their commit takes one warp up to 400 cycles)
+            const int m = warp - (PF_GEMM_EPI_WARPS + 2);
+            const uint32_t d0 = tmem + (uint32_t)m * 256u;
+            int st = 0, k = 0, mine = 0;
+            uint32_t par = 0;
+            for (int tile = blockIdx.x; tile < n_tile && left_ns != 0; tile += gridDim.x) {
+                for (int i = 0; i < n_step; ++i, ++k) {
+                    if ((k & 1) == m) {
+                        mbar_wait_lean(ops_full(st), par, left_ns);
+                        mbar_wait_lean(d_free(m), (uint32_t)mine & 1u, left_ns);
+                        if (left_ns == 0) { break; }
+                        if (mine > 0 && lane == 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }   // (the step before on this buffer has been read)
+                        tc_fence_after();
+                        const uint32_t base = sbase + (uint32_t)st * G::STAGE;
+                        const uint64_t a0 = operand_desc(base, 2048u, 128u), b0 = operand_desc(base + G::RAW, 64u * TT, 128u);
+                        const int n = min(NB, nb - i * NB);
+                        if (elect_one()) {
+#pragma unroll
+                            for (int j = 0; j < NB; ++j) {
+                                if (j < n) {
+#pragma unroll
+                                    for (int h = 0; h < 2; ++h) {
+                                        mma_f16_ss(d0 + (uint32_t)(j * 8 * TT + h * 4 * TT), a0 + (uint64_t)((j * PF_WTILE_F16 + h * 4096) >> 4), b0 + (uint64_t)((j * 256 * TT + h * 128 * TT) >> 4),
+                                                   idesc_f16(4 * TT), 0u);
+                                    }
+                                }
+                            }
+                            mma_commit(d_full(m));
+                        }
+                        __syncwarp();
+                        ++mine;
+                    }
+                    if (++st == NS) { st = 0; par ^= 1u; }
+                }
+            }
+            if (left_ns == 0 && lane == 0) { pf_report(g.error_flag, 5); }
+            // every MMA has completed (it reads shared memory and writes tensor memory) before the CTA leaves
+            if (mine > 0 && !mbar_wait_relaxed(d_full(m), (uint32_t)(mine - 1) & 1u, limit)) { if (lane == 0) { pf_report(g.error_flag, 5); } }
         }
     } else {
-        // ---- epilogue warps: row = 32 (warp % 4) + lane, tokens 8 (warp / 4) .. + 7 of the tile = 64 columns of D, read back 16
-        // columns (two tokens) at a time into two alternating register sets: a set is requested again as soon as its values
-        // have been folded, so that the tensor-memory loads overlap the f32 chains of the other set
-        const int quad = warp & 3;
+        // ---- epilogue: tokens part * TT / 4 .. of the tile as PW packed pairs (tokens 2 u, 2 u + 1), eight accumulators each. D's columns
+        // of block j and half h: 8 TT j + 4 TT h + 8 (t / 2) + 2 n + t % 2, i.e. a pair's accumulator n is a neighbouring pair of columns.
+        const int quad = warp & 3, part = warp >> 2;
         const int row = 32 * quad + lane;
-        const uint32_t dw_addr = a_ring + NA * PF_TILE + 2u * (uint32_t)row;
-        bool ok = true;
-        {
-            // ---- e4m3 operands: D is f32 and holds (float)lane_sum itself, so a lane sum costs half a packed FMA. Sixteen warps:
-            // warp = (row quadrant, quarter of the columns = tokens 4 part .. + 3), both halves of its 32 columns requested
-            // together, so the buffer is free for the next MMA as soon as they have arrived.
-            const int part = warp >> 2;
-            const uint32_t tbase = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(32 * part);
-            const uint32_t dx_addr = y_ring + 2 * PF_TOK * 32 + 16u * (uint32_t)part;
-            uint64_t acc[4][4];   // [token][pair]: accumulators 2 pair and 2 pair + 1 of the token, as one packed f32x2 value
+        const uint32_t tbase = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(part * TT);
+        const uint32_t dw_addr = sbase + 8192u + 4u * (uint32_t)row, dx_addr = sbase + NB * PF_WTILE_F16 + TT * 64 + (uint32_t)(part * TT);
+        uint64_t acc[PW][8];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
+        for (int u = 0; u < PW; ++u) {
 #pragma unroll
-                for (int n = 0; n < 4; ++n) { acc[t][n] = 0ull; }
-            }
-            if (lane == 0) { for (int i = 0; i < PF_DBUF; ++i) { mbar_arrive(d_free(i)); } }
-            uint32_t ra[16], rb[16];
-            auto fold2 = [&](const uint32_t *r, int t0, float sa, float sb) {   // two tokens: columns 8 t0 .. 8 t0 + 15 of the warp's 32
-                const uint64_t sc[2] = {f2_pack(sa, sa), f2_pack(sb, sb)};
+            for (int n = 0; n < 8; ++n) { acc[u][n] = 0ull; }
+        }
+        if (lane == 0) { mbar_arrive(d_free(0)); mbar_arrive(d_free(1)); }
+        uint32_t stage = 0, par = 0;   // (the ring has an even number of stages: a step's stage and its D buffer are even or odd together)
+        uint64_t left_ns = limit;      // (zero once a wait has run out)
+        // one step, its D buffer a constant of the unrolled code; n of its NB blocks lie inside the row
+        auto step = [&](auto buf_c, int n) {
+            constexpr int buf = decltype(buf_c)::value;
+            mbar_wait_lean(d_full(buf), par, left_ns);
+            tc_fence_after();
+            uint64_t sc[PC];
 #pragma unroll
-                for (int t = 0; t < 2; ++t) {
-#pragma unroll
-                    for (int n = 0; n < 4; ++n) { acc[t0 + t][n] = f2_fma(sc[t], f2_pack_bits(r[8 * t + 2 * n], r[8 * t + 2 * n + 1]), acc[t0 + t][n]); }
+            for (int c = 0; c < G::NC; ++c) {   // chunk c: half c % 2 of PC pairs of block c / 2 / (PW / PC)
+                const int cu = (c >> 1) % (PW / PC), j = (c >> 1) / (PW / PC);
+                const uint32_t col = (uint32_t)(buf * 256 + j * 8 * TT + (c & 1) * 4 * TT + cu * 8 * PC);
+                uint32_t r[8 * PC];
+                if (PC == 2) { tmem_ld16(tbase + col, r); } else { tmem_ld8(tbase + col, r); }
+                if ((c & 1) == 0) {
+                    const float dw = lds32f(dw_addr + stage + (uint32_t)j * PF_WTILE_F16);
+                    const uint64_t dw2 = f2_pack(dw, dw);
+                    const uint32_t xa = dx_addr + stage + (uint32_t)(j * YB + cu * 8 * PC);
+                    if (PC == 2) { uint64_t x0, x1; lds128_2x64(xa, x0, x1); sc[0] = f2_mul(dw2, x0); sc[PC - 1] = f2_mul(dw2, x1); }
+                    else { sc[0] = f2_mul(dw2, lds64u(xa)); }
                 }
-            };
-            ok = mbar_wait_bounded(d_full(0), 0u, limit);
-            ok = __all_sync(0xffffffffu, ok);
-            if (ok) { tc_fence_after(); tmem_ld16(tbase, ra); tmem_ld16(tbase + 16u, rb); }
-            static_assert(PF_BATCH == PF_DBUF, "the unrolled epilogue pairs block j of a batch with accumulator buffer j");
-            for (int q = 0; q < n_batch && ok; ++q) {
-                const uint32_t ring_q = (uint32_t)(q % NQ) * PF_BATCH;
-                const uint32_t dw_q = dw_addr + ring_q * PF_WTILE, dx_q = dx_addr + ring_q * YQ;
-#pragma unroll
-                for (int j = 0; j < PF_BATCH; ++j) {
-                    const int b = q * PF_BATCH + j;
-                    if (b >= nb || !ok) { break; }
-                    const float dw = h2f((uint16_t)lds16(dw_q + (uint32_t)j * PF_WTILE));
-                    const float4 dx = lds128f(dx_q + (uint32_t)j * YQ);
-                    tmem_ld_wait();                       // the warp's 32 columns of block b are in registers: the buffer has been read
+                tmem_ld_wait();
+                if (c == G::NC - 1) {           // the whole buffer is in registers and the step's scales have been read
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) { mbar_arrive(d_free(j)); }
-                    fold2(ra, 0, __fmul_rn(dw, dx.x), __fmul_rn(dw, dx.y));
-                    const bool more = b + 1 < nb;
-                    const uint32_t tnext = tbase + (uint32_t)(((j + 1) % PF_DBUF) * PF_N);
-                    if (more) {                           // the next block's columns arrive while the last two tokens are folded
-                        ok = mbar_wait_bounded(d_full((j + 1) % PF_DBUF), (uint32_t)(q + (j + 1) / PF_DBUF) & 1u, limit);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (ok) { tc_fence_after(); tmem_ld16(tnext, ra); }
+                    if (lane == 0) { mbar_arrive(d_free(buf)); }
+                }
+                if (NB == 1 || j < n) {         // (blocks past the end of the row in a tile's last step are not folded)
+#pragma unroll
+                    for (int p = 0; p < PC; ++p) {
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) {
+                            uint64_t &a = acc[PC * cu + p][4 * (c & 1) + m];
+                            a = f2_fma(sc[p], f2_pack_bits(r[8 * p + 2 * m], r[8 * p + 2 * m + 1]), a);
+                        }
                     }
-                    fold2(rb, 2, __fmul_rn(dw, dx.z), __fmul_rn(dw, dx.w));
-                    if (more && ok) { tmem_ld16(tnext + 16u, rb); }
-                    if (lane == 0 && (j == PF_BATCH - 1 || b == nb - 1)) { mbar_arrive(st_free(q % NQ)); }   // the batch's scales have been read
                 }
             }
-            tmem_ld_wait();
-            if (!ok) { if (lane == 0) { pf_report(g.error_flag, 6); } }
-            else {
+            stage += G::STAGE;
+            if (buf) { par ^= 1u; if (stage == NS * G::STAGE) { stage = 0; } }
+        };
+        using B0 = std::integral_constant<int, 0>;
+        using B1 = std::integral_constant<int, 1>;
+        const int n_full = nb / NB, rest = nb % NB;
+        bool odd = false;        // a tile with an odd number of steps leaves the next one starting on buffer 1
+        for (int tile = blockIdx.x; tile < n_tile; tile += gridDim.x) {
+            int i = 0;
+            if (odd && n_full > 0) { step(B1{}, NB); i = 1; }
+#pragma unroll 1
+            for (; i + 2 <= n_full; i += 2) { step(B0{}, NB); step(B1{}, NB); }
+            bool second = odd && n_full == 0;
+            if (i < n_full) { step(B0{}, NB); second = true; }
+            if (rest != 0) {
+                if (second) { step(B1{}, rest); } else { step(B0{}, rest); }
+                second = !second;
+            }
+            odd = second;
+            // hsum_float_8 (vec_util.h:74-81): accumulator n of a half is CPU accumulator 4 + n / n (Q4_0: low / high nibbles) or n / 4 + n
+            // (Q8_0); either way the tree is (c0 + c4) + (c2 + c6) and (c1 + c5) + (c3 + c7)
+            const int64_t orow = (int64_t)(tile / n_tok) * PF_M + row;
+            const int     tok0 = (tile % n_tok) * TT + part * (TT / 4);
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {   // hsum_float_8 (vec_util.h:74-81): column n < 4 is accumulator 4 + n for Q4_0 (low nibbles) and accumulator n for Q8_0; either way the tree is (c0 + c4) + (c2 + c6) and (c1 + c5) + (c3 + c7)
-                    const int token = tok_tile * PF_TOK + 4 * part + t;
-                    if (token < g.T && (int64_t)row_tile * PF_M + row < g.n_rows) {   // (the last row tile may be partly padding)
-                        float c[8];
+            for (int u = 0; u < PW; ++u) {
+                const uint64_t r0 = f2_add(acc[u][0], acc[u][4]), r1 = f2_add(acc[u][1], acc[u][5]), r2 = f2_add(acc[u][2], acc[u][6]), r3 = f2_add(acc[u][3], acc[u][7]);
+                float v[2];
+                f2_unpack(f2_add(f2_add(r0, r2), f2_add(r1, r3)), v[0], v[1]);
 #pragma unroll
-                        for (int n = 0; n < 4; ++n) { f2_unpack(acc[t][n], c[2 * n], c[2 * n + 1]); }
-                        const float r0 = __fadd_rn(c[0], c[4]), r1 = __fadd_rn(c[1], c[5]);
-                        const float r2 = __fadd_rn(c[2], c[6]), r3 = __fadd_rn(c[3], c[7]);
-                        const float v = __fadd_rn(__fadd_rn(r0, r2), __fadd_rn(r1, r3));
-                        const int64_t i = (int64_t)token * g.out_stride + (int64_t)row_tile * PF_M + row;
-                        g.out[i] = g.resid != nullptr ? __fadd_rn(v, g.resid[i]) : v;
+                for (int e = 0; e < 2; ++e) {
+                    const int token = tok0 + 2 * u + e;
+                    if (token < g.T && orow < g.n_rows) {   // (the last row tile may be partly padding)
+                        const int64_t o = (int64_t)token * g.out_stride + orow;
+                        g.out[o] = g.resid != nullptr ? __fadd_rn(v[e], g.resid[o]) : v[e];
                     }
                 }
+#pragma unroll
+                for (int m = 0; m < 8; ++m) { acc[u][m] = 0ull; }
             }
         }
+        if (left_ns == 0 && lane == 0) { pf_report(g.error_flag, 6); }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(PF_DBUF * PF_N) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
     }
 }
 
 // ---------------------------------------------------------------------------------------------
-// activations of T tokens -> compact Q8_0 blocks grouped by (token tile, block): [T/16][nb][16 x 32 s8 | 16 f32 scales].
-// One CTA per token; RMSNorm and the quantizer as in the mat-vec prologue (NormRMS, backend/host/operator/non-linear.cpp:194-223:
-// groups of four squares formed in parallel, the running sum on one thread; Quantizator<FP32,Q8_0>, simd/vec_convert.h:178-261).
-// TOKT tokens per tile; YSUM: the blocks' integer sums follow the scales as floats (the K-quant kernels need them); F8: every
-// activation byte as two e4m3 values (a plane of TOKT x 32 codes each: the multiple of 16 and the rest) for the Q4_0 kernel
-template <bool NORM, int TOKT, bool YSUM, bool F8>
+// activations of T tokens -> compact Q8_0 blocks grouped by (tile of tile_tok tokens, block). One CTA per token; RMSNorm and the
+// quantizer as in the mat-vec prologue (NormRMS, backend/host/operator/non-linear.cpp:194-223: groups of four squares formed in
+// parallel, the running sum on one thread; Quantizator<FP32,Q8_0>, simd/vec_convert.h:178-261).
+// FORM 0 (Q4_0 / Q8_0 weights): the values as f16, then the f32 scales. FORM 1 (Q6_K): s8 values, scales, the blocks' integer sums as
+// floats. FORM 2 (Q4_K): two planes of e4m3 values (the multiple of 16 and the rest), scales, sums.
+template <bool NORM, int FORM>
 __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const float *x, int64_t x_stride, int K, const float *norm_w, float eps, uint8_t *yq,
-                                                                         int part_len, int64_t part_stride) {
-    constexpr int YQB = (F8 ? 2 : 1) * TOKT * 32 + TOKT * 4 * (YSUM ? 2 : 1);
-    constexpr int SCALES = (F8 ? 2 : 1) * TOKT * 32;   // offset of the scales inside a block's record
+                                                                         int TOKT, int part_len, int64_t part_stride) {
+    constexpr bool YSUM = FORM != 0;
+    const int SCALES = (FORM == 1 ? 1 : 2) * TOKT * 32;   // offset of the scales inside a block's record
+    const int YQB = SCALES + TOKT * 4 * (YSUM ? 2 : 1);
     extern __shared__ __align__(16) float v3[];
     __shared__ float scale_s;
     const int tid = threadIdx.x, token = blockIdx.x;
@@ -341,7 +378,10 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
             if (gi < n4) {
                 const int b = gi >> 3, w = gi & 7;
                 uint8_t *blk = tile + (int64_t)b * YQB;
-                if (F8) {
+                if (FORM == 0) {
+                    auto h = [&](int i) { return (uint32_t)__half_as_ushort(__int2half_rn((int)(int8_t)(q >> (8 * i)))); };
+                    reinterpret_cast<uint2 *>(blk + tt * 64)[w] = make_uint2(h(0) | (h(1) << 16), h(2) | (h(3) << 16));
+                } else if (FORM == 2) {
                     uint32_t hi, lo;
                     e4m3_split4(q, hi, lo);
                     reinterpret_cast<uint32_t *>(blk + tt * 32)[w] = hi;
@@ -358,39 +398,38 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
     }
 }
 
-// upload-time re-layout: raw 18-byte / 34-byte blocks of rows [0, n_rows) -> tiles of 128 rows x 1 block: the A operand
-// (core matrices of 8 rows x 16 bytes; Q8_0: the s8 values; Q4_0: element k < 16 is the e4m3 code of (low nibble of byte k - 8),
-// element 16 + k the same of the high nibble) followed by the 128 fp16 block scales
+// upload-time re-layout: raw 18-byte / 34-byte blocks of rows [0, n_rows) -> tiles of 128 rows x 1 block: the f16 A operand (core
+// matrices of 8 rows x 16 bytes: element k of row r at (k / 8) * 2048 + (r / 8) * 128 + (r % 8) * 16 + 2 (k % 8); Q4_0: element k < 16 is
+// the low nibble of byte k minus 8, element 16 + k the high one) followed by the 128 block scales as f32. A warp takes 8 rows x 4
+// neighbouring blocks: its stores are runs of 128 bytes, its loads runs of 72 or 136.
 template <int WT>
 __global__ void prefill_retile_kernel(const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_rows * nb) { return; }
-    const int64_t lrow = i / nb;
-    const int     b = (int)(i - lrow * nb);
-    const uint8_t *src = raw + lrow * row_stride + (int64_t)b * (WT == 2 ? 18 : 34);
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int     lane = threadIdx.x & 31, bq = (nb + 3) >> 2;
+    const int64_t lrow = w / bq * 8 + (lane & 7);
+    const int     b = (int)(w % bq) * 4 + (lane >> 3);
+    if (lrow >= n_rows || b >= nb) { return; }
+    uint16_t src[WT == 2 ? 9 : 17];   // (blocks are 2-byte aligned)
+    const uint16_t *raw16 = reinterpret_cast<const uint16_t *>(raw + lrow * row_stride + (int64_t)b * (WT == 2 ? 18 : 34));
+#pragma unroll
+    for (int i = 0; i < (WT == 2 ? 9 : 17); ++i) { src[i] = raw16[i]; }
     const int64_t row = dst_row0 + lrow;
     const int     r = (int)(row % PF_M);
-    uint8_t *tile = base + ((row / PF_M) * nb + b) * (int64_t)PfGeom<WT>::WTILE;
-    reinterpret_cast<uint16_t *>(tile + PfGeom<WT>::NA * PF_TILE)[r] = (uint16_t)(src[0] | (src[1] << 8));
-    uint32_t *lo = reinterpret_cast<uint32_t *>(tile + (r >> 3) * 256 + (r & 7) * 16), *hi = lo + 32;   // elements 0..15 and 16..31
+    uint8_t *tile = base + ((row / PF_M) * nb + b) * (int64_t)PF_WTILE_F16;
+    reinterpret_cast<float *>(tile + 8192)[r] = h2f(src[0]);
+    auto byte_of = [&](int i) { return (i & 1) ? src[1 + (i >> 1)] >> 8 : src[1 + (i >> 1)] & 0xff; };
+    auto value = [&](int k) {
+        if (WT == 2) { const int byte = byte_of(k & 15); return (k < 16 ? (byte & 15) : (byte >> 4)) - 8; }
+        return (int)(int8_t)byte_of(k);
+    };
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (WT == 2) {
-            uint32_t l = 0u, h = 0u;
+    for (int c = 0; c < 4; ++c) {
+        uint32_t v[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int byte = src[2 + 4 * k + i];
-                l |= e4m3_of_signed((byte & 15) - 8) << (8 * i);
-                h |= e4m3_of_signed((byte >> 4) - 8) << (8 * i);
-            }
-            lo[k] = l;
-            hi[k] = h;
-        } else {   // Q8_0: every s8 weight as two e4m3 values, the multiple of 16 in the first operand tile and the rest in the second
-            const uint32_t w_lo = (uint32_t)(src[2 + 4 * k] | (src[3 + 4 * k] << 8) | (src[4 + 4 * k] << 16) | ((uint32_t)src[5 + 4 * k] << 24));
-            const uint32_t w_hi = (uint32_t)(src[18 + 4 * k] | (src[19 + 4 * k] << 8) | (src[20 + 4 * k] << 16) | ((uint32_t)src[21 + 4 * k] << 24));
-            e4m3_split4(w_lo, lo[k], lo[k + PF_TILE / 4]);
-            e4m3_split4(w_hi, hi[k], hi[k + PF_TILE / 4]);
+        for (int e = 0; e < 4; ++e) {
+            v[e] = (uint32_t)__half_as_ushort(__int2half_rn(value(8 * c + 2 * e))) | ((uint32_t)__half_as_ushort(__int2half_rn(value(8 * c + 2 * e + 1))) << 16);
         }
+        *reinterpret_cast<uint4 *>(tile + c * 2048 + (r >> 3) * 128 + (r & 7) * 16) = make_uint4(v[0], v[1], v[2], v[3]);
     }
 }
 
@@ -429,82 +468,81 @@ __global__ void prefill_silu_mul_kernel(const float *upgate, int T, int F, const
     act[i] = __fmul_rn(up, silu_table[f2h(gate)]);
 }
 
-template <int WT>
+int device_sms() {
+    static int sms[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { return 148; }
+    if (sms[dev] == 0) {
+        int n = 0;
+        sms[dev] = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }
+    return sms[dev];
+}
+
+template <int TT>
 cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream) {
-    const size_t smem = PfGeom<WT>::SMEM;
-    cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(prefill_gemm_kernel<WT>), smem);
+    const size_t smem = PfGeom<TT>::SMEM;
+    cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(prefill_gemm_kernel<TT>), smem);
     if (err != cudaSuccess) { return err; }
-    const dim3 grid((unsigned)((g.T + PF_TOK - 1) / PF_TOK), (unsigned)((g.n_rows + PF_M - 1) / PF_M));
-    prefill_gemm_kernel<WT><<<grid, PfGeom<WT>::THREADS, smem, stream>>>(g);
+    const int64_t tiles = (int64_t)((g.T + TT - 1) / TT) * ((g.n_rows + PF_M - 1) / PF_M);
+    prefill_gemm_kernel<TT><<<(unsigned)std::min<int64_t>(tiles, device_sms()), PF_GEMM_THREADS, smem, stream>>>(g);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-// host-only check of the e4m3 codes the exactness of the prompt GEMM rests on (no device needed): 0 when every code decodes
-// to the integer it stands for and every 8-bit value is the sum of its two parts
-int prefill_e4m3_selftest() {
-    auto decode = [](uint32_t c) {   // e4m3: sign, 4 exponent bits (bias 7), 3 mantissa bits; exponent 0 = subnormal
-        const int e = (int)((c >> 3) & 15u), m = (int)(c & 7u);
-        const double v = e == 0 ? m / 8.0 / 64.0 : (1.0 + m / 8.0) * (double)(1 << e) / 128.0;
-        return (c & 0x80u) ? -v : v;
-    };
-    for (int v = 0; v <= 15; ++v) { if (decode(e4m3_of_small((uint32_t)v)) != (double)v) { return 100 + v; } }
-    for (int v = -15; v <= 15; ++v) { if (decode(e4m3_of_signed(v)) != (double)v) { return 200 + v + 15; } }
-    for (int y = -128; y <= 127; ++y) {   // the split of e4m3_split4, one byte at a time
-        const int yl = y & 15, yh = (y - yl) >> 4;
-        const uint32_t ch = yh == 0 ? 0u : (e4m3_of_signed(yh) + 0x20u), cl = e4m3_of_small((uint32_t)yl);
-        if (decode(ch) != 16.0 * yh || decode(cl) != (double)yl || 16 * yh + yl != y || (ch & 0x7fu) > 0x7eu) { return 1000 + y + 128; }
-    }
-    return 0;
+// Tiles of 16 or of 8 tokens. A tile takes nb TT / 32 steps and the CTAs walk their tiles in rounds, so the width whose busiest CTA has
+// fewer steps to do wins; a step of the narrow tiles costs 1.4 of one of the wide ones (eight MMAs and twice the weight bytes; measured
+// 1.2 to 1.5 on 4096 to 27648 rows). 4096 rows x 32 tokens: 8 wide (20 us against 30); 27648 rows x 32 tokens: 16 wide (91 against 142).
+int prefill_tile_tokens(int type, int64_t n_rows, int T) {
+    if (type == 12 || type == 14) { return PF_KQ_TOK; }
+    const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, sms = device_sms();
+    auto rounds = [&](int tt) { return (row_tiles * ((T + tt - 1) / tt) + sms - 1) / sms; };
+    return 8.0 * 1.4 * (double)rounds(8) < 16.0 * (double)rounds(16) ? 8 : 16;
 }
 
 size_t prefill_weight_bytes(int type, int64_t n_rows, int nb) {
-    const size_t tile = (type == 12 || type == 14) ? (size_t)PF_KQ_WTILE : type == 8 ? (size_t)PfGeom<8>::WTILE : (size_t)PfGeom<2>::WTILE;
+    const size_t tile = (type == 12 || type == 14) ? (size_t)PF_KQ_WTILE : (size_t)PF_WTILE_F16;
     return (size_t)((n_rows + PF_ROWS - 1) / PF_ROWS) * nb * tile;
 }
 size_t prefill_act_bytes(int T, int nb) {   // (the largest of the layouts)
-    return std::max((size_t)((T + PF_TOK - 1) / PF_TOK) * nb * std::max(PF_YQ_BYTES, PF_YQ_BYTES_F8),
+    return std::max((size_t)((T + PF_TOK - 1) / PF_TOK) * PF_TOK * nb * 68,
                     (size_t)((T + PF_KQ_TOK - 1) / PF_KQ_TOK) * nb * std::max(PF_KQ_YQ_BYTES, PF_KQ_YQ_BYTES_F8));
 }
 
 cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream) {
     if (type == 12 || type == 14) { return launch_prefill_retile_kq(type, raw, row_stride, n_rows, nb, base, dst_row0, stream); }
     if ((type != 2 && type != 8) || n_rows < 1 || nb < 1) { return cudaErrorInvalidValue; }
-    const int64_t n = n_rows * nb;
-    const unsigned blocks = (unsigned)((n + 255) / 256);
+    if ((reinterpret_cast<uintptr_t>(raw) & 1) || (row_stride & 1)) { return cudaErrorInvalidValue; }
+    const int64_t warps = (n_rows + 7) / 8 * ((nb + 3) / 4);
+    const unsigned blocks = (unsigned)((warps + 7) / 8);
     if (type == 2) { prefill_retile_kernel<2><<<blocks, 256, 0, stream>>>(raw, row_stride, n_rows, nb, base, dst_row0); }
     else           { prefill_retile_kernel<8><<<blocks, 256, 0, stream>>>(raw, row_stride, n_rows, nb, base, dst_row0); }
     return cudaGetLastError();
 }
 
 cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type,
-                                 int part_len, int64_t part_stride) {
+                                 int tile_tok, int part_len, int64_t part_stride) {
     if (weight_type != 2 && weight_type != 8 && weight_type != 12 && weight_type != 14) { return cudaErrorInvalidValue; }
-    const bool kq_layout = weight_type == 12 || weight_type == 14;
     if (part_len <= 0) { part_len = K; part_stride = 0; }
     if ((part_len & 3) || (part_stride & 3) || K % part_len != 0) { return cudaErrorInvalidValue; }
-    if (T < 1 || K < 32 || (K & 31) || K > PF_MAX_K || (x_stride & 3) || ((uintptr_t)x & 15)) { return cudaErrorInvalidValue; }
+    if (T < 1 || tile_tok < 1 || K < 32 || (K & 31) || K > PF_MAX_K || (x_stride & 3) || ((uintptr_t)x & 15)) { return cudaErrorInvalidValue; }
     const size_t smem = norm_w != nullptr ? (size_t)K : 0;   // K / 4 floats
-    if (weight_type == 12) {
-        if (norm_w != nullptr) { prefill_quant_kernel<true, PF_KQ_TOK, true, true><<<T, PF_QUANT_THREADS, smem, stream>>>(x, x_stride, K, norm_w, eps, yq, part_len, part_stride); }
-        else                   { prefill_quant_kernel<false, PF_KQ_TOK, true, true><<<T, PF_QUANT_THREADS, 0, stream>>>(x, x_stride, K, nullptr, 0.f, yq, part_len, part_stride); }
-    } else if (kq_layout) {
-        if (norm_w != nullptr) { prefill_quant_kernel<true, PF_KQ_TOK, true, false><<<T, PF_QUANT_THREADS, smem, stream>>>(x, x_stride, K, norm_w, eps, yq, part_len, part_stride); }
-        else                   { prefill_quant_kernel<false, PF_KQ_TOK, true, false><<<T, PF_QUANT_THREADS, 0, stream>>>(x, x_stride, K, nullptr, 0.f, yq, part_len, part_stride); }
-    } else {   // Q4_0 and Q8_0 weights: tiles of 16 tokens, the two e4m3 planes
-        if (norm_w != nullptr) { prefill_quant_kernel<true, PF_TOK, false, true><<<T, PF_QUANT_THREADS, smem, stream>>>(x, x_stride, K, norm_w, eps, yq, part_len, part_stride); }
-        else                   { prefill_quant_kernel<false, PF_TOK, false, true><<<T, PF_QUANT_THREADS, 0, stream>>>(x, x_stride, K, nullptr, 0.f, yq, part_len, part_stride); }
-    }
+    auto *kernel = weight_type == 12 ? (norm_w ? prefill_quant_kernel<true, 2> : prefill_quant_kernel<false, 2>)
+                 : weight_type == 14 ? (norm_w ? prefill_quant_kernel<true, 1> : prefill_quant_kernel<false, 1>)
+                                     : (norm_w ? prefill_quant_kernel<true, 0> : prefill_quant_kernel<false, 0>);
+    kernel<<<T, PF_QUANT_THREADS, smem, stream>>>(x, x_stride, K, norm_w, eps, yq, tile_tok, part_len, part_stride);
     return cudaGetLastError();
 }
 
 cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream) {
     if (g.type == 12 || g.type == 14) { return launch_prefill_gemm_kq(g, stream); }
-    if (g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
-    if (g.type == 2) { return launch_gemm_t<2>(g, stream); }
-    if (g.type == 8) { return launch_gemm_t<8>(g, stream); }
-    return cudaErrorInvalidValue;
+    if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
+    switch (g.tile_tok) {
+    case 16: return launch_gemm_t<16>(g, stream);
+    case 8:  return launch_gemm_t<8>(g, stream);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_prefill_qkv_post(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,

@@ -42,14 +42,6 @@ __device__ __forceinline__ float2 lds64f(uint32_t addr) {
     asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ uint64_t lds64u(uint32_t addr) {
-    uint64_t v;
-    asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ void lds128_2x64(uint32_t addr, uint64_t &a, uint64_t &b) {
-    asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
-}
 
 // eight tokens (T0 .. T0 + 7 of a warp's 32) from one register set of 16 columns, two tokens per packed f32x2 operation:
 // columns 4 u, 4 u + 1 hold the first-half sums of tokens T0 + 2 u and T0 + 2 u + 1, columns 4 u + 2, 4 u + 3 their second-half

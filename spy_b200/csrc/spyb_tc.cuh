@@ -14,12 +14,9 @@ constexpr int PF_TILE        = PF_M * 32;          // bytes of one s8 operand ti
 constexpr int PF_EPI_WARPS   = 8;                  // epilogue warps: (row quadrant 0..3) x (half of the columns); 12 warps in all leave them 168 registers
 constexpr int PF_BATCH       = 4;                  // blocks per batch: the unit of the copies, of the expansion and of stage reuse
 constexpr int PF_RING        = 4;                  // batches in the shared-memory rings
-constexpr int PF_STAGES      = PF_RING * PF_BATCH; // blocks in the rings
 constexpr int PF_MMA_WARPS   = 2;                  // warps whose first thread issues the MMAs of every PF_MMA_WARPS-th block
 constexpr int PF_THREADS     = (PF_EPI_WARPS + 2 + PF_MMA_WARPS) * 32;   // + the copy warp and the expander warp
-constexpr int PF_EPI_WARPS_F8 = 16;                // the e4m3 form: (row quadrant) x (quarter of the columns); its epilogue needs under 96 registers
-constexpr int PF_MMA_WARPS_F8 = 2;                 // two MMAs and a commit per block hold the issuing thread ~240 cycles
-constexpr int PF_THREADS_F8  = (PF_EPI_WARPS_F8 + 2 + PF_MMA_WARPS_F8) * 32;
+constexpr int PF_GEMM_EPI_WARPS = 16, PF_GEMM_THREADS = 640;   // the Q4_0 / Q8_0 kernel: sixteen epilogue warps and four feeder warps, 96 registers each
 constexpr int PF_DBUF        = 4;                  // accumulator buffers in tensor memory, PF_NCOL columns each (512 columns = all of it)
 
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
@@ -34,9 +31,18 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) { asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(addr), "r"(a), "r"(b) : "memory"); }
+__device__ __forceinline__ float lds32f(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void lds128_2x64(uint32_t addr, uint64_t &a, uint64_t &b) {
+    asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr));
+}
+__device__ __forceinline__ uint64_t lds64u(uint32_t addr) {
+    uint64_t v;
+    asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr));
     return v;
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -66,6 +72,27 @@ __device__ __forceinline__ void mma_f8_ss(uint32_t d_tmem, uint64_t a_desc, uint
                  "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(PF_IDESC_F8), "r"(accumulate), "r"(zero) : "memory");
 }
+// f16 operands, f32 accumulators, 128 x N x 16: D (+)= A B^T. 8-bit integers are exact in f16, their products and the sums of a
+// block's few products are exact in f32
+__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__host__ __device__ constexpr uint32_t idesc_f16(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(PF_M >> 4) << 24); }
+// K-major operand without swizzle, core matrices of 8 rows x 16 bytes: `lbo` bytes between neighbouring 16-byte K chunks, `sbo` bytes
+// between neighbouring groups of eight rows
+__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
+}
+// one lane of a converged warp, the same one every time. Instructions whose operands go through uniform registers (tcgen05.mma,
+// tcgen05.commit, bulk copies) issue at half the cost under this predicate than under `lane == 0` (measured: 69 against 140 cycles
+// per MMA), because the compiler knows that one thread at most is active.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -74,6 +101,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
                    "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -123,8 +154,15 @@ __device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity,
         if (global_timer_ns() - t0 > limit_ns) { return false; }
     }
 }
-// profiling aid: clock stamps of CTA (0, 0) into g.stamps [8 roles][512 blocks][4] (nullptr: off)
-#define PF_STAMP(role, b, i) do { if (g.stamps != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && (b) < 512) { g.stamps[((role) * 512 + (b)) * 4 + (i)] = clock64(); } } while (0)
+// A wait whose fast path is one test and one branch, for loops that count instructions. When it runs out of time it sets limit_ns to
+// zero and returns, and every later wait with the same limit gives up at once: the caller may run through to its end and report then.
+__device__ __forceinline__ void mbar_wait_lean(uint32_t bar, uint32_t parity, uint64_t &limit_ns) {
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u64 t0, t;\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\tmov.u64 t0, %%globaltimer;\n"
+                 "AGAIN:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\tmov.u64 t, %%globaltimer;\n\tsub.u64 t, t, t0;\n\t"
+                 "setp.lt.u64 q, t, %0;\n\t@q bra AGAIN;\n\tmov.u64 %0, 0;\nDONE:\n\t}"
+                 : "+l"(limit_ns) : "r"(bar), "r"(parity) : "memory");
+}
 __device__ __forceinline__ void pf_report(int *error_flag, int code) {
     if (error_flag != nullptr) { atomicExch(error_flag, code); }
 }

@@ -147,6 +147,19 @@ def test_prefill_matmul_matches_oracle(be, oracle, qt, n, k, t, norm):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
+@pytest.mark.parametrize("n,k,t", [(2560, 32, 160), (2560, 96, 160), (2564, 160, 153), (9600, 160, 24), (9476, 224, 23), (640, 4096, 16)])
+def test_prefill_matmul_walks_tiles_of_both_widths(be, oracle, qt, n, k, t):
+    """More tiles than the chip has SMs (a CTA goes on from one tile to the next) in the wide and in the narrow token tiles, with
+    block counts that end inside a step and odd numbers of steps, so that tiles begin on either accumulator buffer."""
+    rng = np.random.default_rng(n + k + t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    got = be.prefill_matmul(qt, w, n, k, x)
+    want = oracle.matmul(qt, w, k, n, x)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
 @pytest.mark.parametrize("n,k,t,norm", [(128, 256, 1, False), (256, 1024, 70, True), (128, 2048, 64, False), (384, 4096, 129, True), (256, 11008 - 11008 % 256, 33, False)])
 def test_prefill_matmul_k_quants_match_the_restatement(be, oracle, qt, n, k, t, norm):
