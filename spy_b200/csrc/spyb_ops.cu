@@ -369,30 +369,137 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(const AttnParams p) {
     p.scratch[((int64_t)t * p.n_head + h) * n_pad + j] = score_dot(kv, reinterpret_cast<const float4 *>(qf));
 }
 
-// The same for a prompt: ATT_TT consecutive tokens per CTA share the K rows, which stay in the threads' registers while
-// the tokens are walked (the K cache is then read once per ATT_TT tokens instead of once per token)
-constexpr int ATT_TT = 8;
-__global__ void __launch_bounds__(256) attn_scores_tiled_kernel(const AttnParams p) {
-    __shared__ __align__(16) float qf[ATT_TT][ATT_HD];
-    const int h = blockIdx.y, t0 = blockIdx.z * ATT_TT, tid = threadIdx.x;
-    const int nt = min(ATT_TT, p.T - t0);
-    const int n_vis_last = p.pos_base[0] + t0 + nt;          // positions the last token of the tile sees
-    if ((int)blockIdx.x * 256 >= n_vis_last) { return; }
+// The same for a prompt, register-tiled: a CTA takes ATT_SG times ATT_ST tokens x ATT_SP positions of a head, a lane 4 tokens x 4
+// positions at a time. The 32 accumulators of a dot product are walked element by element of the CPU's eight-wide vectors: element e of
+// the four accumulators takes the twelve values 32 s + 8 a + e (s = 0..2, a = 0..3), four chains of three FMAs, so that only one to
+// three partial sums per output live at a time instead of 32 accumulators. K and Q lie in shared memory as f32 in that order, value by
+// value: [value][position] and [value][token].
+// 160 f32 operations per (token, position, head). Shared memory gives a warp one word per lane and cycle however often an address
+// repeats, so a word has to serve several products: 16 products per 8 words here (one K row per thread with Q by uniform 128-bit reads:
+// 4 products per 4 words, and every row widened again for every token). 128 tokens of 32 heads over 2000 positions on average:
+// 180 -> 83 us.
+constexpr int ATT_TT = 8;                                    // tokens per CTA of the PV kernel below
+constexpr int ATT_ST = 16, ATT_SP = 128, ATT_KPITCH = ATT_SP + 4, ATT_SC_THREADS = 128;
+constexpr int ATT_SG = 2;                                    // token tiles a CTA walks with the same K rows
+constexpr size_t ATT_SC_SMEM = (size_t)ATT_HD * (ATT_KPITCH + ATT_SG * ATT_ST) * sizeof(float);
+// value 8 c + e of a row -> its place: 12 e + c for the first 96, then 96 + 4 ((e + 1) % 8) + c - 12 (the rotation keeps the pieces c = 8..15
+// of a row on different banks when they are stored side by side)
+__host__ __device__ constexpr int att_value_row(int c, int e) { return c < 12 ? 12 * e + c : 96 + 4 * ((e + 1) & 7) + c - 12; }
+__global__ void __launch_bounds__(ATT_SC_THREADS) attn_scores_tiled_kernel(const AttnParams p) {
+    extern __shared__ __align__(16) float att_smem[];
+    constexpr int NQ = ATT_SG * ATT_ST;
+    float *ks = att_smem, *qs = att_smem + ATT_HD * ATT_KPITCH;
+    const int h = blockIdx.y, tg = blockIdx.z * NQ, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ng = min(NQ, p.T - tg), j0 = blockIdx.x * ATT_SP;
+    const int n_vis_last = p.pos_base[0] + tg + ng;          // positions the last token of the CTA sees
+    if (j0 >= n_vis_last) { return; }
     const int n_pad = (p.n_ctx + 3) & ~3;
-    for (int i = tid; i < nt * ATT_HD; i += 256) { qf[i / ATT_HD][i % ATT_HD] = __half2float(p.q[(int64_t)(t0 + i / ATT_HD) * p.dl + (int64_t)h * ATT_HD + i % ATT_HD]); }
-    __syncthreads();
-    const int j = blockIdx.x * 256 + tid;
-    if (j >= n_vis_last) { return; }
-    uint4 kv[16];
-    {
-        const uint4 *krow = reinterpret_cast<const uint4 *>(p.k_cache + (int64_t)j * p.dl + (int64_t)h * ATT_HD);
+    {   // a warp reads four rows x 128 bytes at a time and writes them value by value (the pitch keeps the 8 x 4 words of a store on 32 banks)
+        const int row0 = tid >> 3, c0 = tid & 7;             // 16-byte pieces c0 and c0 + 8 of rows row0, row0 + 16, ...
 #pragma unroll
-        for (int a = 0; a < 16; ++a) { kv[a] = krow[a]; }
+        for (int half = 0; half < 2; ++half) {
+            const int c = c0 + 8 * half;
+            const __half *src = p.k_cache + (int64_t)(j0 + row0) * p.dl + (int64_t)h * ATT_HD + 8 * c;
+            uint4 w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { w[i] = j0 + row0 + 16 * i < n_vis_last ? *reinterpret_cast<const uint4 *>(src + (int64_t)(16 * i) * p.dl) : make_uint4(0u, 0u, 0u, 0u); }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                float *dst = ks + att_value_row(c, e) * ATT_KPITCH + row0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t u = e < 2 ? w[i].x : e < 4 ? w[i].y : e < 6 ? w[i].z : w[i].w;
+                    dst[16 * i] = h2f((uint16_t)((e & 1) ? u >> 16 : u));
+                }
+            }
+        }
+        static_assert(ATT_SC_THREADS == 8 * 16 && ATT_SP == 16 * 8, "eight pieces x 16 rows per pass, eight passes");
     }
+    {   // a lane takes 16-byte pieces of one token: a store's 32 words are neighbours
+        static_assert(NQ == 32, "one token per lane");
+        const __half *src = p.q + (int64_t)(tg + min(lane, ng - 1)) * p.dl + (int64_t)h * ATT_HD;   // (tokens past the end repeat the last one; their scores are not stored)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = 4 * i + warp;
+            float f[8];
+            unpack8(*reinterpret_cast<const uint4 *>(src + 8 * c), f);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { qs[att_value_row(c, e) * NQ + lane] = f[e]; }
+        }
+    }
+    __syncthreads();
+    const uint32_t k_s = smem_u32(ks + warp * 32 + (lane & 7) * 4);   // (volatile shared loads: the compiler would keep the whole K tile in registers across the token tiles)
+    auto four = [](const float4 v, float (&f)[4]) { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; };
 #pragma unroll 1
-    for (int tt = 0; tt < nt; ++tt) {
-        if (j > p.pos_base[0] + t0 + tt) { continue; }       // masked for this token
-        p.scratch[((int64_t)(t0 + tt) * p.n_head + h) * n_pad + j] = score_dot(kv, reinterpret_cast<const float4 *>(qf[tt]));
+    for (int t0 = 0; t0 < ng; t0 += ATT_ST) {
+        const uint32_t q_s = smem_u32(qs + t0 + (lane >> 3) * 4);
+        float out[4][4], half_sum[4][4], part[4][4];         // [token][position]
+#pragma unroll
+        for (int eo = 0; eo < 8; ++eo) {                     // elements 0, 4, 1, 5, 2, 6, 3, 7: u_e = v_e + v_(e + 4), then (u_0 + u_1) + (u_2 + u_3)
+            const int e = (eo >> 1) + 4 * (eo & 1);
+            float v[4][4];
+#pragma unroll
+            for (int ap = 0; ap < 2; ++ap) {                 // accumulators ap and ap + 2
+                float a[2][4][4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+#pragma unroll
+                    for (int s = 0; s < 3; ++s) {
+                        const int r = att_value_row(4 * s + ap + 2 * i, e);
+                        float k[4], q[4];
+                        four(lds128f(k_s + 4u * r * ATT_KPITCH), k); four(lds128f(q_s + 4u * r * NQ), q);
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) {
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) { a[i][t][j] = fmaf(k[j], q[t], s == 0 ? 0.f : a[i][t][j]); }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { const float x = __fadd_rn(a[0][t][j], a[1][t][j]); v[t][j] = ap == 0 ? x : __fadd_rn(v[t][j], x); }
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if ((eo & 1) == 0) { part[t][j] = v[t][j]; continue; }
+                    const float u = __fadd_rn(part[t][j], v[t][j]);
+                    if (eo == 1 || eo == 5) { half_sum[t][j] = u; continue; }
+                    const float w = __fadd_rn(half_sum[t][j], u);
+                    out[t][j] = eo == 3 ? w : __fadd_rn(out[t][j], w);
+                }
+            }
+        }
+        float tail[4][4];                                    // elements 96..127: scalar chain
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { tail[t][j] = 0.f; }
+        }
+#pragma unroll
+        for (int d = 96; d < ATT_HD; ++d) {
+            const int r = att_value_row(d >> 3, d & 7);
+            float k[4], q[4];
+            four(lds128f(k_s + 4u * r * ATT_KPITCH), k); four(lds128f(q_s + 4u * r * NQ), q);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { tail[t][j] = fmaf(k[j], q[t], tail[t][j]); }
+            }
+        }
+        // (scores of positions a token does not see are written as they come: nothing reads them)
+        const int j = j0 + warp * 32 + (lane & 7) * 4;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int tt = t0 + (lane >> 3) * 4 + t;
+            if (tt < ng && j < n_vis_last && j < n_pad) {
+                *reinterpret_cast<float4 *>(p.scratch + ((int64_t)(tg + tt) * p.n_head + h) * n_pad + j) =
+                    make_float4(__fadd_rn(tail[t][0], out[t][0]), __fadd_rn(tail[t][1], out[t][1]), __fadd_rn(tail[t][2], out[t][2]), __fadd_rn(tail[t][3], out[t][3]));
+            }
+        }
     }
 }
 
@@ -425,30 +532,33 @@ __global__ void __launch_bounds__(ATT_SM_THREADS) attn_softmax_kernel(const Attn
     m = red[0];
 #pragma unroll
     for (int w = 1; w < ATT_SM_THREADS / WARP; ++w) { if (w < (nthr >> 5)) { m = fmaxf(m, red[w]); } }
-    const int n_tot4 = (n_tot + 3) & ~3;
-    for (int j = tid; j < n_tot4; j += nthr) { sc[j] = (j < n_vis) ? p.exp_table[f2h(__fsub_rn(sc[j], m))] : 0.f; }
+    // (masked positions are exact zeros: they decide which elements form a group of four, but a group of zeros leaves the sum as it is,
+    // so the groups behind the last visible position are left out)
+    const int n_sum = min(n_tot, (n_vis + 3) & ~3), n_sum4 = (n_sum + 3) & ~3;
+    for (int j = tid; j < n_sum4; j += nthr) { sc[j] = (j < n_vis) ? p.exp_table[f2h(__fsub_rn(sc[j], m))] : 0.f; }
     __syncthreads();
-    for (int g = tid; g < (n_tot >> 2); g += nthr) {
+    const int ng = min(n_tot >> 2, n_sum4 >> 2);
+    for (int g = tid; g < ng; g += nthr) {
         const float4 v = reinterpret_cast<const float4 *>(sc)[g];
         gs[g] = __fadd_rn(__fadd_rn(v.x, v.y), __fadd_rn(v.z, v.w));
     }
     __syncthreads();
     if (tid == 0) {
         float sum = 0.f;
-        const int ng = n_tot >> 2;
         int g = 0;
         for (; g + 4 <= ng; g += 4) {
             const float4 v = *reinterpret_cast<const float4 *>(gs + g);
             sum = __fadd_rn(sum, v.x); sum = __fadd_rn(sum, v.y); sum = __fadd_rn(sum, v.z); sum = __fadd_rn(sum, v.w);
         }
         for (; g < ng; ++g) { sum = __fadd_rn(sum, gs[g]); }
-        for (int j = ng << 2; j < n_tot; ++j) { sum = __fadd_rn(sum, sc[j]); }
+        for (int j = ng << 2; j < n_sum; ++j) { sum = __fadd_rn(sum, sc[j]); }
         bcast = __fdiv_rn(1.0f, sum);
     }
     __syncthreads();
     const float inv = bcast;
     // probabilities, rounded to fp16 as the PV MatMul does with its f32 operand
     for (int j = tid; j < n_vis; j += nthr) { row[j] = __half2float(__float2half_rn(__fmul_rn(sc[j], inv))); }
+    if (tid < WARP + ATT_TT) { const int j = n_vis + tid; if (j < min(n_pad, (n_vis + ATT_TT - 1 + 31) & ~31)) { row[j] = 0.f; } }   // (read by the tiled PV kernel)
 }
 
 constexpr int ATT_PV_WARPS = 16;
@@ -496,143 +606,147 @@ __global__ void __launch_bounds__(ATT_PV_WARPS * WARP) attn_pv_kernel(const Attn
     tp_publish(p.tp, p.T);
 }
 
-// PV for a prompt: ATT_TT consecutive tokens per CTA share the V^T rows, and a warp takes ATT_EE output elements, so that a
-// probability read from shared memory serves ATT_EE products. Every token's product is the untiled kernel's (same lanes,
-// same steps, same tail); only the loads are shared.
-constexpr int ATT_EE = 4;
-__global__ void __launch_bounds__(ATT_PV_WARPS * WARP) attn_pv_tiled_kernel(const AttnParams p) {
-    extern __shared__ __align__(16) float att_smem[];
-    constexpr int PER_CTA = ATT_PV_WARPS * ATT_EE;            // output elements per CTA
-    const int per_head = ATT_HD / PER_CTA;
-    const int h = blockIdx.x / per_head, e0 = (blockIdx.x % per_head) * PER_CTA + (threadIdx.x >> 5) * ATT_EE, t0 = blockIdx.y * ATT_TT;
-    const int tid = threadIdx.x, lane = tid & 31;
+// PV for a prompt: a CTA takes ATT_PVT_ELEMS output elements of a head for ATT_TT consecutive tokens. The 32 accumulators of an output
+// (position j of a 32-step belongs to accumulator j % 32) lie in the registers of eight lanes, four each, so that a lane reads four
+// neighbouring positions at once (64 bits of V^T, 128 bits of a token's probabilities); a lane takes two output elements, a warp eight,
+// for all ATT_TT tokens. The eight lanes of an output meet once at the end, halving the number of tokens a lane keeps at every step of
+// the tree, and each lane then runs the scalar tails of its token.
+// 128 f32 operations per (token, position, head). The probabilities of ATT_CH positions at a time run through a ring in shared memory with
+// cp.async (the softmax kernel leaves zeros behind a token's last position, as far as a tile reads): no staging phase in front of the
+// products, and CTAs small enough that four share an SM. 128 tokens of 32 heads over 2000 positions on average: 220 -> 101 us (whole rows
+// staged first, one CTA per SM: 119; four elements per lane: 138; probabilities straight from L1: 290).
+constexpr int ATT_PVT_WARPS = 4, ATT_EE = 2, ATT_PVT_ELEMS = ATT_PVT_WARPS * 4 * ATT_EE;
+constexpr int ATT_CH = 128, ATT_CH_RING = 4;
+__global__ void __launch_bounds__(ATT_PVT_WARPS * WARP, 16 / ATT_PVT_WARPS) attn_pv_tiled_kernel(const AttnParams p) {
+    constexpr int PER_HEAD = ATT_HD / ATT_PVT_ELEMS;
+    const int h = blockIdx.x / PER_HEAD, t0 = blockIdx.y * ATT_TT, tid = threadIdx.x, lane = tid & 31, grp = lane >> 3, lg = lane & 7;
+    const int e0 = (blockIdx.x % PER_HEAD) * ATT_PVT_ELEMS + (tid >> 5) * 4 * ATT_EE + grp * ATT_EE;
     const int nt = min(ATT_TT, p.T - t0);
     const int n_tot = (p.pos_base[1] > 0) ? p.pos_base[1] : p.pos_base[0] + p.T;
     const int n_pad = (p.n_ctx + 3) & ~3;
     const int n_main = ((n_tot - 1) / 32) * 32;
     const int vis0 = p.pos_base[0] + t0 + 1;                  // positions token t0 + tt sees: vis0 + tt
     const int vis_last = vis0 + nt - 1;
-    // probabilities of the tile's tokens; positions a token does not see read as +0 (they leave its accumulators unchanged)
-    for (int tt = 0; tt < nt; ++tt) {
-        const float *row = p.scratch + ((int64_t)(t0 + tt) * p.n_head + h) * n_pad;
-        float *pr = att_smem + (size_t)tt * n_pad;
-        for (int j = tid; j < vis_last; j += ATT_PV_WARPS * WARP) { pr[j] = (j < vis0 + tt) ? row[j] : 0.f; }
-    }
-    __syncthreads();
+    const int n_steps = (min(n_main, vis_last) + 31) >> 5;    // (steps behind the tile's last visible position add nothing)
     const __half *vrow = p.v_cache + ((int64_t)h * ATT_HD + e0) * p.n_ctx;   // row e0 + ee starts ee * n_ctx further
-    float acc[ATT_TT][ATT_EE];
+    constexpr int AHEAD = ATT_CH / 32;                        // steps whose V^T values are in flight
+    uint2 vq[AHEAD][ATT_EE];
+    auto fetch = [&](int step, uint2 (&dst)[ATT_EE]) {
+        const int j = 32 * step + 4 * lg;
+#pragma unroll
+        for (int ee = 0; ee < ATT_EE; ++ee) {
+            dst[ee] = make_uint2(0u, 0u);
+            if (step < n_steps && j < vis_last) { dst[ee] = __ldg(reinterpret_cast<const uint2 *>(vrow + (int64_t)ee * p.n_ctx + j)); }
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < AHEAD; ++s) { fetch(s, vq[s]); }
+    const int64_t row_pitch = (int64_t)p.n_head * n_pad;      // (tokens past the end repeat the last one; their results are not stored)
+    const float *rows = p.scratch + ((int64_t)t0 * p.n_head + h) * n_pad;
+    __shared__ __align__(16) float probs[ATT_CH_RING][ATT_TT][ATT_CH];
+    const int n_chunks = (n_steps + AHEAD - 1) / AHEAD, row_end = 32 * n_steps;
+    auto stage = [&](int c) {   // 16 bytes per thread and pass; one commit group per chunk, empty ones behind the last
+        if (c < n_chunks) {
+#pragma unroll
+            for (int i = tid; i < ATT_TT * (ATT_CH / 4); i += ATT_PVT_WARPS * WARP) {
+                const int tt = i / (ATT_CH / 4), j = 4 * (i % (ATT_CH / 4));
+                if (c * ATT_CH + j < row_end) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&probs[c % ATT_CH_RING][tt][j])), "l"(__cvta_generic_to_global(rows + min(tt, nt - 1) * row_pitch + c * ATT_CH + j)) : "memory");
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int c = 0; c < ATT_CH_RING - 1; ++c) { stage(c); }
+    float acc[ATT_TT][ATT_EE][4];
 #pragma unroll
     for (int tt = 0; tt < ATT_TT; ++tt) {
 #pragma unroll
-        for (int ee = 0; ee < ATT_EE; ++ee) { acc[tt][ee] = 0.f; }
-    }
-    int j0 = 0;
-    if (nt == ATT_TT) {
-        // positions every token of the tile sees, in chunks of four 32-position steps: no masks to test, and the V^T values of
-        // the next chunk are requested before the products of this one, so that their latency hides behind 128 FMAs per thread
-        constexpr int CH = 4;
-        const int full_end = (min(n_main, vis0) / (32 * CH)) * (32 * CH);
-        __half vh[CH][ATT_EE];
-        if (full_end > 0) {
+        for (int ee = 0; ee < ATT_EE; ++ee) {
 #pragma unroll
-            for (int s = 0; s < CH; ++s) {
-#pragma unroll
-                for (int ee = 0; ee < ATT_EE; ++ee) { vh[s][ee] = vrow[(int64_t)ee * p.n_ctx + 32 * s + lane]; }
-            }
-        }
-        for (; j0 < full_end; j0 += 32 * CH) {
-            float v[CH][ATT_EE];
-#pragma unroll
-            for (int s = 0; s < CH; ++s) {
-#pragma unroll
-                for (int ee = 0; ee < ATT_EE; ++ee) { v[s][ee] = __half2float(vh[s][ee]); }
-            }
-            if (j0 + 32 * CH < full_end) {
-#pragma unroll
-                for (int s = 0; s < CH; ++s) {
-#pragma unroll
-                    for (int ee = 0; ee < ATT_EE; ++ee) { vh[s][ee] = vrow[(int64_t)ee * p.n_ctx + j0 + 32 * (CH + s) + lane]; }
-                }
-            }
-#pragma unroll
-            for (int tt = 0; tt < ATT_TT; ++tt) {
-                const float *pr = att_smem + (size_t)tt * n_pad + j0 + lane;
-#pragma unroll
-                for (int s = 0; s < CH; ++s) {
-                    const float pv = pr[32 * s];
-#pragma unroll
-                    for (int ee = 0; ee < ATT_EE; ++ee) { acc[tt][ee] = fmaf(v[s][ee], pv, acc[tt][ee]); }
-                }
-            }
+            for (int k = 0; k < 4; ++k) { acc[tt][ee][k] = 0.f; }
         }
     }
-    for (; j0 + 2 * 32 <= n_main && j0 + 2 * 32 <= vis_last; j0 += 2 * 32) {   // two steps' loads in flight per element
-        float v[2][ATT_EE];
+    auto widen = [](const uint2 w, float (&f)[4]) {
+        const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&w.x)), hi = __half22float2(*reinterpret_cast<const __half2 *>(&w.y));
+        f[0] = lo.x; f[1] = lo.y; f[2] = hi.x; f[3] = hi.y;
+    };
+    for (int c = 0, s0 = 0; c < n_chunks; ++c, s0 += AHEAD) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ATT_CH_RING - 2) : "memory");
+        __syncthreads();                                      // chunk c is there for everyone, and everyone is done with chunk c - 1
+        stage(c + ATT_CH_RING - 1);
+        const float *pr = &probs[c % ATT_CH_RING][0][4 * lg];
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < AHEAD; ++s) {
+            if (s0 + s < n_steps) {
+                float v[ATT_EE][4];
+                const int over = 32 * (s0 + s) + 4 * lg + 4 - vis_last;   // (cache entries behind the last visible position may not be written yet)
+                if (over > 0) {
 #pragma unroll
-            for (int ee = 0; ee < ATT_EE; ++ee) { v[s][ee] = __half2float(vrow[(int64_t)ee * p.n_ctx + j0 + 32 * s + lane]); }
-        }
+                    for (int ee = 0; ee < ATT_EE; ++ee) {
+                        if (over >= 1) { vq[s][ee].y &= 0xffffu; }
+                        if (over >= 2) { vq[s][ee].y = 0u; }
+                        if (over >= 3) { vq[s][ee].x &= 0xffffu; }
+                    }
+                }
 #pragma unroll
-        for (int tt = 0; tt < ATT_TT; ++tt) {
-            if (tt < nt) {
-                const float *pr = att_smem + (size_t)tt * n_pad;
+                for (int ee = 0; ee < ATT_EE; ++ee) { widen(vq[s][ee], v[ee]); }
+                fetch(s0 + s + AHEAD, vq[s]);
 #pragma unroll
-                for (int s = 0; s < 2; ++s) {
-                    if (j0 + 32 * s < vis0 + tt) {   // (a step wholly behind the token's last position adds nothing: skipped as in the untiled kernel)
-                        const float pv = pr[j0 + 32 * s + lane];
+                for (int tt = 0; tt < ATT_TT; ++tt) {
+                    const float4 pv = *reinterpret_cast<const float4 *>(pr + tt * ATT_CH + 32 * s);
 #pragma unroll
-                        for (int ee = 0; ee < ATT_EE; ++ee) { acc[tt][ee] = fmaf(v[s][ee], pv, acc[tt][ee]); }
+                    for (int ee = 0; ee < ATT_EE; ++ee) {
+                        acc[tt][ee][0] = fmaf(v[ee][0], pv.x, acc[tt][ee][0]); acc[tt][ee][1] = fmaf(v[ee][1], pv.y, acc[tt][ee][1]);
+                        acc[tt][ee][2] = fmaf(v[ee][2], pv.z, acc[tt][ee][2]); acc[tt][ee][3] = fmaf(v[ee][3], pv.w, acc[tt][ee][3]);
                     }
                 }
             }
         }
     }
-    for (; j0 < n_main && j0 < vis_last; j0 += 32) {   // (steps behind the tile's last visible position add nothing)
-        const int j = j0 + lane;
-        float v[ATT_EE];
+    // FP16::block_reduce (vec_util.h:61-71): lane lg holds accumulator lg / 2, elements 4 (lg % 2) .. + 3. (s0 + s2) + (s1 + s3) are the
+    // exchanges with lanes lg ^ 4 and lg ^ 2, element l with l + 4 the one with lg ^ 1. At each exchange a lane hands over half of its
+    // tokens and keeps the sums of the others: in the end lane lg holds token lg.
 #pragma unroll
-        for (int ee = 0; ee < ATT_EE; ++ee) { v[ee] = (j < vis_last) ? __half2float(vrow[(int64_t)ee * p.n_ctx + j]) : 0.f; }
+    for (int half = ATT_TT / 2; half > 0; half >>= 1) {       // 4, 2, 1: also the lane distance
+        const bool up = (lg & half) != 0;
 #pragma unroll
-        for (int tt = 0; tt < ATT_TT; ++tt) {
-            if (tt < nt && j < vis0 + tt) {
-                const float pv = att_smem[(size_t)tt * n_pad + j];
+        for (int tt = 0; tt < half; ++tt) {
 #pragma unroll
-                for (int ee = 0; ee < ATT_EE; ++ee) { acc[tt][ee] = fmaf(v[ee], pv, acc[tt][ee]); }
+            for (int ee = 0; ee < ATT_EE; ++ee) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float keep = up ? acc[tt + half][ee][k] : acc[tt][ee][k], give = up ? acc[tt][ee][k] : acc[tt + half][ee][k];
+                    acc[tt][ee][k] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, half));
+                }
             }
         }
     }
-    // The vector parts: reduce_f16dot_lanes leaves every lane with the sum; lane 4 tt + ee keeps that of (token tt, element ee).
-    static_assert(ATT_TT * ATT_EE == WARP, "one lane per (token, element) of the warp's outputs");
-    const int my_tt = lane >> 2, my_ee = lane & 3;
-    float vec = 0.f;
-#pragma unroll
-    for (int tt = 0; tt < ATT_TT; ++tt) {
-#pragma unroll
-        for (int ee = 0; ee < ATT_EE; ++ee) {
-            const float a = reduce_f16dot_lanes(acc[tt][ee]);
-            if (lane == tt * ATT_EE + ee) { vec = a; }
-        }
-    }
-    // The scalar tails (positions n_main .. n_tot - 1, at most 32, one FMA chain per output): each lane runs the chain of its own
-    // (token, element) instead of all lanes running all 32 chains; the V^T value of position n_main + i sits in lane i
-    float vt[ATT_EE];
-#pragma unroll
-    for (int ee = 0; ee < ATT_EE; ++ee) { vt[ee] = (n_main + lane < vis_last) ? __half2float(vrow[(int64_t)ee * p.n_ctx + n_main + lane]) : 0.f; }
-    float tail = 0.f;
-    const float *pr_mine = att_smem + (size_t)my_tt * n_pad + n_main;
-    const int n_tail = min(32, vis0 + my_tt - n_main);        // positions of the tail this lane's token sees (<= 0: none)
-#pragma unroll 4
-    for (int i = 0; i < 32; ++i) {
-        float v = 0.f;
+    static_assert(ATT_TT == 8, "one lane of a group of eight per token");
+    // the scalar tails (positions n_main .. n_tot - 1, at most 32, as far as the lane's token sees them), one FMA chain per output
+    if (lg >= nt) { return; }
+    const int n_tail = min(32, vis0 + lg - n_main);
+    const float *pr = rows + lg * row_pitch + n_main;
+    float tail[ATT_EE] = {};
+    for (int i = 0; i < n_tail; i += 4) {
+        const float4 q = *reinterpret_cast<const float4 *>(pr + i);
 #pragma unroll
         for (int ee = 0; ee < ATT_EE; ++ee) {
-            const float w = __shfl_sync(0xffffffffu, vt[ee], i);
-            if (my_ee == ee) { v = w; }
+            float w[4];
+            widen(*reinterpret_cast<const uint2 *>(vrow + (int64_t)ee * p.n_ctx + n_main + i), w);
+            tail[ee] = fmaf(w[0], q.x, tail[ee]);
+            if (i + 1 < n_tail) { tail[ee] = fmaf(w[1], q.y, tail[ee]); }
+            if (i + 2 < n_tail) { tail[ee] = fmaf(w[2], q.z, tail[ee]); }
+            if (i + 3 < n_tail) { tail[ee] = fmaf(w[3], q.w, tail[ee]); }
         }
-        if (i < n_tail) { tail = fmaf(v, pr_mine[i], tail); }
     }
-    if (my_tt < nt) { p.out[(int64_t)(t0 + my_tt) * (p.out_stride ? p.out_stride : p.dl) + (int64_t)h * ATT_HD + e0 + my_ee] = __fadd_rn(tail, vec); }
+    float *dst = p.out + (int64_t)(t0 + lg) * (p.out_stride ? p.out_stride : p.dl) + (int64_t)h * ATT_HD + e0;
+#pragma unroll
+    for (int ee = 0; ee < ATT_EE; ++ee) {
+        const float vec = __fadd_rn(__fadd_rn(acc[0][ee][0], acc[0][ee][1]), __fadd_rn(acc[0][ee][2], acc[0][ee][3]));
+        dst[ee] = __fadd_rn(tail[ee], vec);
+    }
 }
 
 static cudaError_t launch_with_pdl(const void *kernel, dim3 grid, dim3 block, size_t smem, const AttnParams &p, const LaunchCfg &cfg) {
@@ -656,8 +770,10 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
     const size_t n_pad = ((size_t)p.n_ctx + 3) & ~(size_t)3;
     if ((p.n_ctx > ATT_LONG_MIN || p.force_long) && p.scratch != nullptr) {
         const bool tiled = p.T >= ATT_TT && p.tp.counter == nullptr && !cfg.pdl && p.seq_stride == 0;   // a prompt: tokens share the K rows and the V^T rows
-        cudaError_t err = tiled
-            ? launch_with_pdl(reinterpret_cast<const void *>(attn_scores_tiled_kernel), dim3((unsigned)((p.n_ctx + 255) / 256), p.n_head, (unsigned)((p.T + ATT_TT - 1) / ATT_TT)), dim3(256), 0, p, cfg)
+        cudaError_t err = tiled ? allow_dynamic_smem(reinterpret_cast<const void *>(attn_scores_tiled_kernel), ATT_SC_SMEM) : cudaSuccess;
+        if (err != cudaSuccess) { return err; }
+        err = tiled
+            ? launch_with_pdl(reinterpret_cast<const void *>(attn_scores_tiled_kernel), dim3((unsigned)((p.n_ctx + ATT_SP - 1) / ATT_SP), p.n_head, (unsigned)((p.T + ATT_SG * ATT_ST - 1) / (ATT_SG * ATT_ST))), dim3(ATT_SC_THREADS), ATT_SC_SMEM, p, cfg)
             : launch_with_pdl(reinterpret_cast<const void *>(attn_scores_kernel), dim3((unsigned)((p.n_ctx + 255) / 256), p.n_head, p.T), dim3(256), 0, p, cfg);
         if (err != cudaSuccess) { return err; }
         const size_t sm_smem = (n_pad + n_pad / 4) * sizeof(float) + 16;
@@ -666,12 +782,8 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
         if (err != cudaSuccess) { return err; }
         err = launch_with_pdl(reinterpret_cast<const void *>(attn_softmax_kernel), dim3(p.n_head, p.T), dim3(tiled ? 256 : ATT_SM_THREADS), sm_smem, p, cfg);
         if (err != cudaSuccess) { return err; }
-        if (tiled && (size_t)ATT_TT * n_pad * sizeof(float) + 16 <= 200 * 1024) {
-            const size_t tsm = (size_t)ATT_TT * n_pad * sizeof(float) + 16;
-            err = allow_dynamic_smem(reinterpret_cast<const void *>(attn_pv_tiled_kernel), tsm);
-            if (err != cudaSuccess) { return err; }
-            return launch_with_pdl(reinterpret_cast<const void *>(attn_pv_tiled_kernel), dim3(p.n_head * (ATT_HD / (ATT_PV_WARPS * ATT_EE)), (unsigned)((p.T + ATT_TT - 1) / ATT_TT)),
-                                   dim3(ATT_PV_WARPS * WARP), tsm, p, cfg);
+        if (tiled) {
+            return launch_with_pdl(reinterpret_cast<const void *>(attn_pv_tiled_kernel), dim3(p.n_head * (ATT_HD / ATT_PVT_ELEMS), (unsigned)((p.T + ATT_TT - 1) / ATT_TT)), dim3(ATT_PVT_WARPS * WARP), 0, p, cfg);
         }
         const size_t pv_smem = n_pad * sizeof(float) + 16;
         err = allow_dynamic_smem(reinterpret_cast<const void *>(attn_pv_kernel), pv_smem);

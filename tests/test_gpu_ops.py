@@ -545,6 +545,21 @@ def test_attention_of_a_prompt_shares_k_and_v_rows(be, oracle, pos0, t, n_total)
     assert np.array_equal(bits(got), bits(want))
 
 
+@pytest.mark.parametrize("pos0,t,n_total,n_ctx", [(0, 33, 0, 1028), (95, 34, 0, 1060), (896, 130, 1026, 1032), (1000, 41, 1100, 1100)])
+def test_attention_of_a_prompt_across_its_tiles(be, oracle, pos0, t, n_total, n_ctx):
+    """More than 32 tokens (a second group of the scores kernel), more than one chunk of 128 positions, contexts whose last K rows and
+    last chunk are ragged, and masked positions behind the last token."""
+    rng = np.random.default_rng(pos0 + t)
+    n_head, hd = 2, 128
+    d = n_head * hd
+    q16 = oracle.quantize_f16(rng.standard_normal(t * d).astype(np.float32)).reshape(t, d)
+    k16 = oracle.quantize_f16(rng.standard_normal(n_ctx * d).astype(np.float32)).reshape(n_ctx, d)
+    vt16 = oracle.quantize_f16(rng.standard_normal(n_ctx * d).astype(np.float32)).reshape(d, n_ctx)
+    got = be.attention(q16, k16, vt16, pos0, n_head, hd, n_ctx, n_total)
+    want = _attention_oracle(oracle, q16, k16, vt16, pos0, n_head, hd, n_ctx, n_total)
+    assert np.array_equal(bits(got), bits(want))
+
+
 def test_lookup_tables_identical_for_every_key(be, oracle):
     silu, ex = be.read_tables()
     want_silu, want_exp = oracle.tables()
