@@ -10,14 +10,19 @@
 //   Q6_K:  acc = 0; for the 16 groups g of 16 values:    acc = fma((d * sc_g) * dx_(g/2), (float)sum(q * y), acc)
 // and the row's result = the super-blocks' values added in order. The integer sums are exact, so only this order matters.
 //
-// Mapping: a super-block's value depends on nothing before it, so the lanes of a (half-)warp take the super-blocks of
-// one row side by side - each lane streams its 144 (208 + 2) bytes with 128-bit read-only loads, consecutive lanes
-// consecutive super-blocks, i.e. the warp reads the row as one contiguous run - and the per-row sum is a short ordered
-// walk over the lanes' values. A warp owns a pair of rows (rows 2u, 2u+1 rotate together in RoPE; FFN up row i and gate
-// row i meet in the SiLU epilogue). HBM-bound: rows * K/256 * 144 (210) bytes per launch, read once, no re-tiling for
-// Q4_K; Q6_K rows are re-laid at upload so that every piece is 16-byte aligned (208-byte bodies, the fp16 scales of a
-// row together at its end). Activations: Q8_0 in shared memory, one 68-word stride per super-block so that a block's words
-// are aligned 128-bit reads and the lanes of a quarter-warp, working on different super-blocks, hit different banks.
+// Mapping: a super-block's value depends on nothing before it, so the lanes of a warp take the super-blocks of a unit (NP pairs of
+// neighbouring rows: rows 2q, 2q+1 rotate together in RoPE; FFN up row q and gate row q meet in the SiLU epilogue) side by side, 32 at a
+// time (a round), leave their values in shared memory, and one lane per row and column adds a row's values in order.
+// Streaming: every warp pulls its rounds through a private ring with cp.async.bulk (a round is one or two contiguous runs of 32 x 144 or
+// 208 bytes); the first copies are issued before griddepcontrol.wait, so the previous kernel's tail and the serial prologue pass while
+// the weights arrive; a lane takes its super-block into registers (the 144- and 208-byte pitches are odd multiples of 16: conflict-free
+// 128-bit reads) and the stage is refilled before the arithmetic begins.
+// Roofline: HBM-bound, rows * K/256 * 144 (210) bytes per launch, read once; Q4_K rows as the file has them, Q6_K rows re-laid at upload so
+// that every piece is 16-byte aligned (208-byte bodies, the fp16 scales of a row together at its end).
+// Activations in shared memory as one record per super-block: 64 words of Q8_0 values, 8 scales, 16 sums of 16 values as floats, at a
+// pitch of 92 words, again an odd multiple of 16 bytes, so that the lanes' 128-bit reads of different super-blocks are conflict-free.
+// Against lanes that read their super-blocks from global memory when they got to them: 11008 x 4096 Q4_K, four columns, 22.5 -> 15.4 us; a
+// decode step of eight 7B layers (Q4_K / Q6_K) 0.75 -> 0.52 ms.
 
 #include <algorithm>
 
@@ -30,250 +35,353 @@ namespace spyb {
 
 constexpr int KQ_THREADS = 512;
 constexpr int KQ_WARPS   = KQ_THREADS / WARP;
-constexpr int KQ_SB_WORDS = 68;   // words per super-block of activations in shared memory: 64 + 4, so that a block's eight words are two aligned
-                                  // 128-bit reads and the eight lanes of a quarter-warp (one super-block each) hit distinct banks
+constexpr int KQ_REC = 92;               // words per super-block of activations: 64 values, 8 scales, 16 half-block sums, 4 of padding
+constexpr int KQ_MAX_STAGES = 4;
 
-// the planes of one activation column; column t of a pass lies t * col 32-bit words further (all three planes)
-struct KqPlanes { uint32_t *y; float *dx; int *ysum; int col; };
-
-// NormRMS + Mul(weight) (optional) + Quantizator<FP32,Q8_0> of one activation column into the K-quant planes; the
-// arithmetic is that of the Q4_0 / Q8_0 kernels' prologue (same device functions)
+// NormRMS + Mul(weight) (optional) + Quantizator<FP32,Q8_0> of the pass's columns into the activation records (column t lies col words
+// further); the arithmetic is that of the Q4_0 / Q8_0 kernels' prologue (same device functions). The columns' running sums of squares run
+// side by side, one warp each.
 template <bool NORM>
-__device__ __forceinline__ void kq_prologue(const MatvecParams &p, const float *x, KqPlanes a, float *v3, float *scale_s) {
+__device__ __forceinline__ void kq_prologue(const MatvecParams &p, int nT, uint32_t *rec, int col, float *scale_s) {
     const int tid = threadIdx.x;
     const int n4  = (int)(p.A.k >> 2);
-    const float4 *x4 = reinterpret_cast<const float4 *>(x);
-    float scale = 1.f;
     if (NORM) {
-        for (int g = tid; g < n4; g += KQ_THREADS) {
-            const float4 v = __ldcg(x4 + g);
-            const float v1 = fmaf(v.y, v.y, __fmul_rn(v.x, v.x));
-            const float v2 = fmaf(v.w, v.w, __fmul_rn(v.z, v.z));
-            v3[g] = __fadd_rn(v1, v2);
+#pragma unroll 1
+        for (int t = 0; t < nT; ++t) {
+            const float4 *x4 = reinterpret_cast<const float4 *>(p.x + (int64_t)t * p.x_stride);
+            float *v3 = reinterpret_cast<float *>(rec + t * col);   // (n4 = 64 words per super-block: inside the column's records)
+            for (int g = tid; g < n4; g += KQ_THREADS) {
+                const float4 v = __ldcg(x4 + g);
+                const float v1 = fmaf(v.y, v.y, __fmul_rn(v.x, v.x));
+                const float v2 = fmaf(v.w, v.w, __fmul_rn(v.z, v.z));
+                v3[g] = __fadd_rn(v1, v2);
+            }
         }
         __syncthreads();
-        if (tid == 0) {
-            const float sum  = running_sum_serial(v3, n4);
+        if ((tid & 31) == 0 && (tid >> 5) < nT) {
+            const float sum  = running_sum_serial(reinterpret_cast<const float *>(rec + (tid >> 5) * col), n4);
             const float mean = __fdiv_rn(sum, (float)p.A.k);
-            *scale_s = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
+            scale_s[tid >> 5] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
         }
-        __syncthreads();   // also: the partials (aliasing the planes) are dead from here on
-        scale = *scale_s;
+        __syncthreads();   // also: the partials (aliasing the records) are dead from here on
     }
     const float4 *w4 = reinterpret_cast<const float4 *>(p.norm_w);
-    for (int base = 0; base < n4; base += KQ_THREADS) {   // n4 is a multiple of 64: whole warps, whole blocks
-        const int g = base + tid;
-        const bool valid = g < n4;
-        float4 v = valid ? __ldcg(x4 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (NORM && valid) {
-            const float4 w = w4[g];
-            v.x = __fmul_rn(__fmul_rn(v.x, scale), w.x); v.y = __fmul_rn(__fmul_rn(v.y, scale), w.y);
-            v.z = __fmul_rn(__fmul_rn(v.z, scale), w.z); v.w = __fmul_rn(__fmul_rn(v.w, scale), w.w);
-        }
-        uint16_t dh; int s;
-        const uint32_t q = quantize_q8_lane4(v, dh, s);
-        s += __shfl_xor_sync(0xffffffffu, s, 1); s += __shfl_xor_sync(0xffffffffu, s, 2); s += __shfl_xor_sync(0xffffffffu, s, 4);
-        if (valid) {
-            const int b = g >> 3, w = g & 7;
-            a.y[(b >> 3) * KQ_SB_WORDS + (b & 7) * 8 + w] = q;
-            if (w == 0) { a.dx[b] = h2f(dh); a.ysum[b] = s; }
+#pragma unroll 1
+    for (int t = 0; t < nT; ++t) {
+        const float4 *x4 = reinterpret_cast<const float4 *>(p.x + (int64_t)t * p.x_stride);
+        const float scale = NORM ? scale_s[t] : 1.f;
+        for (int base = 0; base < n4; base += KQ_THREADS) {   // n4 is a multiple of 64: whole warps, whole blocks
+            const int g = base + tid;
+            const bool valid = g < n4;
+            float4 v = valid ? __ldcg(x4 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (NORM && valid) {
+                const float4 w = w4[g];
+                v.x = __fmul_rn(__fmul_rn(v.x, scale), w.x); v.y = __fmul_rn(__fmul_rn(v.y, scale), w.y);
+                v.z = __fmul_rn(__fmul_rn(v.z, scale), w.z); v.w = __fmul_rn(__fmul_rn(v.w, scale), w.w);
+            }
+            uint16_t dh; int s;
+            const uint32_t q = quantize_q8_lane4(v, dh, s);
+            s += __shfl_xor_sync(0xffffffffu, s, 1); s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if (valid) {
+                const int b = g >> 3, w = g & 7;
+                uint32_t *r = rec + t * col + (b >> 3) * KQ_REC;
+                r[(b & 7) * 8 + w] = q;
+                if (w == 0) { r[64 + (b & 7)] = __float_as_uint(h2f(dh)); }
+                if ((w & 3) == 0) { r[72 + 2 * (b & 7) + (w >> 2)] = __float_as_uint((float)s); }
+            }
         }
     }
 }
 
-__device__ __forceinline__ uint4 ldg_nc(const uint8_t *p) {
-    uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
+// byte i of w (a constant) as the float 2^23 + byte: the byte becomes the low bits of a float's mantissa
+template <int I> __device__ __forceinline__ float kq_byte_magic(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 | I)); }
 
-// 6-bit scale / min j of a Q4_K super-block from its 12 packed bytes (three words)
-__device__ __forceinline__ void kq_scale_min(const uint32_t (&sw)[3], int j, float &sc, float &mn) {
-    auto byte = [&](int i) { return (sw[i >> 2] >> (8 * (i & 3))) & 0xffu; };
-    if (j < 4) { sc = (float)(byte(j) & 63u); mn = (float)(byte(j + 4) & 63u); }
-    else { sc = (float)((byte(j + 4) & 0xFu) | ((byte(j - 4) >> 6) << 4)); mn = (float)((byte(j + 4) >> 4) | ((byte(j) >> 6) << 4)); }
-}
-
-// values of one Q4_K super-block for the nT <= TM activation columns of a pass: wb = its 144 bytes in global memory, sb = its
-// index (the activations of column t: 8 blocks x 8 words at a.y + t * a.col + sb * KQ_SB_WORDS, their scales and integer
-// sums at a.dx / a.ysum + t * a.col + 8 * sb). The weights are read and unpacked once for all columns.
-template <int TM>
-__device__ __forceinline__ void kq_values_q4k(const uint8_t *wb, const KqPlanes &a, int sb, int nT, float (&acc)[TM]) {
-    const uint4 hd = ldg_nc(wb);
-    uint4 q[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { q[i] = ldg_nc(wb + 16 + 16 * i); }
-    const float2 dm = __half22float2(*reinterpret_cast<const __half2 *>(&hd.x));   // d, dmin
-    const uint32_t sw[3] = {hd.y, hd.z, hd.w};
+// values of one Q4_K super-block (its 144 bytes in w) for the TM activation columns of a pass: rec_s = shared-space address of the
+// super-block's activation record of column 0, the next column's col_bytes further. The weights are unpacked once for all columns.
+template <int TM, int NW>
+__device__ __forceinline__ void kq_values_q4k(const uint4 (&w)[NW], uint32_t rec_s, uint32_t col_bytes, float (&acc)[TM]) {
+    const float2 dm = __half22float2(*reinterpret_cast<const __half2 *>(&w[0].x));   // d, dmin
+    // the eight 6-bit scales and minima, four to a word; d * sc in one operation: fma(d, 2^23 + sc, -(d * 2^23)) rounds the exact product once
+    const uint32_t scw[2] = {w[0].y & 0x3f3f3f3fu, (w[0].w & 0x0f0f0f0fu) | ((w[0].y >> 2) & 0x30303030u)};
+    const uint32_t mnw[2] = {w[0].z & 0x3f3f3f3fu, ((w[0].w >> 4) & 0x0f0f0f0fu) | ((w[0].z >> 2) & 0x30303030u)};
+    const float dbase = __fmul_rn(dm.x, -8388608.f), mbase = __fmul_rn(dm.y, 8388608.f);
 #pragma unroll
     for (int t = 0; t < TM; ++t) { acc[t] = 0.f; }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {          // sub-block j: bytes 32 * (j / 2) .. + 31 of qs, low nibbles when j is even
-        const uint4 qa = q[2 * (j >> 1)], qb = q[2 * (j >> 1) + 1];
+    for (int jp = 0; jp < 4; ++jp) {           // sub-blocks 2 jp and 2 jp + 1: the low and the high nibbles of bytes 32 jp .. + 31 of qs
+        const uint4 qa = w[1 + 2 * jp], qb = w[2 + 2 * jp];
         const uint32_t w8[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-        uint32_t nib[8];
+        uint32_t nib[2][8];
 #pragma unroll
-        for (int w = 0; w < 8; ++w) { nib[w] = (j & 1) ? (w8[w] >> 4) & 0x0f0f0f0fu : w8[w] & 0x0f0f0f0fu; }
-        float sc, mn; kq_scale_min(sw, j, sc, mn);
-        const float dsc = __fmul_rn(dm.x, sc), dmn = __fmul_rn(dm.y, mn);
+        for (int i = 0; i < 8; ++i) { nib[0][i] = w8[i] & 0x0f0f0f0fu; nib[1][i] = (w8[i] >> 4) & 0x0f0f0f0fu; }
+        const uint32_t sw = scw[jp >> 1], mw = mnw[jp >> 1];
+        const float s0 = (jp & 1) ? kq_byte_magic<2>(sw) : kq_byte_magic<0>(sw), s1 = (jp & 1) ? kq_byte_magic<3>(sw) : kq_byte_magic<1>(sw);
+        const float m0 = (jp & 1) ? kq_byte_magic<2>(mw) : kq_byte_magic<0>(mw), m1 = (jp & 1) ? kq_byte_magic<3>(mw) : kq_byte_magic<1>(mw);
+        const float dsc[2] = {fmaf(dm.x, s0, dbase), fmaf(dm.x, s1, dbase)}, dmn[2] = {fmaf(-dm.y, m0, mbase), fmaf(-dm.y, m1, mbase)};   // (dmn: negated)
 #pragma unroll
         for (int t = 0; t < TM; ++t) {
-            if (TM == 1 || t < nT) {
-                const uint32_t *ysb = a.y + t * a.col + sb * KQ_SB_WORDS;
-                const uint4 ya = *reinterpret_cast<const uint4 *>(ysb + j * 8), yb = *reinterpret_cast<const uint4 *>(ysb + j * 8 + 4);
-                const uint32_t y8[8] = {ya.x, ya.y, ya.z, ya.w, yb.x, yb.y, yb.z, yb.w};
-                int isum = 0;
+            {
+                const uint32_t r = rec_s + t * col_bytes;
+                const float4 ys = lds128f(r + 288u + 16u * jp);   // sums of the four halves
+                float dx[2];
+                asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(dx[0]), "=f"(dx[1]) : "r"(r + 256u + 8u * jp));
 #pragma unroll
-                for (int w = 0; w < 8; ++w) { isum = __dp4a((int)nib[w], (int)y8[w], isum); }
-                const float dxj = a.dx[t * a.col + 8 * sb + j];
-                acc[t] = fmaf(__fmul_rn(dsc, dxj), (float)isum, acc[t]);
-                acc[t] = fmaf(-__fmul_rn(dmn, dxj), (float)a.ysum[t * a.col + 8 * sb + j], acc[t]);
+                for (int o = 0; o < 2; ++o) {
+                    const uint4 ya = lds128(r + 64u * jp + 32u * o), yb = lds128(r + 64u * jp + 32u * o + 16u);
+                    const uint32_t y8[8] = {ya.x, ya.y, ya.z, ya.w, yb.x, yb.y, yb.z, yb.w};
+                    int isum = (int)MAGIC_I;   // (the sum as the bits of the float MAGIC_F + sum)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { isum = __dp4a((int)nib[o][i], (int)y8[i], isum); }
+                    acc[t] = fmaf(__fmul_rn(dsc[o], dx[o]), __int_as_float(isum) - MAGIC_F, acc[t]);
+                    acc[t] = fmaf(__fmul_rn(dmn[o], dx[o]), o ? __fadd_rn(ys.z, ys.w) : __fadd_rn(ys.x, ys.y), acc[t]);   // (small integers: the sum is exact)
+                }
             }
         }
     }
 }
 
-// values of one Q6_K super-block in the upload layout: wb = 208 bytes (ql 128, qh 64, 16 int8 scales), d = its fp16 scale
-template <int TM>
-__device__ __forceinline__ void kq_values_q6k(const uint8_t *wb, uint16_t d_half, const KqPlanes &a, int sb, int nT, float (&acc)[TM]) {
-    uint4 ql[8], qh[4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { ql[i] = ldg_nc(wb + 16 * i); }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { qh[i] = ldg_nc(wb + 128 + 16 * i); }
-    const uint4 scw = ldg_nc(wb + 192);
+// values of one Q6_K super-block in the upload layout: w = its 208 bytes (ql 128, qh 64, 16 int8 scales), d_half = its fp16 scale
+template <int TM, int NW>
+__device__ __forceinline__ void kq_values_q6k(const uint4 (&wv)[NW], uint16_t d_half, uint32_t rec_s, uint32_t col_bytes, float (&acc)[TM]) {
     const float d = h2f(d_half);
-    const uint32_t scs[4] = {scw.x, scw.y, scw.z, scw.w};
+    const uint32_t scs[4] = {wv[12].x, wv[12].y, wv[12].z, wv[12].w};
 #pragma unroll
     for (int t = 0; t < TM; ++t) { acc[t] = 0.f; }
 #pragma unroll
-    for (int g = 0; g < 16; ++g) {
-        // group g = values 16g .. 16g+15: half h of the super-block, segment s of 32 values, l = 16 * (g & 1) .. + 15
-        //   s 0: ql[64h + l] low | qh[32h + l] bits 0-1     s 1: ql[64h + 32 + l] low  | bits 2-3
-        //   s 2: ql[64h + l] high | bits 4-5                s 3: ql[64h + 32 + l] high | bits 6-7
-        const int h = g >> 3, sg = (g >> 1) & 3, l0 = 16 * (g & 1);
-        const uint4 lv = ql[(64 * h + 32 * (sg & 1) + l0) >> 4], hv = qh[(32 * h + l0) >> 4];
-        const uint32_t lw[4] = {lv.x, lv.y, lv.z, lv.w}, hw[4] = {hv.x, hv.y, hv.z, hv.w};
-        uint32_t v6[4];                                          // the group's values 0..63, four per word
+    for (int gq = 0; gq < 4; ++gq) {
+        uint32_t v6[4][4];                      // the values 0..63 of groups 4 gq .. + 3, four per word
+        float    dsc[4];
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const uint32_t lo = (sg & 2) ? (lw[w] >> 4) & 0x0f0f0f0fu : lw[w] & 0x0f0f0f0fu;
-            v6[w] = lo | (((hw[w] >> (2 * sg)) & 0x03030303u) << 4);
+        for (int gi = 0; gi < 4; ++gi) {
+            // group g = values 16g .. 16g+15: half h of the super-block, segment s of 32 values, l = 16 * (g & 1) .. + 15
+            //   s 0: ql[64h + l] low | qh[32h + l] bits 0-1     s 1: ql[64h + 32 + l] low  | bits 2-3
+            //   s 2: ql[64h + l] high | bits 4-5                s 3: ql[64h + 32 + l] high | bits 6-7
+            const int g = 4 * gq + gi, h = g >> 3, sg = (g >> 1) & 3, l0 = 16 * (g & 1);
+            const uint4 lv = wv[(64 * h + 32 * (sg & 1) + l0) >> 4], hv = wv[8 + ((32 * h + l0) >> 4)];
+            const uint32_t lw[4] = {lv.x, lv.y, lv.z, lv.w}, hw[4] = {hv.x, hv.y, hv.z, hv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t lo = (sg & 2) ? (lw[i] >> 4) & 0x0f0f0f0fu : lw[i] & 0x0f0f0f0fu;
+                const uint32_t hi = sg == 0 ? hw[i] << 4 : sg == 1 ? hw[i] << 2 : sg == 2 ? hw[i] : hw[i] >> 2;
+                v6[gi][i] = lo | (hi & 0x30303030u);
+            }
+            const uint32_t su = scs[gq] ^ 0x80808080u;   // scale + 128
+            const float sm = gi == 0 ? kq_byte_magic<0>(su) : gi == 1 ? kq_byte_magic<1>(su) : gi == 2 ? kq_byte_magic<2>(su) : kq_byte_magic<3>(su);
+            dsc[gi] = __fmul_rn(d, sm - 8388736.f);
         }
-        const int sc = (int)(int8_t)((scs[g >> 2] >> (8 * (g & 3))) & 0xffu);
-        const float dsc = __fmul_rn(d, (float)sc);
 #pragma unroll
         for (int t = 0; t < TM; ++t) {
-            if (TM == 1 || t < nT) {
-                const uint4 yv = *reinterpret_cast<const uint4 *>(a.y + t * a.col + sb * KQ_SB_WORDS + (g >> 1) * 8 + 4 * (g & 1));
-                const uint32_t y4[4] = {yv.x, yv.y, yv.z, yv.w};
-                int isum = 0, ys = 0;
+            {
+                const uint32_t r = rec_s + t * col_bytes;
+                const float4 ys4 = lds128f(r + 288u + 16u * gq);   // sums of the groups' activations
+                float dx[2];
+                asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(dx[0]), "=f"(dx[1]) : "r"(r + 256u + 8u * gq));
+                const float ys[4] = {ys4.x, ys4.y, ys4.z, ys4.w};
 #pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    isum = __dp4a((int)v6[w], (int)y4[w], isum);
-                    ys   = __dp4a(0x01010101, (int)y4[w], ys);
+                for (int gi = 0; gi < 4; ++gi) {
+                    const uint4 y = lds128(r + 16u * (4 * gq + gi));
+                    int isum = __dp4a((int)v6[gi][0], (int)y.x, (int)MAGIC_I);
+                    isum = __dp4a((int)v6[gi][1], (int)y.y, isum); isum = __dp4a((int)v6[gi][2], (int)y.z, isum); isum = __dp4a((int)v6[gi][3], (int)y.w, isum);
+                    const float sum = fmaf(-32.f, ys[gi], __int_as_float(isum)) - MAGIC_F;   // value = stored - 32 (integers below 2^24 throughout: exact)
+                    acc[t] = fmaf(__fmul_rn(dsc[gi], dx[gi >> 1]), sum, acc[t]);
                 }
-                isum -= 32 * ys;                                 // value = stored - 32
-                acc[t] = fmaf(__fmul_rn(dsc, a.dx[t * a.col + 8 * sb + (g >> 1)]), (float)isum, acc[t]);
             }
         }
     }
 }
 
-struct KqRow { const uint8_t *w; int type; };
-__device__ __forceinline__ KqRow kq_row(const MatvecParams &p, int64_t row, int pair_second) {
+struct KqRow { const uint8_t *w; int64_t pitch; int type; };
+// where row `row` of the virtual matrix lies (static indexes: the segments stay in the parameter bank)
+__device__ __forceinline__ KqRow kq_row(const MatvecParams &p, int64_t row) {
+    const int64_t n0 = p.kq[0].n_rows, n1 = p.kq[1].n_rows;
+    const bool b1 = p.kq_n > 1 && row >= n0, b2 = p.kq_n > 2 && row >= n0 + n1;
     KqRow r;
-    if (p.pair_mode) { const KqSeg &s = p.kq[pair_second]; r.w = s.w + row * s.row_bytes; r.type = s.type; return r; }
-    int i = 0;
-    while (i + 1 < p.kq_n && row >= p.kq[i].n_rows) { row -= p.kq[i].n_rows; ++i; }
-    r.w = p.kq[i].w + row * p.kq[i].row_bytes; r.type = p.kq[i].type;
+    r.pitch = b2 ? p.kq[2].row_bytes : b1 ? p.kq[1].row_bytes : p.kq[0].row_bytes;
+    r.type  = b2 ? p.kq[2].type : b1 ? p.kq[1].type : p.kq[0].type;
+    r.w     = (b2 ? p.kq[2].w : b1 ? p.kq[1].w : p.kq[0].w) + (row - (b2 ? n0 + n1 : b1 ? n0 : 0)) * r.pitch;
+    return r;
+}
+// first row of the unit that begins at pair `pair0` (side 1: of the second matrix in pair mode). Row r of a unit is row r of the first, or,
+// in pair mode, row r / 2 of side r % 2.
+__device__ __forceinline__ KqRow kq_unit(const MatvecParams &p, int64_t pair0, int side) {
+    if (!p.pair_mode) { return kq_row(p, 2 * pair0); }
+    KqRow r;
+    r.pitch = side ? p.kq[1].row_bytes : p.kq[0].row_bytes; r.type = side ? p.kq[1].type : p.kq[0].type;
+    r.w = (side ? p.kq[1].w : p.kq[0].w) + pair0 * r.pitch;
     return r;
 }
 
-// dot products of one row with the nT <= TM activation columns of the pass, for the lanes [lane0, lane0 + G) of the warp;
-// every lane of the group ends with the same values
-template <int G, int TM>
-__device__ __forceinline__ void kq_row_dot(const KqRow &r, int nsb, const KqPlanes &a, int nT, int l /* lane inside the group */, int lane0, float (&total)[TM]) {
-    constexpr int ROUNDS = 4;      // super-blocks per lane (K <= 256 * G * ROUNDS)
-    float part[ROUNDS][TM];
-#pragma unroll
-    for (int k = 0; k < ROUNDS; ++k) {
-        const int sb = l + k * G;
-#pragma unroll
-        for (int t = 0; t < TM; ++t) { part[k][t] = 0.f; }
-        if (k * G < nsb && sb < nsb) {
-            if (r.type == 12) { kq_values_q4k<TM>(r.w + (size_t)sb * 144, a, sb, nT, part[k]); }
-            else {
-                const uint16_t dh = *reinterpret_cast<const uint16_t *>(r.w + (size_t)nsb * 208 + 2 * sb);
-                kq_values_q6k<TM>(r.w + (size_t)sb * 208, dh, a, sb, nT, part[k]);
-            }
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < TM; ++t) {
-        float sum = 0.f;             // the super-blocks' values in order
-        if (TM == 1 || t < nT) {
-#pragma unroll
-            for (int k = 0; k < ROUNDS; ++k) {
-                if (k * G >= nsb) { break; }
-                for (int i = 0; i < G; ++i) {
-                    const float v = __shfl_sync(0xffffffffu, part[k][t], lane0 + i);
-                    if (i + k * G < nsb) { sum = __fadd_rn(sum, v); }
-                }
-            }
-        }
-        total[t] = sum;
-    }
+struct KqPlan { int np, wact, ns, stage_bytes; };   // pairs per unit, streaming warps per CTA, ring stages per warp, bytes per stage
+struct KqSmem { size_t part, bars, ring, total; };
+__host__ __device__ static inline KqSmem kq_smem_layout(int nsb, int TM, const KqPlan &q) {
+    KqSmem m;
+    m.part = (size_t)TM * nsb * KQ_REC * 4;
+    m.bars = (m.part + (size_t)q.wact * TM * 2 * q.np * nsb * 4 + 15) / 16 * 16;
+    m.ring = (m.bars + (size_t)q.wact * q.ns * 8 + 127) / 128 * 128;
+    m.total = m.ring + (size_t)q.wact * q.ns * q.stage_bytes;
+    return m;
 }
 
-template <int TM>
-__global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecParams p) {
+// TM: columns of the pass, rounded up to 1, 2 or 4 (columns past p.T compute on whatever their records hold and are not stored); TYPE: 12 or
+// 14 when every row is of that type, else 0
+template <int TM, int TYPE>
+__global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecParams p, const KqPlan pl) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    __shared__ float scale_s;
-    const int nb = p.A.nb, nsb = nb >> 3;
-    const int nT = (TM == 1) ? 1 : p.T;
-    KqPlanes a;
-    a.col  = nsb * KQ_SB_WORDS + 2 * nb;
-    a.y    = reinterpret_cast<uint32_t *>(smem_raw);
-    a.dx   = reinterpret_cast<float *>(a.y + (size_t)nsb * KQ_SB_WORDS);
-    a.ysum = reinterpret_cast<int *>(a.dx + nb);
+    __shared__ float scale_s[TM];
+    const int nsb = p.A.nb >> 3, nT = (TM == 1) ? 1 : p.T;
+    const int col = nsb * KQ_REC;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const KqSmem L = kq_smem_layout(nsb, TM, pl);
+    const int n_row = 2 * pl.np, items = n_row * nsb, n_round = (items + 31) >> 5;   // per unit
+    const int64_t n_units  = (p.pair_mode ? p.kq[0].n_rows : (p.A.n_rows >> 1)) / pl.np;
+    const int64_t unit_lo  = n_units * blockIdx.x / gridDim.x, unit_hi = n_units * (blockIdx.x + 1) / gridDim.x;
+    const int64_t my_first = unit_lo + warp;
+    const int     my_units = (warp < pl.wact && my_first < unit_hi) ? (int)((unit_hi - my_first + pl.wact - 1) / pl.wact) : 0;
+    const int     n_stage  = my_units * n_round;
+    const uint32_t ring_s = smem_u32(smem_raw + L.ring) + (uint32_t)warp * pl.ns * pl.stage_bytes;
+    const uint32_t bar_s  = smem_u32(smem_raw + L.bars) + (uint32_t)warp * pl.ns * 8;
+    float *part = reinterpret_cast<float *>(smem_raw + L.part) + (size_t)warp * TM * items;
+    const bool mixed = TYPE == 0 && p.pair_mode && p.kq[0].type != p.kq[1].type;   // (items of a stage then lie at the larger pitch)
+
+    // lane 0: the next 32 super-blocks of the unit at lunit (from super-block lsb of its row lr on) into slot lslot
+    int64_t lunit = my_first; int lr = 0, lsb = 0, lslot = 0, issued = 0;
+    KqRow l0 = {}, l1 = {};
+    auto load_unit = [&]() { l0 = kq_unit(p, lunit * pl.np, 0); if (p.pair_mode) { l1 = kq_unit(p, lunit * pl.np, 1); } };
+    auto issue_next = [&]() {
+        const uint32_t bar = bar_s + lslot * 8;
+        uint32_t dst = ring_s + (uint32_t)(lslot * pl.stage_bytes);
+        int left = min(32, items - (lr * nsb + lsb));
+        if (!p.pair_mode && (TYPE != 0 ? TYPE : l0.type) == 12) {   // the unit's rows are one contiguous run
+            const uint32_t bytes = (uint32_t)left * 144u;
+            mbar_expect_tx(bar, bytes);
+            bulk_copy_g2s(dst, l0.w + (size_t)(lr * nsb + lsb) * 144, bytes, bar);
+            lsb += left;
+            while (lsb >= nsb) { lsb -= nsb; ++lr; }
+        } else {
+            uint32_t bytes = (uint32_t)left * ((TYPE != 0 ? TYPE : l0.type) == 12 ? 144u : 208u);
+            if (mixed) {
+                bytes = 0;
+                for (int q = left, r = lr, o = lsb; q > 0; ++r, o = 0) { const int m = min(q, nsb - o); bytes += (uint32_t)m * (((r & 1) ? l1.type : l0.type) == 12 ? 144u : 208u); q -= m; }
+            }
+            mbar_expect_tx(bar, bytes);
+            while (left > 0) {
+                const int m = min(left, nsb - lsb);
+                const bool second = p.pair_mode && (lr & 1);
+                const uint32_t body = (TYPE != 0 ? TYPE : second ? l1.type : l0.type) == 12 ? 144u : 208u;
+                const uint8_t *src = (second ? l1.w : l0.w) + (int64_t)(p.pair_mode ? lr >> 1 : lr) * (second ? l1.pitch : l0.pitch) + (uint32_t)lsb * body;
+                bulk_copy_g2s(dst, src, (uint32_t)m * body, bar);
+                dst += (uint32_t)m * (mixed ? 208u : body);
+                left -= m; lsb += m;
+                if (lsb == nsb) { lsb = 0; ++lr; }
+            }
+        }
+        ++issued;
+        if (++lslot == pl.ns) { lslot = 0; }
+        if (lr == n_row) { lr = 0; lunit += pl.wact; if (issued < n_stage) { load_unit(); } }
+    };
+
+    // weights never change during a step: the copies may run ahead of the previous kernel's results
     pdl_launch_dependents();
+    if (lane == 0 && n_stage > 0) {
+        for (int s = 0; s < pl.ns; ++s) { mbar_init(bar_s + s * 8, 1); }
+        mbar_init_fence();
+        load_unit();
+        for (int s = 0; s < pl.ns && issued < n_stage; ++s) { issue_next(); }
+    }
+    __syncwarp();
     pdl_wait();
     tp_wait(p.tp, p.error_flag);
-#pragma unroll 1
-    for (int t = 0; t < nT; ++t) {
-        KqPlanes c = a;
-        c.y += t * a.col; c.dx += t * a.col; c.ysum += t * a.col;
-        float *v3 = reinterpret_cast<float *>(c.y);   // nb * 8 floats = the size of the y plane (nb * 32 bytes): aliases it
-        const float *x = p.x + (int64_t)t * p.x_stride;
-        if (p.pro == PRO_NORM_QUANT) { kq_prologue<true>(p, x, c, v3, &scale_s); } else { kq_prologue<false>(p, x, c, v3, &scale_s); }
-        __syncthreads();
-    }
+    uint32_t *rec = reinterpret_cast<uint32_t *>(smem_raw);
+    if (p.pro == PRO_NORM_QUANT) { kq_prologue<true>(p, nT, rec, col, scale_s); } else { kq_prologue<false>(p, nT, rec, col, scale_s); }
+    __syncthreads();
 
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t n_units = p.pair_mode ? p.kq[0].n_rows : (p.A.n_rows >> 1);
-    for (int64_t u = (int64_t)blockIdx.x * KQ_WARPS + warp; u < n_units; u += (int64_t)gridDim.x * KQ_WARPS) {
-        const int64_t row_a = p.pair_mode ? u : 2 * u, row_b = p.pair_mode ? u : 2 * u + 1;
-        float va[TM], vb[TM];
-        if (nsb <= 16) {            // both rows at once, a half-warp each
-            const int half = lane >> 4;
-            const KqRow r = kq_row(p, half ? row_b : row_a, half);
-            float v[TM];
-            kq_row_dot<16, TM>(r, nsb, a, nT, lane & 15, lane & 16, v);
-#pragma unroll
-            for (int t = 0; t < TM; ++t) { va[t] = __shfl_sync(0xffffffffu, v[t], 0); vb[t] = __shfl_sync(0xffffffffu, v[t], 16); }
-        } else {
-            kq_row_dot<32, TM>(kq_row(p, row_a, 0), nsb, a, nT, lane, 0, va);
-            kq_row_dot<32, TM>(kq_row(p, row_b, 1), nsb, a, nT, lane, 0, vb);
+    const uint32_t rec_s = smem_u32(rec), col_bytes = (uint32_t)col * 4u;
+    int64_t unit = my_first;
+    int round = 0, slot = 0, n = 0;
+    uint32_t parity = 0;
+    bool ok = true;
+    // this lane's super-block in the round: sb of row r of the unit, `first` = the first super-block of that row in the round
+    int r = lane / nsb, sb = lane - r * nsb;
+    const int r_0 = r, sb_0 = sb;
+    // the rows' results are finished one unit later: the residual or the SiLU table entry they meet is on its way meanwhile
+    float pend_a = 0.f, pend_b = 0.f;
+    float *pend = nullptr;
+    auto finish_pending = [&]() { if (pend != nullptr) { *pend = p.epi == EPI_SILU_MUL ? __fmul_rn(pend_a, pend_b) : __fadd_rn(pend_a, pend_b); pend = nullptr; } };
+    for (; n < n_stage; ++n) {
+        const int  i = 32 * round + lane;
+        const bool have = i < items;
+        int        type = TYPE;
+        uint16_t   dh = 0;
+        if (TYPE != 12) {
+            const KqRow u = kq_unit(p, unit * pl.np, r & 1);
+            type = u.type;
+            if (have && type != 12) { dh = __ldg(reinterpret_cast<const uint16_t *>(u.w + (int64_t)(p.pair_mode ? r >> 1 : r) * u.pitch + (size_t)nsb * 208) + sb); }   // (arrives while the copy is waited for)
         }
+        const uint32_t body = type == 12 ? 144u : 208u;
+        const int before = min(lane, sb);        // super-blocks of the same row in front of this one in the round
+        ok = mbar_wait_bounded(bar_s + slot * 8, parity, WAIT_LIMIT_NS);
+        if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+        uint4 w[TYPE == 12 ? 9 : 13];
+        const uint32_t src = ring_s + (uint32_t)(slot * pl.stage_bytes) + (uint32_t)(lane - before) * (mixed ? 208u : body) + (uint32_t)before * body;
+        if (have) {
 #pragma unroll
-        for (int t = 0; t < TM; ++t) {
-            const bool store = lane == 0 && t < nT;
-            if (p.epi == EPI_SILU_MUL) { matvec_epilogue_silu(p, u, t, va[t], vb[t], store); }
-            else {
-                matvec_epilogue(p, row_a, t, va[t], vb[t], store);
-                matvec_epilogue(p, row_b, t, vb[t], va[t], store);
+            for (int k = 0; k < 9; ++k) { w[k] = lds128(src + 16u * k); }
+            if (TYPE != 12 && type != 12) {
+#pragma unroll
+                for (int k = 9; k < 13; ++k) { w[k] = lds128(src + 16u * k); }
             }
+        }
+        __syncwarp();   // every lane has its super-block in registers: the stage can be refilled
+        if (lane == 0 && issued < n_stage) { issue_next(); }
+        if (++slot == pl.ns) { slot = 0; parity ^= 1u; }
+        if (have) {
+            float v[TM];
+            if constexpr (TYPE == 12) { kq_values_q4k<TM>(w, rec_s + (uint32_t)(sb * KQ_REC * 4), col_bytes, v); }
+            else if constexpr (TYPE == 14) { kq_values_q6k<TM>(w, dh, rec_s + (uint32_t)(sb * KQ_REC * 4), col_bytes, v); }
+            else if (type == 12) { kq_values_q4k<TM>(w, rec_s + (uint32_t)(sb * KQ_REC * 4), col_bytes, v); }
+            else                 { kq_values_q6k<TM>(w, dh, rec_s + (uint32_t)(sb * KQ_REC * 4), col_bytes, v); }
+#pragma unroll
+            for (int t = 0; t < TM; ++t) { part[t * items + i] = v[t]; }
+        }
+        sb += 32;
+        while (sb >= nsb) { sb -= nsb; ++r; }
+        if (++round == n_round) {   // the unit is complete: lane = (column, row) adds a row's values in order
+            __syncwarp();
+            const int ur = lane % n_row, t = lane / n_row;
+            float sum = 0.f;
+            if (t < nT) {
+                const float *q = part + t * items + ur * nsb;
+                int k = 0;
+#pragma unroll 1
+                for (; k + 8 <= nsb; k += 8) {
+                    float f[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) { f[e] = q[k + e]; }
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) { sum = __fadd_rn(sum, f[e]); }
+                }
+                for (; k < nsb; ++k) { sum = __fadd_rn(sum, q[k]); }
+            }
+            const float partner = __shfl_xor_sync(0xffffffffu, sum, 1);
+            finish_pending();
+            if (p.epi == EPI_SILU_MUL) {
+                if (t < nT && (ur & 1) == 0) { pend = p.out + (int64_t)t * p.out_stride + unit * pl.np + (ur >> 1); pend_a = sum; pend_b = p.silu_table[f2h(partner)]; }
+            } else if (p.epi == EPI_RESID) {
+                if (t < nT) { const int64_t o = (int64_t)t * p.out_stride + 2 * unit * pl.np + ur; pend = p.out + o; pend_a = sum; pend_b = p.resid[o]; }
+            } else { matvec_epilogue(p, 2 * unit * pl.np + ur, t, sum, partner, t < nT); }
+            __syncwarp();   // (the values are overwritten by the next unit)
+            r = r_0; sb = sb_0;
+            round = 0; unit += pl.wact;
+        }
+    }
+    finish_pending();
+    if (!ok) {
+        // a copy did not arrive: report, give the copies still in flight a last bounded chance to land and stop; the host sees the
+        // flag at its next synchronisation
+        if (lane == 0 && p.error_flag != nullptr) { atomicExch(p.error_flag, 1); }
+        for (int k = n; k < __shfl_sync(0xffffffffu, issued, 0); ++k) {
+            mbar_wait_bounded(bar_s + slot * 8, parity, 10000000ull);
+            if (++slot == pl.ns) { slot = 0; parity ^= 1u; }
         }
     }
     tp_publish(p.tp, p.T);
@@ -282,26 +390,54 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
 cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg) {
     if (p.T < 1 || p.T > KQ_MAX_COLUMNS || p.kq_n < 1 || p.kq_n > 3 || p.A.k % 256 != 0 || p.A.k > 256 * 32 * 4 || p.A.nb != (int)(p.A.k / QK)) { return cudaErrorInvalidValue; }
     if (p.pair_mode ? (p.kq_n != 2 || p.kq[0].n_rows != p.kq[1].n_rows || p.epi != EPI_SILU_MUL) : (p.epi == EPI_SILU_MUL || (p.A.n_rows & 1))) { return cudaErrorInvalidValue; }
+    bool q6 = false, q4 = false;
     for (int i = 0; i < p.kq_n; ++i) {
         if ((p.kq[i].type != 12 && p.kq[i].type != 14) || p.kq[i].w == nullptr || (p.kq[i].n_rows & 1) || (reinterpret_cast<uintptr_t>(p.kq[i].w) & 15) || (p.kq[i].row_bytes & 15)) { return cudaErrorInvalidValue; }
+        q6 = q6 || p.kq[i].type == 14; q4 = q4 || p.kq[i].type == 12;
     }
     const int nsb = (int)(p.A.k / 256);
-    const int    TM   = p.T == 1 ? 1 : KQ_MAX_COLUMNS;
-    const size_t smem = (size_t)TM * ((size_t)nsb * KQ_SB_WORDS * 4 + (size_t)p.A.nb * 8) + 16;
-    void (*kernel)(const MatvecParams) = p.T == 1 ? matvec_kq_kernel<1> : matvec_kq_kernel<KQ_MAX_COLUMNS>;
+    const int TM  = p.T <= 2 ? p.T : KQ_MAX_COLUMNS;
+    const int64_t pairs = p.pair_mode ? p.kq[0].n_rows : (p.A.n_rows >> 1);
+    const int64_t grid  = std::max<int64_t>(1, std::min<int64_t>(cfg.num_sms, pairs));
+    // Pairs per unit: a round costs the same however few of its 32 lanes have a super-block, so short rows share a unit; but a CTA's warps
+    // take whole units, so the choice is the one whose busiest warp has the fewest rounds (plus the ordered sum, about 0.7 of a round).
+    // Units do not straddle the segments of a virtual matrix.
+    KqPlan pl = {1, KQ_WARPS, 1, 32 * (q6 ? 208 : 144)};
+    double best = 0.0;
+    for (int np = 1; np <= 4; np *= 2) {
+        bool whole = pairs % np == 0;
+        for (int i = 0; i < p.kq_n && !p.pair_mode; ++i) { whole = whole && p.kq[i].n_rows % (2 * np) == 0; }
+        if (!whole) { break; }
+        const int64_t units_cta = (pairs / np + grid - 1) / grid;
+        const double cost = (double)((units_cta + KQ_WARPS - 1) / KQ_WARPS) * ((2 * np * nsb + 31) / 32 + 0.7);
+        if (np == 1 || cost < best) { best = cost; pl.np = np; }
+    }
+    // Warps that stream: all sixteen when two stages each fit the shared memory, fewer otherwise (Q6_K with four columns), down to one
+    const size_t budget = 224 * 1024;
+    for (pl.wact = KQ_WARPS; pl.wact > 1; --pl.wact) {
+        pl.ns = 2;
+        if (kq_smem_layout(nsb, TM, pl).total <= budget) { break; }
+    }
+    if (pl.wact == 1) { pl.ns = 1; }
+    while (pl.ns < KQ_MAX_STAGES) { ++pl.ns; if (kq_smem_layout(nsb, TM, pl).total > budget) { --pl.ns; break; } }
+    const size_t smem = kq_smem_layout(nsb, TM, pl).total;
+    if (smem > budget) { return cudaErrorInvalidValue; }
+    using Kernel = void (*)(const MatvecParams, const KqPlan);
+    static const Kernel kernels[3][3] = {{matvec_kq_kernel<1, 12>, matvec_kq_kernel<1, 14>, matvec_kq_kernel<1, 0>},
+                                         {matvec_kq_kernel<2, 12>, matvec_kq_kernel<2, 14>, matvec_kq_kernel<2, 0>},
+                                         {matvec_kq_kernel<KQ_MAX_COLUMNS, 12>, matvec_kq_kernel<KQ_MAX_COLUMNS, 14>, matvec_kq_kernel<KQ_MAX_COLUMNS, 0>}};
+    const Kernel kernel = kernels[TM == 1 ? 0 : TM == 2 ? 1 : 2][q4 && q6 ? 2 : q6 ? 1 : 0];
     cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem);
     if (err != cudaSuccess) { return err; }
     MatvecParams q = p;
     if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
-    const int64_t n_units = p.pair_mode ? p.kq[0].n_rows : (p.A.n_rows >> 1);
-    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(cfg.num_sms, (n_units + KQ_WARPS - 1) / KQ_WARPS));
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)grid); lc.blockDim = dim3(KQ_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr; lc.numAttrs = cfg.pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&lc, kernel, q);
+    return cudaLaunchKernelEx(&lc, kernel, q, pl);
 }
 
 // upload-time re-layout of Q6_K rows: [sb][ql 128 | qh 64 | scales 16 | d 2] (210 bytes each) ->

@@ -283,6 +283,25 @@ def test_matmul_on_uploaded_constants_takes_the_model_kernels(be, oracle, qt, n,
         assert np.array_equal(bits(got), bits(want))
 
 
+@pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
+@pytest.mark.parametrize("n,k,t", [(4800, 256, 1), (4796, 1280, 3), (2, 256, 4), (300, 8448, 2), (292, 11008, 4), (9000, 768, 1)])
+def test_k_quant_mat_vec_units_and_rounds(be, oracle, qt, n, k, t):
+    """The K-quant mat-vec kernel on units of one, two and four row pairs, rows of 1 to 43 super-blocks (rounds of 32 that end inside a row
+    and inside a unit), more units than warps and fewer, 1 to 4 columns; bit-identical to the restatement."""
+    rng = np.random.default_rng(n + k + t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    pw, px, po = be.upload_constant(f"kq_units_{qt}_{n}_{k}_{t}", w, qt, (k, n)), be.upload(x), be.alloc_memory(4 * n * t)
+    d = B.OpDesc()
+    d.op_type, d.num_input = B.OP["MatMul"], 2
+    d.input[0] = B.make_tensor(pw, qt, (k, n), None, B.NODE_CONSTANT)
+    d.input[1] = B.make_tensor(px, B.FP32, (k, t))
+    d.output = B.make_tensor(po, B.FP32, (n, t))
+    be.submit(d); be.sync()
+    got = be.download(po, (t, n), np.float32)
+    assert np.array_equal(bits(got), bits(oracle.matmul(qt, w, k, n, x)))
+
+
 def test_matmul_linearity_full_size(be):
     """Size-independent property at the 7B head shape: W(2x) == 2 W(x) exactly (power-of-two scaling commutes with Q8_0)."""
     rng = np.random.default_rng(5)
