@@ -166,6 +166,7 @@ class B200Backend:
     def __init__(self, device_id: int = 0, tp_size: int = 1, tp_rank: int = 0, use_pdl: bool = True,
                  use_graph: bool = True, arena_bytes: int = 0):
         self._l = lib()
+        self._submit = self._l.spyb_submit
         cfg = Config(device_id, tp_size, tp_rank, int(use_pdl), int(use_graph), 0, arena_bytes)
         h = C.c_void_p()
         st = self._l.spyb_create(C.byref(cfg), C.byref(h))
@@ -237,7 +238,9 @@ class B200Backend:
         if callback is not None:
             cb = CALLBACK(lambda _user: callback())
             self._callbacks.append(cb)   # keep alive until it has fired
-        self._check(self._l.spyb_submit(self.h, C.byref(desc), cb, None))
+        st = self._submit(self.h, C.byref(desc), cb, None)
+        if st != SUCCESS:
+            self._check(st)
 
     def submit_timed(self, descs, repeats: int) -> float:
         """Device time in ms of `repeats` submits that walk round-robin over the descriptors (measurement aid)."""

@@ -695,11 +695,67 @@ spyb_status run_matmul(spyb_backend *be, spyb_op_desc *d, void *out_dev) {
     return SPYB_SUCCESS;
 }
 
+// Rows of the (cos, sin) table for the given positions, with the host libm and the CPU operator's repeated f32 multiplication of theta
+// (backend/host/operator/non-linear.cpp:282, 300-309). nullptr when the positions do not fit a table (the caller then builds its own).
+const float2 *rope_rows(spyb_backend *be, const spyb_rope_param &rp, const int32_t *pos, int64_t n_tok, int64_t npair) {
+    constexpr size_t MAX_TABLES = 8, MAX_ROWS = 16384;
+    std::lock_guard<std::mutex> g(be->rope_mutex);
+    RopeTable *t = nullptr;
+    for (RopeTable &c : be->rope_tables) { if (c.freq_base == rp.freq_base && c.num_dim == rp.num_dim && c.npair == npair) { t = &c; break; } }
+    if (t == nullptr) {
+        if (be->rope_tables.size() >= MAX_TABLES || rp.num_context < 1) { return nullptr; }
+        RopeTable c;
+        c.freq_base = rp.freq_base; c.num_dim = rp.num_dim; c.npair = npair;
+        c.have.assign(std::min<size_t>(MAX_ROWS, (size_t)rp.num_context), 0);
+        c.dev = static_cast<float2 *>(be->arena.alloc(c.have.size() * npair * sizeof(float2)));
+        if (c.dev == nullptr) { return nullptr; }
+        be->rope_tables.push_back(std::move(c));
+        t = &be->rope_tables.back();
+    }
+    for (int64_t i = 0; i < n_tok; ++i) { if (pos[i] < 0 || (size_t)pos[i] >= t->have.size()) { return nullptr; } }
+    std::vector<float2> row;
+    const float theta_scale = std::pow(rp.freq_base, -2.0f / (float)rp.num_dim);
+    for (int64_t i = 0; i < n_tok; ++i) {
+        if (t->have[pos[i]]) { continue; }
+        row.resize((size_t)npair);
+        float theta = (float)pos[i];
+        for (int64_t k = 0; k < npair; ++k) { row[(size_t)k] = make_float2(std::cos(theta) * 1.0f, std::sin(theta) * 1.0f); theta *= theta_scale; }
+        if (cudaMemcpyAsync(t->dev + (int64_t)pos[i] * npair, row.data(), row.size() * sizeof(float2), cudaMemcpyHostToDevice, be->stream) != cudaSuccess) { return nullptr; }
+        t->have[pos[i]] = 1;
+    }
+    return t->dev;
+}
+
+// A host mask of +0 and -inf as bits (set = visible); false when it holds anything else or does not fit
+bool pack_mask(const spyb_tensor &scores, const spyb_tensor &mask, MaskBits *out) {
+    const int64_t ne0 = scores.elements[0], ne1 = scores.elements[1];
+    if (mask.node_type != SPYB_NODE_IO || mask.bytes[0] != 4 || mask.elements[0] < ne0 || mask.elements[1] < ne1 || ne0 < 1 || ne1 < 1 || ne0 * ne1 > MASK_BITS) { return false; }
+    const int64_t words = (ne0 * ne1 + 31) / 32;
+    std::memset(out->w, 0, (size_t)words * 4);
+    uint32_t other = 0;
+    for (int64_t r = 0; r < ne1; ++r) {
+        const uint32_t *m = reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(mask.data) + r * mask.bytes[1]);
+        for (int64_t i0 = 0; i0 < ne0;) {   // up to 32 values of one word at a time
+            const int64_t b = r * ne0 + i0, n = std::min<int64_t>(32 - (b & 31), ne0 - i0);
+            uint32_t bits = 0;
+            for (int64_t k = 0; k < n; ++k) { const uint32_t v = m[i0 + k]; bits |= (uint32_t)(v == 0u) << k; other |= (uint32_t)(v != 0u && v != 0xff800000u); }
+            out->w[b >> 5] |= bits << (b & 31);
+            i0 += n;
+        }
+    }
+    return other == 0;
+}
+
+void use_device(int device) {   // (most calls find it current)
+    int cur = -1;
+    if (cudaGetDevice(&cur) != cudaSuccess || cur != device) { cudaSetDevice(device); }
+}
+
 }  // namespace
 
 spyb_status spyb_submit(spyb_backend *be, spyb_op_desc *d, void (*callback)(void *), void *user) {
     if (be == nullptr || d == nullptr) { return SPYB_FAIL; }
-    cudaSetDevice(be->config.device_id);
+    use_device(be->config.device_id);
     spyb_status st = SPYB_SUCCESS;
     Staged in[3], out;
     bool   has_out_copy = false;
@@ -710,7 +766,14 @@ spyb_status spyb_submit(spyb_backend *be, spyb_op_desc *d, void (*callback)(void
     case SPYB_OP_RESHAPE: case SPYB_OP_TRANSPOSE: case SPYB_OP_PERMUTE: d->output.data = d->input[0].data; break;
     case SPYB_OP_VIEW: d->output.data = static_cast<uint8_t *>(d->input[0].data) + d->view_offset; break;
     default: {
-        for (int i = 0; i < d->num_input && i < 3 && st == SPYB_SUCCESS; ++i) { st = stage_in(be, d->input[i], &in[i]); }
+        // operands the host reads itself are not copied to the device: token positions, and a mask that fits the kernel's parameters
+        MaskBits mask;
+        const bool mask_packed = d->op_type == SPYB_OP_SOFTMAX && d->num_input == 2 && tensor_contiguous(d->input[0]) && pack_mask(d->input[0], d->input[1], &mask);
+        const bool host_second = mask_packed || (d->op_type == SPYB_OP_ROPE && d->num_input == 2 && d->input[1].node_type == SPYB_NODE_IO);
+        for (int i = 0; i < d->num_input && i < 3 && st == SPYB_SUCCESS; ++i) {
+            if (i == 1 && host_second) { in[1].dev = d->input[1].data; continue; }
+            st = stage_in(be, d->input[i], &in[i]);
+        }
         if (st == SPYB_SUCCESS && d->op_type != SPYB_OP_COPY) { st = stage_out_begin(be, d->output, &out); has_out_copy = out.temp; }
         if (st != SPYB_SUCCESS) { break; }
         spyb_op_desc local = *d;
@@ -739,6 +802,11 @@ spyb_status spyb_submit(spyb_backend *be, spyb_op_desc *d, void (*callback)(void
         case SPYB_OP_SOFTMAX: {
             if (d->num_input != 2 || !tensor_contiguous(a)) { be->set_error("Softmax: contiguous scores and a mask expected"); st = SPYB_UNSUPPORTED; break; }
             const spyb_tensor &mk = local.input[1];
+            if (mask_packed) {
+                err = launch_softmax_bits(static_cast<const float *>(a.data), mask, static_cast<float *>(out.dev), a.elements[0], a.elements[1], a.elements[2] * a.elements[3],
+                                          d->softmax_scale, be->d_exp_table, be->stream);
+                break;
+            }
             err = launch_softmax_masked(static_cast<const float *>(a.data), static_cast<const float *>(mk.data), static_cast<float *>(out.dev),
                                         a.elements[0], a.elements[1], a.elements[2] * a.elements[3], mk.bytes[1] / 4, d->softmax_scale, be->d_exp_table, be->stream);
         } break;
@@ -747,17 +815,28 @@ spyb_status spyb_submit(spyb_backend *be, spyb_op_desc *d, void (*callback)(void
                 be->set_error("Rope: only mode Norm with default scaling is implemented"); st = SPYB_UNSUPPORTED; break;
             }
             {
-                // (cos, sin) per (token, pair) with the host libm and the CPU operator's repeated f32 multiplication of theta
-                // (backend/host/operator/non-linear.cpp:282, 300-309), so the rotation is bit-identical to the CPU's
                 const int64_t n_tok = a.elements[2], npair = a.elements[0] / 2;
-                std::vector<int32_t> pos((size_t)n_tok);
-                if (d->input[1].node_type == SPYB_NODE_IO) { std::memcpy(pos.data(), d->input[1].data, (size_t)n_tok * 4); }
-                else if (cudaMemcpyAsync(pos.data(), d->input[1].data, (size_t)n_tok * 4, cudaMemcpyDeviceToHost, be->stream) != cudaSuccess ||
-                         cudaStreamSynchronize(be->stream) != cudaSuccess) { be->set_error("Rope: reading positions failed"); st = SPYB_FAIL; break; }
+                std::vector<int32_t> pos_read;
+                const int32_t *pos = static_cast<const int32_t *>(d->input[1].data);
+                if (d->input[1].node_type != SPYB_NODE_IO) {
+                    pos_read.resize((size_t)n_tok);
+                    if (cudaMemcpyAsync(pos_read.data(), d->input[1].data, (size_t)n_tok * 4, cudaMemcpyDeviceToHost, be->stream) != cudaSuccess ||
+                        cudaStreamSynchronize(be->stream) != cudaSuccess) { be->set_error("Rope: reading positions failed"); st = SPYB_FAIL; break; }
+                    pos = pos_read.data();
+                }
+                if (n_tok <= ROPE_ROWS) {
+                    if (const float2 *rows = rope_rows(be, d->rope, pos, n_tok, npair)) {
+                        RopeRows rr;
+                        for (int64_t i = 0; i < n_tok; ++i) { rr.row[i] = pos[i]; }
+                        err = launch_rope_rows(to_strided(a, a.data), rows, rr, to_strided(local.output, out.dev), be->stream);
+                        break;
+                    }
+                }
+                // many tokens, or positions outside the table: (cos, sin) per (token, pair) for this call alone, the same arithmetic
                 std::vector<float2> tab((size_t)(n_tok * npair));
                 const float theta_scale = std::pow(d->rope.freq_base, -2.0f / (float)d->rope.num_dim);
                 for (int64_t i = 0; i < n_tok; ++i) {
-                    float theta = (float)pos[(size_t)i];
+                    float theta = (float)pos[i];
                     for (int64_t k = 0; k < npair; ++k) { tab[(size_t)(i * npair + k)] = make_float2(std::cos(theta) * 1.0f, std::sin(theta) * 1.0f); theta *= theta_scale; }
                 }
                 void *dtab = be->arena.alloc(tab.size() * sizeof(float2));

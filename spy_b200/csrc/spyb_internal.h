@@ -48,6 +48,16 @@ struct PendingCallback {
     void *user;
 };
 
+// (cos, sin) rows of the per-operator Rope, one per position, filled as positions come up and kept: every layer of a step rotates Q and K by
+// the same few rows. Arena memory, released with the backend.
+struct RopeTable {
+    float    freq_base = 0.f;
+    int32_t  num_dim = 0;
+    int64_t  npair = 0;
+    float2  *dev = nullptr;                // [have.size()][npair]
+    std::vector<uint8_t> have;
+};
+
 }  // namespace spyb
 
 struct spyb_backend {
@@ -78,6 +88,9 @@ struct spyb_backend {
     std::unordered_map<const void *, uint8_t *>       kq_relaid;     // raw pointer of a Q6_K constant -> its rows in the K-quant mat-vec kernel's layout (made at first use)
     std::unordered_map<const void *, uint8_t *>       pf_tiles;      // raw pointer -> the same matrix in the prompt GEMM's tile layout (made at first use)
     std::vector<void *>                      owned;   // cudaMalloc'd blocks to release at destroy
+
+    std::mutex                   rope_mutex;
+    std::vector<spyb::RopeTable> rope_tables;   // one per (base, dimensions) seen
 
     // completion callbacks
     std::thread                      cb_thread;

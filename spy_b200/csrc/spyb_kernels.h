@@ -220,8 +220,16 @@ cudaError_t launch_binary_rows(int op /*0 add, 1 mul*/, const float *a, const fl
 cudaError_t launch_silu(const float *x, float *out, int64_t n, const float *silu_table, cudaStream_t s);
 cudaError_t launch_softmax_masked(const float *scores, const float *mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2,
                                   int64_t mask_stride, float scale, const float *exp_table, cudaStream_t s);
+// the same with a mask of zeros (bit set) and -inf packed into the kernel's parameters: bit i1 * ne0 + i0
+constexpr int MASK_BITS = 8192;
+struct MaskBits { uint32_t w[MASK_BITS / 32]; };
+cudaError_t launch_softmax_bits(const float *scores, const MaskBits &mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2, float scale, const float *exp_table, cudaStream_t s);
 // cos_sin: device table [ne2 tokens][ne0/2] of (cos, sin) built on the host with the host libm
+// pos: row of the table for every token (by value: up to ROPE_ROWS tokens)
+constexpr int ROPE_ROWS = 64;
+struct RopeRows { int32_t row[ROPE_ROWS]; };
 cudaError_t launch_rope(const Strided &x, const float2 *cos_sin, const Strided &out, cudaStream_t s);
+cudaError_t launch_rope_rows(const Strided &x, const float2 *cos_sin, const RopeRows &rows, const Strided &out, cudaStream_t s);
 cudaError_t launch_copy_strided(const Strided &src, int src_type, const Strided &dst, int dst_type, cudaStream_t s);
 cudaError_t launch_getrow(const uint8_t *table, int table_type, int64_t row_bytes, int64_t ne0, const int32_t *ids, int64_t n_ids, float *out, cudaStream_t s);
 cudaError_t launch_matmul_f16(const Strided &w /*f16*/, const Strided &x /*f32*/, const Strided &out /*f32*/, cudaStream_t s);

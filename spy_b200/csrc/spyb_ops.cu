@@ -14,6 +14,7 @@
 #include "spyb_common.cuh"
 #include "spyb_kernels.h"
 #include "spyb_tp.cuh"
+#include "spyb_mv_common.cuh"
 
 #include <math_constants.h>
 
@@ -1005,8 +1006,7 @@ __global__ void rmsnorm_kernel(const float *x, float *out, int64_t n, float eps)
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        float sum = 0.f;
-        for (int g = 0; g < n4; ++g) { sum = __fadd_rn(sum, v3[g]); }
+        float sum = running_sum_serial(v3, n4);
         for (int64_t i = (int64_t)n4 * 4; i < n; ++i) { sum = fmaf(xr[i], xr[i], sum); }
         scale_s = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)n), eps)));
     }
@@ -1056,20 +1056,15 @@ cudaError_t launch_silu(const float *x, float *out, int64_t n, const float *silu
 
 // operator_masked_softmax_execute, non-linear.cpp:129-180; one CTA per row (i1, i2), row length ne0,
 // the row kept in shared memory; the sum follows std::reduce's order (reduce4_chain).
-__global__ void softmax_masked_kernel(const float *scores, const float *mask, float *out, int64_t ne0, int64_t ne1,
-                                      int64_t mask_stride, float scale, const float *exp_table) {
+template <class Mask>   // mask_at(i): the row's additive mask
+__device__ __forceinline__ void softmax_masked_row(const float *src, float *dst, int64_t ne0, float scale, const float *exp_table, const Mask &mask_at) {
     extern __shared__ __align__(16) float row_s[];
     __shared__ float red[8];
     __shared__ float bcast;
-    const int64_t row = blockIdx.x;
-    const int64_t i1  = row % ne1;
-    const float  *src = scores + row * ne0;
-    const float  *mk  = mask + i1 * mask_stride;
-    float        *dst = out + row * ne0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float m = -CUDART_INF_F;
     for (int64_t i = threadIdx.x; i < ne0; i += blockDim.x) {
-        const float v = __fmul_rn(__fadd_rn(src[i], mk[i]), scale);
+        const float v = __fmul_rn(__fadd_rn(src[i], mask_at(i)), scale);
         row_s[i] = v;
         m = fmaxf(m, v);
     }
@@ -1079,13 +1074,32 @@ __global__ void softmax_masked_kernel(const float *scores, const float *mask, fl
     m = red[0];
     for (int w = 1; w < nw; ++w) { m = fmaxf(m, red[w]); }
     for (int64_t i = threadIdx.x; i < ne0; i += blockDim.x) {
-        row_s[i] = (mk[i] == -CUDART_INF_F) ? 0.f : exp_table[f2h(__fsub_rn(row_s[i], m))];
+        row_s[i] = (mask_at(i) == -CUDART_INF_F) ? 0.f : exp_table[f2h(__fsub_rn(row_s[i], m))];
     }
     __syncthreads();
     if (threadIdx.x == 0) { bcast = __fdiv_rn(1.0f, reduce4_chain(row_s, (int)ne0)); }
     __syncthreads();
     const float inv = bcast;
     for (int64_t i = threadIdx.x; i < ne0; i += blockDim.x) { dst[i] = __fmul_rn(row_s[i], inv); }
+}
+__global__ void softmax_masked_kernel(const float *scores, const float *mask, float *out, int64_t ne0, int64_t ne1,
+                                      int64_t mask_stride, float scale, const float *exp_table) {
+    const int64_t row = blockIdx.x;
+    const float  *mk  = mask + (row % ne1) * mask_stride;
+    softmax_masked_row(scores + row * ne0, out + row * ne0, ne0, scale, exp_table, [mk](int64_t i) { return mk[i]; });
+}
+__global__ void softmax_bits_kernel(const float *scores, const __grid_constant__ MaskBits mask, float *out, int64_t ne0, int64_t ne1, float scale, const float *exp_table) {
+    const int64_t row = blockIdx.x;
+    const int     bit0 = (int)((row % ne1) * ne0);
+    softmax_masked_row(scores + row * ne0, out + row * ne0, ne0, scale, exp_table, [&mask, bit0](int64_t i) {
+        const int b = bit0 + (int)i;
+        return (mask.w[b >> 5] >> (b & 31)) & 1u ? 0.f : -CUDART_INF_F;
+    });
+}
+cudaError_t launch_softmax_bits(const float *scores, const MaskBits &mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2, float scale, const float *exp_table, cudaStream_t s) {
+    if (ne0 < 1 || ne1 < 1 || ne2 < 1 || ne0 * ne1 > MASK_BITS) { return cudaErrorInvalidValue; }
+    softmax_bits_kernel<<<(unsigned)(ne1 * ne2), 256, (size_t)ne0 * sizeof(float), s>>>(scores, mask, out, ne0, ne1, scale, exp_table);   // (at most 32 KB of shared memory)
+    return launch_check();
 }
 cudaError_t launch_softmax_masked(const float *scores, const float *mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2,
                                   int64_t mask_stride, float scale, const float *exp_table, cudaStream_t s) {
@@ -1109,23 +1123,38 @@ __device__ __forceinline__ int64_t soff(const Strided &t, int64_t i0, int64_t i1
 // OperatorRopeImpl::execute in mode Norm with default YaRN settings, non-linear.cpp:270-371.
 // One thread per (pair, head, token); the (cos, sin) of every (token, pair) comes from a table the host
 // fills with the same libm calls and the same repeated f32 multiplication of theta as the CPU operator.
-__global__ void rope_kernel(const Strided x, const float2 *cos_sin, const Strided out) {
-    const int64_t npair = x.ne[0] >> 1;
-    const int64_t i     = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t tot   = npair * x.ne[1] * x.ne[2];
-    if (i >= tot) { return; }
-    const int64_t k = i % npair, i1 = (i / npair) % x.ne[1], i2 = i / (npair * x.ne[1]);
-    const float2 cs = cos_sin[i2 * npair + k];
+__device__ __forceinline__ void rope_pair(const Strided &x, const Strided &out, float2 cs, int64_t k, int64_t i1, int64_t i2) {
     const float *src = reinterpret_cast<const float *>(reinterpret_cast<const uint8_t *>(x.data) + soff(x, 2 * k, i1, i2, 0));
     float       *dst = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(out.data) + soff(out, 2 * k, i1, i2, 0));
     const float x0 = src[0], x1 = src[1];
     dst[0] = __fsub_rn(__fmul_rn(x0, cs.x), __fmul_rn(x1, cs.y));
     dst[1] = __fadd_rn(__fmul_rn(x0, cs.y), __fmul_rn(x1, cs.x));
 }
+__global__ void rope_kernel(const Strided x, const float2 *cos_sin, const Strided out) {
+    const int64_t npair = x.ne[0] >> 1;
+    const int64_t i     = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= npair * x.ne[1] * x.ne[2]) { return; }
+    const int64_t k = i % npair, i1 = (i / npair) % x.ne[1], i2 = i / (npair * x.ne[1]);
+    rope_pair(x, out, cos_sin[i2 * npair + k], k, i1, i2);
+}
+__global__ void rope_rows_kernel(const Strided x, const float2 *cos_sin, const __grid_constant__ RopeRows rows, const Strided out) {
+    const int64_t npair = x.ne[0] >> 1;
+    const int64_t i     = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= npair * x.ne[1] * x.ne[2]) { return; }
+    const int64_t k = i % npair, i1 = (i / npair) % x.ne[1], i2 = i / (npair * x.ne[1]);
+    rope_pair(x, out, cos_sin[(int64_t)rows.row[i2] * npair + k], k, i1, i2);
+}
 cudaError_t launch_rope(const Strided &x, const float2 *cos_sin, const Strided &out, cudaStream_t s) {
     const int64_t tot = (x.ne[0] >> 1) * x.ne[1] * x.ne[2];
     if (tot == 0) { return cudaSuccess; }
     rope_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, s>>>(x, cos_sin, out);
+    return launch_check();
+}
+cudaError_t launch_rope_rows(const Strided &x, const float2 *cos_sin, const RopeRows &rows, const Strided &out, cudaStream_t s) {
+    const int64_t tot = (x.ne[0] >> 1) * x.ne[1] * x.ne[2];
+    if (tot == 0) { return cudaSuccess; }
+    if (x.ne[2] > ROPE_ROWS) { return cudaErrorInvalidValue; }
+    rope_rows_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, s>>>(x, cos_sin, rows, out);
     return launch_check();
 }
 
