@@ -137,14 +137,15 @@ size_t      prefill_act_bytes(int T, int nb);
 cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);
 // weight_type, tile_tok: the type of the matrix the activations will meet (2, 8, 12 or 14) and its token tile: they decide the layout;
 // part_len > 0: a row lies in K / part_len parts, part_stride floats apart
+// pdl (here and below): launch with the programmatic-stream-serialization attribute; the kernels wait for their predecessor themselves
 cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type, int tile_tok,
-                                 int part_len = 0, int64_t part_stride = 0);
-cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream);   // type 12 = Q4_K, 14 = Q6_K (spyb_prefill_kq.cu)
+                                 int part_len = 0, int64_t part_stride = 0, bool pdl = false);
+cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream, bool pdl);   // type 12 = Q4_K, 14 = Q6_K (spyb_prefill_kq.cu)
 cudaError_t launch_prefill_retile_kq(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);
-cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream);
+cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool pdl = false);
 cudaError_t launch_prefill_qkv_post(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,
-                                    __half *v_cache, int n_ctx, int64_t seq_stride, cudaStream_t stream);
-cudaError_t launch_prefill_silu_mul(const float *upgate, int T, int F, const float *silu_table, float *act, cudaStream_t stream);
+                                    __half *v_cache, int n_ctx, int64_t seq_stride, cudaStream_t stream, bool pdl = false);
+cudaError_t launch_prefill_silu_mul(const float *upgate, int T, int F, const float *silu_table, float *act, cudaStream_t stream, bool pdl = false);
 
 struct AttnParams {
     int           force_long = 0;     // take the three-kernel path (scratch needed) also at short contexts
@@ -173,6 +174,18 @@ struct LaunchCfg {
     int          mv_force_s = 0, mv_force_wact = 0;   // tuning overrides (0 = choose)
     int         *error_flag = nullptr;
 };
+
+// a launch with or without the programmatic-stream-serialization attribute (a kernel launched with it waits for its predecessor itself)
+template <class... KArgs, class... Args>
+inline cudaError_t launch_maybe_pdl(void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, bool pdl, Args... args) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid; lc.blockDim = dim3(threads); lc.dynamicSmemBytes = smem; lc.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr; lc.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&lc, kernel, static_cast<KArgs>(args)...);
+}
 
 // Book-keeping for cudaFuncAttributeMaxDynamicSharedMemorySize, which is set per (device, kernel): decide() says
 // whether a launch that needs `bytes` must raise the attribute first (and records the new mark).

@@ -489,7 +489,8 @@ spyb_status ensure_prefill_buffers(spyb_model *m) {
 spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool batch = false) {
     spyb_backend *be = m->be;
     cudaStream_t s = be->stream;
-    const LaunchCfg cfg = be->launch_cfg(false);
+    const bool pdl = be->config.use_pdl != 0;
+    const LaunchCfg cfg = be->launch_cfg(pdl);
     const int d = m->info.d_model, ff = m->info.n_ff, dl = m->dl, fl = m->fl, hd = m->info.head_dim;
     const int tp = m->info.tp_size, rank = m->info.tp_rank;
     // the quantized activations are laid out for the type of the matrix they meet and for its token tile: quant() makes them for the
@@ -498,7 +499,7 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
     auto layout_of = [](int type) { return type == SPYB_Q4_K ? 3 : type == SPYB_Q6_K ? 1 : 2; };   // (Q4_0 and Q8_0 share one)
     auto quant = [&](const float *x, int part_len, int K, const float *norm_w, const PfMat &W, int64_t part_stride) {
         yq_src = {x, part_len, norm_w, K, part_stride, W.type, prefill_tile_tokens(W.type, W.n_rows, T)};
-        return launch_prefill_quant(x, part_len, T, K, norm_w, norm_w != nullptr ? m->info.rms_eps : 0.f, m->pf_yq, s, W.type, yq_src.tile_tok, part_len, part_stride);
+        return launch_prefill_quant(x, part_len, T, K, norm_w, norm_w != nullptr ? m->info.rms_eps : 0.f, m->pf_yq, s, W.type, yq_src.tile_tok, part_len, part_stride, pdl);
     };
     auto gemm = [&](const PfMat &W, int K, float *out, int64_t out_stride, const float *resid) {
         if (layout_of(W.type) != layout_of(yq_src.type)) {
@@ -509,7 +510,7 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
         PrefillGemm g;
         g.w = W.w; g.type = W.type; g.n_rows = W.n_rows; g.nb = K / 32; g.yq = m->pf_yq; g.tile_tok = yq_src.tile_tok; g.T = T; g.out = out; g.out_stride = out_stride; g.resid = resid;
         g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
-        return launch_prefill_gemm(g, s);
+        return launch_prefill_gemm(g, s, pdl);
     };
     // Tensor parallel: every matrix is split by output rows - this rank's heads, FFN rows, and a slice of the rows of W_o and
     // W_down - so each rank produces, for all T tokens, one contiguous part [T][len] of the attention output, the FFN
@@ -537,7 +538,7 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
             *launches += 2;
         }
         __half *kc = batch ? ly.k_base : ly.k_cache, *vc = batch ? ly.v_base : ly.v_cache;
-        SPYB_CUDA(be, launch_prefill_qkv_post(m->pf_qkv, T, dl, hd, m->d_pos, m->rope_table, m->pf_q, kc, vc, m->info.n_ctx, batch ? m->seq_stride : 0, s));
+        SPYB_CUDA(be, launch_prefill_qkv_post(m->pf_qkv, T, dl, hd, m->d_pos, m->rope_table, m->pf_q, kc, vc, m->info.n_ctx, batch ? m->seq_stride : 0, s, pdl));
         *launches += 3;
         AttnParams a;
         a.k_cache = kc; a.v_cache = vc; a.out_stride = dl; a.exp_table = be->d_exp_table; a.seq_stride = batch ? m->seq_stride : 0;
@@ -561,7 +562,7 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
         SPYB_CUDA(be, quant(m->pf_x, dp, d, ly.ffn_norm, ly.pf_ug, (int64_t)T * dp));
         SPYB_CUDA(be, gemm(ly.pf_ug, d, m->pf_ug, 2 * (int64_t)fl, nullptr));
         if (m->kq) { SPYB_CUDA(be, gemm(ly.pf_gate, d, m->pf_ug + fl, 2 * (int64_t)fl, nullptr)); ++*launches; }
-        SPYB_CUDA(be, launch_prefill_silu_mul(m->pf_ug, T, fl, be->d_silu_table, act_part, s));
+        SPYB_CUDA(be, launch_prefill_silu_mul(m->pf_ug, T, fl, be->d_silu_table, act_part, s, pdl));
         if (gather(m->pf_act, fl) != SPYB_SUCCESS) { return SPYB_FAIL; }
         SPYB_CUDA(be, quant(m->pf_act, fl, ff, nullptr, ly.pf_down, (int64_t)T * fl));
         SPYB_CUDA(be, gemm(ly.pf_down, ff, x_part, dp, x_part));

@@ -391,6 +391,8 @@ __global__ void __launch_bounds__(ATT_SC_THREADS) attn_scores_tiled_kernel(const
     constexpr int NQ = ATT_SG * ATT_ST;
     float *ks = att_smem, *qs = att_smem + ATT_HD * ATT_KPITCH;
     const int h = blockIdx.y, tg = blockIdx.z * NQ, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
     const int ng = min(NQ, p.T - tg), j0 = blockIdx.x * ATT_SP;
     const int n_vis_last = p.pos_base[0] + tg + ng;          // positions the last token of the CTA sees
     if (j0 >= n_vis_last) { return; }
@@ -622,6 +624,8 @@ __global__ void __launch_bounds__(ATT_PVT_WARPS * WARP, 16 / ATT_PVT_WARPS) attn
     constexpr int PER_HEAD = ATT_HD / ATT_PVT_ELEMS;
     const int h = blockIdx.x / PER_HEAD, t0 = blockIdx.y * ATT_TT, tid = threadIdx.x, lane = tid & 31, grp = lane >> 3, lg = lane & 7;
     const int e0 = (blockIdx.x % PER_HEAD) * ATT_PVT_ELEMS + (tid >> 5) * 4 * ATT_EE + grp * ATT_EE;
+    pdl_launch_dependents();
+    pdl_wait();
     const int nt = min(ATT_TT, p.T - t0);
     const int n_tot = (p.pos_base[1] > 0) ? p.pos_base[1] : p.pos_base[0] + p.T;
     const int n_pad = (p.n_ctx + 3) & ~3;
@@ -770,7 +774,7 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
     if (p.hd != ATT_HD || p.T < 1 || p.n_ctx < 1 || (p.n_ctx & 3) || (p.dl & 7)) { return cudaErrorInvalidValue; }
     const size_t n_pad = ((size_t)p.n_ctx + 3) & ~(size_t)3;
     if ((p.n_ctx > ATT_LONG_MIN || p.force_long) && p.scratch != nullptr) {
-        const bool tiled = p.T >= ATT_TT && p.tp.counter == nullptr && !cfg.pdl && p.seq_stride == 0;   // a prompt: tokens share the K rows and the V^T rows
+        const bool tiled = p.T >= ATT_TT && p.tp.counter == nullptr && p.seq_stride == 0;   // a prompt: tokens share the K rows and the V^T rows
         cudaError_t err = tiled ? allow_dynamic_smem(reinterpret_cast<const void *>(attn_scores_tiled_kernel), ATT_SC_SMEM) : cudaSuccess;
         if (err != cudaSuccess) { return err; }
         err = tiled

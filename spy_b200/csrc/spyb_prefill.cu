@@ -78,6 +78,9 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
     const int n_tile = n_tok * (int)((g.n_rows + PF_M - 1) / PF_M);
     const uint64_t limit = g.wait_limit_ns;
 
+    // The barriers, the zeroed B operands, the tensor memory and the first weights need nothing of the previous kernel; every role waits
+    // for it before it touches activations or results.
+    pdl_launch_dependents();
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(raw_full(s), 1); mbar_init(ops_full(s), 1); mbar_init(st_free(s), 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(d_full(i), 1); mbar_init(d_free(i), PF_GEMM_EPI_WARPS); }
@@ -103,6 +106,18 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             int st = 0, k = 0, issued = 0;
             uint32_t par = 1;
             bool ok = true;
+            // the weights of the first tile's first steps, then (the previous kernel is done) their activations with all that follows
+            const int early = blockIdx.x < n_tile ? min(NS, n_step) : 0;
+            if (elect_one()) {
+                for (int i = 0; i < early; ++i) {
+                    if (i == g.selftest_skip_step) { continue; }
+                    const int n = min(NB, nb - i * NB);
+                    mbar_expect_tx(raw_full(i), (uint32_t)(n * (PF_WTILE_F16 + YB)));
+                    bulk_copy_g2s(sbase + (uint32_t)i * G::STAGE, g.w + ((int64_t)(blockIdx.x / n_tok) * nb + i * NB) * PF_WTILE_F16, (uint32_t)(n * PF_WTILE_F16), raw_full(i));
+                }
+            }
+            __syncwarp();
+            pdl_wait();
             for (int tile = blockIdx.x; tile < n_tile && ok; tile += gridDim.x) {
                 const uint8_t *wsrc = g.w + (int64_t)(tile / n_tok) * nb * PF_WTILE_F16;
                 const uint8_t *ysrc = g.yq + (int64_t)(tile % n_tok) * nb * YB;
@@ -114,8 +129,10 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                     const int n = min(NB, nb - i * NB);
                     if (k != g.selftest_skip_step && elect_one()) {   // (failure-path check: that step never arrives)
                         const uint32_t dst = sbase + (uint32_t)st * G::STAGE;
-                        mbar_expect_tx(raw_full(st), (uint32_t)(n * (PF_WTILE_F16 + YB)));
-                        bulk_copy_g2s(dst, wsrc, (uint32_t)(n * PF_WTILE_F16), raw_full(st));
+                        if (k >= early) {
+                            mbar_expect_tx(raw_full(st), (uint32_t)(n * (PF_WTILE_F16 + YB)));
+                            bulk_copy_g2s(dst, wsrc, (uint32_t)(n * PF_WTILE_F16), raw_full(st));
+                        }
                         bulk_copy_g2s(dst + NB * PF_WTILE_F16, ysrc, (uint32_t)(n * YB), raw_full(st));
                     }
                     __syncwarp();
@@ -200,6 +217,7 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             if (mine > 0 && !mbar_wait_relaxed(d_full(m), (uint32_t)(mine - 1) & 1u, limit)) { if (lane == 0) { pf_report(g.error_flag, 5); } }
         }
     } else {
+        pdl_wait();
         // ---- epilogue: tokens part * TT / 4 .. of the tile as PW packed pairs (tokens 2 u, 2 u + 1), eight accumulators each. D's columns
         // of block j and half h: 8 TT j + 4 TT h + 8 (t / 2) + 2 n + t % 2, i.e. a pair's accumulator n is a neighbouring pair of columns.
         const int quad = warp & 3, part = warp >> 2;
@@ -316,6 +334,8 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
     extern __shared__ __align__(16) float v3[];
     __shared__ float scale_s;
     const int tid = threadIdx.x, token = blockIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     const int n4 = K >> 2, nb = K >> 5;
     const int npass = (n4 + PF_QUANT_THREADS - 1) / PF_QUANT_THREADS;
     // a row may lie in parts (the slices the ranks of a tensor-parallel group gathered): elements [i part_len, (i + 1) part_len)
@@ -439,6 +459,8 @@ __global__ void prefill_qkv_post_kernel(const float *qkv, int T, int dl, int hd,
                                         __half *v_cache, int n_ctx, int64_t seq_stride) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t per_token = 3 * (int64_t)dl / 2;
+    pdl_launch_dependents();
+    pdl_wait();
     if (i >= per_token * T) { return; }
     const int t = (int)(i / per_token);
     const int64_t col = 2 * (i - (int64_t)t * per_token);
@@ -461,6 +483,8 @@ __global__ void prefill_qkv_post_kernel(const float *qkv, int T, int dl, int hd,
 // up * silu(gate) (model/src/llm/plugin/ffn.cpp:28-35) on the output [T][2 F] of the stacked up|gate GEMM
 __global__ void prefill_silu_mul_kernel(const float *upgate, int T, int F, const float *silu_table, float *act) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     if (i >= (int64_t)T * F) { return; }
     const int t = (int)(i / F);
     const int64_t f = i - (int64_t)t * F;
@@ -480,13 +504,12 @@ int device_sms() {
 }
 
 template <int TT>
-cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream) {
+cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     const size_t smem = PfGeom<TT>::SMEM;
     cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(prefill_gemm_kernel<TT>), smem);
     if (err != cudaSuccess) { return err; }
     const int64_t tiles = (int64_t)((g.T + TT - 1) / TT) * ((g.n_rows + PF_M - 1) / PF_M);
-    prefill_gemm_kernel<TT><<<(unsigned)std::min<int64_t>(tiles, device_sms()), PF_GEMM_THREADS, smem, stream>>>(g);
-    return cudaGetLastError();
+    return launch_maybe_pdl(prefill_gemm_kernel<TT>, dim3((unsigned)std::min<int64_t>(tiles, device_sms())), PF_GEMM_THREADS, smem, stream, pdl, g);
 }
 
 }  // namespace
@@ -522,7 +545,7 @@ cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stri
 }
 
 cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type,
-                                 int tile_tok, int part_len, int64_t part_stride) {
+                                 int tile_tok, int part_len, int64_t part_stride, bool pdl) {
     if (weight_type != 2 && weight_type != 8 && weight_type != 12 && weight_type != 14) { return cudaErrorInvalidValue; }
     if (part_len <= 0) { part_len = K; part_stride = 0; }
     if ((part_len & 3) || (part_stride & 3) || K % part_len != 0) { return cudaErrorInvalidValue; }
@@ -531,31 +554,28 @@ cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K,
     auto *kernel = weight_type == 12 ? (norm_w ? prefill_quant_kernel<true, 2> : prefill_quant_kernel<false, 2>)
                  : weight_type == 14 ? (norm_w ? prefill_quant_kernel<true, 1> : prefill_quant_kernel<false, 1>)
                                      : (norm_w ? prefill_quant_kernel<true, 0> : prefill_quant_kernel<false, 0>);
-    kernel<<<T, PF_QUANT_THREADS, smem, stream>>>(x, x_stride, K, norm_w, eps, yq, tile_tok, part_len, part_stride);
-    return cudaGetLastError();
+    return launch_maybe_pdl(kernel, dim3((unsigned)T), PF_QUANT_THREADS, smem, stream, pdl, x, x_stride, K, norm_w, eps, yq, tile_tok, part_len, part_stride);
 }
 
-cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream) {
-    if (g.type == 12 || g.type == 14) { return launch_prefill_gemm_kq(g, stream); }
+cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
+    if (g.type == 12 || g.type == 14) { return launch_prefill_gemm_kq(g, stream, pdl); }
     if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
     switch (g.tile_tok) {
-    case 16: return launch_gemm_t<16>(g, stream);
-    case 8:  return launch_gemm_t<8>(g, stream);
+    case 16: return launch_gemm_t<16>(g, stream, pdl);
+    case 8:  return launch_gemm_t<8>(g, stream, pdl);
     default: return cudaErrorInvalidValue;
     }
 }
 
 cudaError_t launch_prefill_qkv_post(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,
-                                    __half *v_cache, int n_ctx, int64_t seq_stride, cudaStream_t stream) {
+                                    __half *v_cache, int n_ctx, int64_t seq_stride, cudaStream_t stream, bool pdl) {
     const int64_t n = 3 * (int64_t)dl / 2 * T;
-    prefill_qkv_post_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(qkv, T, dl, hd, pos_base, rope, q_out, k_cache, v_cache, n_ctx, seq_stride);
-    return cudaGetLastError();
+    return launch_maybe_pdl(prefill_qkv_post_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, pdl, qkv, T, dl, hd, pos_base, rope, q_out, k_cache, v_cache, n_ctx, seq_stride);
 }
 
-cudaError_t launch_prefill_silu_mul(const float *upgate, int T, int F, const float *silu_table, float *act, cudaStream_t stream) {
+cudaError_t launch_prefill_silu_mul(const float *upgate, int T, int F, const float *silu_table, float *act, cudaStream_t stream, bool pdl) {
     const int64_t n = (int64_t)T * F;
-    prefill_silu_mul_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(upgate, T, F, silu_table, act);
-    return cudaGetLastError();
+    return launch_maybe_pdl(prefill_silu_mul_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, pdl, upgate, T, F, silu_table, act);
 }
 
 }  // namespace spyb

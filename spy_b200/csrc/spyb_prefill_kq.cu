@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kq_gemm_kernel(PrefillG
     const uint8_t *wsrc = g.w + ((int64_t)row_tile * nb) * KQ_WT;
     const uint8_t *ysrc = g.yq + ((int64_t)tok_tile * nb) * KQ_YQ;
 
+    pdl_launch_dependents();
     if (tid == 0) {
         for (int q = 0; q < NQ; ++q) { mbar_init(raw_full(q), 1); mbar_init(ops_full(q), 1); mbar_init(st_free(q), PF_EPI_WARPS); }
         for (int i = 0; i < PF_DBUF; ++i) { mbar_init(d_full(i), 1); mbar_init(d_free(i), PF_EPI_WARPS); }
@@ -111,6 +112,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kq_gemm_kernel(PrefillG
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
 
     if (warp >= PF_EPI_WARPS + 2) {
         // ---- MMA warps
@@ -318,21 +320,20 @@ __global__ void prefill_kq_retile_kernel(const uint8_t *raw, int64_t row_stride,
 }
 
 template <int WT>
-cudaError_t launch_kq_t(const PrefillGemm &g, cudaStream_t stream) {
+cudaError_t launch_kq_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     constexpr size_t KQ_SMEM_BYTES = KqGeom<WT>::SMEM;
     cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(prefill_kq_gemm_kernel<WT>), KQ_SMEM_BYTES);
     if (err != cudaSuccess) { return err; }
     const dim3 grid((unsigned)((g.T + KQ_TOK - 1) / KQ_TOK), (unsigned)((g.n_rows + PF_M - 1) / PF_M));
-    prefill_kq_gemm_kernel<WT><<<grid, PF_THREADS, KQ_SMEM_BYTES, stream>>>(g);
-    return cudaGetLastError();
+    return launch_maybe_pdl(prefill_kq_gemm_kernel<WT>, grid, PF_THREADS, KQ_SMEM_BYTES, stream, pdl, g);
 }
 
 }  // namespace
 
-cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream) {
+cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     if (g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 8 || (g.nb & 7) || g.n_rows < 1) { return cudaErrorInvalidValue; }
-    if (g.type == 12) { return launch_kq_t<12>(g, stream); }
-    if (g.type == 14) { return launch_kq_t<14>(g, stream); }
+    if (g.type == 12) { return launch_kq_t<12>(g, stream, pdl); }
+    if (g.type == 14) { return launch_kq_t<14>(g, stream, pdl); }
     return cudaErrorInvalidValue;
 }
 
