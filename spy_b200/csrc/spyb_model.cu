@@ -165,6 +165,7 @@ struct spyb_model {
     std::vector<Layer> layers;
     DevMatrix       head;
     KqSeg           kq_head;
+    PfMat           pf_head;                 // the head in the prompt GEMM's tile layout: batches of sequences take their logits from one GEMM
     bool            kq = false;              // every matrix is a K-quant: the step plan runs on the K-quant mat-vec kernel
     float          *output_norm = nullptr;
     uint8_t        *embd = nullptr;
@@ -861,6 +862,10 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
             if (ps != SPYB_SUCCESS) { m->pf_ok = false; }   // a mix of types inside one stacked matrix: prompts stay on the mat-vec passes
         }
     }
+    if (m->pf_ok) {
+        const std::string head_name = m->kq || f.tensors.count("output.weight") ? "output.weight" : "token_embd.weight";
+        if (upload_pf(head_name, d, I.n_vocab, &m->pf_head, 0, I.n_vocab) == SPYB_FAIL) { return fail(SPYB_FAIL); }   // (another type: the head stays on the mat-vec passes)
+    }
     I.weight_bytes += (uint64_t)(2 * I.n_layer + 1) * d * 4;
     I.kv_bytes_per_token = (uint64_t)2 * I.n_layer * dl * 2;
     m->seq_stride = (int64_t)I.n_ctx * dl;
@@ -1321,7 +1326,7 @@ spyb_status spyb_model_decode_batch(spyb_model *m, const int32_t *first_tokens, 
     if (tp > 1 && !gemm) { be->set_error("decode_batch: a sharded model takes at most %d sequences", m->pf_chunk); return SPYB_UNSUPPORTED; }
     if (gemm && ensure_prefill_buffers(m) != SPYB_SUCCESS) { return SPYB_FAIL; }
     for (int step = 0; step < n_steps; ++step) {
-        if (gemm) {   // the sequences of a step are the "tokens" of one GEMM pass; the head runs on groups of columns
+        if (gemm) {   // the sequences of a step are the "tokens" of one GEMM pass
             if (tp == 1) { SPYB_CUDA(be, launch_embed(m->batch_tokens, n_seq, m->embd, m->embd_type, d, m->pf_x, be->stream)); ++launches; }
             else {        // the residual stream in tp parts [tp][n_seq][d / tp], as for a prompt
                 SPYB_CUDA(be, launch_embed(m->batch_tokens, n_seq, m->embd, m->embd_type, d, m->pf_att, be->stream)); ++launches;
@@ -1331,7 +1336,16 @@ spyb_status spyb_model_decode_batch(spyb_model *m, const int32_t *first_tokens, 
                 }
             }
             if (run_prefill_layers(m, n_seq, &launches, true) != SPYB_SUCCESS) { return SPYB_FAIL; }
-            for (int g0 = 0; g0 < n_seq; g0 += group) {
+            if (m->pf_head.w != nullptr) {   // the logits of all sequences from one GEMM
+                const bool pdl = be->config.use_pdl != 0;
+                PrefillGemm g;
+                g.w = m->pf_head.w; g.type = m->pf_head.type; g.n_rows = V; g.nb = d / 32; g.yq = m->pf_yq; g.tile_tok = prefill_tile_tokens(g.type, V, n_seq);
+                g.T = n_seq; g.out = m->logits_batch; g.out_stride = V; g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
+                SPYB_CUDA(be, launch_prefill_quant(m->pf_x, dp, n_seq, d, m->output_norm, m->info.rms_eps, m->pf_yq, be->stream, g.type, g.tile_tok, dp, (int64_t)n_seq * dp, pdl));
+                SPYB_CUDA(be, launch_prefill_gemm(g, be->stream, pdl));
+                launches += 2;
+            }
+            for (int g0 = 0; m->pf_head.w == nullptr && g0 < n_seq; g0 += group) {
                 const int T = std::min(group, n_seq - g0);
                 for (int i = 0; i < tp; ++i) {   // whole rows of the group's columns from their parts
                     SPYB_CUDA(be, cudaMemcpy2DAsync(m->x + (size_t)i * dp, (size_t)d * 4, m->pf_x + (size_t)i * n_seq * dp + (size_t)g0 * dp, (size_t)dp * 4, (size_t)dp * 4, (size_t)T,
