@@ -200,7 +200,7 @@ spyb_status spyb_matmul_noalloc(spyb_backend *backend, int32_t weight_type, cons
  * Needs k a multiple of 32 (256 for Q4_K / Q6_K; <= 14336) and 1..4096 columns; anything else is SPYB_UNSUPPORTED.
  * Stages everything inside the call (it allocates and synchronises): the entry point of the parity tests, while
  * spyb_model_eval runs the same kernels on resident buffers for prompts of SPYB_PREFILL_MIN_TOKENS tokens and more. */
-#define SPYB_PREFILL_MIN_TOKENS 16
+#define SPYB_PREFILL_MIN_TOKENS 8
 spyb_status spyb_prefill_matmul(spyb_backend *backend, int32_t weight_type, const void *w_rows_host, int64_t n_rows, int64_t k,
                                 const float *x_host, int64_t n_cols, const float *norm_w_host, float eps, float *out_host);
 

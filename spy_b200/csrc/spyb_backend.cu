@@ -520,7 +520,7 @@ void stage_release(spyb_backend *be, Staged *s) {
     s->dev = nullptr; s->temp = false;
 }
 
-// MatMul of 16 and more activation columns against an uploaded constant: the tcgen05 GEMM of the prompt path (same bits as
+// MatMul of several activation columns against an uploaded constant: the tcgen05 GEMM of the prompt path (same bits as
 // the mat-vec kernels). The matrix gets a second copy in that kernel's tile layout at first use, kept with the constant.
 // Returns SPYB_UNSUPPORTED without an error text when the operands do not qualify (the caller then takes the mat-vec route).
 spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_tensor &x, void *out_dev) {
@@ -528,14 +528,14 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
     const bool kq = type == SPYB_Q4_K || type == SPYB_Q6_K;
     if (type != SPYB_Q4_0 && type != SPYB_Q8_0 && !kq) { return SPYB_UNSUPPORTED; }
     const int64_t k = w.elements[0], n_rows = w.elements[1], T = x.elements[1] * x.elements[2] * x.elements[3];
-    if (T < SPYB_PREFILL_MIN_TOKENS || w.node_type != SPYB_NODE_CONSTANT || k != x.elements[0] || k < QK || k % QK != 0 || k > PF_MAX_K || (kq && k % 256 != 0) ||
+    if (T < 5 || w.node_type != SPYB_NODE_CONSTANT || k != x.elements[0] || k < QK || k % QK != 0 || k > PF_MAX_K || (kq && k % 256 != 0) ||
         n_rows < 1 || w.elements[2] != 1 || w.elements[3] != 1 || !tensor_contiguous(w) || !tensor_contiguous(x) ||
         (reinterpret_cast<uintptr_t>(x.data) & 15) || (reinterpret_cast<uintptr_t>(out_dev) & 3)) {
         return SPYB_UNSUPPORTED;
     }
-    // Q4_0 / Q8_0: a GEMM CTA walks all of K for 128 rows x 16 columns, so few tiles leave most SMs idle and passes of four
-    // columns through the mat-vec kernel are faster (measured: 4096 rows x 16 columns slower, 11008 x 16 faster)
-    if (!kq && ((n_rows + PF_ROWS - 1) / PF_ROWS) * ((T + PF_TOK - 1) / PF_TOK) < 74) { return SPYB_UNSUPPORTED; }
+    // Two passes of the mat-vec kernels (up to eight columns) are faster only for long rows of a matrix that leaves half the SMs without a
+    // tile: a GEMM CTA walks all of K (4096 x 11008 x 6 columns: 57 us against 47; 4096 x 4096: 19 against 25; 11008 x 4096: 24 against 39)
+    if (T <= 8 && k > 8192 && (n_rows + PF_ROWS - 1) / PF_ROWS < 74) { return SPYB_UNSUPPORTED; }
     static const bool off = [] { const char *e = std::getenv("SPYB_PREFILL"); return e != nullptr && e[0] == '0'; }();
     if (off) { return SPYB_UNSUPPORTED; }
     const int nb = (int)(k / QK);
@@ -565,21 +565,21 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
     struct Release { spyb_backend *be; void *a; size_t n; ~Release() { be->arena.free(a, n); } } release{be, yq, ybytes};   // (stream-ordered reuse)
     for (int64_t t0 = 0; t0 < T; t0 += chunk) {
         const int Tc = (int)std::min(chunk, T - t0);
-        SPYB_CUDA(be, cudaMemsetAsync(yq, 0, prefill_act_bytes(Tc, nb), be->stream));
+        const bool pdl = be->config.use_pdl != 0;   // (columns that pad the last tile hold whatever the buffer held: their results are not stored)
         PrefillGemm g;
         g.tile_tok = prefill_tile_tokens(type, n_rows, Tc);
-        SPYB_CUDA(be, launch_prefill_quant(static_cast<const float *>(x.data) + t0 * k, k, Tc, (int)k, nullptr, 0.f, static_cast<uint8_t *>(yq), be->stream, type, g.tile_tok));
+        SPYB_CUDA(be, launch_prefill_quant(static_cast<const float *>(x.data) + t0 * k, k, Tc, (int)k, nullptr, 0.f, static_cast<uint8_t *>(yq), be->stream, type, g.tile_tok, 0, 0, pdl));
         g.w = tiles; g.type = type; g.n_rows = n_rows; g.nb = nb; g.yq = static_cast<uint8_t *>(yq); g.T = Tc;
         g.out = static_cast<float *>(out_dev) + t0 * n_rows; g.out_stride = n_rows;
         g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
-        SPYB_CUDA(be, launch_prefill_gemm(g, be->stream));
+        SPYB_CUDA(be, launch_prefill_gemm(g, be->stream, pdl));
     }
     return SPYB_SUCCESS;
 }
 
-// MatMul of fewer than 16 columns against an uploaded Q4_K / Q6_K constant: the model path's K-quant mat-vec kernel, up to four
+// MatMul of a few columns against an uploaded Q4_K / Q6_K constant: the model path's K-quant mat-vec kernel, up to four
 // columns per launch (activations quantized to Q8_0 first, the arithmetic of the restatement; the tensor-core route above gives the
-// same bits for 16 columns and more). Q6_K rows get a copy in that kernel's layout at first use.
+// same bits). Q6_K rows get a copy in that kernel's layout at first use.
 spyb_status run_matmul_kq_constant(spyb_backend *be, const spyb_tensor &w, const spyb_tensor &x, void *out_dev) {
     const int type = w.number_type;
     const int64_t k = w.elements[0], n_rows = w.elements[1], T = x.elements[1] * x.elements[2] * x.elements[3];

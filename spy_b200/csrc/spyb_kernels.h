@@ -111,10 +111,8 @@ struct MatvecParams {
 // activations as compact Q8_0 blocks grouped by (token tile, block).
 constexpr int PF_ROWS = 128, PF_TOK = 16;   // (PF_TOK: fewest tokens worth a pass on this path, and the widest token tile of the Q4_0 / Q8_0 kernel)
 constexpr int PF_WTILE_F16 = 128 * 32 * 2 + 128 * 4;            // Q4_0 / Q8_0: the f16 A operand of a 32-element block (128 rows), then one f32 scale per row
-constexpr int PF_KQ_TOK = 64;                                   // K-quant kernels: 64 tokens per tile, two columns of D per token
-constexpr int PF_KQ_YQ_BYTES = PF_KQ_TOK * 32 + PF_KQ_TOK * 8;   // Q6_K weights: 64 x 32 s8, 64 f32 scales, 64 f32 block sums
-constexpr int PF_KQ_YQ_BYTES_F8 = 2 * PF_KQ_TOK * 32 + PF_KQ_TOK * 8;   // Q4_K weights: two e4m3 planes of 64 x 32, scales, block sums
-constexpr int PF_KQ_WTILE = 128 * 32 + 128 * 8;                 // the s8 A operand of a 32-element block, then two f32 scale products per row
+constexpr int PF_KQ_TOK_MAX = 64;                               // K-quant kernels: the widest token tile
+constexpr int PF_KQ_WTILE = 128 * 32 * 2 + 128 * 8;             // the f16 A operand of a 32-element block, then two f32 scale products per row
 constexpr int PF_MAX_K = 14336;   // widest activation row the quantizer kernel holds in registers
 struct PrefillGemm {
     const uint8_t *w = nullptr;       // [n_rows / PF_ROWS][nb] weight tiles (launch_prefill_retile)
@@ -131,6 +129,7 @@ struct PrefillGemm {
     uint64_t       wait_limit_ns = 1000000000ull;
     int            selftest_skip_step = -1;   // failure-path check: the copy warp leaves this step out, so the waits for it run out
 };
+int         device_sms();         // SMs of the current device
 int         prefill_tile_tokens(int type, int64_t n_rows, int T);   // width of the token tiles for this matrix and number of tokens
 size_t      prefill_weight_bytes(int type, int64_t n_rows, int nb);
 size_t      prefill_act_bytes(int T, int nb);
@@ -139,13 +138,16 @@ cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stri
 // part_len > 0: a row lies in K / part_len parts, part_stride floats apart
 // pdl (here and below): launch with the programmatic-stream-serialization attribute; the kernels wait for their predecessor themselves
 cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type, int tile_tok,
-                                 int part_len = 0, int64_t part_stride = 0, bool pdl = false);
+                                 int part_len = 0, int64_t part_stride = 0, bool pdl = false, uint8_t *tap = nullptr);   // tap: Q8_0 blocks of token 0, reference layout
 cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream, bool pdl);   // type 12 = Q4_K, 14 = Q6_K (spyb_prefill_kq.cu)
 cudaError_t launch_prefill_retile_kq(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);
 cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool pdl = false);
 cudaError_t launch_prefill_qkv_post(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,
                                     __half *v_cache, int n_ctx, int64_t seq_stride, cudaStream_t stream, bool pdl = false);
 cudaError_t launch_prefill_silu_mul(const float *upgate, int T, int F, const float *silu_table, float *act, cudaStream_t stream, bool pdl = false);
+
+struct PrefillKeep { const uint4 *src[4] = {}; uint4 *dst[4] = {}; int64_t n4[4] = {}; };   // up to four 16-byte-aligned copies
+cudaError_t launch_prefill_keep(const PrefillKeep &k, cudaStream_t stream);
 
 struct AttnParams {
     int           force_long = 0;     // take the three-kernel path (scratch needed) also at short contexts

@@ -487,7 +487,7 @@ spyb_status ensure_prefill_buffers(spyb_model *m) {
 //   -> norm + quantize -> up|gate GEMM -> up * silu(gate) -> quantize -> down GEMM + residual
 // with the arithmetic of the five fused kernels of run_layers, so that a prompt gives the same bits on either path.
 // (batch: the T tokens are sequences 0 .. T-1 of a batch in lockstep, each with its own cache, all at position d_pos[0])
-spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool batch = false) {
+spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool batch = false, bool tap = false) {
     spyb_backend *be = m->be;
     cudaStream_t s = be->stream;
     const bool pdl = be->config.use_pdl != 0;
@@ -497,13 +497,13 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
     // the quantized activations are laid out for the type of the matrix they meet and for its token tile: quant() makes them for the
     // first matrix of a group, gemm() makes them again when a later matrix of the group wants another form
     struct { const float *x; int part_len; const float *norm_w; int K; int64_t part_stride; int type, tile_tok; } yq_src = {};
-    auto layout_of = [](int type) { return type == SPYB_Q4_K ? 3 : type == SPYB_Q6_K ? 1 : 2; };   // (Q4_0 and Q8_0 share one)
-    auto quant = [&](const float *x, int part_len, int K, const float *norm_w, const PfMat &W, int64_t part_stride) {
+    auto layout_of = [&](const PfMat &W) { return ((W.type == SPYB_Q4_K || W.type == SPYB_Q6_K) ? 1000 : 0) + prefill_tile_tokens(W.type, W.n_rows, T); };
+    auto quant = [&](const float *x, int part_len, int K, const float *norm_w, const PfMat &W, int64_t part_stride, uint8_t *tap_xq = nullptr) {
         yq_src = {x, part_len, norm_w, K, part_stride, W.type, prefill_tile_tokens(W.type, W.n_rows, T)};
-        return launch_prefill_quant(x, part_len, T, K, norm_w, norm_w != nullptr ? m->info.rms_eps : 0.f, m->pf_yq, s, W.type, yq_src.tile_tok, part_len, part_stride, pdl);
+        return launch_prefill_quant(x, part_len, T, K, norm_w, norm_w != nullptr ? m->info.rms_eps : 0.f, m->pf_yq, s, W.type, yq_src.tile_tok, part_len, part_stride, pdl, tap_xq);
     };
     auto gemm = [&](const PfMat &W, int K, float *out, int64_t out_stride, const float *resid) {
-        if (layout_of(W.type) != layout_of(yq_src.type)) {
+        if (layout_of(W) != ((yq_src.type == SPYB_Q4_K || yq_src.type == SPYB_Q6_K) ? 1000 : 0) + yq_src.tile_tok) {
             cudaError_t e = quant(yq_src.x, yq_src.part_len, yq_src.K, yq_src.norm_w, W, yq_src.part_stride);
             if (e != cudaSuccess) { return e; }
             ++*launches;
@@ -531,7 +531,7 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
     float *att_part = m->pf_att + (size_t)rank * T * dl, *act_part = m->pf_act + (size_t)rank * T * fl;   // (tp == 1: the whole buffers)
     float *x_part = m->pf_x + (size_t)rank * T * dp;
     for (Layer &ly : m->layers) {
-        SPYB_CUDA(be, quant(m->pf_x, dp, d, ly.attn_norm, ly.pf_qkv, (int64_t)T * dp));
+        SPYB_CUDA(be, quant(m->pf_x, dp, d, ly.attn_norm, ly.pf_qkv, (int64_t)T * dp, tap && &ly == &m->layers[0] ? m->d_tap : nullptr));
         SPYB_CUDA(be, gemm(ly.pf_qkv, d, m->pf_qkv, 3 * (int64_t)dl, nullptr));
         if (m->kq) {   // one matrix per tensor: Wk and Wv fill the other two thirds of the QKV rows
             SPYB_CUDA(be, gemm(ly.pf_k, d, m->pf_qkv + dl, 3 * (int64_t)dl, nullptr));
@@ -1031,7 +1031,10 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
         m->last_launches = m->eval1_launches;
         return SPYB_SUCCESS;
     }
-    if (m->pf_ok && n_tokens >= SPYB_PREFILL_MIN_TOKENS) {
+    // columns of a mat-vec pass
+    const int tmax = m->kq ? KQ_MAX_COLUMNS : std::min(8, std::min(matvec_max_columns(m->info.d_model / 32), matvec_max_columns(m->info.n_ff / 32)));
+    const bool small = n_tokens < PF_TOK;   // (these leave what the mat-vec passes leave behind for the parity taps)
+    if (m->pf_ok && n_tokens >= (m->info.tp_size == 1 ? SPYB_PREFILL_MIN_TOKENS : PF_TOK) && (!small || m->pf_chunk >= n_tokens)) {
         // a prompt: chunks of pf_chunk tokens through the tensor-core GEMMs; the score rows of every chunk span all
         // positions known to the step, as in the passes below
         if (ensure_prefill_buffers(m) != SPYB_SUCCESS) { return SPYB_FAIL; }
@@ -1057,7 +1060,17 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
                                                     cudaMemcpyDeviceToDevice, be->stream));
                 }
             }
-            if (run_prefill_layers(m, T, &launches) != SPYB_SUCCESS) { return SPYB_FAIL; }
+            if (run_prefill_layers(m, T, &launches, false, small) != SPYB_SUCCESS) { return SPYB_FAIL; }
+            if (small) {   // the last mat-vec pass would have held tokens l0 .. n_tokens - 1
+                const int l0 = (n_tokens - 1) / tmax * tmax, n = n_tokens - l0, ff = m->info.n_ff;
+                PrefillKeep k;
+                auto seg = [&](int s, const void *src, void *dst, size_t bytes) { k.src[s] = static_cast<const uint4 *>(src); k.dst[s] = static_cast<uint4 *>(dst); k.n4[s] = (int64_t)(bytes / 16); };
+                seg(0, m->pf_q + (size_t)l0 * m->dl, m->q, (size_t)n * m->dl * 2);
+                seg(1, m->pf_att + (size_t)l0 * dmod, m->att, (size_t)n * dmod * 4);
+                seg(2, m->pf_x + (size_t)l0 * dmod, m->x, (size_t)n * dmod * 4);
+                seg(3, m->pf_act + (size_t)l0 * ff, m->act, (size_t)n * ff * 4);
+                SPYB_CUDA(be, launch_prefill_keep(k, be->stream)); ++launches;
+            }
             if (t0 + T == n_tokens) {
                 const float *last_row = m->pf_x + (int64_t)(T - 1) * dmod;
                 if (tp > 1) {   // the last token's row from its parts
@@ -1081,7 +1094,6 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
         return SPYB_SUCCESS;
     }
     SPYB_CUDA(be, cudaEventRecord(m->ev0, be->stream));
-    const int tmax = m->kq ? KQ_MAX_COLUMNS : std::min(8, std::min(matvec_max_columns(m->info.d_model / 32), matvec_max_columns(m->info.n_ff / 32)));
     for (int t0 = 0; t0 < n_tokens; t0 += tmax) {
         const int T = std::min(tmax, n_tokens - t0);
         SPYB_CUDA(be, cudaStreamSynchronize(be->stream));   // pinned staging words are reused per pass

@@ -323,14 +323,13 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
 // activations of T tokens -> compact Q8_0 blocks grouped by (tile of tile_tok tokens, block). One CTA per token; RMSNorm and the
 // quantizer as in the mat-vec prologue (NormRMS, backend/host/operator/non-linear.cpp:194-223: groups of four squares formed in
 // parallel, the running sum on one thread; Quantizator<FP32,Q8_0>, simd/vec_convert.h:178-261).
-// FORM 0 (Q4_0 / Q8_0 weights): the values as f16, then the f32 scales. FORM 1 (Q6_K): s8 values, scales, the blocks' integer sums as
-// floats. FORM 2 (Q4_K): two planes of e4m3 values (the multiple of 16 and the rest), scales, sums.
-template <bool NORM, int FORM>
+// KQ false (Q4_0 / Q8_0 weights): [token][32 values as f16], the scales. KQ true: the f16 B operand itself (16 bytes of eight values of a token at
+// (value / 8) * 16 TOKT + 16 token), the scales, the blocks' integer sums as floats.
+template <bool NORM, bool KQ>
 __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const float *x, int64_t x_stride, int K, const float *norm_w, float eps, uint8_t *yq,
-                                                                         int TOKT, int part_len, int64_t part_stride) {
-    constexpr bool YSUM = FORM != 0;
-    const int SCALES = (FORM == 1 ? 1 : 2) * TOKT * 32;   // offset of the scales inside a block's record
-    const int YQB = SCALES + TOKT * 4 * (YSUM ? 2 : 1);
+                                                                         int TOKT, int part_len, int64_t part_stride, uint8_t *tap) {
+    const int SCALES = TOKT * 64;                         // offset of the scales inside a block's record
+    const int YQB = SCALES + TOKT * (KQ ? 8 : 4);
     extern __shared__ __align__(16) float v3[];
     __shared__ float scale_s;
     const int tid = threadIdx.x, token = blockIdx.x;
@@ -392,26 +391,24 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
             const int gi = tid + k * PF_QUANT_THREADS;
             uint16_t dh; int sum;
             const uint32_t q = quantize_q8_lane4(xv[k], dh, sum);
-            if (YSUM) {   // the block's sum over its eight lanes
+            if (KQ) {   // the block's sum over its eight lanes
                 sum += __shfl_xor_sync(0xffffffffu, sum, 1); sum += __shfl_xor_sync(0xffffffffu, sum, 2); sum += __shfl_xor_sync(0xffffffffu, sum, 4);
             }
             if (gi < n4) {
                 const int b = gi >> 3, w = gi & 7;
                 uint8_t *blk = tile + (int64_t)b * YQB;
-                if (FORM == 0) {
-                    auto h = [&](int i) { return (uint32_t)__half_as_ushort(__int2half_rn((int)(int8_t)(q >> (8 * i)))); };
-                    reinterpret_cast<uint2 *>(blk + tt * 64)[w] = make_uint2(h(0) | (h(1) << 16), h(2) | (h(3) << 16));
-                } else if (FORM == 2) {
-                    uint32_t hi, lo;
-                    e4m3_split4(q, hi, lo);
-                    reinterpret_cast<uint32_t *>(blk + tt * 32)[w] = hi;
-                    reinterpret_cast<uint32_t *>(blk + TOKT * 32 + tt * 32)[w] = lo;
-                } else {
-                    reinterpret_cast<uint32_t *>(blk + tt * 32)[w] = q;
+                auto h = [&](int i) { return (uint32_t)__half_as_ushort(__int2half_rn((int)(int8_t)(q >> (8 * i)))); };
+                const uint2 v = make_uint2(h(0) | (h(1) << 16), h(2) | (h(3) << 16));
+                if (tap != nullptr && token == 0) {   // reference-layout blocks of token 0 (34-byte records: only 2-byte alignment holds)
+                    uint16_t *o = reinterpret_cast<uint16_t *>(tap + (int64_t)b * 34);
+                    o[1 + 2 * w] = (uint16_t)q; o[2 + 2 * w] = (uint16_t)(q >> 16);
+                    if (w == 0) { o[0] = dh; }
                 }
+                if (KQ) { *reinterpret_cast<uint2 *>(blk + (w >> 1) * 16 * TOKT + tt * 16 + (w & 1) * 8) = v; }
+                else    { reinterpret_cast<uint2 *>(blk + tt * 64)[w] = v; }
                 if (w == 0) {
                     reinterpret_cast<float *>(blk + SCALES)[tt] = h2f(dh);
-                    if (YSUM) { reinterpret_cast<float *>(blk + SCALES + TOKT * 4)[tt] = (float)sum; }
+                    if (KQ) { reinterpret_cast<float *>(blk + SCALES + TOKT * 4)[tt] = (float)sum; }
                 }
             }
         }
@@ -492,17 +489,6 @@ __global__ void prefill_silu_mul_kernel(const float *upgate, int T, int F, const
     act[i] = __fmul_rn(up, silu_table[f2h(gate)]);
 }
 
-int device_sms() {
-    static int sms[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { return 148; }
-    if (sms[dev] == 0) {
-        int n = 0;
-        sms[dev] = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
-    }
-    return sms[dev];
-}
-
 template <int TT>
 cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     const size_t smem = PfGeom<TT>::SMEM;
@@ -514,13 +500,27 @@ cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
 
 }  // namespace
 
+int device_sms() {
+    static int sms[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { return 148; }
+    if (sms[dev] == 0) {
+        int n = 0;
+        sms[dev] = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }
+    return sms[dev];
+}
+
 // Tiles of 16 or of 8 tokens. A tile takes nb TT / 32 steps and the CTAs walk their tiles in rounds, so the width whose busiest CTA has
 // fewer steps to do wins; a step of the narrow tiles costs 1.4 of one of the wide ones (eight MMAs and twice the weight bytes; measured
 // 1.2 to 1.5 on 4096 to 27648 rows). 4096 rows x 32 tokens: 8 wide (20 us against 30); 27648 rows x 32 tokens: 16 wide (91 against 142).
 int prefill_tile_tokens(int type, int64_t n_rows, int T) {
-    if (type == 12 || type == 14) { return PF_KQ_TOK; }
     const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, sms = device_sms();
     auto rounds = [&](int tt) { return (row_tiles * ((T + tt - 1) / tt) + sms - 1) / sms; };
+    if (type == 12 || type == 14) {   // K-quants: a tile of 16, 32, 64 tokens costs 1 : 1.35 : 2.3 (measured: the narrow ones are mostly weights)
+        const double c16 = (double)rounds(16), c32 = 1.35 * (double)rounds(32), c64 = 2.3 * (double)rounds(64);
+        return c16 <= c32 && c16 <= c64 ? 16 : c32 <= c64 ? 32 : 64;
+    }
     return 8.0 * 1.4 * (double)rounds(8) < 16.0 * (double)rounds(16) ? 8 : 16;
 }
 
@@ -530,7 +530,7 @@ size_t prefill_weight_bytes(int type, int64_t n_rows, int nb) {
 }
 size_t prefill_act_bytes(int T, int nb) {   // (the largest of the layouts)
     return std::max((size_t)((T + PF_TOK - 1) / PF_TOK) * PF_TOK * nb * 68,
-                    (size_t)((T + PF_KQ_TOK - 1) / PF_KQ_TOK) * nb * std::max(PF_KQ_YQ_BYTES, PF_KQ_YQ_BYTES_F8));
+                    (size_t)((T + PF_KQ_TOK_MAX - 1) / PF_KQ_TOK_MAX) * PF_KQ_TOK_MAX * nb * 72);
 }
 
 cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream) {
@@ -545,16 +545,15 @@ cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stri
 }
 
 cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type,
-                                 int tile_tok, int part_len, int64_t part_stride, bool pdl) {
+                                 int tile_tok, int part_len, int64_t part_stride, bool pdl, uint8_t *tap) {
     if (weight_type != 2 && weight_type != 8 && weight_type != 12 && weight_type != 14) { return cudaErrorInvalidValue; }
     if (part_len <= 0) { part_len = K; part_stride = 0; }
     if ((part_len & 3) || (part_stride & 3) || K % part_len != 0) { return cudaErrorInvalidValue; }
     if (T < 1 || tile_tok < 1 || K < 32 || (K & 31) || K > PF_MAX_K || (x_stride & 3) || ((uintptr_t)x & 15)) { return cudaErrorInvalidValue; }
     const size_t smem = norm_w != nullptr ? (size_t)K : 0;   // K / 4 floats
-    auto *kernel = weight_type == 12 ? (norm_w ? prefill_quant_kernel<true, 2> : prefill_quant_kernel<false, 2>)
-                 : weight_type == 14 ? (norm_w ? prefill_quant_kernel<true, 1> : prefill_quant_kernel<false, 1>)
-                                     : (norm_w ? prefill_quant_kernel<true, 0> : prefill_quant_kernel<false, 0>);
-    return launch_maybe_pdl(kernel, dim3((unsigned)T), PF_QUANT_THREADS, smem, stream, pdl, x, x_stride, K, norm_w, eps, yq, tile_tok, part_len, part_stride);
+    const bool kq = weight_type == 12 || weight_type == 14;
+    auto *kernel = kq ? (norm_w ? prefill_quant_kernel<true, true> : prefill_quant_kernel<false, true>) : (norm_w ? prefill_quant_kernel<true, false> : prefill_quant_kernel<false, false>);
+    return launch_maybe_pdl(kernel, dim3((unsigned)T), PF_QUANT_THREADS, smem, stream, pdl, x, x_stride, K, norm_w, eps, yq, tile_tok, part_len, part_stride, tap);
 }
 
 cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
@@ -571,6 +570,17 @@ cudaError_t launch_prefill_qkv_post(const float *qkv, int T, int dl, int hd, con
                                     __half *v_cache, int n_ctx, int64_t seq_stride, cudaStream_t stream, bool pdl) {
     const int64_t n = 3 * (int64_t)dl / 2 * T;
     return launch_maybe_pdl(prefill_qkv_post_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, pdl, qkv, T, dl, hd, pos_base, rope, q_out, k_cache, v_cache, n_ctx, seq_stride);
+}
+
+// the last pass's columns into the buffers the mat-vec passes leave them in
+__global__ void prefill_keep_kernel(const PrefillKeep k) {
+    for (int s = 0; s < 4; ++s) {
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k.n4[s]; i += (int64_t)gridDim.x * blockDim.x) { k.dst[s][i] = k.src[s][i]; }
+    }
+}
+cudaError_t launch_prefill_keep(const PrefillKeep &k, cudaStream_t stream) {
+    prefill_keep_kernel<<<64, 256, 0, stream>>>(k);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_prefill_silu_mul(const float *upgate, int T, int F, const float *silu_table, float *act, cudaStream_t stream, bool pdl) {

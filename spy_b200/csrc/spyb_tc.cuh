@@ -9,16 +9,7 @@ namespace spyb {
 namespace {
 
 constexpr int PF_M           = PF_ROWS;            // weight rows per CTA = M of the MMA
-constexpr int PF_NCOL        = 128;                // columns of D per block step = N of the MMA
-constexpr int PF_TILE        = PF_M * 32;          // bytes of one s8 operand tile
-constexpr int PF_EPI_WARPS   = 8;                  // epilogue warps: (row quadrant 0..3) x (half of the columns); 12 warps in all leave them 168 registers
-constexpr int PF_BATCH       = 4;                  // blocks per batch: the unit of the copies, of the expansion and of stage reuse
-constexpr int PF_RING        = 4;                  // batches in the shared-memory rings
-constexpr int PF_MMA_WARPS   = 2;                  // warps whose first thread issues the MMAs of every PF_MMA_WARPS-th block
-constexpr int PF_THREADS     = (PF_EPI_WARPS + 2 + PF_MMA_WARPS) * 32;   // + the copy warp and the expander warp
 constexpr int PF_GEMM_EPI_WARPS = 16, PF_GEMM_THREADS = 640;   // the Q4_0 / Q8_0 kernel: sixteen epilogue warps and four feeder warps, 96 registers each
-constexpr int PF_DBUF        = 4;                  // accumulator buffers in tensor memory, PF_NCOL columns each (512 columns = all of it)
-
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -49,29 +40,6 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// shared-memory operand descriptor: K-major, no swizzle; element (row r, byte k) of the tile lies at
-// (r / 8) * 256 + (k / 16) * 128 + (r % 8) * 16 + k % 16: leading (K-chunk) offset 128, stride (8-row group) offset 256
-__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(256u >> 4) << 32) | (1ull << 46);
-}
-// instruction descriptor: D s32, A and B s8 K-major, N = 128, M = 128
-constexpr uint32_t PF_IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(PF_NCOL >> 3) << 17) | ((uint32_t)(PF_M >> 4) << 24);
-
-__device__ __forceinline__ void mma_s8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc) {
-    const uint32_t zero = 0, accumulate = 1;   // D += A B^T: D holds the offset pattern
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(PF_IDESC), "r"(accumulate), "r"(zero) : "memory");
-}
-// e4m3 operands (kind::f8f6f4), f32 accumulators: D (+)= A B^T. Small integers are exact in e4m3 (|v| <= 16, and multiples of 16
-// up to 128), their products and the sums of a block's few products are exact in f32, so D holds (float)(integer sum) itself.
-constexpr uint32_t PF_IDESC_F8 = (1u << 4) | ((uint32_t)(PF_NCOL >> 3) << 17) | ((uint32_t)(PF_M >> 4) << 24);
-__device__ __forceinline__ void mma_f8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
-    const uint32_t zero = 0;
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(PF_IDESC_F8), "r"(accumulate), "r"(zero) : "memory");
-}
 // f16 operands, f32 accumulators, 128 x N x 16: D (+)= A B^T. 8-bit integers are exact in f16, their products and the sums of a
 // block's few products are exact in f32
 __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
@@ -102,46 +70,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
                    "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// the same 32-bit word into 32 consecutive columns of this thread's lane
-__device__ __forceinline__ void tmem_st32_same(uint32_t taddr, uint32_t v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-                 "{%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(v) : "memory");
-}
-// 16 consecutive columns of this thread's lane from 16 registers (callers keep a register set that holds the offset
-// pattern alive across the loop, so that no copies are made per store)
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *v) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-                   "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// e4m3 code of the integer v, 0 <= v <= 15 (exact: three mantissa bits cover 8..15), and of a signed value in [-15, 15]
-__host__ __device__ __forceinline__ uint32_t e4m3_of_small(uint32_t v) {
-    if (v == 0) { return 0u; }
-    const int e = v >= 8 ? 3 : v >= 4 ? 2 : v >= 2 ? 1 : 0;
-    return ((uint32_t)(e + 7) << 3) | ((v << (3 - e)) & 7u);
-}
-__host__ __device__ __forceinline__ uint32_t e4m3_of_signed(int v) { return v < 0 ? (0x80u | e4m3_of_small((uint32_t)-v)) : e4m3_of_small((uint32_t)v); }
-// a Q8_0 activation byte y in [-127, 127] as two e4m3 values: y = hi + lo with lo = y mod 16 in [0, 15] and hi = y - lo a
-// multiple of 16 in [-128, 112] (the code of |hi| / 16 with the exponent raised by four)
-__device__ __forceinline__ void e4m3_split4(uint32_t q, uint32_t &hi, uint32_t &lo) {
-    hi = 0u; lo = 0u;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int y = (int)(int8_t)((q >> (8 * i)) & 0xffu);
-        const int yl = y & 15, yh = (y - yl) >> 4;   // yh in [-8, 7]
-        const uint32_t ch = yh == 0 ? 0u : (e4m3_of_signed(yh) + 0x20u);
-        hi |= ch << (8 * i);
-        lo |= e4m3_of_small((uint32_t)yl) << (8 * i);
-    }
-}
 
 // feeder roles (copy, expansion, MMA issue) run ahead of the epilogue: their waits back off instead of competing with the
 // epilogue warps for issue slots

@@ -116,6 +116,32 @@ def test_activation_blocks_of_first_layer(be, oracle, tmp_models):
     m.close()
 
 
+@pytest.mark.parametrize("n", [8, 9, 12, 13, 15])
+def test_short_gemm_prompts_leave_the_last_pass_behind(n, tmp_models):
+    """Prompts of 8 to 15 tokens run as GEMMs but leave the residual stream, attention output, FFN activation, Q and the tapped Q8_0 blocks
+    of the mat-vec passes they replace, and the same logits."""
+    path = str(tmp_models / f"keep{n}.gguf")
+    gguf_io.make_llama_gguf(path, gguf_io.LlamaConfig(weight_std=0.05), seed=5)
+    prompt = np.arange(3, 3 + n)
+    got = []
+    for env in ("1", "0"):
+        os.environ["SPYB_PREFILL"] = env
+        b = B.B200Backend(0)
+        m = B.LlamaModel(b, path, n_ctx=64)
+        logits = m.eval(prompt, 0)
+        cols = (n - 1) % 4 + 1
+        bufs = []
+        for which, (width, dt) in enumerate([(256, np.uint16), (256, np.float32), (256, np.float32), (512, np.float32)]):
+            a = np.zeros((cols, width), dtype=dt)
+            b._check(b._l.spyb_model_read_activation(m.h, which, a.ctypes.data, a.nbytes))
+            bufs.append(a)
+        got.append([logits, m.tap_xq()] + bufs)
+        m.close(); b.close()
+    del os.environ["SPYB_PREFILL"]
+    for g, w in zip(*got):
+        assert g.tobytes() == w.tobytes()
+
+
 def test_prompt_longer_than_one_pass_and_context_edge(be, oracle, tmp_models):
     """21 prompt tokens (three passes of <= 8 columns), decoding until the context is exactly full."""
     cfg = gguf_io.LlamaConfig(weight_std=0.05)

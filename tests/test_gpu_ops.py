@@ -161,6 +161,19 @@ def test_prefill_matmul_walks_tiles_of_both_widths(be, oracle, qt, n, k, t):
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
+@pytest.mark.parametrize("n,k,t", [(19000, 256, 16), (2564, 768, 250), (1284, 512, 1000), (516, 2304, 31), (132, 256, 48), (640, 4096, 9)])
+def test_prefill_matmul_k_quants_walk_tiles_of_all_widths(be, oracle, qt, n, k, t):
+    """Token tiles of 16, 32 and 64, more tiles than SMs, ragged last tiles in both directions, one super-block and sixteen."""
+    rng = np.random.default_rng(n + k + t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    got = be.prefill_matmul(qt, w, n, k, x)
+    rows, cols = np.unique(np.r_[0, n - 1, rng.integers(0, n, 60)]), np.unique(np.r_[0, t - 1, rng.integers(0, t, 40)])
+    want = oracle.matmul(qt, np.ascontiguousarray(w[rows]), k, len(rows), x[cols])
+    assert np.array_equal(got[np.ix_(cols, rows)].view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
 @pytest.mark.parametrize("n,k,t,norm", [(128, 256, 1, False), (256, 1024, 70, True), (128, 2048, 64, False), (384, 4096, 129, True), (256, 11008 - 11008 % 256, 33, False)])
 def test_prefill_matmul_k_quants_match_the_restatement(be, oracle, qt, n, k, t, norm):
     """K-quant weights through the tensor-core prompt kernel: 1 to 43 super-blocks, ragged tiles of 64 tokens, with and without
