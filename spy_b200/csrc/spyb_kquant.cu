@@ -59,7 +59,7 @@ __device__ __forceinline__ void kq_prologue(const MatvecParams &p, int nT, uint3
         }
         __syncthreads();
         if ((tid & 31) == 0 && (tid >> 5) < nT) {
-            const float sum  = running_sum_serial(reinterpret_cast<const float *>(rec + (tid >> 5) * col), n4);
+            const float sum  = running_sum_serial(smem_u32(rec + (tid >> 5) * col), n4);
             const float mean = __fdiv_rn(sum, (float)p.A.k);
             scale_s[tid >> 5] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
         }

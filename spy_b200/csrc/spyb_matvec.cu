@@ -155,7 +155,7 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
             wv[k] = (k < npass && g < n4) ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         __syncthreads();
-        const float sum = (tid == 0) ? running_sum_serial(v3, n4) : 0.f;
+        const float sum = (tid == 0) ? running_sum_serial(smem_u32(v3), n4) : 0.f;
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
             scales[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));

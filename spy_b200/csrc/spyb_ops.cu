@@ -609,6 +609,225 @@ __global__ void __launch_bounds__(ATT_PV_WARPS * WARP) attn_pv_kernel(const Attn
     tp_publish(p.tp, p.T);
 }
 
+// ---------------------------------------------------------------------------------------------
+// A step over a long context in one kernel: ATL_C CTAs (a cluster) take a head. Each CTA scores its quarter of the positions, the quarters'
+// exponentials meet in every CTA's shared memory, each CTA forms the softmax sum (its order allows no split) and then its quarter of the
+// head's output elements over all positions. Same arithmetic as attention_kernel. HBM-bound: K and V^T are read once. One warp copies
+// both through one ring of stages (32 K rows of 256 bytes, or 512 positions of eight V^T rows) without regard to the phases: while the
+// softmax is formed, V^T fills the ring. (cp.async, 512 bytes an instruction: bulk copies of a row each cost the warp 50 cycles, 54 us in all.) A stage is filled for one warp: no CTA-wide waits on the way.
+// 32 heads over 4000 positions, three kernels (scores, softmax, PV) before: 41 us, now 28; the reads take 10.3.
+constexpr int ATL_C = 4, ATL_WARPS = 8, ATL_THREADS = (ATL_WARPS + 1) * WARP;
+constexpr int ATL_KPITCH = 272, ATL_VCH = 512, ATL_VROWS = 8, ATL_VPITCH = 2 * ATL_VCH + 64, ATL_STAGE = 32 * ATL_KPITCH;   // pitches without bank conflicts
+static_assert(ATL_VROWS * ATL_VPITCH == ATL_STAGE && ATL_C * 4 * ATL_VROWS == ATT_HD, "both kinds of stages fill the slot; four warps take a CTA's elements");
+constexpr int ATL_MAX_STAGES = 22, ATL_MIN_STAGES = 6;
+struct AtlSmem { size_t ex, gs, rs, red, bars, ring; };
+__host__ __device__ static inline AtlSmem atl_smem(int n_ctx) {   // offsets in bytes; q lies in front
+    const size_t n32 = ((size_t)n_ctx + 31) & ~(size_t)31;
+    AtlSmem L;
+    L.ex = ATT_HD * 4; L.gs = L.ex + n32 * 4; L.rs = L.gs + n32; L.red = L.rs + rs_scratch_words(4) * 4; L.bars = L.red + (ATL_C * ATL_WARPS + 4) * 4;
+    L.ring = (L.bars + (2 * ATL_MAX_STAGES + 2) * 8 + 127) / 128 * 128;
+    return L;
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(__cvta_generic_to_global(src)) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ void cluster_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// waits for the cluster's arrivals (phase 0); as mbar_wait_lean, limit_ns becomes zero when they do not come
+__device__ __forceinline__ void cluster_wait(uint32_t bar, uint64_t &limit_ns) {
+    const uint64_t t0 = global_timer_ns();
+    for (;;) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
+        if (ok) { return; }
+        if (global_timer_ns() - t0 >= limit_ns) { limit_ns = 0; return; }
+    }
+}
+__device__ __forceinline__ void atl_wait(uint32_t bar, uint32_t parity, uint64_t &limit_ns) {
+    if (mbar_try_wait(bar, parity)) { return; }
+    if (limit_ns == 0 || !mbar_wait_prompt(bar, parity, limit_ns)) { limit_ns = 0; }
+}
+
+__global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const AttnParams p, const int NS) {
+    extern __shared__ __align__(128) uint8_t atl_raw[];
+    const AtlSmem L = atl_smem(p.n_ctx);
+    float *qf = reinterpret_cast<float *>(atl_raw), *ex = reinterpret_cast<float *>(atl_raw + L.ex), *gs = reinterpret_cast<float *>(atl_raw + L.gs);
+    float *rs = reinterpret_cast<float *>(atl_raw + L.rs), *red = reinterpret_cast<float *>(atl_raw + L.red);
+    const uint32_t ring_s = smem_u32(atl_raw + L.ring), full_s = smem_u32(atl_raw + L.bars), empty_s = full_s + 8 * ATL_MAX_STAGES;
+    const uint32_t max_s = empty_s + 8 * ATL_MAX_STAGES, exp_s = max_s + 8;
+    const int h = blockIdx.x / ATL_C, rank = blockIdx.x % ATL_C, t = blockIdx.y;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    if (tid == 0) {
+        for (int i = 0; i < NS; ++i) { mbar_init(full_s + 8 * i, WARP); mbar_init(empty_s + 8 * i, 1); }
+        mbar_init(max_s, ATL_C * ATL_WARPS); mbar_init(exp_s, ATL_C * ATL_WARPS);
+        mbar_init_fence();
+    }
+    cluster_sync();   // every CTA of the cluster is there, its barriers too
+    pdl_wait();
+    const bool batch = p.seq_stride != 0;
+    const int n_vis = p.pos_base[0] + (batch ? 0 : t) + 1;
+    const int n_tot = batch ? n_vis : (p.pos_base[1] > 0) ? p.pos_base[1] : p.pos_base[0] + p.T;
+    const int slice = ((n_vis + ATL_C * 32 - 1) / (ATL_C * 32)) * 32, start = rank * slice;
+    const int cnt = max(0, min(slice, n_vis - start)), nK = (cnt + 31) >> 5, nC = (n_vis + ATL_VCH - 1) / ATL_VCH;
+    uint64_t limit = WAIT_LIMIT_NS;
+    if (warp == ATL_WARPS) {
+        const __half *K = p.k_cache + (batch ? (int64_t)t * p.seq_stride : 0) + (int64_t)start * p.dl + (int64_t)h * ATT_HD;
+        const __half *V = p.v_cache + (batch ? (int64_t)t * p.seq_stride : 0) + ((int64_t)h * ATT_HD + rank * (ATT_HD / ATL_C)) * p.n_ctx;
+        const int total = nK + 4 * nC;
+        int slot = 0; uint32_t phase = 1;   // (the first round finds every slot empty)
+        int g = 0;
+        for (; g < total && limit != 0; ++g) {
+            if (g >= NS) { atl_wait(empty_s + 8 * slot, phase, limit); }
+            if (!__all_sync(0xffffffffu, limit != 0)) { break; }
+            const uint32_t bar = full_s + 8 * slot, dst = ring_s + slot * ATL_STAGE;
+            if (g < nK) {
+                const __half *row = K + (int64_t)(32 * g + (lane >> 4)) * p.dl + (lane & 15) * 8;
+                const int rows = cnt - 32 * g - (lane >> 4);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) { if (2 * i < rows) { cp_async16(dst + (2 * i + (lane >> 4)) * ATL_KPITCH + (lane & 15) * 16, row + (int64_t)2 * i * p.dl); } }
+            } else {
+                const int c = (g - nK) >> 2, w = (g - nK) & 3;
+                const __half *row = V + (int64_t)(w * ATL_VROWS) * p.n_ctx + c * ATL_VCH + lane * 8;
+                const int left = n_vis - c * ATL_VCH - lane * 8;   // (a whole piece lies inside the row: n_ctx is a multiple of 8)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) { if ((i & 1) * 256 < left) { cp_async16(dst + (i >> 1) * ATL_VPITCH + (i & 1) * 512 + lane * 16, row + (int64_t)(i >> 1) * p.n_ctx + (i & 1) * 256); } }
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+            if (++slot == NS) { slot = 0; phase ^= 1u; }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");   // no copy is in flight when the CTA ends, also when its readers gave up
+    } else {
+        if (tid < ATT_HD) { qf[tid] = __half2float(p.q[(int64_t)t * p.dl + (int64_t)h * ATT_HD + tid]); }
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        // scores of this CTA's positions, a tile of 32 per warp, a position per lane
+        float m = -CUDART_INF_F;
+        for (int k = warp; k < nK; k += ATL_WARPS) {
+            const int slot = k % NS;
+            atl_wait(full_s + 8 * slot, (uint32_t)(k / NS) & 1u, limit);
+            uint4 kv[16];
+            const uint32_t src = ring_s + slot * ATL_STAGE + lane * ATL_KPITCH;
+#pragma unroll
+            for (int a = 0; a < 16; ++a) { kv[a] = lds128(src + 16 * a); }
+            const float s = score_dot(kv, reinterpret_cast<const float4 *>(qf));
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(empty_s + 8 * slot); }
+            const int  j = 32 * k + lane;
+            const float v = j < cnt ? __fmul_rn(__fadd_rn(s, 0.0f), p.scale) : -CUDART_INF_F;
+            ex[start + j] = v;
+            m = fmaxf(m, v);
+        }
+        m = warp_max(m);
+        if (lane < ATL_C) {
+            cluster_store(cluster_map(smem_u32(red + rank * ATL_WARPS + warp), lane), m);
+            cluster_arrive(cluster_map(max_s, lane));
+        }
+        cluster_wait(max_s, limit);
+        m = warp_max(red[lane]);
+        // exponentials and their sums of four, to all CTAs of the cluster
+        for (int k0 = warp; k0 < nK; k0 += 4 * ATL_WARPS) {
+            float e[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int j = 32 * (k0 + i * ATL_WARPS) + lane;
+                e[i] = j < cnt ? p.exp_table[f2h(__fsub_rn(ex[start + j], m))] : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int k = k0 + i * ATL_WARPS, j = 32 * k + lane;
+                if (k < nK) {   // uniform in the warp
+                    const float two = __fadd_rn(e[i], __shfl_xor_sync(0xffffffffu, e[i], 1)), four = __fadd_rn(two, __shfl_xor_sync(0xffffffffu, two, 2));
+                    const uint32_t to = smem_u32(ex + start + j), to4 = smem_u32(gs + ((start + j) >> 2));
+#pragma unroll
+                    for (int r = 0; r < ATL_C; ++r) {
+                        cluster_store(cluster_map(to, r), e[i]);
+                        if ((lane & 3) == 0) { cluster_store(cluster_map(to4, r), four); }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (lane < ATL_C) { cluster_arrive(cluster_map(exp_s, lane)); }
+        cluster_wait(exp_s, limit);
+        // std::reduce: groups of four, in order; masked positions are exact zeros that decide which elements form a group
+        const int n_sum = min(n_tot, (n_vis + 3) & ~3), ng = min(n_tot >> 2, (n_vis + 3) >> 2);
+        if (warp < RS_THREADS / WARP) {
+            float sum = running_sum_wide(smem_u32(gs), ng, smem_u32(rs), rs_scratch_words(4), tid, 1);
+            if (tid == 0) {
+                for (int j = ng << 2; j < n_sum; ++j) { sum = __fadd_rn(sum, ex[j]); }
+                red[ATL_C * ATL_WARPS] = __fdiv_rn(1.0f, sum);
+            }
+        }
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        const float inv = red[ATL_C * ATL_WARPS];
+        auto prob = [inv](float e) { return __half2float(__float2half_rn(__fmul_rn(e, inv))); };   // as the PV MatMul rounds its f32 operand
+        for (int g = tid; g < (n_vis + 3) >> 2; g += ATL_WARPS * WARP) {
+            float4 *e = reinterpret_cast<float4 *>(ex) + g;
+            *e = make_float4(prob(e->x), prob(e->y), prob(e->z), prob(e->w));
+        }
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        // PV: accumulators 8 (lane % 4) .. + 7 of row lane / 4 of the warp's eight (position j of a 32-step belongs to accumulator j % 32)
+        if (warp < 4) {
+            const int n_main = ((n_tot - 1) / 32) * 32, n_full = min(n_main, n_vis) >> 5;
+            const int q = lane & 3;
+            const uint32_t ex_s = smem_u32(ex);
+            float acc[8], tail = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { acc[i] = 0.f; }
+            auto step = [&](uint32_t v_s, int pos, int valid) {
+                const uint4  v = lds128(v_s);
+                const float4 pa = lds128f(ex_s + 4 * pos), pb = lds128f(ex_s + 4 * pos + 16);
+                float f[8]; unpack8(v, f);
+                const float pr[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { if (i < valid) { acc[i] = fmaf(f[i], pr[i], acc[i]); } }
+            };
+            for (int c = 0; c < nC; ++c) {
+                const int g = nK + 4 * c + warp, slot = g % NS;
+                atl_wait(full_s + 8 * slot, (uint32_t)(g / NS) & 1u, limit);
+                const uint32_t row = ring_s + slot * ATL_STAGE + (lane >> 2) * ATL_VPITCH;
+                const int p0 = c * ATL_VCH, steps = min(ATL_VCH / 32, n_full - c * (ATL_VCH / 32));
+#pragma unroll 4
+                for (int s = 0; s < steps; ++s) { step(row + s * 64 + q * 16, p0 + s * 32 + q * 8, 8); }
+                const int part = n_full * 32;   // a step that the causal limit cuts (several tokens in a pass)
+                if (part >= p0 && part < p0 + ATL_VCH && part < n_main && part < n_vis) { step(row + (part - p0) * 2 + q * 16, part + q * 8, n_vis - part - q * 8); }
+                if (n_main >= p0 && n_main < p0 + ATL_VCH) {   // positions n_main .. : scalar chain (at most 32)
+                    const int n = n_vis - n_main;
+                    for (int i0 = 0; i0 < n; i0 += 8) {
+                        float f[8]; unpack8(lds128(row + (n_main - p0 + i0) * 2), f);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) { if (i0 + i < n) { tail = fmaf(f[i], ex[n_main + i0 + i], tail); } }
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) { mbar_arrive(empty_s + 8 * slot); }
+            }
+            float u[4];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {   // FP16::block_reduce: (s0 + s2) + (s1 + s3), then elements e and e + 4, then the two pair steps
+                acc[i] = __fadd_rn(acc[i], __shfl_xor_sync(0xffffffffu, acc[i], 2));
+                acc[i] = __fadd_rn(acc[i], __shfl_xor_sync(0xffffffffu, acc[i], 1));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { u[i] = __fadd_rn(acc[i], acc[i + 4]); }
+            const float simd = __fadd_rn(__fadd_rn(u[0], u[1]), __fadd_rn(u[2], u[3]));
+            if (q == 0) {
+                p.out[(int64_t)t * (p.out_stride ? p.out_stride : p.dl) + (int64_t)h * ATT_HD + rank * (ATT_HD / ATL_C) + warp * ATL_VROWS + (lane >> 2)] = __fadd_rn(tail, simd);
+            }
+        }
+    }
+    if (limit == 0 && p.error_flag != nullptr) { atomicExch(p.error_flag, 1); }   // a copy or a CTA of the cluster did not arrive
+    cluster_sync();   // no CTA ends while another may still write into its shared memory
+}
+
 // PV for a prompt: a CTA takes ATT_PVT_ELEMS output elements of a head for ATT_TT consecutive tokens. The 32 accumulators of an output
 // (position j of a 32-step belongs to accumulator j % 32) lie in the registers of eight lanes, four each, so that a lane reads four
 // neighbouring positions at once (64 bits of V^T, 128 bits of a token's probabilities); a lane takes two output elements, a warp eight,
@@ -765,6 +984,37 @@ static cudaError_t launch_with_pdl(const void *kernel, dim3 grid, dim3 block, si
     return cudaLaunchKernelExC(&lc, kernel, args);
 }
 
+// the cluster kernel: single steps and batches, whole 16-byte pieces of the cache rows, at least ATL_MIN_STAGES stages beside the exponentials
+// (contexts up to some 36000 positions). One CTA per SM with a deep ring while all fit so, else two.
+static int atl_stages(const AttnParams &p, const LaunchCfg &cfg) {
+    const size_t budget = (int64_t)ATL_C * p.n_head * p.T <= cfg.num_sms ? 224 * 1024 : 112 * 1024, fixed = atl_smem(p.n_ctx).ring;
+    auto stages = [&](size_t b) { return b <= fixed ? 0 : (int)std::min<size_t>(ATL_MAX_STAGES, (b - fixed) / ATL_STAGE); };
+    const int ns = stages(budget);
+    return ns >= ATL_MIN_STAGES ? ns : stages(224 * 1024);
+}
+static bool atl_fits(const AttnParams &p, const LaunchCfg &cfg) {
+    return (p.T < ATT_TT || p.seq_stride != 0) && p.tp.counter == nullptr && (p.n_ctx & 7) == 0 && (p.seq_stride & 7) == 0 &&
+           (((uintptr_t)p.k_cache | (uintptr_t)p.v_cache) & 15) == 0 && atl_stages(p, cfg) >= ATL_MIN_STAGES;
+}
+static cudaError_t launch_attn_cluster(const AttnParams &p, const LaunchCfg &cfg) {
+    int ns = atl_stages(p, cfg);
+    const size_t smem = atl_smem(p.n_ctx).ring + (size_t)ns * ATL_STAGE;
+    cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(attn_cluster_kernel), smem);
+    if (err != cudaSuccess) { return err; }
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)(ATL_C * p.n_head), (unsigned)p.T); lc.blockDim = dim3(ATL_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ATL_C; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr; lc.numAttrs = cfg.pdl ? 2 : 1;
+    AttnParams q = p;
+    if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
+    void *args[] = {&q, &ns};
+    return cudaLaunchKernelExC(&lc, reinterpret_cast<const void *>(attn_cluster_kernel), args);
+}
+
 size_t attention_scratch_floats(int n_ctx, int n_head, int T) {   // 0: the single-kernel path serves this context length
     if (n_ctx <= ATT_LONG_MIN) { return 0; }
     return (size_t)T * n_head * (((size_t)n_ctx + 3) & ~(size_t)3);
@@ -774,6 +1024,7 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
     if (p.hd != ATT_HD || p.T < 1 || p.n_ctx < 1 || (p.n_ctx & 3) || (p.dl & 7)) { return cudaErrorInvalidValue; }
     const size_t n_pad = ((size_t)p.n_ctx + 3) & ~(size_t)3;
     if ((p.n_ctx > ATT_LONG_MIN || p.force_long) && p.scratch != nullptr) {
+        if (atl_fits(p, cfg)) { return launch_attn_cluster(p, cfg); }
         const bool tiled = p.T >= ATT_TT && p.tp.counter == nullptr && p.seq_stride == 0;   // a prompt: tokens share the K rows and the V^T rows
         cudaError_t err = tiled ? allow_dynamic_smem(reinterpret_cast<const void *>(attn_scores_tiled_kernel), ATT_SC_SMEM) : cudaSuccess;
         if (err != cudaSuccess) { return err; }
@@ -1009,10 +1260,13 @@ __global__ void rmsnorm_kernel(const float *x, float *out, int64_t n, float eps)
         v3[g] = __fadd_rn(fmaf(v.y, v.y, __fmul_rn(v.x, v.x)), fmaf(v.w, v.w, __fmul_rn(v.z, v.z)));
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float sum = running_sum_serial(v3, n4);
-        for (int64_t i = (int64_t)n4 * 4; i < n; ++i) { sum = fmaf(xr[i], xr[i], sum); }
-        scale_s = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)n), eps)));
+    __shared__ __align__(16) float rs_scratch[rs_scratch_words(4)];
+    if (threadIdx.x < RS_THREADS) {
+        float sum = running_sum_wide(smem_u32(v3), n4, smem_u32(rs_scratch), rs_scratch_words(4), threadIdx.x, 1);
+        if (threadIdx.x == 0) {
+            for (int64_t i = (int64_t)n4 * 4; i < n; ++i) { sum = fmaf(xr[i], xr[i], sum); }
+            scale_s = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)n), eps)));
+        }
     }
     __syncthreads();
     const float scale = scale_s;

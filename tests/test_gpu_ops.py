@@ -380,6 +380,20 @@ def test_rmsnorm_mul_add_silu(be, oracle):
     assert np.array_equal(bits(got), bits(oracle.silu(g)))   # table built with the same libm: identical bits
 
 
+@pytest.mark.parametrize("n", [2300, 2304, 2308, 4096, 4100, 5120, 6144, 6148, 8192, 8196])
+def test_rmsnorm_sum_keeps_its_order(be, oracle, n):
+    """The running sum at the edges of its chunk sizes, bit for bit: plain rows, a few outliers, ties at most additions (small integers times a power
+    of two), powers of two, zeros in front, one huge value, values of many magnitudes."""
+    rng = np.random.default_rng(n)
+    z = rng.standard_normal((9, n)).astype(np.float32)
+    x = [z[0], z[1] * np.where(rng.random(n) < 0.02, 30, 0.3), rng.integers(0, 16, n) * 0.125, 2.0 ** rng.integers(-20, 20, n),
+         np.where(np.arange(n) < n // 2, 0, z[2]), np.where(np.arange(n) == n // 3, 1e4, z[3] * 0.01), z[4] * np.exp(3 * z[5]),
+         np.sqrt(1 + 2.0 ** -rng.integers(1, 24, n)), np.zeros(n), z[6] * 1e-18, z[7] * 1e17]
+    x = np.array(x, dtype=np.float32)
+    got = run(be, "NormRMS", [(x, B.FP32, x.shape[::-1], None, B.NODE_DYNAMIC)], x.shape[::-1], eps=1e-5).reshape(x.shape)
+    assert np.array_equal(bits(got), bits(oracle.rmsnorm(x, 1e-5)))
+
+
 def test_silu_golden(be):
     g = np.load(os.path.join(GOLD, "ops_reference.npz"))
     got = run(be, "Silu", [(g["silu_x"], B.FP32, (2048,), None, B.NODE_DYNAMIC)], (2048,))
@@ -589,6 +603,21 @@ def test_attention_of_a_prompt_across_its_tiles(be, oracle, pos0, t, n_total, n_
     vt16 = oracle.quantize_f16(rng.standard_normal(n_ctx * d).astype(np.float32)).reshape(d, n_ctx)
     got = be.attention(q16, k16, vt16, pos0, n_head, hd, n_ctx, n_total)
     want = _attention_oracle(oracle, q16, k16, vt16, pos0, n_head, hd, n_ctx, n_total)
+    assert np.array_equal(bits(got), bits(want))
+
+
+@pytest.mark.parametrize("pos0,t,n_total,n_ctx,n_head", [(0, 1, 1, 1032, 2), (31, 1, 32, 1032, 1), (32, 1, 33, 1032, 1), (127, 1, 128, 1032, 2), (511, 1, 512, 1032, 1),
+                                                         (512, 1, 513, 2048, 2), (1400, 3, 1403, 1408, 2), (4090, 1, 4091, 4096, 2), (2990, 7, 2997, 3000, 6), (700, 2, 740, 4104, 1)])
+def test_attention_of_a_step_over_a_long_context(be, oracle, pos0, t, n_total, n_ctx, n_head):
+    """One to seven tokens in a context above 1024 positions: fewer positions than the CTAs of a head, ends on and beside the 32-position tiles and the
+    512-position stages, rings that wrap, the smaller ring of many CTAs, masked positions behind the last token."""
+    rng = np.random.default_rng(pos0 + t)
+    d = n_head * 128
+    q16 = oracle.quantize_f16(rng.standard_normal(t * d).astype(np.float32)).reshape(t, d)
+    k16 = oracle.quantize_f16(rng.standard_normal(n_ctx * d).astype(np.float32)).reshape(n_ctx, d)
+    vt16 = oracle.quantize_f16(rng.standard_normal(n_ctx * d).astype(np.float32)).reshape(d, n_ctx)
+    got = be.attention(q16, k16, vt16, pos0, n_head, 128, n_ctx, n_total)
+    want = _attention_oracle(oracle, q16, k16, vt16, pos0, n_head, 128, n_ctx, n_total)
     assert np.array_equal(bits(got), bits(want))
 
 
