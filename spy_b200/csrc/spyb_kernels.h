@@ -68,6 +68,7 @@ struct KqSeg {
 };
 
 struct MatvecParams {
+    int   stages_early = 64;          // single column: stages of each warp's ring whose copies are issued ahead of x (set at the launch)
     DevMatrix A;
     DevMatrix B;               // second matrix when pair_mode == 1 (same shape as A)
     int       pair_mode = 0;   // 1: a warp's tile is rows 4u..4u+3 of A together with the same rows of B (FFN up and gate)

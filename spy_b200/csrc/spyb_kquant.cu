@@ -38,6 +38,20 @@ constexpr int KQ_WARPS   = KQ_THREADS / WARP;
 constexpr int KQ_REC = 92;               // words per super-block of activations: 64 values, 8 scales, 16 half-block sums, 4 of padding
 constexpr int KQ_MAX_STAGES = 4;
 
+// four values (group g of the column) -> their word of the column's records, the block's scale and half-block sums; called by whole warps
+__device__ __forceinline__ void kq_quantize(float4 v, int g, int n4, uint32_t *rec) {
+    uint16_t dh; int s;
+    const uint32_t q = quantize_q8_lane4(v, dh, s);
+    s += __shfl_xor_sync(0xffffffffu, s, 1); s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (g < n4) {
+        const int b = g >> 3, w = g & 7;
+        uint32_t *r = rec + (b >> 3) * KQ_REC;
+        r[(b & 7) * 8 + w] = q;
+        if (w == 0) { r[64 + (b & 7)] = __float_as_uint(h2f(dh)); }
+        if ((w & 3) == 0) { r[72 + 2 * (b & 7) + (w >> 2)] = __float_as_uint((float)s); }
+    }
+}
+
 // NormRMS + Mul(weight) (optional) + Quantizator<FP32,Q8_0> of the pass's columns into the activation records (column t lies col words
 // further); the arithmetic is that of the Q4_0 / Q8_0 kernels' prologue (same device functions). The columns' running sums of squares run
 // side by side, one warp each.
@@ -79,17 +93,58 @@ __device__ __forceinline__ void kq_prologue(const MatvecParams &p, int nT, uint3
                 v.x = __fmul_rn(__fmul_rn(v.x, scale), w.x); v.y = __fmul_rn(__fmul_rn(v.y, scale), w.y);
                 v.z = __fmul_rn(__fmul_rn(v.z, scale), w.z); v.w = __fmul_rn(__fmul_rn(v.w, scale), w.w);
             }
-            uint16_t dh; int s;
-            const uint32_t q = quantize_q8_lane4(v, dh, s);
-            s += __shfl_xor_sync(0xffffffffu, s, 1); s += __shfl_xor_sync(0xffffffffu, s, 2);
-            if (valid) {
-                const int b = g >> 3, w = g & 7;
-                uint32_t *r = rec + t * col + (b >> 3) * KQ_REC;
-                r[(b & 7) * 8 + w] = q;
-                if (w == 0) { r[64 + (b & 7)] = __float_as_uint(h2f(dh)); }
-                if ((w & 3) == 0) { r[72 + 2 * (b & 7) + (w >> 2)] = __float_as_uint((float)s); }
-            }
+            kq_quantize(v, g, n4, rec + t * col);
         }
+    }
+}
+
+// One column of at most 512 PG groups of four: every thread keeps its groups of x in registers from the one global read on; x_requested() is
+// called when the reads are on their way. wearly: the norm weights when the kernel read them at its start (PG == KQ_NORM_EARLY).
+constexpr int KQ_NORM_EARLY = 2, KQ_PRO_GROUPS = 6;
+template <int PG, bool NORM, class Requested>
+__device__ __forceinline__ void kq_prologue_1col(const MatvecParams &p, uint32_t *rec, float *scale_s, const float4 *wearly, Requested x_requested) {
+    const int tid = threadIdx.x;
+    const int n4  = (int)(p.A.k >> 2);   // a multiple of 64: whole warps, whole blocks
+    const float4 *x4 = reinterpret_cast<const float4 *>(p.x), *w4 = reinterpret_cast<const float4 *>(p.norm_w);
+    float4 xv[PG], wv[PG];
+#pragma unroll
+    for (int k = 0; k < PG; ++k) {
+        const int g = tid + k * KQ_THREADS;
+        xv[k] = g < n4 ? __ldcg(x4 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (NORM) {
+#pragma unroll
+        for (int k = 0; k < PG; ++k) {
+            const int g = tid + k * KQ_THREADS;
+            if (PG == KQ_NORM_EARLY) { wv[k] = wearly[k]; }
+            else { wv[k] = g < n4 ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f); }
+        }
+    }
+    x_requested();
+    if (NORM) {
+        float *v3 = reinterpret_cast<float *>(rec);   // (n4 = 64 words per super-block: inside the records; the scratch of the sum behind it)
+#pragma unroll
+        for (int k = 0; k < PG; ++k) {
+            const int g = tid + k * KQ_THREADS;
+            if (g < n4) { v3[g] = __fadd_rn(fmaf(xv[k].y, xv[k].y, __fmul_rn(xv[k].x, xv[k].x)), fmaf(xv[k].w, xv[k].w, __fmul_rn(xv[k].z, xv[k].z))); }
+        }
+        __syncthreads();
+        float sum = 0.f;
+        if (PG == 2 && n4 >= RS_MIN && (n4 >> 6) * (KQ_REC - 64) >= rs_scratch_words(2)) {
+            if (tid < RS_THREADS) { sum = running_sum_chunks<2>(smem_u32(v3), n4, smem_u32(v3 + n4), tid, 1); }
+        } else if (tid == 0) { sum = running_sum_serial(smem_u32(v3), n4); }
+        if (tid == 0) { scale_s[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)p.A.k), p.eps))); }
+        __syncthreads();   // also: the partials (aliasing the records) are dead from here on
+        const float scale = scale_s[0];
+#pragma unroll
+        for (int k = 0; k < PG; ++k) {
+            xv[k].x = __fmul_rn(__fmul_rn(xv[k].x, scale), wv[k].x); xv[k].y = __fmul_rn(__fmul_rn(xv[k].y, scale), wv[k].y);
+            xv[k].z = __fmul_rn(__fmul_rn(xv[k].z, scale), wv[k].z); xv[k].w = __fmul_rn(__fmul_rn(xv[k].w, scale), wv[k].w);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < PG; ++k) {
+        if (k * KQ_THREADS < n4) { kq_quantize(xv[k], tid + k * KQ_THREADS, n4, rec); }
     }
 }
 
@@ -224,7 +279,9 @@ __host__ __device__ static inline KqSmem kq_smem_layout(int nsb, int TM, const K
 
 // TM: columns of the pass, rounded up to 1, 2 or 4 (columns past p.T compute on whatever their records hold and are not stored); TYPE: 12 or
 // 14 when every row is of that type, else 0
-template <int TM, int TYPE>
+// PRO: the prologue the kernel is built with - one column of at most 1024 groups of four or a longer one, with and without the norm; else any
+enum { KQP_ANY, KQP_NORM, KQP_PLAIN, KQP_NORM_LONG, KQP_PLAIN_LONG };
+template <int TM, int TYPE, int PRO>
 __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecParams p, const KqPlan pl) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ float scale_s[TM];
@@ -247,6 +304,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
     int64_t lunit = my_first; int lr = 0, lsb = 0, lslot = 0, issued = 0;
     KqRow l0 = {}, l1 = {};
     auto load_unit = [&]() { l0 = kq_unit(p, lunit * pl.np, 0); if (p.pair_mode) { l1 = kq_unit(p, lunit * pl.np, 1); } };
+    const uint64_t policy = l2_evict_first();
     auto issue_next = [&]() {
         const uint32_t bar = bar_s + lslot * 8;
         uint32_t dst = ring_s + (uint32_t)(lslot * pl.stage_bytes);
@@ -254,7 +312,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
         if (!p.pair_mode && (TYPE != 0 ? TYPE : l0.type) == 12) {   // the unit's rows are one contiguous run
             const uint32_t bytes = (uint32_t)left * 144u;
             mbar_expect_tx(bar, bytes);
-            bulk_copy_g2s(dst, l0.w + (size_t)(lr * nsb + lsb) * 144, bytes, bar);
+            bulk_copy_g2s_once(dst, l0.w + (size_t)(lr * nsb + lsb) * 144, bytes, bar, policy);
             lsb += left;
             while (lsb >= nsb) { lsb -= nsb; ++lr; }
         } else {
@@ -269,7 +327,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
                 const bool second = p.pair_mode && (lr & 1);
                 const uint32_t body = (TYPE != 0 ? TYPE : second ? l1.type : l0.type) == 12 ? 144u : 208u;
                 const uint8_t *src = (second ? l1.w : l0.w) + (int64_t)(p.pair_mode ? lr >> 1 : lr) * (second ? l1.pitch : l0.pitch) + (uint32_t)lsb * body;
-                bulk_copy_g2s(dst, src, (uint32_t)m * body, bar);
+                bulk_copy_g2s_once(dst, src, (uint32_t)m * body, bar, policy);
                 dst += (uint32_t)m * (mixed ? 208u : body);
                 left -= m; lsb += m;
                 if (lsb == nsb) { lsb = 0; ++lr; }
@@ -282,17 +340,31 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
 
     // weights never change during a step: the copies may run ahead of the previous kernel's results
     pdl_launch_dependents();
+    float4 wearly[KQ_NORM_EARLY];
+    if (PRO == KQP_NORM) {
+#pragma unroll
+        for (int k = 0; k < KQ_NORM_EARLY; ++k) {
+            const int g = threadIdx.x + k * KQ_THREADS;
+            wearly[k] = g < (int)(p.A.k >> 2) ? reinterpret_cast<const float4 *>(p.norm_w)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
     if (lane == 0 && n_stage > 0) {
         for (int s = 0; s < pl.ns; ++s) { mbar_init(bar_s + s * 8, 1); }
         mbar_init_fence();
         load_unit();
-        for (int s = 0; s < pl.ns && issued < n_stage; ++s) { issue_next(); }
+        for (int s = 0; s < (PRO == KQP_ANY ? pl.ns : min(pl.ns, p.stages_early)) && issued < n_stage; ++s) { issue_next(); }
     }
     __syncwarp();
     pdl_wait();
     tp_wait(p.tp, p.error_flag);
     uint32_t *rec = reinterpret_cast<uint32_t *>(smem_raw);
-    if (p.pro == PRO_NORM_QUANT) { kq_prologue<true>(p, nT, rec, col, scale_s); } else { kq_prologue<false>(p, nT, rec, col, scale_s); }
+    if constexpr (PRO == KQP_ANY) {
+        if (p.pro == PRO_NORM_QUANT) { kq_prologue<true>(p, nT, rec, col, scale_s); } else { kq_prologue<false>(p, nT, rec, col, scale_s); }
+    } else {
+        auto rest = [&]() { if (lane == 0) { while (issued < min(pl.ns, n_stage)) { issue_next(); } } };
+        constexpr bool NORM = PRO == KQP_NORM || PRO == KQP_NORM_LONG;
+        kq_prologue_1col<(PRO == KQP_NORM || PRO == KQP_PLAIN) ? KQ_NORM_EARLY : KQ_PRO_GROUPS, NORM>(p, rec, scale_s, wearly, rest);
+    }
     __syncthreads();
 
     const uint32_t rec_s = smem_u32(rec), col_bytes = (uint32_t)col * 4u;
@@ -423,14 +495,28 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg) {
     const size_t smem = kq_smem_layout(nsb, TM, pl).total;
     if (smem > budget) { return cudaErrorInvalidValue; }
     using Kernel = void (*)(const MatvecParams, const KqPlan);
-    static const Kernel kernels[3][3] = {{matvec_kq_kernel<1, 12>, matvec_kq_kernel<1, 14>, matvec_kq_kernel<1, 0>},
-                                         {matvec_kq_kernel<2, 12>, matvec_kq_kernel<2, 14>, matvec_kq_kernel<2, 0>},
-                                         {matvec_kq_kernel<KQ_MAX_COLUMNS, 12>, matvec_kq_kernel<KQ_MAX_COLUMNS, 14>, matvec_kq_kernel<KQ_MAX_COLUMNS, 0>}};
-    const Kernel kernel = kernels[TM == 1 ? 0 : TM == 2 ? 1 : 2][q4 && q6 ? 2 : q6 ? 1 : 0];
+    const int ty = q4 && q6 ? 2 : q6 ? 1 : 0;
+    Kernel kernel;
+    if (TM == 1) {
+        static const Kernel one[5][3] = {
+            {matvec_kq_kernel<1, 12, KQP_ANY>, matvec_kq_kernel<1, 14, KQP_ANY>, matvec_kq_kernel<1, 0, KQP_ANY>},
+            {matvec_kq_kernel<1, 12, KQP_NORM>, matvec_kq_kernel<1, 14, KQP_NORM>, matvec_kq_kernel<1, 0, KQP_NORM>},
+            {matvec_kq_kernel<1, 12, KQP_PLAIN>, matvec_kq_kernel<1, 14, KQP_PLAIN>, matvec_kq_kernel<1, 0, KQP_PLAIN>},
+            {matvec_kq_kernel<1, 12, KQP_NORM_LONG>, matvec_kq_kernel<1, 14, KQP_NORM_LONG>, matvec_kq_kernel<1, 0, KQP_NORM_LONG>},
+            {matvec_kq_kernel<1, 12, KQP_PLAIN_LONG>, matvec_kq_kernel<1, 14, KQP_PLAIN_LONG>, matvec_kq_kernel<1, 0, KQP_PLAIN_LONG>}};
+        const int64_t n4 = p.A.k >> 2;
+        const bool norm = p.pro == PRO_NORM_QUANT;
+        kernel = one[n4 <= KQ_NORM_EARLY * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : n4 <= KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY][ty];
+    } else {
+        static const Kernel more[2][3] = {{matvec_kq_kernel<2, 12, KQP_ANY>, matvec_kq_kernel<2, 14, KQP_ANY>, matvec_kq_kernel<2, 0, KQP_ANY>},
+                                          {matvec_kq_kernel<KQ_MAX_COLUMNS, 12, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 14, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 0, KQP_ANY>}};
+        kernel = more[TM == 2 ? 0 : 1][ty];
+    }
     cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem);
     if (err != cudaSuccess) { return err; }
     MatvecParams q = p;
     if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
+    if (cfg.pdl) { q.stages_early = MV_STAGES_EARLY; }
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)grid); lc.blockDim = dim3(KQ_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
     cudaLaunchAttribute attr[1];

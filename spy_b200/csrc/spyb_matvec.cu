@@ -120,8 +120,19 @@ cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
 // Single column, K <= 12288: every thread keeps its (at most PG) float4 groups of x in registers from the one
 // global read through the sum of squares to the quantizer; same arithmetic as the general prologue below.
 constexpr int PRO_GROUPS = 6;
-template <int PG, bool NORM>
-__device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActPlanes act, float *v3, float *scales) {
+// The norm weights of rows of at most NORM_EARLY * 512 groups are read at the start of the kernel, in front of the weight copies: behind a ring
+// full of them on every SM they arrive after the sum of squares is done.
+constexpr int NORM_EARLY = 2;
+__device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float4 (&w)[NORM_EARLY]) {
+    const int n4 = (int)(p.A.k >> 2);
+#pragma unroll
+    for (int k = 0; k < NORM_EARLY; ++k) {
+        const int g = threadIdx.x + k * MV_THREADS;
+        w[k] = (p.pro == PRO_NORM_QUANT && g < n4) ? reinterpret_cast<const float4 *>(p.norm_w)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+template <int PG, bool NORM, class Requested>
+__device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActPlanes act, float *v3, float *scales, const float4 *wearly, Requested x_requested) {
     const int tid = threadIdx.x;
     const int nbp = p.A.nbp;
     const int n4  = (int)(p.A.k >> 2);
@@ -135,6 +146,7 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
         const int g = tid + k * MV_THREADS;
         xv[k] = (k < npass && g < n4) ? __ldcg(x4 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    x_requested();
     if (NORM) {
         const float4 *w4 = reinterpret_cast<const float4 *>(p.norm_w);
 #pragma unroll
@@ -147,15 +159,19 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
                 v3[g] = __fadd_rn(v1, v2);
             }
         }
-        // the norm weights arrive while the sum of squares is formed
+        // the norm weights: in registers already, or arriving while the sum of squares is formed
         float4 wv[PG];
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
             const int g = tid + k * MV_THREADS;
-            wv[k] = (k < npass && g < n4) ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (PG <= NORM_EARLY) { wv[k] = wearly[k]; }
+            else { wv[k] = (k < npass && g < n4) ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f); }
         }
         __syncthreads();
-        const float sum = (tid == 0) ? running_sum_serial(smem_u32(v3), n4) : 0.f;
+        __shared__ __align__(16) float rs_scratch[PG <= 2 ? rs_scratch_words(2) : 4];
+        float sum = 0.f;
+        if (PG <= 2 && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
+        else if (tid == 0) { sum = running_sum_serial(smem_u32(v3), n4); }
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
             scales[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
@@ -314,12 +330,13 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
             src[i] = M.w + (size_t)(p.pair_mode ? u : R * u + i) * tile_bytes;
         }
     };
+    const uint64_t policy = l2_evict_first();
     auto issue_next = [&]() {
         const uint32_t bytes = (uint32_t)min(S, nrec - lrec) * RECB;
         const uint32_t bar = bar_s + lslot * 8, dst = ring_s + lslot * stage_bytes;
         mbar_expect_tx(bar, bytes * R);
 #pragma unroll
-        for (int i = 0; i < R; ++i) { bulk_copy_g2s(dst + i * S * RECB, src[i], bytes, bar); src[i] += bytes; }
+        for (int i = 0; i < R; ++i) { bulk_copy_g2s_once(dst + i * S * RECB, src[i], bytes, bar, policy); src[i] += bytes; }
         ++issued;
         if (++lslot == NS) { lslot = 0; }
         lrec += S;
@@ -329,6 +346,8 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
     // Let the next kernel of the step begin, and start streaming: weights never change during a step, so the
     // copies may run ahead of the previous kernel's results.
     pdl_launch_dependents();
+    float4 wearly[NORM_EARLY];
+    if (TM == 1) { norm_weights_early(p, wearly); }
     stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
     if (lane == 0 && n_items > 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(bar_s + s * 8, 1); }
@@ -347,9 +366,9 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true>(p, act, v3, norm_scales); } else { matvec_prologue_1col<2, false>(p, act, v3, norm_scales); }
+            if (norm) { matvec_prologue_1col<2, true>(p, act, v3, norm_scales, wearly, []() {}); } else { matvec_prologue_1col<2, false>(p, act, v3, norm_scales, wearly, []() {}); }
         } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true>(p, act, v3, norm_scales); } else { matvec_prologue_1col<PRO_GROUPS, false>(p, act, v3, norm_scales); }
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true>(p, act, v3, norm_scales, wearly, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false>(p, act, v3, norm_scales, wearly, []() {}); }
         } else {
             matvec_prologue<TM>(p, act, v3, norm_scales);
         }
@@ -482,7 +501,9 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
 // A record is [TR rows][2 groups x 64 B (Q4_0) or 128 B (Q8_0) | 8 fp16 scales]; the 144-byte (272-byte) row pitch
 // makes the 128-bit reads of eight consecutive rows conflict-free.
 // With fused_pair, rows 0..TR/2-1 of tile u are FFN-up rows (TR/2)u.. and rows TR/2..TR-1 the matching FFN-gate rows.
-template <int WT, int TM, int LPR>
+// the prologue a kernel is built with: rows of at most 1024 groups of four, longer ones, with and without the norm; any number of columns
+enum { MVP_ANY, MVP_NORM, MVP_PLAIN, MVP_NORM_LONG, MVP_PLAIN_LONG };
+template <int WT, int TM, int LPR, int PRO>
 __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const MatvecParams p, const int ring_bytes, const int S, const int wact) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ float norm_scales[8];
@@ -518,11 +539,12 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     int64_t lu = my_first; int lrec = 0, lslot = 0, issued = 0;
     bool    ok = true;
     // lane 0: stage lslot <- the next <= S records (the stage was handed back by this warp's own __syncwarp)
+    const uint64_t policy = l2_evict_first();
     auto issue_next = [&]() {
         const uint32_t bytes = (uint32_t)min(S, nrec - lrec) * RECB;
         const uint32_t bar = full_s + lslot * 8;
         mbar_expect_tx(bar, bytes);
-        bulk_copy_g2s(ring_s + lslot * stage_bytes, src, bytes, bar);
+        bulk_copy_g2s_once(ring_s + lslot * stage_bytes, src, bytes, bar, policy);
         src += bytes;
         ++issued;
         if (++lslot == NS) { lslot = 0; }
@@ -531,29 +553,29 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     };
 
     pdl_launch_dependents();
+    float4 wearly[NORM_EARLY];
+    if (PRO == MVP_NORM) { norm_weights_early(p, wearly); }
     stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
     if (lane == 0 && n_items > 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(full_s + s * 8, 1); }
         mbar_init_fence();
         src = p.A.w + (size_t)lu * tile_bytes;
-        for (int s = 0; s < NS && issued < n_items; ++s) { issue_next(); }
+        for (int s = 0; s < (PRO == MVP_ANY ? NS : min(NS, p.stages_early)) && issued < n_items; ++s) { issue_next(); }
     }
     __syncwarp();
     pdl_wait();
     stamp(p.stamps, 1, false); stamp(p.stamps, 5, true);
     tp_wait(p.tp, p.error_flag);
 
+    auto rest = [&]() { if (lane == 0) { while (issued < min(NS, n_items)) { issue_next(); } } };
     ActPlanes act = act_planes(smem_raw, nbp, TM);
     {
         float *v3 = reinterpret_cast<float *>(smem_raw);
-        const int  n4p  = nbp * 8;
-        const bool norm = p.pro == PRO_NORM_QUANT;
-        if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true>(p, act, v3, norm_scales); } else { matvec_prologue_1col<2, false>(p, act, v3, norm_scales); }
-        } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true>(p, act, v3, norm_scales); } else { matvec_prologue_1col<PRO_GROUPS, false>(p, act, v3, norm_scales); }
-        } else {
-            matvec_prologue<TM>(p, act, v3, norm_scales);
+        if constexpr (PRO == MVP_ANY) { matvec_prologue<TM>(p, act, v3, norm_scales); }
+        else {
+            constexpr bool NORM = PRO == MVP_NORM || PRO == MVP_NORM_LONG;
+            constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 2 : PRO_GROUPS;
+            matvec_prologue_1col<PG, NORM>(p, act, v3, norm_scales, wearly, rest);
         }
     }
     __syncthreads();
@@ -712,11 +734,12 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_mma_kernel(const MatvecP
     const uint8_t *src = nullptr;
     int64_t lu = my_first; int lrec = 0, lslot = 0, issued = 0;
     bool    ok = true;
+    const uint64_t policy = l2_evict_first();
     auto issue_next = [&]() {
         const uint32_t bytes = (uint32_t)min(S, nrec - lrec) * RECB;
         const uint32_t bar = full_s + lslot * 8;
         mbar_expect_tx(bar, bytes);
-        bulk_copy_g2s(ring_s + lslot * stage_bytes, src, bytes, bar);
+        bulk_copy_g2s_once(ring_s + lslot * stage_bytes, src, bytes, bar, policy);
         src += bytes;
         ++issued;
         if (++lslot == NS) { lslot = 0; }
@@ -725,6 +748,8 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_mma_kernel(const MatvecP
     };
 
     pdl_launch_dependents();
+    float4 wearly[NORM_EARLY];
+    if (TM == 1) { norm_weights_early(p, wearly); }
     stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
     if (lane == 0 && n_items > 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(full_s + s * 8, 1); }
@@ -743,9 +768,9 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_mma_kernel(const MatvecP
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true>(p, act, v3, norm_scales); } else { matvec_prologue_1col<2, false>(p, act, v3, norm_scales); }
+            if (norm) { matvec_prologue_1col<2, true>(p, act, v3, norm_scales, wearly, []() {}); } else { matvec_prologue_1col<2, false>(p, act, v3, norm_scales, wearly, []() {}); }
         } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true>(p, act, v3, norm_scales); } else { matvec_prologue_1col<PRO_GROUPS, false>(p, act, v3, norm_scales); }
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true>(p, act, v3, norm_scales, wearly, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false>(p, act, v3, norm_scales, wearly, []() {}); }
         } else {
             matvec_prologue<TM>(p, act, v3, norm_scales);
         }
@@ -837,6 +862,7 @@ static cudaError_t launch_matvec_mma_t(const MatvecParams &p, const LaunchCfg &c
     if (err != cudaSuccess) { return err; }
     MatvecParams q = p;
     if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
+    if (cfg.pdl) { q.stages_early = MV_STAGES_EARLY; }
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)grid); lc.blockDim = dim3(MV_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
     cudaLaunchAttribute attr[1];
@@ -879,17 +905,25 @@ static cudaError_t launch_matvec_rows_t(const MatvecParams &p, const LaunchCfg &
     if (cfg.mv_force_wact > 0) { wact = std::min(cfg.mv_force_wact, MV_WARPS); }
     if (ring / ((size_t)wact * S * RECB) < 1) { return cudaErrorInvalidValue; }
     const size_t smem = fixed.total + ring;
-    cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(matvec_rows_kernel<WT, TM, LPR>), smem);
+    void (*kernel)(const MatvecParams, const int, const int, const int) = matvec_rows_kernel<WT, TM, LPR, MVP_ANY>;
+    if constexpr (TM == 1) {
+        const int  n4p = p.A.nbp * 8;
+        const bool norm = p.pro == PRO_NORM_QUANT;
+        if (n4p <= 2 * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN>; }
+        else if (n4p <= PRO_GROUPS * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM_LONG> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN_LONG>; }
+    }
+    cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem);
     if (err != cudaSuccess) { return err; }
     MatvecParams q = p;
     if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
+    if (cfg.pdl) { q.stages_early = MV_STAGES_EARLY; }
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)grid); lc.blockDim = dim3(MV_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr; lc.numAttrs = cfg.pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&lc, matvec_rows_kernel<WT, TM, LPR>, q, (int)ring, S, wact);
+    return cudaLaunchKernelEx(&lc, kernel, q, (int)ring, S, wact);
 }
 
 template <int WT, int LPR>
@@ -946,6 +980,7 @@ static cudaError_t launch_matvec_t(const MatvecParams &p, const LaunchCfg &cfg) 
     if (err != cudaSuccess) { return err; }
     MatvecParams q = p;
     if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
+    if (cfg.pdl) { q.stages_early = MV_STAGES_EARLY; }
 
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)grid); lc.blockDim = dim3(MV_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
