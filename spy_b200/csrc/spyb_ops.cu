@@ -612,11 +612,11 @@ __global__ void __launch_bounds__(ATT_PV_WARPS * WARP) attn_pv_kernel(const Attn
 // ---------------------------------------------------------------------------------------------
 // A step over a long context in one kernel: ATL_C CTAs (a cluster) take a head. Each CTA scores its quarter of the positions, the quarters'
 // exponentials meet in every CTA's shared memory, each CTA forms the softmax sum (its order allows no split) and then its quarter of the
-// head's output elements over all positions. Same arithmetic as attention_kernel. HBM-bound: K and V^T are read once. One warp copies
+// head's output elements over all positions. Same arithmetic as attention_kernel. HBM-bound: K and V^T are read once. Four warps copy
 // both through one ring of stages (32 K rows of 256 bytes, or 512 positions of eight V^T rows) without regard to the phases: while the
 // softmax is formed, V^T fills the ring. (cp.async, 512 bytes an instruction: bulk copies of a row each cost the warp 50 cycles, 54 us in all.) A stage is filled for one warp: no CTA-wide waits on the way.
 // 32 heads over 4000 positions, three kernels (scores, softmax, PV) before: 41 us, now 28; the reads take 10.3.
-constexpr int ATL_C = 4, ATL_WARPS = 8, ATL_THREADS = (ATL_WARPS + 1) * WARP;
+constexpr int ATL_C = 4, ATL_WARPS = 8, ATL_COPY_WARPS = 4, ATL_THREADS = (ATL_WARPS + ATL_COPY_WARPS) * WARP;
 constexpr int ATL_KPITCH = 272, ATL_VCH = 512, ATL_VROWS = 8, ATL_VPITCH = 2 * ATL_VCH + 64, ATL_STAGE = 32 * ATL_KPITCH;   // pitches without bank conflicts
 static_assert(ATL_VROWS * ATL_VPITCH == ATL_STAGE && ATL_C * 4 * ATL_VROWS == ATT_HD, "both kinds of stages fill the slot; four warps take a CTA's elements");
 constexpr int ATL_MAX_STAGES = 22, ATL_MIN_STAGES = 6;
@@ -679,14 +679,13 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
     const int slice = ((n_vis + ATL_C * 32 - 1) / (ATL_C * 32)) * 32, start = rank * slice;
     const int cnt = max(0, min(slice, n_vis - start)), nK = (cnt + 31) >> 5, nC = (n_vis + ATL_VCH - 1) / ATL_VCH;
     uint64_t limit = WAIT_LIMIT_NS;
-    if (warp == ATL_WARPS) {
+    if (warp >= ATL_WARPS) {
         const __half *K = p.k_cache + (batch ? (int64_t)t * p.seq_stride : 0) + (int64_t)start * p.dl + (int64_t)h * ATT_HD;
         const __half *V = p.v_cache + (batch ? (int64_t)t * p.seq_stride : 0) + ((int64_t)h * ATT_HD + rank * (ATT_HD / ATL_C)) * p.n_ctx;
         const int total = nK + 4 * nC;
-        int slot = 0; uint32_t phase = 1;   // (the first round finds every slot empty)
-        int g = 0;
-        for (; g < total && limit != 0; ++g) {
-            if (g >= NS) { atl_wait(empty_s + 8 * slot, phase, limit); }
+        for (int g = warp - ATL_WARPS; g < total; g += ATL_COPY_WARPS) {
+            const int slot = g % NS;
+            if (g >= NS) { atl_wait(empty_s + 8 * slot, (uint32_t)(g / NS - 1) & 1u, limit); }
             if (!__all_sync(0xffffffffu, limit != 0)) { break; }
             const uint32_t bar = full_s + 8 * slot, dst = ring_s + slot * ATL_STAGE;
             if (g < nK) {
@@ -702,7 +701,6 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
                 for (int i = 0; i < 16; ++i) { if ((i & 1) * 256 < left) { cp_async16(dst + (i >> 1) * ATL_VPITCH + (i & 1) * 512 + lane * 16, row + (int64_t)(i >> 1) * p.n_ctx + (i & 1) * 256); } }
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-            if (++slot == NS) { slot = 0; phase ^= 1u; }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");   // no copy is in flight when the CTA ends, also when its readers gave up
     } else {
