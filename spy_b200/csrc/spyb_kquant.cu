@@ -99,8 +99,8 @@ __device__ __forceinline__ void kq_prologue(const MatvecParams &p, int nT, uint3
 }
 
 // One column of at most 512 PG groups of four: every thread keeps its groups of x in registers from the one global read on; x_requested() is
-// called when the reads are on their way. wearly: the norm weights when the kernel read them at its start (PG == KQ_NORM_EARLY).
-constexpr int KQ_NORM_EARLY = 2, KQ_PRO_GROUPS = 6;
+// called when the reads are on their way. wearly: the norm weights when the kernel read them at its start (PG <= KQ_NORM_EARLY).
+constexpr int KQ_NORM_EARLY = 3, KQ_PRO_GROUPS = 6;
 template <int PG, bool NORM, class Requested>
 __device__ __forceinline__ void kq_prologue_1col(const MatvecParams &p, uint32_t *rec, float *scale_s, const float4 *wearly, Requested x_requested) {
     const int tid = threadIdx.x;
@@ -116,7 +116,7 @@ __device__ __forceinline__ void kq_prologue_1col(const MatvecParams &p, uint32_t
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
             const int g = tid + k * KQ_THREADS;
-            if (PG == KQ_NORM_EARLY) { wv[k] = wearly[k]; }
+            if (PG <= KQ_NORM_EARLY) { wv[k] = wearly[k]; }
             else { wv[k] = g < n4 ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f); }
         }
     }
@@ -130,8 +130,8 @@ __device__ __forceinline__ void kq_prologue_1col(const MatvecParams &p, uint32_t
         }
         __syncthreads();
         float sum = 0.f;
-        if (PG == 2 && n4 >= RS_MIN && (n4 >> 6) * (KQ_REC - 64) >= rs_scratch_words(2)) {
-            if (tid < RS_THREADS) { sum = running_sum_chunks<2>(smem_u32(v3), n4, smem_u32(v3 + n4), tid, 1); }
+        if (PG <= KQ_NORM_EARLY && n4 >= RS_MIN && (n4 >> 6) * (KQ_REC - 64) >= rs_scratch_words(PG)) {
+            if (tid < RS_THREADS) { sum = running_sum_chunks<PG <= KQ_NORM_EARLY ? PG : 2>(smem_u32(v3), n4, smem_u32(v3 + n4), tid, 1); }
         } else if (tid == 0) { sum = running_sum_serial(smem_u32(v3), n4); }
         if (tid == 0) { scale_s[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)p.A.k), p.eps))); }
         __syncthreads();   // also: the partials (aliasing the records) are dead from here on
@@ -279,8 +279,9 @@ __host__ __device__ static inline KqSmem kq_smem_layout(int nsb, int TM, const K
 
 // TM: columns of the pass, rounded up to 1, 2 or 4 (columns past p.T compute on whatever their records hold and are not stored); TYPE: 12 or
 // 14 when every row is of that type, else 0
-// PRO: the prologue the kernel is built with - one column of at most 1024 groups of four or a longer one, with and without the norm; else any
-enum { KQP_ANY, KQP_NORM, KQP_PLAIN, KQP_NORM_LONG, KQP_PLAIN_LONG };
+// PRO: the prologue the kernel is built with - one column of at most 1024 groups of four (with the norm also 1536) or a longer one, with and without the norm;
+// else any
+enum { KQP_ANY, KQP_NORM, KQP_NORM_MID, KQP_PLAIN, KQP_NORM_LONG, KQP_PLAIN_LONG };
 template <int TM, int TYPE, int PRO>
 __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecParams p, const KqPlan pl) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -340,10 +341,11 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
 
     // weights never change during a step: the copies may run ahead of the previous kernel's results
     pdl_launch_dependents();
-    float4 wearly[KQ_NORM_EARLY];
-    if (PRO == KQP_NORM) {
+    constexpr int PG = (PRO == KQP_NORM || PRO == KQP_PLAIN) ? 2 : PRO == KQP_NORM_MID ? 3 : KQ_PRO_GROUPS;
+    float4 wearly[PRO == KQP_NORM_MID ? 3 : 2];
+    if (PRO == KQP_NORM || PRO == KQP_NORM_MID) {
 #pragma unroll
-        for (int k = 0; k < KQ_NORM_EARLY; ++k) {
+        for (int k = 0; k < (PG < 4 ? PG : 0); ++k) {
             const int g = threadIdx.x + k * KQ_THREADS;
             wearly[k] = g < (int)(p.A.k >> 2) ? reinterpret_cast<const float4 *>(p.norm_w)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
@@ -362,8 +364,8 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
         if (p.pro == PRO_NORM_QUANT) { kq_prologue<true>(p, nT, rec, col, scale_s); } else { kq_prologue<false>(p, nT, rec, col, scale_s); }
     } else {
         auto rest = [&]() { if (lane == 0) { while (issued < min(pl.ns, n_stage)) { issue_next(); } } };
-        constexpr bool NORM = PRO == KQP_NORM || PRO == KQP_NORM_LONG;
-        kq_prologue_1col<(PRO == KQP_NORM || PRO == KQP_PLAIN) ? KQ_NORM_EARLY : KQ_PRO_GROUPS, NORM>(p, rec, scale_s, wearly, rest);
+        constexpr bool NORM = PRO == KQP_NORM || PRO == KQP_NORM_MID || PRO == KQP_NORM_LONG;
+        kq_prologue_1col<PG, NORM>(p, rec, scale_s, wearly, rest);
     }
     __syncthreads();
 
@@ -498,15 +500,16 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg) {
     const int ty = q4 && q6 ? 2 : q6 ? 1 : 0;
     Kernel kernel;
     if (TM == 1) {
-        static const Kernel one[5][3] = {
+        static const Kernel one[6][3] = {
             {matvec_kq_kernel<1, 12, KQP_ANY>, matvec_kq_kernel<1, 14, KQP_ANY>, matvec_kq_kernel<1, 0, KQP_ANY>},
             {matvec_kq_kernel<1, 12, KQP_NORM>, matvec_kq_kernel<1, 14, KQP_NORM>, matvec_kq_kernel<1, 0, KQP_NORM>},
+            {matvec_kq_kernel<1, 12, KQP_NORM_MID>, matvec_kq_kernel<1, 14, KQP_NORM_MID>, matvec_kq_kernel<1, 0, KQP_NORM_MID>},
             {matvec_kq_kernel<1, 12, KQP_PLAIN>, matvec_kq_kernel<1, 14, KQP_PLAIN>, matvec_kq_kernel<1, 0, KQP_PLAIN>},
             {matvec_kq_kernel<1, 12, KQP_NORM_LONG>, matvec_kq_kernel<1, 14, KQP_NORM_LONG>, matvec_kq_kernel<1, 0, KQP_NORM_LONG>},
             {matvec_kq_kernel<1, 12, KQP_PLAIN_LONG>, matvec_kq_kernel<1, 14, KQP_PLAIN_LONG>, matvec_kq_kernel<1, 0, KQP_PLAIN_LONG>}};
         const int64_t n4 = p.A.k >> 2;
         const bool norm = p.pro == PRO_NORM_QUANT;
-        kernel = one[n4 <= KQ_NORM_EARLY * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : n4 <= KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY][ty];
+        kernel = one[n4 <= 2 * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : norm && n4 <= 3 * KQ_THREADS ? KQP_NORM_MID : n4 <= KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY][ty];
     } else {
         static const Kernel more[2][3] = {{matvec_kq_kernel<2, 12, KQP_ANY>, matvec_kq_kernel<2, 14, KQP_ANY>, matvec_kq_kernel<2, 0, KQP_ANY>},
                                           {matvec_kq_kernel<KQ_MAX_COLUMNS, 12, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 14, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 0, KQP_ANY>}};

@@ -122,11 +122,12 @@ cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
 constexpr int PRO_GROUPS = 6;
 // The norm weights of rows of at most NORM_EARLY * 512 groups are read at the start of the kernel, in front of the weight copies: behind a ring
 // full of them on every SM they arrive after the sum of squares is done.
-constexpr int NORM_EARLY = 2;
-__device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float4 (&w)[NORM_EARLY]) {
+constexpr int NORM_EARLY = 3;
+template <int PG>
+__device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float4 (&w)[PG]) {
     const int n4 = (int)(p.A.k >> 2);
 #pragma unroll
-    for (int k = 0; k < NORM_EARLY; ++k) {
+    for (int k = 0; k < PG; ++k) {
         const int g = threadIdx.x + k * MV_THREADS;
         w[k] = (p.pro == PRO_NORM_QUANT && g < n4) ? reinterpret_cast<const float4 *>(p.norm_w)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -168,9 +169,9 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
             else { wv[k] = (k < npass && g < n4) ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f); }
         }
         __syncthreads();
-        __shared__ __align__(16) float rs_scratch[PG <= 2 ? rs_scratch_words(2) : 4];
+        __shared__ __align__(16) float rs_scratch[PG <= NORM_EARLY ? rs_scratch_words(PG) : 4];
         float sum = 0.f;
-        if (PG <= 2 && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
+        if (PG <= NORM_EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<PG <= NORM_EARLY ? PG : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
         else if (tid == 0) { sum = running_sum_serial(smem_u32(v3), n4); }
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
@@ -501,8 +502,11 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
 // A record is [TR rows][2 groups x 64 B (Q4_0) or 128 B (Q8_0) | 8 fp16 scales]; the 144-byte (272-byte) row pitch
 // makes the 128-bit reads of eight consecutive rows conflict-free.
 // With fused_pair, rows 0..TR/2-1 of tile u are FFN-up rows (TR/2)u.. and rows TR/2..TR-1 the matching FFN-gate rows.
-// the prologue a kernel is built with: rows of at most 1024 groups of four, longer ones, with and without the norm; any number of columns
-enum { MVP_ANY, MVP_NORM, MVP_PLAIN, MVP_NORM_LONG, MVP_PLAIN_LONG };
+// the prologue a kernel is built with: rows of at most 1024 groups of four (with the norm also 1536), longer ones, with and without the norm; any
+// number of columns.
+// (One kernel with all of them takes 121 registers instead of 79 and its loop is scheduled worse. A Q4_0 layer of a 7B step, with the
+// evict-first copies, the early norm weights and the late ring: 49.1 -> 43.7 us.)
+enum { MVP_ANY, MVP_NORM, MVP_NORM_MID, MVP_PLAIN, MVP_NORM_LONG, MVP_PLAIN_LONG };
 template <int WT, int TM, int LPR, int PRO>
 __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const MatvecParams p, const int ring_bytes, const int S, const int wact) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -553,8 +557,8 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     };
 
     pdl_launch_dependents();
-    float4 wearly[NORM_EARLY];
-    if (PRO == MVP_NORM) { norm_weights_early(p, wearly); }
+    float4 wearly[PRO == MVP_NORM_MID ? 3 : 2];
+    if (PRO == MVP_NORM || PRO == MVP_NORM_MID) { norm_weights_early(p, wearly); }
     stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
     if (lane == 0 && n_items > 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(full_s + s * 8, 1); }
@@ -573,8 +577,8 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
         float *v3 = reinterpret_cast<float *>(smem_raw);
         if constexpr (PRO == MVP_ANY) { matvec_prologue<TM>(p, act, v3, norm_scales); }
         else {
-            constexpr bool NORM = PRO == MVP_NORM || PRO == MVP_NORM_LONG;
-            constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 2 : PRO_GROUPS;
+            constexpr bool NORM = PRO == MVP_NORM || PRO == MVP_NORM_MID || PRO == MVP_NORM_LONG;
+            constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 2 : PRO == MVP_NORM_MID ? 3 : PRO_GROUPS;
             matvec_prologue_1col<PG, NORM>(p, act, v3, norm_scales, wearly, rest);
         }
     }
@@ -910,6 +914,7 @@ static cudaError_t launch_matvec_rows_t(const MatvecParams &p, const LaunchCfg &
         const int  n4p = p.A.nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (n4p <= 2 * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN>; }
+        else if (norm && n4p <= 3 * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_NORM_MID>; }
         else if (n4p <= PRO_GROUPS * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM_LONG> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN_LONG>; }
     }
     cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem);

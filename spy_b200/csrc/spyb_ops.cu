@@ -287,7 +287,8 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
 }
 
 // ---------------------------------------------------------------------------------------------
-// Long contexts (n_ctx > ATT_LONG_MIN): the same arithmetic as attention_kernel, spread over the chip in three kernels
+// Long contexts (n_ctx > ATT_LONG_MIN) where attn_cluster_kernel does not apply, and prompts (token-tiled forms of the first and the
+// last): the same arithmetic as attention_kernel, spread over the chip in three kernels
 // that meet in a scratch buffer [T][n_head][n_ctx] of floats (scores, then probabilities):
 //   attn_scores_kernel   one thread per (position, head, token): Dot<FP16,FP16>(K row, Q), all 32 accumulators in registers
 //   attn_softmax_kernel  one CTA per (head, token): scale, maximum, table exp, std::reduce's grouped running sum, 1/sum,
@@ -615,7 +616,7 @@ __global__ void __launch_bounds__(ATT_PV_WARPS * WARP) attn_pv_kernel(const Attn
 // head's output elements over all positions. Same arithmetic as attention_kernel. HBM-bound: K and V^T are read once. Four warps copy
 // both through one ring of stages (32 K rows of 256 bytes, or 512 positions of eight V^T rows) without regard to the phases: while the
 // softmax is formed, V^T fills the ring. (cp.async, 512 bytes an instruction: bulk copies of a row each cost the warp 50 cycles, 54 us in all.) A stage is filled for one warp: no CTA-wide waits on the way.
-// 32 heads over 4000 positions, three kernels (scores, softmax, PV) before: 41 us, now 28; the reads take 10.3.
+// 32 heads over 4000 positions, three kernels (scores, softmax, PV) before: 41 us, now about 22; the reads take 10.3.
 constexpr int ATL_C = 4, ATL_WARPS = 8, ATL_COPY_WARPS = 4, ATL_THREADS = (ATL_WARPS + ATL_COPY_WARPS) * WARP;
 constexpr int ATL_KPITCH = 272, ATL_VCH = 512, ATL_VROWS = 8, ATL_VPITCH = 2 * ATL_VCH + 64, ATL_STAGE = 32 * ATL_KPITCH;   // pitches without bank conflicts
 static_assert(ATL_VROWS * ATL_VPITCH == ATL_STAGE && ATL_C * 4 * ATL_VROWS == ATT_HD, "both kinds of stages fill the slot; four warps take a CTA's elements");

@@ -30,6 +30,7 @@ constexpr int KQ_EPI_WARPS = 16, KQ_GEMM_THREADS = 608;   // sixteen epilogue wa
 //
 // Bound of the wide tile: issue slots. Per (row, token, block) two multiplications and two FMAs, packed two tokens at a time, and eight
 // uniform 128-bit shared-memory reads of the token scales per 16 tokens.
+// Q4_K_M, 8 layers, 512 tokens: 9.6 ms in all (one 64-token tile per CTA with 8-bit operands: 14.3); 4 layers, 16 tokens: 0.86 (2.43).
 template <int TT> struct KqGeom {
     static constexpr int NB    = TT == 64 ? 2 : 4;            // blocks per step
     static constexpr int YB    = TT * 72;                     // a block's activations: TT x 32 f16, TT scales, TT sums

@@ -354,6 +354,20 @@ def test_step_kernel_wait_runs_out_and_is_reported(oracle, tmp_models, monkeypat
     m.close(); b.close()
 
 
+@pytest.mark.parametrize("d,wtype", [(4352, quants.Q4_K), (5120, quants.Q4_0), (5120, quants.Q4_K), (6144, quants.Q8_0)])
+def test_steps_of_widths_between_the_prologues(be, oracle, tmp_models, d, wtype):
+    """Rows of more than 1024 and at most 1536 groups of four: single steps with the norm in front, whose sum of squares runs in chunks of twelve values
+    (4352 with K-quants: too little scratch beside the records, the plain chain)."""
+    cfg = gguf_io.LlamaConfig(n_layer=1, d_model=d, n_head=d // 128, n_ff=512, n_vocab=64, wtype=wtype, embd_type=quants.Q8_0)
+    path = str(tmp_models / f"mid{d}_{wtype}.gguf")
+    gguf_io.make_llama_gguf(path, cfg, seed=d)
+    want_ids, want_logits = oracle.OracleLlama(path, n_ctx=32).generate([5, 9], 4)
+    m = B.LlamaModel(be, path, n_ctx=32)
+    ids, logits = m.generate([5, 9], 4)
+    assert np.array_equal(ids, want_ids) and logits_ok(logits, want_logits)
+    m.close()
+
+
 @pytest.mark.parametrize("env", [{}, {"SPYB_STEP": "1"}])
 def test_long_context_attention_path_in_the_model(env, oracle, tmp_models, monkeypatch):
     """A context above 1024 positions switches attention to the three-kernel path (scores / softmax / PV spread over the
