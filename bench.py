@@ -387,8 +387,8 @@ def main():
                "launches": int(model.last_launches),
                "tflops": pre_tflops, "frac_of_bf16_peak": pre_tflops / (bf16_peak_tflops() * world),
                "tflops_note": "algorithmic: 2 x layer weights x tokens / time, against the measured dense bf16 peak of the GPUs used; the tensor cores issue 8 x "
-                              "that (one MMA column per accumulator of a token: block-diagonal B operand), times 2 (Q4_0) or 4 (Q8_0) for the e4m3 split of "
-                              "8-bit values, and the f32 chains after them set the time",
+                              "that (one MMA column per accumulator of a token: block-diagonal B operand; K-quants: 1 or 2 x), and the f32 chains after them "
+                              "set the time",
                "note": "one spyb_model_eval over the prompt (device time, CUDA events): chunks of up to 512 tokens through the tcgen05 GEMM kernel when the "
                        "widths fit its tiles (sharded models: each rank its heads and FFN rows, one NCCL all-gather of the attention output and of the FFN activation per layer)"}
     barrier()

@@ -120,7 +120,8 @@ cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
 // Single column, K <= 12288: every thread keeps its (at most PG) float4 groups of x in registers from the one
 // global read through the sum of squares to the quantizer; same arithmetic as the general prologue below.
 constexpr int PRO_GROUPS = 6;
-// The norm weights of rows of at most NORM_EARLY * 512 groups are read at the start of the kernel, in front of the weight copies: behind a ring
+// EARLY (kernels of their own per prologue only: elsewhere its registers cost the other paths): the sum of squares runs on four warps and the
+// norm weights of rows of at most NORM_EARLY * 512 groups are read at the start of the kernel, in front of the weight copies: behind a ring
 // full of them on every SM they arrive after the sum of squares is done.
 constexpr int NORM_EARLY = 3;
 template <int PG>
@@ -132,7 +133,7 @@ __device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float4
         w[k] = (p.pro == PRO_NORM_QUANT && g < n4) ? reinterpret_cast<const float4 *>(p.norm_w)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
-template <int PG, bool NORM, class Requested>
+template <int PG, bool NORM, bool EARLY, class Requested>
 __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActPlanes act, float *v3, float *scales, const float4 *wearly, Requested x_requested) {
     const int tid = threadIdx.x;
     const int nbp = p.A.nbp;
@@ -165,13 +166,13 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
             const int g = tid + k * MV_THREADS;
-            if (PG <= NORM_EARLY) { wv[k] = wearly[k]; }
+            if (EARLY) { wv[k] = wearly[k]; }
             else { wv[k] = (k < npass && g < n4) ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f); }
         }
         __syncthreads();
-        __shared__ __align__(16) float rs_scratch[PG <= NORM_EARLY ? rs_scratch_words(PG) : 4];
+        __shared__ __align__(16) float rs_scratch[EARLY ? rs_scratch_words(PG) : 4];
         float sum = 0.f;
-        if (PG <= NORM_EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<PG <= NORM_EARLY ? PG : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
+        if (EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<EARLY ? PG : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
         else if (tid == 0) { sum = running_sum_serial(smem_u32(v3), n4); }
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
@@ -331,13 +332,12 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
             src[i] = M.w + (size_t)(p.pair_mode ? u : R * u + i) * tile_bytes;
         }
     };
-    const uint64_t policy = l2_evict_first();
     auto issue_next = [&]() {
         const uint32_t bytes = (uint32_t)min(S, nrec - lrec) * RECB;
         const uint32_t bar = bar_s + lslot * 8, dst = ring_s + lslot * stage_bytes;
         mbar_expect_tx(bar, bytes * R);
 #pragma unroll
-        for (int i = 0; i < R; ++i) { bulk_copy_g2s_once(dst + i * S * RECB, src[i], bytes, bar, policy); src[i] += bytes; }
+        for (int i = 0; i < R; ++i) { bulk_copy_g2s(dst + i * S * RECB, src[i], bytes, bar); src[i] += bytes; }
         ++issued;
         if (++lslot == NS) { lslot = 0; }
         lrec += S;
@@ -347,8 +347,6 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
     // Let the next kernel of the step begin, and start streaming: weights never change during a step, so the
     // copies may run ahead of the previous kernel's results.
     pdl_launch_dependents();
-    float4 wearly[NORM_EARLY];
-    if (TM == 1) { norm_weights_early(p, wearly); }
     stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
     if (lane == 0 && n_items > 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(bar_s + s * 8, 1); }
@@ -367,9 +365,9 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true>(p, act, v3, norm_scales, wearly, []() {}); } else { matvec_prologue_1col<2, false>(p, act, v3, norm_scales, wearly, []() {}); }
+            if (norm) { matvec_prologue_1col<2, true, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<2, false, false>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true>(p, act, v3, norm_scales, wearly, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false>(p, act, v3, norm_scales, wearly, []() {}); }
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, false>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else {
             matvec_prologue<TM>(p, act, v3, norm_scales);
         }
@@ -579,7 +577,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
         else {
             constexpr bool NORM = PRO == MVP_NORM || PRO == MVP_NORM_MID || PRO == MVP_NORM_LONG;
             constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 2 : PRO == MVP_NORM_MID ? 3 : PRO_GROUPS;
-            matvec_prologue_1col<PG, NORM>(p, act, v3, norm_scales, wearly, rest);
+            matvec_prologue_1col<PG, NORM, NORM && PG <= NORM_EARLY>(p, act, v3, norm_scales, wearly, rest);
         }
     }
     __syncthreads();
@@ -738,12 +736,11 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_mma_kernel(const MatvecP
     const uint8_t *src = nullptr;
     int64_t lu = my_first; int lrec = 0, lslot = 0, issued = 0;
     bool    ok = true;
-    const uint64_t policy = l2_evict_first();
     auto issue_next = [&]() {
         const uint32_t bytes = (uint32_t)min(S, nrec - lrec) * RECB;
         const uint32_t bar = full_s + lslot * 8;
         mbar_expect_tx(bar, bytes);
-        bulk_copy_g2s_once(ring_s + lslot * stage_bytes, src, bytes, bar, policy);
+        bulk_copy_g2s(ring_s + lslot * stage_bytes, src, bytes, bar);
         src += bytes;
         ++issued;
         if (++lslot == NS) { lslot = 0; }
@@ -752,8 +749,6 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_mma_kernel(const MatvecP
     };
 
     pdl_launch_dependents();
-    float4 wearly[NORM_EARLY];
-    if (TM == 1) { norm_weights_early(p, wearly); }
     stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
     if (lane == 0 && n_items > 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(full_s + s * 8, 1); }
@@ -772,9 +767,9 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_mma_kernel(const MatvecP
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true>(p, act, v3, norm_scales, wearly, []() {}); } else { matvec_prologue_1col<2, false>(p, act, v3, norm_scales, wearly, []() {}); }
+            if (norm) { matvec_prologue_1col<2, true, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<2, false, false>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true>(p, act, v3, norm_scales, wearly, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false>(p, act, v3, norm_scales, wearly, []() {}); }
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, false>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else {
             matvec_prologue<TM>(p, act, v3, norm_scales);
         }
