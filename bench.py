@@ -479,7 +479,7 @@ def main():
                          "tokens_per_s": n_batch * b_steps / (model.last_ms / 1e3), "launches": int(model.last_launches),
                          "sequence0_ids_match_single_sequence_run": bool(np.array_equal(b_ids[:n_cmp, 0], ref_ids[:n_cmp])),
                          "note": "greedy decoding of the sequences in lockstep (spyb_model_decode_batch): per step the layer weights are streamed once per group of 4 sequences "
-                                 "through the mat-vec kernels (fewer than 16 sequences on one GPU), or once for all of them through the tcgen05 GEMM kernels (16 and more, "
+                                 "through the mat-vec kernels (fewer than 8 sequences on one GPU), or once for all of them through the tcgen05 GEMM kernels (8 and more, "
                                  "and every batch of a tensor-parallel model: each rank on its rows, NCCL all-gathers of the whole vectors); device time of rank 0"}
             model.select_sequence(0)
         except Exception as e:  # noqa: BLE001

@@ -133,6 +133,22 @@ __device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float4
         w[k] = (p.pro == PRO_NORM_QUANT && g < n4) ? reinterpret_cast<const float4 *>(p.norm_w)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
+// the running sum in few registers, for kernels that hold several prologues
+__device__ __forceinline__ float running_sum_small(const float *v3, int n4) {
+    const float4 *g4 = reinterpret_cast<const float4 *>(v3);
+    float sum = 0.f;
+    int g = 0;
+    for (; g + 16 <= n4; g += 16) {   // four 128-bit reads ahead of their 16 dependent adds
+        const float4 q0 = g4[(g >> 2)], q1 = g4[(g >> 2) + 1], q2 = g4[(g >> 2) + 2], q3 = g4[(g >> 2) + 3];
+        sum = __fadd_rn(sum, q0.x); sum = __fadd_rn(sum, q0.y); sum = __fadd_rn(sum, q0.z); sum = __fadd_rn(sum, q0.w);
+        sum = __fadd_rn(sum, q1.x); sum = __fadd_rn(sum, q1.y); sum = __fadd_rn(sum, q1.z); sum = __fadd_rn(sum, q1.w);
+        sum = __fadd_rn(sum, q2.x); sum = __fadd_rn(sum, q2.y); sum = __fadd_rn(sum, q2.z); sum = __fadd_rn(sum, q2.w);
+        sum = __fadd_rn(sum, q3.x); sum = __fadd_rn(sum, q3.y); sum = __fadd_rn(sum, q3.z); sum = __fadd_rn(sum, q3.w);
+    }
+    for (; g < n4; ++g) { sum = __fadd_rn(sum, v3[g]); }
+    return sum;
+}
+
 template <int PG, bool NORM, bool EARLY, class Requested>
 __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActPlanes act, float *v3, float *scales, const float4 *wearly, Requested x_requested) {
     const int tid = threadIdx.x;
@@ -173,7 +189,7 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
         __shared__ __align__(16) float rs_scratch[EARLY ? rs_scratch_words(PG) : 4];
         float sum = 0.f;
         if (EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<EARLY ? PG : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
-        else if (tid == 0) { sum = running_sum_serial(smem_u32(v3), n4); }
+        else if (tid == 0) { sum = running_sum_small(v3, n4); }
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
             scales[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
@@ -223,17 +239,7 @@ __device__ __forceinline__ void matvec_prologue(const MatvecParams &p, ActPlanes
         }
         __syncthreads();
         if (tid < p.T) {
-            const float4 *g4 = reinterpret_cast<const float4 *>(v3 + tid * n4);
-            float sum = 0.f;
-            int g = 0;
-            for (; g + 16 <= n4; g += 16) {   // four 128-bit reads ahead of their 16 dependent adds
-                const float4 q0 = g4[(g >> 2)], q1 = g4[(g >> 2) + 1], q2 = g4[(g >> 2) + 2], q3 = g4[(g >> 2) + 3];
-                sum = __fadd_rn(sum, q0.x); sum = __fadd_rn(sum, q0.y); sum = __fadd_rn(sum, q0.z); sum = __fadd_rn(sum, q0.w);
-                sum = __fadd_rn(sum, q1.x); sum = __fadd_rn(sum, q1.y); sum = __fadd_rn(sum, q1.z); sum = __fadd_rn(sum, q1.w);
-                sum = __fadd_rn(sum, q2.x); sum = __fadd_rn(sum, q2.y); sum = __fadd_rn(sum, q2.z); sum = __fadd_rn(sum, q2.w);
-                sum = __fadd_rn(sum, q3.x); sum = __fadd_rn(sum, q3.y); sum = __fadd_rn(sum, q3.z); sum = __fadd_rn(sum, q3.w);
-            }
-            for (; g < n4; ++g) { sum = __fadd_rn(sum, v3[tid * n4 + g]); }
+            const float sum = running_sum_small(v3 + tid * n4, n4);
             const float mean = __fdiv_rn(sum, (float)K);
             scales[tid] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
         }
