@@ -95,8 +95,8 @@ void        spyb_destroy(spyb_backend *backend);
  * spy_assert/std::terminate error path (util/include/util/log/logger.h:96-150) */
 const char *spyb_last_error(const spyb_backend *backend);
 
-/* Host-only self-check of the library's book-keeping (per-device shared-memory limits of the kernels); needs no GPU.
- * 0 = passed. No reference counterpart. */
+/* Host-only self-check of the library's book-keeping (per-device shared-memory limits of the kernels; which warps meet in the
+ * slots of the long-context attention kernel's ring); needs no GPU. 0 = passed. No reference counterpart. */
 int32_t spyb_selftest_host(void);
 
 /* ---- Backend::get_max/avail_memory_capacity (backend.h:46-51) */

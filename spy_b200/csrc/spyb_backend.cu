@@ -162,7 +162,8 @@ using namespace spyb;
 extern "C" {
 
 int32_t spyb_selftest_host(void) {
-    return smem_ledger_selftest();
+    const int ledger = smem_ledger_selftest();
+    return ledger != 0 ? ledger : attn_ring_selftest();
 }
 
 spyb_status spyb_create(const spyb_config *config, spyb_backend **out) {

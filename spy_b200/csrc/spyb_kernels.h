@@ -213,6 +213,7 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg);   // 
 int64_t     kq_row_bytes(int type, int64_t k);                             // bytes of one K-quant row in device memory
 cudaError_t launch_kq_relayout_q6k(const uint8_t *raw, int64_t n_rows, int64_t k, uint8_t *dst, cudaStream_t s);
 cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg);
+int         attn_ring_selftest();   // host-only: 0 when every slot of the step kernel's ring keeps its writer and its reader
 size_t      attention_scratch_floats(int n_ctx, int n_head, int T);
 
 // upload-time re-tiling of raw reference-layout blocks into DevMatrix planes

@@ -620,7 +620,14 @@ __global__ void __launch_bounds__(ATT_PV_WARPS * WARP) attn_pv_kernel(const Attn
 constexpr int ATL_C = 4, ATL_WARPS = 8, ATL_COPY_WARPS = 4, ATL_THREADS = (ATL_WARPS + ATL_COPY_WARPS) * WARP;
 constexpr int ATL_KPITCH = 272, ATL_VCH = 512, ATL_VROWS = 8, ATL_VPITCH = 2 * ATL_VCH + 64, ATL_STAGE = 32 * ATL_KPITCH;   // pitches without bank conflicts
 static_assert(ATL_VROWS * ATL_VPITCH == ATL_STAGE && ATL_C * 4 * ATL_VROWS == ATT_HD, "both kinds of stages fill the slot; four warps take a CTA's elements");
-constexpr int ATL_MAX_STAGES = 22, ATL_MIN_STAGES = 6;
+// Which warps meet in a slot of the ring: a barrier's parity tells a phase only from its neighbours, so a warp may wait for a slot's next phase
+// only when it knows the one before to be complete. Slot g % NS therefore always has the same copy warp (NS is a multiple of their number)
+// and, K stage after K stage and V stage after V stage, the same reader (NS is a multiple of the score warps, of which small rings use
+// fewer); between the two kinds lies the exchange of the exponentials, which follows every K stage.
+constexpr int ATL_MAX_STAGES = 16, ATL_MIN_STAGES = 4;   // 4, 8 or 16
+__host__ __device__ constexpr int atl_copy_warp(int g) { return g % ATL_COPY_WARPS; }
+__host__ __device__ constexpr int atl_score_warps(int ns) { return ns < ATL_WARPS ? ns : ATL_WARPS; }
+__host__ __device__ constexpr int atl_reader(int g, int nK, int ns) { return g < nK ? g % atl_score_warps(ns) : (g - nK) & 3; }
 struct AtlSmem { size_t ex, gs, rs, red, bars, ring; };   // gs: the sums of four, then the probabilities as f16
 __host__ __device__ static inline AtlSmem atl_smem(int n_ctx) {   // offsets in bytes; q lies in front
     const size_t n32 = ((size_t)n_ctx + 31) & ~(size_t)31;
@@ -692,7 +699,7 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
         const __half *K = p.k_cache + (batch ? (int64_t)t * p.seq_stride : 0) + (int64_t)start * p.dl + (int64_t)h * ATT_HD;
         const __half *V = p.v_cache + (batch ? (int64_t)t * p.seq_stride : 0) + ((int64_t)h * ATT_HD + rank * (ATT_HD / ATL_C)) * p.n_ctx;
         const int total = nK + 4 * nC;
-        for (int g = warp - ATL_WARPS; g < total; g += ATL_COPY_WARPS) {
+        for (int g = warp - ATL_WARPS; g < total; g += ATL_COPY_WARPS) {   // (atl_copy_warp)
             const int slot = g % NS;
             if (g >= NS) { atl_wait(empty_s + 8 * slot, (uint32_t)(g / NS - 1) & 1u, limit); }
             if (!__all_sync(0xffffffffu, limit != 0)) { break; }
@@ -717,7 +724,8 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
         asm volatile("bar.sync 2, 256;" ::: "memory");
         // scores of this CTA's positions, a tile of 32 per warp, a position per lane
         float m = -CUDART_INF_F;
-        for (int k = warp; k < nK; k += ATL_WARPS) {
+        const int n_score = atl_score_warps(NS);
+        for (int k = warp; warp < n_score && k < nK; k += n_score) {   // (atl_reader)
             const int slot = k % NS;
             atl_wait(full_s + 8 * slot, (uint32_t)(k / NS) & 1u, limit);
             uint4 kv[16];
@@ -733,6 +741,7 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
             m = fmaxf(m, v);
         }
         m = warp_max(m);
+        __syncwarp();   // (the warp's scores are read by others when small rings have fewer score warps)
         if (lane < ATL_C) {
             cluster_store(cluster_map(smem_u32(red + rank * ATL_WARPS + warp), lane), m);
             cluster_arrive(cluster_map(max_s, lane));
@@ -990,13 +999,34 @@ static cudaError_t launch_with_pdl(const void *kernel, dim3 grid, dim3 block, si
     return cudaLaunchKernelExC(&lc, kernel, args);
 }
 
-// the cluster kernel: single steps and batches, whole 16-byte pieces of the cache rows, at least ATL_MIN_STAGES stages beside the exponentials
-// (contexts up to some 36000 positions). One CTA per SM with a deep ring while all fit so, else two.
-static int atl_stages(const AttnParams &p, const LaunchCfg &cfg) {
-    const size_t budget = (int64_t)ATL_C * p.n_head * p.T <= cfg.num_sms ? 224 * 1024 : 112 * 1024, fixed = atl_smem(p.n_ctx).ring;
-    auto stages = [&](size_t b) { return b <= fixed ? 0 : (int)std::min<size_t>(ATL_MAX_STAGES, (b - fixed) / ATL_STAGE); };
-    const int ns = stages(budget);
-    return ns >= ATL_MIN_STAGES ? ns : stages(224 * 1024);
+// the cluster kernel: single steps and batches, whole 16-byte pieces of the cache rows, ATL_MIN_STAGES stages beside the exponentials
+// (contexts up to 31,840 positions). One CTA per SM with a deep ring while all fit so, else two with eight stages each where they fit.
+static int atl_stage_count(int n_ctx, int64_t ctas, int num_sms) {
+    const size_t fixed = atl_smem(n_ctx).ring;
+    auto stages = [&](size_t b) {
+        for (int ns = ATL_MAX_STAGES; ns >= ATL_MIN_STAGES; ns /= 2) { if (fixed + (size_t)ns * ATL_STAGE <= b) { return ns; } }
+        return 0;
+    };
+    const int ns = stages(ctas <= num_sms ? 224 * 1024 : 112 * 1024);
+    return ns >= 8 ? ns : stages(224 * 1024);
+}
+static int atl_stages(const AttnParams &p, const LaunchCfg &cfg) { return atl_stage_count(p.n_ctx, (int64_t)ATL_C * p.n_head * p.T, cfg.num_sms); }
+// host-only: 0 when, for every ring that the rule above gives, a slot's successive stages have one copy warp and, within K and within V, one reader
+int attn_ring_selftest() {
+    for (int ctas = 4; ctas <= 4096; ctas *= 8) {
+        for (int n_ctx = 8; n_ctx <= 40000; n_ctx += 8) {
+            const int ns = atl_stage_count(n_ctx, ctas, 140);
+            if (ns == 0) { continue; }
+            if (ns > ATL_MAX_STAGES || atl_smem(n_ctx).ring + (size_t)ns * ATL_STAGE > 224 * 1024) { return 101; }
+            for (int nK = 0; nK <= 2 * ns; ++nK) {
+                for (int g = 0; g < nK + 3 * ns; ++g) {
+                    if (atl_copy_warp(g) != atl_copy_warp(g + ns)) { return 102; }
+                    if ((g < nK) == (g + ns < nK) && atl_reader(g, nK, ns) != atl_reader(g + ns, nK, ns)) { return 103; }
+                }
+            }
+        }
+    }
+    return 0;
 }
 static bool atl_fits(const AttnParams &p, const LaunchCfg &cfg) {
     return (p.T < ATT_TT || p.seq_stride != 0) && p.tp.counter == nullptr && (p.n_ctx & 7) == 0 && (p.seq_stride & 7) == 0 &&

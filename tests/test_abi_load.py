@@ -38,3 +38,10 @@ def test_shared_memory_ledger_is_kept_per_device_and_kernel():
     """cudaFuncAttributeMaxDynamicSharedMemorySize belongs to a (device, kernel) pair: the library's record of what it
     has already raised must be kept per pair, or the second device of a process never gets the attribute set."""
     assert backend.lib().spyb_selftest_host() == 0
+
+
+def test_attention_ring_slots_keep_their_warps():
+    """The ring of the long-context attention kernel, for all contexts and numbers of CTAs: a slot's successive stages come from one copy warp
+    and go to one reader, or a wait by parity could take a phase for the one two before it (stages overwritten while they are read, or a
+    wait that never ends)."""
+    assert backend.lib().spyb_selftest_host() == 0

@@ -237,6 +237,41 @@ def test_batch_of_sequences_equals_single_sequence_runs(n_seq, n_ctx, kq, oracle
     m.close(); b.close()
 
 
+@pytest.mark.parametrize("n_seq,n_ctx", [(3, 1104), (9, 2048), (21, 2048)])
+def test_batch_over_a_long_context(n_seq, n_ctx, oracle, tmp_models):
+    """Batches whose contexts are long enough for the cluster attention kernel and its ring to go round: on the mat-vec passes, on the GEMMs, and
+    with more CTAs than SMs (two per SM, the smaller ring). The first and the last sequence against the oracle, the others against the same
+    sequence decoded alone in a context the kernel does not take (no multiple of eight: the three-kernel attention)."""
+    cfg = gguf_io.LlamaConfig(n_layer=1, d_model=256, n_head=2, n_ff=512, n_vocab=400, weight_std=0.06)
+    path = str(tmp_models / "batch_long.gguf")
+    if not os.path.exists(path):
+        gguf_io.make_llama_gguf(path, cfg, seed=67)
+    rng = np.random.default_rng(n_seq)
+    n_prompt, n_steps = n_ctx - 48, 12
+    prompts = [rng.integers(3, cfg.n_vocab, size=n_prompt) for _ in range(n_seq)]
+    b = B.B200Backend(0)
+    alone = B.LlamaModel(b, path, n_ctx=n_ctx - 4)
+    m = B.LlamaModel(b, path, n_ctx=n_ctx)
+    m.set_sequences(n_seq)
+    first, want = [], []
+    for c, p in enumerate(prompts):
+        if c in (0, n_seq - 1):
+            ids, logits = oracle.OracleLlama(path, n_ctx=n_ctx).generate(p, n_steps + 1)
+        else:
+            ids, logits = alone.generate(p, n_steps + 1)
+        want.append((ids, logits))
+        m.select_sequence(c)
+        lg = m.eval(p, 0)
+        assert np.array_equal(lg.view(np.uint32), logits[0].view(np.uint32)), c
+        first.append(int(ids[0]))
+    for _ in range(3):
+        ids, logits = m.decode_batch(first, n_prompt, n_steps, want_logits=True)
+        for c in range(n_seq):
+            assert np.array_equal(ids[:, c], want[c][0][1:]), c
+            assert np.array_equal(np.ascontiguousarray(logits[:, c]).view(np.uint32), want[c][1][1:].view(np.uint32)), c
+    m.close(); alone.close(); b.close()
+
+
 def test_long_context_attention(be, oracle, tmp_models):
     """A 600-token prompt in a 1024-token context: many 32-wide accumulator steps and ragged tails in both
     attention products."""

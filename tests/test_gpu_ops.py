@@ -607,10 +607,12 @@ def test_attention_of_a_prompt_across_its_tiles(be, oracle, pos0, t, n_total, n_
 
 
 @pytest.mark.parametrize("pos0,t,n_total,n_ctx,n_head", [(0, 1, 1, 1032, 2), (31, 1, 32, 1032, 1), (32, 1, 33, 1032, 1), (127, 1, 128, 1032, 2), (511, 1, 512, 1032, 1),
-                                                         (512, 1, 513, 2048, 2), (1400, 3, 1403, 1408, 2), (4090, 1, 4091, 4096, 2), (2990, 7, 2997, 3000, 6), (700, 2, 740, 4104, 1)])
+                                                         (512, 1, 513, 2048, 2), (1400, 3, 1403, 1408, 2), (4090, 1, 4091, 4096, 2), (2990, 7, 2997, 3000, 6), (700, 2, 740, 4104, 1),
+                                                         (5000, 1, 5001, 16384, 1), (2500, 3, 2503, 8192, 12), (4100, 1, 4101, 28000, 1), (600, 1, 601, 31840, 1), (600, 1, 601, 31848, 1)])
 def test_attention_of_a_step_over_a_long_context(be, oracle, pos0, t, n_total, n_ctx, n_head):
     """One to seven tokens in a context above 1024 positions: fewer positions than the CTAs of a head, ends on and beside the 32-position tiles and the
-    512-position stages, rings that wrap, the smaller ring of many CTAs, masked positions behind the last token."""
+    512-position stages, rings of sixteen, eight and four stages that wrap, the smaller ring of many CTAs, the longest context whose ring fits and the one
+    behind it, masked positions behind the last token."""
     rng = np.random.default_rng(pos0 + t)
     d = n_head * 128
     q16 = oracle.quantize_f16(rng.standard_normal(t * d).astype(np.float32)).reshape(t, d)
