@@ -556,6 +556,9 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
             tiles = static_cast<uint8_t *>(raw);
             if (n_rows % PF_ROWS != 0) { SPYB_CUDA(be, cudaMemsetAsync(tiles, 0, wbytes, be->stream)); }   // (rows that pad the last tile stay zero)
             SPYB_CUDA(be, launch_prefill_retile(type, static_cast<const uint8_t *>(w.data), rb, n_rows, nb, tiles, 0, be->stream));
+            // The GEMM copies its first weights before it waits for the kernels in front of it, whichever thread enqueues it: the tiles are
+            // finished before anyone can find them
+            SPYB_CUDA(be, cudaStreamSynchronize(be->stream));
             be->pf_tiles[w.data] = tiles;
         }
     }

@@ -2,6 +2,7 @@
 Integer and byte results must be identical; f32 results differ only by summation order."""
 import ctypes as C
 import os
+import threading
 
 import numpy as np
 import pytest
@@ -294,6 +295,39 @@ def test_matmul_on_uploaded_constants_takes_the_model_kernels(be, oracle, qt, n,
         got = be.download(po, (t, n), np.float32)
         be.dealloc_memory(px, x.nbytes); be.dealloc_memory(po, n * t * 4)
         assert np.array_equal(bits(got), bits(want))
+
+
+@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0, quants.Q4_K, quants.Q6_K])
+def test_first_gemm_submit_of_a_constant_reads_finished_tiles(be, oracle, qt):
+    """The submit that makes a constant's tile copy and the ones right behind it, from two threads, against the oracle on a row sample: the
+    GEMM reads its first weights ahead of the kernels in front of it, so the copy has to be complete before any GEMM is enqueued."""
+    n, k, t = 19072, 1024, 16
+    rng = np.random.default_rng(qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    rows = np.unique(np.r_[0, n - 1, rng.integers(0, n, 60)])
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    want = oracle.matmul(qt, np.ascontiguousarray(w[rows]), k, len(rows), x)
+    px = be.upload(x)
+    for i in range(4):
+        pw, po = be.upload_constant(f"first_{qt}_{i}", w.copy(), qt, (k, n)), [be.alloc_memory(4 * n * t) for _ in range(2)]
+
+        def one(p):
+            d = B.OpDesc(); d.op_type, d.num_input = B.OP["MatMul"], 2
+            d.input[0] = B.make_tensor(pw, qt, (k, n), None, B.NODE_CONSTANT)
+            d.input[1] = B.make_tensor(px, B.FP32, (k, t))
+            d.output = B.make_tensor(p, B.FP32, (n, t))
+            be.submit(d)
+
+        threads = [threading.Thread(target=one, args=(p,)) for p in po]
+        for th in threads:
+            th.start()
+        for th in threads:
+            th.join()
+        be.sync()
+        for p in po:
+            assert np.array_equal(bits(be.download(p, (t, n), np.float32)[:, rows]), bits(want))
+            be.dealloc_memory(p, 4 * n * t)
+    be.dealloc_memory(px, x.nbytes)
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
