@@ -875,7 +875,7 @@ __global__ void __launch_bounds__(ATT_PVT_WARPS * WARP, 16 / ATT_PVT_WARPS) attn
 #pragma unroll
         for (int ee = 0; ee < ATT_EE; ++ee) {
             dst[ee] = make_uint2(0u, 0u);
-            if (step < n_steps && j < vis_last) { dst[ee] = __ldg(reinterpret_cast<const uint2 *>(vrow + (int64_t)ee * p.n_ctx + j)); }
+            if (step < n_steps && j < vis_last) { dst[ee] = *reinterpret_cast<const uint2 *>(vrow + (int64_t)ee * p.n_ctx + j); }   // (a plain load: this kernel may be resident before the cache rows of its prompt are written)
         }
     };
 #pragma unroll

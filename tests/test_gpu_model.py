@@ -186,6 +186,22 @@ def test_prompt_on_the_tensor_cores(env, wtype, oracle, tmp_models, monkeypatch)
     m.close(); m2.close(); b.close()
 
 
+def test_prompts_of_a_reused_cache_read_their_own_rows(tmp_models):
+    """Prompts one after the other over the same cache, their kernels launched ahead of their predecessors' ends: each attention pass must read
+    the K and V^T rows its own prompt has just written, not what the cache held before. Same bits as with plain launches."""
+    cfg = gguf_io.LlamaConfig(n_layer=2, d_model=512, n_head=4, n_ff=640, n_vocab=500, weight_std=0.05)
+    path = str(tmp_models / "reused_cache.gguf")
+    gguf_io.make_llama_gguf(path, cfg, seed=71)
+    prompts = np.random.default_rng(10).integers(3, cfg.n_vocab, size=(6, 1400))
+    got = []
+    for pdl in (True, False):
+        b = B.B200Backend(0, use_pdl=pdl)
+        m = B.LlamaModel(b, path, n_ctx=1536)
+        got.append(np.array([m.eval(p, 0) for p in prompts]))
+        m.close(); b.close()
+    assert np.isfinite(got[0]).all() and np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
+
+
 def test_prompt_widths_the_gemm_tile_does_not_divide(be, oracle, tmp_models):
     """n_ff = 416 is no multiple of the 128-row GEMM tile (the stacked up|gate matrix has 832 rows: the last tile is half
     padding, and W_gate starts in the middle of a tile): the padded rows are neither computed into anything nor stored."""
