@@ -1061,7 +1061,9 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
     const size_t n_pad = ((size_t)p.n_ctx + 3) & ~(size_t)3;
     if ((p.n_ctx > ATT_LONG_MIN || p.force_long) && p.scratch != nullptr) {
         if (atl_fits(p, cfg)) { return launch_attn_cluster(p, cfg); }
-        const bool tiled = p.T >= ATT_TT && p.tp.counter == nullptr && p.seq_stride == 0;   // a prompt: tokens share the K rows and the V^T rows
+        // a prompt: tokens share the K rows and the V^T rows, read in pieces of 16 (K, Q) and 8 bytes (V^T); Q and V^T of any other alignment go
+        // through the kernels that read them value by value
+        const bool tiled = p.T >= ATT_TT && p.tp.counter == nullptr && p.seq_stride == 0 && ((uintptr_t)p.q & 15) == 0 && ((uintptr_t)p.v_cache & 7) == 0;
         cudaError_t err = tiled ? allow_dynamic_smem(reinterpret_cast<const void *>(attn_scores_tiled_kernel), ATT_SC_SMEM) : cudaSuccess;
         if (err != cudaSuccess) { return err; }
         err = tiled

@@ -640,6 +640,24 @@ def test_attention_of_a_prompt_across_its_tiles(be, oracle, pos0, t, n_total, n_
     assert np.array_equal(bits(got), bits(want))
 
 
+@pytest.mark.parametrize("t", [9, 3])
+@pytest.mark.parametrize("q_off,v_off", [(2, 0), (0, 2), (0, 4), (8, 8), (16, 8)])
+def test_attention_takes_q_and_v_of_any_alignment(be, oracle, t, q_off, v_off):
+    """Q and V^T at addresses that only halves are aligned to: views into larger buffers, as before the tiled kernels read them in wider pieces."""
+    rng = np.random.default_rng(q_off + v_off)
+    n_head, n_ctx, pos0 = 1, 1032, 70
+    q16 = oracle.quantize_f16(rng.standard_normal(t * 128).astype(np.float32)).reshape(t, 128)
+    k16 = oracle.quantize_f16(rng.standard_normal(n_ctx * 128).astype(np.float32)).reshape(n_ctx, 128)
+    vt16 = oracle.quantize_f16(rng.standard_normal(n_ctx * 128).astype(np.float32)).reshape(128, n_ctx)
+    shift = lambda a, off: np.concatenate([np.zeros(off // 2, dtype=np.uint16), a.ravel()])
+    pq, pk, pv, po = be.upload(shift(q16, q_off)), be.upload(k16), be.upload(shift(vt16, v_off)), be.alloc_memory(t * 128 * 4)
+    be._check(be._l.spyb_attention(be.h, pq + q_off, pk, pv + v_off, po, pos0, t, pos0 + t, n_head, 128, n_ctx))
+    got = be.download(po, (t, 128), np.float32)
+    for p, n in ((pq, q16.nbytes + q_off), (pk, k16.nbytes), (pv, vt16.nbytes + v_off), (po, t * 128 * 4)):
+        be.dealloc_memory(p, n)
+    assert np.array_equal(bits(got), bits(_attention_oracle(oracle, q16, k16, vt16, pos0, n_head, 128, n_ctx, pos0 + t)))
+
+
 @pytest.mark.parametrize("pos0,t,n_total,n_ctx,n_head", [(0, 1, 1, 1032, 2), (31, 1, 32, 1032, 1), (32, 1, 33, 1032, 1), (127, 1, 128, 1032, 2), (511, 1, 512, 1032, 1),
                                                          (512, 1, 513, 2048, 2), (1400, 3, 1403, 1408, 2), (4090, 1, 4091, 4096, 2), (2990, 7, 2997, 3000, 6), (700, 2, 740, 4104, 1),
                                                          (5000, 1, 5001, 16384, 1), (2500, 3, 2503, 8192, 12), (4100, 1, 4101, 28000, 1), (600, 1, 601, 31840, 1), (600, 1, 601, 31848, 1)])
