@@ -156,10 +156,9 @@ template <int I> __device__ __forceinline__ float kq_byte_magic(uint32_t w) { re
 template <int TM, int NW>
 __device__ __forceinline__ void kq_values_q4k(const uint4 (&w)[NW], uint32_t rec_s, uint32_t col_bytes, float (&acc)[TM]) {
     const float2 dm = __half22float2(*reinterpret_cast<const __half2 *>(&w[0].x));   // d, dmin
-    // the eight 6-bit scales and minima, four to a word; d * sc in one operation: fma(d, 2^23 + sc, -(d * 2^23)) rounds the exact product once
+    // the eight 6-bit scales and minima, four to a word
     const uint32_t scw[2] = {w[0].y & 0x3f3f3f3fu, (w[0].w & 0x0f0f0f0fu) | ((w[0].y >> 2) & 0x30303030u)};
     const uint32_t mnw[2] = {w[0].z & 0x3f3f3f3fu, ((w[0].w >> 4) & 0x0f0f0f0fu) | ((w[0].z >> 2) & 0x30303030u)};
-    const float dbase = __fmul_rn(dm.x, -8388608.f), mbase = __fmul_rn(dm.y, 8388608.f);
 #pragma unroll
     for (int t = 0; t < TM; ++t) { acc[t] = 0.f; }
 #pragma unroll
@@ -172,7 +171,8 @@ __device__ __forceinline__ void kq_values_q4k(const uint4 (&w)[NW], uint32_t rec
         const uint32_t sw = scw[jp >> 1], mw = mnw[jp >> 1];
         const float s0 = (jp & 1) ? kq_byte_magic<2>(sw) : kq_byte_magic<0>(sw), s1 = (jp & 1) ? kq_byte_magic<3>(sw) : kq_byte_magic<1>(sw);
         const float m0 = (jp & 1) ? kq_byte_magic<2>(mw) : kq_byte_magic<0>(mw), m1 = (jp & 1) ? kq_byte_magic<3>(mw) : kq_byte_magic<1>(mw);
-        const float dsc[2] = {fmaf(dm.x, s0, dbase), fmaf(dm.x, s1, dbase)}, dmn[2] = {fmaf(-dm.y, m0, mbase), fmaf(-dm.y, m1, mbase)};   // (dmn: negated)
+        // (2^23 is taken off before the product, not with it: an infinite d would meet its own opposite)
+        const float dsc[2] = {__fmul_rn(dm.x, s0 - 8388608.f), __fmul_rn(dm.x, s1 - 8388608.f)}, dmn[2] = {__fmul_rn(-dm.y, m0 - 8388608.f), __fmul_rn(-dm.y, m1 - 8388608.f)};   // (dmn: negated)
 #pragma unroll
         for (int t = 0; t < TM; ++t) {
             {

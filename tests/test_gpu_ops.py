@@ -349,6 +349,32 @@ def test_k_quant_mat_vec_units_and_rounds(be, oracle, qt, n, k, t):
     assert np.array_equal(bits(got), bits(oracle.matmul(qt, w, k, n, x)))
 
 
+@pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
+@pytest.mark.parametrize("t", [1, 2, 4, 16])
+def test_k_quant_scales_beyond_the_half_range(be, oracle, qt, t):
+    """Super-blocks whose f16 scale (or minimum) is infinite, as files written from very large weights hold: infinities where the restatement has
+    them, NaN where it has NaN, on the mat-vec kernel and on the GEMM."""
+    n, k = 64, 768
+    rng = np.random.default_rng(t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    blocks = w.view(np.uint8).reshape(n, k // 256, -1)
+    at = {quants.Q4_K: (0, 2), quants.Q6_K: (208,)}[qt]
+    for row, (off, half) in enumerate([(o, h) for o in at for h in (0x7c00, 0xfc00)]):
+        blocks[8 * row, 1, off:off + 2] = np.frombuffer(np.uint16(half).tobytes(), dtype=np.uint8)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    pw, px, po = be.upload_constant(f"inf_{qt}_{t}", w, qt, (k, n)), be.upload(x), be.alloc_memory(4 * n * t)
+    d = B.OpDesc()
+    d.op_type, d.num_input = B.OP["MatMul"], 2
+    d.input[0] = B.make_tensor(pw, qt, (k, n), None, B.NODE_CONSTANT)
+    d.input[1] = B.make_tensor(px, B.FP32, (k, t))
+    d.output = B.make_tensor(po, B.FP32, (n, t))
+    be.submit(d); be.sync()
+    got, want = be.download(po, (t, n), np.float32), oracle.matmul(qt, w, k, n, x)
+    nan = np.isnan(want)
+    assert (~np.isfinite(want)).any() and np.array_equal(np.isnan(got), nan)
+    assert np.array_equal(bits(got[~nan]), bits(want[~nan]))
+
+
 def test_matmul_linearity_full_size(be):
     """Size-independent property at the 7B head shape: W(2x) == 2 W(x) exactly (power-of-two scaling commutes with Q8_0)."""
     rng = np.random.default_rng(5)
