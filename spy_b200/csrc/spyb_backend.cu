@@ -521,6 +521,21 @@ void stage_release(spyb_backend *be, Staged *s) {
     s->dev = nullptr; s->temp = false;
 }
 
+// Whether two passes of the mat-vec kernels (five to eight columns) take less time than the GEMM. A GEMM CTA walks all of K for its 128 rows:
+// one round of tiles costs about the same however many rows it has, while a pass grows with rows, K and columns (the second pass runs on
+// a kernel for 1, 2 or 4). Planes through measurements at 512 to 8192 rows, K of 1536 to 11008, in us, K and rows in thousands (a pass
+// gets no shorter below 2048 rows, a tile's weights come faster there); within 10 % of the better one throughout, 0.3 % on average.
+// Q4_0 with 5, 6, 8 columns: 4096 x 4096 22.6, 24.7, 28.7 against 23.6; 4096 x 8192 35.5, 37.1, 45.4 against 43.0; 2048 x 8192 29.9, 30.9, 37.1
+// against 41.9; 8192 x 4096 30.9, 32.9, 39.0 against 24.8. From nine columns (three passes) or 74 tiles on, the GEMM.
+bool matvec_passes_win(int type, int64_t n_rows, int64_t k, int T) {
+    struct Plane { double m0, mk, mr, mc, mrc, g0, gk, gr; };
+    static const Plane q0 = {12.5, 1.09, 0.373, 0.197, 0.055, 2.9, 3.51, 0.738}, q4k = {13.0, 0.49, 0.356, 0.183, 0.060, 3.9, 3.22, 0.349}, q6k = {14.9, 0.24, 0.525, 0.203, 0.088, 3.6, 3.15, 0.386};
+    if (T > 8 || (n_rows + PF_ROWS - 1) / PF_ROWS >= 74) { return false; }
+    const Plane &l = type == SPYB_Q4_K ? q4k : type == SPYB_Q6_K ? q6k : q0;
+    const double K = (double)k / 1000.0, R = (double)n_rows / 1000.0, Rm = std::max(R, 2.048), Rg = std::min(R, 2.048), c = T <= 6 ? T - 4 : 4;
+    return l.m0 + K * (l.mk + l.mr * Rm + c * (l.mc + l.mrc * Rm)) < l.g0 + K * (l.gk + l.gr * Rg);
+}
+
 // MatMul of several activation columns against an uploaded constant: the tcgen05 GEMM of the prompt path (same bits as
 // the mat-vec kernels). The matrix gets a second copy in that kernel's tile layout at first use, kept with the constant.
 // Returns SPYB_UNSUPPORTED without an error text when the operands do not qualify (the caller then takes the mat-vec route).
@@ -534,9 +549,7 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
         (reinterpret_cast<uintptr_t>(x.data) & 15) || (reinterpret_cast<uintptr_t>(out_dev) & 3)) {
         return SPYB_UNSUPPORTED;
     }
-    // Two passes of the mat-vec kernels (up to eight columns) are faster only for long rows of a matrix that leaves half the SMs without a
-    // tile: a GEMM CTA walks all of K (4096 x 11008 x 6 columns: 57 us against 47; 4096 x 4096: 19 against 25; 11008 x 4096: 24 against 39)
-    if (T <= 8 && k > 8192 && (n_rows + PF_ROWS - 1) / PF_ROWS < 74) { return SPYB_UNSUPPORTED; }
+    if (T <= 8 && matvec_passes_win(type, n_rows, k, (int)T)) { return SPYB_UNSUPPORTED; }
     static const bool off = [] { const char *e = std::getenv("SPYB_PREFILL"); return e != nullptr && e[0] == '0'; }();
     if (off) { return SPYB_UNSUPPORTED; }
     const int nb = (int)(k / QK);

@@ -274,12 +274,12 @@ def test_matmul_operator_sweep(be, oracle, qt, n, k, t):
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0, quants.Q4_K, quants.Q6_K])
-@pytest.mark.parametrize("n,k,t", [(132, 512, 1), (132, 512, 5), (200, 1024, 16), (260, 2816, 41), (1100, 512, 150)])
+@pytest.mark.parametrize("n,k,t", [(132, 512, 1), (132, 512, 5), (200, 1024, 16), (260, 2816, 41), (1100, 512, 150), (132, 8192, 5), (64, 11008, 7), (2052, 6144, 8), (64, 8192, 9)])
 def test_matmul_on_uploaded_constants_takes_the_model_kernels(be, oracle, qt, n, k, t):
     """MatMul through spyb_submit against a constant from spyb_upload_constant: K-quant constants run the K-quant mat-vec
-    kernel in passes of four columns, and 16 columns and more run the tcgen05 GEMM against a tile copy made at first use (K-quants
-    always, Q4_0 / Q8_0 when rows x columns give the GEMM enough tiles: the last case). Either way the oracle's bits (for
-    K-quants: the restatement's)."""
+    kernel in passes of four columns, nine columns and more run the tcgen05 GEMM against a tile copy made at first use, five to eight
+    columns whichever of the two is faster (long rows of a low matrix: two mat-vec passes). Either way the oracle's bits (for K-quants:
+    the restatement's)."""
     rng = np.random.default_rng(n + k + t + qt)
     w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
     x = rng.standard_normal((t, k)).astype(np.float32)
