@@ -509,7 +509,10 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg) {
             {matvec_kq_kernel<1, 12, KQP_PLAIN_LONG>, matvec_kq_kernel<1, 14, KQP_PLAIN_LONG>, matvec_kq_kernel<1, 0, KQP_PLAIN_LONG>}};
         const int64_t n4 = p.A.k >> 2;
         const bool norm = p.pro == PRO_NORM_QUANT;
-        kernel = one[n4 <= 2 * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : norm && n4 <= 3 * KQ_THREADS ? KQP_NORM_MID : n4 <= KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY][ty];
+        // (narrow models: a layer's matrices of both types on one kernel, whose instructions the next launch finds in the caches; four layers of
+        // Q4_K / Q6_K with d = 512, ff 1536: 125.2 -> 105.7 us a step; 1024, 2816: 129.3 -> 109.8; 2048, 5632: 137.0 -> 133.8; 3072, 8192: 188.2 ->
+        // 186.9; but 4096, 11008: 227.2 -> 235.9)
+        kernel = p.narrow ? one[KQP_ANY][2] : one[n4 <= 2 * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : norm && n4 <= 3 * KQ_THREADS ? KQP_NORM_MID : n4 <= KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY][ty];
     } else {
         static const Kernel more[2][3] = {{matvec_kq_kernel<2, 12, KQP_ANY>, matvec_kq_kernel<2, 14, KQP_ANY>, matvec_kq_kernel<2, 0, KQP_ANY>},
                                           {matvec_kq_kernel<KQ_MAX_COLUMNS, 12, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 14, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 0, KQP_ANY>}};

@@ -120,10 +120,12 @@ cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
 // Single column, K <= 12288: every thread keeps its (at most PG) float4 groups of x in registers from the one
 // global read through the sum of squares to the quantizer; same arithmetic as the general prologue below.
 constexpr int PRO_GROUPS = 6;
-// EARLY (kernels of their own per prologue only: elsewhere its registers cost the other paths): the sum of squares runs on four warps and the
+// SUM: how the sum of squares is formed. SUM_FEW: by one thread in few registers (kernels with other paths to serve); SUM_CHAIN: by one thread
+// that reads ahead; SUM_WIDE (kernels of their own per prologue): the sum of squares runs on four warps and the
 // norm weights of rows of at most NORM_EARLY * 512 groups are read at the start of the kernel, in front of the weight copies: behind a ring
 // full of them on every SM they arrive after the sum of squares is done.
 constexpr int NORM_EARLY = 3;
+enum { SUM_FEW, SUM_CHAIN, SUM_WIDE };
 template <int PG>
 __device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float4 (&w)[PG]) {
     const int n4 = (int)(p.A.k >> 2);
@@ -149,8 +151,9 @@ __device__ __forceinline__ float running_sum_small(const float *v3, int n4) {
     return sum;
 }
 
-template <int PG, bool NORM, bool EARLY, class Requested>
+template <int PG, bool NORM, int SUM, class Requested>
 __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActPlanes act, float *v3, float *scales, const float4 *wearly, Requested x_requested) {
+    constexpr bool EARLY = SUM == SUM_WIDE;
     const int tid = threadIdx.x;
     const int nbp = p.A.nbp;
     const int n4  = (int)(p.A.k >> 2);
@@ -189,7 +192,7 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
         __shared__ __align__(16) float rs_scratch[EARLY ? rs_scratch_words(PG) : 4];
         float sum = 0.f;
         if (EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<EARLY ? PG : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
-        else if (tid == 0) { sum = running_sum_small(v3, n4); }
+        else if (tid == 0) { sum = SUM == SUM_CHAIN ? running_sum_serial(smem_u32(v3), n4) : running_sum_small(v3, n4); }
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
             scales[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
@@ -371,9 +374,9 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<2, false, false>(p, act, v3, norm_scales, nullptr, []() {}); }
+            if (norm) { matvec_prologue_1col<2, true, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<2, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, false>(p, act, v3, norm_scales, nullptr, []() {}); }
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else {
             matvec_prologue<TM>(p, act, v3, norm_scales);
         }
@@ -510,7 +513,10 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
 // number of columns.
 // (One kernel with all of them takes 121 registers instead of 79 and its loop is scheduled worse. A Q4_0 layer of a 7B step, with the
 // evict-first copies, the early norm weights and the late ring: 49.1 -> 43.7 us.)
-enum { MVP_ANY, MVP_NORM, MVP_NORM_MID, MVP_PLAIN, MVP_NORM_LONG, MVP_PLAIN_LONG };
+// MVP_ONE: any single column, for narrow models: a layer's four matrices on one kernel. There a launch is short, and the next one finding its
+// instructions in the caches is worth more than a better loop (four layers of d = 512, ff 5632, Q4_0: 102.3 -> 94.1 us a step; 1024, 2816:
+// 99.6 -> 93.5; 2048, 5632: 121.4 -> 117.7; 3072, 8192: 158.1 -> 153.8; but 4096, 11008: 188.2 -> 190.9).
+enum { MVP_ANY, MVP_NORM, MVP_NORM_MID, MVP_PLAIN, MVP_NORM_LONG, MVP_PLAIN_LONG, MVP_ONE };
 template <int WT, int TM, int LPR, int PRO>
 __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const MatvecParams p, const int ring_bytes, const int S, const int wact) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -580,10 +586,18 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     {
         float *v3 = reinterpret_cast<float *>(smem_raw);
         if constexpr (PRO == MVP_ANY) { matvec_prologue<TM>(p, act, v3, norm_scales); }
+        else if constexpr (PRO == MVP_ONE) {
+            const bool norm = p.pro == PRO_NORM_QUANT;
+            if (nbp * 8 <= 2 * MV_THREADS) {
+                if (norm) { matvec_prologue_1col<2, true, SUM_CHAIN>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<2, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, rest); }
+            } else {
+                if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_CHAIN>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, rest); }
+            }
+        }
         else {
             constexpr bool NORM = PRO == MVP_NORM || PRO == MVP_NORM_MID || PRO == MVP_NORM_LONG;
             constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 2 : PRO == MVP_NORM_MID ? 3 : PRO_GROUPS;
-            matvec_prologue_1col<PG, NORM, NORM && PG <= NORM_EARLY>(p, act, v3, norm_scales, wearly, rest);
+            matvec_prologue_1col<PG, NORM, NORM && PG <= NORM_EARLY ? SUM_WIDE : SUM_FEW>(p, act, v3, norm_scales, wearly, rest);
         }
     }
     __syncthreads();
@@ -773,9 +787,9 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_mma_kernel(const MatvecP
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<2, false, false>(p, act, v3, norm_scales, nullptr, []() {}); }
+            if (norm) { matvec_prologue_1col<2, true, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<2, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, false>(p, act, v3, norm_scales, nullptr, []() {}); }
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else {
             matvec_prologue<TM>(p, act, v3, norm_scales);
         }
@@ -914,7 +928,8 @@ static cudaError_t launch_matvec_rows_t(const MatvecParams &p, const LaunchCfg &
     if constexpr (TM == 1) {
         const int  n4p = p.A.nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
-        if (n4p <= 2 * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN>; }
+        if (p.narrow && n4p <= PRO_GROUPS * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_ONE>; }
+        else if (n4p <= 2 * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN>; }
         else if (norm && n4p <= 3 * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_NORM_MID>; }
         else if (n4p <= PRO_GROUPS * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM_LONG> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN_LONG>; }
     }

@@ -405,9 +405,10 @@ def test_step_kernel_wait_runs_out_and_is_reported(oracle, tmp_models, monkeypat
     m.close(); b.close()
 
 
-@pytest.mark.parametrize("d,wtype", [(4352, quants.Q4_K), (5120, quants.Q4_0), (5120, quants.Q4_K), (6144, quants.Q8_0)])
+@pytest.mark.parametrize("d,wtype", [(2176, quants.Q8_0), (3072, quants.Q4_0), (3200, quants.Q4_0), (4096, quants.Q8_0),
+                                     (4352, quants.Q4_K), (5120, quants.Q4_0), (5120, quants.Q4_K), (6144, quants.Q8_0)])
 def test_steps_of_widths_between_the_prologues(be, oracle, tmp_models, d, wtype):
-    """Rows of more than 1024 and at most 1536 groups of four: single steps with the norm in front, whose sum of squares runs in chunks of twelve values
+    """Both sides of the width up to which a layer's matrices share one kernel, and rows of more than 1024 and at most 1536 groups of four: single steps with the norm in front, whose sum of squares runs in chunks of twelve values
     (4352 with K-quants: too little scratch beside the records, the plain chain)."""
     cfg = gguf_io.LlamaConfig(n_layer=1, d_model=d, n_head=d // 128, n_ff=512, n_vocab=64, wtype=wtype, embd_type=quants.Q8_0)
     path = str(tmp_models / f"mid{d}_{wtype}.gguf")
