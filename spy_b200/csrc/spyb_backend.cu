@@ -40,7 +40,7 @@ void *Arena::alloc(size_t bytes) {
         }
     }
     void *p = nullptr;   // arena exhausted: fall back to the CUDA allocator rather than fail
-    if (cudaMalloc(&p, need) != cudaSuccess) { return nullptr; }
+    if (cudaMalloc(&p, need) != cudaSuccess) { cudaGetLastError(); return nullptr; }   // (not left for the next launch to find)
     overflow_[p] = need;
     return p;
 }
@@ -538,7 +538,7 @@ bool matvec_passes_win(int type, int64_t n_rows, int64_t k, int T) {
 
 // MatMul of several activation columns against an uploaded constant: the tcgen05 GEMM of the prompt path (same bits as
 // the mat-vec kernels). The matrix gets a second copy in that kernel's tile layout at first use, kept with the constant.
-// Returns SPYB_UNSUPPORTED without an error text when the operands do not qualify (the caller then takes the mat-vec route).
+// Returns SPYB_UNSUPPORTED without an error text when the operands do not qualify or the memory is not there (the caller then takes the mat-vec route).
 spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_tensor &x, void *out_dev) {
     const int type = w.number_type;
     const bool kq = type == SPYB_Q4_K || type == SPYB_Q6_K;
@@ -564,7 +564,7 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
             const int64_t rb = kq ? (k / 256) * (type == SPYB_Q4_K ? 144 : 210) : (int64_t)nb * (type == SPYB_Q4_0 ? 18 : 34);
             const size_t wbytes = prefill_weight_bytes(type, n_rows, nb);
             void *raw = nullptr;
-            SPYB_CUDA(be, cudaMalloc(&raw, wbytes));
+            if (cudaMalloc(&raw, wbytes) != cudaSuccess) { cudaGetLastError(); return SPYB_UNSUPPORTED; }   // no room for the copy: the mat-vec kernels need none
             be->owned.push_back(raw);
             tiles = static_cast<uint8_t *>(raw);
             if (n_rows % PF_ROWS != 0) { SPYB_CUDA(be, cudaMemsetAsync(tiles, 0, wbytes, be->stream)); }   // (rows that pad the last tile stay zero)
@@ -578,7 +578,7 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
     const int64_t chunk = 1024;
     const size_t ybytes = prefill_act_bytes((int)std::min(chunk, T), nb);
     void *yq = be->arena.alloc(ybytes);
-    if (yq == nullptr) { be->set_error("MatMul: out of device memory for the quantized activations"); return SPYB_FAIL; }
+    if (yq == nullptr) { return SPYB_UNSUPPORTED; }
     struct Release { spyb_backend *be; void *a; size_t n; ~Release() { be->arena.free(a, n); } } release{be, yq, ybytes};   // (stream-ordered reuse)
     for (int64_t t0 = 0; t0 < T; t0 += chunk) {
         const int Tc = (int)std::min(chunk, T - t0);

@@ -330,6 +330,34 @@ def test_first_gemm_submit_of_a_constant_reads_finished_tiles(be, oracle, qt):
     be.dealloc_memory(px, x.nbytes)
 
 
+@pytest.mark.parametrize("qt", [quants.Q8_0, quants.Q4_K])
+def test_matmul_without_room_for_the_tile_copy(oracle, qt):
+    """Several columns against a constant when the device has no memory left for the copy the GEMM reads: the mat-vec kernels take the call, and the GEMM
+    later calls once there is room. The same bits each time."""
+    b = B.B200Backend(0, arena_bytes=1 << 24)
+    n, k, t = 8192, 8192, 12
+    rng = np.random.default_rng(qt)
+    rows = rng.integers(0, n, 40)
+    w = np.tile(quants.quantize((rng.standard_normal((64, k)) * 0.02).astype(np.float32), qt).reshape(64, -1), (n // 64, 1))
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    want = oracle.matmul(qt, np.ascontiguousarray(w[rows]), k, len(rows), x)
+    pw, px, po = b.upload_constant("tight", w.reshape(-1), qt, (k, n)), b.upload(x), b.alloc_memory(4 * n * t)
+    d = B.OpDesc(); d.op_type, d.num_input = B.OP["MatMul"], 2
+    d.input[0] = B.make_tensor(pw, qt, (k, n), None, B.NODE_CONSTANT)
+    d.input[1] = B.make_tensor(px, B.FP32, (k, t))
+    d.output = B.make_tensor(po, B.FP32, (n, t))
+    hog_bytes = b.get_avail_memory_capacity() - (100 << 20)
+    hog = b.alloc_memory(hog_bytes)
+    with pytest.raises(B.SpybError):
+        b.alloc_memory(2 * n * k)      # (the copy takes more than two bytes a weight)
+    for full in (True, True, False):
+        if not full and hog:
+            b.dealloc_memory(hog, hog_bytes)
+        b.submit(d); b.sync()
+        assert np.array_equal(bits(b.download(po, (t, n), np.float32)[:, rows]), bits(want))
+    b.close()
+
+
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
 @pytest.mark.parametrize("n,k,t", [(4800, 256, 1), (4796, 1280, 3), (2, 256, 4), (300, 8448, 2), (292, 11008, 4), (9000, 768, 1)])
 def test_k_quant_mat_vec_units_and_rounds(be, oracle, qt, n, k, t):
