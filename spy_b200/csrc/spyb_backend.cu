@@ -549,6 +549,9 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
         (reinterpret_cast<uintptr_t>(x.data) & 15) || (reinterpret_cast<uintptr_t>(out_dev) & 3)) {
         return SPYB_UNSUPPORTED;
     }
+    // (Q4_0 / Q8_0 rows that are no multiple of four have no mat-vec kernel to give the same answer at fewer columns: refused below, but for
+    // the large products that always came here)
+    if (!kq && (n_rows & 3) != 0 && (T < PF_TOK || (n_rows + PF_ROWS - 1) / PF_ROWS * ((T + PF_TOK - 1) / PF_TOK) < 74)) { return SPYB_UNSUPPORTED; }
     if (T <= 8 && matvec_passes_win(type, n_rows, k, (int)T)) { return SPYB_UNSUPPORTED; }
     static const bool off = [] { const char *e = std::getenv("SPYB_PREFILL"); return e != nullptr && e[0] == '0'; }();
     if (off) { return SPYB_UNSUPPORTED; }

@@ -330,6 +330,28 @@ def test_first_gemm_submit_of_a_constant_reads_finished_tiles(be, oracle, qt):
     be.dealloc_memory(px, x.nbytes)
 
 
+@pytest.mark.parametrize("n,t,taken", [(6, 1, False), (6, 5, False), (126, 15, False), (6, 40, False), (9470, 16, True), (9470, 15, False)])
+def test_rows_that_are_no_multiple_of_four(be, oracle, n, t, taken):
+    """Q4_0 constants with such row counts: refused, with a reason, whatever the number of columns, but for products large enough that they always ran
+    on the GEMM."""
+    rng = np.random.default_rng(n + t)
+    w = quants.quantize((rng.standard_normal((n, 64)) * 0.02).astype(np.float32), quants.Q4_0)
+    x = rng.standard_normal((t, 64)).astype(np.float32)
+    pw, px, po = be.upload_constant(f"odd_rows_{n}_{t}", w, quants.Q4_0, (64, n)), be.upload(x), be.alloc_memory(4 * n * t)
+    d = B.OpDesc(); d.op_type, d.num_input = B.OP["MatMul"], 2
+    d.input[0] = B.make_tensor(pw, quants.Q4_0, (64, n), None, B.NODE_CONSTANT)
+    d.input[1] = B.make_tensor(px, B.FP32, (64, t))
+    d.output = B.make_tensor(po, B.FP32, (n, t))
+    if taken:
+        be.submit(d); be.sync()
+        assert np.array_equal(bits(be.download(po, (t, n), np.float32)), bits(oracle.matmul(quants.Q4_0, w, 64, n, x)))
+    else:
+        with pytest.raises(B.SpybError, match="multiple of 4") as e:
+            be.submit(d)
+        assert e.value.status == B.UNSUPPORTED
+    be.dealloc_memory(px, x.nbytes); be.dealloc_memory(po, 4 * n * t)
+
+
 @pytest.mark.parametrize("qt", [quants.Q8_0, quants.Q4_K])
 def test_matmul_without_room_for_the_tile_copy(oracle, qt):
     """Several columns against a constant when the device has no memory left for the copy the GEMM reads: the mat-vec kernels take the call, and the GEMM
