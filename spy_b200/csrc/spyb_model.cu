@@ -13,6 +13,7 @@
 // then NormRMS + Mul(output_norm) + quantize -> output mat-vec -> logits, and a greedy argmax that
 // also gathers the next token's embedding.
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <dlfcn.h>
@@ -224,7 +225,11 @@ spyb_status build_step_plan(spyb_model *m);
 template <class T>
 spyb_status dev_alloc(spyb_model *m, T **p, size_t count) {
     void *raw = nullptr;
-    SPYB_CUDA(m->be, cudaMalloc(&raw, count * sizeof(T) + 64));
+    if (cudaMalloc(&raw, count * sizeof(T) + 64) != cudaSuccess) {
+        cudaGetLastError();   // (some callers go on without: not left for the next launch to find)
+        m->be->set_error("out of device memory allocating %llu bytes", (unsigned long long)(count * sizeof(T)));
+        return SPYB_FAIL;
+    }
     SPYB_CUDA(m->be, cudaMemsetAsync(raw, 0, count * sizeof(T) + 64, m->be->stream));
     SPYB_CUDA(m->be, cudaStreamSynchronize(m->be->stream));   // uploads that follow use other streams: order them after the clearing
     m->owned.push_back(raw);
@@ -459,26 +464,26 @@ spyb_status run_head(spyb_model *m, int col, int64_t *launches, const float *x_r
     return SPYB_SUCCESS;
 }
 
-// buffers of the tensor-core prompt path, allocated at the first long prompt
+// buffers of the tensor-core prompt path, allocated at the first long prompt (what one call could not allocate, the next one tries again)
 spyb_status ensure_prefill_buffers(spyb_model *m) {
     if (m->pf_buffers) { return SPYB_SUCCESS; }
     spyb_backend *be = m->be;
     const size_t C = (size_t)m->pf_chunk, d = m->info.d_model, ff = m->info.n_ff, dl = m->dl;
     const int nb_max = (int)(std::max(d, ff) / 32);
-    bool ok = dev_alloc(m, &m->pf_x, C * d) == SPYB_SUCCESS && dev_alloc(m, &m->pf_qkv, C * 3 * dl) == SPYB_SUCCESS && dev_alloc(m, &m->pf_att, C * d) == SPYB_SUCCESS &&
-              dev_alloc(m, &m->pf_ug, C * 2 * ff) == SPYB_SUCCESS && dev_alloc(m, &m->pf_act, C * ff) == SPYB_SUCCESS && dev_alloc(m, &m->pf_q, C * dl) == SPYB_SUCCESS &&
-              dev_alloc(m, &m->pf_yq, prefill_act_bytes((int)C, nb_max)) == SPYB_SUCCESS && dev_alloc(m, &m->pf_tokens, C) == SPYB_SUCCESS &&
-              dev_alloc(m, &m->pf_pos, 2 * (C / TMAX + 1)) == SPYB_SUCCESS;   // (sized for the smallest group)
+    auto have = [&](auto **p, size_t n) { return *p != nullptr || dev_alloc(m, p, n) == SPYB_SUCCESS; };
+    bool ok = have(&m->pf_x, C * d) && have(&m->pf_qkv, C * 3 * dl) && have(&m->pf_att, C * d) && have(&m->pf_ug, C * 2 * ff) && have(&m->pf_act, C * ff) &&
+              have(&m->pf_q, C * dl) && have(&m->pf_yq, prefill_act_bytes((int)C, nb_max)) && have(&m->pf_tokens, C) &&
+              have(&m->pf_pos, 2 * (C / TMAX + 1));   // (sized for the smallest group)
     if (!ok) { return SPYB_FAIL; }
     // prompts share K rows and V^T rows among tiles of eight tokens at every context length (SPYB_PF_ATT_TILED=0: contexts up to
     // 1024 positions keep one CTA per head and token, as single-token steps do)
     const char *tiled_env = std::getenv("SPYB_PF_ATT_TILED");
     if (m->att_scratch == nullptr && (tiled_env == nullptr || std::atoi(tiled_env) != 0)) {
         const size_t n_pad = ((size_t)m->info.n_ctx + 3) & ~(size_t)3;
-        if (dev_alloc(m, &m->pf_att_scratch, (size_t)m->att_group * (dl / m->info.head_dim) * n_pad) != SPYB_SUCCESS) { return SPYB_FAIL; }
+        if (!have(&m->pf_att_scratch, (size_t)m->att_group * (dl / m->info.head_dim) * n_pad)) { return SPYB_FAIL; }
     }
-    if (cudaMallocHost(reinterpret_cast<void **>(&m->h_pf_tokens), C * 4) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void **>(&m->h_pf_pos), 2 * (C / TMAX + 1) * 4) != cudaSuccess) { be->set_error("pinned host allocation failed"); return SPYB_FAIL; }
+    auto pinned = [&](auto **p, size_t bytes) { return *p != nullptr || cudaMallocHost(reinterpret_cast<void **>(p), bytes) == cudaSuccess; };
+    if (!pinned(&m->h_pf_tokens, C * 4) || !pinned(&m->h_pf_pos, 2 * (C / TMAX + 1) * 4)) { cudaGetLastError(); be->set_error("pinned host allocation failed"); return SPYB_FAIL; }
     m->pf_buffers = true;
     return SPYB_SUCCESS;
 }
@@ -691,6 +696,7 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
         I.weight_bytes += (uint64_t)n_rows * rb_file;
         return SPYB_SUCCESS;
     };
+    bool pf_no_room = false;
     // the tile layout of the tensor-core prompt kernel: rows [0, rows_full) of a tensor into rows [dst_row, ...) of a matrix of total_rows rows
     // (rows [row0, row0 + n_rows) of the tensor; n_rows < 0: all of them)
     auto upload_pf = [&](const std::string &name, int64_t k_full, int64_t rows_full, PfMat *into, int64_t dst_row, int64_t total_rows, int64_t row0 = 0, int64_t n_rows = -1) {
@@ -700,13 +706,18 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
         if (t->ne[0] != k_full || t->ne[1] != rows_full || (t->type != SPYB_Q4_0 && t->type != SPYB_Q8_0 && t->type != SPYB_Q4_K && t->type != SPYB_Q6_K)) { return SPYB_UNSUPPORTED; }
         const int nb = (int)(k_full / 32);
         if (into->w == nullptr) {
-            if (dev_alloc(m, &into->w, prefill_weight_bytes(t->type, total_rows, nb)) != SPYB_SUCCESS) { return SPYB_FAIL; }
+            if (dev_alloc(m, &into->w, prefill_weight_bytes(t->type, total_rows, nb)) != SPYB_SUCCESS) { pf_no_room = true; return SPYB_UNSUPPORTED; }
             into->type = t->type; into->n_rows = total_rows; into->nb = nb;
         } else if (into->type != t->type) { return SPYB_UNSUPPORTED; }
         const int64_t rb = GgufFile::row_bytes(t->type, k_full);
         const int64_t max_rows = std::max<int64_t>(1, (int64_t)(64u << 20) / rb);   // 64 MiB staging pieces
         void *stage = nullptr;
-        SPYB_CUDA(be, cudaMalloc(&stage, (size_t)std::min(max_rows, n_rows) * rb + 64));
+        if (cudaMalloc(&stage, (size_t)std::min(max_rows, n_rows) * rb + 64) != cudaSuccess) {
+            cudaGetLastError();
+            be->set_error("GGUF: %s: out of device memory", name.c_str());
+            pf_no_room = true;
+            return SPYB_UNSUPPORTED;
+        }
         for (int64_t r0 = 0; r0 < n_rows; r0 += max_rows) {
             const int64_t nr = std::min(max_rows, n_rows - r0);
             cudaError_t e = cudaMemcpyAsync(stage, data + (row0 + r0) * rb, (size_t)nr * rb, cudaMemcpyHostToDevice, be->stream);
@@ -792,17 +803,6 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
                 (st = upload_kq(p + "ffn_down.weight", I.n_ff, d, 0, d, &ly.kq_down)) != SPYB_SUCCESS) { return fail(st); }
             if (dev_alloc(m, &ly.k_cache, (size_t)I.n_ctx * dl) != SPYB_SUCCESS || dev_alloc(m, &ly.v_cache, (size_t)I.n_ctx * dl) != SPYB_SUCCESS) { return fail(SPYB_FAIL); }
             ly.k_base = ly.k_cache; ly.v_base = ly.v_cache;
-            if (m->pf_ok) {   // the same tensors in the tile layout of the tensor-core prompt kernel, one matrix per tensor
-                spyb_status ps = upload_pf(p + "attn_q.weight", d, d, &ly.pf_qkv, 0, d);
-                if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_k.weight", d, d, &ly.pf_k, 0, d); }
-                if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_v.weight", d, d, &ly.pf_v, 0, d); }
-                if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_output.weight", d, d, &ly.pf_wo, 0, d); }
-                if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_up.weight", d, I.n_ff, &ly.pf_ug, 0, I.n_ff); }
-                if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_gate.weight", d, I.n_ff, &ly.pf_gate, 0, I.n_ff); }
-                if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_down.weight", I.n_ff, d, &ly.pf_down, 0, d); }
-                if (ps == SPYB_FAIL) { return fail(ps); }
-                if (ps != SPYB_SUCCESS) { m->pf_ok = false; }
-            }
             continue;
         }
         // heads: rows [r*dl, (r+1)*dl) of Wq, Wk, Wv, stacked into one [3*dl, d] matrix
@@ -849,23 +849,6 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
         if (st != SPYB_SUCCESS) { return fail(st); }
         if (dev_alloc(m, &ly.k_cache, (size_t)I.n_ctx * dl) != SPYB_SUCCESS || dev_alloc(m, &ly.v_cache, (size_t)I.n_ctx * dl) != SPYB_SUCCESS) { return fail(SPYB_FAIL); }
         ly.k_base = ly.k_cache; ly.v_base = ly.v_cache;
-        if (m->pf_ok) {
-            const int64_t q0 = (int64_t)r * dl, f0 = (int64_t)r * fl;   // this rank's heads and FFN rows
-            spyb_status ps = upload_pf(p + "attn_q.weight", d, d, &ly.pf_qkv, 0, 3 * (int64_t)dl, q0, dl);
-            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_k.weight", d, d, &ly.pf_qkv, dl, 3 * (int64_t)dl, q0, dl); }
-            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_v.weight", d, d, &ly.pf_qkv, 2 * (int64_t)dl, 3 * (int64_t)dl, q0, dl); }
-            const int64_t dp = d / tp, o0 = (int64_t)r * dp;            // and its slice of the output rows of W_o and W_down
-            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_output.weight", d, d, &ly.pf_wo, 0, dp, o0, dp); }
-            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_up.weight", d, I.n_ff, &ly.pf_ug, 0, 2 * (int64_t)fl, f0, fl); }
-            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_gate.weight", d, I.n_ff, &ly.pf_ug, fl, 2 * (int64_t)fl, f0, fl); }
-            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_down.weight", I.n_ff, d, &ly.pf_down, 0, dp, o0, dp); }
-            if (ps == SPYB_FAIL) { return fail(ps); }
-            if (ps != SPYB_SUCCESS) { m->pf_ok = false; }   // a mix of types inside one stacked matrix: prompts stay on the mat-vec passes
-        }
-    }
-    if (m->pf_ok) {
-        const std::string head_name = m->kq || f.tensors.count("output.weight") ? "output.weight" : "token_embd.weight";
-        if (upload_pf(head_name, d, I.n_vocab, &m->pf_head, 0, I.n_vocab) == SPYB_FAIL) { return fail(SPYB_FAIL); }   // (another type: the head stays on the mat-vec passes)
     }
     I.weight_bytes += (uint64_t)(2 * I.n_layer + 1) * d * 4;
     I.kv_bytes_per_token = (uint64_t)2 * I.n_layer * dl * 2;
@@ -910,6 +893,49 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
     if (cudaEventCreate(&m->ev0) != cudaSuccess || cudaEventCreate(&m->ev1) != cudaSuccess) { be->set_error("event creation failed"); return fail(SPYB_FAIL); }
     if (cudaDeviceSynchronize() != cudaSuccess) { be->set_error("device synchronisation after the upload failed"); return fail(SPYB_FAIL); }
     if (build_step_plan(m) != SPYB_SUCCESS) { return fail(SPYB_FAIL); }
+    // The tile copies come last: they take more memory than the weights themselves (over two bytes a weight). Where they do not fit beside what
+    // every call needs, a model on one GPU gives them back and runs its prompts and batches as mat-vec passes (the ranks of a sharded one
+    // have to take the same path, so there it is an error).
+    for (int L = 0; L < I.n_layer && m->pf_ok; ++L) {
+        Layer &ly = m->layers[L];
+        const std::string p = "blk." + std::to_string(L) + ".";
+        spyb_status ps;
+        if (m->kq) {   // one matrix per tensor
+            ps = upload_pf(p + "attn_q.weight", d, d, &ly.pf_qkv, 0, d);
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_k.weight", d, d, &ly.pf_k, 0, d); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_v.weight", d, d, &ly.pf_v, 0, d); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_output.weight", d, d, &ly.pf_wo, 0, d); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_up.weight", d, I.n_ff, &ly.pf_ug, 0, I.n_ff); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_gate.weight", d, I.n_ff, &ly.pf_gate, 0, I.n_ff); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_down.weight", I.n_ff, d, &ly.pf_down, 0, d); }
+        } else {
+            const int64_t q0 = (int64_t)r * dl, f0 = (int64_t)r * fl;   // this rank's heads and FFN rows
+            ps = upload_pf(p + "attn_q.weight", d, d, &ly.pf_qkv, 0, 3 * (int64_t)dl, q0, dl);
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_k.weight", d, d, &ly.pf_qkv, dl, 3 * (int64_t)dl, q0, dl); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_v.weight", d, d, &ly.pf_qkv, 2 * (int64_t)dl, 3 * (int64_t)dl, q0, dl); }
+            const int64_t dp = d / tp, o0 = (int64_t)r * dp;            // and its slice of the output rows of W_o and W_down
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "attn_output.weight", d, d, &ly.pf_wo, 0, dp, o0, dp); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_up.weight", d, I.n_ff, &ly.pf_ug, 0, 2 * (int64_t)fl, f0, fl); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_gate.weight", d, I.n_ff, &ly.pf_ug, fl, 2 * (int64_t)fl, f0, fl); }
+            if (ps == SPYB_SUCCESS) { ps = upload_pf(p + "ffn_down.weight", I.n_ff, d, &ly.pf_down, 0, dp, o0, dp); }
+        }
+        if (ps == SPYB_FAIL) { return fail(ps); }
+        if (ps != SPYB_SUCCESS) { m->pf_ok = false; }   // no room, or a mix of types inside one stacked matrix: prompts stay on the mat-vec passes
+    }
+    if (m->pf_ok) {
+        const std::string head_name = m->kq || f.tensors.count("output.weight") ? "output.weight" : "token_embd.weight";
+        if (upload_pf(head_name, d, I.n_vocab, &m->pf_head, 0, I.n_vocab) == SPYB_FAIL) { return fail(SPYB_FAIL); }   // (no room, or another type: the head stays on the mat-vec passes)
+    }
+    if (pf_no_room && tp > 1) { return fail(SPYB_FAIL); }
+    if (!m->pf_ok) {
+        auto drop = [&](PfMat &W) {
+            if (W.w == nullptr) { return; }
+            m->owned.erase(std::find(m->owned.begin(), m->owned.end(), static_cast<void *>(W.w)));
+            cudaFree(W.w);
+            W = PfMat();
+        };
+        for (Layer &ly : m->layers) { for (PfMat *W : {&ly.pf_qkv, &ly.pf_k, &ly.pf_v, &ly.pf_wo, &ly.pf_ug, &ly.pf_gate, &ly.pf_down}) { drop(*W); } }
+    }
     *out = m;
     return SPYB_SUCCESS;
 }
@@ -1035,10 +1061,14 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
     // columns of a mat-vec pass
     const int tmax = m->kq ? KQ_MAX_COLUMNS : std::min(8, std::min(matvec_max_columns(m->info.d_model / 32), matvec_max_columns(m->info.n_ff / 32)));
     const bool small = n_tokens < PF_TOK;   // (these leave what the mat-vec passes leave behind for the parity taps)
-    if (m->pf_ok && n_tokens >= (m->info.tp_size == 1 ? SPYB_PREFILL_MIN_TOKENS : PF_TOK) && (!small || m->pf_chunk >= n_tokens)) {
+    bool gemm = m->pf_ok && n_tokens >= (m->info.tp_size == 1 ? SPYB_PREFILL_MIN_TOKENS : PF_TOK);
+    if (gemm && ensure_prefill_buffers(m) != SPYB_SUCCESS) {
+        if (m->info.tp_size > 1) { return SPYB_FAIL; }
+        gemm = false;   // (no memory for the prompt path's buffers: the mat-vec passes have theirs)
+    }
+    if (gemm) {
         // a prompt: chunks of pf_chunk tokens through the tensor-core GEMMs; the score rows of every chunk span all
         // positions known to the step, as in the passes below
-        if (ensure_prefill_buffers(m) != SPYB_SUCCESS) { return SPYB_FAIL; }
         SPYB_CUDA(be, cudaEventRecord(m->ev0, be->stream));
         for (int t0 = 0; t0 < n_tokens; t0 += m->pf_chunk) {
             const int T = std::min(m->pf_chunk, n_tokens - t0);
@@ -1335,9 +1365,12 @@ spyb_status spyb_model_decode_batch(spyb_model *m, const int32_t *first_tokens, 
     SPYB_CUDA(be, cudaEventRecord(m->ev0, be->stream));
     // enough sequences to fill the tensor-core tiles; a sharded model always takes that path (its all-gathers of whole vectors)
     const int  tp   = m->info.tp_size, dp = d / tp;
-    const bool gemm = m->pf_ok && n_seq <= m->pf_chunk && (n_seq >= SPYB_PREFILL_MIN_TOKENS || tp > 1);
+    bool gemm = m->pf_ok && n_seq <= m->pf_chunk && (n_seq >= SPYB_PREFILL_MIN_TOKENS || tp > 1);
     if (tp > 1 && !gemm) { be->set_error("decode_batch: a sharded model takes at most %d sequences", m->pf_chunk); return SPYB_UNSUPPORTED; }
-    if (gemm && ensure_prefill_buffers(m) != SPYB_SUCCESS) { return SPYB_FAIL; }
+    if (gemm && ensure_prefill_buffers(m) != SPYB_SUCCESS) {
+        if (tp > 1) { return SPYB_FAIL; }
+        gemm = false;
+    }
     for (int step = 0; step < n_steps; ++step) {
         if (gemm) {   // the sequences of a step are the "tokens" of one GEMM pass
             if (tp == 1) { SPYB_CUDA(be, launch_embed(m->batch_tokens, n_seq, m->embd, m->embd_type, d, m->pf_x, be->stream)); ++launches; }

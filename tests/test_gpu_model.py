@@ -202,6 +202,49 @@ def test_prompts_of_a_reused_cache_read_their_own_rows(tmp_models):
     assert np.isfinite(got[0]).all() and np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
 
 
+@pytest.mark.parametrize("kq", [False, True])
+def test_models_and_prompts_with_little_memory_left(kq, tmp_models):
+    """A device with room for a model but not for the tile copies of its weights, and one whose memory runs out between the load and the first prompt:
+    prompts and batches run as mat-vec passes, with the bits of a model that has everything."""
+    cfg = gguf_io.LlamaConfig(n_layer=6, d_model=1024, n_head=8, n_ff=2816, n_vocab=500, weight_std=0.03,
+                              **(dict(wtype=quants.Q4_K, overrides={"attn_v": quants.Q6_K, "ffn_down": quants.Q6_K, "output": quants.Q6_K}) if kq else {}))
+    path = str(tmp_models / f"tight{int(kq)}.gguf")
+    gguf_io.make_llama_gguf(path, cfg, seed=73)
+    prompts = [np.random.default_rng(n).integers(3, cfg.n_vocab, size=n) for n in (24, 10)]
+    b = B.B200Backend(0, arena_bytes=1 << 24)
+
+    def outputs(m):
+        got = [m.eval(p, 0) for p in prompts]
+        for c in range(9):
+            m.select_sequence(c)
+            m.eval(prompts[1], 0)
+        ids, logits = m.decode_batch(np.arange(3, 12), len(prompts[1]), 3, want_logits=True)
+        m.select_sequence(0)
+        return np.concatenate([np.ravel(a) for a in got + [logits]]), ids, m.last_launches
+
+    def fill(leave):
+        n = b.get_avail_memory_capacity() - leave
+        return b.alloc_memory(n), n
+
+    m = B.LlamaModel(b, path, n_ctx=64)
+    m.set_sequences(9)
+    m.decode_batch(np.arange(3, 5), 0, 3)
+    hog = fill(24 << 20)                       # less than the prompt buffers take
+    late = outputs(m)
+    b.dealloc_memory(*hog)
+    want = outputs(m)
+    m.close()
+    hog = fill(140 << 20)                      # the weights fit, their tile copies (over 160 MB) do not
+    m = B.LlamaModel(b, path, n_ctx=64)
+    b.dealloc_memory(*hog)
+    m.set_sequences(9)
+    without = outputs(m)
+    m.close(); b.close()
+    assert late[2] == without[2] != want[2]    # (launches of the batch: the two kinds of passes)
+    for got in (late, without):
+        assert np.array_equal(got[0].view(np.uint32), want[0].view(np.uint32)) and np.array_equal(got[1], want[1])
+
+
 def test_prompt_widths_the_gemm_tile_does_not_divide(be, oracle, tmp_models):
     """n_ff = 416 is no multiple of the 128-row GEMM tile (the stacked up|gate matrix has 832 rows: the last tile is half
     padding, and W_gate starts in the middle of a tile): the padded rows are neither computed into anything nor stored."""
