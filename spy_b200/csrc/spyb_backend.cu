@@ -2,6 +2,7 @@
 // This is the part that stands in for the reference's DefaultGPUBackend
 // (backend/cuda/include/default_backend.h:22-99) behind Backend::{alloc_memory, dealloc_memory, submit}.
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -715,35 +716,50 @@ spyb_status run_matmul(spyb_backend *be, spyb_op_desc *d, void *out_dev) {
     return SPYB_SUCCESS;
 }
 
-// Rows of the (cos, sin) table for the given positions, with the host libm and the CPU operator's repeated f32 multiplication of theta
-// (backend/host/operator/non-linear.cpp:282, 300-309). nullptr when the positions do not fit a table (the caller then builds its own).
-const float2 *rope_rows(spyb_backend *be, const spyb_rope_param &rp, const int32_t *pos, int64_t n_tok, int64_t npair) {
+// Rope of up to ROPE_ROWS tokens from the kept table of (cos, sin) rows, with the host libm and the CPU operator's repeated f32 multiplication
+// of theta (backend/host/operator/non-linear.cpp:282, 300-309). A table grows to the positions it meets (up to MAX_ROWS) and the least
+// recently used of MAX_TABLES makes room for a new one: what a call costs does not depend on whose calls came first. The launch is
+// enqueued under the lock: a table that another thread replaces is handed back behind it in stream order.
+// False when the positions do not fit a table (the caller then builds its own).
+bool rope_from_table(spyb_backend *be, const spyb_rope_param &rp, const int32_t *pos, int64_t npair, const Strided &x, const Strided &out, cudaError_t *err) {
     constexpr size_t MAX_TABLES = 8, MAX_ROWS = 16384;
+    const int64_t n_tok = x.ne[2];
+    if (n_tok < 1 || n_tok > ROPE_ROWS || npair < 1) { return false; }
+    int32_t last = 0;
+    for (int64_t i = 0; i < n_tok; ++i) { if (pos[i] < 0 || (size_t)pos[i] >= MAX_ROWS) { return false; } last = std::max(last, pos[i]); }
     std::lock_guard<std::mutex> g(be->rope_mutex);
-    RopeTable *t = nullptr;
-    for (RopeTable &c : be->rope_tables) { if (c.freq_base == rp.freq_base && c.num_dim == rp.num_dim && c.npair == npair) { t = &c; break; } }
-    if (t == nullptr) {
-        if (be->rope_tables.size() >= MAX_TABLES || rp.num_context < 1) { return nullptr; }
+    std::vector<RopeTable> &tables = be->rope_tables;   // the most recently used one last
+    auto drop = [&](size_t i) { be->arena.free(tables[i].dev, tables[i].have.size() * tables[i].npair * sizeof(float2)); tables.erase(tables.begin() + (ptrdiff_t)i); };
+    size_t at = 0;
+    while (at < tables.size() && !(tables[at].freq_base == rp.freq_base && tables[at].num_dim == rp.num_dim && tables[at].npair == npair)) { ++at; }
+    size_t rows = std::max(std::min<size_t>(MAX_ROWS, (size_t)std::max(rp.num_context, 1)), (size_t)last + 1);
+    if (at < tables.size() && (size_t)last < tables[at].have.size()) {
+        std::rotate(tables.begin() + (ptrdiff_t)at, tables.begin() + (ptrdiff_t)at + 1, tables.end());
+    } else {
+        if (at < tables.size()) { rows = std::max(rows, std::min(MAX_ROWS, 2 * tables[at].have.size())); drop(at); }
+        else if (tables.size() >= MAX_TABLES) { drop(0); }
         RopeTable c;
         c.freq_base = rp.freq_base; c.num_dim = rp.num_dim; c.npair = npair;
-        c.have.assign(std::min<size_t>(MAX_ROWS, (size_t)rp.num_context), 0);
-        c.dev = static_cast<float2 *>(be->arena.alloc(c.have.size() * npair * sizeof(float2)));
-        if (c.dev == nullptr) { return nullptr; }
-        be->rope_tables.push_back(std::move(c));
-        t = &be->rope_tables.back();
+        c.have.assign(rows, 0);
+        c.dev = static_cast<float2 *>(be->arena.alloc(rows * npair * sizeof(float2)));
+        if (c.dev == nullptr) { return false; }
+        tables.push_back(std::move(c));
     }
-    for (int64_t i = 0; i < n_tok; ++i) { if (pos[i] < 0 || (size_t)pos[i] >= t->have.size()) { return nullptr; } }
+    RopeTable &t = tables.back();
     std::vector<float2> row;
     const float theta_scale = std::pow(rp.freq_base, -2.0f / (float)rp.num_dim);
+    RopeRows rr;
     for (int64_t i = 0; i < n_tok; ++i) {
-        if (t->have[pos[i]]) { continue; }
+        rr.row[i] = pos[i];
+        if (t.have[pos[i]]) { continue; }
         row.resize((size_t)npair);
         float theta = (float)pos[i];
         for (int64_t k = 0; k < npair; ++k) { row[(size_t)k] = make_float2(std::cos(theta) * 1.0f, std::sin(theta) * 1.0f); theta *= theta_scale; }
-        if (cudaMemcpyAsync(t->dev + (int64_t)pos[i] * npair, row.data(), row.size() * sizeof(float2), cudaMemcpyHostToDevice, be->stream) != cudaSuccess) { return nullptr; }
-        t->have[pos[i]] = 1;
+        if (cudaMemcpyAsync(t.dev + (int64_t)pos[i] * npair, row.data(), row.size() * sizeof(float2), cudaMemcpyHostToDevice, be->stream) != cudaSuccess) { return false; }
+        t.have[pos[i]] = 1;
     }
-    return t->dev;
+    *err = launch_rope_rows(x, t.dev, rr, out, be->stream);
+    return true;
 }
 
 // A host mask of +0 and -inf as bits (set = visible); false when it holds anything else or does not fit
@@ -844,14 +860,7 @@ spyb_status spyb_submit(spyb_backend *be, spyb_op_desc *d, void (*callback)(void
                         cudaStreamSynchronize(be->stream) != cudaSuccess) { be->set_error("Rope: reading positions failed"); st = SPYB_FAIL; break; }
                     pos = pos_read.data();
                 }
-                if (n_tok <= ROPE_ROWS) {
-                    if (const float2 *rows = rope_rows(be, d->rope, pos, n_tok, npair)) {
-                        RopeRows rr;
-                        for (int64_t i = 0; i < n_tok; ++i) { rr.row[i] = pos[i]; }
-                        err = launch_rope_rows(to_strided(a, a.data), rows, rr, to_strided(local.output, out.dev), be->stream);
-                        break;
-                    }
-                }
+                if (rope_from_table(be, d->rope, pos, npair, to_strided(a, a.data), to_strided(local.output, out.dev), &err)) { break; }
                 // many tokens, or positions outside the table: (cos, sin) per (token, pair) for this call alone, the same arithmetic
                 std::vector<float2> tab((size_t)(n_tok * npair));
                 const float theta_scale = std::pow(d->rope.freq_base, -2.0f / (float)d->rope.num_dim);

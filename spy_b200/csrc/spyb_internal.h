@@ -90,7 +90,7 @@ struct spyb_backend {
     std::vector<void *>                      owned;   // cudaMalloc'd blocks to release at destroy
 
     std::mutex                   rope_mutex;
-    std::vector<spyb::RopeTable> rope_tables;   // one per (base, dimensions) seen
+    std::vector<spyb::RopeTable> rope_tables;   // one per (base, dimensions), the eight used last
 
     // completion callbacks
     std::thread                      cb_thread;

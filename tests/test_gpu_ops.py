@@ -59,8 +59,8 @@ def run(be, op, inputs, out_ne, out_type=B.FP32, host_out=False, **params):
     d.view_offset = params.get("offset", 0)
     if op == "Rope":
         r = d.rope
-        r.mode, r.num_dim, r.num_context, r.num_origin_context = 0, params["n_dim"], 512, 4096
-        r.freq_base, r.freq_scale, r.extend_factor, r.attention_factor, r.beta_fast, r.beta_slow = 10000.0, 1.0, 0.0, 1.0, 32.0, 1.0
+        r.mode, r.num_dim, r.num_context, r.num_origin_context = 0, params["n_dim"], params.get("n_context", 512), 4096
+        r.freq_base, r.freq_scale, r.extend_factor, r.attention_factor, r.beta_fast, r.beta_slow = params.get("base", 10000.0), 1.0, 0.0, 1.0, 32.0, 1.0
     be.submit(d)
     be.sync()
     if op == "Copy":
@@ -530,6 +530,31 @@ def test_rope_with_host_positions(be, oracle):
     pos = np.array([0, 17, 511], dtype=np.int32)
     got = run(be, "Rope", [(x, B.FP32, (128, 4, 3), None, B.NODE_DYNAMIC), (pos, B.INT32, (3,), None, B.NODE_IO)], (128, 4, 3), n_dim=128).reshape(3, 4, 128)
     assert np.array_equal(bits(got), bits(oracle.rope(x, pos, 10000.0)))   # cos/sin come from the host libm
+
+
+def test_rope_tables_grow_and_make_room(oracle):
+    """A backend whose first Rope calls have short contexts and many bases, and whose later ones need longer tables and further bases: the oracle's bits
+    throughout, every call served from a kept table (the arena shrinks at a growth) and no more than eight of them kept."""
+    b = B.B200Backend(0)
+    rng = np.random.default_rng(8)
+
+    def rope(base, positions, n_context=512):
+        x = rng.standard_normal((len(positions), 2, 128)).astype(np.float32)
+        pos = np.array(positions, dtype=np.int32)
+        got = run(b, "Rope", [(x, B.FP32, (128, 2, len(pos)), None, B.NODE_DYNAMIC), (pos, B.INT32, (len(pos),), None, B.NODE_IO)], (128, 2, len(pos)),
+                  n_dim=128, base=base, n_context=n_context)
+        assert np.array_equal(bits(got.reshape(x.shape)), bits(oracle.rope(x, pos, base)))
+        return b.get_avail_memory_capacity()
+
+    short = rope(10000.0, [0, 511])
+    assert rope(10000.0, [512, 3, 4095], 4096) <= short - (4096 - 512) * 64 * 8
+    rope(10000.0, [4096, 511, 16383])
+    rope(10000.0, [16384, 1])                       # beyond the longest table: a table for the call alone
+    rope(10000.0, [40000])
+    kept = [rope(5000.0 + 1000 * i, [i, 300]) for i in range(12)]
+    assert kept[8] == kept[11]                      # eight tables of one size: each new one replaces the oldest
+    rope(10000.0, [7, 2000])
+    b.close()
 
 
 def test_getrow_f32_and_q8_0(be, oracle):
