@@ -69,7 +69,7 @@ struct KqSeg {
 
 constexpr int MV_NARROW = 3072;   // widest d_model of a narrow model
 struct MatvecParams {
-    int   stages_early = 64;          // single column: stages of each warp's ring whose copies are issued ahead of x (set at the launch)
+    int   stages_early = 64;          // single column, kernels built for one prologue: stages of each warp's ring whose copies are issued ahead of x (set at the launch)
     int   narrow = 0;                 // the matrix of a narrow model (MV_NARROW): single columns on the kernel that serves all of a layer's
     DevMatrix A;
     DevMatrix B;               // second matrix when pair_mode == 1 (same shape as A)
@@ -112,7 +112,7 @@ struct MatvecParams {
 
 // Prompt evaluation as a GEMM on the tcgen05 tensor cores (spyb_prefill.cu). Weights in tiles of PF_ROWS rows x 1 block,
 // activations as compact Q8_0 blocks grouped by (token tile, block).
-constexpr int PF_ROWS = 128, PF_TOK = 16;   // (PF_TOK: fewest tokens worth a pass on this path, and the widest token tile of the Q4_0 / Q8_0 kernel)
+constexpr int PF_ROWS = 128, PF_TOK = 16;   // (PF_TOK: the widest token tile of the Q4_0 / Q8_0 kernel, and the shortest prompt a sharded model runs on it)
 constexpr int PF_WTILE_F16 = 128 * 32 * 2 + 128 * 4;            // Q4_0 / Q8_0: the f16 A operand of a 32-element block (128 rows), then one f32 scale per row
 constexpr int PF_KQ_TOK_MAX = 64;                               // K-quant kernels: the widest token tile
 constexpr int PF_KQ_WTILE = 128 * 32 * 2 + 128 * 8;             // the f16 A operand of a 32-element block, then two f32 scale products per row

@@ -881,7 +881,6 @@ static cudaError_t launch_matvec_mma_t(const MatvecParams &p, const LaunchCfg &c
     if (err != cudaSuccess) { return err; }
     MatvecParams q = p;
     if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
-    if (cfg.pdl) { q.stages_early = MV_STAGES_EARLY; }
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)grid); lc.blockDim = dim3(MV_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;
     cudaLaunchAttribute attr[1];
@@ -1001,7 +1000,6 @@ static cudaError_t launch_matvec_t(const MatvecParams &p, const LaunchCfg &cfg) 
     if (err != cudaSuccess) { return err; }
     MatvecParams q = p;
     if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
-    if (cfg.pdl) { q.stages_early = MV_STAGES_EARLY; }
 
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)grid); lc.blockDim = dim3(MV_THREADS); lc.dynamicSmemBytes = smem; lc.stream = cfg.stream;

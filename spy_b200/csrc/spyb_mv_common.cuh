@@ -6,7 +6,7 @@
 
 namespace spyb {
 
-// Single-column mat-vecs of a step (launched ahead of their predecessor's end): stages of each warp's ring whose copies are issued before the
+// Single-column mat-vecs of a step on matvec_rows_kernel and matvec_kq_kernel (launched ahead of their predecessor's end): stages of each warp's ring whose copies are issued before the
 // previous kernel's results are waited for; the rest follow when the reads of x are on their way. Issuing takes the warp some 50 cycles a
 // copy, which the last CTA to start (its SM was the last to become free) would add to the step, and x does not queue behind a ring full
 // of weights on every SM. A launch of its own has nothing to wait for and issues all of them first.

@@ -205,9 +205,8 @@ def dequantize(raw: np.ndarray, number_type: int) -> np.ndarray:
 
 
 # ---------------------------------------------------------------------------------------------
-# e4m3 codes of small integers, as the prompt GEMM feeds them to the tensor cores (spyb_prefill.cu: a Q4_0 weight nibble - 8
-# directly; an 8-bit value y as the two codes of y - y mod 16 and y mod 16). Kept here for tools that want to read or build
-# the kernel's operand tiles on the host, and checked against an independent e4m3 decoder in the tests.
+# e4m3 codes of small integers, and of an 8-bit value y as the two codes of y - y mod 16 and y mod 16, for host tools that prepare
+# operands in that form (the prompt GEMM's are f16); checked against an independent e4m3 decoder in the tests.
 def e4m3_of_small(v: int) -> int:
     """Code of the integer 0 <= v <= 15 (exact: three mantissa bits cover 8..15)."""
     if v == 0:

@@ -1,4 +1,4 @@
-"""The e4m3 codes of the prompt GEMM's operands against torch's float8_e4m3fn decoder (CPU only): every code stands for the
+"""The e4m3 codes of spy_b200.quants against torch's float8_e4m3fn decoder (CPU only): every code stands for the
 integer it was made from, and the two parts of every 8-bit value add up to it."""
 import torch
 

@@ -265,8 +265,8 @@ def test_batch_of_sequences_equals_single_sequence_runs(n_seq, n_ctx, kq, oracle
     """Independent sequences that share the weights and advance in lockstep: every sequence must give the ids and the
     logits of a run on its own (the batch > 1 configurations are replicas of the single-sequence reference). Prompts of
     one length, different contents; 3 sequences = one group of activation columns, 8 and 6 = two groups; 16 and more go
-    through the tensor-core GEMM kernels as the tokens of one pass; a context above 1024 positions takes the three-kernel
-    attention. kq: the Q4_K_M-style mix (groups of four columns through the K-quant mat-vec kernel, or the K-quant GEMM)."""
+    through the tensor-core GEMM kernels as the tokens of one pass; a context above 1024 positions that is no
+    multiple of eight takes the three-kernel attention. kq: the Q4_K_M-style mix (groups of four columns through the K-quant mat-vec kernel, or the K-quant GEMM)."""
     cfg = gguf_io.LlamaConfig(n_layer=2, d_model=256, n_head=2, n_ff=512, n_vocab=400, weight_std=0.06,
                               **(dict(wtype=quants.Q4_K, overrides={"attn_v": quants.Q6_K, "ffn_down": quants.Q6_K, "output": quants.Q6_K}) if kq else {}))
     path = str(tmp_models / ("batch_kq.gguf" if kq else "batch.gguf"))
@@ -465,8 +465,8 @@ def test_steps_of_widths_between_the_prologues(be, oracle, tmp_models, d, wtype)
 
 @pytest.mark.parametrize("env", [{}, {"SPYB_STEP": "1"}])
 def test_long_context_attention_path_in_the_model(env, oracle, tmp_models, monkeypatch):
-    """A context above 1024 positions switches attention to the three-kernel path (scores / softmax / PV spread over the
-    chip); prompt passes of several tokens and single-token steps through it must give the CPU's bits."""
+    """A context above 1024 positions switches attention to the kernels for long contexts (token-tiled scores / softmax / PV for
+    the prompt, one cluster kernel for single-token steps); both must give the CPU's bits."""
     cfg = gguf_io.LlamaConfig(n_layer=2, d_model=256, n_head=2, n_ff=512, n_vocab=512, weight_std=0.05)
     path = str(tmp_models / "longctx.gguf")
     if not os.path.exists(path):

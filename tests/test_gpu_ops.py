@@ -193,8 +193,8 @@ def test_prefill_matmul_k_quants_match_the_restatement(be, oracle, qt, n, k, t, 
 @pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
 def test_prefill_matmul_extreme_bytes(be, oracle, qt):
     """Weight blocks written byte by byte over the whole range (Q8_0: -128 and 127 included, Q4_0: nibbles 0 and 15) against
-    activations whose blocks quantize to +-127 and to zeros: the tensor-core operands split every 8-bit value into two e4m3
-    values, and every split must add up."""
+    activations whose blocks quantize to +-127 and to zeros: every 8-bit value must be exact as an f16 operand of the tensor
+    cores, and every sum in their f32 accumulators."""
     rng = np.random.default_rng(77 + qt)
     n, k, t = 136, 512, 21
     nb = k // 32
@@ -695,8 +695,7 @@ def test_fused_attention_bits(be, oracle, pos0, t, n_total, spread):
                                                   (0, 1, 0, 2048), (5, 3, 0, 2048), (1500, 2, 0, 2048), (3000, 3, 3010, 4096), (4094, 2, 0, 4096), (4095, 1, 0, 4096)])
 def test_fused_attention_long_rows(be, oracle, pos0, t, n_total, n_ctx):
     """Rows longer than the CTA (more than 256 positions: several positions per thread, many 32-position PV steps) up to
-    a full context, against the oracle. Contexts above 1024 positions take the three-kernel path (scores, softmax and PV
-    spread over the chip), at short and at full rows."""
+    a full context, against the oracle. Contexts above 1024 positions take the cluster kernel, at short and at full rows."""
     rng = np.random.default_rng(pos0 + n_ctx)
     n_head, hd = 1, 128
     d = n_head * hd
