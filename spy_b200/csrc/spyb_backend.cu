@@ -522,21 +522,6 @@ void stage_release(spyb_backend *be, Staged *s) {
     s->dev = nullptr; s->temp = false;
 }
 
-// Whether two passes of the mat-vec kernels (five to eight columns) take less time than the GEMM. A GEMM CTA walks all of K for its 128 rows:
-// one round of tiles costs about the same however many rows it has, while a pass grows with rows, K and columns (the second pass runs on
-// a kernel for 1, 2 or 4). Planes through measurements at 512 to 8192 rows, K of 1536 to 11008, in us, K and rows in thousands (a pass
-// gets no shorter below 2048 rows, a tile's weights come faster there); within 10 % of the better one throughout, 0.3 % on average.
-// Q4_0 with 5, 6, 8 columns: 4096 x 4096 22.6, 24.7, 28.7 against 23.6; 4096 x 8192 35.5, 37.1, 45.4 against 43.0; 2048 x 8192 29.9, 30.9, 37.1
-// against 41.9; 8192 x 4096 30.9, 32.9, 39.0 against 24.8. From nine columns (three passes) or 74 tiles on, the GEMM.
-bool matvec_passes_win(int type, int64_t n_rows, int64_t k, int T) {
-    struct Plane { double m0, mk, mr, mc, mrc, g0, gk, gr; };
-    static const Plane q0 = {12.5, 1.09, 0.373, 0.197, 0.055, 2.9, 3.51, 0.738}, q4k = {13.0, 0.49, 0.356, 0.183, 0.060, 3.9, 3.22, 0.349}, q6k = {14.9, 0.24, 0.525, 0.203, 0.088, 3.6, 3.15, 0.386};
-    if (T > 8 || (n_rows + PF_ROWS - 1) / PF_ROWS >= 74) { return false; }
-    const Plane &l = type == SPYB_Q4_K ? q4k : type == SPYB_Q6_K ? q6k : q0;
-    const double K = (double)k / 1000.0, R = (double)n_rows / 1000.0, Rm = std::max(R, 2.048), Rg = std::min(R, 2.048), c = T <= 6 ? T - 4 : 4;
-    return l.m0 + K * (l.mk + l.mr * Rm + c * (l.mc + l.mrc * Rm)) < l.g0 + K * (l.gk + l.gr * Rg);
-}
-
 // MatMul of several activation columns against an uploaded constant: the tcgen05 GEMM of the prompt path (same bits as
 // the mat-vec kernels). The matrix gets a second copy in that kernel's tile layout at first use, kept with the constant.
 // Returns SPYB_UNSUPPORTED without an error text when the operands do not qualify or the memory is not there (the caller then takes the mat-vec route).
@@ -545,6 +530,11 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
     const bool kq = type == SPYB_Q4_K || type == SPYB_Q6_K;
     if (type != SPYB_Q4_0 && type != SPYB_Q8_0 && !kq) { return SPYB_UNSUPPORTED; }
     const int64_t k = w.elements[0], n_rows = w.elements[1], T = x.elements[1] * x.elements[2] * x.elements[3];
+    // From five columns on, which are two mat-vec passes. The GEMM is launched ahead of its predecessor's end; the passes are plain launches. Q4_0,
+    // one matrix again and again: 1024 x 8192 x 5 11.3 us against 20.9, 4096 x 11008 x 8 21.0 against 46.4. W_down inside a layer: d = 4096, ff
+    // 11008, eight columns 152 us against 182 for the layer; d = 3072, ff 8192 112 against 130. Only back-to-back submits that walk over more
+    // matrices than the L2 holds see the passes ahead, on low matrices with long rows, whose tiles few SMs fetch (2048 x 8192 x 5: 41.9 against
+    // 29.9; 4096 x 11008 x 8: 57 against 59; 8192 x 4096 x 5: 25 against 31).
     if (T < 5 || w.node_type != SPYB_NODE_CONSTANT || k != x.elements[0] || k < QK || k % QK != 0 || k > PF_MAX_K || (kq && k % 256 != 0) ||
         n_rows < 1 || w.elements[2] != 1 || w.elements[3] != 1 || !tensor_contiguous(w) || !tensor_contiguous(x) ||
         (reinterpret_cast<uintptr_t>(x.data) & 15) || (reinterpret_cast<uintptr_t>(out_dev) & 3)) {
@@ -553,7 +543,6 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
     // (Q4_0 / Q8_0 rows that are no multiple of four have no mat-vec kernel to give the same answer at fewer columns: refused below, but for
     // the large products that always came here)
     if (!kq && (n_rows & 3) != 0 && (T < PF_TOK || (n_rows + PF_ROWS - 1) / PF_ROWS * ((T + PF_TOK - 1) / PF_TOK) < 74)) { return SPYB_UNSUPPORTED; }
-    if (T <= 8 && matvec_passes_win(type, n_rows, k, (int)T)) { return SPYB_UNSUPPORTED; }
     static const bool off = [] { const char *e = std::getenv("SPYB_PREFILL"); return e != nullptr && e[0] == '0'; }();
     if (off) { return SPYB_UNSUPPORTED; }
     const int nb = (int)(k / QK);

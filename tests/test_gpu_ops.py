@@ -277,8 +277,7 @@ def test_matmul_operator_sweep(be, oracle, qt, n, k, t):
 @pytest.mark.parametrize("n,k,t", [(132, 512, 1), (132, 512, 5), (200, 1024, 16), (260, 2816, 41), (1100, 512, 150), (132, 8192, 5), (64, 11008, 7), (2052, 6144, 8), (64, 8192, 9)])
 def test_matmul_on_uploaded_constants_takes_the_model_kernels(be, oracle, qt, n, k, t):
     """MatMul through spyb_submit against a constant from spyb_upload_constant: K-quant constants run the K-quant mat-vec
-    kernel in passes of four columns, nine columns and more run the tcgen05 GEMM against a tile copy made at first use, five to eight
-    columns whichever of the two is faster (long rows of a low matrix: two mat-vec passes). Either way the oracle's bits (for K-quants:
+    kernel, five columns and more run the tcgen05 GEMM against a tile copy made at first use. Either way the oracle's bits (for K-quants:
     the restatement's)."""
     rng = np.random.default_rng(n + k + t + qt)
     w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
