@@ -163,6 +163,88 @@ __device__ __forceinline__ uint32_t quantize_q8_lane4(float4 v, uint16_t &d_half
     return (uint32_t)(q0 & 0xff) | ((uint32_t)(q1 & 0xff) << 8) | ((uint32_t)(q2 & 0xff) << 16) | ((uint32_t)(q3 & 0xff) << 24);
 }
 
+// The same for PG groups of eight values per lane (the groups of one block in four consecutive lanes), of which the first npass are there
+// (npass is the same in the whole warp). Same bits, fewer instructions and no conversion unit:
+//   - the quotients of a block are the same in its four lanes, so with several groups each lane takes other ones (1 or 2 divisions
+//     instead of 2 PG) and the reciprocals come back by shuffle;
+//   - x * id is rounded by adding 1.5 * 2^23, whose low byte then is the value (|x * id| <= 127.0001). What is not a finite number shows in
+//     the exponent of the sum; its low byte is made that of the conversion above (not a number: 0, infinities: the byte of the largest
+//     and the smallest integer).
+// q: a group's eight values in order. Returns the lane's share of the scales: d of group `kd` in the lanes that have one (kd < 0: none).
+template <int PG>
+__device__ __forceinline__ float quantize_q8_groups(const float (&v)[PG][8], int npass, uint2 (&q)[PG], int &kd) {
+    static_assert(PG >= 1 && PG <= 4, "one lane of a block per quotient");
+    const int lane = threadIdx.x & 31, l = lane & 3;
+    float amax[PG];
+#pragma unroll
+    for (int k = 0; k < PG; ++k) {
+        amax[k] = 0.f;
+        if (k < npass) {
+            float a = fmaxf(fmaxf(fabsf(v[k][0]), fabsf(v[k][1])), fmaxf(fabsf(v[k][2]), fabsf(v[k][3])));
+            a = fmaxf(a, fmaxf(fmaxf(fabsf(v[k][4]), fabsf(v[k][5])), fmaxf(fabsf(v[k][6]), fabsf(v[k][7]))));
+            a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 1));
+            amax[k] = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 2));
+        }
+    }
+    float mine = amax[0], quot, d;   // mine: of the lane's group
+    if (PG == 1) {          // (the shuffle would cost more than the second division)
+        quot = mine != 0.0f ? __fdiv_rn(127.0f, mine) : 0.0f;
+        d = __fdiv_rn(mine, 127.0f);
+        kd = l == 0 ? 0 : -1;
+    } else if (PG == 2) {   // lanes 0, 1 of a block: id of groups 0, 1; lanes 2, 3: d
+        if (l & 1) { mine = amax[PG - 1]; }
+        const bool inv = l < 2;
+        quot = __fdiv_rn(inv ? 127.0f : mine, inv ? mine : 127.0f);
+        d = quot;
+        if (inv && mine == 0.0f) { quot = 0.0f; }
+        kd = inv ? -1 : l - 2;
+    } else {                // lane k: both of group k
+#pragma unroll
+        for (int k = 1; k < PG; ++k) { if (l == k) { mine = amax[k]; } }
+        quot = mine != 0.0f ? __fdiv_rn(127.0f, mine) : 0.0f;
+        d = __fdiv_rn(mine, 127.0f);
+        kd = l;
+    }
+    if (kd >= PG || kd >= npass) { kd = -1; }
+    const float magic = __int_as_float(0x4B400000);
+#pragma unroll
+    for (int k = 0; k < PG; ++k) {
+        q[k] = make_uint2(0u, 0u);
+        if (k < npass) {
+            const float id = PG == 1 ? quot : __shfl_sync(0xffffffffu, quot, (lane & 28) | k);
+            uint32_t b[8], seen = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { b[i] = __float_as_uint(__fadd_rn(__fmul_rn(v[k][i], id), magic)); seen |= b[i]; }
+            if ((seen & 0x30000000u) != 0) {   // (a sum in [2^23, 2^24) has neither bit, infinities and what is not a number - 0x7fffffff - have both)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { if ((b[i] & 0xB0000000u) == 0x30000000u) { b[i] ^= 0xffu; } }
+            }
+            q[k].x = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+            q[k].y = __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410);
+        }
+    }
+    return d;
+}
+// the sum of a group's eight values
+__device__ __forceinline__ int q8_sum8(uint2 q) { return __dp4a((int)q.y, 0x01010101, __dp4a((int)q.x, 0x01010101, 0)); }
+
+// eight floats past L1: one 256-bit load, or two of 128 bits where p may lie on 16 bytes only (A32: it lies on 32)
+template <bool A32 = false>
+__device__ __forceinline__ void load8_cg(const float *p, float (&v)[8]) {
+    if (A32 || (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+        asm volatile("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(__cvta_generic_to_global(p)));
+    } else {
+        const float4 a = __ldcg(reinterpret_cast<const float4 *>(p)), b = __ldcg(reinterpret_cast<const float4 *>(p) + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+}
+// the two sums of four squares that NormRMS adds to its running sum for eight values (groups of four: (x0^2 + x1^2) + (x2^2 + x3^2), see the mat-vec prologue)
+__device__ __forceinline__ float2 squares8(const float (&v)[8]) {
+    return make_float2(__fadd_rn(fmaf(v[1], v[1], __fmul_rn(v[0], v[0])), fmaf(v[3], v[3], __fmul_rn(v[2], v[2]))),
+                       __fadd_rn(fmaf(v[5], v[5], __fmul_rn(v[4], v[4])), fmaf(v[7], v[7], __fmul_rn(v[6], v[6]))));
+}
+
 // ---------------------------------------------------------------------------------------------
 // Integer lane sums are produced directly as floats: the accumulator operand of the byte dot product
 // carries MAGIC_I, so that the result's bit

@@ -38,18 +38,26 @@ constexpr int KQ_WARPS   = KQ_THREADS / WARP;
 constexpr int KQ_REC = 92;               // words per super-block of activations: 64 values, 8 scales, 16 half-block sums, 4 of padding
 constexpr int KQ_MAX_STAGES = 4;
 
-// four values (group g of the column) -> their word of the column's records, the block's scale and half-block sums; called by whole warps
-__device__ __forceinline__ void kq_quantize(float4 v, int g, int n4, uint32_t *rec) {
-    uint16_t dh; int s;
-    const uint32_t q = quantize_q8_lane4(v, dh, s);
-    s += __shfl_xor_sync(0xffffffffu, s, 1); s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (g < n4) {
-        const int b = g >> 3, w = g & 7;
-        uint32_t *r = rec + (b >> 3) * KQ_REC;
-        r[(b & 7) * 8 + w] = q;
-        if (w == 0) { r[64 + (b & 7)] = __float_as_uint(h2f(dh)); }
-        if ((w & 3) == 0) { r[72 + 2 * (b & 7) + (w >> 2)] = __float_as_uint((float)s); }
+// PG groups of eight values (groups g0, g0 + KQ_THREADS, ... of the column's n8) -> their words of the column's records, the blocks' scales
+// and half-block sums; called by whole warps
+template <int PG>
+__device__ __forceinline__ void kq_quantize(const float (&v)[PG][8], int g0, int n8, uint32_t *rec) {
+    const int npass = min(PG, (n8 - (g0 & ~31) + KQ_THREADS - 1) / KQ_THREADS);   // (n8 is a multiple of 32: the same in the whole warp)
+    uint2 q[PG];
+    int kd;
+    const float d = quantize_q8_groups<PG>(v, npass, q, kd);
+#pragma unroll
+    for (int k = 0; k < PG; ++k) {
+        if (k < npass) {
+            int s = q8_sum8(q[k]);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            const int g = g0 + k * KQ_THREADS, b = g >> 2, w = g & 3;
+            uint32_t *r = rec + (b >> 3) * KQ_REC;
+            *reinterpret_cast<uint2 *>(r + (b & 7) * 8 + 2 * w) = q[k];
+            if ((w & 1) == 0) { r[72 + 2 * (b & 7) + (w >> 1)] = __float_as_uint((float)s); }
+        }
     }
+    if (kd >= 0) { const int b = (g0 + kd * KQ_THREADS) >> 2; rec[(b >> 3) * KQ_REC + 64 + (b & 7)] = __float_as_uint(h2f(f2h(d))); }
 }
 
 // NormRMS + Mul(weight) (optional) + Quantizator<FP32,Q8_0> of the pass's columns into the activation records (column t lies col words
@@ -79,45 +87,57 @@ __device__ __forceinline__ void kq_prologue(const MatvecParams &p, int nT, uint3
         }
         __syncthreads();   // also: the partials (aliasing the records) are dead from here on
     }
-    const float4 *w4 = reinterpret_cast<const float4 *>(p.norm_w);
+    const int n8 = n4 >> 1;
 #pragma unroll 1
     for (int t = 0; t < nT; ++t) {
-        const float4 *x4 = reinterpret_cast<const float4 *>(p.x + (int64_t)t * p.x_stride);
+        const float *x = p.x + (int64_t)t * p.x_stride;
         const float scale = NORM ? scale_s[t] : 1.f;
-        for (int base = 0; base < n4; base += KQ_THREADS) {   // n4 is a multiple of 64: whole warps, whole blocks
+        for (int base = 0; base < n8; base += KQ_THREADS) {   // n8 is a multiple of 32: whole warps, whole blocks
             const int g = base + tid;
-            const bool valid = g < n4;
-            float4 v = valid ? __ldcg(x4 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (NORM && valid) {
-                const float4 w = w4[g];
-                v.x = __fmul_rn(__fmul_rn(v.x, scale), w.x); v.y = __fmul_rn(__fmul_rn(v.y, scale), w.y);
-                v.z = __fmul_rn(__fmul_rn(v.z, scale), w.z); v.w = __fmul_rn(__fmul_rn(v.w, scale), w.w);
+            const bool valid = g < n8;
+            float v[1][8];
+            if (valid) { load8_cg(x + 8 * g, v[0]); }
+            else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { v[0][i] = 0.f; }
             }
-            kq_quantize(v, g, n4, rec + t * col);
+            if (NORM && valid) {
+                float w[8];
+                load8_cg(p.norm_w + 8 * g, w);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { v[0][i] = __fmul_rn(__fmul_rn(v[0][i], scale), w[i]); }
+            }
+            kq_quantize<1>(v, g, n8, rec + t * col);
         }
     }
 }
 
-// One column of at most 512 PG groups of four: every thread keeps its groups of x in registers from the one global read on; x_requested() is
+// One column of at most 512 PG groups of eight: every thread keeps its groups of x in registers from the one global read on; x_requested() is
 // called when the reads are on their way. wearly: the norm weights when the kernel read them at its start (PG <= KQ_NORM_EARLY).
-constexpr int KQ_NORM_EARLY = 3, KQ_PRO_GROUPS = 6;
+constexpr int KQ_NORM_EARLY = 2, KQ_PRO_GROUPS = 3;
 template <int PG, bool NORM, class Requested>
-__device__ __forceinline__ void kq_prologue_1col(const MatvecParams &p, uint32_t *rec, float *scale_s, const float4 *wearly, Requested x_requested) {
+__device__ __forceinline__ void kq_prologue_1col(const MatvecParams &p, uint32_t *rec, float *scale_s, const float (*wearly)[8], Requested x_requested) {
+    constexpr int CQ = PG == 1 ? 2 : 3;                          // (quads per thread of the wide sum: rows of at most 4096 or 6144 values)
     const int tid = threadIdx.x;
-    const int n4  = (int)(p.A.k >> 2);   // a multiple of 64: whole warps, whole blocks
-    const float4 *x4 = reinterpret_cast<const float4 *>(p.x), *w4 = reinterpret_cast<const float4 *>(p.norm_w);
-    float4 xv[PG], wv[PG];
+    const int n4  = (int)(p.A.k >> 2), n8 = (int)(p.A.k >> 3);   // multiples of 64 and 32: whole warps, whole blocks
+    float xv[PG][8], wv[PG][8];
+    auto zero = [](float (&v)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { v[i] = 0.f; }
+    };
 #pragma unroll
     for (int k = 0; k < PG; ++k) {
         const int g = tid + k * KQ_THREADS;
-        xv[k] = g < n4 ? __ldcg(x4 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (g < n8) { load8_cg(p.x + 8 * g, xv[k]); } else { zero(xv[k]); }
     }
     if (NORM) {
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
             const int g = tid + k * KQ_THREADS;
-            if (PG <= KQ_NORM_EARLY) { wv[k] = wearly[k]; }
-            else { wv[k] = g < n4 ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f); }
+            if (PG <= KQ_NORM_EARLY) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { wv[k][i] = wearly[k][i]; }
+            } else if (g < n8) { load8_cg(p.norm_w + 8 * g, wv[k]); } else { zero(wv[k]); }
         }
     }
     x_requested();
@@ -126,26 +146,23 @@ __device__ __forceinline__ void kq_prologue_1col(const MatvecParams &p, uint32_t
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
             const int g = tid + k * KQ_THREADS;
-            if (g < n4) { v3[g] = __fadd_rn(fmaf(xv[k].y, xv[k].y, __fmul_rn(xv[k].x, xv[k].x)), fmaf(xv[k].w, xv[k].w, __fmul_rn(xv[k].z, xv[k].z))); }
+            if (g < n8) { reinterpret_cast<float2 *>(v3)[g] = squares8(xv[k]); }
         }
         __syncthreads();
         float sum = 0.f;
-        if (PG <= KQ_NORM_EARLY && n4 >= RS_MIN && (n4 >> 6) * (KQ_REC - 64) >= rs_scratch_words(PG)) {
-            if (tid < RS_THREADS) { sum = running_sum_chunks<PG <= KQ_NORM_EARLY ? PG : 2>(smem_u32(v3), n4, smem_u32(v3 + n4), tid, 1); }
+        if (PG <= KQ_NORM_EARLY && n4 >= RS_MIN && n4 <= CQ * 512 && (n4 >> 6) * (KQ_REC - 64) >= rs_scratch_words(CQ)) {
+            if (tid < RS_THREADS) { sum = running_sum_chunks<PG <= KQ_NORM_EARLY ? CQ : 2>(smem_u32(v3), n4, smem_u32(v3 + n4), tid, 1); }
         } else if (tid == 0) { sum = running_sum_serial(smem_u32(v3), n4); }
         if (tid == 0) { scale_s[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)p.A.k), p.eps))); }
         __syncthreads();   // also: the partials (aliasing the records) are dead from here on
         const float scale = scale_s[0];
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
-            xv[k].x = __fmul_rn(__fmul_rn(xv[k].x, scale), wv[k].x); xv[k].y = __fmul_rn(__fmul_rn(xv[k].y, scale), wv[k].y);
-            xv[k].z = __fmul_rn(__fmul_rn(xv[k].z, scale), wv[k].z); xv[k].w = __fmul_rn(__fmul_rn(xv[k].w, scale), wv[k].w);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { xv[k][i] = __fmul_rn(__fmul_rn(xv[k][i], scale), wv[k][i]); }
         }
     }
-#pragma unroll
-    for (int k = 0; k < PG; ++k) {
-        if (k * KQ_THREADS < n4) { kq_quantize(xv[k], tid + k * KQ_THREADS, n4, rec); }
-    }
+    kq_quantize<PG>(xv, tid, n8, rec);
 }
 
 // byte i of w (a constant) as the float 2^23 + byte: the byte becomes the low bits of a float's mantissa
@@ -341,13 +358,17 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
 
     // weights never change during a step: the copies may run ahead of the previous kernel's results
     pdl_launch_dependents();
-    constexpr int PG = (PRO == KQP_NORM || PRO == KQP_PLAIN) ? 2 : PRO == KQP_NORM_MID ? 3 : KQ_PRO_GROUPS;
-    float4 wearly[PRO == KQP_NORM_MID ? 3 : 2];
+    constexpr int PG = (PRO == KQP_NORM || PRO == KQP_PLAIN) ? 1 : PRO == KQP_NORM_MID ? 2 : KQ_PRO_GROUPS;
+    float wearly[PRO == KQP_NORM_MID ? 2 : 1][8];
     if (PRO == KQP_NORM || PRO == KQP_NORM_MID) {
 #pragma unroll
         for (int k = 0; k < (PG < 4 ? PG : 0); ++k) {
             const int g = threadIdx.x + k * KQ_THREADS;
-            wearly[k] = g < (int)(p.A.k >> 2) ? reinterpret_cast<const float4 *>(p.norm_w)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (g < (int)(p.A.k >> 3)) { load8_cg(p.norm_w + 8 * g, wearly[k]); }
+            else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { wearly[k][i] = 0.f; }
+            }
         }
     }
     if (lane == 0 && n_stage > 0) {
@@ -513,7 +534,7 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg) {
         // (narrow models: a layer's matrices of both types on one kernel, whose instructions the next launch finds in the caches; four layers of
         // Q4_K / Q6_K with d = 512, ff 1536: 125.2 -> 105.7 us a step; 1024, 2816: 129.3 -> 109.8; 2048, 5632: 137.0 -> 133.8; 3072, 8192: 188.2 ->
         // 186.9; but 4096, 11008: 227.2 -> 235.9)
-        kernel = p.narrow ? one[KQP_ANY][2] : one[n4 <= 2 * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : norm && n4 <= 3 * KQ_THREADS ? KQP_NORM_MID : n4 <= KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY][ty];
+        kernel = p.narrow ? one[KQP_ANY][2] : one[n4 <= 2 * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : norm && n4 <= 3 * KQ_THREADS ? KQP_NORM_MID : n4 <= 2 * KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY][ty];
     } else {
         static const Kernel more[2][3] = {{matvec_kq_kernel<2, 12, KQP_ANY>, matvec_kq_kernel<2, 14, KQP_ANY>, matvec_kq_kernel<2, 0, KQP_ANY>},
                                           {matvec_kq_kernel<KQ_MAX_COLUMNS, 12, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 14, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 0, KQP_ANY>}};

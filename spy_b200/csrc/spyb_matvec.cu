@@ -117,22 +117,28 @@ cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
 //   product of each pair plain, the second fused into an FMA, as the CPU build evaluates it) and added to
 //   the running sum one group after the other; y = x * (1 / sqrt(sum/n + eps)). The groups are formed in
 //   parallel, the running sum is one thread's chain. Mul (basic.cpp:15-50): y * norm_weight.
-// Single column, K <= 12288: every thread keeps its (at most PG) float4 groups of x in registers from the one
+// Single column, K <= 12288: every thread keeps its (at most PG) groups of eight x in registers from the one
 // global read through the sum of squares to the quantizer; same arithmetic as the general prologue below.
-constexpr int PRO_GROUPS = 6;
+// (Eight values a thread: a 256-bit load each, half the shuffles and lane bookkeeping of groups of four. Behind the last read of 11008 values:
+// 2.1 us with groups of four, two quotients each and the conversion unit, 1.3 now; a 7B Q4_0 layer 45.9 -> 44.8 us.)
+constexpr int PRO_GROUPS = 3;
 // SUM: how the sum of squares is formed. SUM_FEW: by one thread in few registers (kernels with other paths to serve); SUM_CHAIN: by one thread
 // that reads ahead; SUM_WIDE (kernels of their own per prologue): the sum of squares runs on four warps and the
-// norm weights of rows of at most NORM_EARLY * 512 groups are read at the start of the kernel, in front of the weight copies: behind a ring
+// norm weights of rows of at most NORM_EARLY * 4096 values are read at the start of the kernel, in front of the weight copies: behind a ring
 // full of them on every SM they arrive after the sum of squares is done.
-constexpr int NORM_EARLY = 3;
+constexpr int NORM_EARLY = 2;
 enum { SUM_FEW, SUM_CHAIN, SUM_WIDE };
 template <int PG>
-__device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float4 (&w)[PG]) {
-    const int n4 = (int)(p.A.k >> 2);
+__device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float (&w)[PG][8]) {
+    const int n8 = (int)(p.A.k >> 3);
 #pragma unroll
     for (int k = 0; k < PG; ++k) {
         const int g = threadIdx.x + k * MV_THREADS;
-        w[k] = (p.pro == PRO_NORM_QUANT && g < n4) ? reinterpret_cast<const float4 *>(p.norm_w)[g] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p.pro == PRO_NORM_QUANT && g < n8) { load8_cg<true>(p.norm_w + 8 * g, w[k]); }
+        else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { w[k][i] = 0.f; }
+        }
     }
 }
 // the running sum in few registers, for kernels that hold several prologues
@@ -151,47 +157,55 @@ __device__ __forceinline__ float running_sum_small(const float *v3, int n4) {
     return sum;
 }
 
-template <int PG, bool NORM, int SUM, class Requested>
-__device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActPlanes act, float *v3, float *scales, const float4 *wearly, Requested x_requested) {
+// an eight-value group's words in the activation planes, and a block's scale
+__device__ __forceinline__ void act_store(const MatvecParams &p, uint32_t *Yw, int g, uint2 q) {
+    const int b = g >> 2, at = ((b >> 2) * 8 + 2 * (g & 3)) * 4 + (b & 3);
+    Yw[at] = q.x; Yw[at + 4] = q.y;
+}
+__device__ __forceinline__ float act_scale(const MatvecParams &p, float d) { const float r = h2f(f2h(d)); return (p.A.type == 2) ? __fmul_rn(r, 0.0625f) : r; }
+
+template <int PG, bool NORM, int SUM, bool A32, class Requested>
+__device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActPlanes act, float *v3, float *scales, const float (*wearly)[8], Requested x_requested) {
     constexpr bool EARLY = SUM == SUM_WIDE;
+    constexpr int  CQ = PG == 1 ? 2 : 3;                       // (quads per thread of the wide sum: rows of at most 4096 or 6144 values)
     const int tid = threadIdx.x;
     const int nbp = p.A.nbp;
-    const int n4  = (int)(p.A.k >> 2);
-    const int n4p = nbp * 8;                                   // float4 groups including the zero padding up to nbp blocks
-    const int npass = (n4p + MV_THREADS - 1) / MV_THREADS;     // <= PG
-    const float4 *x4 = reinterpret_cast<const float4 *>(p.x);
-    float4 xv[PG];
+    const int n4  = (int)(p.A.k >> 2), n8 = (int)(p.A.k >> 3);
+    const int n8p = nbp * 4;                                   // groups of eight including the zero padding up to nbp blocks
+    const int npass = (n8p + MV_THREADS - 1) / MV_THREADS;     // <= PG
+    float xv[PG][8];
     // (activations are read past L1: under tensor parallelism other GPUs wrote part of them)
 #pragma unroll
     for (int k = 0; k < PG; ++k) {
         const int g = tid + k * MV_THREADS;
-        xv[k] = (k < npass && g < n4) ? __ldcg(x4 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k < npass && g < n8) { load8_cg<A32>(p.x + 8 * g, xv[k]); }
+        else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { xv[k][i] = 0.f; }
+        }
     }
     x_requested();
     if (NORM) {
-        const float4 *w4 = reinterpret_cast<const float4 *>(p.norm_w);
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
             const int g = tid + k * MV_THREADS;
-            if (k < npass && g < n4) {
-                const float4 v = xv[k];
-                const float v1 = fmaf(v.y, v.y, __fmul_rn(v.x, v.x));
-                const float v2 = fmaf(v.w, v.w, __fmul_rn(v.z, v.z));
-                v3[g] = __fadd_rn(v1, v2);
-            }
+            if (k < npass && g < n8) { reinterpret_cast<float2 *>(v3)[g] = squares8(xv[k]); }
         }
         // the norm weights: in registers already, or arriving while the sum of squares is formed
-        float4 wv[PG];
+        float wv[PG][8];
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
             const int g = tid + k * MV_THREADS;
-            if (EARLY) { wv[k] = wearly[k]; }
-            else { wv[k] = (k < npass && g < n4) ? w4[g] : make_float4(0.f, 0.f, 0.f, 0.f); }
+            if (!EARLY && k < npass && g < n8) { load8_cg<A32>(p.norm_w + 8 * g, wv[k]); }
+            else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { wv[k][i] = EARLY ? wearly[k][i] : 0.f; }
+            }
         }
         __syncthreads();
-        __shared__ __align__(16) float rs_scratch[EARLY ? rs_scratch_words(PG) : 4];
+        __shared__ __align__(16) float rs_scratch[EARLY ? rs_scratch_words(CQ) : 4];
         float sum = 0.f;
-        if (EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<EARLY ? PG : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
+        if (EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<EARLY ? CQ : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
         else if (tid == 0) { sum = SUM == SUM_CHAIN ? running_sum_serial(smem_u32(v3), n4) : running_sum_small(v3, n4); }
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
@@ -201,27 +215,19 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
         const float scale = scales[0];
 #pragma unroll
         for (int k = 0; k < PG; ++k) {
-            xv[k].x = __fmul_rn(__fmul_rn(xv[k].x, scale), wv[k].x);
-            xv[k].y = __fmul_rn(__fmul_rn(xv[k].y, scale), wv[k].y);
-            xv[k].z = __fmul_rn(__fmul_rn(xv[k].z, scale), wv[k].z);
-            xv[k].w = __fmul_rn(__fmul_rn(xv[k].w, scale), wv[k].w);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { xv[k][i] = __fmul_rn(__fmul_rn(xv[k][i], scale), wv[k][i]); }
         }
     }
-    uint32_t *Yw = reinterpret_cast<uint32_t *>(act.Y);
-    float    *DS = reinterpret_cast<float *>(act.DS);
+    uint2 q[PG];
+    int   kd;
+    const float d = quantize_q8_groups<PG>(xv, npass, q, kd);   // (npass is uniform over the CTA: the quantizer's shuffles see full warps)
 #pragma unroll
     for (int k = 0; k < PG; ++k) {
-        if (k < npass) {   // uniform over the CTA: the quantizer's shuffles see full warps
-            const int g = tid + k * MV_THREADS;
-            uint16_t dh; int sum;
-            const uint32_t q = quantize_q8_lane4(xv[k], dh, sum);
-            if (g < n4p) {
-                const int b = g >> 3, w = g & 7;
-                Yw[(((b >> 2)) * 8 + w) * 4 + (b & 3)] = q;
-                if (w == 0) { const float d = h2f(dh); DS[b] = (p.A.type == 2) ? __fmul_rn(d, 0.0625f) : d; }
-            }
-        }
+        const int g = tid + k * MV_THREADS;
+        if (k < npass && g < n8p) { act_store(p, reinterpret_cast<uint32_t *>(act.Y), g, q[k]); }
     }
+    if (kd >= 0 && tid + kd * MV_THREADS < n8p) { reinterpret_cast<float *>(act.DS)[(tid + kd * MV_THREADS) >> 2] = act_scale(p, d); }
 }
 
 template <int TM>
@@ -250,31 +256,33 @@ __device__ __forceinline__ void matvec_prologue(const MatvecParams &p, ActPlanes
     }
     uint32_t *Yw = reinterpret_cast<uint32_t *>(act.Y);
     float    *DS = reinterpret_cast<float *>(act.DS);
-    const int n4p = nbp * 8;   // float4 groups including the zero padding up to nbp blocks
+    const int n8 = (int)(K >> 3), n8p = nbp * 4;   // groups of eight; including the zero padding up to nbp blocks
 #pragma unroll 1
     for (int t = 0; t < TM; ++t) {
         const bool    col  = t < p.T;    // unused columns are zeros with zero scales: every contribution vanishes
-        const float4 *x4 = reinterpret_cast<const float4 *>(p.x + (int64_t)(col ? t : 0) * p.x_stride);
-        const float4 *w4 = reinterpret_cast<const float4 *>(p.norm_w);
+        const float  *x = p.x + (int64_t)(col ? t : 0) * p.x_stride;
         const float scale = (col && p.pro == PRO_NORM_QUANT) ? scales[t] : 1.f;
-        for (int base = 0; base < n4p; base += MV_THREADS) {
+        for (int base = 0; base < n8p; base += MV_THREADS) {
             const int  g     = base + tid;
-            const bool valid = col && g < n4;
-            float4 v = valid ? __ldcg(x4 + g) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (p.pro == PRO_NORM_QUANT && valid) {
-                const float4 w = w4[g];
-                v.x = __fmul_rn(__fmul_rn(v.x, scale), w.x);
-                v.y = __fmul_rn(__fmul_rn(v.y, scale), w.y);
-                v.z = __fmul_rn(__fmul_rn(v.z, scale), w.z);
-                v.w = __fmul_rn(__fmul_rn(v.w, scale), w.w);
+            const bool valid = col && g < n8;
+            float v[1][8];
+            if (valid) { load8_cg(x + 8 * g, v[0]); }
+            else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { v[0][i] = 0.f; }
             }
-            uint16_t dh; int s;
-            const uint32_t q = quantize_q8_lane4(v, dh, s);
-            if (g < n4p) {
-                const int b = g >> 3, w = g & 7;
-                const int idx = ((t * (nbp >> 2) + (b >> 2)) * 8 + w) * 4 + (b & 3);
-                Yw[idx] = q;
-                if (w == 0) { const float d = h2f(dh); DS[t * nbp + b] = (p.A.type == 2) ? __fmul_rn(d, 0.0625f) : d; }
+            if (p.pro == PRO_NORM_QUANT && valid) {
+                float w[8];
+                load8_cg(p.norm_w + 8 * g, w);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { v[0][i] = __fmul_rn(__fmul_rn(v[0][i], scale), w[i]); }
+            }
+            uint2 q[1];
+            int kd;
+            const float d = quantize_q8_groups<1>(v, 1, q, kd);
+            if (g < n8p) {
+                act_store(p, Yw + (size_t)t * nbp * 8, g, q[0]);
+                if (kd == 0) { DS[t * nbp + (g >> 2)] = act_scale(p, d); }
             }
         }
     }
@@ -374,9 +382,9 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<2, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); }
-        } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); }
+            if (norm) { matvec_prologue_1col<1, true, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<1, false, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); }
+        } else if (TM == 1 && n4p <= 2 * PRO_GROUPS * MV_THREADS) {
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else {
             matvec_prologue<TM>(p, act, v3, norm_scales);
         }
@@ -567,7 +575,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     };
 
     pdl_launch_dependents();
-    float4 wearly[PRO == MVP_NORM_MID ? 3 : 2];
+    float wearly[PRO == MVP_NORM_MID ? 2 : 1][8];
     if (PRO == MVP_NORM || PRO == MVP_NORM_MID) { norm_weights_early(p, wearly); }
     stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
     if (lane == 0 && n_items > 0) {
@@ -589,15 +597,15 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
         else if constexpr (PRO == MVP_ONE) {
             const bool norm = p.pro == PRO_NORM_QUANT;
             if (nbp * 8 <= 2 * MV_THREADS) {
-                if (norm) { matvec_prologue_1col<2, true, SUM_CHAIN>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<2, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, rest); }
+                if (norm) { matvec_prologue_1col<1, true, SUM_CHAIN, true>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<1, false, SUM_FEW, true>(p, act, v3, norm_scales, nullptr, rest); }
             } else {
-                if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_CHAIN>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, rest); }
+                if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_CHAIN, true>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW, true>(p, act, v3, norm_scales, nullptr, rest); }
             }
         }
         else {
             constexpr bool NORM = PRO == MVP_NORM || PRO == MVP_NORM_MID || PRO == MVP_NORM_LONG;
-            constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 2 : PRO == MVP_NORM_MID ? 3 : PRO_GROUPS;
-            matvec_prologue_1col<PG, NORM, NORM && PG <= NORM_EARLY ? SUM_WIDE : SUM_FEW>(p, act, v3, norm_scales, wearly, rest);
+            constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 1 : PRO == MVP_NORM_MID ? 2 : PRO_GROUPS;
+            matvec_prologue_1col<PG, NORM, NORM && PG <= NORM_EARLY ? SUM_WIDE : SUM_FEW, true>(p, act, v3, norm_scales, wearly, rest);
         }
     }
     __syncthreads();
@@ -787,9 +795,9 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_mma_kernel(const MatvecP
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<2, true, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<2, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); }
-        } else if (TM == 1 && n4p <= PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW>(p, act, v3, norm_scales, nullptr, []() {}); }
+            if (norm) { matvec_prologue_1col<1, true, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<1, false, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); }
+        } else if (TM == 1 && n4p <= 2 * PRO_GROUPS * MV_THREADS) {
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else {
             matvec_prologue<TM>(p, act, v3, norm_scales);
         }
@@ -924,13 +932,15 @@ static cudaError_t launch_matvec_rows_t(const MatvecParams &p, const LaunchCfg &
     if (ring / ((size_t)wact * S * RECB) < 1) { return cudaErrorInvalidValue; }
     const size_t smem = fixed.total + ring;
     void (*kernel)(const MatvecParams, const int, const int, const int) = matvec_rows_kernel<WT, TM, LPR, MVP_ANY>;
-    if constexpr (TM == 1) {
+    // (the kernels of single prologues read x and the norm weights 32 bytes at a time; a model's buffers lie on 256)
+    const bool aligned = ((reinterpret_cast<uintptr_t>(p.x) | (p.pro == PRO_NORM_QUANT ? reinterpret_cast<uintptr_t>(p.norm_w) : 0)) & 31) == 0;
+    if constexpr (TM == 1) if (aligned) {
         const int  n4p = p.A.nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
-        if (p.narrow && n4p <= PRO_GROUPS * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_ONE>; }
+        if (p.narrow && n4p <= 2 * PRO_GROUPS * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_ONE>; }
         else if (n4p <= 2 * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN>; }
         else if (norm && n4p <= 3 * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_NORM_MID>; }
-        else if (n4p <= PRO_GROUPS * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM_LONG> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN_LONG>; }
+        else if (n4p <= 2 * PRO_GROUPS * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM_LONG> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN_LONG>; }
     }
     cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem);
     if (err != cudaSuccess) { return err; }

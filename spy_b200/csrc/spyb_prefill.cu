@@ -29,7 +29,7 @@ namespace spyb {
 namespace {
 
 constexpr int PF_QUANT_THREADS = 512;
-constexpr int PF_QUANT_GROUPS  = PF_MAX_K / (4 * PF_QUANT_THREADS);   // float4 groups per thread
+constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF_QUANT_THREADS);   // groups of eight values per thread
 
 // ---------------------------------------------------------------------------------------------
 // the GEMM: persistent CTAs (one per SM, all 512 tensor-memory columns), each walking tiles of 128 rows x TT tokens along K in
@@ -335,31 +335,42 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
     const int tid = threadIdx.x, token = blockIdx.x;
     pdl_launch_dependents();
     pdl_wait();
-    const int n4 = K >> 2, nb = K >> 5;
-    const int npass = (n4 + PF_QUANT_THREADS - 1) / PF_QUANT_THREADS;
+    const int n4 = K >> 2, n8 = K >> 3, nb = K >> 5;
+    const int npass = (n8 + PF_QUANT_THREADS - 1) / PF_QUANT_THREADS;
     // a row may lie in parts (the slices the ranks of a tensor-parallel group gathered): elements [i part_len, (i + 1) part_len)
-    // of token t at x + i part_stride + t x_stride; one part = the plain row
+    // of token t at x + i part_stride + t x_stride; one part = the plain row (parts are multiples of four values)
     const float *xrow = x + (int64_t)token * x_stride;
-    float4 xv[PF_QUANT_GROUPS];
+    float xv[PF_QUANT_GROUPS][8];
 #pragma unroll
     for (int k = 0; k < PF_QUANT_GROUPS; ++k) {
         const int gi = tid + k * PF_QUANT_THREADS;
-        if (k < npass && gi < n4) {
-            const int e = 4 * gi, part = e / part_len;
-            xv[k] = *reinterpret_cast<const float4 *>(xrow + (int64_t)part * part_stride + (e - part * part_len));
-        } else { xv[k] = make_float4(0.f, 0.f, 0.f, 0.f); }
+        if (k < npass && gi < n8) {
+            if (part_len == K) { load8_cg(xrow + 8 * gi, xv[k]); }
+            else {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int e = 8 * gi + 4 * h, part = e / part_len;
+                    const float4 v = *reinterpret_cast<const float4 *>(xrow + (int64_t)part * part_stride + (e - part * part_len));
+                    xv[k][4 * h] = v.x; xv[k][4 * h + 1] = v.y; xv[k][4 * h + 2] = v.z; xv[k][4 * h + 3] = v.w;
+                }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { xv[k][i] = 0.f; }
+        }
     }
     if (NORM) {
-        const float4 *w4 = reinterpret_cast<const float4 *>(norm_w);
-        float4 wv[PF_QUANT_GROUPS];
+        float wv[PF_QUANT_GROUPS][8];
 #pragma unroll
         for (int k = 0; k < PF_QUANT_GROUPS; ++k) {
             const int gi = tid + k * PF_QUANT_THREADS;
-            if (k < npass && gi < n4) {
-                const float4 v = xv[k];
-                v3[gi] = __fadd_rn(fmaf(v.y, v.y, __fmul_rn(v.x, v.x)), fmaf(v.w, v.w, __fmul_rn(v.z, v.z)));
-                wv[k] = w4[gi];
-            } else { wv[k] = make_float4(0.f, 0.f, 0.f, 0.f); }
+            if (k < npass && gi < n8) {
+                reinterpret_cast<float2 *>(v3)[gi] = squares8(xv[k]);
+                load8_cg(norm_w + 8 * gi, wv[k]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { wv[k][i] = 0.f; }
+            }
         }
         __syncthreads();
         if (tid == 0) {
@@ -377,39 +388,47 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
         const float scale = scale_s;
 #pragma unroll
         for (int k = 0; k < PF_QUANT_GROUPS; ++k) {
-            xv[k].x = __fmul_rn(__fmul_rn(xv[k].x, scale), wv[k].x);
-            xv[k].y = __fmul_rn(__fmul_rn(xv[k].y, scale), wv[k].y);
-            xv[k].z = __fmul_rn(__fmul_rn(xv[k].z, scale), wv[k].z);
-            xv[k].w = __fmul_rn(__fmul_rn(xv[k].w, scale), wv[k].w);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { xv[k][i] = __fmul_rn(__fmul_rn(xv[k][i], scale), wv[k][i]); }
         }
     }
     uint8_t *tile = yq + ((int64_t)(token / TOKT) * nb) * YQB;
     const int tt = token % TOKT;
+    uint2 qv[PF_QUANT_GROUPS];
+    int kd;
+    const float d = quantize_q8_groups<PF_QUANT_GROUPS>(xv, npass, qv, kd);   // (npass is uniform over the CTA: the quantizer's shuffles see full warps)
+    if (kd >= 0 && tid + kd * PF_QUANT_THREADS < n8) {
+        const int b = (tid + kd * PF_QUANT_THREADS) >> 2;
+        const uint16_t dh = f2h(d);
+        reinterpret_cast<float *>(tile + (int64_t)b * YQB + SCALES)[tt] = h2f(dh);
+        if (tap != nullptr && token == 0) { *reinterpret_cast<uint16_t *>(tap + (int64_t)b * 34) = dh; }
+    }
 #pragma unroll
     for (int k = 0; k < PF_QUANT_GROUPS; ++k) {
-        if (k < npass) {   // uniform over the CTA: the quantizer's shuffles see full warps
+        if (k < npass) {
             const int gi = tid + k * PF_QUANT_THREADS;
-            uint16_t dh; int sum;
-            const uint32_t q = quantize_q8_lane4(xv[k], dh, sum);
-            if (KQ) {   // the block's sum over its eight lanes
-                sum += __shfl_xor_sync(0xffffffffu, sum, 1); sum += __shfl_xor_sync(0xffffffffu, sum, 2); sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+            const uint2 q = qv[k];
+            int sum = 0;
+            if (KQ) {   // the block's sum over its four lanes
+                sum = q8_sum8(q);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1); sum += __shfl_xor_sync(0xffffffffu, sum, 2);
             }
-            if (gi < n4) {
-                const int b = gi >> 3, w = gi & 7;
+            if (gi < n8) {
+                const int b = gi >> 2, w = gi & 3;
                 uint8_t *blk = tile + (int64_t)b * YQB;
-                auto h = [&](int i) { return (uint32_t)__half_as_ushort(__int2half_rn((int)(int8_t)(q >> (8 * i)))); };
-                const uint2 v = make_uint2(h(0) | (h(1) << 16), h(2) | (h(3) << 16));
+                // byte + 128 as the low byte of the f16 1024 + (byte + 128), less 1152: the value as f16
+                auto halves = [](uint32_t bytes, uint32_t sel) {
+                    uint32_t h = __byte_perm(bytes ^ 0x80808080u, 0x64646464u, sel);
+                    *reinterpret_cast<__half2 *>(&h) = __hsub2(*reinterpret_cast<__half2 *>(&h), __float2half2_rn(1152.f));
+                    return h;
+                };
+                const uint4 v = make_uint4(halves(q.x, 0x4140), halves(q.x, 0x4342), halves(q.y, 0x4140), halves(q.y, 0x4342));
                 if (tap != nullptr && token == 0) {   // reference-layout blocks of token 0 (34-byte records: only 2-byte alignment holds)
-                    uint16_t *o = reinterpret_cast<uint16_t *>(tap + (int64_t)b * 34);
-                    o[1 + 2 * w] = (uint16_t)q; o[2 + 2 * w] = (uint16_t)(q >> 16);
-                    if (w == 0) { o[0] = dh; }
+                    uint16_t *o = reinterpret_cast<uint16_t *>(tap + (int64_t)b * 34) + 1 + 4 * w;
+                    o[0] = (uint16_t)q.x; o[1] = (uint16_t)(q.x >> 16); o[2] = (uint16_t)q.y; o[3] = (uint16_t)(q.y >> 16);
                 }
-                if (KQ) { *reinterpret_cast<uint2 *>(blk + (w >> 1) * 16 * TOKT + tt * 16 + (w & 1) * 8) = v; }
-                else    { reinterpret_cast<uint2 *>(blk + tt * 64)[w] = v; }
-                if (w == 0) {
-                    reinterpret_cast<float *>(blk + SCALES)[tt] = h2f(dh);
-                    if (KQ) { reinterpret_cast<float *>(blk + SCALES + TOKT * 4)[tt] = (float)sum; }
-                }
+                *reinterpret_cast<uint4 *>(KQ ? blk + w * 16 * TOKT + tt * 16 : blk + tt * 64 + w * 16) = v;
+                if (KQ && w == 0) { reinterpret_cast<float *>(blk + SCALES + TOKT * 4)[tt] = (float)sum; }
             }
         }
     }

@@ -779,3 +779,49 @@ def test_lookup_tables_identical_for_every_key(be, oracle):
     want_silu, want_exp = oracle.tables()
     assert np.array_equal(bits(silu), bits(want_silu))
     assert np.array_equal(bits(ex), bits(want_exp))
+
+
+# --------------------------------------------------------------------------- the mat-vec kernels' quantizer on values that are hard to round
+HARD_K = [32, 96, 1024, 4096, 4128, 6144, 8224, 11008]
+
+
+def hard_values(k: int, seed: int) -> np.ndarray:
+    """Blocks of ties (odd multiples of half a step), of zeros, of subnormal and of huge values, of one outlier, and of ordinary ones."""
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal(k).astype(np.float32).reshape(-1, 32)
+    kind = np.arange(len(x)) % 7
+    x[kind == 1] = 0.0
+    ties = (rng.integers(-126, 126, size=(int((kind == 2).sum()), 32)) + 0.5).astype(np.float32)
+    ties[:, 0] = 127.0
+    x[kind == 2] = ties
+    x[kind == 3] *= np.float32(1e-38)
+    x[kind == 4] *= np.float32(1e5)
+    x[kind == 5, 7] = 3000.0
+    return x.reshape(-1)
+
+
+@pytest.mark.parametrize("k", HARD_K)
+@pytest.mark.parametrize("cols", [1, 3, 9])
+@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_quantizer_on_hard_values(be, oracle, qt, cols, k, offset):
+    """Each row of W picks one value of the quantized activations (a single nonzero weight), so that every byte shows: the oracle's bits from
+    the mat-vec kernels and the GEMM, over the remainders and numbers of values per thread of their quantizers, and for activations that
+    lie on 16 bytes only (offset: floats)."""
+    n = 64
+    x = np.stack([hard_values(k, 91 + c) for c in range(cols)])
+    rng = np.random.default_rng(5)
+    w = np.zeros((n, k), dtype=np.float32)
+    w[np.arange(n), rng.integers(0, k, n)] = 1.0
+    raw = quants.quantize(w, qt)
+    px = be.upload(np.concatenate([np.zeros(offset, dtype=np.float32), x.reshape(-1)]))
+    pw, po = be.upload_constant(f"hard {qt} {k} {cols} {offset}", raw, qt, (k, n)), be.alloc_memory(4 * n * cols)
+    d = B.OpDesc()
+    d.op_type, d.num_input = B.OP["MatMul"], 2
+    d.input[0] = B.make_tensor(pw, qt, (k, n), None, B.NODE_CONSTANT)
+    d.input[1] = B.make_tensor(px + 4 * offset, B.FP32, (k, cols))
+    d.output = B.make_tensor(po, B.FP32, (n, cols))
+    be.submit(d)
+    got = be.download(po, (cols, n), np.float32)
+    be.dealloc_memory(px, 4 * (x.size + offset)); be.dealloc_memory(po, 4 * n * cols)
+    assert close(got, oracle.matmul(qt, raw, k, n, x))
