@@ -152,8 +152,10 @@ cudaError_t launch_prefill_silu_mul(const float *upgate, int T, int F, const flo
 struct PrefillKeep { const uint4 *src[4] = {}; uint4 *dst[4] = {}; int64_t n4[4] = {}; };   // up to four 16-byte-aligned copies
 cudaError_t launch_prefill_keep(const PrefillKeep &k, cudaStream_t stream);
 
+enum { ATT_BY_CONTEXT, ATT_ONE_CTA, ATT_CLUSTER };
 struct AttnParams {
     int           force_long = 0;     // take the three-kernel path (scratch needed) also at short contexts
+    int           form = ATT_BY_CONTEXT;   // of a single token's step: by the context length, or the kernel that its position makes the faster one
     const __half *q = nullptr;        // [T][dl], already rounded to fp16
     const __half *k_cache = nullptr;  // [n_ctx][dl]
     const __half *v_cache = nullptr;  // [dl][n_ctx]
@@ -215,6 +217,7 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg);   // 
 int64_t     kq_row_bytes(int type, int64_t k);                             // bytes of one K-quant row in device memory
 cudaError_t launch_kq_relayout_q6k(const uint8_t *raw, int64_t n_rows, int64_t k, uint8_t *dst, cudaStream_t s);
 cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg);
+int         attention_form(const AttnParams &p, const LaunchCfg &cfg, int pos);   // AttnParams::form for a single token at position pos
 int         attn_ring_selftest();   // host-only: 0 when every slot of the step kernel's ring keeps its writer and its reader
 size_t      attention_scratch_floats(int n_ctx, int n_head, int T);
 

@@ -210,11 +210,15 @@ struct spyb_model {
     float   *logits_batch = nullptr;
     int32_t *batch_tokens = nullptr, *batch_ids = nullptr;
     int64_t  batch_ids_cap = 0;
-    cudaGraphExec_t graph_exec = nullptr;
-    cudaGraphExec_t graph_eval1 = nullptr;   // single-token spyb_model_eval: staging copies, embedding, layers, head, logits copy
+    // Captured steps: a captured step holds the cache addresses of its sequence and the attention kernel of its form. The least recently used
+    // goes when there are MAX_STEP_GRAPHS.
+    struct StepGraph { cudaGraphExec_t exec; int kind, seq, form; int64_t launches; uint64_t used; };
+    std::vector<StepGraph> graphs;
+    uint64_t graph_uses = 0;
+    int      att_form = ATT_BY_CONTEXT;      // of the step that is being enqueued
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float   last_ms = 0.f;
-    int64_t last_launches = 0, eval1_launches = 0;
+    int64_t last_launches = 0;
     std::vector<void *> owned;
 };
 
@@ -420,7 +424,7 @@ spyb_status run_layers(spyb_model *m, int T, bool tap, int64_t *launches, int se
             a.pos_base = m->d_pos; a.exp_table = be->d_exp_table;
             a.n_head = m->dl / m->info.head_dim; a.hd = m->info.head_dim; a.dl = m->dl; a.T = T; a.n_ctx = m->info.n_ctx;
             a.scale = 1.0f / std::sqrt((float)m->info.head_dim);
-            a.stamps = stamps(1); a.error_flag = be->d_error_flag; a.scratch = m->att_scratch;
+            a.stamps = stamps(1); a.error_flag = be->d_error_flag; a.scratch = m->att_scratch; a.form = T == 1 && seq0 < 0 ? m->att_form : ATT_BY_CONTEXT;
             if (seq0 >= 0) { a.seq_stride = m->seq_stride; a.k_cache = ly.k_base + (int64_t)seq0 * m->seq_stride; a.v_cache = ly.v_base + (int64_t)seq0 * m->seq_stride; }
             if (fused) { tp_produce(m, a.tp, 2 * L, true); }
             SPYB_CUDA(be, launch_attention(a, cfg)); ++*launches;
@@ -586,6 +590,34 @@ spyb_status run_head_columns(spyb_model *m, int T, float *out, int64_t *launches
     p.norm_w = m->output_norm; p.eps = m->info.rms_eps; p.epi = EPI_STORE; p.out = out; p.out_stride = m->info.n_vocab;
     SPYB_CUDA(m->be, launch_matvec(p, m->be->launch_cfg(m->be->config.use_pdl != 0))); ++*launches;
     return SPYB_SUCCESS;
+}
+
+// the attention kernel of a single token's step at position pos
+int step_form(const spyb_model *m, int pos) {
+    if (m->step_ok || m->info.tp_size != 1 || m->layers.empty()) { return ATT_BY_CONTEXT; }
+    AttnParams a;
+    a.k_cache = m->layers[0].k_cache; a.v_cache = m->layers[0].v_cache;
+    a.n_head = m->dl / m->info.head_dim; a.hd = m->info.head_dim; a.dl = m->dl; a.n_ctx = m->info.n_ctx;
+    return attention_form(a, m->be->launch_cfg(false), pos);
+}
+
+// the captured step of this kind for the model's sequence and m->att_form; null: not captured yet
+enum { GRAPH_DECODE, GRAPH_EVAL };
+constexpr size_t MAX_STEP_GRAPHS = 32;
+spyb_model::StepGraph *find_graph(spyb_model *m, int kind) {
+    for (auto &g : m->graphs) {
+        if (g.kind == kind && g.seq == m->cur_seq && g.form == m->att_form) { g.used = ++m->graph_uses; return &g; }
+    }
+    return nullptr;
+}
+spyb_model::StepGraph *keep_graph(spyb_model *m, int kind, cudaGraphExec_t exec, int64_t launches) {   // (the stream is idle: called behind a capture)
+    if (m->graphs.size() >= MAX_STEP_GRAPHS) {
+        auto oldest = std::min_element(m->graphs.begin(), m->graphs.end(), [](const auto &a, const auto &b) { return a.used < b.used; });
+        cudaGraphExecDestroy(oldest->exec);
+        m->graphs.erase(oldest);
+    }
+    m->graphs.push_back({exec, kind, m->cur_seq, m->att_form, launches, ++m->graph_uses});
+    return &m->graphs.back();
 }
 
 spyb_status run_decode_step(spyb_model *m, int64_t *launches) {
@@ -944,8 +976,7 @@ void spyb_model_free(spyb_model *m) {
     if (m == nullptr) { return; }
     cudaSetDevice(m->be->config.device_id);
     cudaStreamSynchronize(m->be->stream);
-    if (m->graph_exec) { cudaGraphExecDestroy(m->graph_exec); }
-    if (m->graph_eval1) { cudaGraphExecDestroy(m->graph_eval1); }
+    for (auto &g : m->graphs) { cudaGraphExecDestroy(g.exec); }
     if (m->nccl_comm && g_nccl.CommDestroy) { g_nccl.CommDestroy(m->nccl_comm); }
     for (void *p : m->owned) { cudaFree(p); }
     if (m->h_pos_pinned) { cudaFreeHost(m->h_pos_pinned); }
@@ -1016,13 +1047,16 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
     for (int i = 0; i < n_tokens; ++i) { if (tokens[i] < 0 || tokens[i] >= m->info.n_vocab) { be->set_error("token id %d out of range", tokens[i]); return SPYB_FAIL; } }
     int64_t launches = 0;
     if (n_tokens == 1 && be->config.use_graph != 0 && (m->info.tp_size == 1 || std::getenv("SPYB_TP_NO_GRAPH") == nullptr)) {
-        // the host-driven token loop: one captured graph per model (staging words and the logits go through pinned
+        // the host-driven token loop: one captured graph per sequence and form of the attention (staging words and the logits go through pinned
         // memory whose addresses are fixed, so the graph replays unchanged for every token)
         SPYB_CUDA(be, cudaStreamSynchronize(be->stream));
         m->h_pos_pinned[0] = n_past; m->h_pos_pinned[1] = n_past + 1; m->h_pos_pinned[2] = ++m->epoch;
         m->h_tok_pinned[0] = tokens[0];
-        for (int attempt = 0; m->graph_eval1 == nullptr; ++attempt) {
+        m->att_form = step_form(m, n_past);
+        spyb_model::StepGraph *step = find_graph(m, GRAPH_EVAL);
+        for (int attempt = 0; step == nullptr; ++attempt) {
             cudaGraph_t graph = nullptr;
+            cudaGraphExec_t exec = nullptr;
             SPYB_CUDA(be, cudaStreamBeginCapture(be->stream, cudaStreamCaptureModeThreadLocal));
             spyb_status st = SPYB_SUCCESS;
             cudaError_t ce = cudaMemcpyAsync(m->d_pos, m->h_pos_pinned, 12, cudaMemcpyHostToDevice, be->stream);
@@ -1038,24 +1072,24 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
             const cudaError_t ee = cudaStreamEndCapture(be->stream, &graph);
             cudaError_t ie = cudaSuccess;
             if (ce == cudaSuccess && st == SPYB_SUCCESS && ee == cudaSuccess) {
-                ie = cudaGraphInstantiate(&m->graph_eval1, graph, 0);
-                if (ie != cudaSuccess) { m->graph_eval1 = nullptr; }
+                ie = cudaGraphInstantiate(&exec, graph, 0);
+                if (ie != cudaSuccess) { exec = nullptr; }
             }
             if (graph) { cudaGraphDestroy(graph); }
-            if (m->graph_eval1 != nullptr) { m->eval1_launches = n; break; }
+            if (exec != nullptr) { step = keep_graph(m, GRAPH_EVAL, exec, n); break; }
             cudaGetLastError();
             if (attempt == 0 && m->step_ok && m->step_coop) { m->step_coop = false; continue; }   // a cooperative launch the capture refuses: plain launch of the same grid
             if (st == SPYB_SUCCESS) { be->set_error("CUDA graph capture of the single-token step failed: %s", cudaGetErrorString(ce != cudaSuccess ? ce : ee != cudaSuccess ? ee : ie)); }
             return SPYB_FAIL;
         }
         SPYB_CUDA(be, cudaEventRecord(m->ev0, be->stream));
-        SPYB_CUDA(be, cudaGraphLaunch(m->graph_eval1, be->stream));
+        SPYB_CUDA(be, cudaGraphLaunch(step->exec, be->stream));
         SPYB_CUDA(be, cudaEventRecord(m->ev1, be->stream));
         SPYB_CUDA(be, cudaStreamSynchronize(be->stream));
         if (be->device_error()) { return SPYB_FAIL; }
         if (logits_host != nullptr) { std::memcpy(logits_host, m->h_logits_pinned, (size_t)m->info.n_vocab * 4); }
         SPYB_CUDA(be, cudaEventElapsedTime(&m->last_ms, m->ev0, m->ev1));
-        m->last_launches = m->eval1_launches;
+        m->last_launches = step->launches;
         return SPYB_SUCCESS;
     }
     // columns of a mat-vec pass
@@ -1135,6 +1169,7 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
         SPYB_CUDA(be, cudaMemcpyAsync(m->d_pos, m->h_pos_pinned, 12, cudaMemcpyHostToDevice, be->stream));
         SPYB_CUDA(be, cudaMemcpyAsync(m->d_tokens_in, m->h_tok_pinned, (size_t)T * 4, cudaMemcpyHostToDevice, be->stream));
         SPYB_CUDA(be, launch_embed(m->d_tokens_in, T, m->embd, m->embd_type, m->info.d_model, m->x, be->stream)); ++launches;
+        m->att_form = n_tokens == 1 ? step_form(m, n_past) : ATT_BY_CONTEXT;
         if (run_layers(m, T, t0 == 0, &launches) != SPYB_SUCCESS) { return SPYB_FAIL; }
         if (t0 + T == n_tokens) {
             if (run_head(m, T - 1, &launches) != SPYB_SUCCESS) { return SPYB_FAIL; }
@@ -1166,32 +1201,41 @@ spyb_status spyb_model_decode(spyb_model *m, int32_t first_token, int32_t n_past
     SPYB_CUDA(be, launch_embed(m->d_tokens_in, 1, m->embd, m->embd_type, m->info.d_model, m->x, be->stream));
 
     const bool use_graph = be->config.use_graph != 0 && (m->info.tp_size == 1 || std::getenv("SPYB_TP_NO_GRAPH") == nullptr);   // the all-reduces of the prompt pass have warmed NCCL up before the capture
-    int64_t per_step = 0;
-    for (int attempt = 0; use_graph && m->graph_exec == nullptr; ++attempt) {
-        // one decode step captured once; positions and the token live in device memory, so the
-        // same graph replays for every later step
-        cudaGraph_t graph = nullptr;
-        SPYB_CUDA(be, cudaStreamSynchronize(be->stream));
-        SPYB_CUDA(be, cudaStreamBeginCapture(be->stream, cudaStreamCaptureModeThreadLocal));
-        int64_t n = 0;
-        const spyb_status st = run_decode_step(m, &n);
-        const cudaError_t ce = cudaStreamEndCapture(be->stream, &graph);
-        cudaError_t ie = cudaSuccess;
-        if (st == SPYB_SUCCESS && ce == cudaSuccess) {
-            ie = cudaGraphInstantiate(&m->graph_exec, graph, 0);
-            if (ie != cudaSuccess) { m->graph_exec = nullptr; }
+    // one decode step captured once per sequence and form of the attention; positions and the token live in device memory, so the same
+    // graph replays for every later step
+    auto captured_step = [&]() -> spyb_model::StepGraph * {
+        if (auto *have = find_graph(m, GRAPH_DECODE)) { return have; }
+        for (int attempt = 0;; ++attempt) {
+            cudaGraph_t graph = nullptr;
+            cudaGraphExec_t exec = nullptr;
+            cudaError_t ce = cudaStreamSynchronize(be->stream), ie = cudaSuccess;
+            if (ce == cudaSuccess) { ce = cudaStreamBeginCapture(be->stream, cudaStreamCaptureModeThreadLocal); }
+            if (ce != cudaSuccess) { be->set_error("CUDA graph capture failed: %s", cudaGetErrorString(ce)); return nullptr; }
+            int64_t n = 0;
+            const spyb_status st = run_decode_step(m, &n);
+            ce = cudaStreamEndCapture(be->stream, &graph);
+            if (st == SPYB_SUCCESS && ce == cudaSuccess) {
+                ie = cudaGraphInstantiate(&exec, graph, 0);
+                if (ie != cudaSuccess) { exec = nullptr; }
+            }
+            if (graph) { cudaGraphDestroy(graph); }
+            if (exec != nullptr) { return keep_graph(m, GRAPH_DECODE, exec, n); }
+            cudaGetLastError();
+            if (attempt == 0 && m->step_ok && m->step_coop) { m->step_coop = false; continue; }   // a cooperative launch the capture refuses: plain launch of the same grid
+            if (st == SPYB_SUCCESS) { be->set_error("CUDA graph capture failed: %s", cudaGetErrorString(ce != cudaSuccess ? ce : ie)); }
+            return nullptr;
         }
-        if (graph) { cudaGraphDestroy(graph); }
-        if (m->graph_exec != nullptr) { break; }
-        cudaGetLastError();
-        if (attempt == 0 && m->step_ok && m->step_coop) { m->step_coop = false; continue; }   // a cooperative launch the capture refuses: plain launch of the same grid
-        if (st == SPYB_SUCCESS) { be->set_error("CUDA graph capture failed: %s", cudaGetErrorString(ce != cudaSuccess ? ce : ie)); }
-        return SPYB_FAIL;
-    }
-    per_step = m->step_ok ? 2 : (int64_t)m->layers.size() * 5 + 2;
+    };
+    // (steps that will be needed are captured before the first one runs: a capture waits for the stream)
+    m->att_form = step_form(m, n_past + n_steps - 1);
+    if (use_graph && captured_step() == nullptr) { return SPYB_FAIL; }
+    m->att_form = step_form(m, n_past);
+    if (use_graph && captured_step() == nullptr) { return SPYB_FAIL; }
+    int64_t per_step = m->step_ok ? 2 : (int64_t)m->layers.size() * 5 + 2;
     SPYB_CUDA(be, cudaEventRecord(m->ev0, be->stream));
     for (int s = 0; s < n_steps; ++s) {
-        if (use_graph) { SPYB_CUDA(be, cudaGraphLaunch(m->graph_exec, be->stream)); }
+        m->att_form = step_form(m, n_past + s);
+        if (use_graph) { SPYB_CUDA(be, cudaGraphLaunch(find_graph(m, GRAPH_DECODE)->exec, be->stream)); }
         else { int64_t n = 0; if (run_decode_step(m, &n) != SPYB_SUCCESS) { return SPYB_FAIL; } per_step = n; }
         if (logits_host != nullptr) {
             // parity mode: logits of every step come back (argmax_embed does not modify them)
@@ -1304,8 +1348,8 @@ spyb_status spyb_model_selftest_wait_timeout(spyb_model *m, uint64_t limit_ns, i
 
 // ---- batches of independent sequences that share the weights (every step reads them once for all sequences)
 static void drop_graphs(spyb_model *m) {
-    if (m->graph_exec) { cudaGraphExecDestroy(m->graph_exec); m->graph_exec = nullptr; }
-    if (m->graph_eval1) { cudaGraphExecDestroy(m->graph_eval1); m->graph_eval1 = nullptr; }
+    for (auto &g : m->graphs) { cudaGraphExecDestroy(g.exec); }
+    m->graphs.clear();
 }
 
 spyb_status spyb_model_set_sequences(spyb_model *m, int32_t n_seq) {
@@ -1334,7 +1378,6 @@ spyb_status spyb_model_select_sequence(spyb_model *m, int32_t seq) {
     if (seq == m->cur_seq) { return SPYB_SUCCESS; }
     cudaSetDevice(m->be->config.device_id);
     SPYB_CUDA(m->be, cudaStreamSynchronize(m->be->stream));
-    drop_graphs(m);   // the captured steps hold the cache addresses of the sequence they were captured for
     for (Layer &ly : m->layers) { ly.k_cache = ly.k_base + (int64_t)seq * m->seq_stride; ly.v_cache = ly.v_base + (int64_t)seq * m->seq_stride; }
     m->cur_seq = seq;
     return SPYB_SUCCESS;

@@ -1085,10 +1085,19 @@ size_t attention_scratch_floats(int n_ctx, int n_head, int T) {   // 0: the sing
     return (size_t)T * n_head * (((size_t)n_ctx + 3) & ~(size_t)3);
 }
 
+// The form for a single token at position pos, where both kernels take the context. A layer's attention, us, one CTA a head / a cluster of four:
+// position 8: 4.8 / 7.5; 100: 5.3 / 8.0; 250: 8.2 / 8.2; 460: 14.3 / 8.9; 900: 28 / 10.7.
+constexpr int ATT_CLUSTER_POS = 240, ATT_ONE_CTA_CTX = 8192;   // (the score row of the longest context: 40 KB)
+int attention_form(const AttnParams &p, const LaunchCfg &cfg, int pos) {
+    if (p.T != 1 || p.seq_stride != 0 || p.n_ctx > ATT_ONE_CTA_CTX || !atl_fits(p, cfg)) { return ATT_BY_CONTEXT; }
+    return pos < ATT_CLUSTER_POS ? ATT_ONE_CTA : ATT_CLUSTER;
+}
+
 cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
     if (p.hd != ATT_HD || p.T < 1 || p.n_ctx < 1 || (p.n_ctx & 3) || (p.dl & 7)) { return cudaErrorInvalidValue; }
     const size_t n_pad = ((size_t)p.n_ctx + 3) & ~(size_t)3;
-    if ((p.n_ctx > ATT_LONG_MIN || p.force_long) && p.scratch != nullptr) {
+    if (p.form == ATT_CLUSTER && atl_fits(p, cfg)) { return launch_attn_cluster(p, cfg); }
+    if (p.form != ATT_ONE_CTA && (p.n_ctx > ATT_LONG_MIN || p.force_long) && p.scratch != nullptr) {
         if (atl_fits(p, cfg)) { return launch_attn_cluster(p, cfg); }
         // a prompt: tokens share the K rows and the V^T rows, read in pieces of 16 (K, Q) and 8 bytes (V^T); Q and V^T of any other alignment go
         // through the kernels that read them value by value

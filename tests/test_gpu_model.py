@@ -482,6 +482,33 @@ def test_long_context_attention_path_in_the_model(env, oracle, tmp_models, monke
     m.close(); b.close()
 
 
+@pytest.mark.parametrize("n_ctx", [264, 512, 508, 1280])
+def test_steps_on_both_sides_of_the_attention_switch(n_ctx, oracle, tmp_models):
+    """From position 240 on a single-token step takes the cluster kernel, where the context's length allows it (508: not a multiple of 8), in
+    device-side decoding and in host-driven steps; two conversations take turns, each on captured steps of its own."""
+    cfg = gguf_io.LlamaConfig(n_layer=2, d_model=256, n_head=2, n_ff=512, n_vocab=512, weight_std=0.05)
+    path = str(tmp_models / "switch.gguf")
+    if not os.path.exists(path):
+        gguf_io.make_llama_gguf(path, cfg, seed=48)
+    prompts = [np.random.default_rng(s).integers(3, cfg.n_vocab, size=234) for s in (13, 14)]
+    want = [oracle.OracleLlama(path, n_ctx=n_ctx).generate(p, 13) for p in prompts]
+    b = B.B200Backend(0)
+    m = B.LlamaModel(b, path, n_ctx=n_ctx)
+    m.set_sequences(2)
+    for turn in range(2):
+        for c in (0, 1):
+            m.select_sequence(c)
+            logits = [m.eval(prompts[c], 0)]
+            if turn == 0:
+                ids, more = m.decode(int(np.argmax(logits[0])), 234, 12, want_logits=True)
+                logits = np.concatenate([logits, more])
+            else:
+                for i in range(12):
+                    logits.append(m.eval(np.array([np.argmax(logits[-1])]), 234 + i))
+            assert np.array_equal(np.argmax(logits, axis=1), want[c][0]) and logits_ok(np.array(logits), want[c][1])
+    m.close(); b.close()
+
+
 def test_rmsnorm_running_sum_on_hard_inputs(oracle, tmp_models):
     """The RMSNorm sum of squares is a serial f32 running sum on the CPU (groups of four squares added to one
     accumulator in order); the GPU forms the groups in parallel and runs the same chain on one thread. Inputs that
