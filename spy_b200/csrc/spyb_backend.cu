@@ -611,6 +611,7 @@ spyb_status run_matmul_kq_constant(spyb_backend *be, const spyb_tensor &w, const
                 SPYB_CUDA(be, cudaMalloc(&raw, (size_t)n_rows * kq_row_bytes(type, k) + 64));
                 be->owned.push_back(raw);
                 SPYB_CUDA(be, launch_kq_relayout_q6k(static_cast<const uint8_t *>(w.data), n_rows, k, static_cast<uint8_t *>(raw), be->stream));
+                SPYB_CUDA(be, cudaStreamSynchronize(be->stream));   // (the mat-vec copies its first weights ahead of its wait for the kernels in front)
                 be->kq_relaid[w.data] = static_cast<uint8_t *>(raw);
                 rows = static_cast<const uint8_t *>(raw);
             }
@@ -622,7 +623,7 @@ spyb_status run_matmul_kq_constant(spyb_backend *be, const spyb_tensor &w, const
         p.kq[0].w = rows; p.kq[0].type = type; p.kq[0].n_rows = n_rows; p.kq[0].row_bytes = kq_row_bytes(type, k); p.kq_n = 1;
         p.T = (int)std::min<int64_t>(KQ_MAX_COLUMNS, T - t); p.pro = PRO_QUANT; p.x = static_cast<const float *>(x.data) + t * k; p.x_stride = k;
         p.epi = EPI_STORE; p.out = static_cast<float *>(out_dev) + t * n_rows; p.out_stride = n_rows;
-        SPYB_CUDA(be, launch_matvec_kq(p, be->launch_cfg(false)));
+        SPYB_CUDA(be, launch_matvec_kq(p, be->launch_cfg(be->config.use_pdl != 0)));
     }
     return SPYB_SUCCESS;
 }
@@ -635,7 +636,7 @@ spyb_status run_matmul(spyb_backend *be, spyb_op_desc *d, void *out_dev) {
         if (st != SPYB_UNSUPPORTED) { return st; }
     }
     if (w.number_type == SPYB_FP16) {
-        SPYB_CUDA(be, launch_matmul_f16(to_strided(w, w.data), to_strided(x, x.data), to_strided(d->output, out_dev), be->stream));
+        SPYB_CUDA(be, launch_matmul_f16(to_strided(w, w.data), to_strided(x, x.data), to_strided(d->output, out_dev), be->stream, be->config.use_pdl != 0));
         return SPYB_SUCCESS;
     }
     if (w.number_type == SPYB_Q4_K || w.number_type == SPYB_Q6_K) {
@@ -700,7 +701,9 @@ spyb_status run_matmul(spyb_backend *be, spyb_op_desc *d, void *out_dev) {
         p.A = m; p.T = (int)std::min<int64_t>(tmax, T - t0);
         p.pro = PRO_QUANT; p.x = static_cast<const float *>(x.data) + t0 * m.k; p.x_stride = m.k;
         p.epi = EPI_STORE; p.out = static_cast<float *>(out_dev) + t0 * m.n_rows; p.out_stride = m.n_rows;
-        SPYB_CUDA(be, launch_matvec(p, be->launch_cfg(false)));
+        // A constant's tiles were finished before its upload returned: its kernel may start, and copy its first weights, beside the kernel in
+        // front (5120 x 5120 Q8_0, submits one after the other: 6.48 -> 6.30 us, 11008 x 4096 Q4_K of four columns 15.4 -> 14.5).
+        SPYB_CUDA(be, launch_matvec(p, be->launch_cfg(found && be->config.use_pdl != 0)));
     }
     return SPYB_SUCCESS;
 }
@@ -747,7 +750,7 @@ bool rope_from_table(spyb_backend *be, const spyb_rope_param &rp, const int32_t 
         if (cudaMemcpyAsync(t.dev + (int64_t)pos[i] * npair, row.data(), row.size() * sizeof(float2), cudaMemcpyHostToDevice, be->stream) != cudaSuccess) { return false; }
         t.have[pos[i]] = 1;
     }
-    *err = launch_rope_rows(x, t.dev, rr, out, be->stream);
+    *err = launch_rope_rows(x, t.dev, rr, out, be->stream, be->config.use_pdl != 0);
     return true;
 }
 
@@ -814,26 +817,26 @@ spyb_status spyb_submit(spyb_backend *be, spyb_op_desc *d, void (*callback)(void
             }
             const int64_t rows = tensor_elems(a) / a.elements[0], brows = tensor_elems(b) / b.elements[0];
             err = launch_binary_rows(d->op_type == SPYB_OP_ADD ? 0 : 1, static_cast<const float *>(a.data), static_cast<const float *>(b.data),
-                                     static_cast<float *>(out.dev), a.elements[0], rows, brows, be->stream);
+                                     static_cast<float *>(out.dev), a.elements[0], rows, brows, be->stream, be->config.use_pdl != 0);
         } break;
         case SPYB_OP_NORM_RMS:
             if (!tensor_contiguous(a) || a.number_type != SPYB_FP32) { be->set_error("NormRMS: contiguous f32 expected"); st = SPYB_UNSUPPORTED; break; }
-            err = launch_rmsnorm(static_cast<const float *>(a.data), static_cast<float *>(out.dev), a.elements[0], tensor_elems(a) / a.elements[0], d->norm_eps, be->stream);
+            err = launch_rmsnorm(static_cast<const float *>(a.data), static_cast<float *>(out.dev), a.elements[0], tensor_elems(a) / a.elements[0], d->norm_eps, be->stream, be->config.use_pdl != 0);
             break;
         case SPYB_OP_SILU:
             if (!tensor_contiguous(a) || a.number_type != SPYB_FP32) { be->set_error("Silu: contiguous f32 expected"); st = SPYB_UNSUPPORTED; break; }
-            err = launch_silu(static_cast<const float *>(a.data), static_cast<float *>(out.dev), tensor_elems(a), be->d_silu_table, be->stream);
+            err = launch_silu(static_cast<const float *>(a.data), static_cast<float *>(out.dev), tensor_elems(a), be->d_silu_table, be->stream, be->config.use_pdl != 0);
             break;
         case SPYB_OP_SOFTMAX: {
             if (d->num_input != 2 || !tensor_contiguous(a)) { be->set_error("Softmax: contiguous scores and a mask expected"); st = SPYB_UNSUPPORTED; break; }
             const spyb_tensor &mk = local.input[1];
             if (mask_packed) {
                 err = launch_softmax_bits(static_cast<const float *>(a.data), mask, static_cast<float *>(out.dev), a.elements[0], a.elements[1], a.elements[2] * a.elements[3],
-                                          d->softmax_scale, be->d_exp_table, be->stream);
+                                          d->softmax_scale, be->d_exp_table, be->stream, be->config.use_pdl != 0);
                 break;
             }
             err = launch_softmax_masked(static_cast<const float *>(a.data), static_cast<const float *>(mk.data), static_cast<float *>(out.dev),
-                                        a.elements[0], a.elements[1], a.elements[2] * a.elements[3], mk.bytes[1] / 4, d->softmax_scale, be->d_exp_table, be->stream);
+                                        a.elements[0], a.elements[1], a.elements[2] * a.elements[3], mk.bytes[1] / 4, d->softmax_scale, be->d_exp_table, be->stream, be->config.use_pdl != 0);
         } break;
         case SPYB_OP_ROPE:
             if (d->rope.mode != 0 || d->rope.extend_factor != 0.f || d->rope.freq_scale != 1.f || d->rope.attention_factor != 1.f) {
@@ -860,17 +863,17 @@ spyb_status spyb_submit(spyb_backend *be, spyb_op_desc *d, void (*callback)(void
                 void *dtab = be->arena.alloc(tab.size() * sizeof(float2));
                 if (dtab == nullptr) { be->set_error("Rope: out of device memory"); st = SPYB_FAIL; break; }
                 err = cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(float2), cudaMemcpyHostToDevice, be->stream);
-                if (err == cudaSuccess) { err = launch_rope(to_strided(a, a.data), static_cast<const float2 *>(dtab), to_strided(local.output, out.dev), be->stream); }
+                if (err == cudaSuccess) { err = launch_rope(to_strided(a, a.data), static_cast<const float2 *>(dtab), to_strided(local.output, out.dev), be->stream, be->config.use_pdl != 0); }
                 be->arena.free(dtab, tab.size() * sizeof(float2));
             }
             break;
         case SPYB_OP_COPY: {   // destination = input[1]; the output aliases it (view.cpp:216-227)
             const spyb_tensor &dst = local.input[1];
-            err = launch_copy_strided(to_strided(a, a.data), a.number_type, to_strided(dst, dst.data), dst.number_type, be->stream);
+            err = launch_copy_strided(to_strided(a, a.data), a.number_type, to_strided(dst, dst.data), dst.number_type, be->stream, be->config.use_pdl != 0);
             d->output.data = d->input[1].data;
         } break;
         case SPYB_OP_DUP: case SPYB_OP_CONTIGUOUS:
-            err = launch_copy_strided(to_strided(a, a.data), a.number_type, to_strided(local.output, out.dev), local.output.number_type, be->stream);
+            err = launch_copy_strided(to_strided(a, a.data), a.number_type, to_strided(local.output, out.dev), local.output.number_type, be->stream, be->config.use_pdl != 0);
             break;
         case SPYB_OP_GETROW: {
             const spyb_tensor &ids = local.input[1];

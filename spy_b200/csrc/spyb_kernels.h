@@ -237,24 +237,24 @@ struct Strided {   // a tensor as the reference's Shape describes it: elements +
     int64_t ne[4];
     int64_t nb[4];
 };
-cudaError_t launch_rmsnorm(const float *x, float *out, int64_t n, int64_t rows, float eps, cudaStream_t s);
-cudaError_t launch_binary_rows(int op /*0 add, 1 mul*/, const float *a, const float *b, float *out, int64_t n, int64_t rows, int64_t b_rows, cudaStream_t s);
-cudaError_t launch_silu(const float *x, float *out, int64_t n, const float *silu_table, cudaStream_t s);
+cudaError_t launch_rmsnorm(const float *x, float *out, int64_t n, int64_t rows, float eps, cudaStream_t s, bool pdl = false);
+cudaError_t launch_binary_rows(int op /*0 add, 1 mul*/, const float *a, const float *b, float *out, int64_t n, int64_t rows, int64_t b_rows, cudaStream_t s, bool pdl = false);
+cudaError_t launch_silu(const float *x, float *out, int64_t n, const float *silu_table, cudaStream_t s, bool pdl = false);
 cudaError_t launch_softmax_masked(const float *scores, const float *mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2,
-                                  int64_t mask_stride, float scale, const float *exp_table, cudaStream_t s);
+                                  int64_t mask_stride, float scale, const float *exp_table, cudaStream_t s, bool pdl = false);
 // the same with a mask of zeros (bit set) and -inf packed into the kernel's parameters: bit i1 * ne0 + i0
 constexpr int MASK_BITS = 8192;
 struct MaskBits { uint32_t w[MASK_BITS / 32]; };
-cudaError_t launch_softmax_bits(const float *scores, const MaskBits &mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2, float scale, const float *exp_table, cudaStream_t s);
+cudaError_t launch_softmax_bits(const float *scores, const MaskBits &mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2, float scale, const float *exp_table, cudaStream_t s, bool pdl = false);
 // cos_sin: device table [ne2 tokens][ne0/2] of (cos, sin) built on the host with the host libm
 // pos: row of the table for every token (by value: up to ROPE_ROWS tokens)
 constexpr int ROPE_ROWS = 64;
 struct RopeRows { int32_t row[ROPE_ROWS]; };
-cudaError_t launch_rope(const Strided &x, const float2 *cos_sin, const Strided &out, cudaStream_t s);
-cudaError_t launch_rope_rows(const Strided &x, const float2 *cos_sin, const RopeRows &rows, const Strided &out, cudaStream_t s);
-cudaError_t launch_copy_strided(const Strided &src, int src_type, const Strided &dst, int dst_type, cudaStream_t s);
+cudaError_t launch_rope(const Strided &x, const float2 *cos_sin, const Strided &out, cudaStream_t s, bool pdl = false);
+cudaError_t launch_rope_rows(const Strided &x, const float2 *cos_sin, const RopeRows &rows, const Strided &out, cudaStream_t s, bool pdl = false);
+cudaError_t launch_copy_strided(const Strided &src, int src_type, const Strided &dst, int dst_type, cudaStream_t s, bool pdl = false);
 cudaError_t launch_getrow(const uint8_t *table, int table_type, int64_t row_bytes, int64_t ne0, const int32_t *ids, int64_t n_ids, float *out, cudaStream_t s);
-cudaError_t launch_matmul_f16(const Strided &w /*f16*/, const Strided &x /*f32*/, const Strided &out /*f32*/, cudaStream_t s);
+cudaError_t launch_matmul_f16(const Strided &w /*f16*/, const Strided &x /*f32*/, const Strided &out /*f32*/, cudaStream_t s, bool pdl = false);
 // K-quant weights (raw GGUF rows: Q4_K = 12, Q6_K = 14) times f32 activations [n_cols][k] -> out [n_cols][n_rows]
 cudaError_t launch_matmul_kquant(int type, const uint8_t *w, int64_t n_rows, int64_t k, const float *x, int64_t n_cols, float *out, cudaStream_t s);
 cudaError_t launch_argmax_embed_batch(const float *logits, int64_t n_vocab, int n_seq, int32_t *tokens, int32_t *ids_out, const uint8_t *embd, int embd_type,

@@ -1331,6 +1331,8 @@ __global__ void rmsnorm_kernel(const float *x, float *out, int64_t n, float eps)
     const float *xr = x + (int64_t)blockIdx.x * n;
     float       *o  = out + (int64_t)blockIdx.x * n;
     const int n4 = (int)(n >> 2);
+    pdl_launch_dependents();
+    pdl_wait();
     for (int g = threadIdx.x; g < n4; g += blockDim.x) {
         const float4 v = reinterpret_cast<const float4 *>(xr)[g];
         v3[g] = __fadd_rn(fmaf(v.y, v.y, __fmul_rn(v.x, v.x)), fmaf(v.w, v.w, __fmul_rn(v.z, v.z)));
@@ -1348,7 +1350,7 @@ __global__ void rmsnorm_kernel(const float *x, float *out, int64_t n, float eps)
     const float scale = scale_s;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) { o[i] = __fmul_rn(xr[i], scale); }
 }
-cudaError_t launch_rmsnorm(const float *x, float *out, int64_t n, int64_t rows, float eps, cudaStream_t s) {
+cudaError_t launch_rmsnorm(const float *x, float *out, int64_t n, int64_t rows, float eps, cudaStream_t s, bool pdl) {
     if (rows == 0 || n == 0) { return cudaSuccess; }
     if ((n & 3) != 0 || n > 180 * 1024) { return cudaErrorNotSupported; }   // rows are read as float4 groups
     const size_t smem = (size_t)n;   // n/4 floats
@@ -1358,34 +1360,34 @@ cudaError_t launch_rmsnorm(const float *x, float *out, int64_t n, int64_t rows, 
         if (err != cudaSuccess) { return err; }
         smem_allowed = smem;
     }
-    rmsnorm_kernel<<<(unsigned)rows, 256, smem, s>>>(x, out, n, eps);
-    return launch_check();
+    return launch_maybe_pdl(rmsnorm_kernel, dim3((unsigned)rows), 256, smem, s, pdl, x, out, n, eps);
 }
 
 // binary_execution<plus / multiplies>, basic.cpp:15-50: row r of `a` with row (r % b_rows) of `b`
 __global__ void binary_rows_kernel(int op, const float *a, const float *b, float *out, int64_t n, int64_t rows, int64_t b_rows) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, r = i / n, c = i - r * n;
+    pdl_launch_dependents();
+    pdl_wait();
     if (i >= n * rows) { return; }
-    const int64_t r = i / n, c = i - r * n;
     const float   y = b[(r % b_rows) * n + c];
     out[i] = op == 0 ? __fadd_rn(a[i], y) : __fmul_rn(a[i], y);
 }
-cudaError_t launch_binary_rows(int op, const float *a, const float *b, float *out, int64_t n, int64_t rows, int64_t b_rows, cudaStream_t s) {
+cudaError_t launch_binary_rows(int op, const float *a, const float *b, float *out, int64_t n, int64_t rows, int64_t b_rows, cudaStream_t s, bool pdl) {
     const int64_t tot = n * rows;
     if (tot == 0) { return cudaSuccess; }
-    binary_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(op, a, b, out, n, rows, b_rows);
-    return launch_check();
+    return launch_maybe_pdl(binary_rows_kernel, dim3((unsigned)((tot + 255) / 256)), 256, 0, s, pdl, op, a, b, out, n, rows, b_rows);
 }
 
 // OperatorSiluImpl::execute, non-linear.cpp:57-77
 __global__ void silu_kernel(const float *x, float *out, int64_t n, const float *table) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     if (i < n) { out[i] = table[f2h(x[i])]; }
 }
-cudaError_t launch_silu(const float *x, float *out, int64_t n, const float *silu_table, cudaStream_t s) {
+cudaError_t launch_silu(const float *x, float *out, int64_t n, const float *silu_table, cudaStream_t s, bool pdl) {
     if (n == 0) { return cudaSuccess; }
-    silu_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, out, n, silu_table);
-    return launch_check();
+    return launch_maybe_pdl(silu_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, s, pdl, x, out, n, silu_table);
 }
 
 // operator_masked_softmax_execute, non-linear.cpp:129-180; one CTA per row (i1, i2), row length ne0,
@@ -1396,6 +1398,8 @@ __device__ __forceinline__ void softmax_masked_row(const float *src, float *dst,
     __shared__ float red[8];
     __shared__ float bcast;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
     float m = -CUDART_INF_F;
     for (int64_t i = threadIdx.x; i < ne0; i += blockDim.x) {
         const float v = __fmul_rn(__fadd_rn(src[i], mask_at(i)), scale);
@@ -1430,13 +1434,12 @@ __global__ void softmax_bits_kernel(const float *scores, const __grid_constant__
         return (mask.w[b >> 5] >> (b & 31)) & 1u ? 0.f : -CUDART_INF_F;
     });
 }
-cudaError_t launch_softmax_bits(const float *scores, const MaskBits &mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2, float scale, const float *exp_table, cudaStream_t s) {
+cudaError_t launch_softmax_bits(const float *scores, const MaskBits &mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2, float scale, const float *exp_table, cudaStream_t s, bool pdl) {
     if (ne0 < 1 || ne1 < 1 || ne2 < 1 || ne0 * ne1 > MASK_BITS) { return cudaErrorInvalidValue; }
-    softmax_bits_kernel<<<(unsigned)(ne1 * ne2), 256, (size_t)ne0 * sizeof(float), s>>>(scores, mask, out, ne0, ne1, scale, exp_table);   // (at most 32 KB of shared memory)
-    return launch_check();
+    return launch_maybe_pdl(softmax_bits_kernel, dim3((unsigned)(ne1 * ne2)), 256, (size_t)ne0 * sizeof(float), s, pdl, scores, mask, out, ne0, ne1, scale, exp_table);   // (at most 32 KB of shared memory)
 }
 cudaError_t launch_softmax_masked(const float *scores, const float *mask, float *out, int64_t ne0, int64_t ne1, int64_t ne2,
-                                  int64_t mask_stride, float scale, const float *exp_table, cudaStream_t s) {
+                                  int64_t mask_stride, float scale, const float *exp_table, cudaStream_t s, bool pdl) {
     if (ne0 == 0 || ne1 * ne2 == 0) { return cudaSuccess; }
     const size_t smem = (size_t)ne0 * sizeof(float);
     if (smem > 200 * 1024) { return cudaErrorNotSupported; }
@@ -1446,8 +1449,7 @@ cudaError_t launch_softmax_masked(const float *scores, const float *mask, float 
         if (err != cudaSuccess) { return err; }
         smem_allowed = smem;
     }
-    softmax_masked_kernel<<<(unsigned)(ne1 * ne2), 256, smem, s>>>(scores, mask, out, ne0, ne1, mask_stride, scale, exp_table);
-    return launch_check();
+    return launch_maybe_pdl(softmax_masked_kernel, dim3((unsigned)(ne1 * ne2)), 256, smem, s, pdl, scores, mask, out, ne0, ne1, mask_stride, scale, exp_table);
 }
 
 __device__ __forceinline__ int64_t soff(const Strided &t, int64_t i0, int64_t i1, int64_t i2, int64_t i3) {
@@ -1467,6 +1469,8 @@ __device__ __forceinline__ void rope_pair(const Strided &x, const Strided &out, 
 __global__ void rope_kernel(const Strided x, const float2 *cos_sin, const Strided out) {
     const int64_t npair = x.ne[0] >> 1;
     const int64_t i     = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     if (i >= npair * x.ne[1] * x.ne[2]) { return; }
     const int64_t k = i % npair, i1 = (i / npair) % x.ne[1], i2 = i / (npair * x.ne[1]);
     rope_pair(x, out, cos_sin[i2 * npair + k], k, i1, i2);
@@ -1474,22 +1478,22 @@ __global__ void rope_kernel(const Strided x, const float2 *cos_sin, const Stride
 __global__ void rope_rows_kernel(const Strided x, const float2 *cos_sin, const __grid_constant__ RopeRows rows, const Strided out) {
     const int64_t npair = x.ne[0] >> 1;
     const int64_t i     = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     if (i >= npair * x.ne[1] * x.ne[2]) { return; }
     const int64_t k = i % npair, i1 = (i / npair) % x.ne[1], i2 = i / (npair * x.ne[1]);
     rope_pair(x, out, cos_sin[(int64_t)rows.row[i2] * npair + k], k, i1, i2);
 }
-cudaError_t launch_rope(const Strided &x, const float2 *cos_sin, const Strided &out, cudaStream_t s) {
+cudaError_t launch_rope(const Strided &x, const float2 *cos_sin, const Strided &out, cudaStream_t s, bool pdl) {
     const int64_t tot = (x.ne[0] >> 1) * x.ne[1] * x.ne[2];
     if (tot == 0) { return cudaSuccess; }
-    rope_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, s>>>(x, cos_sin, out);
-    return launch_check();
+    return launch_maybe_pdl(rope_kernel, dim3((unsigned)((tot + 127) / 128)), 128, 0, s, pdl, x, cos_sin, out);
 }
-cudaError_t launch_rope_rows(const Strided &x, const float2 *cos_sin, const RopeRows &rows, const Strided &out, cudaStream_t s) {
+cudaError_t launch_rope_rows(const Strided &x, const float2 *cos_sin, const RopeRows &rows, const Strided &out, cudaStream_t s, bool pdl) {
     const int64_t tot = (x.ne[0] >> 1) * x.ne[1] * x.ne[2];
     if (tot == 0) { return cudaSuccess; }
     if (x.ne[2] > ROPE_ROWS) { return cudaErrorInvalidValue; }
-    rope_rows_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, s>>>(x, cos_sin, rows, out);
-    return launch_check();
+    return launch_maybe_pdl(rope_rows_kernel, dim3((unsigned)((tot + 127) / 128)), 128, 0, s, pdl, x, cos_sin, rows, out);
 }
 
 // dup_execute (Copy / Contiguous), view.cpp:83-227, 285-321: element (i0..i3) of src in source order goes to
@@ -1497,6 +1501,8 @@ cudaError_t launch_rope_rows(const Strided &x, const float2 *cos_sin, const Rope
 __global__ void copy_strided_kernel(const Strided src, int src_type, const Strided dst, int dst_type) {
     const int64_t tot = src.ne[0] * src.ne[1] * src.ne[2] * src.ne[3];
     const int64_t i   = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
     if (i >= tot) { return; }
     const int64_t s0 = i % src.ne[0], s1 = (i / src.ne[0]) % src.ne[1], s2 = (i / (src.ne[0] * src.ne[1])) % src.ne[2],
                   s3 = i / (src.ne[0] * src.ne[1] * src.ne[2]);
@@ -1507,12 +1513,11 @@ __global__ void copy_strided_kernel(const Strided src, int src_type, const Strid
     const float v = (src_type == 0) ? *reinterpret_cast<const float *>(sp) : h2f(*reinterpret_cast<const uint16_t *>(sp));
     if (dst_type == 0) { *reinterpret_cast<float *>(dp) = v; } else { *reinterpret_cast<uint16_t *>(dp) = f2h(v); }
 }
-cudaError_t launch_copy_strided(const Strided &src, int src_type, const Strided &dst, int dst_type, cudaStream_t s) {
+cudaError_t launch_copy_strided(const Strided &src, int src_type, const Strided &dst, int dst_type, cudaStream_t s, bool pdl) {
     if ((src_type != 0 && src_type != 1) || (dst_type != 0 && dst_type != 1)) { return cudaErrorNotSupported; }
     const int64_t tot = src.ne[0] * src.ne[1] * src.ne[2] * src.ne[3];
     if (tot == 0) { return cudaSuccess; }
-    copy_strided_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(src, src_type, dst, dst_type);
-    return launch_check();
+    return launch_maybe_pdl(copy_strided_kernel, dim3((unsigned)((tot + 255) / 256)), 256, 0, s, pdl, src, src_type, dst, dst_type);
 }
 
 // bytes of one table row of ne0 elements
@@ -1578,34 +1583,31 @@ __global__ void matmul_f16_kernel(const Strided w, const Strided x, const Stride
     const int64_t n_out = out.ne[0] * out.ne[1] * out.ne[2];
     const int64_t o     = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int     lane  = threadIdx.x & 31;
-    if (o >= n_out) { return; }
     const int64_t i01 = o % out.ne[0], i11 = (o / out.ne[0]) % out.ne[1], i02 = o / (out.ne[0] * out.ne[1]);
     const uint8_t *wp = reinterpret_cast<const uint8_t *>(w.data) + soff(w, 0, i01, i02, 0);
     const uint8_t *xp = reinterpret_cast<const uint8_t *>(x.data) + soff(x, 0, i11, i02, 0);
     const int64_t n = w.ne[0];
     const int64_t n_main = n > 0 ? ((n - 1) / 32) * 32 : 0;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (o >= n_out) { return; }
+    auto w_at = [&](int64_t k) { return h2f(*reinterpret_cast<const uint16_t *>(wp + k * w.nb[0])); };
+    auto x_at = [&](int64_t k) { return h2f(f2h(*reinterpret_cast<const float *>(xp + k * x.nb[0]))); };
+    // the scalar tail's (at most 32) elements, one to a lane, in flight with the rest: 32 x 200 scores of heads of 128 7.9 -> 6.8 us
+    const float wt = n_main + lane < n ? w_at(n_main + lane) : 0.f, xt = n_main + lane < n ? x_at(n_main + lane) : 0.f;
     float acc = 0.f;
-    for (int64_t k = 0; k < n_main; k += 32) {
-        const float a = h2f(*reinterpret_cast<const uint16_t *>(wp + (k + lane) * w.nb[0]));
-        const float b = h2f(f2h(*reinterpret_cast<const float *>(xp + (k + lane) * x.nb[0])));
-        acc = fmaf(a, b, acc);
-    }
+#pragma unroll 4
+    for (int64_t k = 0; k < n_main; k += 32) { acc = fmaf(w_at(k + lane), x_at(k + lane), acc); }
     acc = reduce_f16dot_lanes(acc);
-    if (lane == 0) {
-        float tail = 0.f;
-        for (int64_t k = n_main; k < n; ++k) {
-            const float a = h2f(*reinterpret_cast<const uint16_t *>(wp + k * w.nb[0]));
-            const float b = h2f(f2h(*reinterpret_cast<const float *>(xp + k * x.nb[0])));
-            tail = fmaf(a, b, tail);
-        }
-        *reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(out.data) + soff(out, i01, i11, i02, 0)) = __fadd_rn(tail, acc);
-    }
+    float tail = 0.f;
+    const int n_tail = (int)(n - n_main);
+    for (int k = 0; k < n_tail; ++k) { tail = fmaf(__shfl_sync(0xffffffffu, wt, k), __shfl_sync(0xffffffffu, xt, k), tail); }
+    if (lane == 0) { *reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(out.data) + soff(out, i01, i11, i02, 0)) = __fadd_rn(tail, acc); }
 }
-cudaError_t launch_matmul_f16(const Strided &w, const Strided &x, const Strided &out, cudaStream_t s) {
+cudaError_t launch_matmul_f16(const Strided &w, const Strided &x, const Strided &out, cudaStream_t s, bool pdl) {
     const int64_t n_out = out.ne[0] * out.ne[1] * out.ne[2];
     if (n_out == 0) { return cudaSuccess; }
-    matmul_f16_kernel<<<(unsigned)((n_out * 32 + 255) / 256), 256, 0, s>>>(w, x, out);
-    return launch_check();
+    return launch_maybe_pdl(matmul_f16_kernel, dim3((unsigned)((n_out * 32 + 255) / 256)), 256, 0, s, pdl, w, x, out);
 }
 
 // Greedy sampling on the device (first maximum wins, model/include/llm/sampler/greedy.h:20-25), followed by
