@@ -139,7 +139,11 @@ struct NcclApi {
 static NcclApi g_nccl;
 
 constexpr int TMAX_COLUMNS = 8;        // activation columns the mat-vec passes hold
-constexpr int PF_ATT_GROUP = 128;      // tokens per attention launch of the prompt path (their score rows stay in L2: 67 MB for 32 heads x 4096 positions)
+// Tokens per attention launch of the prompt path: a chunk's 512 where their score rows take little memory (and stay in L2), else 256 (134 MB for
+// 32 heads x 4096 positions) or 128. Launches of few CTAs end in waves that are nearly empty: 3968 tokens of 32 heads 5.4 ms a layer in groups
+// of 128, 4.8 in groups of 256.
+constexpr int PF_ATT_GROUP = 128, PF_ATT_GROUP_MAX = 512;
+constexpr size_t PF_ATT_BYTES = 144u << 20;
 
 struct PfMat { uint8_t *w = nullptr; int type = 0; int64_t n_rows = 0; int nb = 0; };
 
@@ -484,7 +488,10 @@ spyb_status ensure_prefill_buffers(spyb_model *m) {
     const char *tiled_env = std::getenv("SPYB_PF_ATT_TILED");
     if (m->att_scratch == nullptr && (tiled_env == nullptr || std::atoi(tiled_env) != 0)) {
         const size_t n_pad = ((size_t)m->info.n_ctx + 3) & ~(size_t)3;
-        if (!have(&m->pf_att_scratch, (size_t)m->att_group * (dl / m->info.head_dim) * n_pad)) { return SPYB_FAIL; }
+        while (!have(&m->pf_att_scratch, (size_t)m->att_group * (dl / m->info.head_dim) * n_pad)) {
+            if (m->att_group <= PF_ATT_GROUP) { return SPYB_FAIL; }
+            m->att_group /= 2;   // (little memory left)
+        }
     }
     auto pinned = [&](auto **p, size_t bytes) { return *p != nullptr || cudaMallocHost(reinterpret_cast<void **>(p), bytes) == cudaSuccess; };
     if (!pinned(&m->h_pf_tokens, C * 4) || !pinned(&m->h_pf_pos, 2 * (C / TMAX + 1) * 4)) { cudaGetLastError(); be->set_error("pinned host allocation failed"); return SPYB_FAIL; }
@@ -907,10 +914,18 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
         m->tp_peer[I.tp_rank] = m->tp_local;
         m->att = tp_att(m, m->tp_local); m->act = tp_act(m, m->tp_local);
     }
-    m->att_group = m->pf_ok ? PF_ATT_GROUP : TMAX;
-    const size_t att_scratch = attention_scratch_floats(I.n_ctx, dl / I.head_dim, m->att_group);
+    m->att_group = TMAX;
+    if (m->pf_ok) {
+        const size_t row_bytes = 4 * (size_t)(dl / I.head_dim) * (((size_t)I.n_ctx + 3) & ~(size_t)3);
+        for (m->att_group = PF_ATT_GROUP_MAX; m->att_group > PF_ATT_GROUP && m->att_group * row_bytes > PF_ATT_BYTES;) { m->att_group /= 2; }
+    }
+    size_t att_scratch = attention_scratch_floats(I.n_ctx, dl / I.head_dim, m->att_group);
+    while (att_scratch != 0 && m->att_group > PF_ATT_GROUP && dev_alloc(m, &m->att_scratch, att_scratch) != SPYB_SUCCESS) {   // (little memory left: smaller groups)
+        m->att_group /= 2;
+        att_scratch = attention_scratch_floats(I.n_ctx, dl / I.head_dim, m->att_group);
+    }
     bool ok = dev_alloc(m, &m->x, (size_t)TMAX * d) == SPYB_SUCCESS && dev_alloc(m, &m->scratch, (size_t)TMAX * d) == SPYB_SUCCESS &&
-              (att_scratch == 0 || dev_alloc(m, &m->att_scratch, att_scratch) == SPYB_SUCCESS) &&
+              (att_scratch == 0 || m->att_scratch != nullptr || dev_alloc(m, &m->att_scratch, att_scratch) == SPYB_SUCCESS) &&
               dev_alloc(m, &m->logits, (size_t)I.n_vocab) == SPYB_SUCCESS && dev_alloc(m, &m->q, (size_t)TMAX * dl) == SPYB_SUCCESS &&
               dev_alloc(m, &m->d_pos, 4) == SPYB_SUCCESS && dev_alloc(m, &m->d_token, 4) == SPYB_SUCCESS &&
               dev_alloc(m, &m->d_tokens_in, TMAX) == SPYB_SUCCESS && dev_alloc(m, &m->d_history, (size_t)I.n_ctx + 8) == SPYB_SUCCESS &&

@@ -400,26 +400,35 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(const AttnParams p) {
     p.scratch[((int64_t)t * p.n_head + h) * n_pad + j] = score_dot(kv, reinterpret_cast<const float4 *>(qf));
 }
 
-// The same for a prompt, register-tiled: a CTA takes ATT_SG times ATT_ST tokens x ATT_SP positions of a head, a lane 4 tokens x 4
+// a * b + c of the f16 values in the low halves of a and b: the fmaf of the widened values (their product is exact in f32) without widening
+// them; it issues as fast as fmaf, and half the bytes of its operands come out of shared memory
+__device__ __forceinline__ float fma_f16(uint32_t a, uint32_t b, float c) {
+    float d;
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"((uint16_t)a), "h"((uint16_t)b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t half_of(const uint32_t *w, int i) { return w[i >> 1] >> (16 * (i & 1)); }
+
+// The same for a prompt, register-tiled: a CTA takes ATT_SG times ATT_ST tokens x ATT_SP positions of a head, a lane 4 tokens x 8
 // positions at a time. The 32 accumulators of a dot product are walked element by element of the CPU's eight-wide vectors: element e of
 // the four accumulators takes the twelve values 32 s + 8 a + e (s = 0..2, a = 0..3), four chains of three FMAs, so that only one to
-// three partial sums per output live at a time instead of 32 accumulators. K and Q lie in shared memory as f32 in that order, value by
+// three partial sums per output live at a time instead of 32 accumulators. K and Q lie in shared memory as f16 in that order, value by
 // value: [value][position] and [value][token].
 // 160 f32 operations per (token, position, head). Shared memory gives a warp one word per lane and cycle however often an address
-// repeats, so a word has to serve several products: 16 products per 8 words here (one K row per thread with Q by uniform 128-bit reads:
-// 4 products per 4 words, and every row widened again for every token). 128 tokens of 32 heads over 2000 positions on average:
-// 180 -> 83 us.
+// repeats, so a word has to serve several products: 32 products per 6 words here. Bound: the FMA pipes, busy 61 % (eight warps an SM, 237
+// registers). 128 tokens of 32 heads over 2000 positions on average: 67 us (f32 copies of K and Q, 4 x 4 outputs a lane, 16 products per 8
+// words: 83; the 5000 FMAs of a tile unrolled, beyond the instruction caches: 87; one K row per thread: 180).
 constexpr int ATT_TT = 8;                                    // tokens per CTA of the PV kernel below
-constexpr int ATT_ST = 16, ATT_SP = 128, ATT_KPITCH = ATT_SP + 4, ATT_SC_THREADS = 128;
+constexpr int ATT_ST = 32, ATT_SP = 128, ATT_KPITCH = ATT_SP + 8, ATT_SC_THREADS = 128;
 constexpr int ATT_SG = 2;                                    // token tiles a CTA walks with the same K rows
-constexpr size_t ATT_SC_SMEM = (size_t)ATT_HD * (ATT_KPITCH + ATT_SG * ATT_ST) * sizeof(float);
+constexpr size_t ATT_SC_SMEM = (size_t)ATT_HD * (ATT_KPITCH + ATT_SG * ATT_ST) * sizeof(__half);
 // value 8 c + e of a row -> its place: 12 e + c for the first 96, then 96 + 4 ((e + 1) % 8) + c - 12 (the rotation keeps the pieces c = 8..15
 // of a row on different banks when they are stored side by side)
 __host__ __device__ constexpr int att_value_row(int c, int e) { return c < 12 ? 12 * e + c : 96 + 4 * ((e + 1) & 7) + c - 12; }
-__global__ void __launch_bounds__(ATT_SC_THREADS) attn_scores_tiled_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(ATT_SC_THREADS, 2) attn_scores_tiled_kernel(const AttnParams p) {
     extern __shared__ __align__(16) float att_smem[];
     constexpr int NQ = ATT_SG * ATT_ST;
-    float *ks = att_smem, *qs = att_smem + ATT_HD * ATT_KPITCH;
+    __half *ks = reinterpret_cast<__half *>(att_smem), *qs = ks + ATT_HD * ATT_KPITCH;
     const int h = blockIdx.y, tg = blockIdx.z * NQ, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_launch_dependents();
     pdl_wait();
@@ -427,110 +436,136 @@ __global__ void __launch_bounds__(ATT_SC_THREADS) attn_scores_tiled_kernel(const
     const int n_vis_last = p.pos_base[0] + tg + ng;          // positions the last token of the CTA sees
     if (j0 >= n_vis_last) { return; }
     const int n_pad = (p.n_ctx + 3) & ~3;
-    {   // a warp reads four rows x 128 bytes at a time and writes them value by value (the pitch keeps the 8 x 4 words of a store on 32 banks)
-        const int row0 = tid >> 3, c0 = tid & 7;             // 16-byte pieces c0 and c0 + 8 of rows row0, row0 + 16, ...
+    {   // a warp reads four pairs of neighbouring rows x 128 bytes at a time and writes the pairs value by value (the pitch keeps the 8 x 4 words of a store on 32 banks)
+        const int row0 = 2 * (tid >> 3), c0 = tid & 7;       // 16-byte pieces c0 and c0 + 8 of rows row0 + 32 i, row0 + 32 i + 1
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int c = c0 + 8 * half;
             const __half *src = p.k_cache + (int64_t)(j0 + row0) * p.dl + (int64_t)h * ATT_HD + 8 * c;
             uint4 w[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { w[i] = j0 + row0 + 16 * i < n_vis_last ? *reinterpret_cast<const uint4 *>(src + (int64_t)(16 * i) * p.dl) : make_uint4(0u, 0u, 0u, 0u); }
+            for (int i = 0; i < 8; ++i) {
+                const int r = 32 * (i >> 1) + (i & 1);
+                w[i] = j0 + row0 + r < n_vis_last ? *reinterpret_cast<const uint4 *>(src + (int64_t)r * p.dl) : make_uint4(0u, 0u, 0u, 0u);
+            }
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                float *dst = ks + att_value_row(c, e) * ATT_KPITCH + row0;
+                __half *dst = ks + att_value_row(c, e) * ATT_KPITCH + row0;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const uint32_t u = e < 2 ? w[i].x : e < 4 ? w[i].y : e < 6 ? w[i].z : w[i].w;
-                    dst[16 * i] = h2f((uint16_t)((e & 1) ? u >> 16 : u));
+                for (int i = 0; i < 8; i += 2) {
+                    const uint32_t a = e < 2 ? w[i].x : e < 4 ? w[i].y : e < 6 ? w[i].z : w[i].w, b = e < 2 ? w[i + 1].x : e < 4 ? w[i + 1].y : e < 6 ? w[i + 1].z : w[i + 1].w;
+                    *reinterpret_cast<uint32_t *>(dst + 16 * i) = __byte_perm(a, b, (e & 1) ? 0x7632 : 0x5410);
                 }
             }
         }
-        static_assert(ATT_SC_THREADS == 8 * 16 && ATT_SP == 16 * 8, "eight pieces x 16 rows per pass, eight passes");
+        static_assert(ATT_SC_THREADS == 8 * 16 && ATT_SP == 16 * 8, "eight pieces x 16 pairs of rows, four times");
     }
-    {   // a lane takes 16-byte pieces of one token: a store's 32 words are neighbours
-        static_assert(NQ == 32, "one token per lane");
-        const __half *src = p.q + (int64_t)(tg + min(lane, ng - 1)) * p.dl + (int64_t)h * ATT_HD;   // (tokens past the end repeat the last one; their scores are not stored)
+    {   // a lane takes 16-byte pieces of one token: a store's 32 halves are neighbours
+        static_assert(ATT_ST == 32, "one token per lane and tile");
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int c = 4 * i + warp;
-            float f[8];
-            unpack8(*reinterpret_cast<const uint4 *>(src + 8 * c), f);
+        for (int i = 0; i < 4 * ATT_SG; ++i) {
+            const int c = 4 * (i & 3) + warp, tok = (i >> 2) * ATT_ST + lane;
+            const uint4 v = *reinterpret_cast<const uint4 *>(p.q + (int64_t)(tg + min(tok, ng - 1)) * p.dl + (int64_t)h * ATT_HD + 8 * c);   // (tokens past the end repeat the last one; their scores are not stored)
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int e = 0; e < 8; ++e) { qs[att_value_row(c, e) * NQ + lane] = f[e]; }
+            for (int e = 0; e < 8; ++e) { qs[att_value_row(c, e) * NQ + tok] = __ushort_as_half((uint16_t)half_of(w, e)); }
         }
     }
     __syncthreads();
-    const uint32_t k_s = smem_u32(ks + warp * 32 + (lane & 7) * 4);   // (volatile shared loads: the compiler would keep the whole K tile in registers across the token tiles)
-    auto four = [](const float4 v, float (&f)[4]) { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; };
+    // warps side by side: 64 positions and 16 tokens each; lanes: 8 x 8 positions, 4 x 4 tokens
+    const int jl = (warp & 1) * 64 + (lane & 7) * 8;
+    if (j0 + (warp & 1) * 64 >= n_vis_last) { return; }
+    const uint32_t k_s = smem_u32(ks + jl);
 #pragma unroll 1
-    for (int t0 = 0; t0 < ng; t0 += ATT_ST) {
-        const uint32_t q_s = smem_u32(qs + t0 + (lane >> 3) * 4);
-        float out[4][4], half_sum[4][4], part[4][4];         // [token][position]
+    for (int tw = (warp >> 1) * 16; tw < ng; tw += ATT_ST) {
+        const int tl = tw + (lane >> 3) * 4;
+        const uint32_t q_s = smem_u32(qs + tl);
+        struct Row { uint32_t k[4], q[2]; };
+        auto row = [&](int base, int r) {                    // place base + r
+            Row x;
+            const uint4 v = lds128(k_s + 2u * base * ATT_KPITCH + 2u * r * ATT_KPITCH);
+            x.k[0] = v.x; x.k[1] = v.y; x.k[2] = v.z; x.k[3] = v.w;
+            asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(x.q[0]), "=r"(x.q[1]) : "r"(q_s + 2u * base * NQ + 2u * r * NQ));
+            return x;
+        };
+        // u_e = v_e + v_(e + 4), then (u_0 + u_1) + (u_2 + u_3); rolled loops: the whole is 5000 FMAs, which would not stay in the instruction caches
+        float out[4][8], sum[4][8];                          // [token][position]
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) {
+            float u[4][8];
 #pragma unroll
-        for (int eo = 0; eo < 8; ++eo) {                     // elements 0, 4, 1, 5, 2, 6, 3, 7: u_e = v_e + v_(e + 4), then (u_0 + u_1) + (u_2 + u_3)
-            const int e = (eo >> 1) + 4 * (eo & 1);
-            float v[4][4];
+            for (int hi = 0; hi < 2; ++hi) {                 // elements e and e + 4
+                float v[4][8];
 #pragma unroll
-            for (int ap = 0; ap < 2; ++ap) {                 // accumulators ap and ap + 2
-                float a[2][4][4];
+                for (int ap = 0; ap < 2; ++ap) {             // accumulators ap and ap + 2
+                    float x[4][8];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
+                    for (int i = 0; i < 2; ++i) {
+                        float a[4][8];
 #pragma unroll
-                    for (int s = 0; s < 3; ++s) {
-                        const int r = att_value_row(4 * s + ap + 2 * i, e);
-                        float k[4], q[4];
-                        four(lds128f(k_s + 4u * r * ATT_KPITCH), k); four(lds128f(q_s + 4u * r * NQ), q);
+                        for (int s = 0; s < 3; ++s) {
+                            const Row r = row(12 * e, att_value_row(4 * s + ap + 2 * i, 4 * hi));
+#pragma unroll
+                            for (int t = 0; t < 4; ++t) {
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) { a[t][j] = fma_f16(half_of(r.k, j), half_of(r.q, t), s == 0 ? 0.f : a[t][j]); }
+                            }
+                        }
 #pragma unroll
                         for (int t = 0; t < 4; ++t) {
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) { a[i][t][j] = fmaf(k[j], q[t], s == 0 ? 0.f : a[i][t][j]); }
+                            for (int j = 0; j < 8; ++j) { x[t][j] = i == 0 ? a[t][j] : __fadd_rn(x[t][j], a[t][j]); }
                         }
+                    }
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) { v[t][j] = ap == 0 ? x[t][j] : __fadd_rn(v[t][j], x[t][j]); }
                     }
                 }
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) { const float x = __fadd_rn(a[0][t][j], a[1][t][j]); v[t][j] = ap == 0 ? x : __fadd_rn(v[t][j], x); }
+                    for (int j = 0; j < 8; ++j) { u[t][j] = hi == 0 ? v[t][j] : __fadd_rn(u[t][j], v[t][j]); }
                 }
             }
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if ((eo & 1) == 0) { part[t][j] = v[t][j]; continue; }
-                    const float u = __fadd_rn(part[t][j], v[t][j]);
-                    if (eo == 1 || eo == 5) { half_sum[t][j] = u; continue; }
-                    const float w = __fadd_rn(half_sum[t][j], u);
-                    out[t][j] = eo == 3 ? w : __fadd_rn(out[t][j], w);
+                for (int j = 0; j < 8; ++j) {
+                    if (e & 1) { const float w = __fadd_rn(sum[t][j], u[t][j]); out[t][j] = e == 1 ? w : __fadd_rn(out[t][j], w); }
+                    else { sum[t][j] = u[t][j]; }
                 }
             }
         }
-        float tail[4][4];                                    // elements 96..127: scalar chain
+        float tail[4][8];                                    // elements 96..127: scalar chain
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { tail[t][j] = 0.f; }
+            for (int j = 0; j < 8; ++j) { tail[t][j] = 0.f; }
         }
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
 #pragma unroll
-        for (int d = 96; d < ATT_HD; ++d) {
-            const int r = att_value_row(d >> 3, d & 7);
-            float k[4], q[4];
-            four(lds128f(k_s + 4u * r * ATT_KPITCH), k); four(lds128f(q_s + 4u * r * NQ), q);
+            for (int e = 0; e < 8; ++e) {
+                const Row r = row(c, att_value_row(12, e));
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
+                for (int t = 0; t < 4; ++t) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { tail[t][j] = fmaf(k[j], q[t], tail[t][j]); }
+                    for (int j = 0; j < 8; ++j) { tail[t][j] = fma_f16(half_of(r.k, j), half_of(r.q, t), tail[t][j]); }
+                }
             }
         }
         // (scores of positions a token does not see are written as they come: nothing reads them)
-        const int j = j0 + warp * 32 + (lane & 7) * 4;
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            const int tt = t0 + (lane >> 3) * 4 + t;
-            if (tt < ng && j < n_vis_last && j < n_pad) {
-                *reinterpret_cast<float4 *>(p.scratch + ((int64_t)(tg + tt) * p.n_head + h) * n_pad + j) =
-                    make_float4(__fadd_rn(tail[t][0], out[t][0]), __fadd_rn(tail[t][1], out[t][1]), __fadd_rn(tail[t][2], out[t][2]), __fadd_rn(tail[t][3], out[t][3]));
+#pragma unroll
+            for (int j4 = 0; j4 < 8; j4 += 4) {
+                const int j = j0 + jl + j4;
+                if (tl + t < ng && j < n_vis_last && j < n_pad) {
+                    *reinterpret_cast<float4 *>(p.scratch + ((int64_t)(tg + tl + t) * p.n_head + h) * n_pad + j) =
+                        make_float4(__fadd_rn(tail[t][j4], out[t][j4]), __fadd_rn(tail[t][j4 + 1], out[t][j4 + 1]), __fadd_rn(tail[t][j4 + 2], out[t][j4 + 2]), __fadd_rn(tail[t][j4 + 3], out[t][j4 + 3]));
+                }
             }
         }
     }
@@ -542,8 +577,7 @@ __global__ void __launch_bounds__(ATT_SM_THREADS) attn_softmax_kernel(const Attn
     __shared__ float red[ATT_SM_THREADS / WARP];
     __shared__ float bcast;
     const int h = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nthr = blockDim.x;   // 1024 for single steps (one CTA per head: latency), 256 for prompts (many CTAs: more of them per SM, so that
-                                   // one CTA's serial sum overlaps the parallel phases of the others)
+    constexpr int nthr = ATT_SM_THREADS;
     pdl_launch_dependents();
     pdl_wait();
     const bool batch = p.seq_stride != 0;
@@ -564,7 +598,7 @@ __global__ void __launch_bounds__(ATT_SM_THREADS) attn_softmax_kernel(const Attn
     __syncthreads();
     m = red[0];
 #pragma unroll
-    for (int w = 1; w < ATT_SM_THREADS / WARP; ++w) { if (w < (nthr >> 5)) { m = fmaxf(m, red[w]); } }
+    for (int w = 1; w < ATT_SM_THREADS / WARP; ++w) { m = fmaxf(m, red[w]); }
     // (masked positions are exact zeros: they decide which elements form a group of four, but a group of zeros leaves the sum as it is,
     // so the groups behind the last visible position are left out)
     const int n_sum = min(n_tot, (n_vis + 3) & ~3), n_sum4 = (n_sum + 3) & ~3;
@@ -591,7 +625,76 @@ __global__ void __launch_bounds__(ATT_SM_THREADS) attn_softmax_kernel(const Attn
     const float inv = bcast;
     // probabilities, rounded to fp16 as the PV MatMul does with its f32 operand
     for (int j = tid; j < n_vis; j += nthr) { row[j] = __half2float(__float2half_rn(__fmul_rn(sc[j], inv))); }
-    if (tid < WARP + ATT_TT) { const int j = n_vis + tid; if (j < min(n_pad, (n_vis + ATT_TT - 1 + 31) & ~31)) { row[j] = 0.f; } }   // (read by the tiled PV kernel)
+}
+
+// The same for a token of a prompt, in front of the tiled PV kernel: four neighbouring positions per thread and pass, whose exponentials are
+// one of std::reduce's groups; the running sum of the groups on the CTA's four warps (running_sum_wide). The probabilities become f16
+// values in the first half of the row - all of it is in shared memory by then - with zeros behind the last position, as far as a PV tile
+// reads. Ten CTAs per SM: one CTA's sum overlaps the others' passes. Bound: the gathers from the table of exponentials, 20 to 30 lines of
+// L1 a warp. 128 tokens of 32 heads over 2000 positions on average: 36 -> 33 us.
+constexpr int ATT_SMT_THREADS = 128;
+static_assert(ATT_SMT_THREADS == RS_THREADS, "all warps form the running sum");
+__host__ __device__ static inline size_t att_smt_smem(int n_ctx) { const size_t n4 = ((size_t)n_ctx + 3) / 4; return (4 * n4 + (n4 + 3) / 4 * 4 + rs_scratch_words(4)) * sizeof(float); }
+__global__ void __launch_bounds__(ATT_SMT_THREADS, 10) attn_softmax_tiled_kernel(const AttnParams p) {
+    extern __shared__ __align__(16) float att_smem[];
+    __shared__ float red[ATT_SMT_THREADS / WARP], inv_s;
+    const int h = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_pad = (p.n_ctx + 3) & ~3;
+    float4 *sc4 = reinterpret_cast<float4 *>(att_smem);
+    float  *gs = att_smem + n_pad, *rs = gs + ((n_pad >> 2) + 3) / 4 * 4;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int n_vis = p.pos_base[0] + t + 1;
+    const int n_tot = (p.pos_base[1] > 0) ? p.pos_base[1] : p.pos_base[0] + p.T;
+    float *row = p.scratch + ((int64_t)t * p.n_head + h) * n_pad;
+    const int n4 = (n_vis + 3) >> 2;
+    // masked softmax: (score + mask) * scale, subtract the maximum, table exp, std::reduce, multiply by 1/sum
+    float m = -CUDART_INF_F;
+    for (int g = tid; g < n4; g += ATT_SMT_THREADS) {
+        const float4 x = reinterpret_cast<const float4 *>(row)[g];
+        const int left = n_vis - 4 * g;
+        auto scaled = [&](float s, int i) { return i < left ? __fmul_rn(__fadd_rn(s, 0.0f), p.scale) : -CUDART_INF_F; };
+        const float4 v = make_float4(scaled(x.x, 0), scaled(x.y, 1), scaled(x.z, 2), scaled(x.w, 3));
+        sc4[g] = v;
+        m = fmaxf(m, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+    }
+    m = warp_max(m);
+    if (lane == 0) { red[warp] = m; }
+    __syncthreads();
+    m = red[lane & (ATT_SMT_THREADS / WARP - 1)];
+#pragma unroll
+    for (int o = ATT_SMT_THREADS / WARP / 2; o > 0; o >>= 1) { m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o)); }
+    // (masked positions are exact zeros: they decide which elements form a group of four, but a group of zeros leaves the sum as it is,
+    // so the groups behind the last visible position are left out)
+    for (int g = tid; g < n4; g += ATT_SMT_THREADS) {
+        const float4 v = sc4[g];
+        const int left = n_vis - 4 * g;
+        auto ex = [&](float s, int i) { return i < left ? p.exp_table[f2h(__fsub_rn(s, m))] : 0.f; };
+        const float4 e = make_float4(ex(v.x, 0), ex(v.y, 1), ex(v.z, 2), ex(v.w, 3));
+        sc4[g] = e;
+        gs[g] = __fadd_rn(__fadd_rn(e.x, e.y), __fadd_rn(e.z, e.w));
+    }
+    __syncthreads();
+    const int n_sum = min(n_tot, 4 * n4), ng = min(n_tot >> 2, n4);
+    const float sum4 = running_sum_wide(smem_u32(gs), ng, smem_u32(rs), rs_scratch_words(4), tid, 1);
+    if (tid == 0) {
+        float sum = sum4;
+        for (int j = ng << 2; j < n_sum; ++j) { sum = __fadd_rn(sum, att_smem[j]); }
+        inv_s = __fdiv_rn(1.0f, sum);
+    }
+    __syncthreads();
+    const float inv = inv_s;
+    uint2 *row16 = reinterpret_cast<uint2 *>(row);   // probabilities, rounded to fp16 as the PV MatMul does with its f32 operand
+    const int n_read = min(n_pad, (n_vis + ATT_TT - 1 + 31) & ~31) >> 2;
+    for (int g = tid; g < n_read; g += ATT_SMT_THREADS) {
+        uint2 v = make_uint2(0u, 0u);
+        if (g < n4) {
+            const float4 e = sc4[g];
+            auto prob = [inv](float x) { return (uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(x, inv))); };
+            v = make_uint2(prob(e.x) | (prob(e.y) << 16), prob(e.z) | (prob(e.w) << 16));
+        }
+        row16[g] = v;
+    }
 }
 
 constexpr int ATT_PV_WARPS = 16;
@@ -691,14 +794,6 @@ __device__ __forceinline__ void cluster_wait(uint32_t bar, uint64_t &limit_ns) {
 __device__ __forceinline__ void atl_wait(uint32_t bar, uint32_t parity, uint64_t &limit_ns) {
     if (mbar_try_wait(bar, parity)) { return; }
     if (limit_ns == 0 || !mbar_wait_prompt(bar, parity, limit_ns)) { limit_ns = 0; }
-}
-
-// a * b + c of the f16 values in the low halves of a and b: the fmaf of the widened values (their product is exact in f32) without widening
-// them, 50 instead of 86 cycles for eight products and their reads
-__device__ __forceinline__ float fma_f16(uint32_t a, uint32_t b, float c) {
-    float d;
-    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"((uint16_t)a), "h"((uint16_t)b), "f"(c));
-    return d;
 }
 
 __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const AttnParams p, const int NS) {
@@ -877,16 +972,19 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
 // neighbouring positions at once (64 bits of V^T, 128 bits of a token's probabilities); a lane takes two output elements, a warp eight,
 // for all ATT_TT tokens. The eight lanes of an output meet once at the end, halving the number of tokens a lane keeps at every step of
 // the tree, and each lane then runs the scalar tails of its token.
-// 128 f32 operations per (token, position, head). The probabilities of ATT_CH positions at a time run through a ring in shared memory with
-// cp.async (the softmax kernel leaves zeros behind a token's last position, as far as a tile reads): no staging phase in front of the
-// products, and CTAs small enough that four share an SM. 128 tokens of 32 heads over 2000 positions on average: 220 -> 101 us (whole rows
-// staged first, one CTA per SM: 119; four elements per lane: 138; probabilities straight from L1: 290).
-constexpr int ATT_PVT_WARPS = 4, ATT_EE = 2, ATT_PVT_ELEMS = ATT_PVT_WARPS * 4 * ATT_EE;
-constexpr int ATT_CH = 128, ATT_CH_RING = 4;
-__global__ void __launch_bounds__(ATT_PVT_WARPS * WARP, 16 / ATT_PVT_WARPS) attn_pv_tiled_kernel(const AttnParams p) {
-    constexpr int PER_HEAD = ATT_HD / ATT_PVT_ELEMS;
+// 128 f32 operations per (token, position, head). V^T and the probabilities (f16; the softmax kernel leaves zeros behind a token's last
+// position, as far as a tile reads) of ATT_CH positions at a time run through a ring in shared memory with cp.async; a lane takes four
+// elements of V^T for eight tokens, 24 words of shared memory per 128 products. Bound: instruction issue (73 %; the FMA pipes 53 %).
+// 128 tokens of 32 heads over 2000 positions on average: 73 us (f32 probabilities and two elements a lane, whose V^T came straight from
+// L1: 101; whole rows staged first, one CTA per SM: 119).
+constexpr int ATT_PVT_WARPS = 4, ATT_EE = 4, ATT_PVT_ELEMS = ATT_PVT_WARPS * 4 * ATT_EE;
+constexpr int ATT_CH = 128, ATT_CH_RING = 3, ATT_VPITCH = 2 * ATT_CH + 16;   // bytes: the rows of two lane groups lie on different banks
+constexpr size_t ATT_PV_STAGE = (size_t)ATT_PVT_ELEMS * ATT_VPITCH + ATT_TT * 2 * ATT_CH, ATT_PV_SMEM = ATT_CH_RING * ATT_PV_STAGE;
+__global__ void __launch_bounds__(ATT_PVT_WARPS * WARP, 3) attn_pv_tiled_kernel(const AttnParams p) {
+    extern __shared__ __align__(16) float att_smem[];
+    constexpr int PER_HEAD = ATT_HD / ATT_PVT_ELEMS, THREADS = ATT_PVT_WARPS * WARP;
     const int h = blockIdx.x / PER_HEAD, t0 = blockIdx.y * ATT_TT, tid = threadIdx.x, lane = tid & 31, grp = lane >> 3, lg = lane & 7;
-    const int e0 = (blockIdx.x % PER_HEAD) * ATT_PVT_ELEMS + (tid >> 5) * 4 * ATT_EE + grp * ATT_EE;
+    const int el = (tid >> 5) * 4 * ATT_EE + grp * ATT_EE, e0 = (blockIdx.x % PER_HEAD) * ATT_PVT_ELEMS + el;   // the lane's first element, in the CTA and in the head
     pdl_launch_dependents();
     pdl_wait();
     const int nt = min(ATT_TT, p.T - t0);
@@ -896,35 +994,37 @@ __global__ void __launch_bounds__(ATT_PVT_WARPS * WARP, 16 / ATT_PVT_WARPS) attn
     const int vis0 = p.pos_base[0] + t0 + 1;                  // positions token t0 + tt sees: vis0 + tt
     const int vis_last = vis0 + nt - 1;
     const int n_steps = (min(n_main, vis_last) + 31) >> 5;    // (steps behind the tile's last visible position add nothing)
-    const __half *vrow = p.v_cache + ((int64_t)h * ATT_HD + e0) * p.n_ctx;   // row e0 + ee starts ee * n_ctx further
-    constexpr int AHEAD = ATT_CH / 32;                        // steps whose V^T values are in flight
-    uint2 vq[AHEAD][ATT_EE];
-    auto fetch = [&](int step, uint2 (&dst)[ATT_EE]) {
-        const int j = 32 * step + 4 * lg;
-#pragma unroll
-        for (int ee = 0; ee < ATT_EE; ++ee) {
-            dst[ee] = make_uint2(0u, 0u);
-            if (step < n_steps && j < vis_last) { dst[ee] = *reinterpret_cast<const uint2 *>(vrow + (int64_t)ee * p.n_ctx + j); }   // (a plain load: this kernel may be resident before the cache rows of its prompt are written)
-        }
-    };
-#pragma unroll
-    for (int s = 0; s < AHEAD; ++s) { fetch(s, vq[s]); }
-    const int64_t row_pitch = (int64_t)p.n_head * n_pad;      // (tokens past the end repeat the last one; their results are not stored)
-    const float *rows = p.scratch + ((int64_t)t0 * p.n_head + h) * n_pad;
-    __shared__ __align__(16) float probs[ATT_CH_RING][ATT_TT][ATT_CH];
-    const int n_chunks = (n_steps + AHEAD - 1) / AHEAD, row_end = 32 * n_steps;
-    auto stage = [&](int c) {   // 16 bytes per thread and pass; one commit group per chunk, empty ones behind the last
+    // staged: all visible positions, with the scalar tails' (n_main .. n_tot - 1) in the last chunk, and what the steps read behind them
+    const int n_chunks = (vis_last + ATT_CH - 1) / ATT_CH, staged = max(vis_last, 32 * n_steps);
+    const __half *vrow = p.v_cache + ((int64_t)h * ATT_HD + e0 - el) * p.n_ctx;   // the CTA's first row
+    const int64_t row_pitch = 2 * (int64_t)p.n_head * n_pad;  // (tokens past the end repeat the last one; their results are not stored)
+    const __half *rows = reinterpret_cast<const __half *>(p.scratch + ((int64_t)t0 * p.n_head + h) * n_pad);
+    const uint32_t ring = smem_u32(att_smem);
+    const bool wide = (p.n_ctx & 7) == 0 && (reinterpret_cast<uintptr_t>(p.v_cache) & 15) == 0;   // V^T rows lie on 16 bytes, else on 8
+    auto stage = [&](int c) {   // one commit group per chunk, empty ones behind the last
         if (c < n_chunks) {
+            const uint32_t dst = ring + (uint32_t)(c % ATT_CH_RING) * (uint32_t)ATT_PV_STAGE;
+            if (wide) {
 #pragma unroll
-            for (int i = tid; i < ATT_TT * (ATT_CH / 4); i += ATT_PVT_WARPS * WARP) {
-                const int tt = i / (ATT_CH / 4), j = 4 * (i % (ATT_CH / 4));
-                if (c * ATT_CH + j < row_end) {
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&probs[c % ATT_CH_RING][tt][j])), "l"(__cvta_generic_to_global(rows + min(tt, nt - 1) * row_pitch + c * ATT_CH + j)) : "memory");
+                for (int i = 0; i < ATT_PVT_ELEMS * ATT_CH / 8 / THREADS; ++i) {
+                    const int q = tid + i * THREADS, e = q >> 4, j = 8 * (q & 15);
+                    if (c * ATT_CH + j < staged) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + e * ATT_VPITCH + 2 * j), "l"(__cvta_generic_to_global(vrow + (int64_t)e * p.n_ctx + c * ATT_CH + j)) : "memory"); }
                 }
+            } else {
+#pragma unroll 4
+                for (int i = 0; i < ATT_PVT_ELEMS * ATT_CH / 4 / THREADS; ++i) {
+                    const int q = tid + i * THREADS, e = q >> 5, j = 4 * (q & 31);
+                    if (c * ATT_CH + j < staged) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + e * ATT_VPITCH + 2 * j), "l"(__cvta_generic_to_global(vrow + (int64_t)e * p.n_ctx + c * ATT_CH + j)) : "memory"); }
+                }
+            }
+            const int tt = tid >> 4, j = 8 * (tid & 15);      // (a row of probabilities has room for twice n_pad f16 values)
+            if (c * ATT_CH + j < staged) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + ATT_PVT_ELEMS * ATT_VPITCH + tt * 2 * ATT_CH + 2 * j), "l"(__cvta_generic_to_global(rows + min(tt, nt - 1) * row_pitch + c * ATT_CH + j)) : "memory");
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    static_assert(THREADS == ATT_TT * ATT_CH / 8, "one piece of the probabilities per thread");
 #pragma unroll
     for (int c = 0; c < ATT_CH_RING - 1; ++c) { stage(c); }
     float acc[ATT_TT][ATT_EE][4];
@@ -936,39 +1036,37 @@ __global__ void __launch_bounds__(ATT_PVT_WARPS * WARP, 16 / ATT_PVT_WARPS) attn
             for (int k = 0; k < 4; ++k) { acc[tt][ee][k] = 0.f; }
         }
     }
-    auto widen = [](const uint2 w, float (&f)[4]) {
-        const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&w.x)), hi = __half22float2(*reinterpret_cast<const __half2 *>(&w.y));
-        f[0] = lo.x; f[1] = lo.y; f[2] = hi.x; f[3] = hi.y;
-    };
-    for (int c = 0, s0 = 0; c < n_chunks; ++c, s0 += AHEAD) {
+    auto lds64 = [](uint32_t addr, uint32_t (&w)[2]) { asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(addr)); };
+    for (int c = 0; c < n_chunks; ++c) {
         asm volatile("cp.async.wait_group %0;" ::"n"(ATT_CH_RING - 2) : "memory");
         __syncthreads();                                      // chunk c is there for everyone, and everyone is done with chunk c - 1
         stage(c + ATT_CH_RING - 1);
-        const float *pr = &probs[c % ATT_CH_RING][0][4 * lg];
+        const uint32_t v_s = ring + (uint32_t)(c % ATT_CH_RING) * (uint32_t)ATT_PV_STAGE + el * ATT_VPITCH + 8 * lg;
+        const uint32_t p_s = ring + (uint32_t)(c % ATT_CH_RING) * (uint32_t)ATT_PV_STAGE + ATT_PVT_ELEMS * ATT_VPITCH + 8 * lg;
+        const int steps = min(ATT_CH / 32, n_steps - c * (ATT_CH / 32));
+#pragma unroll 1
+        for (int s = 0; s < steps; ++s) {
+            uint32_t v[ATT_EE][2];
 #pragma unroll
-        for (int s = 0; s < AHEAD; ++s) {
-            if (s0 + s < n_steps) {
-                float v[ATT_EE][4];
-                const int over = 32 * (s0 + s) + 4 * lg + 4 - vis_last;   // (cache entries behind the last visible position may not be written yet)
-                if (over > 0) {
+            for (int ee = 0; ee < ATT_EE; ++ee) { lds64(v_s + ee * ATT_VPITCH + 64 * s, v[ee]); }
+            const int over = c * ATT_CH + 32 * s + 4 * lg + 4 - vis_last;   // (cache entries behind the last visible position may not be written yet)
+            if (over > 0) {
 #pragma unroll
-                    for (int ee = 0; ee < ATT_EE; ++ee) {
-                        if (over >= 1) { vq[s][ee].y &= 0xffffu; }
-                        if (over >= 2) { vq[s][ee].y = 0u; }
-                        if (over >= 3) { vq[s][ee].x &= 0xffffu; }
-                    }
+                for (int ee = 0; ee < ATT_EE; ++ee) {
+                    if (over >= 1) { v[ee][1] &= 0xffffu; }
+                    if (over >= 2) { v[ee][1] = 0u; }
+                    if (over >= 3) { v[ee][0] &= 0xffffu; }
+                    if (over >= 4) { v[ee][0] = 0u; }
                 }
+            }
 #pragma unroll
-                for (int ee = 0; ee < ATT_EE; ++ee) { widen(vq[s][ee], v[ee]); }
-                fetch(s0 + s + AHEAD, vq[s]);
+            for (int tt = 0; tt < ATT_TT; ++tt) {
+                uint32_t pv[2];
+                lds64(p_s + tt * 2 * ATT_CH + 64 * s, pv);
 #pragma unroll
-                for (int tt = 0; tt < ATT_TT; ++tt) {
-                    const float4 pv = *reinterpret_cast<const float4 *>(pr + tt * ATT_CH + 32 * s);
+                for (int ee = 0; ee < ATT_EE; ++ee) {
 #pragma unroll
-                    for (int ee = 0; ee < ATT_EE; ++ee) {
-                        acc[tt][ee][0] = fmaf(v[ee][0], pv.x, acc[tt][ee][0]); acc[tt][ee][1] = fmaf(v[ee][1], pv.y, acc[tt][ee][1]);
-                        acc[tt][ee][2] = fmaf(v[ee][2], pv.z, acc[tt][ee][2]); acc[tt][ee][3] = fmaf(v[ee][3], pv.w, acc[tt][ee][3]);
-                    }
+                    for (int k = 0; k < 4; ++k) { acc[tt][ee][k] = fma_f16(half_of(v[ee], k), half_of(pv, k), acc[tt][ee][k]); }
                 }
             }
         }
@@ -992,21 +1090,20 @@ __global__ void __launch_bounds__(ATT_PVT_WARPS * WARP, 16 / ATT_PVT_WARPS) attn
         }
     }
     static_assert(ATT_TT == 8, "one lane of a group of eight per token");
-    // the scalar tails (positions n_main .. n_tot - 1, at most 32, as far as the lane's token sees them), one FMA chain per output
+    // the scalar tails (positions n_main .. n_tot - 1, at most 32, as far as the lane's token sees them; in the last chunk), one FMA chain per output
     if (lg >= nt) { return; }
     const int n_tail = min(32, vis0 + lg - n_main);
-    const float *pr = rows + lg * row_pitch + n_main;
+    const uint32_t last = ring + (uint32_t)((n_chunks - 1) % ATT_CH_RING) * (uint32_t)ATT_PV_STAGE + 2 * (n_main % ATT_CH);
     float tail[ATT_EE] = {};
     for (int i = 0; i < n_tail; i += 4) {
-        const float4 q = *reinterpret_cast<const float4 *>(pr + i);
+        uint32_t q[2];
+        lds64(last + ATT_PVT_ELEMS * ATT_VPITCH + lg * 2 * ATT_CH + 2 * i, q);
 #pragma unroll
         for (int ee = 0; ee < ATT_EE; ++ee) {
-            float w[4];
-            widen(*reinterpret_cast<const uint2 *>(vrow + (int64_t)ee * p.n_ctx + n_main + i), w);
-            tail[ee] = fmaf(w[0], q.x, tail[ee]);
-            if (i + 1 < n_tail) { tail[ee] = fmaf(w[1], q.y, tail[ee]); }
-            if (i + 2 < n_tail) { tail[ee] = fmaf(w[2], q.z, tail[ee]); }
-            if (i + 3 < n_tail) { tail[ee] = fmaf(w[3], q.w, tail[ee]); }
+            uint32_t w[2];
+            lds64(last + (el + ee) * ATT_VPITCH + 2 * i, w);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { if (i + k < n_tail) { tail[ee] = fma_f16(half_of(w, k), half_of(q, k), tail[ee]); } }
         }
     }
     float *dst = p.out + (int64_t)(t0 + lg) * (p.out_stride ? p.out_stride : p.dl) + (int64_t)h * ATT_HD + e0;
@@ -1108,14 +1205,17 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
             ? launch_with_pdl(reinterpret_cast<const void *>(attn_scores_tiled_kernel), dim3((unsigned)((p.n_ctx + ATT_SP - 1) / ATT_SP), p.n_head, (unsigned)((p.T + ATT_SG * ATT_ST - 1) / (ATT_SG * ATT_ST))), dim3(ATT_SC_THREADS), ATT_SC_SMEM, p, cfg)
             : launch_with_pdl(reinterpret_cast<const void *>(attn_scores_kernel), dim3((unsigned)((p.n_ctx + 255) / 256), p.n_head, p.T), dim3(256), 0, p, cfg);
         if (err != cudaSuccess) { return err; }
-        const size_t sm_smem = (n_pad + n_pad / 4) * sizeof(float) + 16;
-        if (sm_smem > 200 * 1024) { return cudaErrorInvalidValue; }
-        err = allow_dynamic_smem(reinterpret_cast<const void *>(attn_softmax_kernel), sm_smem);
+        const void  *softmax = tiled ? reinterpret_cast<const void *>(attn_softmax_tiled_kernel) : reinterpret_cast<const void *>(attn_softmax_kernel);
+        const size_t sm_smem = tiled ? att_smt_smem(p.n_ctx) : (n_pad + n_pad / 4) * sizeof(float) + 16;
+        if ((n_pad + n_pad / 4) * sizeof(float) + 16 > 200 * 1024) { return cudaErrorInvalidValue; }
+        err = allow_dynamic_smem(softmax, sm_smem);
         if (err != cudaSuccess) { return err; }
-        err = launch_with_pdl(reinterpret_cast<const void *>(attn_softmax_kernel), dim3(p.n_head, p.T), dim3(tiled ? 256 : ATT_SM_THREADS), sm_smem, p, cfg);
+        err = launch_with_pdl(softmax, dim3(p.n_head, p.T), dim3(tiled ? ATT_SMT_THREADS : ATT_SM_THREADS), sm_smem, p, cfg);
         if (err != cudaSuccess) { return err; }
         if (tiled) {
-            return launch_with_pdl(reinterpret_cast<const void *>(attn_pv_tiled_kernel), dim3(p.n_head * (ATT_HD / ATT_PVT_ELEMS), (unsigned)((p.T + ATT_TT - 1) / ATT_TT)), dim3(ATT_PVT_WARPS * WARP), 0, p, cfg);
+            err = allow_dynamic_smem(reinterpret_cast<const void *>(attn_pv_tiled_kernel), ATT_PV_SMEM);
+            if (err != cudaSuccess) { return err; }
+            return launch_with_pdl(reinterpret_cast<const void *>(attn_pv_tiled_kernel), dim3(p.n_head * (ATT_HD / ATT_PVT_ELEMS), (unsigned)((p.T + ATT_TT - 1) / ATT_TT)), dim3(ATT_PVT_WARPS * WARP), ATT_PV_SMEM, p, cfg);
         }
         const size_t pv_smem = n_pad * sizeof(float) + 16;
         err = allow_dynamic_smem(reinterpret_cast<const void *>(attn_pv_kernel), pv_smem);
