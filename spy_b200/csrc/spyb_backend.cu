@@ -424,7 +424,7 @@ spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const voi
         be->set_error("prefill_matmul: needs k a multiple of 32 up to %d, 1..4096 columns", PF_MAX_K); return SPYB_UNSUPPORTED;
     }
     cudaSetDevice(be->config.device_id);
-    const int nb = (int)(k / QK), T = (int)n_cols, tile_tok = prefill_tile_tokens(weight_type, n_rows, T);
+    const int nb = (int)(k / QK), T = (int)n_cols, tile_tok = prefill_tile_tokens(weight_type, n_rows, nb, T);
     const int64_t rb = kq ? (k / 256) * (weight_type == SPYB_Q4_K ? 144 : 210) : (int64_t)nb * (weight_type == SPYB_Q4_0 ? 18 : 34);
     const size_t wbytes = prefill_weight_bytes(weight_type, n_rows, nb), ybytes = prefill_act_bytes(T, nb);
     uint8_t *raw = nullptr, *w = nullptr, *yq = nullptr; float *x = nullptr, *nw = nullptr, *out = nullptr;
@@ -456,16 +456,16 @@ spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const voi
     return SPYB_SUCCESS;
 }
 
-// Failure-path check of the prompt GEMM that faults nothing: one small launch whose copy thread leaves the second batch of
-// blocks out, with `limit_ns` as the bound of every wait. The roles that wait for that batch give up one after the other,
-// the kernel frees its tensor memory and returns, and the error word holds a code of the prompt kernel (4, 5 or 6).
+// Failure-path check of the prompt GEMM that faults nothing: a small launch of one CTA, then one of a cluster of two (more blocks a row), whose
+// copy thread leaves the second batch of blocks out, with `limit_ns` as the bound of every wait. The roles that wait for that batch give up
+// one after the other, the kernel frees its tensor memory and returns, and the error word holds a code of the prompt kernel (4, 5 or 6).
 spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *be, uint64_t limit_ns, int32_t *error_code_out) {
     if (be == nullptr || limit_ns == 0) { return SPYB_FAIL; }
     cudaSetDevice(be->config.device_id);
     SPYB_CUDA(be, cudaStreamSynchronize(be->stream));
     if (be->device_error()) { return SPYB_FAIL; }
-    const int nb = 12, T = PF_TOK;
-    const size_t wbytes = prefill_weight_bytes(SPYB_Q8_0, PF_ROWS, nb), ybytes = prefill_act_bytes(T, nb);
+    constexpr int nb_max = 128, T = PF_TOK;
+    const size_t wbytes = prefill_weight_bytes(SPYB_Q8_0, PF_ROWS, nb_max), ybytes = prefill_act_bytes(T, nb_max);
     uint8_t *w = nullptr, *yq = nullptr; float *out = nullptr;
     auto release = [&]() { cudaFree(w); cudaFree(yq); cudaFree(out); };
     cudaError_t err = cudaMalloc(&w, wbytes);
@@ -473,18 +473,21 @@ spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *be, uint64_t limit_
     if (err == cudaSuccess) { err = cudaMalloc(&out, (size_t)T * PF_ROWS * 4); }
     if (err == cudaSuccess) { err = cudaMemsetAsync(w, 0, wbytes, be->stream); }
     if (err == cudaSuccess) { err = cudaMemsetAsync(yq, 0, ybytes, be->stream); }
-    if (err == cudaSuccess) {
+    int code = 0;
+    for (const int nb : {12, nb_max}) {
+        if (err != cudaSuccess) { break; }
         PrefillGemm g;
-        g.w = w; g.type = SPYB_Q8_0; g.n_rows = PF_ROWS; g.nb = nb; g.yq = yq; g.tile_tok = prefill_tile_tokens(SPYB_Q8_0, PF_ROWS, T); g.T = T; g.out = out; g.out_stride = PF_ROWS;
+        g.w = w; g.type = SPYB_Q8_0; g.n_rows = PF_ROWS; g.nb = nb; g.yq = yq; g.tile_tok = prefill_tile_tokens(SPYB_Q8_0, PF_ROWS, nb, T); g.T = T; g.out = out; g.out_stride = PF_ROWS;
         g.error_flag = be->d_error_flag; g.wait_limit_ns = limit_ns; g.selftest_skip_step = 1;
         err = launch_prefill_gemm(g, be->stream);
+        if (err == cudaSuccess) { err = cudaStreamSynchronize(be->stream); }   // returns: the kernel ended by itself
+        code = *reinterpret_cast<volatile int *>(be->h_error_flag);
+        *reinterpret_cast<volatile int *>(be->h_error_flag) = 0;   // the check leaves the backend usable
+        if (code < 4 || code > 6) { break; }
     }
-    if (err == cudaSuccess) { err = cudaStreamSynchronize(be->stream); }   // returns: the kernel ended by itself
     release();
     if (err != cudaSuccess) { be->set_error("prefill selftest: %s", cudaGetErrorString(err)); return SPYB_FAIL; }
-    const int code = *reinterpret_cast<volatile int *>(be->h_error_flag);
     if (error_code_out != nullptr) { *error_code_out = code; }
-    *reinterpret_cast<volatile int *>(be->h_error_flag) = 0;   // the check leaves the backend usable
     if (code < 4 || code > 6) { be->set_error("prefill selftest: expected a wait of the prompt kernel to give up (codes 4-6), got %d", code); return SPYB_FAIL; }
     return SPYB_SUCCESS;
 }
@@ -577,7 +580,7 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
         const int Tc = (int)std::min(chunk, T - t0);
         const bool pdl = be->config.use_pdl != 0;   // (columns that pad the last tile hold whatever the buffer held: their results are not stored)
         PrefillGemm g;
-        g.tile_tok = prefill_tile_tokens(type, n_rows, Tc);
+        g.tile_tok = prefill_tile_tokens(type, n_rows, nb, Tc);
         SPYB_CUDA(be, launch_prefill_quant(static_cast<const float *>(x.data) + t0 * k, k, Tc, (int)k, nullptr, 0.f, static_cast<uint8_t *>(yq), be->stream, type, g.tile_tok, 0, 0, pdl));
         g.w = tiles; g.type = type; g.n_rows = n_rows; g.nb = nb; g.yq = static_cast<uint8_t *>(yq); g.T = Tc;
         g.out = static_cast<float *>(out_dev) + t0 * n_rows; g.out_stride = n_rows;

@@ -105,6 +105,28 @@ __device__ __forceinline__ bool mbar_wait_prompt(uint32_t bar, uint32_t parity, 
     }
     return mbar_wait_bounded(bar, parity, limit_ns);
 }
+// thread-block clusters: an address in another CTA's shared memory, a store and an arrival there, the barrier of all threads
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ void cluster_store64(uint32_t addr, uint64_t v) { asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
+__device__ __forceinline__ void cluster_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// waits for arrivals of other CTAs of the cluster, and sees what they wrote before; limit_ns becomes zero when they do not come in time
+__device__ __forceinline__ void cluster_wait(uint32_t bar, uint32_t parity, uint64_t &limit_ns) {
+    const uint64_t t0 = global_timer_ns();
+    for (;;) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) { return; }
+        if (global_timer_ns() - t0 >= limit_ns) { limit_ns = 0; return; }
+    }
+}
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst_smem, const void *src_gmem, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst_smem), "l"(__cvta_generic_to_global(src_gmem)), "r"(bytes), "r"(bar) : "memory");

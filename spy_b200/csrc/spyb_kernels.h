@@ -133,7 +133,7 @@ struct PrefillGemm {
     int            selftest_skip_step = -1;   // failure-path check: the copy warp leaves this step out, so the waits for it run out
 };
 int         device_sms();         // SMs of the current device
-int         prefill_tile_tokens(int type, int64_t n_rows, int T);   // width of the token tiles for this matrix and number of tokens
+int         prefill_tile_tokens(int type, int64_t n_rows, int nb, int T);   // width of the token tiles for this matrix and number of tokens
 size_t      prefill_weight_bytes(int type, int64_t n_rows, int nb);
 size_t      prefill_act_bytes(int T, int nb);
 cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);

@@ -514,13 +514,13 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
     // the quantized activations are laid out for the type of the matrix they meet and for its token tile: quant() makes them for the
     // first matrix of a group, gemm() makes them again when a later matrix of the group wants another form
     struct { const float *x; int part_len; const float *norm_w; int K; int64_t part_stride; int type, tile_tok; } yq_src = {};
-    auto layout_of = [&](const PfMat &W) { return ((W.type == SPYB_Q4_K || W.type == SPYB_Q6_K) ? 1000 : 0) + prefill_tile_tokens(W.type, W.n_rows, T); };
+    auto layout_of = [&](const PfMat &W, int K) { return ((W.type == SPYB_Q4_K || W.type == SPYB_Q6_K) ? 1000 : 0) + prefill_tile_tokens(W.type, W.n_rows, K / 32, T); };
     auto quant = [&](const float *x, int part_len, int K, const float *norm_w, const PfMat &W, int64_t part_stride, uint8_t *tap_xq = nullptr) {
-        yq_src = {x, part_len, norm_w, K, part_stride, W.type, prefill_tile_tokens(W.type, W.n_rows, T)};
+        yq_src = {x, part_len, norm_w, K, part_stride, W.type, prefill_tile_tokens(W.type, W.n_rows, K / 32, T)};
         return launch_prefill_quant(x, part_len, T, K, norm_w, norm_w != nullptr ? m->info.rms_eps : 0.f, m->pf_yq, s, W.type, yq_src.tile_tok, part_len, part_stride, pdl, tap_xq);
     };
     auto gemm = [&](const PfMat &W, int K, float *out, int64_t out_stride, const float *resid) {
-        if (layout_of(W) != ((yq_src.type == SPYB_Q4_K || yq_src.type == SPYB_Q6_K) ? 1000 : 0) + yq_src.tile_tok) {
+        if (layout_of(W, K) != ((yq_src.type == SPYB_Q4_K || yq_src.type == SPYB_Q6_K) ? 1000 : 0) + yq_src.tile_tok) {
             cudaError_t e = quant(yq_src.x, yq_src.part_len, yq_src.K, yq_src.norm_w, W, yq_src.part_stride);
             if (e != cudaSuccess) { return e; }
             ++*launches;
@@ -1443,7 +1443,7 @@ spyb_status spyb_model_decode_batch(spyb_model *m, const int32_t *first_tokens, 
             if (m->pf_head.w != nullptr) {   // the logits of all sequences from one GEMM
                 const bool pdl = be->config.use_pdl != 0;
                 PrefillGemm g;
-                g.w = m->pf_head.w; g.type = m->pf_head.type; g.n_rows = V; g.nb = d / 32; g.yq = m->pf_yq; g.tile_tok = prefill_tile_tokens(g.type, V, n_seq);
+                g.w = m->pf_head.w; g.type = m->pf_head.type; g.n_rows = V; g.nb = d / 32; g.yq = m->pf_yq; g.tile_tok = prefill_tile_tokens(g.type, V, d / 32, n_seq);
                 g.T = n_seq; g.out = m->logits_batch; g.out_stride = V; g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
                 SPYB_CUDA(be, launch_prefill_quant(m->pf_x, dp, n_seq, d, m->output_norm, m->info.rms_eps, m->pf_yq, be->stream, g.type, g.tile_tok, dp, (int64_t)n_seq * dp, pdl));
                 SPYB_CUDA(be, launch_prefill_gemm(g, be->stream, pdl));

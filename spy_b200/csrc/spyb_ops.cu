@@ -771,26 +771,6 @@ __host__ __device__ static inline AtlSmem atl_smem(int n_ctx) {   // offsets in 
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(__cvta_generic_to_global(src)) : "memory");
 }
-__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_store(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
-__device__ __forceinline__ void cluster_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-// waits for the cluster's arrivals (phase 0); as mbar_wait_lean, limit_ns becomes zero when they do not come
-__device__ __forceinline__ void cluster_wait(uint32_t bar, uint64_t &limit_ns) {
-    const uint64_t t0 = global_timer_ns();
-    for (;;) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
-        if (ok) { return; }
-        if (global_timer_ns() - t0 >= limit_ns) { limit_ns = 0; return; }
-    }
-}
 __device__ __forceinline__ void atl_wait(uint32_t bar, uint32_t parity, uint64_t &limit_ns) {
     if (mbar_try_wait(bar, parity)) { return; }
     if (limit_ns == 0 || !mbar_wait_prompt(bar, parity, limit_ns)) { limit_ns = 0; }
@@ -870,7 +850,7 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
             cluster_store(cluster_map(smem_u32(red + rank * ATL_WARPS + warp), lane), m);
             cluster_arrive(cluster_map(max_s, lane));
         }
-        cluster_wait(max_s, limit);
+        cluster_wait(max_s, 0u, limit);
         m = warp_max(red[lane]);
         // exponentials and their sums of four, to all CTAs of the cluster
         for (int k0 = warp; k0 < nK; k0 += 4 * ATL_WARPS) {
@@ -896,7 +876,7 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
         }
         __syncwarp();
         if (lane < ATL_C) { cluster_arrive(cluster_map(exp_s, lane)); }
-        cluster_wait(exp_s, limit);
+        cluster_wait(exp_s, 0u, limit);
         // std::reduce: groups of four, in order; masked positions are exact zeros that decide which elements form a group
         const int n_sum = min(n_tot, (n_vis + 3) & ~3), ng = min(n_tot >> 2, (n_vis + 3) >> 2);
         if (warp < RS_THREADS / WARP) {

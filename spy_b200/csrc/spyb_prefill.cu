@@ -28,12 +28,13 @@ namespace spyb {
 
 namespace {
 
+constexpr int PF_HALF = 4096;   // bytes of half a block's weights: 16 f16 values of 128 rows
 constexpr int PF_QUANT_THREADS = 512;
 constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF_QUANT_THREADS);   // groups of eight values per thread
 
 // ---------------------------------------------------------------------------------------------
 // the GEMM: persistent CTAs (one per SM, all 512 tensor-memory columns), each walking tiles of 128 rows x TT tokens along K in
-// steps of NB = 32 / TT blocks, so that a step is 256 columns of D whatever the tile's width; two D buffers. 20 warps (96 registers):
+// steps of NB = 32 S / TT blocks, so that a step is 256 columns of D whatever the tile's width; two D buffers. 20 warps (96 registers):
 //   warps 0-15  epilogue: row = 32 (warp % 4) + lane, a quarter of the tile's tokens; four warps per scheduler hide the latency of tensor
 //               memory and of the hand-offs behind one another's FMAs
 //   warp 16     streams the operands of step after step with cp.async.bulk (weights: A operands as they are; compact activations)
@@ -43,39 +44,56 @@ constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF
 //
 // Bound: issue slots. A step is 32 packed FMAs (two slots each: a packed FMA measures no faster than 2.5 cycles per scheduler) and 4 packed
 // multiplies per epilogue warp, i.e. 290 slots per scheduler, and everything else around them another 165; the loop is written for few
-// instructions (waits of one test and one branch, D buffers as constants of the unrolled code, one arrival per step), and measures 600
-// cycles per step: 4096 x 4096 x 448 tokens 155 us, 22016 rows 690 us (the e4m3 form: 216 and 1017 us). Tiles of 32 tokens halve the
-// weight bytes per FMA but need 110 registers: spills, 265 us. Eight epilogue warps with 216 registers each: 186-208 us.
-template <int TT> struct PfGeom {
-    static constexpr int NB     = 32 / TT;                                // blocks per step
+// instructions (waits of one test and one branch, D buffers as constants of the unrolled code, one arrival per step), and measures 570
+// cycles per step: 4096 x 4096 x 448 tokens 138 us, 22016 rows 644 us (the e4m3 form: 216 and 1017 us). Tiles of 32 tokens halve the
+// weight bytes per FMA but need 110 registers: spills, 265 us. Eight epilogue warps with 216 registers each: 186-208 us. (The epilogue's
+// registers are all taken: the same source with signed tile numbers, or with the expansion's two offsets computed for S = 2 in both forms,
+// is allocated differently and measures 709 or 668 us on the 22016 rows.)
+//
+// S = 2: few tokens of a matrix of few rows are fewer tiles than SMs, and a CTA takes no more than some 55 GB/s of weights. A cluster of two
+// CTAs then shares a tile by the halves of its blocks: the eight accumulators of an output are independent chains until the row's end, four
+// of them read the first 16 values of every block and four the others, so each CTA streams and multiplies one half of the weights (the
+// scales lie between the halves) for four chains of twice the blocks per step, and at the end of a tile the second CTA's epilogue warps leave their sums in
+// the first one's shared memory, where they are added in the tree's order. 4096 x 11008 x 8 tokens 52 -> 31.5 us, 4096 x 4096 x 8 21 -> 15.
+// Where the tiles fill the chip it costs more (a scale product for every four FMAs, the scales twice): prefill_tile_tokens has the line.
+template <int TT, int S> struct PfGeom {
+    static constexpr int NB     = 32 * S / TT;                            // blocks per step
     static constexpr int YB     = TT * 64 + TT * 4;                       // a block's compact activations: TT x 32 f16, TT f32 scales
-    static constexpr int RAW    = NB * (PF_WTILE_F16 + YB);               // a step as it arrives
+    static constexpr int HS     = 2 / S;                                  // halves of a block that a CTA takes
+    static constexpr int WB     = HS * PF_HALF + 512;                     // a block's weights: its halves, the scales (between them, so that both lie beside either)
+    static constexpr int RAW    = NB * (WB + YB);                         // a step as it arrives
     static constexpr int STAGE  = RAW + 8192;                             // ... and its B operands
     static constexpr int NS     = TT == 16 ? 6 : 4;                       // steps in the ring (even)
     static constexpr int PW     = TT / 8;                                 // token pairs per epilogue warp
     static constexpr int PC     = PW < 2 ? 1 : 2;                         // pairs per chunk of tensor-memory columns (8 columns each)
-    static constexpr int NC     = NB * 2 * (PW / PC);                     // chunks per step and warp
-    static constexpr size_t SMEM = (size_t)NS * STAGE + 8 * (3 * NS + 4) + 16;
+    static constexpr int NC     = NB * HS * (PW / PC);                    // chunks per step and warp
+    static constexpr int XCH    = S == 2 ? PF_GEMM_EPI_WARPS * 32 * PW * 4 * 8 : 0;   // the other CTA's accumulators
+    static constexpr int BARS   = NS * STAGE + XCH;
+    static constexpr int N_BAR  = 3 * NS + 4 + (S == 2 ? 2 * PF_GEMM_EPI_WARPS : 0);
+    static constexpr size_t SMEM = (size_t)BARS + 8 * N_BAR + 16;
 };
 
-template <int TT>
+template <int TT, int S>
 __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(PrefillGemm g) {
-    using G = PfGeom<TT>;
-    constexpr int NB = G::NB, NS = G::NS, PW = G::PW, PC = G::PC, YB = G::YB;
+    using G = PfGeom<TT, S>;
+    constexpr int NB = G::NB, NS = G::NS, PW = G::PW, PC = G::PC, YB = G::YB, HS = G::HS, WB = G::WB;
     extern __shared__ __align__(128) uint8_t smem[];
-    const uint32_t sbase = smem_u32(smem), bars = sbase + NS * G::STAGE;
-    // a stage: [NB weight tiles][NB compact activation blocks][8192 bytes of B operands]
+    const uint32_t sbase = smem_u32(smem), bars = sbase + G::BARS;
+    // a stage: [NB blocks of weights: first half, 128 scales, second half (S = 2: the CTA's half and the scales)][NB compact activation blocks][8192 bytes of B operands]
     auto raw_full = [&](int s) { return bars + 8u * s; };                       // the step's weights and activations have landed
     auto ops_full = [&](int s) { return bars + 8u * (NS + s); };                // its B operands are written and fenced
     auto st_free  = [&](int s) { return bars + 8u * (2 * NS + s); };            // the stage may be refilled: its step's D buffer and scales have been read (arrival by the MMA warp, which waits for that anyway)
     auto d_full   = [&](int i) { return bars + 8u * (3 * NS + i); };            // the MMAs into buffer i have completed
     auto d_free   = [&](int i) { return bars + 8u * (3 * NS + 2 + i); };        // buffer i has been read (one arrival per epilogue warp)
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + (size_t)NS * G::STAGE + 8 * (3 * NS + 4));
+    auto x_full   = [&](int w) { return bars + 8u * (3 * NS + 4 + w); };        // (S = 2) epilogue warp w of the other CTA has left its accumulators here
+    auto x_free   = [&](int w) { return bars + 8u * (3 * NS + 4 + PF_GEMM_EPI_WARPS + w); };   // ... and here: the other CTA has read them
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + G::BARS + 8 * G::N_BAR);
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nb = g.nb, n_step = (nb + NB - 1) / NB;
     const int n_tok = (g.T + TT - 1) / TT;
     const int n_tile = n_tok * (int)((g.n_rows + PF_M - 1) / PF_M);
+    const int rank = S == 2 ? (int)(blockIdx.x & 1) : 0;   // (the CTAs of a cluster walk the same tiles)
     const uint64_t limit = g.wait_limit_ns;
 
     // The barriers, the zeroed B operands, the tensor memory and the first weights need nothing of the previous kernel; every role waits
@@ -84,6 +102,9 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(raw_full(s), 1); mbar_init(ops_full(s), 1); mbar_init(st_free(s), 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(d_full(i), 1); mbar_init(d_free(i), PF_GEMM_EPI_WARPS); }
+        if (S == 2) {
+            for (int w = 0; w < PF_GEMM_EPI_WARPS; ++w) { mbar_init(x_full(w), 1); mbar_init(x_free(w), 1); }
+        }
         mbar_init_fence();
     }
     // the B operands are zero except where the expansion writes, and it writes the same places in every step
@@ -95,6 +116,7 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
+    if (S == 2) { cluster_sync(); }   // (the other CTA's barriers are there)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
@@ -107,18 +129,39 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             uint32_t par = 1;
             bool ok = true;
             // the weights of the first tile's first steps, then (the previous kernel is done) their activations with all that follows
-            const int early = blockIdx.x < n_tile ? min(NS, n_step) : 0;
+            const int early = blockIdx.x / S < n_tile ? min(NS, n_step) : 0;
+            // One copy a step where the weights' way through HBM is the bound (32000 x 4096 x 16 tokens 49.7 us, in pieces 50.1); with more
+            // tokens, when the epilogue is and the weights come out of L2, halves of blocks (22016 x 4096 x 448 tokens 659 us in one copy,
+            // 649 in blocks, 643 in halves, 646 in quarters: short bursts into shared memory are in the epilogue's way for less long)
+            const bool pieces = n_tok > 4;
+            // n blocks of weights at `w` into stage st
+            auto copy_weights = [&](int st, const uint8_t *w, int n) {
+                const uint32_t dst = sbase + (uint32_t)st * G::STAGE;
+                if (S == 1 && (TT == 8 || !pieces)) { bulk_copy_g2s(dst, w, (uint32_t)(n * WB), raw_full(st)); }
+                else if (S == 1) {
+#pragma unroll
+                    for (int j = 0; j < 2 * NB; ++j) {
+                        if (j < 2 * n) { bulk_copy_g2s(dst + j * (WB / 2), w + (int64_t)j * (WB / 2), WB / 2, raw_full(st)); }
+                    }
+                }
+                else {
+#pragma unroll
+                    for (int j = 0; j < NB; ++j) {
+                        if (j < n) { bulk_copy_g2s(dst + j * WB, w + (int64_t)j * PF_WTILE_F16 + rank * PF_HALF, WB, raw_full(st)); }
+                    }
+                }
+            };
             if (elect_one()) {
                 for (int i = 0; i < early; ++i) {
                     if (i == g.selftest_skip_step) { continue; }
                     const int n = min(NB, nb - i * NB);
-                    mbar_expect_tx(raw_full(i), (uint32_t)(n * (PF_WTILE_F16 + YB)));
-                    bulk_copy_g2s(sbase + (uint32_t)i * G::STAGE, g.w + ((int64_t)(blockIdx.x / n_tok) * nb + i * NB) * PF_WTILE_F16, (uint32_t)(n * PF_WTILE_F16), raw_full(i));
+                    mbar_expect_tx(raw_full(i), (uint32_t)(n * (WB + YB)));
+                    copy_weights(i, g.w + ((int64_t)(blockIdx.x / S / n_tok) * nb + i * NB) * PF_WTILE_F16, n);
                 }
             }
             __syncwarp();
             pdl_wait();
-            for (int tile = blockIdx.x; tile < n_tile && ok; tile += gridDim.x) {
+            for (int tile = blockIdx.x / S; tile < n_tile && ok; tile += gridDim.x / S) {
                 const uint8_t *wsrc = g.w + (int64_t)(tile / n_tok) * nb * PF_WTILE_F16;
                 const uint8_t *ysrc = g.yq + (int64_t)(tile % n_tok) * nb * YB;
                 for (int i = 0; i < n_step; ++i, ++k) {
@@ -130,10 +173,10 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                     if (k != g.selftest_skip_step && elect_one()) {   // (failure-path check: that step never arrives)
                         const uint32_t dst = sbase + (uint32_t)st * G::STAGE;
                         if (k >= early) {
-                            mbar_expect_tx(raw_full(st), (uint32_t)(n * (PF_WTILE_F16 + YB)));
-                            bulk_copy_g2s(dst, wsrc, (uint32_t)(n * PF_WTILE_F16), raw_full(st));
+                            mbar_expect_tx(raw_full(st), (uint32_t)(n * (WB + YB)));
+                            copy_weights(st, wsrc, n);
                         }
-                        bulk_copy_g2s(dst + NB * PF_WTILE_F16, ysrc, (uint32_t)(n * YB), raw_full(st));
+                        bulk_copy_g2s(dst + NB * WB, ysrc, (uint32_t)(n * YB), raw_full(st));
                     }
                     __syncwarp();
                     issued = k + 1;
@@ -149,22 +192,24 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
         } else if (warp == PF_GEMM_EPI_WARPS + 1) {
             // ---- expansion. The four values of accumulator n of token t in half h of a block go to row 8 (t / 2) + 2 n + t % 2 of the half's
             // B operand (4 TT rows x 16), at their place 4 n; the rest of B stays zero. A lane takes 16 bytes (accumulators 2 np and
-            // 2 np + 1) at a time.
+            // 2 np + 1) at a time, four times in a step.
             int st = 0;
             uint32_t par = 0;
-            const int h = (lane >> 1) & 1, np = lane & 1, t0 = lane >> 2;   // token t0 + 8 k of the step (block (t0 + 8 k) / TT)
-            const uint32_t dst_lane = (uint32_t)(h * 128 * TT + np * (64 * TT + 64) + (t0 >> 1) * 128 + (t0 & 1) * 16);
-            for (int tile = blockIdx.x; tile < n_tile && left_ns != 0; tile += gridDim.x) {
+            constexpr int TK = 8 * S;   // token t0 + TK k of the step (block (t0 + TK k) / TT), of the one half that a CTA takes or of both
+            const int h = S == 2 ? 0 : (lane >> 1) & 1, np = lane & 1, t0 = S == 2 ? lane >> 1 : lane >> 2;
+            const uint32_t dst_lane = (uint32_t)((S == 2 ? (t0 / TT) * 128 * TT : 0) + h * 128 * TT + np * (64 * TT + 64) + ((S == 2 ? t0 % TT : t0) >> 1) * 128 + (t0 & 1) * 16);
+            const uint32_t src_lane = (uint32_t)(S == 2 ? (t0 / TT) * YB + (t0 % TT) * 64 + rank * 32 + np * 16 : lane * 16);
+            for (int tile = blockIdx.x / S; tile < n_tile && left_ns != 0; tile += gridDim.x / S) {
                 for (int i = 0; i < n_step; ++i) {
                     mbar_wait_lean(raw_full(st), par, left_ns);
                     if (left_ns == 0) { break; }
-                    const uint32_t base = sbase + (uint32_t)st * G::STAGE, src = base + NB * PF_WTILE_F16 + (uint32_t)lane * 16u, dst = base + G::RAW + dst_lane;
+                    const uint32_t base = sbase + (uint32_t)st * G::STAGE, src = base + NB * WB + src_lane, dst = base + G::RAW + dst_lane;
                     uint4 v[4];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) { v[k] = lds128(src + (uint32_t)((k * 8 / TT) * YB + (k * 8 % TT) * 64)); }   // all loads in flight before the first store
+                    for (int k = 0; k < 4; ++k) { v[k] = lds128(src + (uint32_t)((k * TK / TT) * YB + (k * TK % TT) * 64)); }   // all loads in flight before the first store
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        const uint32_t d = dst + (uint32_t)((k * 8 / TT) * 256 * TT + (k * 8 % TT) * 64);
+                        const uint32_t d = dst + (uint32_t)((k * TK / TT) * HS * 128 * TT + (k * TK % TT) * 64);
                         sts64(d, v[k].x, v[k].y);
                         sts64(d + 40u, v[k].z, v[k].w);
                     }
@@ -182,7 +227,7 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             const uint32_t d0 = tmem + (uint32_t)m * 256u;
             int st = 0, k = 0, mine = 0;
             uint32_t par = 0;
-            for (int tile = blockIdx.x; tile < n_tile && left_ns != 0; tile += gridDim.x) {
+            for (int tile = blockIdx.x / S; tile < n_tile && left_ns != 0; tile += gridDim.x / S) {
                 for (int i = 0; i < n_step; ++i, ++k) {
                     if ((k & 1) == m) {
                         mbar_wait_lean(ops_full(st), par, left_ns);
@@ -191,15 +236,15 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                         if (mine > 0 && lane == 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }   // (the step before on this buffer has been read)
                         tc_fence_after();
                         const uint32_t base = sbase + (uint32_t)st * G::STAGE;
-                        const uint64_t a0 = operand_desc(base, 2048u, 128u), b0 = operand_desc(base + G::RAW, 64u * TT, 128u);
+                        const uint64_t a0 = operand_desc(base + (uint32_t)rank * 512u, 2048u, 128u), b0 = operand_desc(base + G::RAW, 64u * TT, 128u);
                         const int n = min(NB, nb - i * NB);
                         if (elect_one()) {
 #pragma unroll
                             for (int j = 0; j < NB; ++j) {
                                 if (j < n) {
 #pragma unroll
-                                    for (int h = 0; h < 2; ++h) {
-                                        mma_f16_ss(d0 + (uint32_t)(j * 8 * TT + h * 4 * TT), a0 + (uint64_t)((j * PF_WTILE_F16 + h * 4096) >> 4), b0 + (uint64_t)((j * 256 * TT + h * 128 * TT) >> 4),
+                                    for (int h = 0; h < HS; ++h) {
+                                        mma_f16_ss(d0 + (uint32_t)((j * HS + h) * 4 * TT), a0 + (uint64_t)((j * WB + h * (PF_HALF + 512)) >> 4), b0 + (uint64_t)(((j * HS + h) * 128 * TT) >> 4),
                                                    idesc_f16(4 * TT), 0u);
                                     }
                                 }
@@ -223,12 +268,12 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
         const int quad = warp & 3, part = warp >> 2;
         const int row = 32 * quad + lane;
         const uint32_t tbase = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(part * TT);
-        const uint32_t dw_addr = sbase + 8192u + 4u * (uint32_t)row, dx_addr = sbase + NB * PF_WTILE_F16 + TT * 64 + (uint32_t)(part * TT);
-        uint64_t acc[PW][8];
+        const uint32_t dw_addr = sbase + (rank == 0 ? (uint32_t)PF_HALF : 0u) + 4u * (uint32_t)row, dx_addr = sbase + NB * WB + TT * 64 + (uint32_t)(part * TT);
+        uint64_t acc[PW][4 * HS];
 #pragma unroll
         for (int u = 0; u < PW; ++u) {
 #pragma unroll
-            for (int n = 0; n < 8; ++n) { acc[u][n] = 0ull; }
+            for (int n = 0; n < 4 * HS; ++n) { acc[u][n] = 0ull; }
         }
         if (lane == 0) { mbar_arrive(d_free(0)); mbar_arrive(d_free(1)); }
         uint32_t stage = 0, par = 0;   // (the ring has an even number of stages: a step's stage and its D buffer are even or odd together)
@@ -240,13 +285,13 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             tc_fence_after();
             uint64_t sc[PC];
 #pragma unroll
-            for (int c = 0; c < G::NC; ++c) {   // chunk c: half c % 2 of PC pairs of block c / 2 / (PW / PC)
-                const int cu = (c >> 1) % (PW / PC), j = (c >> 1) / (PW / PC);
-                const uint32_t col = (uint32_t)(buf * 256 + j * 8 * TT + (c & 1) * 4 * TT + cu * 8 * PC);
+            for (int c = 0; c < G::NC; ++c) {   // chunk c: half c % HS of PC pairs of block c / HS / (PW / PC)
+                const int cu = (c / HS) % (PW / PC), j = (c / HS) / (PW / PC);
+                const uint32_t col = (uint32_t)(buf * 256 + (j * HS + c % HS) * 4 * TT + cu * 8 * PC);
                 uint32_t r[8 * PC];
                 if (PC == 2) { tmem_ld16(tbase + col, r); } else { tmem_ld8(tbase + col, r); }
-                if ((c & 1) == 0) {
-                    const float dw = lds32f(dw_addr + stage + (uint32_t)j * PF_WTILE_F16);
+                if (c % HS == 0) {
+                    const float dw = lds32f(dw_addr + stage + (uint32_t)(j * WB));
                     const uint64_t dw2 = f2_pack(dw, dw);
                     const uint32_t xa = dx_addr + stage + (uint32_t)(j * YB + cu * 8 * PC);
                     if (PC == 2) { uint64_t x0, x1; lds128_2x64(xa, x0, x1); sc[0] = f2_mul(dw2, x0); sc[PC - 1] = f2_mul(dw2, x1); }
@@ -263,7 +308,7 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                     for (int p = 0; p < PC; ++p) {
 #pragma unroll
                         for (int m = 0; m < 4; ++m) {
-                            uint64_t &a = acc[PC * cu + p][4 * (c & 1) + m];
+                            uint64_t &a = acc[PC * cu + p][4 * (c % HS) + m];
                             a = f2_fma(sc[p], f2_pack_bits(r[8 * p + 2 * m], r[8 * p + 2 * m + 1]), a);
                         }
                     }
@@ -275,8 +320,9 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
         using B0 = std::integral_constant<int, 0>;
         using B1 = std::integral_constant<int, 1>;
         const int n_full = nb / NB, rest = nb % NB;
+        uint32_t x_par = 0;      // phase of the hand-over between the CTAs of a cluster
         bool odd = false;        // a tile with an odd number of steps leaves the next one starting on buffer 1
-        for (int tile = blockIdx.x; tile < n_tile; tile += gridDim.x) {
+        for (int tile = blockIdx.x / S; tile < n_tile; tile += gridDim.x / S) {
             int i = 0;
             if (odd && n_full > 0) { step(B1{}, NB); i = 1; }
 #pragma unroll 1
@@ -292,27 +338,51 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             // (Q8_0); either way the tree is (c0 + c4) + (c2 + c6) and (c1 + c5) + (c3 + c7)
             const int64_t orow = (int64_t)(tile / n_tok) * PF_M + row;
             const int     tok0 = (tile % n_tok) * TT + part * (TT / 4);
+            if constexpr (S == 2) {   // the second half's accumulators are those of the same thread of the cluster's other CTA
+                const uint32_t xch = sbase + (uint32_t)(NS * G::STAGE) + 8u * (uint32_t)tid;
+                if (rank == 1) {
+                    if (tile != blockIdx.x / S) { cluster_wait(x_free(warp), x_par ^ 1u, left_ns); }   // (the tile before has been read)
+                    const uint32_t to = cluster_map(xch, 0);
+#pragma unroll
+                    for (int i = 0; i < 4 * PW; ++i) { cluster_store64(to + (uint32_t)(i * PF_GEMM_EPI_WARPS * 32 * 8), acc[i >> 2][i & 3]); }
+                    __syncwarp();
+                    if (lane == 0) { cluster_arrive(cluster_map(x_full(warp), 0)); }
+                } else {
+                    cluster_wait(x_full(warp), x_par, left_ns);
+#pragma unroll
+                    for (int i = 0; i < 4 * PW; ++i) { acc[i >> 2][i & 3] = f2_add(acc[i >> 2][i & 3], lds64u(xch + (uint32_t)(i * PF_GEMM_EPI_WARPS * 32 * 8))); }
+                    __syncwarp();
+                    if (lane == 0) { cluster_arrive(cluster_map(x_free(warp), 1)); }
+                }
+                x_par ^= 1u;
+            }
 #pragma unroll
             for (int u = 0; u < PW; ++u) {
-                const uint64_t r0 = f2_add(acc[u][0], acc[u][4]), r1 = f2_add(acc[u][1], acc[u][5]), r2 = f2_add(acc[u][2], acc[u][6]), r3 = f2_add(acc[u][3], acc[u][7]);
-                float v[2];
-                f2_unpack(f2_add(f2_add(r0, r2), f2_add(r1, r3)), v[0], v[1]);
+                if (S == 1 || rank == 0) {
+                    if constexpr (S == 1) {
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int token = tok0 + 2 * u + e;
-                    if (token < g.T && orow < g.n_rows) {   // (the last row tile may be partly padding)
-                        const int64_t o = (int64_t)token * g.out_stride + orow;
-                        g.out[o] = g.resid != nullptr ? __fadd_rn(v[e], g.resid[o]) : v[e];
+                        for (int m = 0; m < 4; ++m) { acc[u][m] = f2_add(acc[u][m], acc[u][4 + m]); }
+                    }
+                    float v[2];
+                    f2_unpack(f2_add(f2_add(acc[u][0], acc[u][2]), f2_add(acc[u][1], acc[u][3])), v[0], v[1]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int token = tok0 + 2 * u + e;
+                        if (token < g.T && orow < g.n_rows) {   // (the last row tile may be partly padding)
+                            const int64_t o = (int64_t)token * g.out_stride + orow;
+                            g.out[o] = g.resid != nullptr ? __fadd_rn(v[e], g.resid[o]) : v[e];
+                        }
                     }
                 }
 #pragma unroll
-                for (int m = 0; m < 8; ++m) { acc[u][m] = 0ull; }
+                for (int m = 0; m < 4 * HS; ++m) { acc[u][m] = 0ull; }
             }
         }
         if (left_ns == 0 && lane == 0) { pf_report(g.error_flag, 6); }
     }
     tc_fence_before();
     __syncthreads();
+    if (S == 2) { cluster_sync(); }   // (neither CTA's shared memory goes while the other may still reach into it)
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
@@ -434,10 +504,10 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
     }
 }
 
-// upload-time re-layout: raw 18-byte / 34-byte blocks of rows [0, n_rows) -> tiles of 128 rows x 1 block: the f16 A operand (core
-// matrices of 8 rows x 16 bytes: element k of row r at (k / 8) * 2048 + (r / 8) * 128 + (r % 8) * 16 + 2 (k % 8); Q4_0: element k < 16 is
-// the low nibble of byte k minus 8, element 16 + k the high one) followed by the 128 block scales as f32. A warp takes 8 rows x 4
-// neighbouring blocks: its stores are runs of 128 bytes, its loads runs of 72 or 136.
+// upload-time re-layout: raw 18-byte / 34-byte blocks of rows [0, n_rows) -> tiles of 128 rows x 1 block: the first half of the block's
+// values, the 128 scales as f32, the second half. A half is an f16 A operand (core matrices of 8 rows x 16 bytes: element k of row r at
+// (k / 8) * 2048 + (r / 8) * 128 + (r % 8) * 16 + 2 (k % 8)); Q4_0: element k of the first half is the low nibble of byte k minus 8, of
+// the second half the high one. A warp takes 8 rows x 4 neighbouring blocks: its stores are runs of 128 bytes, its loads runs of 72 or 136.
 template <int WT>
 __global__ void prefill_retile_kernel(const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0) {
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -452,7 +522,7 @@ __global__ void prefill_retile_kernel(const uint8_t *raw, int64_t row_stride, in
     const int64_t row = dst_row0 + lrow;
     const int     r = (int)(row % PF_M);
     uint8_t *tile = base + ((row / PF_M) * nb + b) * (int64_t)PF_WTILE_F16;
-    reinterpret_cast<float *>(tile + 8192)[r] = h2f(src[0]);
+    reinterpret_cast<float *>(tile + PF_HALF)[r] = h2f(src[0]);
     auto byte_of = [&](int i) { return (i & 1) ? src[1 + (i >> 1)] >> 8 : src[1 + (i >> 1)] & 0xff; };
     auto value = [&](int k) {
         if (WT == 2) { const int byte = byte_of(k & 15); return (k < 16 ? (byte & 15) : (byte >> 4)) - 8; }
@@ -465,7 +535,7 @@ __global__ void prefill_retile_kernel(const uint8_t *raw, int64_t row_stride, in
         for (int e = 0; e < 4; ++e) {
             v[e] = (uint32_t)__half_as_ushort(__int2half_rn(value(8 * c + 2 * e))) | ((uint32_t)__half_as_ushort(__int2half_rn(value(8 * c + 2 * e + 1))) << 16);
         }
-        *reinterpret_cast<uint4 *>(tile + c * 2048 + (r >> 3) * 128 + (r & 7) * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<uint4 *>(tile + c * 2048 + (c >> 1) * 512 + (r >> 3) * 128 + (r & 7) * 16) = make_uint4(v[0], v[1], v[2], v[3]);
     }
 }
 
@@ -508,13 +578,23 @@ __global__ void prefill_silu_mul_kernel(const float *upgate, int T, int F, const
     act[i] = __fmul_rn(up, silu_table[f2h(gate)]);
 }
 
-template <int TT>
+template <int TT, int S>
 cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
-    const size_t smem = PfGeom<TT>::SMEM;
-    cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(prefill_gemm_kernel<TT>), smem);
+    const void *kernel = reinterpret_cast<const void *>(prefill_gemm_kernel<TT, S>);
+    const size_t smem = PfGeom<TT, S>::SMEM;
+    cudaError_t err = allow_dynamic_smem(kernel, smem);
     if (err != cudaSuccess) { return err; }
     const int64_t tiles = (int64_t)((g.T + TT - 1) / TT) * ((g.n_rows + PF_M - 1) / PF_M);
-    return launch_maybe_pdl(prefill_gemm_kernel<TT>, dim3((unsigned)std::min<int64_t>(tiles, device_sms())), PF_GEMM_THREADS, smem, stream, pdl, g);
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)(S * std::min<int64_t>(tiles, device_sms() / S))); lc.blockDim = dim3(PF_GEMM_THREADS); lc.dynamicSmemBytes = smem; lc.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = S; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    lc.attrs = attr; lc.numAttrs = S > 1 ? 2 : 1;
+    void *args[] = {const_cast<PrefillGemm *>(&g)};
+    return cudaLaunchKernelExC(&lc, kernel, args);
 }
 
 }  // namespace
@@ -530,17 +610,33 @@ int device_sms() {
     return sms[dev];
 }
 
-// Tiles of 16 or of 8 tokens. A tile takes nb TT / 32 steps and the CTAs walk their tiles in rounds, so the width whose busiest CTA has
-// fewer steps to do wins; a step of the narrow tiles costs 1.4 of one of the wide ones (eight MMAs and twice the weight bytes; measured
-// 1.2 to 1.5 on 4096 to 27648 rows). 4096 rows x 32 tokens: 8 wide (20 us against 30); 27648 rows x 32 tokens: 16 wide (91 against 142).
-int prefill_tile_tokens(int type, int64_t n_rows, int T) {
-    const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, sms = device_sms();
-    auto rounds = [&](int tt) { return (row_tiles * ((T + tt - 1) / tt) + sms - 1) / sms; };
+// The form of the Q4_0 / Q8_0 kernel for a matrix and a number of tokens: tiles of 16 or of 8 tokens, by one CTA each or by a cluster of
+// two. The clusters walk the tiles in rounds, and the form whose rounds take least is the one. Fitted to 10 matrices from 1024 x 1024 to
+// 27648 x 5120 with 2 to 448 tokens (at each of 120 sizes within 3 % of the fastest form): a round costs a time for each block of the
+// row (less for narrow tiles, whose weights bound them, and about half for two CTAs), a launch what fills its pipelines and joins the
+// halves. us, one CTA / two: 4096 x 4096 x 8 tokens 21.3 / 14.8, 4096 x 11008 x 21 52 / 36, 22016 x 4096 x 16 49.6 / 44.5; and 12288 x 4096 x 8
+// tokens, whose 96 tiles need most of the chip, 24.2 / 28.4, 22016 x 4096 x 448 643 / 827.
+struct PfForm { int tok, split; double block_ns, launch_ns; };
+static PfForm best_form(int64_t n_rows, int nb, int T, int tok) {   // tok 0: of either width
+    static constexpr PfForm FORMS[4] = {{16, 1, 153, 3500}, {8, 1, 135, 2500}, {16, 2, 97, 4800}, {8, 2, 72, 5000}};
+    PfForm best = {};
+    double best_ns = 0.0;
+    for (const PfForm &f : FORMS) {
+        if (tok != 0 && tok != f.tok) { continue; }
+        const int64_t tiles = (n_rows + PF_M - 1) / PF_M * ((T + f.tok - 1) / f.tok), walks = std::max(1, device_sms() / f.split);
+        const double ns = (double)((tiles + walks - 1) / walks) * nb * f.block_ns + f.launch_ns;
+        if (best.tok == 0 || ns < best_ns) { best = f; best_ns = ns; }
+    }
+    return best;
+}
+int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T) {
     if (type == 12 || type == 14) {   // K-quants: a tile of 16, 32, 64 tokens costs 1 : 1.35 : 2.3 (measured: the narrow ones are mostly weights)
+        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, sms = device_sms();
+        auto rounds = [&](int tt) { return (row_tiles * ((T + tt - 1) / tt) + sms - 1) / sms; };
         const double c16 = (double)rounds(16), c32 = 1.35 * (double)rounds(32), c64 = 2.3 * (double)rounds(64);
         return c16 <= c32 && c16 <= c64 ? 16 : c32 <= c64 ? 32 : 64;
     }
-    return 8.0 * 1.4 * (double)rounds(8) < 16.0 * (double)rounds(16) ? 8 : 16;
+    return best_form(n_rows, nb, T, 0).tok;
 }
 
 size_t prefill_weight_bytes(int type, int64_t n_rows, int nb) {
@@ -578,11 +674,10 @@ cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K,
 cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     if (g.type == 12 || g.type == 14) { return launch_prefill_gemm_kq(g, stream, pdl); }
     if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
-    switch (g.tile_tok) {
-    case 16: return launch_gemm_t<16>(g, stream, pdl);
-    case 8:  return launch_gemm_t<8>(g, stream, pdl);
-    default: return cudaErrorInvalidValue;
-    }
+    if (g.tile_tok != 16 && g.tile_tok != 8) { return cudaErrorInvalidValue; }
+    const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok).split == 2;
+    return g.tile_tok == 16 ? (pair ? launch_gemm_t<16, 2>(g, stream, pdl) : launch_gemm_t<16, 1>(g, stream, pdl))
+                            : (pair ? launch_gemm_t<8, 2>(g, stream, pdl) : launch_gemm_t<8, 1>(g, stream, pdl));
 }
 
 cudaError_t launch_prefill_qkv_post(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,

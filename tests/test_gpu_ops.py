@@ -161,6 +161,20 @@ def test_prefill_matmul_walks_tiles_of_both_widths(be, oracle, qt, n, k, t):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
+@pytest.mark.parametrize("n,k,t", [(19204, 1600, 7), (19204, 2880, 15), (132, 3104, 9), (516, 2976, 32)])
+def test_prefill_matmul_shared_by_two_ctas(be, oracle, qt, n, k, t):
+    """The form whose tiles are shared by a cluster of two CTAs, in narrow and in wide token tiles: three rounds of tiles (the hand-over's
+    buffer is used again), odd numbers of steps that end inside a step, a last row tile of four rows, ragged and full token tiles."""
+    rng = np.random.default_rng(n + k + t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    x[rng.integers(0, t, 8), rng.integers(0, k, 8)] *= 40.0
+    got = be.prefill_matmul(qt, w, n, k, x)
+    want = oracle.matmul(qt, w, k, n, x)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
 @pytest.mark.parametrize("n,k,t", [(19000, 256, 16), (2564, 768, 250), (1284, 512, 1000), (516, 2304, 31), (132, 256, 48), (640, 4096, 9)])
 def test_prefill_matmul_k_quants_walk_tiles_of_all_widths(be, oracle, qt, n, k, t):
