@@ -20,6 +20,7 @@
 // cp.async.bulk (weights in a 128-row x 1-block tile layout made at upload, activations as compact blocks); an expander warp writes the
 // activations into the canonical K-major no-swizzle operand layout (core matrices of 8 rows x 16 bytes). Every wait is bounded.
 #include "spyb_tc.cuh"
+#include "spyb_mv_common.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -30,7 +31,7 @@ namespace {
 
 constexpr int PF_HALF = 4096;   // bytes of half a block's weights: 16 f16 values of 128 rows
 constexpr int PF_QUANT_THREADS = 512;
-constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF_QUANT_THREADS);   // groups of eight values per thread
+constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF_QUANT_THREADS);   // groups of eight values per thread of the widest row
 
 // ---------------------------------------------------------------------------------------------
 // the GEMM: persistent CTAs (one per SM, all 512 tensor-memory columns), each walking tiles of 128 rows x TT tokens along K in
@@ -73,7 +74,7 @@ template <int TT, int S> struct PfGeom {
     static constexpr size_t SMEM = (size_t)BARS + 8 * N_BAR + 16;
 };
 
-template <int TT, int S>
+template <int TT, int S, bool MANY>
 __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(PrefillGemm g) {
     using G = PfGeom<TT, S>;
     constexpr int NB = G::NB, NS = G::NS, PW = G::PW, PC = G::PC, YB = G::YB, HS = G::HS, WB = G::WB;
@@ -130,14 +131,10 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             bool ok = true;
             // the weights of the first tile's first steps, then (the previous kernel is done) their activations with all that follows
             const int early = blockIdx.x / S < n_tile ? min(NS, n_step) : 0;
-            // One copy a step where the weights' way through HBM is the bound (32000 x 4096 x 16 tokens 49.7 us, in pieces 50.1); with more
-            // tokens, when the epilogue is and the weights come out of L2, halves of blocks (22016 x 4096 x 448 tokens 659 us in one copy,
-            // 649 in blocks, 643 in halves, 646 in quarters: short bursts into shared memory are in the epilogue's way for less long)
-            const bool pieces = n_tok > 4;
             // n blocks of weights at `w` into stage st
             auto copy_weights = [&](int st, const uint8_t *w, int n) {
                 const uint32_t dst = sbase + (uint32_t)st * G::STAGE;
-                if (S == 1 && (TT == 8 || !pieces)) { bulk_copy_g2s(dst, w, (uint32_t)(n * WB), raw_full(st)); }
+                if (S == 1 && !MANY) { bulk_copy_g2s(dst, w, (uint32_t)(n * WB), raw_full(st)); }
                 else if (S == 1) {
 #pragma unroll
                     for (int j = 0; j < 2 * NB; ++j) {
@@ -392,27 +389,41 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
 // ---------------------------------------------------------------------------------------------
 // activations of T tokens -> compact Q8_0 blocks grouped by (tile of tile_tok tokens, block). One CTA per token; RMSNorm and the
 // quantizer as in the mat-vec prologue (NormRMS, backend/host/operator/non-linear.cpp:194-223: groups of four squares formed in
-// parallel, the running sum on one thread; Quantizator<FP32,Q8_0>, simd/vec_convert.h:178-261).
+// parallel, the running sum on four warps; Quantizator<FP32,Q8_0>, simd/vec_convert.h:178-261). Bound: that sum's chain; the
+// norm's weights are read before the wait for the previous kernel. PG groups of eight values a thread: one fits most models, and two CTAs an
+// SM. us with the norm, one thread's sum / this: 8 tokens x 5120 9.8 / 7.4, 32 x 5120 9.6 / 7.0, 448 x 4096 26.5 / 10.7.
 // KQ false (Q4_0 / Q8_0 weights): [token][32 values as f16], the scales. KQ true: the f16 B operand itself (16 bytes of eight values of a token at
 // (value / 8) * 16 TOKT + 16 token), the scales, the blocks' integer sums as floats.
-template <bool NORM, bool KQ>
-__global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const float *x, int64_t x_stride, int K, const float *norm_w, float eps, uint8_t *yq,
+template <bool NORM, bool KQ, int PG>
+__global__ void __launch_bounds__(PF_QUANT_THREADS, PG <= 2 ? 2 : 1) prefill_quant_kernel(const float *x, int64_t x_stride, int K, const float *norm_w, float eps, uint8_t *yq,
                                                                          int TOKT, int part_len, int64_t part_stride, uint8_t *tap) {
     const int SCALES = TOKT * 64;                         // offset of the scales inside a block's record
     const int YQB = SCALES + TOKT * (KQ ? 8 : 4);
     extern __shared__ __align__(16) float v3[];
     __shared__ float scale_s;
     const int tid = threadIdx.x, token = blockIdx.x;
-    pdl_launch_dependents();
-    pdl_wait();
     const int n4 = K >> 2, n8 = K >> 3, nb = K >> 5;
     const int npass = (n8 + PF_QUANT_THREADS - 1) / PF_QUANT_THREADS;
+    pdl_launch_dependents();
+    float wv[NORM ? PG : 1][8];
+    if (NORM) {   // the norm's weights are constants: they are there before the previous kernel is done
+#pragma unroll
+        for (int k = 0; k < PG; ++k) {
+            const int gi = tid + k * PF_QUANT_THREADS;
+            if (k < npass && gi < n8) { load8_cg(norm_w + 8 * gi, wv[NORM ? k : 0]); }
+            else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { wv[NORM ? k : 0][i] = 0.f; }
+            }
+        }
+    }
+    pdl_wait();
     // a row may lie in parts (the slices the ranks of a tensor-parallel group gathered): elements [i part_len, (i + 1) part_len)
     // of token t at x + i part_stride + t x_stride; one part = the plain row (parts are multiples of four values)
     const float *xrow = x + (int64_t)token * x_stride;
-    float xv[PF_QUANT_GROUPS][8];
+    float xv[PG][8];
 #pragma unroll
-    for (int k = 0; k < PF_QUANT_GROUPS; ++k) {
+    for (int k = 0; k < PG; ++k) {
         const int gi = tid + k * PF_QUANT_THREADS;
         if (k < npass && gi < n8) {
             if (part_len == K) { load8_cg(xrow + 8 * gi, xv[k]); }
@@ -430,43 +441,31 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
         }
     }
     if (NORM) {
-        float wv[PF_QUANT_GROUPS][8];
 #pragma unroll
-        for (int k = 0; k < PF_QUANT_GROUPS; ++k) {
+        for (int k = 0; k < PG; ++k) {
             const int gi = tid + k * PF_QUANT_THREADS;
-            if (k < npass && gi < n8) {
-                reinterpret_cast<float2 *>(v3)[gi] = squares8(xv[k]);
-                load8_cg(norm_w + 8 * gi, wv[k]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) { wv[k][i] = 0.f; }
-            }
+            if (k < npass && gi < n8) { reinterpret_cast<float2 *>(v3)[gi] = squares8(xv[k]); }
         }
         __syncthreads();
+        __shared__ __align__(16) float rs[rs_scratch_words(4)];
+        float sum = 0.f;
+        if (tid < RS_THREADS) { sum = running_sum_wide(smem_u32(v3), n4, smem_u32(rs), rs_scratch_words(4), tid, 1); }
         if (tid == 0) {
-            float sum = 0.f;
-            const float4 *g4 = reinterpret_cast<const float4 *>(v3);
-            int gi = 0;
-            for (; gi + 4 <= n4; gi += 4) {
-                const float4 q = g4[gi >> 2];
-                sum = __fadd_rn(sum, q.x); sum = __fadd_rn(sum, q.y); sum = __fadd_rn(sum, q.z); sum = __fadd_rn(sum, q.w);
-            }
-            for (; gi < n4; ++gi) { sum = __fadd_rn(sum, v3[gi]); }
             scale_s = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)K), eps)));
         }
         __syncthreads();
         const float scale = scale_s;
 #pragma unroll
-        for (int k = 0; k < PF_QUANT_GROUPS; ++k) {
+        for (int k = 0; k < PG; ++k) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { xv[k][i] = __fmul_rn(__fmul_rn(xv[k][i], scale), wv[k][i]); }
+            for (int i = 0; i < 8; ++i) { xv[k][i] = __fmul_rn(__fmul_rn(xv[k][i], scale), wv[NORM ? k : 0][i]); }
         }
     }
     uint8_t *tile = yq + ((int64_t)(token / TOKT) * nb) * YQB;
     const int tt = token % TOKT;
-    uint2 qv[PF_QUANT_GROUPS];
+    uint2 qv[PG];
     int kd;
-    const float d = quantize_q8_groups<PF_QUANT_GROUPS>(xv, npass, qv, kd);   // (npass is uniform over the CTA: the quantizer's shuffles see full warps)
+    const float d = quantize_q8_groups<PG>(xv, npass, qv, kd);   // (npass is uniform over the CTA: the quantizer's shuffles see full warps)
     if (kd >= 0 && tid + kd * PF_QUANT_THREADS < n8) {
         const int b = (tid + kd * PF_QUANT_THREADS) >> 2;
         const uint16_t dh = f2h(d);
@@ -474,7 +473,7 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS) prefill_quant_kernel(const f
         if (tap != nullptr && token == 0) { *reinterpret_cast<uint16_t *>(tap + (int64_t)b * 34) = dh; }
     }
 #pragma unroll
-    for (int k = 0; k < PF_QUANT_GROUPS; ++k) {
+    for (int k = 0; k < PG; ++k) {
         if (k < npass) {
             const int gi = tid + k * PF_QUANT_THREADS;
             const uint2 q = qv[k];
@@ -578,9 +577,9 @@ __global__ void prefill_silu_mul_kernel(const float *upgate, int T, int F, const
     act[i] = __fmul_rn(up, silu_table[f2h(gate)]);
 }
 
-template <int TT, int S>
+template <int TT, int S, bool MANY = false>
 cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
-    const void *kernel = reinterpret_cast<const void *>(prefill_gemm_kernel<TT, S>);
+    const void *kernel = reinterpret_cast<const void *>(prefill_gemm_kernel<TT, S, MANY>);
     const size_t smem = PfGeom<TT, S>::SMEM;
     cudaError_t err = allow_dynamic_smem(kernel, smem);
     if (err != cudaSuccess) { return err; }
@@ -667,7 +666,12 @@ cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K,
     if (T < 1 || tile_tok < 1 || K < 32 || (K & 31) || K > PF_MAX_K || (x_stride & 3) || ((uintptr_t)x & 15)) { return cudaErrorInvalidValue; }
     const size_t smem = norm_w != nullptr ? (size_t)K : 0;   // K / 4 floats
     const bool kq = weight_type == 12 || weight_type == 14;
-    auto *kernel = kq ? (norm_w ? prefill_quant_kernel<true, true> : prefill_quant_kernel<false, true>) : (norm_w ? prefill_quant_kernel<true, false> : prefill_quant_kernel<false, false>);
+    auto of_groups = [&](auto pg) {
+        constexpr int PG = decltype(pg)::value;
+        return kq ? (norm_w ? prefill_quant_kernel<true, true, PG> : prefill_quant_kernel<false, true, PG>) : (norm_w ? prefill_quant_kernel<true, false, PG> : prefill_quant_kernel<false, false, PG>);
+    };
+    const int groups = (K / 8 + PF_QUANT_THREADS - 1) / PF_QUANT_THREADS;
+    auto *kernel = groups == 1 ? of_groups(std::integral_constant<int, 1>{}) : groups == 2 ? of_groups(std::integral_constant<int, 2>{}) : of_groups(std::integral_constant<int, PF_QUANT_GROUPS>{});
     return launch_maybe_pdl(kernel, dim3((unsigned)T), PF_QUANT_THREADS, smem, stream, pdl, x, x_stride, K, norm_w, eps, yq, tile_tok, part_len, part_stride, tap);
 }
 
@@ -676,8 +680,12 @@ cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool 
     if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
     if (g.tile_tok != 16 && g.tile_tok != 8) { return cudaErrorInvalidValue; }
     const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok).split == 2;
-    return g.tile_tok == 16 ? (pair ? launch_gemm_t<16, 2>(g, stream, pdl) : launch_gemm_t<16, 1>(g, stream, pdl))
-                            : (pair ? launch_gemm_t<8, 2>(g, stream, pdl) : launch_gemm_t<8, 1>(g, stream, pdl));
+    // Many tokens (MANY): the epilogue is the bound and the weights come out of L2; copies of half a block are in its way for less long.
+    // 22016 x 4096 x 448 tokens 659 us with one copy a step, 649 by blocks, 642 by halves, 646 by quarters. Where the weights' way
+    // through HBM is the bound one copy is better: 4096 x 11008 x 64 tokens 55.8 us, by halves 56.2.
+    const bool many = g.T > 64;
+    if (g.tile_tok == 8) { return pair ? launch_gemm_t<8, 2>(g, stream, pdl) : launch_gemm_t<8, 1>(g, stream, pdl); }
+    return pair ? launch_gemm_t<16, 2>(g, stream, pdl) : many ? launch_gemm_t<16, 1, true>(g, stream, pdl) : launch_gemm_t<16, 1>(g, stream, pdl);
 }
 
 cudaError_t launch_prefill_qkv_post(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,

@@ -175,6 +175,22 @@ def test_prefill_matmul_shared_by_two_ctas(be, oracle, qt, n, k, t):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("qt,k", [(quants.Q4_0, 2272), (quants.Q4_0, 4128), (quants.Q8_0, 8192), (quants.Q4_0, 8224), (quants.Q4_K, 4352), (quants.Q4_K, 9216)])
+def test_prefill_quantizer_of_normed_rows(be, oracle, qt, k):
+    """RMSNorm in front of the quantizer at the edges of its forms: one, two and four groups a thread, rows below and above what the four
+    warps' running sum takes; a row of zeros among the others (the sum then falls back to the plain chain)."""
+    rng = np.random.default_rng(k)
+    n, t = 8, 3
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    x[1] = 0.0
+    nw = (1.0 + 0.1 * rng.standard_normal(k)).astype(np.float32)
+    got = be.prefill_matmul(qt, w, n, k, x, nw, 1e-5)
+    xin = oracle.mul_rows(oracle.rmsnorm(x, 1e-5), nw)
+    want = oracle.matmul(qt, w, k, n, xin)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
 @pytest.mark.parametrize("n,k,t", [(19000, 256, 16), (2564, 768, 250), (1284, 512, 1000), (516, 2304, 31), (132, 256, 48), (640, 4096, 9)])
 def test_prefill_matmul_k_quants_walk_tiles_of_all_widths(be, oracle, qt, n, k, t):
