@@ -55,7 +55,7 @@ constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF
 // CTAs then shares a tile by the halves of its blocks: the eight accumulators of an output are independent chains until the row's end, four
 // of them read the first 16 values of every block and four the others, so each CTA streams and multiplies one half of the weights (the
 // scales lie between the halves) for four chains of twice the blocks per step, and at the end of a tile the second CTA's epilogue warps leave their sums in
-// the first one's shared memory, where they are added in the tree's order. 4096 x 11008 x 8 tokens 52 -> 31.5 us, 4096 x 4096 x 8 21 -> 15.
+// the first one's shared memory, where they are added in the tree's order. 4096 x 11008 x 8 tokens 52 -> 32.5 us, 4096 x 4096 x 8 20.8 -> 15.1.
 // Where the tiles fill the chip it costs more (a scale product for every four FMAs, the scales twice): prefill_tile_tokens has the line.
 template <int TT, int S> struct PfGeom {
     static constexpr int NB     = 32 * S / TT;                            // blocks per step
@@ -611,9 +611,9 @@ int device_sms() {
 
 // The form of the Q4_0 / Q8_0 kernel for a matrix and a number of tokens: tiles of 16 or of 8 tokens, by one CTA each or by a cluster of
 // two. The clusters walk the tiles in rounds, and the form whose rounds take least is the one. Fitted to 10 matrices from 1024 x 1024 to
-// 27648 x 5120 with 2 to 448 tokens (at each of 120 sizes within 3 % of the fastest form): a round costs a time for each block of the
+// 27648 x 5120 with 2 to 448 tokens (at 119 of 120 sizes within 3 % of the fastest form): a round costs a time for each block of the
 // row (less for narrow tiles, whose weights bound them, and about half for two CTAs), a launch what fills its pipelines and joins the
-// halves. us, one CTA / two: 4096 x 4096 x 8 tokens 21.3 / 14.8, 4096 x 11008 x 21 52 / 36, 22016 x 4096 x 16 49.6 / 44.5; and 12288 x 4096 x 8
+// halves. us, one CTA / two: 4096 x 4096 x 8 tokens 20.8 / 15.1, 4096 x 11008 x 21 51 / 36.5, 22016 x 4096 x 16 49.6 / 44.5; and 12288 x 4096 x 8
 // tokens, whose 96 tiles need most of the chip, 24.2 / 28.4, 22016 x 4096 x 448 643 / 827.
 struct PfForm { int tok, split; double block_ns, launch_ns; };
 static PfForm best_form(int64_t n_rows, int nb, int T, int tok) {   // tok 0: of either width
