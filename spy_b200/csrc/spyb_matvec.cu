@@ -116,7 +116,7 @@ cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
 //   order for random-access ranges is: groups of four combined as (x0^2 + x1^2) + (x2^2 + x3^2) (the first
 //   product of each pair plain, the second fused into an FMA, as the CPU build evaluates it) and added to
 //   the running sum one group after the other; y = x * (1 / sqrt(sum/n + eps)). The groups are formed in
-//   parallel, the running sum is one thread's chain. Mul (basic.cpp:15-50): y * norm_weight.
+//   parallel, the running sum is a chain in this order (or its exact form on four warps). Mul (basic.cpp:15-50): y * norm_weight.
 // Single column, K <= 12288: every thread keeps its (at most PG) groups of eight x in registers from the one
 // global read through the sum of squares to the quantizer; same arithmetic as the general prologue below.
 // (Eight values a thread: a 256-bit load each, half the shuffles and lane bookkeeping of groups of four. Behind the last read of 11008 values:

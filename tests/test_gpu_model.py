@@ -482,6 +482,23 @@ def test_long_context_attention_path_in_the_model(env, oracle, tmp_models, monke
     m.close(); b.close()
 
 
+@pytest.mark.parametrize("n,n_ctx", [(129, 508), (300, 512), (511, 516), (530, 1284)])
+def test_prompt_attention_in_large_groups(n, n_ctx, oracle, tmp_models):
+    """Prompts of more than 128 tokens take their attention in groups of up to 512: ragged last tiles of tokens and positions, contexts that
+    are multiples of 8 or only of 4 (V^T in pieces of 8 bytes), and a second pass behind a full one."""
+    cfg = gguf_io.LlamaConfig(n_layer=2, d_model=256, n_head=2, n_ff=512, n_vocab=512, weight_std=0.05)
+    path = str(tmp_models / "groups.gguf")
+    if not os.path.exists(path):
+        gguf_io.make_llama_gguf(path, cfg, seed=49)
+    prompt = np.random.default_rng(n).integers(3, cfg.n_vocab, size=n)
+    want_ids, want_logits = oracle.OracleLlama(path, n_ctx=n_ctx).generate(prompt, 3)
+    b = B.B200Backend(0)
+    m = B.LlamaModel(b, path, n_ctx=n_ctx)
+    ids, logits = m.generate(prompt, 3)
+    assert np.array_equal(ids, want_ids) and logits_ok(logits, want_logits)
+    m.close(); b.close()
+
+
 @pytest.mark.parametrize("n_ctx", [264, 512, 508, 1280])
 def test_steps_on_both_sides_of_the_attention_switch(n_ctx, oracle, tmp_models):
     """From position 240 on a single-token step takes the cluster kernel, where the context's length allows it (508: not a multiple of 8), in
