@@ -617,8 +617,33 @@ spyb_model::StepGraph *find_graph(spyb_model *m, int kind) {
     }
     return nullptr;
 }
-spyb_model::StepGraph *keep_graph(spyb_model *m, int kind, cudaGraphExec_t exec, int64_t launches) {   // (the stream is idle: called behind a capture)
+// the same, captured now where there is none: enqueue(&launches) issues the step
+template <class Enqueue>
+spyb_model::StepGraph *captured_step(spyb_model *m, int kind, Enqueue enqueue) {
+    if (auto *have = find_graph(m, kind)) { return have; }
+    spyb_backend *be = m->be;
+    cudaGraphExec_t exec = nullptr;
+    int64_t launches = 0;
+    if (m->nccl_comm != nullptr) { cudaStreamSynchronize(be->stream); }   // (no collectives in flight beside captured ones)
+    for (bool again = true; again;) {
+        again = false;
+        cudaGraph_t graph = nullptr;
+        cudaError_t err = cudaStreamBeginCapture(be->stream, cudaStreamCaptureModeThreadLocal);
+        if (err != cudaSuccess) { be->set_error("CUDA graph capture failed: %s", cudaGetErrorString(err)); return nullptr; }
+        launches = 0;
+        const spyb_status st = enqueue(&launches);
+        err = cudaStreamEndCapture(be->stream, &graph);
+        if (st == SPYB_SUCCESS && err == cudaSuccess) { err = cudaGraphInstantiate(&exec, graph, 0); }
+        if (graph) { cudaGraphDestroy(graph); }
+        if (st == SPYB_SUCCESS && err == cudaSuccess) { break; }
+        exec = nullptr;
+        cudaGetLastError();
+        if (m->step_ok && m->step_coop) { m->step_coop = false; again = true; }   // a cooperative launch the capture refuses: plain launch of the same grid
+        else if (st == SPYB_SUCCESS) { be->set_error("CUDA graph capture failed: %s", cudaGetErrorString(err)); }
+    }
+    if (exec == nullptr) { return nullptr; }
     if (m->graphs.size() >= MAX_STEP_GRAPHS) {
+        cudaStreamSynchronize(be->stream);   // (the one that goes may be running)
         auto oldest = std::min_element(m->graphs.begin(), m->graphs.end(), [](const auto &a, const auto &b) { return a.used < b.used; });
         cudaGraphExecDestroy(oldest->exec);
         m->graphs.erase(oldest);
@@ -1068,35 +1093,16 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
         m->h_pos_pinned[0] = n_past; m->h_pos_pinned[1] = n_past + 1; m->h_pos_pinned[2] = ++m->epoch;
         m->h_tok_pinned[0] = tokens[0];
         m->att_form = step_form(m, n_past);
-        spyb_model::StepGraph *step = find_graph(m, GRAPH_EVAL);
-        for (int attempt = 0; step == nullptr; ++attempt) {
-            cudaGraph_t graph = nullptr;
-            cudaGraphExec_t exec = nullptr;
-            SPYB_CUDA(be, cudaStreamBeginCapture(be->stream, cudaStreamCaptureModeThreadLocal));
-            spyb_status st = SPYB_SUCCESS;
-            cudaError_t ce = cudaMemcpyAsync(m->d_pos, m->h_pos_pinned, 12, cudaMemcpyHostToDevice, be->stream);
-            if (ce == cudaSuccess) { ce = cudaMemcpyAsync(m->d_tokens_in, m->h_tok_pinned, 4, cudaMemcpyHostToDevice, be->stream); }
-            if (ce == cudaSuccess) { ce = launch_embed(m->d_tokens_in, 1, m->embd, m->embd_type, m->info.d_model, m->x, be->stream); }
-            int64_t n = 1;
-            if (ce == cudaSuccess && m->step_ok) { st = run_step(m, true, &n); }
-            else {
-                if (ce == cudaSuccess) { st = run_layers(m, 1, true, &n); }
-                if (ce == cudaSuccess && st == SPYB_SUCCESS) { st = run_head(m, 0, &n); }
-            }
-            if (ce == cudaSuccess && st == SPYB_SUCCESS) { ce = cudaMemcpyAsync(m->h_logits_pinned, m->logits, (size_t)m->info.n_vocab * 4, cudaMemcpyDeviceToHost, be->stream); }
-            const cudaError_t ee = cudaStreamEndCapture(be->stream, &graph);
-            cudaError_t ie = cudaSuccess;
-            if (ce == cudaSuccess && st == SPYB_SUCCESS && ee == cudaSuccess) {
-                ie = cudaGraphInstantiate(&exec, graph, 0);
-                if (ie != cudaSuccess) { exec = nullptr; }
-            }
-            if (graph) { cudaGraphDestroy(graph); }
-            if (exec != nullptr) { step = keep_graph(m, GRAPH_EVAL, exec, n); break; }
-            cudaGetLastError();
-            if (attempt == 0 && m->step_ok && m->step_coop) { m->step_coop = false; continue; }   // a cooperative launch the capture refuses: plain launch of the same grid
-            if (st == SPYB_SUCCESS) { be->set_error("CUDA graph capture of the single-token step failed: %s", cudaGetErrorString(ce != cudaSuccess ? ce : ee != cudaSuccess ? ee : ie)); }
-            return SPYB_FAIL;
-        }
+        const spyb_model::StepGraph *step = captured_step(m, GRAPH_EVAL, [&](int64_t *n) {
+            SPYB_CUDA(be, cudaMemcpyAsync(m->d_pos, m->h_pos_pinned, 12, cudaMemcpyHostToDevice, be->stream));
+            SPYB_CUDA(be, cudaMemcpyAsync(m->d_tokens_in, m->h_tok_pinned, 4, cudaMemcpyHostToDevice, be->stream));
+            SPYB_CUDA(be, launch_embed(m->d_tokens_in, 1, m->embd, m->embd_type, m->info.d_model, m->x, be->stream)); ++*n;
+            if (m->step_ok) { if (run_step(m, true, n) != SPYB_SUCCESS) { return SPYB_FAIL; } }
+            else if (run_layers(m, 1, true, n) != SPYB_SUCCESS || run_head(m, 0, n) != SPYB_SUCCESS) { return SPYB_FAIL; }
+            SPYB_CUDA(be, cudaMemcpyAsync(m->h_logits_pinned, m->logits, (size_t)m->info.n_vocab * 4, cudaMemcpyDeviceToHost, be->stream));
+            return SPYB_SUCCESS;
+        });
+        if (step == nullptr) { return SPYB_FAIL; }
         SPYB_CUDA(be, cudaEventRecord(m->ev0, be->stream));
         SPYB_CUDA(be, cudaGraphLaunch(step->exec, be->stream));
         SPYB_CUDA(be, cudaEventRecord(m->ev1, be->stream));
@@ -1216,41 +1222,19 @@ spyb_status spyb_model_decode(spyb_model *m, int32_t first_token, int32_t n_past
     SPYB_CUDA(be, launch_embed(m->d_tokens_in, 1, m->embd, m->embd_type, m->info.d_model, m->x, be->stream));
 
     const bool use_graph = be->config.use_graph != 0 && (m->info.tp_size == 1 || std::getenv("SPYB_TP_NO_GRAPH") == nullptr);   // the all-reduces of the prompt pass have warmed NCCL up before the capture
-    // one decode step captured once per sequence and form of the attention; positions and the token live in device memory, so the same
-    // graph replays for every later step
-    auto captured_step = [&]() -> spyb_model::StepGraph * {
-        if (auto *have = find_graph(m, GRAPH_DECODE)) { return have; }
-        for (int attempt = 0;; ++attempt) {
-            cudaGraph_t graph = nullptr;
-            cudaGraphExec_t exec = nullptr;
-            cudaError_t ce = cudaStreamSynchronize(be->stream), ie = cudaSuccess;
-            if (ce == cudaSuccess) { ce = cudaStreamBeginCapture(be->stream, cudaStreamCaptureModeThreadLocal); }
-            if (ce != cudaSuccess) { be->set_error("CUDA graph capture failed: %s", cudaGetErrorString(ce)); return nullptr; }
-            int64_t n = 0;
-            const spyb_status st = run_decode_step(m, &n);
-            ce = cudaStreamEndCapture(be->stream, &graph);
-            if (st == SPYB_SUCCESS && ce == cudaSuccess) {
-                ie = cudaGraphInstantiate(&exec, graph, 0);
-                if (ie != cudaSuccess) { exec = nullptr; }
-            }
-            if (graph) { cudaGraphDestroy(graph); }
-            if (exec != nullptr) { return keep_graph(m, GRAPH_DECODE, exec, n); }
-            cudaGetLastError();
-            if (attempt == 0 && m->step_ok && m->step_coop) { m->step_coop = false; continue; }   // a cooperative launch the capture refuses: plain launch of the same grid
-            if (st == SPYB_SUCCESS) { be->set_error("CUDA graph capture failed: %s", cudaGetErrorString(ce != cudaSuccess ? ce : ie)); }
-            return nullptr;
-        }
+    // one decode step captured once per sequence and form of the attention, when the first step of that form comes (a capture leaves the steps in
+    // front of it running); positions and the token live in device memory, so the same graph replays for every later step
+    auto step_at = [&](int pos) {
+        m->att_form = step_form(m, pos);
+        return use_graph ? captured_step(m, GRAPH_DECODE, [&](int64_t *n) { return run_decode_step(m, n); }) : nullptr;
     };
-    // (steps that will be needed are captured before the first one runs: a capture waits for the stream)
-    m->att_form = step_form(m, n_past + n_steps - 1);
-    if (use_graph && captured_step() == nullptr) { return SPYB_FAIL; }
-    m->att_form = step_form(m, n_past);
-    if (use_graph && captured_step() == nullptr) { return SPYB_FAIL; }
+    if (step_at(n_past) == nullptr && use_graph) { return SPYB_FAIL; }
     int64_t per_step = m->step_ok ? 2 : (int64_t)m->layers.size() * 5 + 2;
     SPYB_CUDA(be, cudaEventRecord(m->ev0, be->stream));
     for (int s = 0; s < n_steps; ++s) {
-        m->att_form = step_form(m, n_past + s);
-        if (use_graph) { SPYB_CUDA(be, cudaGraphLaunch(find_graph(m, GRAPH_DECODE)->exec, be->stream)); }
+        const spyb_model::StepGraph *step = step_at(n_past + s);
+        if (step == nullptr && use_graph) { cudaStreamSynchronize(be->stream); return SPYB_FAIL; }
+        if (use_graph) { SPYB_CUDA(be, cudaGraphLaunch(step->exec, be->stream)); }
         else { int64_t n = 0; if (run_decode_step(m, &n) != SPYB_SUCCESS) { return SPYB_FAIL; } per_step = n; }
         if (logits_host != nullptr) {
             // parity mode: logits of every step come back (argmax_embed does not modify them)

@@ -526,6 +526,30 @@ def test_steps_on_both_sides_of_the_attention_switch(n_ctx, oracle, tmp_models):
     m.close(); b.close()
 
 
+def test_more_captured_steps_than_are_kept(oracle, tmp_models):
+    """18 conversations that cross the attention switch are 36 captured steps, four more than are kept: each turn of the second round finds its
+    steps gone and captures them again, the second one while steps are running. Host-driven steps of the same conversations go among them."""
+    cfg = gguf_io.LlamaConfig(n_layer=2, d_model=256, n_head=2, n_ff=512, n_vocab=512, weight_std=0.05)
+    path, n_ctx, n_seq, n = str(tmp_models / "evict.gguf"), 264, 18, 236
+    if not os.path.exists(path):
+        gguf_io.make_llama_gguf(path, cfg, seed=48)
+    prompts = [np.random.default_rng(s).integers(3, cfg.n_vocab, size=n) for s in (15, 16)]
+    want = [oracle.OracleLlama(path, n_ctx=n_ctx).generate(p, 13) for p in prompts]
+    b = B.B200Backend(0)
+    m = B.LlamaModel(b, path, n_ctx=n_ctx)
+    m.set_sequences(n_seq)
+    for turn in range(2):
+        for c in range(n_seq):
+            m.select_sequence(c)
+            ids, logits = want[c % 2]
+            if turn == 0:
+                assert int(np.argmax(m.eval(prompts[c % 2], 0))) == ids[0]
+            assert np.array_equal(m.decode(int(ids[0]), n, 12)[0], ids[1:])
+            if c % 5 == 0:
+                assert logits_ok(m.eval(np.array([ids[2]]), n + 2)[None], logits[3:4])
+    m.close(); b.close()
+
+
 def test_rmsnorm_running_sum_on_hard_inputs(oracle, tmp_models):
     """The RMSNorm sum of squares is a serial f32 running sum on the CPU (groups of four squares added to one
     accumulator in order); the GPU forms the groups in parallel and runs the same chain on one thread. Inputs that
