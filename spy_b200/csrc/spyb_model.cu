@@ -608,6 +608,10 @@ int step_form(const spyb_model *m, int pos) {
     return attention_form(a, m->be->launch_cfg(false), pos);
 }
 
+void drop_graphs(spyb_model *m) {
+    for (auto &g : m->graphs) { cudaGraphExecDestroy(g.exec); }
+    m->graphs.clear();
+}
 // the captured step of this kind for the model's sequence and m->att_form; null: not captured yet
 enum { GRAPH_DECODE, GRAPH_EVAL };
 constexpr size_t MAX_STEP_GRAPHS = 32;
@@ -638,7 +642,12 @@ spyb_model::StepGraph *captured_step(spyb_model *m, int kind, Enqueue enqueue) {
         if (st == SPYB_SUCCESS && err == cudaSuccess) { break; }
         exec = nullptr;
         cudaGetLastError();
-        if (m->step_ok && m->step_coop) { m->step_coop = false; again = true; }   // a cooperative launch the capture refuses: plain launch of the same grid
+        if (err == cudaErrorMemoryAllocation && !m->graphs.empty()) {   // (some 0.5 MB a step of 32 layers: the kept ones make room)
+            cudaStreamSynchronize(be->stream);
+            drop_graphs(m);
+            again = true;
+        }
+        else if (m->step_ok && m->step_coop) { m->step_coop = false; again = true; }   // a cooperative launch the capture refuses: plain launch of the same grid
         else if (st == SPYB_SUCCESS) { be->set_error("CUDA graph capture failed: %s", cudaGetErrorString(err)); }
     }
     if (exec == nullptr) { return nullptr; }
@@ -1016,7 +1025,7 @@ void spyb_model_free(spyb_model *m) {
     if (m == nullptr) { return; }
     cudaSetDevice(m->be->config.device_id);
     cudaStreamSynchronize(m->be->stream);
-    for (auto &g : m->graphs) { cudaGraphExecDestroy(g.exec); }
+    drop_graphs(m);
     if (m->nccl_comm && g_nccl.CommDestroy) { g_nccl.CommDestroy(m->nccl_comm); }
     for (void *p : m->owned) { cudaFree(p); }
     if (m->h_pos_pinned) { cudaFreeHost(m->h_pos_pinned); }
@@ -1346,11 +1355,6 @@ spyb_status spyb_model_selftest_wait_timeout(spyb_model *m, uint64_t limit_ns, i
 }
 
 // ---- batches of independent sequences that share the weights (every step reads them once for all sequences)
-static void drop_graphs(spyb_model *m) {
-    for (auto &g : m->graphs) { cudaGraphExecDestroy(g.exec); }
-    m->graphs.clear();
-}
-
 spyb_status spyb_model_set_sequences(spyb_model *m, int32_t n_seq) {
     if (m == nullptr) { return SPYB_FAIL; }
     spyb_backend *be = m->be;

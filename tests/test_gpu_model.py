@@ -550,6 +550,38 @@ def test_more_captured_steps_than_are_kept(oracle, tmp_models):
     m.close(); b.close()
 
 
+def test_captured_steps_with_no_memory_left(tmp_models):
+    """20 conversations on a device that is full once the first one has its captured steps: the kept steps make room for those of the others."""
+    cfg = gguf_io.LlamaConfig(n_layer=32, d_model=256, n_head=2, n_ff=256, n_vocab=500, weight_std=0.05)
+    path = str(tmp_models / "deep.gguf")
+    gguf_io.make_llama_gguf(path, cfg, seed=50)
+    prompt = np.random.default_rng(3).integers(3, cfg.n_vocab, size=236)
+    b = B.B200Backend(0, arena_bytes=1 << 22)
+    m = B.LlamaModel(b, path, n_ctx=264)
+    m.set_sequences(20)
+    for c in range(20):
+        m.select_sequence(c)
+        first = int(np.argmax(m.eval(prompt, 0)))
+    want = m.decode(first, len(prompt), 12)[0]
+    hogs = []
+    size = b.get_avail_memory_capacity()
+    while size >= 1 << 20:
+        try:
+            hogs.append((b.alloc_memory(size), size))
+        except B.SpybError:
+            size //= 2
+    try:
+        got = []
+        for c in range(20):
+            m.select_sequence(c)
+            got.append(m.decode(first, len(prompt), 12)[0])
+    finally:
+        for h in hogs:
+            b.dealloc_memory(*h)
+    m.close(); b.close()
+    assert all(np.array_equal(g, want) for g in got)
+
+
 def test_rmsnorm_running_sum_on_hard_inputs(oracle, tmp_models):
     """The RMSNorm sum of squares is a serial f32 running sum on the CPU (groups of four squares added to one
     accumulator in order); the GPU forms the groups in parallel and runs the same chain on one thread. Inputs that
