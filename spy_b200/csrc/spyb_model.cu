@@ -230,11 +230,41 @@ namespace {
 
 spyb_status build_step_plan(spyb_model *m);
 
+void drop_graphs(spyb_model *m) {
+    for (auto &g : m->graphs) { cudaGraphExecDestroy(g.exec); }
+    m->graphs.clear();
+}
+
+// fewer tokens per attention launch of a prompt, and room for their score rows only
+void shrink_att_group(spyb_model *m, int group) {
+    m->att_group = group;
+    float *&rows = m->att_scratch != nullptr ? m->att_scratch : m->pf_att_scratch;
+    if (rows == nullptr) { return; }
+    cudaStreamSynchronize(m->be->stream);
+    drop_graphs(m);   // (captured steps may hold the address)
+    auto at = std::find(m->owned.begin(), m->owned.end(), static_cast<void *>(rows));
+    m->owned.erase(at);
+    cudaFree(rows);
+    rows = nullptr;
+    void *raw = nullptr;
+    if (cudaMalloc(&raw, (size_t)group * (m->dl / m->info.head_dim) * (((size_t)m->info.n_ctx + 3) & ~(size_t)3) * sizeof(float) + 64) != cudaSuccess) { cudaGetLastError(); return; }
+    m->owned.push_back(raw);
+    rows = static_cast<float *>(raw);
+}
+
+// Device memory has run out: gives back score rows that only make prompts faster. False: nothing is left.
+bool give_back(spyb_model *m) {
+    cudaGetLastError();   // (some callers go on without: not left for the next launch to find)
+    if ((m->att_scratch == nullptr && m->pf_att_scratch == nullptr) || m->att_group <= PF_ATT_GROUP) { return false; }
+    shrink_att_group(m, m->att_group / 2);
+    return true;
+}
+
 template <class T>
 spyb_status dev_alloc(spyb_model *m, T **p, size_t count) {
     void *raw = nullptr;
-    if (cudaMalloc(&raw, count * sizeof(T) + 64) != cudaSuccess) {
-        cudaGetLastError();   // (some callers go on without: not left for the next launch to find)
+    while (cudaMalloc(&raw, count * sizeof(T) + 64) != cudaSuccess) {
+        if (give_back(m)) { continue; }
         m->be->set_error("out of device memory allocating %llu bytes", (unsigned long long)(count * sizeof(T)));
         return SPYB_FAIL;
     }
@@ -608,10 +638,6 @@ int step_form(const spyb_model *m, int pos) {
     return attention_form(a, m->be->launch_cfg(false), pos);
 }
 
-void drop_graphs(spyb_model *m) {
-    for (auto &g : m->graphs) { cudaGraphExecDestroy(g.exec); }
-    m->graphs.clear();
-}
 // the captured step of this kind for the model's sequence and m->att_form; null: not captured yet
 enum { GRAPH_DECODE, GRAPH_EVAL };
 constexpr size_t MAX_STEP_GRAPHS = 32;
@@ -785,8 +811,8 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
         const int64_t rb = GgufFile::row_bytes(t->type, k_full);
         const int64_t max_rows = std::max<int64_t>(1, (int64_t)(64u << 20) / rb);   // 64 MiB staging pieces
         void *stage = nullptr;
-        if (cudaMalloc(&stage, (size_t)std::min(max_rows, n_rows) * rb + 64) != cudaSuccess) {
-            cudaGetLastError();
+        while (cudaMalloc(&stage, (size_t)std::min(max_rows, n_rows) * rb + 64) != cudaSuccess) {
+            if (give_back(m)) { continue; }
             be->set_error("GGUF: %s: out of device memory", name.c_str());
             pf_no_room = true;
             return SPYB_UNSUPPORTED;

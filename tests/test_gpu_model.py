@@ -202,6 +202,57 @@ def test_prompts_of_a_reused_cache_read_their_own_rows(tmp_models):
     assert np.isfinite(got[0]).all() and np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
 
 
+def _wide_context_model(tmp_models):
+    """One layer of 8 heads and a context of 16384: the score rows of a prompt's attention take 134 MB in groups of 256 tokens, 67 MB in groups of 128."""
+    cfg = gguf_io.LlamaConfig(n_layer=1, d_model=1024, n_head=8, n_ff=2816, n_vocab=500, weight_std=0.03)
+    path = str(tmp_models / "wide_context.gguf")
+    if not os.path.exists(path):
+        gguf_io.make_llama_gguf(path, cfg, seed=74)
+    return path, np.random.default_rng(5).integers(3, cfg.n_vocab, size=300)
+
+
+def _fill(b, leave):
+    n = b.get_avail_memory_capacity() - leave
+    return b.alloc_memory(n), n
+
+
+def test_sequences_take_the_room_of_large_attention_groups(tmp_models):
+    """KV caches that only fit beside the score rows of smaller groups of prompt tokens: the groups become smaller, the bits stay."""
+    path, prompt = _wide_context_model(tmp_models)
+    b = B.B200Backend(0, arena_bytes=1 << 22)
+    m = B.LlamaModel(b, path, n_ctx=16384)
+    want = m.eval(prompt, 0)
+    m.close()
+    m = B.LlamaModel(b, path, n_ctx=16384)
+    hog = _fill(b, 44 << 20)
+    try:
+        m.set_sequences(1)                     # 64 MB of caches
+        got = m.eval(prompt, 0)
+    finally:
+        b.dealloc_memory(*hog)
+    m.close(); b.close()
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+def test_tile_copies_take_the_room_of_large_attention_groups(tmp_models):
+    """A load whose tile copies only fit beside the score rows of smaller groups: the model still runs its prompts as GEMMs."""
+    path, prompt = _wide_context_model(tmp_models)
+    b = B.B200Backend(0, arena_bytes=1 << 22)
+    before = b.get_avail_memory_capacity()
+    m = B.LlamaModel(b, path, n_ctx=16384)
+    used = before - b.get_avail_memory_capacity()
+    want, launches = m.eval(prompt[:100], 0), m.last_launches
+    m.close()
+    hog = _fill(b, used - (20 << 20))
+    try:
+        m = B.LlamaModel(b, path, n_ctx=16384)
+    finally:
+        b.dealloc_memory(*hog)
+    got = m.eval(prompt[:100], 0)
+    assert m.last_launches == launches and np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    m.close(); b.close()
+
+
 @pytest.mark.parametrize("kq", [False, True])
 def test_models_and_prompts_with_little_memory_left(kq, tmp_models):
     """A device with room for a model but not for the tile copies of its weights, and one whose memory runs out between the load and the first prompt:
