@@ -1042,6 +1042,7 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
             W = PfMat();
         };
         for (Layer &ly : m->layers) { for (PfMat *W : {&ly.pf_qkv, &ly.pf_k, &ly.pf_v, &ly.pf_wo, &ly.pf_ug, &ly.pf_gate, &ly.pf_down}) { drop(*W); } }
+        if (m->att_group > TMAX) { shrink_att_group(m, TMAX); }   // (a mat-vec pass holds no more tokens)
     }
     *out = m;
     return SPYB_SUCCESS;

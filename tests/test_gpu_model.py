@@ -253,6 +253,27 @@ def test_tile_copies_take_the_room_of_large_attention_groups(tmp_models):
     m.close(); b.close()
 
 
+def test_models_on_mat_vec_passes_keep_the_score_rows_of_a_pass(tmp_models):
+    """No room for the tile copies beside the smallest groups either: prompts run as mat-vec passes, and only the score rows of one are kept."""
+    path, prompt = _wide_context_model(tmp_models)
+    b = B.B200Backend(0, arena_bytes=1 << 22)
+    before = b.get_avail_memory_capacity()
+    m = B.LlamaModel(b, path, n_ctx=16384)
+    used = before - b.get_avail_memory_capacity()
+    want = m.eval(prompt[:40], 0)
+    m.close()
+    hog = _fill(b, used - (90 << 20))
+    try:
+        before = b.get_avail_memory_capacity()
+        m = B.LlamaModel(b, path, n_ctx=16384)
+        without = before - b.get_avail_memory_capacity()
+    finally:
+        b.dealloc_memory(*hog)
+    assert used - without > 134 << 20          # 27 MB of tile copies, and 130 of 134 MB
+    assert np.array_equal(m.eval(prompt[:40], 0).view(np.uint32), want.view(np.uint32))
+    m.close(); b.close()
+
+
 @pytest.mark.parametrize("kq", [False, True])
 def test_models_and_prompts_with_little_memory_left(kq, tmp_models):
     """A device with room for a model but not for the tile copies of its weights, and one whose memory runs out between the load and the first prompt:
