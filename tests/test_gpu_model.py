@@ -262,7 +262,7 @@ def test_models_on_mat_vec_passes_keep_the_score_rows_of_a_pass(tmp_models):
     used = before - b.get_avail_memory_capacity()
     want = m.eval(prompt[:40], 0)
     m.close()
-    hog = _fill(b, used - (90 << 20))
+    hog = _fill(b, used - (81 << 20))
     try:
         before = b.get_avail_memory_capacity()
         m = B.LlamaModel(b, path, n_ctx=16384)
