@@ -203,9 +203,14 @@ spyb_status spyb_matmul_noalloc(spyb_backend *backend, int32_t weight_type, cons
 #define SPYB_PREFILL_MIN_TOKENS 8
 spyb_status spyb_prefill_matmul(spyb_backend *backend, int32_t weight_type, const void *w_rows_host, int64_t n_rows, int64_t k,
                                 const float *x_host, int64_t n_cols, const float *norm_w_host, float eps, float *out_host);
+/* The same in a given form of the kernel, for the tests of the forms (0: by the sizes, as above): tiles of tile_tokens tokens (Q4_0 / Q8_0: 8 or
+ * 16; K-quants: 16, 32 or 64), each by tile_ctas CTAs (1, or for Q4_0 / Q8_0 a cluster of 2). */
+spyb_status spyb_prefill_matmul_form(spyb_backend *backend, int32_t weight_type, const void *w_rows_host, int64_t n_rows, int64_t k,
+                                     const float *x_host, int64_t n_cols, const float *norm_w_host, float eps, int32_t tile_tokens, int32_t tile_ctas,
+                                     float *out_host);
 
 /* Failure-path check of the prompt kernel that faults nothing: a small launch whose second batch of blocks is never
- * copied, with `limit_ns` as the bound of every wait. Succeeds when the kernel returned by itself and recorded one of
+ * copied, by one CTA and then by a cluster of two, with `limit_ns` as the bound of every wait. Succeeds when the kernel returned by itself and recorded one of
  * its codes (4 = a shared-memory stage, 5 = operands or a free accumulator buffer, 6 = a tensor-core result; also
  * written to *error_code_out); the record is cleared again, so the backend stays usable. No reference counterpart. */
 spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *backend, uint64_t limit_ns, int32_t *error_code_out);

@@ -415,6 +415,10 @@ spyb_status spyb_matmul_noalloc(spyb_backend *be, int32_t weight_type, const voi
 // uses the same kernels on resident buffers.
 spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const void *w_rows_host, int64_t n_rows, int64_t k, const float *x_host,
                                 int64_t n_cols, const float *norm_w_host, float eps, float *out_host) {
+    return spyb_prefill_matmul_form(be, weight_type, w_rows_host, n_rows, k, x_host, n_cols, norm_w_host, eps, 0, 0, out_host);
+}
+spyb_status spyb_prefill_matmul_form(spyb_backend *be, int32_t weight_type, const void *w_rows_host, int64_t n_rows, int64_t k, const float *x_host,
+                                     int64_t n_cols, const float *norm_w_host, float eps, int32_t tile_tokens, int32_t tile_ctas, float *out_host) {
     if (be == nullptr) { return SPYB_FAIL; }
     const bool kq = weight_type == SPYB_Q4_K || weight_type == SPYB_Q6_K;
     if (weight_type != SPYB_Q4_0 && weight_type != SPYB_Q8_0 && !kq) { be->set_error("prefill_matmul: weight type %d", weight_type); return SPYB_UNSUPPORTED; }
@@ -423,8 +427,10 @@ spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const voi
         n_cols < 1 || n_cols > 4096) {
         be->set_error("prefill_matmul: needs k a multiple of 32 up to %d, 1..4096 columns", PF_MAX_K); return SPYB_UNSUPPORTED;
     }
+    const bool width_ok = kq ? tile_tokens == 16 || tile_tokens == 32 || tile_tokens == 64 : tile_tokens == 8 || tile_tokens == 16;
+    if ((tile_tokens != 0 && !width_ok) || tile_ctas < 0 || tile_ctas > (kq ? 1 : 2)) { be->set_error("prefill_matmul: no form with tiles of %d tokens by %d CTAs", tile_tokens, tile_ctas); return SPYB_UNSUPPORTED; }
     cudaSetDevice(be->config.device_id);
-    const int nb = (int)(k / QK), T = (int)n_cols, tile_tok = prefill_tile_tokens(weight_type, n_rows, nb, T);
+    const int nb = (int)(k / QK), T = (int)n_cols, tile_tok = tile_tokens != 0 ? tile_tokens : prefill_tile_tokens(weight_type, n_rows, nb, T);
     const int64_t rb = kq ? (k / 256) * (weight_type == SPYB_Q4_K ? 144 : 210) : (int64_t)nb * (weight_type == SPYB_Q4_0 ? 18 : 34);
     const size_t wbytes = prefill_weight_bytes(weight_type, n_rows, nb), ybytes = prefill_act_bytes(T, nb);
     uint8_t *raw = nullptr, *w = nullptr, *yq = nullptr; float *x = nullptr, *nw = nullptr, *out = nullptr;
@@ -444,7 +450,7 @@ spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const voi
     if (err == cudaSuccess) { err = launch_prefill_quant(x, k, T, (int)k, nw, eps, yq, be->stream, weight_type, tile_tok); }
     if (err == cudaSuccess) {
         PrefillGemm g;
-        g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.tile_tok = tile_tok; g.T = T; g.out = out; g.out_stride = n_rows;
+        g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.tile_tok = tile_tok; g.split = tile_ctas; g.T = T; g.out = out; g.out_stride = n_rows;
         g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
         err = launch_prefill_gemm(g, be->stream);
     }
@@ -456,7 +462,7 @@ spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const voi
     return SPYB_SUCCESS;
 }
 
-// Failure-path check of the prompt GEMM that faults nothing: a small launch of one CTA, then one of a cluster of two (more blocks a row), whose
+// Failure-path check of the prompt GEMM that faults nothing: a small launch of one CTA, then one of a cluster of two, whose
 // copy thread leaves the second batch of blocks out, with `limit_ns` as the bound of every wait. The roles that wait for that batch give up
 // one after the other, the kernel frees its tensor memory and returns, and the error word holds a code of the prompt kernel (4, 5 or 6).
 spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *be, uint64_t limit_ns, int32_t *error_code_out) {
@@ -474,10 +480,11 @@ spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *be, uint64_t limit_
     if (err == cudaSuccess) { err = cudaMemsetAsync(w, 0, wbytes, be->stream); }
     if (err == cudaSuccess) { err = cudaMemsetAsync(yq, 0, ybytes, be->stream); }
     int code = 0;
-    for (const int nb : {12, nb_max}) {
+    for (const int split : {1, 2}) {
+        const int nb = split == 1 ? 12 : nb_max;
         if (err != cudaSuccess) { break; }
         PrefillGemm g;
-        g.w = w; g.type = SPYB_Q8_0; g.n_rows = PF_ROWS; g.nb = nb; g.yq = yq; g.tile_tok = prefill_tile_tokens(SPYB_Q8_0, PF_ROWS, nb, T); g.T = T; g.out = out; g.out_stride = PF_ROWS;
+        g.w = w; g.type = SPYB_Q8_0; g.n_rows = PF_ROWS; g.nb = nb; g.yq = yq; g.tile_tok = PF_TOK; g.split = split; g.T = T; g.out = out; g.out_stride = PF_ROWS;
         g.error_flag = be->d_error_flag; g.wait_limit_ns = limit_ns; g.selftest_skip_step = 1;
         err = launch_prefill_gemm(g, be->stream);
         if (err == cudaSuccess) { err = cudaStreamSynchronize(be->stream); }   // returns: the kernel ended by itself

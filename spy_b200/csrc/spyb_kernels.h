@@ -124,6 +124,7 @@ struct PrefillGemm {
     int            nb = 0;            // blocks per row
     const uint8_t *yq = nullptr;      // [token tiles][nb] blocks of activations (launch_prefill_quant for this weight type and tile_tok)
     int            tile_tok = 0;      // tokens per tile: prefill_tile_tokens()
+    int            split = 0;         // Q4_0 / Q8_0: CTAs that share a tile, 1 or 2 (0: by the sizes)
     int            T = 0;
     float         *out = nullptr;     // [T][out_stride]
     int64_t        out_stride = 0;

@@ -678,8 +678,8 @@ cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K,
 cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     if (g.type == 12 || g.type == 14) { return launch_prefill_gemm_kq(g, stream, pdl); }
     if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
-    if (g.tile_tok != 16 && g.tile_tok != 8) { return cudaErrorInvalidValue; }
-    const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok).split == 2;
+    if ((g.tile_tok != 16 && g.tile_tok != 8) || g.split < 0 || g.split > 2) { return cudaErrorInvalidValue; }
+    const bool pair = (g.split != 0 ? g.split : best_form(g.n_rows, g.nb, g.T, g.tile_tok).split) == 2;
     // Many tokens (MANY): the epilogue is the bound and the weights come out of L2; copies of half a block are in its way for less long.
     // 22016 x 4096 x 448 tokens 659 us with one copy a step, 649 by blocks, 642 by halves, 646 by quarters. Where the weights' way
     // through HBM is the bound one copy is better: 4096 x 11008 x 64 tokens 55.8 us, by halves 56.2.

@@ -164,18 +164,20 @@ def test_prefill_matmul_walks_tiles_of_both_widths(be, oracle, qt, n, k, t):
 @pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
 @pytest.mark.parametrize("n,k,t", [(19204, 1600, 7), (19204, 2880, 15), (132, 3104, 9), (516, 2976, 32)])
 def test_prefill_matmul_shared_by_two_ctas(be, oracle, qt, n, k, t):
-    """The form whose tiles are shared by a cluster of two CTAs, in narrow and in wide token tiles: three rounds of tiles (the hand-over's
-    buffer is used again), odd numbers of steps that end inside a step, a last row tile of four rows, ragged and full token tiles."""
+    """The form whose tiles are shared by a cluster of two CTAs beside that of one CTA a tile, in narrow and in wide token tiles: three rounds of tiles
+    (the hand-over's buffer is used again), odd numbers of steps that end inside a step, a last row tile of four rows, ragged and full token tiles."""
     rng = np.random.default_rng(n + k + t + qt)
     w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
     x = rng.standard_normal((t, k)).astype(np.float32)
     x[rng.integers(0, t, 8), rng.integers(0, k, 8)] *= 40.0
-    got = be.prefill_matmul(qt, w, n, k, x)
     want = oracle.matmul(qt, w, k, n, x)
-    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    for form in [(0, 0), (8, 1), (16, 1), (8, 2), (16, 2)]:
+        got = be.prefill_matmul(qt, w, n, k, x, form=form)
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), form
 
 
-@pytest.mark.parametrize("qt,k", [(quants.Q4_0, 2272), (quants.Q4_0, 4128), (quants.Q8_0, 8192), (quants.Q4_0, 8224), (quants.Q4_K, 4352), (quants.Q4_K, 9216)])
+@pytest.mark.parametrize("qt,k", [(quants.Q4_0, 2272), (quants.Q4_0, 4128), (quants.Q8_0, 8192), (quants.Q4_0, 8224), (quants.Q4_K, 4352), (quants.Q4_K, 9216),
+                                  (quants.Q8_0, 13824), (quants.Q4_0, 14336), (quants.Q4_K, 13824), (quants.Q6_K, 14336)])
 def test_prefill_quantizer_of_normed_rows(be, oracle, qt, k):
     """RMSNorm in front of the quantizer at the edges of its forms: one, two and four groups a thread, rows below and above what the four
     warps' running sum takes; a row of zeros among the others (the sum then falls back to the plain chain)."""
@@ -275,6 +277,10 @@ def test_prefill_matmul_rejects_what_does_not_fit(be):
     with pytest.raises(B.SpybError) as e:
         be.prefill_matmul(quants.Q4_0, w, 100, 48, x)          # k not a multiple of 32
     assert e.value.status == B.UNSUPPORTED
+    for qt, form in [(quants.Q4_0, (32, 1)), (quants.Q8_0, (0, 3)), (quants.Q4_K, (8, 0)), (quants.Q6_K, (16, 2)), (quants.Q4_0, (-8, 0))]:
+        with pytest.raises(B.SpybError) as e:
+            be.prefill_matmul(qt, w, 4, 256, np.zeros((2, 256), dtype=np.float32), form=form)          # no such form of the kernel
+        assert e.value.status == B.UNSUPPORTED
     with pytest.raises(B.SpybError) as e:
         be.prefill_matmul(quants.Q4_K, w, 128, 128, np.zeros((2, 128), dtype=np.float32))   # K-quant rows: k a multiple of 256
     assert e.value.status == B.UNSUPPORTED
