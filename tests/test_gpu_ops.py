@@ -817,12 +817,14 @@ def test_lookup_tables_identical_for_every_key(be, oracle):
     assert np.array_equal(bits(ex), bits(want_exp))
 
 
-# --------------------------------------------------------------------------- the mat-vec kernels' quantizer on values that are hard to round
-HARD_K = [32, 96, 1024, 4096, 4128, 6144, 8224, 11008]
+# --------------------------------------------------------------------------- the mat-vec and GEMM quantizers on values that are hard to round
+HARD_K = [32, 96, 1024, 4096, 4128, 6144, 8224, 11008, 13824, 14336]
+HARD_KQ = [256, 4096, 4352, 6144, 8448, 12288, 13824, 14336]
 
 
 def hard_values(k: int, seed: int) -> np.ndarray:
-    """Blocks of ties (odd multiples of half a step), of zeros, of subnormal and of huge values, of one outlier, and of ordinary ones."""
+    """Blocks of ties (odd multiples of half a step), of zeros, of values so small that their f16 scale is zero (whatever the bytes are), of huge
+    values, of one outlier, and of ordinary ones."""
     rng = np.random.default_rng(seed)
     x = rng.standard_normal(k).astype(np.float32).reshape(-1, 32)
     kind = np.arange(len(x)) % 7
@@ -836,22 +838,18 @@ def hard_values(k: int, seed: int) -> np.ndarray:
     return x.reshape(-1)
 
 
-@pytest.mark.parametrize("k", HARD_K)
-@pytest.mark.parametrize("cols", [1, 3, 9])
-@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
-@pytest.mark.parametrize("offset", [0, 4])
-def test_quantizer_on_hard_values(be, oracle, qt, cols, k, offset):
-    """Each row of W picks one value of the quantized activations (a single nonzero weight), so that every byte shows: the oracle's bits from
-    the mat-vec kernels and the GEMM, over the remainders and numbers of values per thread of their quantizers, and for activations that
-    lie on 16 bytes only (offset: floats)."""
-    n = 64
-    x = np.stack([hard_values(k, 91 + c) for c in range(cols)])
-    rng = np.random.default_rng(5)
+def pick_rows(qt: int, n: int, k: int) -> np.ndarray:
+    """Rows that pick one value each (a single nonzero weight)."""
     w = np.zeros((n, k), dtype=np.float32)
-    w[np.arange(n), rng.integers(0, k, n)] = 1.0
-    raw = quants.quantize(w, qt)
+    w[np.arange(n), np.random.default_rng(5).integers(0, k, n) if n != k else np.arange(n)] = 1.0
+    return quants.quantize(w, qt)
+
+
+def constant_matmul(be, name: str, qt: int, raw: np.ndarray, n: int, x: np.ndarray, offset: int = 0) -> np.ndarray:
+    """x [columns, k] times an uploaded constant; the activations lie `offset` floats behind an allocation's start."""
+    cols, k = x.shape
     px = be.upload(np.concatenate([np.zeros(offset, dtype=np.float32), x.reshape(-1)]))
-    pw, po = be.upload_constant(f"hard {qt} {k} {cols} {offset}", raw, qt, (k, n)), be.alloc_memory(4 * n * cols)
+    pw, po = be.upload_constant(name, raw, qt, (k, n)), be.alloc_memory(4 * n * cols)
     d = B.OpDesc()
     d.op_type, d.num_input = B.OP["MatMul"], 2
     d.input[0] = B.make_tensor(pw, qt, (k, n), None, B.NODE_CONSTANT)
@@ -860,4 +858,72 @@ def test_quantizer_on_hard_values(be, oracle, qt, cols, k, offset):
     be.submit(d)
     got = be.download(po, (cols, n), np.float32)
     be.dealloc_memory(px, 4 * (x.size + offset)); be.dealloc_memory(po, 4 * n * cols)
-    assert close(got, oracle.matmul(qt, raw, k, n, x))
+    return got
+
+
+@pytest.mark.parametrize("qt,k", [(qt, k) for qt in (quants.Q4_0, quants.Q8_0) for k in HARD_K] + [(qt, k) for qt in (quants.Q4_K, quants.Q6_K) for k in HARD_KQ])
+@pytest.mark.parametrize("cols", [1, 3, 9])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_quantizer_on_hard_values(be, oracle, qt, cols, k, offset):
+    """Each row of W picks one value of the quantized activations, so that the bytes show: the oracle's bits (K-quants: the restatement's) from the
+    mat-vec kernels and the GEMM, over the remainders and numbers of values per thread of their quantizers, and for activations that lie on
+    16 bytes only (offset: floats)."""
+    x = np.stack([hard_values(k, 91 + c) for c in range(cols)])
+    raw = pick_rows(qt, 64, k)
+    got = constant_matmul(be, f"hard {qt} {k} {cols} {offset}", qt, raw, 64, x, offset)
+    assert close(got, oracle.matmul(qt, raw, k, 64, x))
+
+
+@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0, quants.Q4_K, quants.Q6_K])
+@pytest.mark.parametrize("cols", [1, 3, 9])
+@pytest.mark.parametrize("k", [256, 8192])
+def test_quantizer_takes_what_is_not_a_number_as_zero(be, oracle, qt, cols, k):
+    """A NaN among ordinary values does not count for its block's scale and becomes the byte 0, as in the conversion to integers: the bits of the
+    same activations with zeros there."""
+    rng = np.random.default_rng(k + cols)
+    x = rng.standard_normal((cols, k)).astype(np.float32)
+    at = rng.random((cols, k)) < 0.05
+    raw = quants.quantize((rng.standard_normal((64, k)) * 0.02).astype(np.float32), qt)
+    want = oracle.matmul(qt, raw, k, 64, np.where(at, np.float32(0), x))
+    for nan in (np.float32(np.nan), -np.float32(np.nan)):
+        got = constant_matmul(be, f"nan {qt} {k} {cols}", qt, raw, 64, np.where(at, nan, x))
+        assert np.array_equal(bits(got), bits(want))
+
+
+@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
+@pytest.mark.parametrize("cols", [1, 3, 9])
+def test_quantizer_on_infinities(be, qt, cols):
+    """A block that holds an infinity has an infinite scale and bytes of 0 throughout (0 * infinity is not a number): every product is NaN, while any
+    other byte would give an infinity. Each row picks one of the block's values."""
+    for inf in (np.inf, -np.inf):
+        x = np.random.default_rng(cols).standard_normal((cols, 32)).astype(np.float32)
+        x[:, 11] = inf
+        got = constant_matmul(be, f"inf {qt} {cols} {inf}", qt, pick_rows(qt, 32, 32), 32, x)
+        assert np.isnan(got).all()
+
+
+# --------------------------------------------------------------------------- operators beside their predecessors
+@pytest.mark.parametrize("wtype,tokens", [("q4_0", 1), ("q8_0", 3), ("q4_0", 7)])
+def test_operator_chain_with_and_without_programmatic_launch(wtype, tokens, monkeypatch):
+    """The operators of a decoder layer, passes submitted one behind the other without a wait between them: kernels that start beside their
+    predecessors (use_pdl) leave the same bits in the output and the caches as kernels that wait for them."""
+    import functools
+
+    import torch
+
+    from perf import cases
+
+    case = dict(kind="layer", wtype=wtype, n_head=6, n_ff=2112, tokens=tokens, past=37, n_ctx=64)
+    make = B.B200Backend
+    out = []
+    for use_pdl in (True, False):
+        monkeypatch.setattr(cases.B, "B200Backend", functools.partial(make, use_pdl=use_pdl))
+        state = cases.prepare(case, 11)
+        torch.cuda.synchronize()
+        for _ in range(5):
+            res = cases.run(state)
+        state.backend.sync()
+        out.append({name: t.cpu().numpy() for name, t in res.items()})
+        state.backend.close()
+    assert np.isfinite(out[0]["x"]).all()
+    assert all(np.array_equal(out[0][name], out[1][name]) for name in out[0])
