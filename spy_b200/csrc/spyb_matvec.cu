@@ -158,7 +158,7 @@ __device__ __forceinline__ float running_sum_small(const float *v3, int n4) {
 }
 
 // an eight-value group's words in the activation planes, and a block's scale
-__device__ __forceinline__ void act_store(const MatvecParams &p, uint32_t *Yw, int g, uint2 q) {
+__device__ __forceinline__ void act_store(uint32_t *Yw, int g, uint2 q) {
     const int b = g >> 2, at = ((b >> 2) * 8 + 2 * (g & 3)) * 4 + (b & 3);
     Yw[at] = q.x; Yw[at + 4] = q.y;
 }
@@ -225,7 +225,7 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
 #pragma unroll
     for (int k = 0; k < PG; ++k) {
         const int g = tid + k * MV_THREADS;
-        if (k < npass && g < n8p) { act_store(p, reinterpret_cast<uint32_t *>(act.Y), g, q[k]); }
+        if (k < npass && g < n8p) { act_store(reinterpret_cast<uint32_t *>(act.Y), g, q[k]); }
     }
     if (kd >= 0 && tid + kd * MV_THREADS < n8p) { reinterpret_cast<float *>(act.DS)[(tid + kd * MV_THREADS) >> 2] = act_scale(p, d); }
 }
@@ -281,7 +281,7 @@ __device__ __forceinline__ void matvec_prologue(const MatvecParams &p, ActPlanes
             int kd;
             const float d = quantize_q8_groups<1>(v, 1, q, kd);
             if (g < n8p) {
-                act_store(p, Yw + (size_t)t * nbp * 8, g, q[0]);
+                act_store(Yw + (size_t)t * nbp * 8, g, q[0]);
                 if (kd == 0) { DS[t * nbp + (g >> 2)] = act_scale(p, d); }
             }
         }
