@@ -209,6 +209,9 @@ spyb_status spyb_prefill_matmul_form(spyb_backend *backend, int32_t weight_type,
                                      const float *x_host, int64_t n_cols, const float *norm_w_host, float eps, int32_t tile_tokens, int32_t tile_ctas,
                                      float *out_host);
 
+/* The form that a Q4_0 / Q8_0 MatMul of these sizes takes on a device of n_sms SMs (host arithmetic only, no GPU needed). */
+spyb_status spyb_prefill_form(int64_t n_rows, int64_t k, int64_t n_cols, int32_t n_sms, int32_t *tile_tokens, int32_t *tile_ctas);
+
 /* Failure-path check of the prompt kernel that faults nothing: a small launch whose second batch of blocks is never
  * copied, by one CTA and then by a cluster of two, with `limit_ns` as the bound of every wait. Succeeds when the kernel returned by itself and recorded one of
  * its codes (4 = a shared-memory stage, 5 = operands or a free accumulator buffer, 6 = a tensor-core result; also

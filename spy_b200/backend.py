@@ -111,6 +111,7 @@ def lib():
         "spyb_matmul_noalloc": (i32, [vp, i32, vp, i64, i64, vp, i64, vp]),
         "spyb_prefill_matmul": (i32, [vp, i32, vp, i64, i64, vp, i64, vp, C.c_float, vp]),
         "spyb_prefill_matmul_form": (i32, [vp, i32, vp, i64, i64, vp, i64, vp, C.c_float, i32, i32, vp]),
+        "spyb_prefill_form": (i32, [i64, i64, i64, i32, C.POINTER(i32), C.POINTER(i32)]),
         "spyb_prefill_selftest_wait_timeout": (i32, [vp, u64, C.POINTER(i32)]),
         "spyb_model_tp_export": (i32, [vp, vp]),
         "spyb_model_tp_import": (i32, [vp, vp]),

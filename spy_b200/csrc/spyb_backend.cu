@@ -462,6 +462,12 @@ spyb_status spyb_prefill_matmul_form(spyb_backend *be, int32_t weight_type, cons
     return SPYB_SUCCESS;
 }
 
+spyb_status spyb_prefill_form(int64_t n_rows, int64_t k, int64_t n_cols, int32_t n_sms, int32_t *tile_tokens, int32_t *tile_ctas) {
+    if (n_rows < 1 || k < QK || k % QK != 0 || k > PF_MAX_K || n_cols < 1 || n_cols > 4096 || n_sms < 2 || tile_tokens == nullptr || tile_ctas == nullptr) { return SPYB_FAIL; }
+    prefill_form(n_rows, (int)(k / QK), (int)n_cols, n_sms, tile_tokens, tile_ctas);
+    return SPYB_SUCCESS;
+}
+
 // Failure-path check of the prompt GEMM that faults nothing: a small launch of one CTA, then one of a cluster of two, whose
 // copy thread leaves the second batch of blocks out, with `limit_ns` as the bound of every wait. The roles that wait for that batch give up
 // one after the other, the kernel frees its tensor memory and returns, and the error word holds a code of the prompt kernel (4, 5 or 6).

@@ -135,6 +135,7 @@ struct PrefillGemm {
 };
 int         device_sms();         // SMs of the current device
 int         prefill_tile_tokens(int type, int64_t n_rows, int nb, int T);   // width of the token tiles for this matrix and number of tokens
+void        prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split);   // host-only: the Q4_0 / Q8_0 kernel's form on a device of so many SMs
 size_t      prefill_weight_bytes(int type, int64_t n_rows, int nb);
 size_t      prefill_act_bytes(int T, int nb);
 cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);

@@ -610,23 +610,29 @@ int device_sms() {
 }
 
 // The form of the Q4_0 / Q8_0 kernel for a matrix and a number of tokens: tiles of 16 or of 8 tokens, by one CTA each or by a cluster of
-// two. The clusters walk the tiles in rounds, and the form whose rounds take least is the one. Fitted to 10 matrices from 1024 x 1024 to
-// 27648 x 5120 with 2 to 448 tokens (at 119 of 120 sizes within 3 % of the fastest form): a round costs a time for each block of the
-// row (less for narrow tiles, whose weights bound them, and about half for two CTAs), a launch what fills its pipelines and joins the
-// halves. us, one CTA / two: 4096 x 4096 x 8 tokens 20.8 / 15.1, 4096 x 11008 x 21 51 / 36.5, 22016 x 4096 x 16 49.6 / 44.5; and 12288 x 4096 x 8
-// tokens, whose 96 tiles need most of the chip, 24.2 / 28.4, 22016 x 4096 x 448 643 / 827.
-struct PfForm { int tok, split; double block_ns, launch_ns; };
-static PfForm best_form(int64_t n_rows, int nb, int T, int tok) {   // tok 0: of either width
-    static constexpr PfForm FORMS[4] = {{16, 1, 153, 3500}, {8, 1, 135, 2500}, {16, 2, 97, 4800}, {8, 2, 72, 5000}};
+// two; the one whose cost is least. CTAs or clusters walk the tiles in rounds: a launch costs what fills its pipelines, a round what a tile does
+// once (its drain, and for two CTAs the joining of the halves) and a time for each block of the row (less for narrow tiles, whose weights bound
+// them, and about half for two CTAs), and every block of the matrix some time for its bytes, in proportion to the chip. Fitted to 1450 sizes, ten
+// matrices of models and 1330 drawn ones from 1024 x 1024 to 32000 x 14336, with 5 to 512 tokens: within 3 % of the fastest form but at 8 of them (4 to
+// 13 %). (A cost of blocks and launches alone, fitted to the models' matrices, is off by 3 to 25 % at 55 of them, mostly rows of 1300 to 3000 values.)
+// us with the activations' quantizer, one CTA / two: 4096 x 4096 x 8 tokens 18.1 / 15.2, 4096 x 11008 x 16 54.7 / 34.9; and 1680 x 2208 x 79 tokens
+// 13.3 / 16.2, 22148 x 1728 x 5 17.0 / 20.1, 22016 x 4096 x 448 655 / 826.
+struct PfForm { int tok, split; double launch_ns, tile_ns, block_ns, rows_ns; };
+static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int sms) {   // tok 0: of either width
+    static constexpr PfForm FORMS[4] = {{16, 1, 5480, 1140, 144.6, 23.7}, {8, 1, 3010, 130, 124.2, 56.9}, {16, 2, 9920, 980, 84.3, 4.0}, {8, 2, 5520, 800, 68.3, 38.1}};
     PfForm best = {};
     double best_ns = 0.0;
     for (const PfForm &f : FORMS) {
         if (tok != 0 && tok != f.tok) { continue; }
-        const int64_t tiles = (n_rows + PF_M - 1) / PF_M * ((T + f.tok - 1) / f.tok), walks = std::max(1, device_sms() / f.split);
-        const double ns = (double)((tiles + walks - 1) / walks) * nb * f.block_ns + f.launch_ns;
+        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, tiles = row_tiles * ((T + f.tok - 1) / f.tok), walks = std::max(1, sms / f.split);
+        const double ns = f.launch_ns + (double)((tiles + walks - 1) / walks) * (f.tile_ns + nb * f.block_ns) + (double)row_tiles / sms * nb * f.rows_ns;
         if (best.tok == 0 || ns < best_ns) { best = f; best_ns = ns; }
     }
     return best;
+}
+void prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split) {
+    const PfForm f = best_form(n_rows, nb, T, 0, sms);
+    *tile_tok = f.tok; *split = f.split;
 }
 int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T) {
     if (type == 12 || type == 14) {   // K-quants: a tile of 16, 32, 64 tokens costs 1 : 1.35 : 2.3 (measured: the narrow ones are mostly weights)
@@ -635,7 +641,7 @@ int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T) {
         const double c16 = (double)rounds(16), c32 = 1.35 * (double)rounds(32), c64 = 2.3 * (double)rounds(64);
         return c16 <= c32 && c16 <= c64 ? 16 : c32 <= c64 ? 32 : 64;
     }
-    return best_form(n_rows, nb, T, 0).tok;
+    return best_form(n_rows, nb, T, 0, device_sms()).tok;
 }
 
 size_t prefill_weight_bytes(int type, int64_t n_rows, int nb) {
@@ -679,7 +685,7 @@ cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool 
     if (g.type == 12 || g.type == 14) { return launch_prefill_gemm_kq(g, stream, pdl); }
     if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
     if ((g.tile_tok != 16 && g.tile_tok != 8) || g.split < 0 || g.split > 2) { return cudaErrorInvalidValue; }
-    const bool pair = (g.split != 0 ? g.split : best_form(g.n_rows, g.nb, g.T, g.tile_tok).split) == 2;
+    const bool pair = (g.split != 0 ? g.split : best_form(g.n_rows, g.nb, g.T, g.tile_tok, device_sms()).split) == 2;
     // Many tokens (MANY): the epilogue is the bound and the weights come out of L2; copies of half a block are in its way for less long.
     // 22016 x 4096 x 448 tokens 659 us with one copy a step, 649 by blocks, 642 by halves, 646 by quarters. Where the weights' way
     // through HBM is the bound one copy is better: 4096 x 11008 x 64 tokens 55.8 us, by halves 56.2.

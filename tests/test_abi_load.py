@@ -45,3 +45,22 @@ def test_attention_ring_slots_keep_their_warps():
     and go to one reader, or a wait by parity could take a phase for the one two before it (stages overwritten while they are read, or a
     wait that never ends)."""
     assert backend.lib().spyb_selftest_host() == 0
+
+
+@pytest.mark.parametrize("rows,k,tokens,form", [
+    # measured on 148 SMs, us with tiles of 16 / 8 tokens by one CTA, 16 / 8 by two
+    (22148, 1728, 5, (8, 1)),       # 22.3 / 17.0 / 25.0 / 20.1
+    (1548, 2304, 58, (8, 1)),       # 16.2 / 12.7 / 14.0 / 17.8
+    (10192, 1088, 54, (8, 1)),      # 22.5 / 20.7 / 29.7 / 32.5
+    (4140, 2464, 23, (8, 1)),       # 16.7 / 13.2 / 14.7 / 18.5
+    (1680, 2208, 79, (8, 1)),       # 15.6 / 13.3 / 16.2 / 18.8
+    (8348, 4160, 12, (16, 2)),      # 25.8 / 22.5 / 19.7 / 28.5
+    (4096, 11008, 8, (8, 2)),       # 59.2 / 51.3 / 38.2 / 33.9
+    (7560, 5792, 15, (16, 2)),      # 34.4 / 32.1 / 24.3 / 38.4
+    (22016, 4096, 448, (16, 1)),    # 655 / 993 / 826 / 1185
+    (32000, 4096, 16, (16, 1)),     # 54.7 / 82.7 / 63.1 / 85.3
+])
+def test_prompt_gemm_takes_the_form_that_measures_fastest(rows, k, tokens, form):
+    tok, ctas = C.c_int32(0), C.c_int32(0)
+    assert backend.lib().spyb_prefill_form(rows, k, tokens, 148, C.byref(tok), C.byref(ctas)) == backend.SUCCESS
+    assert (tok.value, ctas.value) == form
