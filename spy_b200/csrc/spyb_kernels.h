@@ -157,6 +157,7 @@ cudaError_t launch_prefill_keep(const PrefillKeep &k, cudaStream_t stream);
 enum { ATT_BY_CONTEXT, ATT_ONE_CTA, ATT_CLUSTER };
 struct AttnParams {
     int           force_long = 0;     // take the three-kernel path (scratch needed) also at short contexts
+    int           early = 1;          // of a single token's step: cache rows of earlier steps are read before the wait for the kernel in front
     int           form = ATT_BY_CONTEXT;   // of a single token's step: by the context length, or the kernel that its position makes the faster one
     const __half *q = nullptr;        // [T][dl], already rounded to fp16
     const __half *k_cache = nullptr;  // [n_ctx][dl]
@@ -219,6 +220,7 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg);   // 
 int64_t     kq_row_bytes(int type, int64_t k);                             // bytes of one K-quant row in device memory
 cudaError_t launch_kq_relayout_q6k(const uint8_t *raw, int64_t n_rows, int64_t k, uint8_t *dst, cudaStream_t s);
 cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg);
+int         attention_early(int n_head, int n_ctx, bool kq);   // AttnParams::early for a model's steps
 int         attention_form(const AttnParams &p, const LaunchCfg &cfg, int pos);   // AttnParams::form for a single token at position pos
 int         attn_ring_selftest();   // host-only: 0 when every slot of the step kernel's ring keeps its writer and its reader
 size_t      attention_scratch_floats(int n_ctx, int n_head, int T);

@@ -459,6 +459,7 @@ spyb_status run_layers(spyb_model *m, int T, bool tap, int64_t *launches, int se
             a.n_head = m->dl / m->info.head_dim; a.hd = m->info.head_dim; a.dl = m->dl; a.T = T; a.n_ctx = m->info.n_ctx;
             a.scale = 1.0f / std::sqrt((float)m->info.head_dim);
             a.stamps = stamps(1); a.error_flag = be->d_error_flag; a.scratch = m->att_scratch; a.form = T == 1 && seq0 < 0 ? m->att_form : ATT_BY_CONTEXT;
+            a.early = attention_early(a.n_head, a.n_ctx, m->kq);
             if (seq0 >= 0) { a.seq_stride = m->seq_stride; a.k_cache = ly.k_base + (int64_t)seq0 * m->seq_stride; a.v_cache = ly.v_base + (int64_t)seq0 * m->seq_stride; }
             if (fused) { tp_produce(m, a.tp, 2 * L, true); }
             SPYB_CUDA(be, launch_attention(a, cfg)); ++*launches;

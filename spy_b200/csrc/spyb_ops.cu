@@ -12,6 +12,7 @@
 #include <cstdlib>
 
 #include "spyb_common.cuh"
+#include <type_traits>
 #include "spyb_kernels.h"
 #include "spyb_tp.cuh"
 #include "spyb_mv_common.cuh"
@@ -88,29 +89,34 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
     // the cache and changes nothing else in it; behind the wait only Q and what holds the new position is read. Whether the position
     // counter that was read early is the step's own shows then (the kernel that advances it may not have run; all is read again). L1 is not
     // coherent with the kernel in front: only K rows of earlier steps, which share no line with the new one, go through it before the wait.
-    // (7B, 8 to 40 positions: 5.5 -> 4.8 us a layer.)
+    // (7B, 8 to 40 positions: 5.5 -> 4.8 us a layer.) Passes of several tokens, batches and the layers that attention_early() leaves out read everything
+    // behind the wait and through L1, where the threads' 8 bytes of V^T share sectors.
     const int pv_e = tid >> 1, pv_half = tid & 1;
     const __half *vrow = v_cache + ((int64_t)h * ATT_HD + pv_e) * p.n_ctx;
     uint2 v_first[4], v_tail[8];
     uint4 kv[16];                                    // a whole K row in flight at once
     // the words of V^T and the K row of which positions lo <= j < n_vis (K: lo <= tid) are wanted; words that reach past n_vis, which may be
-    // new in part, belong to the second pass
-    auto request = [&](int lo, int n_vis, int n_main, bool last) {
+    // new in part, belong to the second pass, which goes past L1 where there was a first one
+    using PastL1 = std::true_type;
+    using ByL1   = std::false_type;
+    auto request = [&](auto past_l1, int lo, int n_vis, int n_main, bool last) {
+        constexpr bool PAST = decltype(past_l1)::value;
+        auto load_v = [&](int j) { const uint2 *src = reinterpret_cast<const uint2 *>(vrow + j); return PAST ? __ldcg(src) : *src; };
         auto wanted = [&](int j) { return j < n_vis && j + 4 > lo && (last || j + 4 <= n_vis); };
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const int j = 8 * a + 4 * pv_half;
-            if (0 < n_main && wanted(j)) { v_first[a] = __ldcg(reinterpret_cast<const uint2 *>(vrow + j)); }
+            if (0 < n_main && wanted(j)) { v_first[a] = load_v(j); }
         }
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             const int j = n_main + 4 * c;
-            if (wanted(j)) { v_tail[c] = __ldcg(reinterpret_cast<const uint2 *>(vrow + j)); }
+            if (wanted(j)) { v_tail[c] = load_v(j); }
         }
         if (tid >= lo && tid < n_vis) {
             const uint4 *krow = reinterpret_cast<const uint4 *>(k_cache + (int64_t)tid * p.dl + (int64_t)h * ATT_HD);
 #pragma unroll
-            for (int a = 0; a < 16; ++a) { kv[a] = last ? __ldcg(krow + a) : krow[a]; }
+            for (int a = 0; a < 16; ++a) { kv[a] = PAST && last ? __ldcg(krow + a) : krow[a]; }
         }
     };
 #pragma unroll
@@ -118,16 +124,16 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
 #pragma unroll
     for (int c = 0; c < 8; ++c) { v_tail[c] = make_uint2(0u, 0u); }
     int early = -1, early_tot = 0;
-    if (gridDim.y == 1 && !batch) {
+    if (p.early && gridDim.y == 1 && !batch) {
         const int2 known = __ldcg(reinterpret_cast<const int2 *>(p.pos_base));
         if (known.x >= 0 && known.x < p.n_ctx) { early = known.x; early_tot = row_length(known.x, known.y); }
-        request(0, early, ((early_tot - 1) / 32) * 32, false);
+        request(PastL1{}, 0, early, ((early_tot - 1) / 32) * 32, false);
     }
     pdl_wait();
     stamp(p.stamps, 1, false); stamp(p.stamps, 5, true);
     const int2 base = __ldcg(reinterpret_cast<const int2 *>(p.pos_base));
     const __half q_mine = (tid < ATT_HD) ? p.q[(int64_t)t * p.dl + (int64_t)h * ATT_HD + tid] : __float2half(0.f);
-    if (early >= 0) { request(early & ~3, early + 1, ((early_tot - 1) / 32) * 32, true); }   // (without waiting for the counter)
+    if (early >= 0) { request(PastL1{}, early & ~3, early + 1, ((early_tot - 1) / 32) * 32, true); }   // (without waiting for the counter)
     const int pos   = base.x + (batch ? 0 : t);
     const int n_vis = pos + 1;                   // causal mask: positions 0..pos are visible
     const int n_tot = row_length(base.x, base.y), n_main = ((n_tot - 1) / 32) * 32;
@@ -136,7 +142,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
         for (int a = 0; a < 4; ++a) { v_first[a] = make_uint2(0u, 0u); }
 #pragma unroll
         for (int c = 0; c < 8; ++c) { v_tail[c] = make_uint2(0u, 0u); }
-        request(0, n_vis, n_main, true);
+        if (early >= 0) { request(PastL1{}, 0, n_vis, n_main, true); } else { request(ByL1{}, 0, n_vis, n_main, true); }
     }
     if (tid < ATT_HD) { qf[tid] = __half2float(q_mine); }
     __syncthreads();
@@ -630,7 +636,8 @@ __global__ void __launch_bounds__(ATT_SM_THREADS) attn_softmax_kernel(const Attn
 // The same for a token of a prompt, in front of the tiled PV kernel: four neighbouring positions per thread and pass, whose exponentials are
 // one of std::reduce's groups; the running sum of the groups on the CTA's four warps (running_sum_wide). The probabilities become f16
 // values in the first half of the row - all of it is in shared memory by then - with zeros behind the last position, as far as a PV tile
-// reads. Ten CTAs per SM: one CTA's sum overlaps the others' passes. Bound: the gathers from the table of exponentials, 20 to 30 lines of
+// reads. Up to ten CTAs per SM (contexts below some 3900; nine at 4096, five at 8192: the shared memory is that of the whole context): one CTA's sum
+// overlaps the others' passes. Bound: the gathers from the table of exponentials, 20 to 30 lines of
 // L1 a warp. 128 tokens of 32 heads over 2000 positions on average: 36 -> 33 us.
 constexpr int ATT_SMT_THREADS = 128;
 static_assert(ATT_SMT_THREADS == RS_THREADS, "all warps form the running sum");
@@ -1162,8 +1169,20 @@ size_t attention_scratch_floats(int n_ctx, int n_head, int T) {   // 0: the sing
     return (size_t)T * n_head * (((size_t)n_ctx + 3) & ~(size_t)3);
 }
 
-// The form for a single token at position pos, where both kernels take the context. A layer's attention, us, one CTA a head / a cluster of four:
-// position 8: 4.8 / 7.5; 100: 5.3 / 8.0; 250: 8.2 / 8.2; 460: 14.3 / 8.9; 900: 28 / 10.7.
+// Whether the steps of a model read the cache rows of earlier steps before they wait for the QKV kernel. One attention CTA fills an SM, and the
+// mat-vec grids leave eight SMs free: CTAs of further heads start when a QKV CTA ends and hide nothing. The CTAs of the K-quant kernel end together,
+// and with up to 24 heads, where V^T's rows do not begin on lines (reads of eight bytes past L1 then take more sectors), the late reads cost more than
+// the early ones save. Steps of 4 layers, us, reads behind the wait / early, behind 20, 60, 220 positions. A context of 844: Q4_K_M 8 heads 104.7 /
+// 103.2, 106.5 / 103.4, 113.1 / 107.5; 12 heads 110.8 / 112.1, 113.1 / 114.7, 122.3 / 130.0; 20 heads 158.7 / 159.2, 160.7 / 161.8, 170.2 / 176.9; 32 heads 192.5 /
+// 191.7, 194.0 / 192.5, 203.8 / 201.5; Q4_0 12 heads 99.3 / 98.3, 101.1 / 99.6, 107.2 / 107.8. A context of 512: Q4_K_M 12 heads 111.6 / 111.1, 113.6 / 111.9, 123.6 /
+// 128.3; 24 heads 170.2 / 167.9, 172.3 / 168.9, 184.1 / 185.3.
+int attention_early(int n_head, int n_ctx, bool kq) { return !kq || n_head <= 8 || n_head > 24 || n_ctx % 64 == 0 ? 1 : 0; }
+
+// The form for a single token at position pos, where both kernels take the context. A layer's attention, us, one CTA a head / a cluster of four, 32
+// heads: position 8: 4.8 / 7.5; 100: 5.3 / 8.0; 250: 8.2 / 8.2; 460: 14.3 / 8.9; 900: 28 / 10.7. The line for other numbers of heads, from steps
+// of 8-layer models with little beside the attention, us a layer: 2 heads 248: 17.7 / 18.2, 280: 18.7 / 18.4; 8 heads 248: 20.6 / 21.4, 280: 21.5 / 21.5;
+// 16 heads 216: 24.9 / 24.7, 248: 25.5 / 24.7; 24 heads 248: 29.0 / 29.1, 280: 29.9 / 29.3; 32 heads 248: 32.0 / 32.5, 280: 33.1 / 32.7; 40 heads 248:
+// 41.7 / 42.2, 280: 42.7 / 42.5. They meet between 210 (16 heads) and 280: 240 is off by at most 4 % of such a layer.
 constexpr int ATT_CLUSTER_POS = 240, ATT_ONE_CTA_CTX = 8192;   // (the score row of the longest context: 40 KB)
 int attention_form(const AttnParams &p, const LaunchCfg &cfg, int pos) {
     if (p.T != 1 || p.seq_stride != 0 || p.n_ctx > ATT_ONE_CTA_CTX || !atl_fits(p, cfg)) { return ATT_BY_CONTEXT; }

@@ -598,6 +598,25 @@ def test_steps_on_both_sides_of_the_attention_switch(n_ctx, oracle, tmp_models):
     m.close(); b.close()
 
 
+@pytest.mark.parametrize("n_ctx", [128, 108])
+def test_steps_of_k_quants_with_heads_beyond_the_free_sms(n_ctx, oracle, tmp_models):
+    """Ten heads: attention CTAs of some start late. With cache rows that begin on lines (128 positions) the older ones are read before the wait for the
+    QKV kernel, else (108) behind it; from the first position on, over the ends of words and of groups of 32."""
+    cfg = gguf_io.LlamaConfig(n_layer=2, d_model=1280, n_head=10, n_ff=512, n_vocab=512, weight_std=0.05, wtype=quants.Q4_K)
+    path = str(tmp_models / "ten_heads.gguf")
+    if not os.path.exists(path):
+        gguf_io.make_llama_gguf(path, cfg, seed=52)
+    prompt = np.array([7])
+    want_ids, want_logits = oracle.OracleLlama(path, n_ctx=n_ctx).generate(prompt, 70)
+    b = B.B200Backend(0)
+    m = B.LlamaModel(b, path, n_ctx=n_ctx)
+    ids, logits = m.generate(prompt, 3)
+    assert np.array_equal(ids, want_ids[:3]) and logits_ok(logits, want_logits[:3])
+    ids, logits = m.decode(int(want_ids[0]), 1, 69, want_logits=True)
+    assert np.array_equal(ids, want_ids[1:]) and logits_ok(logits, want_logits[1:])
+    m.close(); b.close()
+
+
 def test_more_captured_steps_than_are_kept(oracle, tmp_models):
     """18 conversations that cross the attention switch are 36 captured steps, four more than are kept: each turn of the second round finds its
     steps gone and captures them again, the second one while steps are running. Host-driven steps of the same conversations go among them."""
