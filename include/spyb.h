@@ -48,7 +48,7 @@ typedef struct {
     int32_t device_id;     /* CUDA device ordinal */
     int32_t tp_size;       /* tensor-parallel world size, 1 = single GPU */
     int32_t tp_rank;       /* this process's rank in [0, tp_size) */
-    int32_t use_pdl;       /* 1 = programmatic dependent launch between the kernels of a step */
+    int32_t use_pdl;       /* 1 = programmatic dependent launch: kernels of a step and of operators start beside their predecessors */
     int32_t use_graph;     /* 1 = replay decode steps from a captured CUDA graph */
     int32_t reserved;
     uint64_t arena_bytes;  /* size of the device arena behind spyb_alloc, 0 = default (256 MiB) */

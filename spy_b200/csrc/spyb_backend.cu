@@ -546,11 +546,11 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
     const bool kq = type == SPYB_Q4_K || type == SPYB_Q6_K;
     if (type != SPYB_Q4_0 && type != SPYB_Q8_0 && !kq) { return SPYB_UNSUPPORTED; }
     const int64_t k = w.elements[0], n_rows = w.elements[1], T = x.elements[1] * x.elements[2] * x.elements[3];
-    // From five columns on, which are two mat-vec passes. The GEMM is launched ahead of its predecessor's end; the passes are plain launches. Q4_0,
-    // one matrix again and again: 1024 x 8192 x 5 11.3 us against 20.9, 4096 x 11008 x 8 21.0 against 46.4. W_down inside a layer: d = 4096, ff
-    // 11008, eight columns 152 us against 182 for the layer; d = 3072, ff 8192 112 against 130. Only back-to-back submits that walk over more
-    // matrices than the L2 holds see the passes ahead, on low matrices with long rows, whose tiles few SMs fetch (2048 x 8192 x 5: 41.9 against
-    // 29.9; 4096 x 11008 x 8: 57 against 59; 8192 x 4096 x 5: 25 against 31).
+    // From five columns on, which are two mat-vec passes. Submits over more matrices (rows x K) than the L2 holds, us, GEMM / passes at 5, 6 and 8
+    // columns: Q4_0 11008 x 4096 25.2 / 28.7, 25.1 / 32.3, 25.0 / 38.7; 5120 x 13824 43.4 / 50.6, 43.5 / 58.1, 43.3 / 72.1; 4096 x 11008 35.5 / 36.1, 35.5 /
+    // 41.2, 35.5 / 50.2; 4096 x 4096 17.0 / 15.7, 17.0 / 17.5, 17.0 / 20.9. The passes are ahead on few rows of long K, whose tiles few SMs walk:
+    // 1024 x 8192 26.4 / 20.6, 26.4 / 21.1, 26.4 / 24.9; and on K-quants, where such a walk is no shared one: Q4_K 4096 x 4096 19.4 / 13.6, 19.5 / 15.0,
+    // 19.4 / 17.8; 4096 x 11008 44.4 / 29.9, 44.4 / 34.1, 44.6 / 42.2; but 11008 x 4096 21.8 / 23.1, 21.8 / 25.8, 21.7 / 31.4.
     if (T < 5 || w.node_type != SPYB_NODE_CONSTANT || k != x.elements[0] || k < QK || k % QK != 0 || k > PF_MAX_K || (kq && k % 256 != 0) ||
         n_rows < 1 || w.elements[2] != 1 || w.elements[3] != 1 || !tensor_contiguous(w) || !tensor_contiguous(x) ||
         (reinterpret_cast<uintptr_t>(x.data) & 15) || (reinterpret_cast<uintptr_t>(out_dev) & 3)) {
@@ -718,7 +718,7 @@ spyb_status run_matmul(spyb_backend *be, spyb_op_desc *d, void *out_dev) {
         p.pro = PRO_QUANT; p.x = static_cast<const float *>(x.data) + t0 * m.k; p.x_stride = m.k;
         p.epi = EPI_STORE; p.out = static_cast<float *>(out_dev) + t0 * m.n_rows; p.out_stride = m.n_rows;
         // A constant's tiles were finished before its upload returned: its kernel may start, and copy its first weights, beside the kernel in
-        // front (5120 x 5120 Q8_0, submits one after the other: 6.48 -> 6.30 us, 11008 x 4096 Q4_K of four columns 15.4 -> 14.5).
+        // front (submits one after the other against one matrix, 5120 x 5120 Q8_0: 6.48 -> 6.30 us; on an idle stream there is nothing to start beside).
         SPYB_CUDA(be, launch_matvec(p, be->launch_cfg(found && be->config.use_pdl != 0)));
     }
     return SPYB_SUCCESS;
