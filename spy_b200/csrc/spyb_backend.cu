@@ -164,7 +164,9 @@ extern "C" {
 
 int32_t spyb_selftest_host(void) {
     const int ledger = smem_ledger_selftest();
-    return ledger != 0 ? ledger : attn_ring_selftest();
+    if (ledger != 0) { return ledger; }
+    const int ring = attn_ring_selftest();
+    return ring != 0 ? ring : prefill_share_selftest();
 }
 
 spyb_status spyb_create(const spyb_config *config, spyb_backend **out) {
@@ -214,6 +216,9 @@ spyb_status spyb_create(const spyb_config *config, spyb_backend **out) {
               cudaMemcpy(be->d_silu_table, silu.data(), 65536 * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(be->d_exp_table, ex.data(), 65536 * 4, cudaMemcpyHostToDevice) == cudaSuccess;
     if (!ok) { spyb_destroy(be); return SPYB_FAIL; }
+    const size_t handoff = (size_t)be->num_sms_total * (PF_HANDOFF_BYTES + PF_HANDOFF_FLAGS * sizeof(unsigned));
+    if (cudaMalloc(&be->pf_handoff, handoff) != cudaSuccess) { cudaGetLastError(); be->pf_handoff = nullptr; }   // (the GEMMs go without)
+    else if (cudaMemset(be->pf_handoff, 0, handoff) != cudaSuccess) { spyb_destroy(be); return SPYB_FAIL; }
     be->cb_thread = std::thread(callback_worker, be);
     *out = be;
     return SPYB_SUCCESS;
@@ -229,6 +234,7 @@ void spyb_destroy(spyb_backend *be) {
         be->cb_thread.join();
     }
     for (void *p : be->owned) { cudaFree(p); }
+    if (be->pf_handoff) { cudaFree(be->pf_handoff); }
     if (be->d_silu_table) { cudaFree(be->d_silu_table); }
     if (be->d_exp_table) { cudaFree(be->d_exp_table); }
     if (be->h_error_flag) { cudaFreeHost(be->h_error_flag); }
@@ -451,7 +457,7 @@ spyb_status spyb_prefill_matmul_form(spyb_backend *be, int32_t weight_type, cons
     if (err == cudaSuccess) {
         PrefillGemm g;
         g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.tile_tok = tile_tok; g.split = tile_ctas; g.T = T; g.out = out; g.out_stride = n_rows;
-        g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
+        be->prefill_shared(g);
         err = launch_prefill_gemm(g, be->stream);
     }
     if (err == cudaSuccess) { err = cudaMemcpyAsync(out_host, out, (size_t)T * n_rows * 4, cudaMemcpyDeviceToHost, be->stream); }
@@ -597,7 +603,7 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
         SPYB_CUDA(be, launch_prefill_quant(static_cast<const float *>(x.data) + t0 * k, k, Tc, (int)k, nullptr, 0.f, static_cast<uint8_t *>(yq), be->stream, type, g.tile_tok, 0, 0, pdl));
         g.w = tiles; g.type = type; g.n_rows = n_rows; g.nb = nb; g.yq = static_cast<uint8_t *>(yq); g.T = Tc;
         g.out = static_cast<float *>(out_dev) + t0 * n_rows; g.out_stride = n_rows;
-        g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
+        be->prefill_shared(g);
         SPYB_CUDA(be, launch_prefill_gemm(g, be->stream, pdl));
     }
     return SPYB_SUCCESS;

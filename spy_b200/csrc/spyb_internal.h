@@ -73,6 +73,7 @@ struct spyb_backend {
     spyb::Arena  arena;
     int         *h_error_flag = nullptr;   // mapped pinned word the kernels set when a bounded wait runs out
     int         *d_error_flag = nullptr;   // its device address
+    void        *pf_handoff = nullptr;     // prompt GEMMs, one after the other on the stream: PrefillGemm::handoff, and behind it the flags
     uint8_t     *noalloc_scratch = nullptr; // device address of the scratch array of spyb_matmul_noalloc (looked up once)
     float       *d_silu_table = nullptr;   // 65536 entries: xh / (1 + expf(-xh)) for the fp16 value xh
     float       *d_exp_table = nullptr;    // 65536 entries: expf(xh)
@@ -115,6 +116,11 @@ struct spyb_backend {
             return true;
         }
         return false;
+    }
+    void prefill_shared(spyb::PrefillGemm &g) const {   // what every prompt GEMM on this backend's stream has in common
+        g.error_flag = d_error_flag; g.wait_limit_ns = wait_limit_ns;
+        g.handoff = pf_handoff;
+        if (pf_handoff != nullptr) { g.handoff_flags = reinterpret_cast<unsigned *>(static_cast<uint8_t *>(pf_handoff) + (size_t)num_sms_total * spyb::PF_HANDOFF_BYTES); }
     }
     spyb::LaunchCfg launch_cfg(bool pdl) const {
         spyb::LaunchCfg c; c.stream = stream; c.pdl = pdl; c.num_sms = num_sms; c.mv_ctas_per_sm = mv_ctas_per_sm;

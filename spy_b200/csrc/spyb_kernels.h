@@ -117,6 +117,9 @@ constexpr int PF_WTILE_F16 = 128 * 32 * 2 + 128 * 4;            // Q4_0 / Q8_0: 
 constexpr int PF_KQ_TOK_MAX = 64;                               // K-quant kernels: the widest token tile
 constexpr int PF_KQ_WTILE = 128 * 32 * 2 + 128 * 8;             // the f16 A operand of a 32-element block, then two f32 scale products per row
 constexpr int PF_MAX_K = 14336;   // widest activation row the quantizer kernel holds in registers
+constexpr size_t PF_HANDOFF_BYTES = 65536;   // 128 rows x 16 tokens x 8 accumulators
+constexpr int    PF_HANDOFF_FLAGS = 16;      // one word per epilogue warp
+struct PfShare { int rounds, len, rem; uint64_t magic; };   // whole rounds of tiles; steps of the rest that every walker takes (rem of them one more); 2^32 / steps of a tile, rounded up
 struct PrefillGemm {
     const uint8_t *w = nullptr;       // [n_rows / PF_ROWS][nb] weight tiles (launch_prefill_retile)
     int            type = 0;          // 2 = Q4_0, 8 = Q8_0, 12 = Q4_K, 14 = Q6_K
@@ -129,6 +132,9 @@ struct PrefillGemm {
     float         *out = nullptr;     // [T][out_stride]
     int64_t        out_stride = 0;
     const float   *resid = nullptr;   // optional [T][out_stride]: out = W x + resid (may alias out)
+    PfShare        share = {};                // set by the launch
+    void          *handoff = nullptr;         // PF_HANDOFF_BYTES per SM for accumulators that one CTA begins and another finishes; null: every tile is one CTA's
+    unsigned      *handoff_flags = nullptr;   // sixteen words per SM, zero between launches
     int           *error_flag = nullptr;
     uint64_t       wait_limit_ns = 1000000000ull;
     int            selftest_skip_step = -1;   // failure-path check: the copy warp leaves this step out, so the waits for it run out
@@ -136,6 +142,7 @@ struct PrefillGemm {
 int         device_sms();         // SMs of the current device
 int         prefill_tile_tokens(int type, int64_t n_rows, int nb, int T);   // width of the token tiles for this matrix and number of tokens
 void        prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split);   // host-only: the Q4_0 / Q8_0 kernel's form on a device of so many SMs
+int         prefill_share_selftest();   // host-only: the cuts of shared tiles; 0 when they hold
 size_t      prefill_weight_bytes(int type, int64_t n_rows, int nb);
 size_t      prefill_act_bytes(int T, int nb);
 cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);

@@ -558,7 +558,7 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
         }
         PrefillGemm g;
         g.w = W.w; g.type = W.type; g.n_rows = W.n_rows; g.nb = K / 32; g.yq = m->pf_yq; g.tile_tok = yq_src.tile_tok; g.T = T; g.out = out; g.out_stride = out_stride; g.resid = resid;
-        g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
+        be->prefill_shared(g);
         return launch_prefill_gemm(g, s, pdl);
     };
     // Tensor parallel: every matrix is split by output rows - this rank's heads, FFN rows, and a slice of the rows of W_o and
@@ -1460,7 +1460,7 @@ spyb_status spyb_model_decode_batch(spyb_model *m, const int32_t *first_tokens, 
                 const bool pdl = be->config.use_pdl != 0;
                 PrefillGemm g;
                 g.w = m->pf_head.w; g.type = m->pf_head.type; g.n_rows = V; g.nb = d / 32; g.yq = m->pf_yq; g.tile_tok = prefill_tile_tokens(g.type, V, d / 32, n_seq);
-                g.T = n_seq; g.out = m->logits_batch; g.out_stride = V; g.error_flag = be->d_error_flag; g.wait_limit_ns = be->wait_limit_ns;
+                g.T = n_seq; g.out = m->logits_batch; g.out_stride = V; be->prefill_shared(g);
                 SPYB_CUDA(be, launch_prefill_quant(m->pf_x, dp, n_seq, d, m->output_norm, m->info.rms_eps, m->pf_yq, be->stream, g.type, g.tile_tok, dp, (int64_t)n_seq * dp, pdl));
                 SPYB_CUDA(be, launch_prefill_gemm(g, be->stream, pdl));
                 launches += 2;

@@ -24,6 +24,7 @@
 
 #include <algorithm>
 #include <type_traits>
+#include <vector>
 
 namespace spyb {
 
@@ -57,14 +58,16 @@ constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF
 // scales lie between the halves) for four chains of twice the blocks per step, and at the end of a tile the second CTA's epilogue warps leave their sums in
 // the first one's shared memory, where they are added in the tree's order. 4096 x 11008 x 8 tokens 52 -> 32.5 us, 4096 x 4096 x 8 20.8 -> 15.1.
 // Where the tiles fill the chip it costs more (a scale product for every four FMAs, the scales twice): prefill_tile_tokens has the line.
-template <int TT, int S> struct PfGeom {
+template <int TT, int S, bool MANY> struct PfGeom {
     static constexpr int NB     = 32 * S / TT;                            // blocks per step
     static constexpr int YB     = TT * 64 + TT * 4;                       // a block's compact activations: TT x 32 f16, TT f32 scales
     static constexpr int HS     = 2 / S;                                  // halves of a block that a CTA takes
     static constexpr int WB     = HS * PF_HALF + 512;                     // a block's weights: its halves, the scales (between them, so that both lie beside either)
     static constexpr int RAW    = NB * (WB + YB);                         // a step as it arrives
     static constexpr int STAGE  = RAW + 8192;                             // ... and its B operands
-    static constexpr int NS     = TT == 16 ? 6 : 4;                       // steps in the ring (even)
+    // steps in the ring (even). Few tokens of wide tiles wait for weights: eight steps, 22016 x 4096 x 32 tokens 63.4 -> 57.9 us, 15360 x 5120 x 32 57.6 ->
+    // 53.2. Many tokens find them in L2: 4096 x 4096 x 448 126.0 with six, 127.8 with eight; 4096 x 11008 x 448 327.7 / 320.8; 22016 x 4096 x 448 640 / 648.
+    static constexpr int NS     = TT == 16 ? (S == 1 && !MANY ? 8 : 6) : 4;
     static constexpr int PW     = TT / 8;                                 // token pairs per epilogue warp
     static constexpr int PC     = PW < 2 ? 1 : 2;                         // pairs per chunk of tensor-memory columns (8 columns each)
     static constexpr int NC     = NB * HS * (PW / PC);                    // chunks per step and warp
@@ -74,9 +77,90 @@ template <int TT, int S> struct PfGeom {
     static constexpr size_t SMEM = (size_t)BARS + 8 * N_BAR + 16;
 };
 
-template <int TT, int S, bool MANY>
+
+// The epilogue's loop over the steps of 16-token tiles, two a turn (D buffers 0 and 1), as one piece of PTX: the accumulators stay where they are. The same
+// loop in C++ is at the mercy of what surrounds it: its accumulators are given other registers from copy to copy of the step, and some ten moves
+// per step and warp bring them back (12288 x 4096 x 448 tokens, shared tiles: 412 us; as PTX 366).
+// A step's chunks are 16 columns of D, half a block's sums of the warp's four tokens; the second block's are requested under the folds of
+// the first one's. (Each chunk requested, waited for and folded in turn: 401 us where this takes 381; one chunk ahead 426, its registers spill.)
+// Operands: %0-%15 accumulators [pair][4 half + n], %16 tensor-memory address, %17 limit (ns), %18 stage offset, %19 parity, %20 turns; %21, %22 addresses of the
+// row's and the tokens' scales in stage 0, %23 d_full(0), %24 lane; %25 bytes of a stage, %26 of the ring, %27 of a block's weights, %28 of its activations.
+#define PF_FMA(A, SC, X, Y) "mov.b64 t, {" X ", " Y "};\n\tfma.rn.f32x2 %" A ", " SC ", t, %" A ";\n\t"
+#define PF_FOLD(R, A0, A1, A2, A3, A4, A5, A6, A7) PF_FMA(A0, "s0", R "0", R "1") PF_FMA(A1, "s0", R "2", R "3") PF_FMA(A2, "s0", R "4", R "5") PF_FMA(A3, "s0", R "6", R "7") \
+    PF_FMA(A4, "s1", R "8", R "9") PF_FMA(A5, "s1", R "10", R "11") PF_FMA(A6, "s1", R "12", R "13") PF_FMA(A7, "s1", R "14", R "15")
+#define PF_FOLD_FIRST(R)  PF_FOLD(R, "0", "1", "2", "3", "8", "9", "10", "11")
+#define PF_FOLD_SECOND(R) PF_FOLD(R, "4", "5", "6", "7", "12", "13", "14", "15")
+#define PF_READ(R, COL) "add.u32 a, %16, " COL ";\n\ttcgen05.ld.sync.aligned.32x32b.x16.b32 {" R "0," R "1," R "2," R "3," R "4," R "5," R "6," R "7," R "8," R "9," R "10," R "11," R "12," R "13," R "14," R "15}, [a];\n\t"
+#define PF_READ_WAIT "tcgen05.wait::ld.sync.aligned;\n\t"
+#define PF_SCALES(W, Y) "add.u32 a, %21, %18;\n\tld.shared.f32 dw, [a+" W "];\n\tadd.u32 a, %22, %18;\n\tld.shared.v2.b64 {x0, x1}, [a+" Y "];\n\t"
+#define PF_PRODUCTS "mov.b64 t, {dw, dw};\n\tmul.rn.f32x2 s0, t, x0;\n\tmul.rn.f32x2 s1, t, x1;\n\t"
+#define PF_D_FULL(OFF, L) "mbarrier.try_wait.parity.shared::cta.b64 p, [%23+" OFF "], %19;\n\t@p bra D" L "_%=;\n\tmov.u64 t0, %%globaltimer;\nA" L "_%=:\n\t" \
+    "mbarrier.try_wait.parity.shared::cta.b64 p, [%23+" OFF "], %19;\n\t@p bra D" L "_%=;\n\tmov.u64 t1, %%globaltimer;\n\tsub.u64 t1, t1, t0;\n\tsetp.lt.u64 q, t1, %17;\n\t@q bra A" L "_%=;\n\tmov.u64 %17, 0;\nD" L "_%=:\n\ttcgen05.fence::after_thread_sync;\n\t"
+#define PF_D_FREE(OFF) "tcgen05.fence::before_thread_sync;\n\tbar.warp.sync 0xffffffff;\n\t@lead mbarrier.arrive.shared::cta.b64 _, [%23+" OFF "];\n\t"
+#define PF_STEP(C0, C1, C2, C3, FULL, FREE, L) PF_D_FULL(FULL, L) \
+    PF_READ("r", C0) PF_READ("u", C1) PF_SCALES("0", "0") PF_PRODUCTS PF_READ_WAIT PF_FOLD_FIRST("r") PF_READ("r", C2) PF_SCALES("%27", "%28") PF_FOLD_SECOND("u") PF_PRODUCTS \
+    PF_READ("u", C3) PF_READ_WAIT PF_D_FREE(FREE) PF_FOLD_FIRST("r") PF_FOLD_SECOND("u") "add.u32 %18, %18, %25;\n\t"
+template <class G>
+__device__ __forceinline__ void pf_fold_steps(uint64_t (&acc)[2][8], int turns, uint32_t tbase, uint32_t dw_addr, uint32_t dx_addr, uint32_t d_bars, int lane, uint32_t &stage, uint32_t &par, uint64_t &limit_ns) {
+    static_assert(G::NB == 2 && G::HS == 2 && G::PW == 2 && G::NS % 2 == 0, "16 tokens, whole blocks");
+    asm volatile("{\n\t.reg .b32 r<16>, u<16>, a;\n\t.reg .f32 dw;\n\t.reg .b64 t, x0, x1, s0, s1, t0, t1;\n\t.reg .pred p, q, lead;\n\tsetp.eq.u32 lead, %24, 0;\nLOOP_%=:\n\t"
+                 PF_STEP("0", "64", "128", "192", "0", "16", "0") PF_STEP("256", "320", "384", "448", "8", "24", "1")
+                 "setp.eq.u32 p, %18, %26;\n\t@p mov.u32 %18, 0;\n\txor.b32 %19, %19, 1;\n\tsub.u32 %20, %20, 1;\n\tsetp.ne.u32 p, %20, 0;\n\t@p bra LOOP_%=;\n\t}"
+                 : "+l"(acc[0][0]), "+l"(acc[0][1]), "+l"(acc[0][2]), "+l"(acc[0][3]), "+l"(acc[0][4]), "+l"(acc[0][5]), "+l"(acc[0][6]), "+l"(acc[0][7]),
+                   "+l"(acc[1][0]), "+l"(acc[1][1]), "+l"(acc[1][2]), "+l"(acc[1][3]), "+l"(acc[1][4]), "+l"(acc[1][5]), "+l"(acc[1][6]), "+l"(acc[1][7]),
+                   "+r"(tbase), "+l"(limit_ns), "+r"(stage), "+r"(par), "+r"(turns)
+                 : "r"(dw_addr), "r"(dx_addr), "r"(d_bars), "r"(lane), "n"(G::STAGE), "n"(G::NS * G::STAGE), "n"(G::WB), "n"(G::YB) : "memory");
+}
+#undef PF_FMA
+#undef PF_FOLD
+#undef PF_FOLD_FIRST
+#undef PF_FOLD_SECOND
+#undef PF_READ
+#undef PF_READ_WAIT
+#undef PF_SCALES
+#undef PF_PRODUCTS
+#undef PF_D_FULL
+#undef PF_D_FREE
+#undef PF_STEP
+
+// SHARE: the tiles are no whole number of rounds, and what is left after all rounds but one - one to two tiles a walker (CTA or cluster) - is laid end
+// to end and cut into equal stretches, one a walker, from the last one down. A tile on a cut is two walkers': the lower one takes its first
+// steps before the rest of its stretch and leaves the accumulators in the handoff buffer, the higher one takes the last steps at the end of
+// its own. Whoever waits thus waits for a CTA that was started before itself, and for steps that were done by then if all walk at one pace
+// (a stretch is at least a tile long). Whole rounds come first, in step: walkers that are beside each other then read the same weights at the same time.
+// Whole tiles / shared, us with the quantizer: 4096 x 4096 x 448 tokens (6.05 rounds) 142.5 / 126, 5120 x 13824 x 32 (1.08 rounds of clusters) 73.3 / 54, 12288
+// x 4096 x 32 (1.30 rounds) 45.8 / 37; 488 sizes: 6 % on average. What a cut costs, 2.5 to 5.7 us, is in best_form. Whole rounds keep a kernel of their own,
+// whose registers do not suffer from the handing over.
+struct PfItem { int tile, from, to, q; };   // steps [from, to) of a tile: a walker's item q
+__host__ __device__ __forceinline__ PfItem pf_share_item(const PfShare &h, int n_tile, int n_step, int walker, int walkers, int q) {
+    const int base = h.rounds * walkers, r = walkers - 1 - walker;
+    const int lo = r * h.len + (r < h.rem ? r : h.rem), hi = lo + h.len + (r < h.rem ? 1 : 0);   // (a stretch is at least a tile long)
+    const int t0 = (int)(((uint64_t)lo * h.magic) >> 32), x0 = lo - t0 * n_step, t1 = (int)(((uint64_t)hi * h.magic) >> 32), x1 = hi - t1 * n_step;
+    const int early = x0 != 0 ? 1 : 0, mid = q - h.rounds - early, n_mid = t1 - t0 - early;
+    if (q < h.rounds) { return {walker + q * walkers, 0, n_step, q}; }
+    if (mid < 0) { return {base + t0, 0, n_step - x0, q}; }
+    if (mid < n_mid) { return {base + t0 + early + mid, 0, n_step, q}; }
+    return {mid == n_mid && x1 != 0 ? base + t1 : n_tile, n_step - x1, n_step, q};
+}
+inline PfShare pf_share(int n_tile, int n_step, int walkers) {   // n_tile > walkers
+    const int rounds = n_tile / walkers - 1, steps = (n_tile - rounds * walkers) * n_step;
+    return {rounds, steps / walkers, steps % walkers, (0x100000000ull + n_step - 1) / n_step};
+}
+// the word that says that a warp's accumulators lie in the handoff buffer; only the walker they are meant for clears it again
+__device__ __forceinline__ void handoff_publish(unsigned *flag) { asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory"); }
+__device__ __forceinline__ void handoff_wait(const unsigned *flag, uint64_t &limit_ns) {
+    const uint64_t t0 = global_timer_ns();
+    for (;;) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+        if (__all_sync(0xffffffffu, v != 0u)) { return; }
+        if (__any_sync(0xffffffffu, global_timer_ns() - t0 >= limit_ns)) { limit_ns = 0; return; }
+    }
+}
+
+template <int TT, int S, bool MANY, bool SHARE>
 __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(PrefillGemm g) {
-    using G = PfGeom<TT, S>;
+    using G = PfGeom<TT, S, MANY>;
     constexpr int NB = G::NB, NS = G::NS, PW = G::PW, PC = G::PC, YB = G::YB, HS = G::HS, WB = G::WB;
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem), bars = sbase + G::BARS;
@@ -121,6 +205,17 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    const int walker = (int)blockIdx.x / S;
+    const int total_steps = SHARE ? g.share.rounds * n_step + g.share.len + ((int)gridDim.x / S - 1 - walker < g.share.rem ? 1 : 0) : (g.share.rounds + (walker < g.share.rem ? 1 : 0)) * n_step;
+    auto first_item = [&]() -> PfItem {
+        if constexpr (SHARE) { return pf_share_item(g.share, n_tile, n_step, (int)blockIdx.x / S, (int)gridDim.x / S, 0); }
+        return {(int)blockIdx.x / S, 0, n_step, 0};
+    };
+    auto next_item = [&](PfItem &it) {
+        if constexpr (SHARE) { it = pf_share_item(g.share, n_tile, n_step, (int)blockIdx.x / S, (int)gridDim.x / S, it.q + 1); }
+        else { it.tile += gridDim.x / S; }
+    };
+
     // CTAs that run together take neighbouring token tiles of the same rows: a weight tile crosses HBM once
     if (warp >= PF_GEMM_EPI_WARPS) {
         uint64_t left_ns = limit;   // (zero once a wait has run out)
@@ -130,7 +225,8 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             uint32_t par = 1;
             bool ok = true;
             // the weights of the first tile's first steps, then (the previous kernel is done) their activations with all that follows
-            const int early = blockIdx.x / S < n_tile ? min(NS, n_step) : 0;
+            const PfItem first = first_item();
+            const int early = first.tile < n_tile ? min(NS, first.to - first.from) : 0;
             // n blocks of weights at `w` into stage st
             auto copy_weights = [&](int st, const uint8_t *w, int n) {
                 const uint32_t dst = sbase + (uint32_t)st * G::STAGE;
@@ -151,17 +247,17 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             if (elect_one()) {
                 for (int i = 0; i < early; ++i) {
                     if (i == g.selftest_skip_step) { continue; }
-                    const int n = min(NB, nb - i * NB);
+                    const int n = min(NB, nb - (first.from + i) * NB);
                     mbar_expect_tx(raw_full(i), (uint32_t)(n * (WB + YB)));
-                    copy_weights(i, g.w + ((int64_t)(blockIdx.x / S / n_tok) * nb + i * NB) * PF_WTILE_F16, n);
+                    copy_weights(i, g.w + ((int64_t)(first.tile / n_tok) * nb + (first.from + i) * NB) * PF_WTILE_F16, n);
                 }
             }
             __syncwarp();
             pdl_wait();
-            for (int tile = blockIdx.x / S; tile < n_tile && ok; tile += gridDim.x / S) {
-                const uint8_t *wsrc = g.w + (int64_t)(tile / n_tok) * nb * PF_WTILE_F16;
-                const uint8_t *ysrc = g.yq + (int64_t)(tile % n_tok) * nb * YB;
-                for (int i = 0; i < n_step; ++i, ++k) {
+            for (PfItem it = first; it.tile < n_tile && ok; next_item(it)) {
+                const uint8_t *wsrc = g.w + ((int64_t)(it.tile / n_tok) * nb + it.from * NB) * PF_WTILE_F16;
+                const uint8_t *ysrc = g.yq + ((int64_t)(it.tile % n_tok) * nb + it.from * NB) * YB;
+                for (int i = it.from; i < it.to; ++i, ++k) {
                     if (k >= NS) {
                         ok = __all_sync(0xffffffffu, mbar_wait_relaxed(st_free(st), par, limit));
                         if (!ok) { break; }
@@ -196,25 +292,23 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             const int h = S == 2 ? 0 : (lane >> 1) & 1, np = lane & 1, t0 = S == 2 ? lane >> 1 : lane >> 2;
             const uint32_t dst_lane = (uint32_t)((S == 2 ? (t0 / TT) * 128 * TT : 0) + h * 128 * TT + np * (64 * TT + 64) + ((S == 2 ? t0 % TT : t0) >> 1) * 128 + (t0 & 1) * 16);
             const uint32_t src_lane = (uint32_t)(S == 2 ? (t0 / TT) * YB + (t0 % TT) * 64 + rank * 32 + np * 16 : lane * 16);
-            for (int tile = blockIdx.x / S; tile < n_tile && left_ns != 0; tile += gridDim.x / S) {
-                for (int i = 0; i < n_step; ++i) {
-                    mbar_wait_lean(raw_full(st), par, left_ns);
-                    if (left_ns == 0) { break; }
-                    const uint32_t base = sbase + (uint32_t)st * G::STAGE, src = base + NB * WB + src_lane, dst = base + G::RAW + dst_lane;
-                    uint4 v[4];
+            for (int k = 0; k < total_steps; ++k) {
+                mbar_wait_lean(raw_full(st), par, left_ns);
+                if (left_ns == 0) { break; }
+                const uint32_t base = sbase + (uint32_t)st * G::STAGE, src = base + NB * WB + src_lane, dst = base + G::RAW + dst_lane;
+                uint4 v[4];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) { v[k] = lds128(src + (uint32_t)((k * TK / TT) * YB + (k * TK % TT) * 64)); }   // all loads in flight before the first store
+                for (int k = 0; k < 4; ++k) { v[k] = lds128(src + (uint32_t)((k * TK / TT) * YB + (k * TK % TT) * 64)); }   // all loads in flight before the first store
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const uint32_t d = dst + (uint32_t)((k * TK / TT) * HS * 128 * TT + (k * TK % TT) * 64);
-                        sts64(d, v[k].x, v[k].y);
-                        sts64(d + 40u, v[k].z, v[k].w);
-                    }
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) { mbar_arrive(ops_full(st)); }
-                    if (++st == NS) { st = 0; par ^= 1u; }
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t d = dst + (uint32_t)((k * TK / TT) * HS * 128 * TT + (k * TK % TT) * 64);
+                    sts64(d, v[k].x, v[k].y);
+                    sts64(d + 40u, v[k].z, v[k].w);
                 }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) { mbar_arrive(ops_full(st)); }
+                if (++st == NS) { st = 0; par ^= 1u; }
             }
             if (left_ns == 0 && lane == 0) { pf_report(g.error_flag, 4); }
         } else {
@@ -224,35 +318,33 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             const uint32_t d0 = tmem + (uint32_t)m * 256u;
             int st = 0, k = 0, mine = 0;
             uint32_t par = 0;
-            for (int tile = blockIdx.x / S; tile < n_tile && left_ns != 0; tile += gridDim.x / S) {
-                for (int i = 0; i < n_step; ++i, ++k) {
-                    if ((k & 1) == m) {
-                        mbar_wait_lean(ops_full(st), par, left_ns);
-                        mbar_wait_lean(d_free(m), (uint32_t)mine & 1u, left_ns);
-                        if (left_ns == 0) { break; }
-                        if (mine > 0 && lane == 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }   // (the step before on this buffer has been read)
-                        tc_fence_after();
-                        const uint32_t base = sbase + (uint32_t)st * G::STAGE;
-                        const uint64_t a0 = operand_desc(base + (uint32_t)rank * 512u, 2048u, 128u), b0 = operand_desc(base + G::RAW, 64u * TT, 128u);
-                        const int n = min(NB, nb - i * NB);
-                        if (elect_one()) {
+            for (; k < total_steps; ++k) {
+                if ((k & 1) == m) {
+                    mbar_wait_lean(ops_full(st), par, left_ns);
+                    mbar_wait_lean(d_free(m), (uint32_t)mine & 1u, left_ns);
+                    if (left_ns == 0) { break; }
+                    // (the step before on this buffer has been read. One CTA a tile: by the thread that issues, which is the quicker way to the MMAs and makes
+                    // 448 tokens 5 % faster; with two CTAs, which wait for their weights, 2 % are the other way)
+                    if (S == 2 && mine > 0 && lane == 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }
+                    tc_fence_after();
+                    const uint32_t base = sbase + (uint32_t)st * G::STAGE;
+                    const uint64_t a0 = operand_desc(base + (uint32_t)rank * 512u, 2048u, 128u), b0 = operand_desc(base + G::RAW, 64u * TT, 128u);
+                    if (elect_one()) {
+                        if (S == 1 && mine > 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }
 #pragma unroll
-                            for (int j = 0; j < NB; ++j) {
-                                if (j < n) {
+                        for (int j = 0; j < NB; ++j) {   // (blocks past the end of a row are multiplied too, whatever lies there: nobody folds them)
 #pragma unroll
-                                    for (int h = 0; h < HS; ++h) {
-                                        mma_f16_ss(d0 + (uint32_t)((j * HS + h) * 4 * TT), a0 + (uint64_t)((j * WB + h * (PF_HALF + 512)) >> 4), b0 + (uint64_t)(((j * HS + h) * 128 * TT) >> 4),
-                                                   idesc_f16(4 * TT), 0u);
-                                    }
-                                }
+                            for (int h = 0; h < HS; ++h) {
+                                mma_f16_ss(d0 + (uint32_t)((j * HS + h) * 4 * TT), a0 + (uint64_t)((j * WB + h * (PF_HALF + 512)) >> 4), b0 + (uint64_t)(((j * HS + h) * 128 * TT) >> 4),
+                                           idesc_f16(4 * TT), 0u);
                             }
-                            mma_commit(d_full(m));
                         }
-                        __syncwarp();
-                        ++mine;
+                        mma_commit(d_full(m));
                     }
-                    if (++st == NS) { st = 0; par ^= 1u; }
+                    __syncwarp();
+                    ++mine;
                 }
+                if (++st == NS) { st = 0; par ^= 1u; }
             }
             if (left_ns == 0 && lane == 0) { pf_report(g.error_flag, 5); }
             // every MMA has completed (it reads shared memory and writes tensor memory) before the CTA leaves
@@ -316,21 +408,50 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
         };
         using B0 = std::integral_constant<int, 0>;
         using B1 = std::integral_constant<int, 1>;
-        const int n_full = nb / NB, rest = nb % NB;
+        const int rest = nb % NB;
         uint32_t x_par = 0;      // phase of the hand-over between the CTAs of a cluster
-        bool odd = false;        // a tile with an odd number of steps leaves the next one starting on buffer 1
-        for (int tile = blockIdx.x / S; tile < n_tile; tile += gridDim.x / S) {
+        bool odd = false;        // an item with an odd number of steps leaves the next one starting on buffer 1
+        [[maybe_unused]] bool joined = false;   // (S = 2) a tile's halves have been joined already
+        for (PfItem it = first_item(); it.tile < n_tile; next_item(it)) {
+            const int n_full = SHARE ? min(it.to, nb / NB) - it.from : nb / NB;
+            const int tile = it.tile;
+            if constexpr (SHARE) if (it.from > 0) {   // another walker's accumulators
+                const int64_t at = (int64_t)((int)blockIdx.x - S) * PF_GEMM_EPI_WARPS + warp;
+                handoff_wait(g.handoff_flags + at, left_ns);
+#pragma unroll
+                for (int n = 0; n < 4 * HS * PW; ++n) { acc[n / (4 * HS)][n % (4 * HS)] = __ldcg(reinterpret_cast<const unsigned long long *>(g.handoff) + (at * 16 + n) * 32 + lane); }
+                __syncwarp();
+                if (lane == 0) { g.handoff_flags[at] = 0u; }
+            }
             int i = 0;
             if (odd && n_full > 0) { step(B1{}, NB); i = 1; }
+            if constexpr (TT == 16 && S == 1) {
+                const int turns = (n_full - i) >> 1;
+                if (turns > 0) { pf_fold_steps<G>(acc, turns, tbase, dw_addr, dx_addr, d_full(0), lane, stage, par, left_ns); }
+                i += 2 * turns;
+            } else {
 #pragma unroll 1
-            for (; i + 2 <= n_full; i += 2) { step(B0{}, NB); step(B1{}, NB); }
+                for (; i + 2 <= n_full; i += 2) { step(B0{}, NB); step(B1{}, NB); }
+            }
             bool second = odd && n_full == 0;
             if (i < n_full) { step(B0{}, NB); second = true; }
-            if (rest != 0) {
+            if (rest != 0 && (!SHARE || it.to == n_step)) {
                 if (second) { step(B1{}, rest); } else { step(B0{}, rest); }
                 second = !second;
             }
             odd = second;
+            if constexpr (SHARE) if (it.to < n_step) {   // another walker goes on with these accumulators
+                const int64_t at = (int64_t)blockIdx.x * PF_GEMM_EPI_WARPS + warp;
+#pragma unroll
+                for (int n = 0; n < 4 * HS * PW; ++n) {
+                    uint64_t &a = acc[n / (4 * HS)][n % (4 * HS)];
+                    __stcg(reinterpret_cast<unsigned long long *>(g.handoff) + (at * 16 + n) * 32 + lane, (unsigned long long)a);
+                    a = 0ull;
+                }
+                __syncwarp();
+                if (lane == 0) { handoff_publish(g.handoff_flags + at); }
+                continue;
+            }
             // hsum_float_8 (vec_util.h:74-81): accumulator n of a half is CPU accumulator 4 + n / n (Q4_0: low / high nibbles) or n / 4 + n
             // (Q8_0); either way the tree is (c0 + c4) + (c2 + c6) and (c1 + c5) + (c3 + c7)
             const int64_t orow = (int64_t)(tile / n_tok) * PF_M + row;
@@ -338,7 +459,8 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             if constexpr (S == 2) {   // the second half's accumulators are those of the same thread of the cluster's other CTA
                 const uint32_t xch = sbase + (uint32_t)(NS * G::STAGE) + 8u * (uint32_t)tid;
                 if (rank == 1) {
-                    if (tile != blockIdx.x / S) { cluster_wait(x_free(warp), x_par ^ 1u, left_ns); }   // (the tile before has been read)
+                    if (SHARE ? joined : tile != blockIdx.x / S) { cluster_wait(x_free(warp), x_par ^ 1u, left_ns); }   // (the tile before has been read)
+                    joined = true;
                     const uint32_t to = cluster_map(xch, 0);
 #pragma unroll
                     for (int i = 0; i < 4 * PW; ++i) { cluster_store64(to + (uint32_t)(i * PF_GEMM_EPI_WARPS * 32 * 8), acc[i >> 2][i & 3]); }
@@ -577,22 +699,25 @@ __global__ void prefill_silu_mul_kernel(const float *upgate, int T, int F, const
     act[i] = __fmul_rn(up, silu_table[f2h(gate)]);
 }
 
-template <int TT, int S, bool MANY = false>
+template <int TT, int S, bool MANY = false, bool SHARE = false>
 cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
-    const void *kernel = reinterpret_cast<const void *>(prefill_gemm_kernel<TT, S, MANY>);
-    const size_t smem = PfGeom<TT, S>::SMEM;
+    const void *kernel = reinterpret_cast<const void *>(prefill_gemm_kernel<TT, S, MANY, SHARE>);
+    const size_t smem = PfGeom<TT, S, MANY>::SMEM;
     cudaError_t err = allow_dynamic_smem(kernel, smem);
     if (err != cudaSuccess) { return err; }
-    const int64_t tiles = (int64_t)((g.T + TT - 1) / TT) * ((g.n_rows + PF_M - 1) / PF_M);
+    const int64_t tiles = (int64_t)((g.T + TT - 1) / TT) * ((g.n_rows + PF_M - 1) / PF_M), walkers = std::min<int64_t>(tiles, device_sms() / S);
+    PrefillGemm h = g;
+    h.share = {(int)(tiles / walkers), 0, (int)(tiles % walkers), 0};
+    if (SHARE) { h.share = pf_share((int)tiles, (g.nb + PfGeom<TT, S, MANY>::NB - 1) / PfGeom<TT, S, MANY>::NB, (int)walkers); }
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)(S * std::min<int64_t>(tiles, device_sms() / S))); lc.blockDim = dim3(PF_GEMM_THREADS); lc.dynamicSmemBytes = smem; lc.stream = stream;
+    lc.gridDim = dim3((unsigned)(S * walkers)); lc.blockDim = dim3(PF_GEMM_THREADS); lc.dynamicSmemBytes = smem; lc.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = S; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     lc.attrs = attr; lc.numAttrs = S > 1 ? 2 : 1;
-    void *args[] = {const_cast<PrefillGemm *>(&g)};
+    void *args[] = {&h};
     return cudaLaunchKernelExC(&lc, kernel, args);
 }
 
@@ -610,29 +735,65 @@ int device_sms() {
 }
 
 // The form of the Q4_0 / Q8_0 kernel for a matrix and a number of tokens: tiles of 16 or of 8 tokens, by one CTA each or by a cluster of
-// two; the one whose cost is least. CTAs or clusters walk the tiles in rounds: a launch costs what fills its pipelines, a round what a tile does
-// once (its drain, and for two CTAs the joining of the halves) and a time for each block of the row (less for narrow tiles, whose weights bound
-// them, and about half for two CTAs), and every block of the matrix some time for its bytes, in proportion to the chip. Fitted to 1450 sizes, ten
-// matrices of models and 1330 drawn ones from 1024 x 1024 to 32000 x 14336, with 5 to 512 tokens: within 3 % of the fastest form but at 8 of them (4 to
-// 13 %). (A cost of blocks and launches alone, fitted to the models' matrices, is off by 3 to 25 % at 55 of them, mostly rows of 1300 to 3000 values.)
-// us with the activations' quantizer, one CTA / two: 4096 x 4096 x 8 tokens 18.1 / 15.2, 4096 x 11008 x 16 54.7 / 34.9; and 1680 x 2208 x 79 tokens
-// 13.3 / 16.2, 22148 x 1728 x 5 17.0 / 20.1, 22016 x 4096 x 448 655 / 826.
-struct PfForm { int tok, split; double launch_ns, tile_ns, block_ns, rows_ns; };
-static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int sms) {   // tok 0: of either width
-    static constexpr PfForm FORMS[4] = {{16, 1, 5480, 1140, 144.6, 23.7}, {8, 1, 3010, 130, 124.2, 56.9}, {16, 2, 9920, 980, 84.3, 4.0}, {8, 2, 5520, 800, 68.3, 38.1}};
+// two, the last ones whole or shared; the one whose cost is least. CTAs or clusters walk the tiles in rounds: a launch costs what fills its
+// pipelines, a round what a tile does once (its drain, and for two CTAs the joining of the halves) and a time for each block of the row (less
+// for narrow tiles, whose weights bound them, and about half for two CTAs), and every block of the matrix some time for its bytes, in
+// proportion to the chip. Shared tiles make the rounds a fraction, for the handing over and, for two CTAs, slower blocks; they are taken for a gain of
+// 2 % and 1 us, because the SMs that a last whole round leaves idle already copy the next GEMM's first weights (32000 x 4096 x 16, one submit after the other:
+// whole 44.5 us, shared 48.7). Fitted to 488 sizes, ten matrices of models and 70 drawn ones from 1024 x 1024 to 32000 x 14336, with 5 to 512 tokens: the rule's
+// choice is 0.3 % behind the fastest on average, more than 3 % behind it at 19 of them (3900 x 7136 x 38 tokens 10 %, 7980 x 2208 x 11 8 %). us with the activations'
+// quantizer, one CTA / two: 4096 x 4096 x 8 tokens 18.1 / 15.2, 4096 x 11008 x 16 54.7 / 34.9; and 1680 x 2208 x 79 tokens 13.3 / 16.2, 22016 x 4096 x 448
+// 655 / 826; whole / shared tiles: 14968 x 1088 x 22 19.5 / 21.8, and the sizes above.
+struct PfForm { int tok, split; double launch_ns, tile_ns, block_ns, rows_ns, handoff_ns, slower; };
+static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int split, int sms, bool *share) {   // tok, split 0: any
+    static constexpr PfForm FORMS[4] = {{16, 1, 4240, 730, 149.9, 28.3, 5720, -0.025}, {8, 1, 3210, 0, 119.2, 87.6, 2510, 0.019},
+                                        {16, 2, 5790, 1740, 84.5, 22.0, 5320, 0.065}, {8, 2, 5250, 1070, 65.1, 68.1, 3790, 0.020}};
     PfForm best = {};
     double best_ns = 0.0;
     for (const PfForm &f : FORMS) {
-        if (tok != 0 && tok != f.tok) { continue; }
-        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, tiles = row_tiles * ((T + f.tok - 1) / f.tok), walks = std::max(1, sms / f.split);
-        const double ns = f.launch_ns + (double)((tiles + walks - 1) / walks) * (f.tile_ns + nb * f.block_ns) + (double)row_tiles / sms * nb * f.rows_ns;
-        if (best.tok == 0 || ns < best_ns) { best = f; best_ns = ns; }
+        if ((tok != 0 && tok != f.tok) || (split != 0 && split != f.split)) { continue; }
+        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, tiles = row_tiles * ((T + f.tok - 1) / f.tok), walkers = std::max(1, sms / f.split);
+        const double once = f.launch_ns + (double)row_tiles / sms * nb * f.rows_ns;
+        double ns = once + (double)((tiles + walkers - 1) / walkers) * (f.tile_ns + nb * f.block_ns);
+        bool shared = false;
+        if (tiles > walkers && tiles % walkers != 0) {
+            const double ns_shared = 1000.0 + 1.02 * (once + f.handoff_ns + (double)tiles / walkers * (f.tile_ns + nb * f.block_ns * (1.0 + f.slower)));
+            if (ns_shared < ns) { ns = ns_shared; shared = true; }
+        }
+        if (best.tok == 0 || ns < best_ns) { best = f; best_ns = ns; *share = shared; }
     }
     return best;
 }
 void prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split) {
-    const PfForm f = best_form(n_rows, nb, T, 0, sms);
+    bool share;
+    const PfForm f = best_form(n_rows, nb, T, 0, 0, sms, &share);
     *tile_tok = f.tok; *split = f.split;
+}
+// host-only check of the shared tiles: every step of every tile is some walker's exactly once, and a tile's first steps are the lower neighbour's of the
+// walker that goes on with it, and done by the time it does
+int prefill_share_selftest() {
+    for (int walkers : {2, 3, 74, 148}) {
+        for (int n_step : {1, 2, 3, 7, 64, 65, 172, 448}) {
+            for (int n_tile = walkers + 1; n_tile < 4 * walkers; n_tile += 1 + walkers / 20) {
+                if (n_tile % walkers == 0) { continue; }
+                const PfShare h = pf_share(n_tile, n_step, walkers);
+                std::vector<int> begun(n_tile, 0), begun_by(n_tile, -1), begun_at(n_tile, 0), done(n_tile, 0);
+                for (int w = 0; w < walkers; ++w) {
+                    int at = 0;
+                    for (PfItem it = pf_share_item(h, n_tile, n_step, w, walkers, 0); it.tile < n_tile; it = pf_share_item(h, n_tile, n_step, w, walkers, it.q + 1)) {
+                        if (it.tile < 0 || it.from < 0 || it.from >= it.to || it.to > n_step) { return 101; }
+                        if (it.from > 0 && (begun[it.tile] != it.from || begun_by[it.tile] != w - 1 || begun_at[it.tile] > at)) { return 102; }
+                        at += it.to - it.from;
+                        done[it.tile] += it.to - it.from;
+                        if (it.to < n_step) { begun[it.tile] = it.to; begun_by[it.tile] = w; begun_at[it.tile] = at; }
+                    }
+                    if (at != h.rounds * n_step + h.len + (walkers - 1 - w < h.rem ? 1 : 0)) { return 103; }
+                }
+                for (int t = 0; t < n_tile; ++t) { if (done[t] != n_step) { return 104; } }
+            }
+        }
+    }
+    return 0;
 }
 int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T) {
     if (type == 12 || type == 14) {   // K-quants: a tile of 16, 32, 64 tokens costs 1 : 1.35 : 2.3 (measured: the narrow ones are mostly weights)
@@ -641,7 +802,8 @@ int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T) {
         const double c16 = (double)rounds(16), c32 = 1.35 * (double)rounds(32), c64 = 2.3 * (double)rounds(64);
         return c16 <= c32 && c16 <= c64 ? 16 : c32 <= c64 ? 32 : 64;
     }
-    return best_form(n_rows, nb, T, 0, device_sms()).tok;
+    bool share;
+    return best_form(n_rows, nb, T, 0, 0, device_sms(), &share).tok;
 }
 
 size_t prefill_weight_bytes(int type, int64_t n_rows, int nb) {
@@ -685,12 +847,18 @@ cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool 
     if (g.type == 12 || g.type == 14) { return launch_prefill_gemm_kq(g, stream, pdl); }
     if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
     if ((g.tile_tok != 16 && g.tile_tok != 8) || g.split < 0 || g.split > 2) { return cudaErrorInvalidValue; }
-    const bool pair = (g.split != 0 ? g.split : best_form(g.n_rows, g.nb, g.T, g.tile_tok, device_sms()).split) == 2;
+    bool share = false;
+    const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok, g.split, device_sms(), &share).split == 2;
+    share = share && g.handoff != nullptr;
     // Many tokens (MANY): the epilogue is the bound and the weights come out of L2; copies of half a block are in its way for less long.
     // 22016 x 4096 x 448 tokens 659 us with one copy a step, 649 by blocks, 642 by halves, 646 by quarters. Where the weights' way
     // through HBM is the bound one copy is better: 4096 x 11008 x 64 tokens 55.8 us, by halves 56.2.
     const bool many = g.T > 64;
-    if (g.tile_tok == 8) { return pair ? launch_gemm_t<8, 2>(g, stream, pdl) : launch_gemm_t<8, 1>(g, stream, pdl); }
+    if (g.tile_tok == 8) {
+        if (share) { return pair ? launch_gemm_t<8, 2, false, true>(g, stream, pdl) : launch_gemm_t<8, 1, false, true>(g, stream, pdl); }
+        return pair ? launch_gemm_t<8, 2>(g, stream, pdl) : launch_gemm_t<8, 1>(g, stream, pdl);
+    }
+    if (share) { return pair ? launch_gemm_t<16, 2, false, true>(g, stream, pdl) : many ? launch_gemm_t<16, 1, true, true>(g, stream, pdl) : launch_gemm_t<16, 1, false, true>(g, stream, pdl); }
     return pair ? launch_gemm_t<16, 2>(g, stream, pdl) : many ? launch_gemm_t<16, 1, true>(g, stream, pdl) : launch_gemm_t<16, 1>(g, stream, pdl);
 }
 

@@ -176,6 +176,21 @@ def test_prefill_matmul_shared_by_two_ctas(be, oracle, qt, n, k, t):
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), form
 
 
+@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
+@pytest.mark.parametrize("n,k,t", [(9604, 4128, 32), (2564, 4128, 118), (6148, 2080, 130), (19204, 1568, 36)])
+def test_prefill_matmul_shares_its_last_tiles(be, oracle, qt, n, k, t):
+    """One to four rounds and a fraction of tiles in every form: the last tiles are cut between neighbours at odd and even steps, rows end inside a step, and
+    calls follow one another (what one leaves in the buffer of the handing over, the next one does not find)."""
+    rng = np.random.default_rng(n + k + t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    rows = np.unique(np.r_[np.arange(0, n, 128), n - 1, rng.integers(0, n, 60)])
+    want = oracle.matmul(qt, np.ascontiguousarray(w[rows]), k, len(rows), x)
+    for form in [(16, 1), (8, 1), (16, 2), (8, 2), (0, 0), (16, 1)]:
+        got = be.prefill_matmul(qt, w, n, k, x, form=form)
+        assert np.array_equal(got[:, rows].view(np.uint32), want.view(np.uint32)), form
+
+
 @pytest.mark.parametrize("qt,k", [(quants.Q4_0, 2272), (quants.Q4_0, 4128), (quants.Q8_0, 8192), (quants.Q4_0, 8224), (quants.Q4_K, 4352), (quants.Q4_K, 9216),
                                   (quants.Q8_0, 13824), (quants.Q4_0, 14336), (quants.Q4_K, 13824), (quants.Q6_K, 14336)])
 def test_prefill_quantizer_of_normed_rows(be, oracle, qt, k):
