@@ -57,7 +57,7 @@ constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF
 // of them read the first 16 values of every block and four the others, so each CTA streams and multiplies one half of the weights (the
 // scales lie between the halves) for four chains of twice the blocks per step, and at the end of a tile the second CTA's epilogue warps leave their sums in
 // the first one's shared memory, where they are added in the tree's order. 4096 x 11008 x 8 tokens 52 -> 32.5 us, 4096 x 4096 x 8 20.8 -> 15.1.
-// Where the tiles fill the chip it costs more (a scale product for every four FMAs, the scales twice): prefill_tile_tokens has the line.
+// Where the tiles fill the chip it costs more (a scale product for every four FMAs, the scales twice): best_form has the line.
 template <int TT, int S, bool MANY> struct PfGeom {
     static constexpr int NB     = 32 * S / TT;                            // blocks per step
     static constexpr int YB     = TT * 64 + TT * 4;                       // a block's compact activations: TT x 32 f16, TT f32 scales
@@ -123,41 +123,7 @@ __device__ __forceinline__ void pf_fold_steps(uint64_t (&acc)[2][8], int turns, 
 #undef PF_D_FREE
 #undef PF_STEP
 
-// SHARE: the tiles are no whole number of rounds, and what is left after all rounds but one - one to two tiles a walker (CTA or cluster) - is laid end
-// to end and cut into equal stretches, one a walker, from the last one down. A tile on a cut is two walkers': the lower one takes its first
-// steps before the rest of its stretch and leaves the accumulators in the handoff buffer, the higher one takes the last steps at the end of
-// its own. Whoever waits thus waits for a CTA that was started before itself, and for steps that were done by then if all walk at one pace
-// (a stretch is at least a tile long). Whole rounds come first, in step: walkers that are beside each other then read the same weights at the same time.
-// Whole tiles / shared, us with the quantizer: 4096 x 4096 x 448 tokens (6.05 rounds) 142.5 / 126, 5120 x 13824 x 32 (1.08 rounds of clusters) 73.3 / 54, 12288
-// x 4096 x 32 (1.30 rounds) 45.8 / 37; 488 sizes: 6 % on average. What a cut costs, 2.5 to 5.7 us, is in best_form. Whole rounds keep a kernel of their own,
-// whose registers do not suffer from the handing over.
-struct PfItem { int tile, from, to, q; };   // steps [from, to) of a tile: a walker's item q
-__host__ __device__ __forceinline__ PfItem pf_share_item(const PfShare &h, int n_tile, int n_step, int walker, int walkers, int q) {
-    const int base = h.rounds * walkers, r = walkers - 1 - walker;
-    const int lo = r * h.len + (r < h.rem ? r : h.rem), hi = lo + h.len + (r < h.rem ? 1 : 0);   // (a stretch is at least a tile long)
-    const int t0 = (int)(((uint64_t)lo * h.magic) >> 32), x0 = lo - t0 * n_step, t1 = (int)(((uint64_t)hi * h.magic) >> 32), x1 = hi - t1 * n_step;
-    const int early = x0 != 0 ? 1 : 0, mid = q - h.rounds - early, n_mid = t1 - t0 - early;
-    if (q < h.rounds) { return {walker + q * walkers, 0, n_step, q}; }
-    if (mid < 0) { return {base + t0, 0, n_step - x0, q}; }
-    if (mid < n_mid) { return {base + t0 + early + mid, 0, n_step, q}; }
-    return {mid == n_mid && x1 != 0 ? base + t1 : n_tile, n_step - x1, n_step, q};
-}
-inline PfShare pf_share(int n_tile, int n_step, int walkers) {   // n_tile > walkers
-    const int rounds = n_tile / walkers - 1, steps = (n_tile - rounds * walkers) * n_step;
-    return {rounds, steps / walkers, steps % walkers, (0x100000000ull + n_step - 1) / n_step};
-}
-// the word that says that a warp's accumulators lie in the handoff buffer; only the walker they are meant for clears it again
-__device__ __forceinline__ void handoff_publish(unsigned *flag) { asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory"); }
-__device__ __forceinline__ void handoff_wait(const unsigned *flag, uint64_t &limit_ns) {
-    const uint64_t t0 = global_timer_ns();
-    for (;;) {
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-        if (__all_sync(0xffffffffu, v != 0u)) { return; }
-        if (__any_sync(0xffffffffu, global_timer_ns() - t0 >= limit_ns)) { limit_ns = 0; return; }
-    }
-}
-
+// SHARE: the last tiles are cut among the CTAs or clusters (PfItem in spyb_tc.cuh)
 template <int TT, int S, bool MANY, bool SHARE>
 __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(PrefillGemm g) {
     using G = PfGeom<TT, S, MANY>;
@@ -796,13 +762,8 @@ int prefill_share_selftest() {
     return 0;
 }
 int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T) {
-    if (type == 12 || type == 14) {   // K-quants: a tile of 16, 32, 64 tokens costs 1 : 1.35 : 2.3 (measured: the narrow ones are mostly weights)
-        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, sms = device_sms();
-        auto rounds = [&](int tt) { return (row_tiles * ((T + tt - 1) / tt) + sms - 1) / sms; };
-        const double c16 = (double)rounds(16), c32 = 1.35 * (double)rounds(32), c64 = 2.3 * (double)rounds(64);
-        return c16 <= c32 && c16 <= c64 ? 16 : c32 <= c64 ? 32 : 64;
-    }
     bool share;
+    if (type == 12 || type == 14) { return prefill_kq_tile_tokens(n_rows, nb, T, 0, device_sms(), &share); }
     return best_form(n_rows, nb, T, 0, 0, device_sms(), &share).tok;
 }
 

@@ -18,6 +18,7 @@
 #include "spyb_tc.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace spyb {
 
@@ -30,7 +31,7 @@ constexpr int KQ_EPI_WARPS = 16, KQ_GEMM_THREADS = 608;   // sixteen epilogue wa
 //
 // Bound of the wide tile: issue slots. Per (row, token, block) two multiplications and two FMAs, packed two tokens at a time, and eight
 // uniform 128-bit shared-memory reads of the token scales per 16 tokens.
-// Q4_K_M, 8 layers, 512 tokens: 9.6 ms in all (one 64-token tile per CTA with 8-bit operands: 14.3); 4 layers, 16 tokens: 0.86 (2.43).
+// Q4_K_M, 8 layers, 512 tokens: 8.2 ms in all (whole tiles only: 8.7; one 64-token tile per CTA with 8-bit operands: 14.3); 4 layers, 16 tokens: 0.86 (2.43).
 template <int TT> struct KqGeom {
     static constexpr int NB    = TT == 64 ? 2 : 4;            // blocks per step
     static constexpr int YB    = TT * 72;                     // a block's activations: TT x 32 f16, TT scales, TT sums
@@ -49,7 +50,7 @@ template <int N> __device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint3
     if constexpr (N == 16) { tmem_ld16(taddr, r); } else if constexpr (N == 8) { tmem_ld8(taddr, r); } else { tmem_ld4(taddr, r); }
 }
 
-template <int WT, int TT>   // WT: 12 = Q4_K, 14 = Q6_K
+template <int WT, int TT, bool SHARE>   // WT: 12 = Q4_K, 14 = Q6_K; SHARE: the last tiles are cut among the CTAs, between super-blocks (PfItem)
 __global__ void __launch_bounds__(KQ_GEMM_THREADS, 1) prefill_kq_gemm_kernel(PrefillGemm g) {
     using G = KqGeom<TT>;
     constexpr int NB = G::NB, NS = G::NS, PW = G::PW, YB = G::YB, H = WT == 14 ? 2 : 1, TW = TT / 4;   // H sums per (row, token, block), TW tokens per epilogue warp
@@ -64,10 +65,20 @@ __global__ void __launch_bounds__(KQ_GEMM_THREADS, 1) prefill_kq_gemm_kernel(Pre
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + (size_t)NS * G::STAGE + 8 * (2 * NS + 4));
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int nb = g.nb, n_step = nb / NB;                                      // (nb is a multiple of 8)
+    const int nb = g.nb;                                                        // (a multiple of 8)
     const int n_tok = (g.T + TT - 1) / TT;
     const int n_tile = n_tok * (int)((g.n_rows + PF_M - 1) / PF_M);
     const uint64_t limit = g.wait_limit_ns;
+    constexpr int SB = 8 / NB;                                                  // steps of a super-block
+    const int n_super = nb / 8;
+    auto first_item = [&]() -> PfItem {
+        if constexpr (SHARE) { return pf_share_item(g.share, n_tile, n_super, (int)blockIdx.x, (int)gridDim.x, 0); }
+        return {(int)blockIdx.x, 0, n_super, 0};
+    };
+    auto next_item = [&](PfItem &it) {
+        if constexpr (SHARE) { it = pf_share_item(g.share, n_tile, n_super, (int)blockIdx.x, (int)gridDim.x, it.q + 1); }
+        else { it.tile += gridDim.x; }
+    };
 
     pdl_launch_dependents();
     if (tid == 0) {
@@ -91,19 +102,20 @@ __global__ void __launch_bounds__(KQ_GEMM_THREADS, 1) prefill_kq_gemm_kernel(Pre
         int st = 0, k = 0, issued = 0;
         uint32_t par = 1;
         bool ok = true;
-        const int early = blockIdx.x < n_tile ? min(NS, n_step) : 0;
+        const PfItem first = first_item();
+        const int early = first.tile < n_tile ? min(NS, (first.to - first.from) * SB) : 0;
         if (elect_one()) {
             for (int i = 0; i < early; ++i) {
                 mbar_expect_tx(raw_full(i), (uint32_t)G::STAGE);
-                bulk_copy_g2s(sbase + (uint32_t)i * G::STAGE, g.w + ((int64_t)(blockIdx.x / n_tok) * nb + i * NB) * KQ_WT, (uint32_t)(NB * KQ_WT), raw_full(i));
+                bulk_copy_g2s(sbase + (uint32_t)i * G::STAGE, g.w + ((int64_t)(first.tile / n_tok) * nb + first.from * 8 + i * NB) * KQ_WT, (uint32_t)(NB * KQ_WT), raw_full(i));
             }
         }
         __syncwarp();
         pdl_wait();
-        for (int tile = blockIdx.x; tile < n_tile && ok; tile += gridDim.x) {
-            const uint8_t *wsrc = g.w + (int64_t)(tile / n_tok) * nb * KQ_WT;
-            const uint8_t *ysrc = g.yq + (int64_t)(tile % n_tok) * nb * YB;
-            for (int i = 0; i < n_step; ++i, ++k) {
+        for (PfItem it = first; it.tile < n_tile && ok; next_item(it)) {
+            const uint8_t *wsrc = g.w + ((int64_t)(it.tile / n_tok) * nb + it.from * 8) * KQ_WT;
+            const uint8_t *ysrc = g.yq + ((int64_t)(it.tile % n_tok) * nb + it.from * 8) * YB;
+            for (int i = it.from * SB; i < it.to * SB; ++i, ++k) {
                 if (k >= NS) {
                     ok = __all_sync(0xffffffffu, mbar_wait_relaxed(st_free(st), par, limit));
                     if (!ok) { break; }
@@ -133,8 +145,8 @@ __global__ void __launch_bounds__(KQ_GEMM_THREADS, 1) prefill_kq_gemm_kernel(Pre
         const uint32_t d0 = tmem + (uint32_t)m * 256u;
         int st = 0, k = 0, mine = 0;
         uint32_t par = 0;
-        for (int tile = blockIdx.x; tile < n_tile && left_ns != 0; tile += gridDim.x) {
-            for (int i = 0; i < n_step; ++i, ++k) {
+        for (PfItem it = first_item(); it.tile < n_tile && left_ns != 0; next_item(it)) {
+            for (int i = it.from * SB; i < it.to * SB; ++i, ++k) {
                 if ((k & 1) == m) {
                     mbar_wait_lean(d_free(m), (uint32_t)mine & 1u, left_ns);
                     if (left_ns != 0 && mine > 0 && lane == 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }   // (the step before on this buffer has been read)
@@ -175,9 +187,18 @@ __global__ void __launch_bounds__(KQ_GEMM_THREADS, 1) prefill_kq_gemm_kernel(Pre
         for (int u = 0; u < PW; ++u) { acc[u] = 0ull; tot[u] = 0ull; }
         if (lane == 0) { mbar_arrive(d_free(0)); mbar_arrive(d_free(1)); }
         int st = 0, k = 0;
-        for (int tile = blockIdx.x; tile < n_tile; tile += gridDim.x) {
+        for (PfItem it = first_item(); it.tile < n_tile; next_item(it)) {
+            const int tile = it.tile;
+            if constexpr (SHARE) if (it.from > 0) {   // the sums of the super-blocks in front are another CTA's
+                const int64_t at = (int64_t)((int)blockIdx.x - 1) * KQ_EPI_WARPS + warp;
+                handoff_wait(g.handoff_flags + at, left_ns);
+#pragma unroll
+                for (int u = 0; u < PW; ++u) { tot[u] = __ldcg(reinterpret_cast<const unsigned long long *>(g.handoff) + (at * 16 + u) * 32 + lane); }
+                __syncwarp();
+                if (lane == 0) { g.handoff_flags[at] = 0u; }
+            }
 #pragma unroll 1
-            for (int i = 0; i < n_step; ++i, ++k) {
+            for (int i = SHARE ? it.from * SB : 0; i < it.to * SB; ++i, ++k) {
                 const int buf = k & 1;
                 const uint32_t stage = (uint32_t)st * G::STAGE, tb = tbase + (uint32_t)buf * 256u;
                 mbar_wait_lean(d_full(buf), (uint32_t)(k >> 1) & 1u, left_ns);
@@ -217,6 +238,14 @@ __global__ void __launch_bounds__(KQ_GEMM_THREADS, 1) prefill_kq_gemm_kernel(Pre
                     for (int u = 0; u < PW; ++u) { tot[u] = f2_add(tot[u], acc[u]); acc[u] = 0ull; }
                 }
                 if (++st == NS) { st = 0; }
+            }
+            if constexpr (SHARE) if (it.to < n_super) {   // another CTA goes on with these sums
+                const int64_t at = (int64_t)blockIdx.x * KQ_EPI_WARPS + warp;
+#pragma unroll
+                for (int u = 0; u < PW; ++u) { __stcg(reinterpret_cast<unsigned long long *>(g.handoff) + (at * 16 + u) * 32 + lane, (unsigned long long)tot[u]); tot[u] = 0ull; }
+                __syncwarp();
+                if (lane == 0) { handoff_publish(g.handoff_flags + at); }
+                continue;
             }
             const int64_t orow = (int64_t)(tile / n_tok) * PF_M + row;
             const int     tok0 = (tile % n_tok) * TT + part * TW;
@@ -303,23 +332,57 @@ __global__ void prefill_kq_retile_kernel(const uint8_t *raw, int64_t row_stride,
     }
 }
 
-template <int WT, int TT>
+template <int WT, int TT, bool SHARE>
 cudaError_t launch_kq_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     const size_t smem = KqGeom<TT>::SMEM;
-    cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(prefill_kq_gemm_kernel<WT, TT>), smem);
+    cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(prefill_kq_gemm_kernel<WT, TT, SHARE>), smem);
     if (err != cudaSuccess) { return err; }
-    const int64_t tiles = (int64_t)((g.T + TT - 1) / TT) * ((g.n_rows + PF_M - 1) / PF_M);
-    return launch_maybe_pdl(prefill_kq_gemm_kernel<WT, TT>, dim3((unsigned)std::min<int64_t>(tiles, device_sms())), KQ_GEMM_THREADS, smem, stream, pdl, g);
+    const int64_t tiles = (int64_t)((g.T + TT - 1) / TT) * ((g.n_rows + PF_M - 1) / PF_M), walkers = std::min<int64_t>(tiles, device_sms());
+    PrefillGemm h = g;
+    h.share = {(int)(tiles / walkers), 0, (int)(tiles % walkers), 0};
+    if (SHARE) { h.share = pf_share((int)tiles, g.nb / 8, (int)walkers); }
+    return launch_maybe_pdl(prefill_kq_gemm_kernel<WT, TT, SHARE>, dim3((unsigned)walkers), KQ_GEMM_THREADS, smem, stream, pdl, h);
 }
 
 }  // namespace
 
+// Tokens a tile: 16, 32 or 64 (tok 0: any), and whether the last tiles are shared; by a cost as in best_form of the Q4_0 / Q8_0 kernel, one for both types, so
+// that the matrices of a layer that read the same activations agree on a width. Fitted to 411 sizes of both (1024 x 1024 to 32000 x 14336, 8 to 512 tokens): 4.9 %
+// faster on average than the widths by whole rounds alone, 0.1 % behind the fastest choice, more than 3 % at 6 of them (Q4_K 8696 x 1536 x 82 9 %). us, whole
+// tiles / shared: Q4_K 11008 x 4096 x 64 41.7 / 31.9, 5120 x 5120 x 512 127.8 / 107.8, 4096 x 4096 x 512 78.7 / 72.2; Q6_K 4096 x 11008 x 512 193.9 / 174.4.
+int prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int sms, bool *share) {
+    static constexpr struct { int tok; double launch_ns, tile_ns, block_ns, rows_ns, handoff_ns, slower; } WIDTHS[3] = {
+        {16, 4230, 100, 102.6, 49.7, 3770, 0.0}, {32, 4810, 280, 139.9, 33.1, 3780, -0.009}, {64, 4540, 880, 274.4, 4.3, 5230, -0.018}};
+    int best = 0;
+    double best_ns = 0.0;
+    for (const auto &w : WIDTHS) {
+        if (tok != 0 && tok != w.tok) { continue; }
+        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, tiles = row_tiles * ((T + w.tok - 1) / w.tok);
+        const double once = w.launch_ns + (double)row_tiles / sms * nb * w.rows_ns;
+        double ns = once + (double)((tiles + sms - 1) / sms) * (w.tile_ns + nb * w.block_ns);
+        bool shared = false;
+        if (tiles > sms && tiles % sms != 0 && nb >= 16) {
+            const double ns_shared = 500.0 + 1.01 * (once + w.handoff_ns + (double)tiles / sms * (w.tile_ns + nb * w.block_ns * (1.0 + w.slower)));
+            if (ns_shared < ns) { ns = ns_shared; shared = true; }
+        }
+        if (best == 0 || ns < best_ns) { best = w.tok; best_ns = ns; *share = shared; }
+    }
+    return best;
+}
+
 cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     if (g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 8 || (g.nb & 7) || g.n_rows < 1 || (g.type != 12 && g.type != 14)) { return cudaErrorInvalidValue; }
+    bool share = false;
+    prefill_kq_tile_tokens(g.n_rows, g.nb, g.T, g.tile_tok, device_sms(), &share);
+    auto of_width = [&](auto tt) {
+        constexpr int TT = decltype(tt)::value;
+        if (share && g.handoff != nullptr) { return g.type == 12 ? launch_kq_t<12, TT, true>(g, stream, pdl) : launch_kq_t<14, TT, true>(g, stream, pdl); }
+        return g.type == 12 ? launch_kq_t<12, TT, false>(g, stream, pdl) : launch_kq_t<14, TT, false>(g, stream, pdl);
+    };
     switch (g.tile_tok) {
-    case 64: return g.type == 12 ? launch_kq_t<12, 64>(g, stream, pdl) : launch_kq_t<14, 64>(g, stream, pdl);
-    case 32: return g.type == 12 ? launch_kq_t<12, 32>(g, stream, pdl) : launch_kq_t<14, 32>(g, stream, pdl);
-    case 16: return g.type == 12 ? launch_kq_t<12, 16>(g, stream, pdl) : launch_kq_t<14, 16>(g, stream, pdl);
+    case 64: return of_width(std::integral_constant<int, 64>{});
+    case 32: return of_width(std::integral_constant<int, 32>{});
+    case 16: return of_width(std::integral_constant<int, 16>{});
     default: return cudaErrorInvalidValue;
     }
 }

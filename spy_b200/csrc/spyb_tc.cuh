@@ -91,5 +91,40 @@ __device__ __forceinline__ void pf_report(int *error_flag, int code) {
     if (error_flag != nullptr) { atomicExch(error_flag, code); }
 }
 
+// Shared tiles: where the tiles are no whole number of rounds, what is left after all rounds but one - one to two tiles a walker (CTA or cluster) - is laid end
+// to end and cut into equal stretches, one a walker, from the last one down. A tile on a cut is two walkers': the lower one takes its first
+// steps before the rest of its stretch and leaves the accumulators in the handoff buffer, the higher one takes the last steps at the end of
+// its own. Whoever waits thus waits for a CTA that was started before itself, and for steps that were done by then if all walk at one pace
+// (a stretch is at least a tile long). Whole rounds come first, in step: walkers that are beside each other then read the same weights at the same time.
+// Whole tiles / shared, us with the quantizer: 4096 x 4096 x 448 tokens (6.05 rounds) 142.5 / 126, 5120 x 13824 x 32 (1.08 rounds of clusters) 73.3 / 54, 12288
+// x 4096 x 32 (1.30 rounds) 45.8 / 37; 488 sizes: 6 % on average. What a cut costs, 2.5 to 5.7 us, is in best_form. Whole rounds keep a kernel of their own,
+// whose registers do not suffer from the handing over.
+struct PfItem { int tile, from, to, q; };   // steps (K-quants: super-blocks) [from, to) of a tile: a walker's item q
+__host__ __device__ __forceinline__ PfItem pf_share_item(const PfShare &h, int n_tile, int n_step, int walker, int walkers, int q) {
+    const int base = h.rounds * walkers, r = walkers - 1 - walker;
+    const int lo = r * h.len + (r < h.rem ? r : h.rem), hi = lo + h.len + (r < h.rem ? 1 : 0);   // (a stretch is at least a tile long)
+    const int t0 = (int)(((uint64_t)lo * h.magic) >> 32), x0 = lo - t0 * n_step, t1 = (int)(((uint64_t)hi * h.magic) >> 32), x1 = hi - t1 * n_step;
+    const int early = x0 != 0 ? 1 : 0, mid = q - h.rounds - early, n_mid = t1 - t0 - early;
+    if (q < h.rounds) { return {walker + q * walkers, 0, n_step, q}; }
+    if (mid < 0) { return {base + t0, 0, n_step - x0, q}; }
+    if (mid < n_mid) { return {base + t0 + early + mid, 0, n_step, q}; }
+    return {mid == n_mid && x1 != 0 ? base + t1 : n_tile, n_step - x1, n_step, q};
+}
+inline PfShare pf_share(int n_tile, int n_step, int walkers) {   // n_tile > walkers
+    const int rounds = n_tile / walkers - 1, steps = (n_tile - rounds * walkers) * n_step;
+    return {rounds, steps / walkers, steps % walkers, (0x100000000ull + n_step - 1) / n_step};
+}
+// the word that says that a warp's accumulators lie in the handoff buffer; only the walker they are meant for clears it again
+__device__ __forceinline__ void handoff_publish(unsigned *flag) { asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory"); }
+__device__ __forceinline__ void handoff_wait(const unsigned *flag, uint64_t &limit_ns) {
+    const uint64_t t0 = global_timer_ns();
+    for (;;) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+        if (__all_sync(0xffffffffu, v != 0u)) { return; }
+        if (__any_sync(0xffffffffu, global_timer_ns() - t0 >= limit_ns)) { limit_ns = 0; return; }
+    }
+}
+
 }  // namespace
 }  // namespace spyb

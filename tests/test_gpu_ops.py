@@ -222,6 +222,20 @@ def test_prefill_matmul_k_quants_walk_tiles_of_all_widths(be, oracle, qt, n, k, 
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
+@pytest.mark.parametrize("n,k,t", [(2564, 2304, 490), (9604, 4352, 63), (19204, 2560, 9), (1028, 5632, 600)])
+def test_prefill_matmul_k_quants_share_their_last_tiles(be, oracle, qt, n, k, t):
+    """One to four rounds and a fraction of tiles in every width, cut between neighbours at super-blocks; calls follow one another."""
+    rng = np.random.default_rng(n + k + t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    rows, cols = np.unique(np.r_[np.arange(0, n, 128), n - 1, rng.integers(0, n, 20)]), np.unique(np.r_[np.arange(0, t, 16), t - 1])
+    want = oracle.matmul(qt, np.ascontiguousarray(w[rows]), k, len(rows), x[cols])
+    for form in [(64, 1), (32, 1), (16, 1), (0, 0), (64, 1)]:
+        got = be.prefill_matmul(qt, w, n, k, x, form=form)
+        assert np.array_equal(got[np.ix_(cols, rows)].view(np.uint32), want.view(np.uint32)), form
+
+
+@pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
 @pytest.mark.parametrize("n,k,t,norm", [(128, 256, 1, False), (256, 1024, 70, True), (128, 2048, 64, False), (384, 4096, 129, True), (256, 11008 - 11008 % 256, 33, False)])
 def test_prefill_matmul_k_quants_match_the_restatement(be, oracle, qt, n, k, t, norm):
     """K-quant weights through the tensor-core prompt kernel: 1 to 43 super-blocks, ragged tiles of 64 tokens, with and without
