@@ -151,6 +151,8 @@ cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stri
 // pdl (here and below): launch with the programmatic-stream-serialization attribute; the kernels wait for their predecessor themselves
 cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type, int tile_tok,
                                  int part_len = 0, int64_t part_stride = 0, bool pdl = false, uint8_t *tap = nullptr);   // tap: Q8_0 blocks of token 0, reference layout
+// up * silu(gate) of [T][2 F] and its Q8_0 blocks in one kernel; act [T][F]: also in f32 (null: not wanted)
+cudaError_t launch_prefill_silu_quant(const float *upgate, int T, int F, const float *silu_table, float *act, uint8_t *yq, cudaStream_t stream, int weight_type, int tile_tok, bool pdl);
 int         prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int sms, bool *share);   // host-only: the K-quant kernel's width, and whether its last tiles are shared
 cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream, bool pdl);   // type 12 = Q4_K, 14 = Q6_K (spyb_prefill_kq.cu)
 cudaError_t launch_prefill_retile_kq(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);

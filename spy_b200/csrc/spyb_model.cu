@@ -535,7 +535,8 @@ spyb_status ensure_prefill_buffers(spyb_model *m) {
 //   -> norm + quantize -> up|gate GEMM -> up * silu(gate) -> quantize -> down GEMM + residual
 // with the arithmetic of the five fused kernels of run_layers, so that a prompt gives the same bits on either path.
 // (batch: the T tokens are sequences 0 .. T-1 of a batch in lockstep, each with its own cache, all at position d_pos[0])
-spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool batch = false, bool tap = false) {
+// (keep_act: the last layer's FFN activation is wanted in f32 too)
+spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool batch = false, bool tap = false, bool keep_act = false) {
     spyb_backend *be = m->be;
     cudaStream_t s = be->stream;
     const bool pdl = be->config.use_pdl != 0;
@@ -611,9 +612,16 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
         SPYB_CUDA(be, quant(m->pf_x, dp, d, ly.ffn_norm, ly.pf_ug, (int64_t)T * dp));
         SPYB_CUDA(be, gemm(ly.pf_ug, d, m->pf_ug, 2 * (int64_t)fl, nullptr));
         if (m->kq) { SPYB_CUDA(be, gemm(ly.pf_gate, d, m->pf_ug + fl, 2 * (int64_t)fl, nullptr)); ++*launches; }
-        SPYB_CUDA(be, launch_prefill_silu_mul(m->pf_ug, T, fl, be->d_silu_table, act_part, s, pdl));
-        if (gather(m->pf_act, fl) != SPYB_SUCCESS) { return SPYB_FAIL; }
-        SPYB_CUDA(be, quant(m->pf_act, fl, ff, nullptr, ly.pf_down, (int64_t)T * fl));
+        if (tp == 1) {
+            const int tile_tok = prefill_tile_tokens(ly.pf_down.type, ly.pf_down.n_rows, ff / 32, T);
+            yq_src = {nullptr, ff, nullptr, ff, 0, ly.pf_down.type, tile_tok};
+            SPYB_CUDA(be, launch_prefill_silu_quant(m->pf_ug, T, ff, be->d_silu_table, keep_act && &ly == &m->layers.back() ? m->pf_act : nullptr, m->pf_yq, s, ly.pf_down.type, tile_tok, pdl));
+            --*launches;
+        } else {
+            SPYB_CUDA(be, launch_prefill_silu_mul(m->pf_ug, T, fl, be->d_silu_table, act_part, s, pdl));
+            if (gather(m->pf_act, fl) != SPYB_SUCCESS) { return SPYB_FAIL; }
+            SPYB_CUDA(be, quant(m->pf_act, fl, ff, nullptr, ly.pf_down, (int64_t)T * fl));
+        }
         SPYB_CUDA(be, gemm(ly.pf_down, ff, x_part, dp, x_part));
         if (gather(m->pf_x, dp) != SPYB_SUCCESS) { return SPYB_FAIL; }
         *launches += 7;
@@ -1183,7 +1191,7 @@ spyb_status spyb_model_eval(spyb_model *m, const int32_t *tokens, int32_t n_toke
                                                     cudaMemcpyDeviceToDevice, be->stream));
                 }
             }
-            if (run_prefill_layers(m, T, &launches, false, small) != SPYB_SUCCESS) { return SPYB_FAIL; }
+            if (run_prefill_layers(m, T, &launches, false, small, small) != SPYB_SUCCESS) { return SPYB_FAIL; }
             if (small) {   // the last mat-vec pass would have held tokens l0 .. n_tokens - 1
                 const int l0 = (n_tokens - 1) / tmax * tmax, n = n_tokens - l0, ff = m->info.n_ff;
                 PrefillKeep k;

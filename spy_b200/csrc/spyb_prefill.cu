@@ -482,9 +482,12 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
 // SM. us with the norm, one thread's sum / this: 8 tokens x 5120 9.8 / 7.4, 32 x 5120 9.6 / 7.0, 448 x 4096 26.5 / 10.7.
 // KQ false (Q4_0 / Q8_0 weights): [token][32 values as f16], the scales. KQ true: the f16 B operand itself (16 bytes of eight values of a token at
 // (value / 8) * 16 TOKT + 16 token), the scales, the blocks' integer sums as floats.
-template <bool NORM, bool KQ, int PG>
+// SILU: a token's row is [K up | K gate] as the stacked GEMM leaves it, and what is quantized is up * silu(gate) (model/src/llm/plugin/ffn.cpp:28-35),
+// which goes to act only where somebody wants it. (As two kernels, 512 x 11008: 27 + 14 us, 90 MB; this 21 us, 46 MB.)
+template <bool NORM, bool KQ, int PG, bool SILU>
 __global__ void __launch_bounds__(PF_QUANT_THREADS, PG <= 2 ? 2 : 1) prefill_quant_kernel(const float *x, int64_t x_stride, int K, const float *norm_w, float eps, uint8_t *yq,
-                                                                         int TOKT, int part_len, int64_t part_stride, uint8_t *tap) {
+                                                                         int TOKT, int part_len, int64_t part_stride, uint8_t *tap, const float *silu_table, float *act) {
+    static_assert(!(NORM && SILU), "");
     const int SCALES = TOKT * 64;                         // offset of the scales inside a block's record
     const int YQB = SCALES + TOKT * (KQ ? 8 : 4);
     extern __shared__ __align__(16) float v3[];
@@ -514,7 +517,18 @@ __global__ void __launch_bounds__(PF_QUANT_THREADS, PG <= 2 ? 2 : 1) prefill_qua
     for (int k = 0; k < PG; ++k) {
         const int gi = tid + k * PF_QUANT_THREADS;
         if (k < npass && gi < n8) {
-            if (part_len == K) { load8_cg(xrow + 8 * gi, xv[k]); }
+            if (SILU) {
+                float gate[8];
+                load8_cg(xrow + 8 * gi, xv[k]);
+                load8_cg(xrow + K + 8 * gi, gate);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { xv[k][i] = __fmul_rn(xv[k][i], silu_table[f2h(gate[i])]); }
+                if (act != nullptr) {
+                    float4 *to = reinterpret_cast<float4 *>(act + (int64_t)token * K + 8 * gi);
+                    to[0] = make_float4(xv[k][0], xv[k][1], xv[k][2], xv[k][3]); to[1] = make_float4(xv[k][4], xv[k][5], xv[k][6], xv[k][7]);
+                }
+            }
+            else if (part_len == K) { load8_cg(xrow + 8 * gi, xv[k]); }
             else {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
@@ -627,30 +641,50 @@ __global__ void prefill_retile_kernel(const uint8_t *raw, int64_t row_stride, in
 }
 
 // RoPE(Q, K) + fp16 stores of Q / K / V after the QKV GEMM (the arithmetic of the mat-vec epilogue EPI_QKV_ROPE:
-// backend/host/operator/non-linear.cpp:270-371, view.cpp:163-191). One thread per pair of neighbouring elements.
-__global__ void prefill_qkv_post_kernel(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,
-                                        __half *v_cache, int n_ctx, int64_t seq_stride) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t per_token = 3 * (int64_t)dl / 2;
+// backend/host/operator/non-linear.cpp:270-371, view.cpp:163-191). The first qk_blocks blocks rotate, a thread per pair of neighbouring elements of a
+// token; the others turn 64 elements x 32 tokens of V over in shared memory, because the cache holds a row per element: a warp then writes
+// 32 neighbouring positions of a row, 64 bytes, where a thread per element wrote two bytes into a line of its own (512 tokens x 12288: 31.5 us,
+// 7 now; 38 MB). A batch in lockstep (seq_stride > 0: token t is sequence t, with its own cache) has nothing to turn over: a thread per element.
+constexpr int PF_POST_THREADS = 256, PF_POST_E = 64, PF_POST_T = 32;
+__global__ void __launch_bounds__(PF_POST_THREADS) prefill_qkv_post_kernel(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,
+                                        __half *v_cache, int n_ctx, int64_t seq_stride, int qk_blocks) {
+    __shared__ __half vt[PF_POST_T][PF_POST_E + 2];
     pdl_launch_dependents();
     pdl_wait();
-    if (i >= per_token * T) { return; }
-    const int t = (int)(i / per_token);
-    const int64_t col = 2 * (i - (int64_t)t * per_token);
-    const int sec = (int)(col / dl), e = (int)(col - (int64_t)sec * dl);
-    const int pos = *pos_base + (seq_stride ? 0 : t);   // (seq_stride > 0: token t is sequence t of a batch in lockstep, with its own cache)
-    k_cache += seq_stride ? (int64_t)t * seq_stride : 0; v_cache += seq_stride ? (int64_t)t * seq_stride : 0;
-    const float2 x = *reinterpret_cast<const float2 *>(qkv + (int64_t)t * 3 * dl + col);
-    if (sec == 2) {
-        v_cache[(int64_t)e * n_ctx + pos] = __float2half_rn(x.x);
-        v_cache[(int64_t)(e + 1) * n_ctx + pos] = __float2half_rn(x.y);
+    if ((int)blockIdx.x < qk_blocks) {
+        const int64_t i = (int64_t)blockIdx.x * PF_POST_THREADS + threadIdx.x;
+        if (i >= (int64_t)dl * T) { return; }
+        const int t = (int)(i / dl), col = 2 * (int)(i - (int64_t)t * dl);
+        const bool is_k = col >= dl;
+        const int e = is_k ? col - dl : col, pos = *pos_base + (seq_stride ? 0 : t);
+        const float2 x = *reinterpret_cast<const float2 *>(qkv + (int64_t)t * 3 * dl + col), cs = rope[(int64_t)pos * (hd >> 1) + ((e % hd) >> 1)];
+        const float a0 = __fsub_rn(__fmul_rn(x.x, cs.x), __fmul_rn(x.y, cs.y));
+        const float a1 = __fadd_rn(__fmul_rn(x.x, cs.y), __fmul_rn(x.y, cs.x));
+        __half *dst = is_k ? k_cache + (seq_stride ? (int64_t)t * seq_stride : 0) + (int64_t)pos * dl + e : q_out + (int64_t)t * dl + e;
+        *reinterpret_cast<__half2 *>(dst) = __halves2half2(__float2half_rn(a0), __float2half_rn(a1));
         return;
     }
-    const float2 cs = rope[(int64_t)pos * (hd >> 1) + ((e % hd) >> 1)];
-    const float a0 = __fsub_rn(__fmul_rn(x.x, cs.x), __fmul_rn(x.y, cs.y));
-    const float a1 = __fadd_rn(__fmul_rn(x.x, cs.y), __fmul_rn(x.y, cs.x));
-    __half *dst = (sec == 0) ? q_out + (int64_t)t * dl + e : k_cache + (int64_t)pos * dl + e;
-    *reinterpret_cast<__half2 *>(dst) = __halves2half2(__float2half_rn(a0), __float2half_rn(a1));
+    const int vb = (int)blockIdx.x - qk_blocks;
+    if (seq_stride) {
+        const int64_t i = (int64_t)vb * PF_POST_THREADS + threadIdx.x;
+        if (i >= (int64_t)dl * T) { return; }
+        const int t = (int)(i / dl), e = (int)(i - (int64_t)t * dl);
+        v_cache[(int64_t)t * seq_stride + (int64_t)e * n_ctx + *pos_base] = __float2half_rn(qkv[(int64_t)t * 3 * dl + 2 * dl + e]);
+        return;
+    }
+    const int e_tiles = (dl + PF_POST_E - 1) / PF_POST_E, e0 = vb % e_tiles * PF_POST_E, t0 = vb / e_tiles * PF_POST_T;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int t = w; t < PF_POST_T; t += PF_POST_THREADS / 32) {
+        const int e = e0 + 2 * lane;   // (dl is even: heads are rotated in pairs)
+        if (t0 + t < T && e < dl) {
+            const float2 x = *reinterpret_cast<const float2 *>(qkv + (int64_t)(t0 + t) * 3 * dl + 2 * dl + e);
+            *reinterpret_cast<__half2 *>(&vt[t][2 * lane]) = __halves2half2(__float2half_rn(x.x), __float2half_rn(x.y));
+        }
+    }
+    __syncthreads();
+    if (t0 + lane >= T) { return; }
+    __half *row = v_cache + (int64_t)e0 * n_ctx + *pos_base + t0 + lane;
+    for (int e = w; e < min(PF_POST_E, dl - e0); e += PF_POST_THREADS / 32) { row[(int64_t)e * n_ctx] = vt[lane][e]; }
 }
 
 // up * silu(gate) (model/src/llm/plugin/ffn.cpp:28-35) on the output [T][2 F] of the stacked up|gate GEMM
@@ -787,21 +821,30 @@ cudaError_t launch_prefill_retile(int type, const uint8_t *raw, int64_t row_stri
     return cudaGetLastError();
 }
 
-cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type,
-                                 int tile_tok, int part_len, int64_t part_stride, bool pdl, uint8_t *tap) {
+template <bool SILU>
+static cudaError_t launch_quant_t(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type,
+                                  int tile_tok, int part_len, int64_t part_stride, bool pdl, uint8_t *tap, const float *silu_table, float *act) {
     if (weight_type != 2 && weight_type != 8 && weight_type != 12 && weight_type != 14) { return cudaErrorInvalidValue; }
     if (part_len <= 0) { part_len = K; part_stride = 0; }
     if ((part_len & 3) || (part_stride & 3) || K % part_len != 0) { return cudaErrorInvalidValue; }
-    if (T < 1 || tile_tok < 1 || K < 32 || (K & 31) || K > PF_MAX_K || (x_stride & 3) || ((uintptr_t)x & 15)) { return cudaErrorInvalidValue; }
+    if (T < 1 || tile_tok < 1 || K < 32 || (K & 31) || K > PF_MAX_K || (x_stride & 3) || ((uintptr_t)x & 15) || ((uintptr_t)act & 15)) { return cudaErrorInvalidValue; }
     const size_t smem = norm_w != nullptr ? (size_t)K : 0;   // K / 4 floats
     const bool kq = weight_type == 12 || weight_type == 14;
     auto of_groups = [&](auto pg) {
         constexpr int PG = decltype(pg)::value;
-        return kq ? (norm_w ? prefill_quant_kernel<true, true, PG> : prefill_quant_kernel<false, true, PG>) : (norm_w ? prefill_quant_kernel<true, false, PG> : prefill_quant_kernel<false, false, PG>);
+        if constexpr (SILU) { return kq ? prefill_quant_kernel<false, true, PG, true> : prefill_quant_kernel<false, false, PG, true>; }
+        else { return kq ? (norm_w ? prefill_quant_kernel<true, true, PG, false> : prefill_quant_kernel<false, true, PG, false>) : (norm_w ? prefill_quant_kernel<true, false, PG, false> : prefill_quant_kernel<false, false, PG, false>); }
     };
     const int groups = (K / 8 + PF_QUANT_THREADS - 1) / PF_QUANT_THREADS;
     auto *kernel = groups == 1 ? of_groups(std::integral_constant<int, 1>{}) : groups == 2 ? of_groups(std::integral_constant<int, 2>{}) : of_groups(std::integral_constant<int, PF_QUANT_GROUPS>{});
-    return launch_maybe_pdl(kernel, dim3((unsigned)T), PF_QUANT_THREADS, smem, stream, pdl, x, x_stride, K, norm_w, eps, yq, tile_tok, part_len, part_stride, tap);
+    return launch_maybe_pdl(kernel, dim3((unsigned)T), PF_QUANT_THREADS, smem, stream, pdl, x, x_stride, K, norm_w, eps, yq, tile_tok, part_len, part_stride, tap, silu_table, act);
+}
+cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K, const float *norm_w, float eps, uint8_t *yq, cudaStream_t stream, int weight_type,
+                                 int tile_tok, int part_len, int64_t part_stride, bool pdl, uint8_t *tap) {
+    return launch_quant_t<false>(x, x_stride, T, K, norm_w, eps, yq, stream, weight_type, tile_tok, part_len, part_stride, pdl, tap, nullptr, nullptr);
+}
+cudaError_t launch_prefill_silu_quant(const float *upgate, int T, int F, const float *silu_table, float *act, uint8_t *yq, cudaStream_t stream, int weight_type, int tile_tok, bool pdl) {
+    return launch_quant_t<true>(upgate, 2 * (int64_t)F, T, F, nullptr, 0.f, yq, stream, weight_type, tile_tok, 0, 0, pdl, nullptr, silu_table, act);
 }
 
 cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
@@ -825,8 +868,9 @@ cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool 
 
 cudaError_t launch_prefill_qkv_post(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,
                                     __half *v_cache, int n_ctx, int64_t seq_stride, cudaStream_t stream, bool pdl) {
-    const int64_t n = 3 * (int64_t)dl / 2 * T;
-    return launch_maybe_pdl(prefill_qkv_post_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, pdl, qkv, T, dl, hd, pos_base, rope, q_out, k_cache, v_cache, n_ctx, seq_stride);
+    const int64_t qk_blocks = ((int64_t)dl * T + PF_POST_THREADS - 1) / PF_POST_THREADS;
+    const int64_t v_blocks = seq_stride ? qk_blocks : (int64_t)((dl + PF_POST_E - 1) / PF_POST_E) * ((T + PF_POST_T - 1) / PF_POST_T);
+    return launch_maybe_pdl(prefill_qkv_post_kernel, dim3((unsigned)(qk_blocks + v_blocks)), PF_POST_THREADS, 0, stream, pdl, qkv, T, dl, hd, pos_base, rope, q_out, k_cache, v_cache, n_ctx, seq_stride, (int)qk_blocks);
 }
 
 // the last pass's columns into the buffers the mat-vec passes leave them in
