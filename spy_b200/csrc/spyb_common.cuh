@@ -36,6 +36,11 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
     return v;
 }
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
+}
 __device__ __forceinline__ float4 lds128f(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
@@ -294,6 +299,14 @@ __device__ __forceinline__ uint32_t lane_bits16_q4_0(uint32_t w_x88, uint32_t mu
     return (uint32_t)__dp4a((int)((w_x88 * mult) & 0xf0f0f0f0u), (int)y, (int)MAGIC_I);
 }
 __device__ __forceinline__ uint32_t lane_bits_q8_0(uint32_t w, uint32_t y) { return (uint32_t)__dp4a((int)w, (int)y, (int)MAGIC_I); }
+
+// the product of the f16 values in the low halves of a and b in f32, where it is exact: one mixed-precision FMA onto -0 in place of two
+// conversions and a product
+__device__ __forceinline__ float mul_f16(uint32_t a, uint32_t b) {
+    float d;
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"((uint16_t)a), "h"((uint16_t)b), "f"(-0.0f));
+    return d;
+}
 
 // Two f32 operations per instruction (sm_100 packed f32x2): each half is the IEEE round-to-nearest operation of the
 // scalar instruction, so results are the bits of two fmaf / __fadd_rn calls at half the issue slots.

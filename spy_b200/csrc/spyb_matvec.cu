@@ -162,9 +162,14 @@ __device__ __forceinline__ void act_store(uint32_t *Yw, int g, uint2 q) {
     const int b = g >> 2, at = ((b >> 2) * 8 + 2 * (g & 3)) * 4 + (b & 3);
     Yw[at] = q.x; Yw[at + 4] = q.y;
 }
-__device__ __forceinline__ float act_scale(const MatvecParams &p, float d) { const float r = h2f(f2h(d)); return (p.A.type == 2) ? __fmul_rn(r, 0.0625f) : r; }
+// (HS: as the f16 value it is, for the mixed-precision product of matvec_rows_kernel)
+template <bool HS>
+__device__ __forceinline__ void act_store_scale(const MatvecParams &p, float4 *ds, int b, float d) {
+    if (HS) { reinterpret_cast<uint16_t *>(ds)[b] = f2h(d); }
+    else { const float r = h2f(f2h(d)); reinterpret_cast<float *>(ds)[b] = (p.A.type == 2) ? __fmul_rn(r, 0.0625f) : r; }
+}
 
-template <int PG, bool NORM, int SUM, bool A32, class Requested>
+template <int PG, bool NORM, int SUM, bool A32, bool HS = false, class Requested>
 __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActPlanes act, float *v3, float *scales, const float (*wearly)[8], Requested x_requested) {
     constexpr bool EARLY = SUM == SUM_WIDE;
     constexpr int  CQ = PG == 1 ? 2 : 3;                       // (quads per thread of the wide sum: rows of at most 4096 or 6144 values)
@@ -227,10 +232,10 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
         const int g = tid + k * MV_THREADS;
         if (k < npass && g < n8p) { act_store(reinterpret_cast<uint32_t *>(act.Y), g, q[k]); }
     }
-    if (kd >= 0 && tid + kd * MV_THREADS < n8p) { reinterpret_cast<float *>(act.DS)[(tid + kd * MV_THREADS) >> 2] = act_scale(p, d); }
+    if (kd >= 0 && tid + kd * MV_THREADS < n8p) { act_store_scale<HS>(p, act.DS, (tid + kd * MV_THREADS) >> 2, d); }
 }
 
-template <int TM>
+template <int TM, bool HS = false>
 __device__ __forceinline__ void matvec_prologue(const MatvecParams &p, ActPlanes act, float *v3, float *scales) {
     const int     tid = threadIdx.x;
     const int64_t K   = p.A.k;
@@ -255,7 +260,6 @@ __device__ __forceinline__ void matvec_prologue(const MatvecParams &p, ActPlanes
         __syncthreads();   // also: the partials (aliasing Y) are dead from here on
     }
     uint32_t *Yw = reinterpret_cast<uint32_t *>(act.Y);
-    float    *DS = reinterpret_cast<float *>(act.DS);
     const int n8 = (int)(K >> 3), n8p = nbp * 4;   // groups of eight; including the zero padding up to nbp blocks
 #pragma unroll 1
     for (int t = 0; t < TM; ++t) {
@@ -282,7 +286,7 @@ __device__ __forceinline__ void matvec_prologue(const MatvecParams &p, ActPlanes
             const float d = quantize_q8_groups<1>(v, 1, q, kd);
             if (g < n8p) {
                 act_store(Yw + (size_t)t * nbp * 8, g, q[0]);
-                if (kd == 0) { DS[t * nbp + (g >> 2)] = act_scale(p, d); }
+                if (kd == 0) { act_store_scale<HS>(p, act.DS, t * nbp + (g >> 2), d); }
             }
         }
     }
@@ -290,6 +294,7 @@ __device__ __forceinline__ void matvec_prologue(const MatvecParams &p, ActPlanes
 }
 
 // reference-layout copy of column 0 (34-byte blocks) for parity taps
+template <bool HS = false>
 __device__ __forceinline__ void matvec_tap(const MatvecParams &p, ActPlanes act) {
     if (p.tap_xq == nullptr || blockIdx.x != 0) { return; }
     const uint32_t *Yw = reinterpret_cast<const uint32_t *>(act.Y);
@@ -300,7 +305,7 @@ __device__ __forceinline__ void matvec_tap(const MatvecParams &p, ActPlanes act)
             const uint32_t v = Yw[((b >> 2) * 8 + w) * 4 + (b & 3)];
             o[2 + 4 * w] = (uint8_t)v; o[3 + 4 * w] = (uint8_t)(v >> 8); o[4 + 4 * w] = (uint8_t)(v >> 16); o[5 + 4 * w] = (uint8_t)(v >> 24);
         }
-        *reinterpret_cast<volatile uint16_t *>(p.tap_xq + (size_t)b * 34) = f2h((p.A.type == 2) ? __fmul_rn(DS[b], 16.0f) : DS[b]);
+        *reinterpret_cast<volatile uint16_t *>(p.tap_xq + (size_t)b * 34) = HS ? reinterpret_cast<const uint16_t *>(DS)[b] : f2h((p.A.type == 2) ? __fmul_rn(DS[b], 16.0f) : DS[b]);
     }
 }
 
@@ -593,29 +598,29 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     ActPlanes act = act_planes(smem_raw, nbp, TM);
     {
         float *v3 = reinterpret_cast<float *>(smem_raw);
-        if constexpr (PRO == MVP_ANY) { matvec_prologue<TM>(p, act, v3, norm_scales); }
+        if constexpr (PRO == MVP_ANY) { matvec_prologue<TM, true>(p, act, v3, norm_scales); }
         else if constexpr (PRO == MVP_ONE) {
             const bool norm = p.pro == PRO_NORM_QUANT;
             if (nbp * 8 <= 2 * MV_THREADS) {
-                if (norm) { matvec_prologue_1col<1, true, SUM_CHAIN, true>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<1, false, SUM_FEW, true>(p, act, v3, norm_scales, nullptr, rest); }
+                if (norm) { matvec_prologue_1col<1, true, SUM_CHAIN, true, true>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<1, false, SUM_FEW, true, true>(p, act, v3, norm_scales, nullptr, rest); }
             } else {
-                if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_CHAIN, true>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW, true>(p, act, v3, norm_scales, nullptr, rest); }
+                if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_CHAIN, true, true>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW, true, true>(p, act, v3, norm_scales, nullptr, rest); }
             }
         }
         else {
             constexpr bool NORM = PRO == MVP_NORM || PRO == MVP_NORM_MID || PRO == MVP_NORM_LONG;
             constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 1 : PRO == MVP_NORM_MID ? 2 : PRO_GROUPS;
-            matvec_prologue_1col<PG, NORM, NORM && PG <= NORM_EARLY ? SUM_WIDE : SUM_FEW, true>(p, act, v3, norm_scales, wearly, rest);
+            matvec_prologue_1col<PG, NORM, NORM && PG <= NORM_EARLY ? SUM_WIDE : SUM_FEW, true, true>(p, act, v3, norm_scales, wearly, rest);
         }
     }
     __syncthreads();
     stamp(p.stamps, 2, false); stamp(p.stamps, 6, true);
-    matvec_tap(p, act);
+    matvec_tap<true>(p, act);
 
     const uint32_t y_s   = smem_u32(act.Y);
     const uint32_t ds_s  = smem_u32(act.DS);
     const uint32_t row_s = ring_s + lrow * ROWB;
-    const uint32_t col_y = (uint32_t)ng * 128, col_ds = (uint32_t)ng * 16;
+    const uint32_t col_y = (uint32_t)ng * 128, col_ds = (uint32_t)ng * 8;
 
     // pair k of column t as one packed f32x2 value: low half = accumulator j, high half = accumulator j + 4, j = part * NP + k
     // (both take the same scale in every step, so one packed subtraction and one packed FMA serve the two)
@@ -639,9 +644,8 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
         for (int rc = 0; rc < cnt; ++rc, ra += RECB) {
             const uint4 sc = lds128(ra + 2 * GRPB);
 #pragma unroll
-            for (int gg = 0; gg < 2; ++gg, ya += 128, da += 16) {
+            for (int gg = 0; gg < 2; ++gg, ya += 128, da += 8) {
                 const uint32_t s01 = gg ? sc.z : sc.x, s23 = gg ? sc.w : sc.y;
-                const float2   f01 = __half22float2(*reinterpret_cast<const __half2 *>(&s01)), f23 = __half22float2(*reinterpret_cast<const __half2 *>(&s23));
                 uint4 w[(WT == 8) ? 2 * NP : NP];
 #pragma unroll
                 for (int k = 0; k < NP; ++k) {
@@ -651,8 +655,8 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
                 }
 #pragma unroll
                 for (int t = 0; t < TM; ++t) {
-                    const float4 ds = lds128f(da + t * col_ds);
-                    const float  s0 = __fmul_rn(f01.x, ds.x), s1 = __fmul_rn(f01.y, ds.y), s2 = __fmul_rn(f23.x, ds.z), s3 = __fmul_rn(f23.y, ds.w);
+                    const uint2 ds = lds64(da + t * col_ds);
+                    const float s0 = mul_f16(s01, ds.x), s1 = mul_f16(s01 >> 16, ds.x >> 16), s2 = mul_f16(s23, ds.y), s3 = mul_f16(s23 >> 16, ds.y >> 16);
                     const uint64_t S0 = f2_pack(s0, s0), S1 = f2_pack(s1, s1), S2 = f2_pack(s2, s2), S3 = f2_pack(s3, s3);
 #pragma unroll
                     for (int k = 0; k < NP; ++k) {
@@ -704,6 +708,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
             }
 #pragma unroll
             for (int t = 0; t < TM; ++t) {
+                if (WT == 2) { h[t] = __fmul_rn(h[t], 0.0625f); }   // (exact, as the 16 times in every accumulator were: all are multiples of 2^-48 and far from the largest f32)
                 if (p.epi == EPI_SILU_MUL) {
                     const float gate = __shfl_down_sync(0xffffffffu, h[t], TR / 2);
                     matvec_epilogue_silu(p, (TR / 2) * cu + lane, t, h[t], gate, lane < TR / 2 && t < p.T);

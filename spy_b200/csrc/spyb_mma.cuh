@@ -74,11 +74,6 @@ __device__ __forceinline__ void lds128_if(uint4 &v, uint32_t addr, uint32_t pred
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\t@p ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
                  : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "r"(addr), "r"(pred));
 }
-__device__ __forceinline__ uint2 lds64(uint32_t addr) {
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
-    return v;
-}
 
 // Operands of one group of four consecutive blocks, as they come out of shared memory. The loop over a stage keeps two
 // of these: the loads of group i + 1 are in flight while group i is computed.
