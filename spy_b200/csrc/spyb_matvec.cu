@@ -43,8 +43,10 @@ constexpr int MAX_STAGES = 16;              // ring stages per warp (mbarriers p
 
 // shared memory: per column t, per group g of four blocks
 //   Y [t][g][w][i]  (w = 0..7, i = 0..3)  word w of the 32 int8 values of block 4g+i (w 0..3 = values 0..15)
-//   DS[t][b]        f32 of the fp16-rounded scale; divided by 16 (exact) for Q4_0 weights, whose lane sums come
-//                   scaled by 16
+//   DS[t][b]        the scale: the f16 value, so that d_w * d_x is one mixed-precision FMA (mul_f16; with two conversions and a product, which
+//                   count in loops that are bound by instruction issue, 5120 x 5120 Q8_0 7.13 -> 6.83 us, 32000 x 4096 Q4_0 21.1 -> 19.2).
+//                   matvec_mma_kernel: an f32, divided by 16 (exact) for Q4_0 weights, whose lane sums come scaled by 16; the others take the 16
+//                   out of the finished dot product, where it is as exact: all accumulators are multiples of 2^-48 and far from the largest f32
 // The sum-of-squares partials of the RMSNorm prologue alias Y (they are dead before Y is written).
 struct ActPlanes {
     uint4  *Y;
@@ -387,16 +389,16 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
         const int  n4p  = nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
         if (TM == 1 && n4p <= 2 * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<1, true, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<1, false, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); }
+            if (norm) { matvec_prologue_1col<1, true, SUM_FEW, false, true>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<1, false, SUM_FEW, false, true>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else if (TM == 1 && n4p <= 2 * PRO_GROUPS * MV_THREADS) {
-            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW, false>(p, act, v3, norm_scales, nullptr, []() {}); }
+            if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_FEW, false, true>(p, act, v3, norm_scales, nullptr, []() {}); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW, false, true>(p, act, v3, norm_scales, nullptr, []() {}); }
         } else {
-            matvec_prologue<TM>(p, act, v3, norm_scales);
+            matvec_prologue<TM, true>(p, act, v3, norm_scales);
         }
     }
     __syncthreads();
     stamp(p.stamps, 2, false); stamp(p.stamps, 6, true);
-    matvec_tap(p, act);
+    matvec_tap<true>(p, act);
 
     // this lane's operands, as 32-bit shared-space addresses: activation word (Q8_0 weights: word l; Q4_0: lanes 0..3
     // hold the high nibbles, which meet values 16..31 = words 4..7), the scales, its row and word in a record; and, for
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
     const uint32_t row_s = ring_s + r * ROWB + ((WT == 8) ? l : (l & 3)) * 16;
     const uint32_t mult  = (l < 4) ? 1u : 16u;
     const uint32_t tile_off = (uint32_t)S * RECB;        // second tile of the unit inside a stage
-    const uint32_t col_y = (uint32_t)ng * 128, col_ds = (uint32_t)ng * 16;   // next activation column
+    const uint32_t col_y = (uint32_t)ng * 128, col_ds = (uint32_t)ng * 8;   // next activation column
 
     float acc[TM][R];
 #pragma unroll
@@ -435,32 +437,27 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
                 sc[i]    = lds128(rowa - ((WT == 8) ? l : (l & 3)) * 16 + (ROWB - 16));
             }
 #pragma unroll
-            for (int gg = 0; gg < 2; ++gg, ya += 128, da += 16) {
-                float s[R][4];
-#pragma unroll
-                for (int i = 0; i < R; ++i) {
-                    const uint32_t s01 = gg ? sc[i].z : sc[i].x, s23 = gg ? sc[i].w : sc[i].y;
-                    const float2   f01 = __half22float2(*reinterpret_cast<const __half2 *>(&s01)), f23 = __half22float2(*reinterpret_cast<const __half2 *>(&s23));
-                    s[i][0] = f01.x; s[i][1] = f01.y; s[i][2] = f23.x; s[i][3] = f23.y;
-                }
+            for (int gg = 0; gg < 2; ++gg, ya += 128, da += 8) {
 #pragma unroll
                 for (int t = 0; t < TM; ++t) {
                     const uint4  y  = lds128(ya + t * col_y);
-                    const float4 ds = lds128f(da + t * col_ds);
+                    const uint2  ds = lds64(da + t * col_ds);
 #pragma unroll
                     for (int i = 0; i < R; ++i) {
                         const uint4 w = wq[i][gg];
                         float a = acc[t][i];
+                        const uint32_t s01 = gg ? sc[i].z : sc[i].x, s23 = gg ? sc[i].w : sc[i].y;
+                        const float s0 = mul_f16(s01, ds.x), s1 = mul_f16(s01 >> 16, ds.x >> 16), s2 = mul_f16(s23, ds.y), s3 = mul_f16(s23 >> 16, ds.y >> 16);
                         if (WT == 2) {
-                            a = fmaf(__fmul_rn(s[i][0], ds.x), lane_sum16_q4_0(w.x, mult, y.x), a);
-                            a = fmaf(__fmul_rn(s[i][1], ds.y), lane_sum16_q4_0(w.y, mult, y.y), a);
-                            a = fmaf(__fmul_rn(s[i][2], ds.z), lane_sum16_q4_0(w.z, mult, y.z), a);
-                            a = fmaf(__fmul_rn(s[i][3], ds.w), lane_sum16_q4_0(w.w, mult, y.w), a);
+                            a = fmaf(s0, lane_sum16_q4_0(w.x, mult, y.x), a);
+                            a = fmaf(s1, lane_sum16_q4_0(w.y, mult, y.y), a);
+                            a = fmaf(s2, lane_sum16_q4_0(w.z, mult, y.z), a);
+                            a = fmaf(s3, lane_sum16_q4_0(w.w, mult, y.w), a);
                         } else {
-                            a = fmaf(__fmul_rn(s[i][0], ds.x), lane_sum_q8_0(w.x, y.x), a);
-                            a = fmaf(__fmul_rn(s[i][1], ds.y), lane_sum_q8_0(w.y, y.y), a);
-                            a = fmaf(__fmul_rn(s[i][2], ds.z), lane_sum_q8_0(w.z, y.z), a);
-                            a = fmaf(__fmul_rn(s[i][3], ds.w), lane_sum_q8_0(w.w, y.w), a);
+                            a = fmaf(s0, lane_sum_q8_0(w.x, y.x), a);
+                            a = fmaf(s1, lane_sum_q8_0(w.y, y.y), a);
+                            a = fmaf(s2, lane_sum_q8_0(w.z, y.z), a);
+                            a = fmaf(s3, lane_sum_q8_0(w.w, y.w), a);
                         }
                         acc[t][i] = a;
                     }
@@ -476,7 +473,7 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
             for (int t = 0; t < TM; ++t) {
                 float h[R];
 #pragma unroll
-                for (int i = 0; i < R; ++i) { h[i] = hsum8_lanes(acc[t][i]); acc[t][i] = 0.f; }
+                for (int i = 0; i < R; ++i) { h[i] = hsum8_lanes(acc[t][i]); if (WT == 2) { h[i] = __fmul_rn(h[i], 0.0625f); } acc[t][i] = 0.f; }
                 const bool    writer = (l == 0) && (t < p.T);
                 const int64_t row0 = p.pair_mode ? 4 * cu + r : 4 * R * cu + r;
                 if (p.epi == EPI_SILU_MUL) {
@@ -708,7 +705,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
             }
 #pragma unroll
             for (int t = 0; t < TM; ++t) {
-                if (WT == 2) { h[t] = __fmul_rn(h[t], 0.0625f); }   // (exact, as the 16 times in every accumulator were: all are multiples of 2^-48 and far from the largest f32)
+                if (WT == 2) { h[t] = __fmul_rn(h[t], 0.0625f); }
                 if (p.epi == EPI_SILU_MUL) {
                     const float gate = __shfl_down_sync(0xffffffffu, h[t], TR / 2);
                     matvec_epilogue_silu(p, (TR / 2) * cu + lane, t, h[t], gate, lane < TR / 2 && t < p.T);
