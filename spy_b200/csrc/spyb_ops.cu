@@ -51,6 +51,7 @@ __device__ __forceinline__ float reduce4_chain(const float *v, int n) {
 constexpr int ATT_THREADS = 256;
 constexpr int ATT_WARPS   = ATT_THREADS / WARP;
 constexpr int ATT_HD      = 128;
+constexpr int ATT_MANY    = 2;      // CTAs an SM holds of a launch that has more of them than the chip has SMs
 
 __device__ __forceinline__ void unpack8(const uint4 v, float f[8]) {
     const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
@@ -59,8 +60,12 @@ __device__ __forceinline__ void unpack8(const uint4 v, float f[8]) {
 }
 
 // EARLY: a step that reads cache rows ahead of its wait (a kernel of its own: 7B steps 0.6 % slower with both in one)
-template <bool EARLY>
-__global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams p) {
+// CTAS > 1: for launches of more CTAs than SMs, so many of them side by side on one: a K row and the V^T values are read when they are needed instead
+// of being held ahead in 248 registers, with which one CTA fills an SM. us a step of four layers, one CTA an SM / 2 / 3 / 4: 40 heads x 32 sequences at
+// 10 positions 1229 / 1162 / 1155 / 1161; 16 x 32 at 400 637 / 588 / 615 / 677; 32 x 16 at 200 740 / 717 / 726 / 753; 32 x 8 at 900 828 / 824 / 936 /
+// 1063 (more CTAs share an L1 that the V^T rows then leave).
+template <bool EARLY, int CTAS>
+__global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const AttnParams p) {
     extern __shared__ __align__(16) float att_smem[];
     __shared__ float red[ATT_WARPS];
     __shared__ float bcast;
@@ -95,10 +100,11 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
     const int pv_e = tid >> 1, pv_half = tid & 1;
     const __half *vrow = v_cache + ((int64_t)h * ATT_HD + pv_e) * p.n_ctx;
     uint2 v_first[4], v_tail[8];
-    uint4 kv[16];                                    // a whole K row in flight at once
+    constexpr bool AHEAD = CTAS == 1;
+    uint4 kv[AHEAD ? 16 : 4];                        // a whole K row in flight at once
     // the words of V^T and the K row of which positions lo <= j < n_vis (K: lo <= tid) are wanted; words that reach past n_vis, which may be
     // new in part, belong to the second pass, which goes past L1 where there was a first one
-    auto request = [&](int lo, int n_vis, int n_main, bool last) {
+    auto request_v = [&](int lo, int n_vis, int n_main, bool last) {
         auto load_v = [&](int j) { const uint2 *src = reinterpret_cast<const uint2 *>(vrow + j); return EARLY ? __ldcg(src) : *src; };
         auto wanted = [&](int j) { return j < n_vis && j + 4 > lo && (last || j + 4 <= n_vis); };
 #pragma unroll
@@ -111,10 +117,13 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
             const int j = n_main + 4 * c;
             if (wanted(j)) { v_tail[c] = load_v(j); }
         }
+    };
+    auto request = [&](int lo, int n_vis, int n_main, bool last) {
+        request_v(lo, n_vis, n_main, last);
         if (tid >= lo && tid < n_vis) {
             const uint4 *krow = reinterpret_cast<const uint4 *>(k_cache + (int64_t)tid * p.dl + (int64_t)h * ATT_HD);
 #pragma unroll
-            for (int a = 0; a < 16; ++a) { kv[a] = EARLY && last ? __ldcg(krow + a) : krow[a]; }
+            for (int a = 0; a < (AHEAD ? 16 : 0); ++a) { kv[a] = EARLY && last ? __ldcg(krow + a) : krow[a]; }
         }
     };
 #pragma unroll
@@ -135,7 +144,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
     const int pos   = base.x + (batch ? 0 : t);
     const int n_vis = pos + 1;                   // causal mask: positions 0..pos are visible
     const int n_tot = row_length(base.x, base.y), n_main = ((n_tot - 1) / 32) * 32;
-    if (early != pos || early_tot != n_tot) {
+    if (AHEAD && (early != pos || early_tot != n_tot)) {
 #pragma unroll
         for (int a = 0; a < 4; ++a) { v_first[a] = make_uint2(0u, 0u); }
 #pragma unroll
@@ -146,14 +155,22 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
     __syncthreads();
 
     // ---- scores of the visible positions: one thread per position
+#pragma unroll 1
     for (int j = tid; j < n_vis; j += ATT_THREADS) {
         const uint4  *krow = reinterpret_cast<const uint4 *>(k_cache + (int64_t)j * p.dl + (int64_t)h * ATT_HD);
         const float4 *q4   = reinterpret_cast<const float4 *>(qf);
         float acc[4][8];
-        if (j != tid) {
+        if (AHEAD && j != tid) {
 #pragma unroll
-            for (int a = 0; a < 16; ++a) { kv[a] = krow[a]; }
+            for (int a = 0; a < (AHEAD ? 16 : 0); ++a) { kv[a] = krow[a]; }
         }
+        auto part = [&](int step) {                  // 32 elements of the row
+            if constexpr (!AHEAD) {
+                asm volatile("" ::: "memory");       // (not all of them ahead)
+#pragma unroll
+                for (int a = 0; a < 4; ++a) { kv[a] = krow[4 * step + a]; }
+            }
+        };
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
 #pragma unroll
@@ -161,9 +178,10 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
         }
 #pragma unroll
         for (int step = 0; step < 3; ++step) {       // elements 0..95: accumulator a takes elements 32 * step + 8a .. + 7
+            part(step);
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                float kf[8]; unpack8(kv[4 * step + a], kf);
+                float kf[8]; unpack8(kv[AHEAD ? 4 * step + a : a], kf);
                 const float4 qa = q4[(4 * step + a) * 2], qb = q4[(4 * step + a) * 2 + 1];
                 const float  qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
 #pragma unroll
@@ -179,9 +197,10 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
         }
         const float simd = __fadd_rn(__fadd_rn(u[0], u[1]), __fadd_rn(u[2], u[3]));
         float tail = 0.f;                             // elements 96..127: scalar chain
+        part(3);
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            float kf[8]; unpack8(kv[12 + a], kf);
+            float kf[8]; unpack8(kv[AHEAD ? 12 + a : a], kf);
             const float4 qa = q4[(12 + a) * 2], qb = q4[(12 + a) * 2 + 1];
             const float  qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
 #pragma unroll
@@ -191,9 +210,10 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
     }
     // The V^T values of the next PV steps are requested now (the K row's registers are free), so that they arrive
     // during the softmax instead of costing one memory round trip per 32 positions afterwards.
-    constexpr int PV_AHEAD = 6;
+    if (!AHEAD) { request_v(0, n_vis, n_main, true); }
+    constexpr int PV_AHEAD = AHEAD ? 6 : 0;
     constexpr int n_ahead = PV_AHEAD;
-    uint2 v_ahead[PV_AHEAD][4];
+    uint2 v_ahead[AHEAD ? PV_AHEAD : 1][4];
 #pragma unroll
     for (int s = 0; s < PV_AHEAD; ++s) {
 #pragma unroll
@@ -285,6 +305,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_kernel(const AttnParams
                 }
             };
             fetch(vv, j0);
+#pragma unroll 1
             for (; j0 < n_main && j0 < n_vis; j0 += 32) {
                 fetch(vn, j0 + 32);
                 pv_step(vv, j0);
@@ -1221,7 +1242,8 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
     }
     const size_t smem = (n_pad + n_pad / 4 + ATT_HD) * sizeof(float) + 16;
     if (smem > 200 * 1024) { return cudaErrorInvalidValue; }
-    const void *kernel = reinterpret_cast<const void *>(p.early && p.T == 1 && p.seq_stride == 0 ? attention_kernel<true> : attention_kernel<false>);
+    const bool many = (int64_t)p.n_head * p.T > device_sms();
+    const void *kernel = reinterpret_cast<const void *>(many ? attention_kernel<false, ATT_MANY> : p.early && p.T == 1 && p.seq_stride == 0 ? attention_kernel<true, 1> : attention_kernel<false, 1>);
     cudaError_t err = allow_dynamic_smem(kernel, smem);
     if (err != cudaSuccess) { return err; }
     return launch_with_pdl(kernel, dim3(p.n_head, p.T, 1), dim3(ATT_THREADS), smem, p, cfg);

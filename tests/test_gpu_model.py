@@ -331,6 +331,29 @@ def test_prompt_widths_the_gemm_tile_does_not_divide(be, oracle, tmp_models):
     m.close()
 
 
+def test_batch_of_more_heads_than_sms_equals_single_sequence_runs(tmp_models):
+    """A batch whose attention has more CTAs than the chip has SMs (40 sequences of four heads), against the same sequences decoded one by one."""
+    cfg = gguf_io.LlamaConfig(n_layer=2, d_model=512, n_head=4, n_ff=512, n_vocab=400, weight_std=0.06)
+    path = str(tmp_models / "batch_heads.gguf")
+    gguf_io.make_llama_gguf(path, cfg, seed=61)
+    n_seq, n_prompt, n_steps = 40, 27, 12
+    rng = np.random.default_rng(n_seq)
+    b = B.B200Backend(0)
+    m = B.LlamaModel(b, path, n_ctx=64)
+    m.set_sequences(n_seq)
+    first, want = [], []
+    for c in range(n_seq):
+        m.select_sequence(c)
+        first.append(int(np.argmax(m.eval(rng.integers(3, cfg.n_vocab, size=n_prompt), 0))))
+        want.append(m.decode(first[-1], n_prompt, n_steps, want_logits=True))
+    ids, logits = m.decode_batch(first, n_prompt, n_steps, want_logits=True)
+    for c in range(n_seq):
+        assert np.array_equal(ids[:, c], want[c][0]), c
+        assert np.array_equal(np.ascontiguousarray(logits[:, c]).view(np.uint32), want[c][1].view(np.uint32)), c
+    m.close()
+    b.close()
+
+
 @pytest.mark.parametrize("n_seq,n_ctx,kq", [(3, 64, False), (8, 64, False), (6, 1100, False), (20, 64, False), (17, 1100, False),
                                             (3, 64, True), (6, 64, True), (18, 64, True)])
 def test_batch_of_sequences_equals_single_sequence_runs(n_seq, n_ctx, kq, oracle, tmp_models):
