@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "spyb_common.cuh"
 #include "spyb_kernels.h"
@@ -213,7 +214,7 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
         __shared__ __align__(16) float rs_scratch[EARLY ? rs_scratch_words(CQ) : 4];
         float sum = 0.f;
         if (EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<EARLY ? CQ : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
-        else if (tid == 0) { sum = SUM == SUM_CHAIN ? running_sum_serial(smem_u32(v3), n4) : running_sum_small(v3, n4); }
+        else if (tid == 0) { sum = EARLY ? running_sum_cold(smem_u32(v3), n4) : SUM == SUM_CHAIN ? running_sum_serial(smem_u32(v3), n4) : running_sum_small(v3, n4); }
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
             scales[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
@@ -527,7 +528,7 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
 // instructions in the caches is worth more than a better loop (four layers of d = 512, ff 5632, Q4_0: 102.3 -> 94.1 us a step; 1024, 2816:
 // 99.6 -> 93.5; 2048, 5632: 121.4 -> 117.7; 3072, 8192: 158.1 -> 153.8; but 4096, 11008: 188.2 -> 190.9).
 enum { MVP_ANY, MVP_NORM, MVP_NORM_MID, MVP_PLAIN, MVP_NORM_LONG, MVP_PLAIN_LONG, MVP_ONE };
-template <int WT, int TM, int LPR, int PRO>
+template <int WT, int TM, int LPR, int PRO, int EPI = -1>
 __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const MatvecParams p, const int ring_bytes, const int S, const int wact) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ float norm_scales[8];
@@ -535,6 +536,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     constexpr int ROWB = ((WT == 8) ? 256 : 128) + 16;
     constexpr int RECB = TR * ROWB;
     constexpr int GRPB = (WT == 8) ? 128 : 64;
+    constexpr bool LEAN = EPI >= 0;                      // a launch of one GPU's that nobody watches: no exchange, time stamps and tap
     constexpr int NP   = 4 / LPR;                        // accumulator pairs (j, j + 4) per lane
 
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
@@ -579,7 +581,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     pdl_launch_dependents();
     float wearly[PRO == MVP_NORM_MID ? 2 : 1][8];
     if (PRO == MVP_NORM || PRO == MVP_NORM_MID) { norm_weights_early(p, wearly); }
-    stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
+    if (!LEAN) { stamp(p.stamps, 0, false); stamp(p.stamps, 4, true); }
     if (lane == 0 && n_items > 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(full_s + s * 8, 1); }
         mbar_init_fence();
@@ -588,8 +590,10 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     }
     __syncwarp();
     pdl_wait();
-    stamp(p.stamps, 1, false); stamp(p.stamps, 5, true);
-    tp_wait(p.tp, p.error_flag);
+    if (!LEAN) {
+        stamp(p.stamps, 1, false); stamp(p.stamps, 5, true);
+        tp_wait(p.tp, p.error_flag);
+    }
 
     auto rest = [&]() { if (lane == 0) { while (issued < min(NS, n_items)) { issue_next(); } } };
     ActPlanes act = act_planes(smem_raw, nbp, TM);
@@ -611,8 +615,10 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
         }
     }
     __syncthreads();
-    stamp(p.stamps, 2, false); stamp(p.stamps, 6, true);
-    matvec_tap<true>(p, act);
+    if (!LEAN) {
+        stamp(p.stamps, 2, false); stamp(p.stamps, 6, true);
+        matvec_tap<true>(p, act);
+    }
 
     const uint32_t y_s   = smem_u32(act.Y);
     const uint32_t ds_s  = smem_u32(act.DS);
@@ -706,12 +712,12 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
 #pragma unroll
             for (int t = 0; t < TM; ++t) {
                 if (WT == 2) { h[t] = __fmul_rn(h[t], 0.0625f); }
-                if (p.epi == EPI_SILU_MUL) {
+                if ((LEAN ? EPI : p.epi) == EPI_SILU_MUL) {
                     const float gate = __shfl_down_sync(0xffffffffu, h[t], TR / 2);
                     matvec_epilogue_silu(p, (TR / 2) * cu + lane, t, h[t], gate, lane < TR / 2 && t < p.T);
                 } else {
                     const float partner = __shfl_xor_sync(0xffffffffu, h[t], 1);
-                    matvec_epilogue(p, TR * cu + lane, t, h[t], partner, lane < TR && t < p.T);
+                    matvec_epilogue<EPI>(p, TR * cu + lane, t, h[t], partner, lane < TR && t < p.T);
                 }
             }
             crec = 0; cu += wact; ya = y_s; da = ds_s;
@@ -726,8 +732,10 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
             if (++slot == NS) { slot = 0; parity ^= 1u; }
         }
     }
-    tp_publish(p.tp, p.T);
-    if (p.stamps != nullptr) { __syncthreads(); stamp(p.stamps, 3, true); }
+    if (!LEAN) {
+        tp_publish(p.tp, p.T);
+        if (p.stamps != nullptr) { __syncthreads(); stamp(p.stamps, 3, true); }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -939,10 +947,20 @@ static cudaError_t launch_matvec_rows_t(const MatvecParams &p, const LaunchCfg &
     if constexpr (TM == 1) if (aligned) {
         const int  n4p = p.A.nbp * 8;
         const bool norm = p.pro == PRO_NORM_QUANT;
+        const bool lean = p.stamps == nullptr && p.tap_xq == nullptr && p.tp.counter == nullptr && p.tp.flag_in == nullptr;
+        auto normed = [&](auto pro) {
+            constexpr int P = decltype(pro)::value;
+            return !lean ? matvec_rows_kernel<WT, 1, LPR, P> : p.epi == EPI_QKV_ROPE ? matvec_rows_kernel<WT, 1, LPR, P, EPI_QKV_ROPE> : p.epi == EPI_SILU_MUL ? matvec_rows_kernel<WT, 1, LPR, P, EPI_SILU_MUL>
+                 : p.epi == EPI_STORE ? matvec_rows_kernel<WT, 1, LPR, P, EPI_STORE> : matvec_rows_kernel<WT, 1, LPR, P>;
+        };
+        auto plain = [&](auto pro) {
+            constexpr int P = decltype(pro)::value;
+            return lean && p.epi == EPI_RESID ? matvec_rows_kernel<WT, 1, LPR, P, EPI_RESID> : matvec_rows_kernel<WT, 1, LPR, P>;
+        };
         if (p.narrow && n4p <= 2 * PRO_GROUPS * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_ONE>; }
-        else if (n4p <= 2 * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN>; }
-        else if (norm && n4p <= 3 * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_NORM_MID>; }
-        else if (n4p <= 2 * PRO_GROUPS * MV_THREADS) { kernel = norm ? matvec_rows_kernel<WT, 1, LPR, MVP_NORM_LONG> : matvec_rows_kernel<WT, 1, LPR, MVP_PLAIN_LONG>; }
+        else if (n4p <= 2 * MV_THREADS) { kernel = norm ? normed(std::integral_constant<int, MVP_NORM>{}) : plain(std::integral_constant<int, MVP_PLAIN>{}); }
+        else if (norm && n4p <= 3 * MV_THREADS) { kernel = normed(std::integral_constant<int, MVP_NORM_MID>{}); }
+        else if (n4p <= 2 * PRO_GROUPS * MV_THREADS) { kernel = norm ? normed(std::integral_constant<int, MVP_NORM_LONG>{}) : plain(std::integral_constant<int, MVP_PLAIN_LONG>{}); }
     }
     cudaError_t err = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), smem);
     if (err != cudaSuccess) { return err; }

@@ -37,6 +37,9 @@ __device__ __forceinline__ float running_sum_serial(uint32_t v3, int n4) {   // 
     return sum;
 }
 
+// (out of line: what is rarely taken shall not lie between what always is)
+static __device__ __noinline__ float running_sum_cold(uint32_t v3, int n4) { return running_sum_serial(v3, n4); }
+
 // The same sum, the same bits, by four consecutive warps: the chain is 4.4 cycles per value (4450 cycles for the 1024 groups of a row of
 // 4096), which every RMSNorm of a decode step would wait for; this takes 2200. While the running sum stays in one binade it is an integer S
 // times its ulp, and adding v >= 0 adds the integer nearest to v / ulp - at a tie the one that leaves S even, so that only S's parity
@@ -130,6 +133,7 @@ __device__ __forceinline__ float running_sum_chunks(uint32_t v3, int n4, uint32_
             c[4 * q] = x.x; c[4 * q + 1] = x.y; c[4 * q + 2] = x.z; c[4 * q + 3] = x.w;
         }
         uint32_t from = 0;
+#pragma unroll 1
         for (int i0 = 0; i0 < total; i0 += 4) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -144,7 +148,8 @@ __device__ __forceinline__ float running_sum_chunks(uint32_t v3, int n4, uint32_
         const uint32_t to = from + en.x + (from & 1u) * en.y;
         ok = __all_sync(0xffffffffu, ez < 0 || ((int)(from >> 23) == ez && (int)(to >> 23) == ez));
     }
-    if (!ok) { return running_sum_serial(v3, n4); }
+    if (!ok) { return running_sum_cold(v3, n4); }
+#pragma unroll 1
     for (int g = 4 * q4; g < n4; ++g) { s = __fadd_rn(s, __uint_as_float(lds32(v3 + 4 * g))); }
     return s;
 }
@@ -160,8 +165,10 @@ static __device__ __noinline__ float running_sum_wide(uint32_t v3, int n4, uint3
 // ---------------------------------------------------------------------------------------------
 // epilogue for one finished dot product `v` (identical on the 8 lanes of its row) of row `row`, column t.
 // `partner` is the value of the neighbouring row (row ^ 1), needed by RoPE. Called by all lanes; lane l == 0 writes.
+// EPI >= 0: the epilogue of a kernel that has this one only
+template <int EPI = -1>
 __device__ __forceinline__ void matvec_epilogue(const MatvecParams &p, int64_t row, int t, float v, float partner, bool writer) {
-    switch (p.epi) {
+    switch (EPI >= 0 ? EPI : p.epi) {
     case EPI_STORE:
         if (writer) { p.out[(int64_t)t * p.out_stride + row] = v; }
         break;
@@ -170,8 +177,8 @@ __device__ __forceinline__ void matvec_epilogue(const MatvecParams &p, int64_t r
         break;
     case EPI_QKV_ROPE: {
         if (!writer) { break; }
-        const int sec = (int)(row / p.dl);
-        const int e   = (int)(row - (int64_t)sec * p.dl);
+        const int sec = (int)row >= 2 * p.dl ? 2 : (int)row >= p.dl ? 1 : 0;
+        const int e   = (int)row - sec * p.dl;
         const int pos = *p.pos_base + (p.seq_stride ? 0 : t);          // a batch in lockstep: every column at the same position,
         const int64_t seq_off = p.seq_stride ? (int64_t)t * p.seq_stride : 0;   // each in its own cache
         if (sec == 2) {   // V: f32 -> f16 RNE into the transposed cache [dl][n_ctx] (dup_execute, backend/host/operator/view.cpp:163-191)
