@@ -25,6 +25,7 @@
 // decode step of eight 7B layers (Q4_K / Q6_K) 0.75 -> 0.52 ms.
 
 #include <algorithm>
+#include <type_traits>
 
 #include "spyb_common.cuh"
 #include "spyb_kernels.h"
@@ -81,7 +82,7 @@ __device__ __forceinline__ void kq_prologue(const MatvecParams &p, int nT, uint3
         }
         __syncthreads();
         if ((tid & 31) == 0 && (tid >> 5) < nT) {
-            const float sum  = running_sum_serial(smem_u32(rec + (tid >> 5) * col), n4);
+            const float sum  = running_sum_cold(smem_u32(rec + (tid >> 5) * col), n4);
             const float mean = __fdiv_rn(sum, (float)p.A.k);
             scale_s[tid >> 5] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
         }
@@ -152,7 +153,7 @@ __device__ __forceinline__ void kq_prologue_1col(const MatvecParams &p, uint32_t
         float sum = 0.f;
         if (PG <= KQ_NORM_EARLY && n4 >= RS_MIN && n4 <= CQ * 512 && (n4 >> 6) * (KQ_REC - 64) >= rs_scratch_words(CQ)) {
             if (tid < RS_THREADS) { sum = running_sum_chunks<PG <= KQ_NORM_EARLY ? CQ : 2>(smem_u32(v3), n4, smem_u32(v3 + n4), tid, 1); }
-        } else if (tid == 0) { sum = running_sum_serial(smem_u32(v3), n4); }
+        } else if (tid == 0) { sum = running_sum_cold(smem_u32(v3), n4); }
         if (tid == 0) { scale_s[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)p.A.k), p.eps))); }
         __syncthreads();   // also: the partials (aliasing the records) are dead from here on
         const float scale = scale_s[0];
@@ -275,8 +276,10 @@ __device__ __forceinline__ KqRow kq_row(const MatvecParams &p, int64_t row) {
 }
 // first row of the unit that begins at pair `pair0` (side 1: of the second matrix in pair mode). Row r of a unit is row r of the first, or,
 // in pair mode, row r / 2 of side r % 2.
+template <int EPI>
 __device__ __forceinline__ KqRow kq_unit(const MatvecParams &p, int64_t pair0, int side) {
-    if (!p.pair_mode) { return kq_row(p, 2 * pair0); }
+    if constexpr (EPI == EPI_RESID || EPI == EPI_STORE) { return {p.kq[0].w + 2 * pair0 * p.kq[0].row_bytes, p.kq[0].row_bytes, p.kq[0].type}; }   // (one matrix)
+    if (EPI >= 0 ? EPI != EPI_SILU_MUL : !p.pair_mode) { return kq_row(p, 2 * pair0); }
     KqRow r;
     r.pitch = side ? p.kq[1].row_bytes : p.kq[0].row_bytes; r.type = side ? p.kq[1].type : p.kq[0].type;
     r.w = (side ? p.kq[1].w : p.kq[0].w) + pair0 * r.pitch;
@@ -298,17 +301,20 @@ __host__ __device__ static inline KqSmem kq_smem_layout(int nsb, int TM, const K
 // 14 when every row is of that type, else 0
 // PRO: the prologue the kernel is built with - one column of at most 1024 groups of four (with the norm also 1536) or a longer one, with and without the norm;
 // else any
+// EPI >= 0: of one epilogue (SILU_MUL: in pair mode; STORE and RESID: of one matrix), without the exchange between GPUs, as in matvec_rows_kernel
 enum { KQP_ANY, KQP_NORM, KQP_NORM_MID, KQP_PLAIN, KQP_NORM_LONG, KQP_PLAIN_LONG };
-template <int TM, int TYPE, int PRO>
+template <int TM, int TYPE, int PRO, int EPI = -1>
 __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecParams p, const KqPlan pl) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ float scale_s[TM];
+    const bool pair_mode = EPI >= 0 ? EPI == EPI_SILU_MUL : p.pair_mode != 0;
+    const int  epi = EPI >= 0 ? EPI : p.epi;
     const int nsb = p.A.nb >> 3, nT = (TM == 1) ? 1 : p.T;
     const int col = nsb * KQ_REC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const KqSmem L = kq_smem_layout(nsb, TM, pl);
     const int n_row = 2 * pl.np, items = n_row * nsb, n_round = (items + 31) >> 5;   // per unit
-    const int64_t n_units  = (p.pair_mode ? p.kq[0].n_rows : (p.A.n_rows >> 1)) / pl.np;
+    const int64_t n_units  = (pair_mode ? p.kq[0].n_rows : (p.A.n_rows >> 1)) / pl.np;
     const int64_t unit_lo  = n_units * blockIdx.x / gridDim.x, unit_hi = n_units * (blockIdx.x + 1) / gridDim.x;
     const int64_t my_first = unit_lo + warp;
     const int     my_units = (warp < pl.wact && my_first < unit_hi) ? (int)((unit_hi - my_first + pl.wact - 1) / pl.wact) : 0;
@@ -316,35 +322,38 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
     const uint32_t ring_s = smem_u32(smem_raw + L.ring) + (uint32_t)warp * pl.ns * pl.stage_bytes;
     const uint32_t bar_s  = smem_u32(smem_raw + L.bars) + (uint32_t)warp * pl.ns * 8;
     float *part = reinterpret_cast<float *>(smem_raw + L.part) + (size_t)warp * TM * items;
-    const bool mixed = TYPE == 0 && p.pair_mode && p.kq[0].type != p.kq[1].type;   // (items of a stage then lie at the larger pitch)
+    const bool mixed = TYPE == 0 && pair_mode && p.kq[0].type != p.kq[1].type;   // (items of a stage then lie at the larger pitch)
 
     // lane 0: the next 32 super-blocks of the unit at lunit (from super-block lsb of its row lr on) into slot lslot
     int64_t lunit = my_first; int lr = 0, lsb = 0, lslot = 0, issued = 0;
     KqRow l0 = {}, l1 = {};
-    auto load_unit = [&]() { l0 = kq_unit(p, lunit * pl.np, 0); if (p.pair_mode) { l1 = kq_unit(p, lunit * pl.np, 1); } };
+    auto load_unit = [&]() { l0 = kq_unit<EPI>(p, lunit * pl.np, 0); if (pair_mode) { l1 = kq_unit<EPI>(p, lunit * pl.np, 1); } };
     const uint64_t policy = l2_evict_first();
     auto issue_next = [&]() {
         const uint32_t bar = bar_s + lslot * 8;
         uint32_t dst = ring_s + (uint32_t)(lslot * pl.stage_bytes);
         int left = min(32, items - (lr * nsb + lsb));
-        if (!p.pair_mode && (TYPE != 0 ? TYPE : l0.type) == 12) {   // the unit's rows are one contiguous run
+        if (!pair_mode && (TYPE != 0 ? TYPE : l0.type) == 12) {   // the unit's rows are one contiguous run
             const uint32_t bytes = (uint32_t)left * 144u;
             mbar_expect_tx(bar, bytes);
             bulk_copy_g2s_once(dst, l0.w + (size_t)(lr * nsb + lsb) * 144, bytes, bar, policy);
             lsb += left;
+#pragma unroll 1
             while (lsb >= nsb) { lsb -= nsb; ++lr; }
         } else {
             uint32_t bytes = (uint32_t)left * ((TYPE != 0 ? TYPE : l0.type) == 12 ? 144u : 208u);
             if (mixed) {
                 bytes = 0;
+#pragma unroll 1
                 for (int q = left, r = lr, o = lsb; q > 0; ++r, o = 0) { const int m = min(q, nsb - o); bytes += (uint32_t)m * (((r & 1) ? l1.type : l0.type) == 12 ? 144u : 208u); q -= m; }
             }
             mbar_expect_tx(bar, bytes);
+#pragma unroll 1
             while (left > 0) {
                 const int m = min(left, nsb - lsb);
-                const bool second = p.pair_mode && (lr & 1);
+                const bool second = pair_mode && (lr & 1);
                 const uint32_t body = (TYPE != 0 ? TYPE : second ? l1.type : l0.type) == 12 ? 144u : 208u;
-                const uint8_t *src = (second ? l1.w : l0.w) + (int64_t)(p.pair_mode ? lr >> 1 : lr) * (second ? l1.pitch : l0.pitch) + (uint32_t)lsb * body;
+                const uint8_t *src = (second ? l1.w : l0.w) + (int64_t)(pair_mode ? lr >> 1 : lr) * (second ? l1.pitch : l0.pitch) + (uint32_t)lsb * body;
                 bulk_copy_g2s_once(dst, src, (uint32_t)m * body, bar, policy);
                 dst += (uint32_t)m * (mixed ? 208u : body);
                 left -= m; lsb += m;
@@ -372,19 +381,26 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
         }
     }
     if (lane == 0 && n_stage > 0) {
+#pragma unroll 1
         for (int s = 0; s < pl.ns; ++s) { mbar_init(bar_s + s * 8, 1); }
         mbar_init_fence();
         load_unit();
+#pragma unroll 1
         for (int s = 0; s < (PRO == KQP_ANY ? pl.ns : min(pl.ns, p.stages_early)) && issued < n_stage; ++s) { issue_next(); }
     }
     __syncwarp();
     pdl_wait();
-    tp_wait(p.tp, p.error_flag);
+    if (EPI < 0) { tp_wait(p.tp, p.error_flag); }
     uint32_t *rec = reinterpret_cast<uint32_t *>(smem_raw);
     if constexpr (PRO == KQP_ANY) {
         if (p.pro == PRO_NORM_QUANT) { kq_prologue<true>(p, nT, rec, col, scale_s); } else { kq_prologue<false>(p, nT, rec, col, scale_s); }
     } else {
-        auto rest = [&]() { if (lane == 0) { while (issued < min(pl.ns, n_stage)) { issue_next(); } } };
+        auto rest = [&]() {
+            if (lane == 0) {
+#pragma unroll 1
+                while (issued < min(pl.ns, n_stage)) { issue_next(); }
+            }
+        };
         constexpr bool NORM = PRO == KQP_NORM || PRO == KQP_NORM_MID || PRO == KQP_NORM_LONG;
         kq_prologue_1col<PG, NORM>(p, rec, scale_s, wearly, rest);
     }
@@ -401,16 +417,16 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
     // the rows' results are finished one unit later: the residual or the SiLU table entry they meet is on its way meanwhile
     float pend_a = 0.f, pend_b = 0.f;
     float *pend = nullptr;
-    auto finish_pending = [&]() { if (pend != nullptr) { *pend = p.epi == EPI_SILU_MUL ? __fmul_rn(pend_a, pend_b) : __fadd_rn(pend_a, pend_b); pend = nullptr; } };
+    auto finish_pending = [&]() { if (pend != nullptr) { *pend = epi == EPI_SILU_MUL ? __fmul_rn(pend_a, pend_b) : __fadd_rn(pend_a, pend_b); pend = nullptr; } };
     for (; n < n_stage; ++n) {
         const int  i = 32 * round + lane;
         const bool have = i < items;
         int        type = TYPE;
         uint16_t   dh = 0;
         if (TYPE != 12) {
-            const KqRow u = kq_unit(p, unit * pl.np, r & 1);
+            const KqRow u = kq_unit<EPI>(p, unit * pl.np, r & 1);
             type = u.type;
-            if (have && type != 12) { dh = __ldg(reinterpret_cast<const uint16_t *>(u.w + (int64_t)(p.pair_mode ? r >> 1 : r) * u.pitch + (size_t)nsb * 208) + sb); }   // (arrives while the copy is waited for)
+            if (have && type != 12) { dh = __ldg(reinterpret_cast<const uint16_t *>(u.w + (int64_t)(pair_mode ? r >> 1 : r) * u.pitch + (size_t)nsb * 208) + sb); }   // (arrives while the copy is waited for)
         }
         const uint32_t body = type == 12 ? 144u : 208u;
         const int before = min(lane, sb);        // super-blocks of the same row in front of this one in the round
@@ -439,6 +455,7 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
             for (int t = 0; t < TM; ++t) { part[t * items + i] = v[t]; }
         }
         sb += 32;
+#pragma unroll 1
         while (sb >= nsb) { sb -= nsb; ++r; }
         if (++round == n_round) {   // the unit is complete: lane = (column, row) adds a row's values in order
             __syncwarp();
@@ -455,15 +472,16 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
 #pragma unroll
                     for (int e = 0; e < 8; ++e) { sum = __fadd_rn(sum, f[e]); }
                 }
+#pragma unroll 1
                 for (; k < nsb; ++k) { sum = __fadd_rn(sum, q[k]); }
             }
             const float partner = __shfl_xor_sync(0xffffffffu, sum, 1);
             finish_pending();
-            if (p.epi == EPI_SILU_MUL) {
+            if (epi == EPI_SILU_MUL) {
                 if (t < nT && (ur & 1) == 0) { pend = p.out + (int64_t)t * p.out_stride + unit * pl.np + (ur >> 1); pend_a = sum; pend_b = p.silu_table[f2h(partner)]; }
-            } else if (p.epi == EPI_RESID) {
+            } else if (epi == EPI_RESID) {
                 if (t < nT) { const int64_t o = (int64_t)t * p.out_stride + 2 * unit * pl.np + ur; pend = p.out + o; pend_a = sum; pend_b = p.resid[o]; }
-            } else { matvec_epilogue(p, 2 * unit * pl.np + ur, t, sum, partner, t < nT); }
+            } else { matvec_epilogue<EPI>(p, 2 * unit * pl.np + ur, t, sum, partner, t < nT); }
             __syncwarp();   // (the values are overwritten by the next unit)
             r = r_0; sb = sb_0;
             round = 0; unit += pl.wact;
@@ -474,12 +492,13 @@ __global__ void __launch_bounds__(KQ_THREADS, 1) matvec_kq_kernel(const MatvecPa
         // a copy did not arrive: report, give the copies still in flight a last bounded chance to land and stop; the host sees the
         // flag at its next synchronisation
         if (lane == 0 && p.error_flag != nullptr) { atomicExch(p.error_flag, 1); }
+#pragma unroll 1
         for (int k = n; k < __shfl_sync(0xffffffffu, issued, 0); ++k) {
             mbar_wait_bounded(bar_s + slot * 8, parity, 10000000ull);
             if (++slot == pl.ns) { slot = 0; parity ^= 1u; }
         }
     }
-    tp_publish(p.tp, p.T);
+    if (EPI < 0) { tp_publish(p.tp, p.T); }
 }
 
 cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg) {
@@ -534,7 +553,23 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg) {
         // (narrow models: a layer's matrices of both types on one kernel, whose instructions the next launch finds in the caches; four layers of
         // Q4_K / Q6_K with d = 512, ff 1536: 125.2 -> 105.7 us a step; 1024, 2816: 129.3 -> 109.8; 2048, 5632: 137.0 -> 133.8; 3072, 8192: 188.2 ->
         // 186.9; but 4096, 11008: 227.2 -> 235.9)
-        kernel = p.narrow ? one[KQP_ANY][2] : one[n4 <= 2 * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : norm && n4 <= 3 * KQ_THREADS ? KQP_NORM_MID : n4 <= 2 * KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY][ty];
+        const int pro = n4 <= 2 * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : norm && n4 <= 3 * KQ_THREADS ? KQP_NORM_MID : n4 <= 2 * KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY;
+        kernel = p.narrow ? one[KQP_ANY][2] : one[pro][ty];
+        if (!p.narrow && p.tp.counter == nullptr && p.tp.flag_in == nullptr && (p.epi == EPI_SILU_MUL || p.epi == EPI_QKV_ROPE || p.kq_n == 1)) {
+            auto of_type = [&](auto pr, auto ep) -> Kernel {
+                constexpr int P = decltype(pr)::value, E = decltype(ep)::value;
+                return ty == 0 ? matvec_kq_kernel<1, 12, P, E> : ty == 1 ? matvec_kq_kernel<1, 14, P, E> : matvec_kq_kernel<1, 0, P, E>;
+            };
+            auto normed = [&](auto pr) -> Kernel {
+                return p.epi == EPI_QKV_ROPE ? of_type(pr, std::integral_constant<int, EPI_QKV_ROPE>{}) : p.epi == EPI_SILU_MUL ? of_type(pr, std::integral_constant<int, EPI_SILU_MUL>{})
+                     : p.epi == EPI_STORE ? of_type(pr, std::integral_constant<int, EPI_STORE>{}) : kernel;
+            };
+            if (pro == KQP_NORM) { kernel = normed(std::integral_constant<int, KQP_NORM>{}); }
+            else if (pro == KQP_NORM_MID) { kernel = normed(std::integral_constant<int, KQP_NORM_MID>{}); }
+            else if (pro == KQP_NORM_LONG) { kernel = normed(std::integral_constant<int, KQP_NORM_LONG>{}); }
+            else if (pro == KQP_PLAIN && p.epi == EPI_RESID) { kernel = of_type(std::integral_constant<int, KQP_PLAIN>{}, std::integral_constant<int, EPI_RESID>{}); }
+            else if (pro == KQP_PLAIN_LONG && p.epi == EPI_RESID) { kernel = of_type(std::integral_constant<int, KQP_PLAIN_LONG>{}, std::integral_constant<int, EPI_RESID>{}); }
+        }
     } else {
         static const Kernel more[2][3] = {{matvec_kq_kernel<2, 12, KQP_ANY>, matvec_kq_kernel<2, 14, KQP_ANY>, matvec_kq_kernel<2, 0, KQP_ANY>},
                                           {matvec_kq_kernel<KQ_MAX_COLUMNS, 12, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 14, KQP_ANY>, matvec_kq_kernel<KQ_MAX_COLUMNS, 0, KQP_ANY>}};
