@@ -64,7 +64,7 @@ __device__ __forceinline__ void unpack8(const uint4 v, float f[8]) {
 // of being held ahead in 248 registers, with which one CTA fills an SM. us a step of four layers, one CTA an SM / 2 / 3 / 4: 40 heads x 32 sequences at
 // 10 positions 1229 / 1162 / 1155 / 1161; 16 x 32 at 400 637 / 588 / 615 / 677; 32 x 16 at 200 740 / 717 / 726 / 753; 32 x 8 at 900 828 / 824 / 936 /
 // 1063 (more CTAs share an L1 that the V^T rows then leave).
-template <bool EARLY, int CTAS>
+template <bool EARLY, int CTAS, bool LEAN>
 __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const AttnParams p) {
     extern __shared__ __align__(16) float att_smem[];
     __shared__ float red[ATT_WARPS];
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     pdl_launch_dependents();
-    stamp(p.stamps, 0, false); stamp(p.stamps, 4, true);
+    if (!LEAN) { stamp(p.stamps, 0, false); stamp(p.stamps, 4, true); }
 
     const bool batch = p.seq_stride != 0;        // token t = sequence t of a batch in lockstep: own cache, same position, nothing else visible
     const __half *k_cache = p.k_cache + (batch ? (int64_t)t * p.seq_stride : 0), *v_cache = p.v_cache + (batch ? (int64_t)t * p.seq_stride : 0);
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
         request(0, early, ((early_tot - 1) / 32) * 32, false);
     }
     pdl_wait();
-    stamp(p.stamps, 1, false); stamp(p.stamps, 5, true);
+    if (!LEAN) { stamp(p.stamps, 1, false); stamp(p.stamps, 5, true); }
     const int2 base = __ldcg(reinterpret_cast<const int2 *>(p.pos_base));
     const __half q_mine = (tid < ATT_HD) ? p.q[(int64_t)t * p.dl + (int64_t)h * ATT_HD + tid] : __float2half(0.f);
     if (EARLY && early >= 0) { request(early & ~3, early + 1, ((early_tot - 1) / 32) * 32, true); }   // (without waiting for the counter)
@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
 
     // ---- masked softmax: (score + mask) * scale, subtract the maximum, table exp, std::reduce, multiply by 1/sum
     float m = -CUDART_INF_F;
+#pragma unroll 1
     for (int j = tid; j < n_vis; j += ATT_THREADS) {
         const float v = __fmul_rn(__fadd_rn(sc[j], 0.0f), p.scale);
         sc[j] = v;
@@ -238,10 +239,12 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
 #pragma unroll
     for (int w = 1; w < ATT_WARPS; ++w) { m = fmaxf(m, red[w]); }
     const int n_tot4 = (n_tot + 3) & ~3;
+#pragma unroll 1
     for (int j = tid; j < n_tot4; j += ATT_THREADS) { sc[j] = (j < n_vis) ? p.exp_table[f2h(__fsub_rn(sc[j], m))] : 0.f; }
     __syncthreads();
     // std::reduce: groups of four as (e0 + e1) + (e2 + e3), formed in parallel, then one thread's running sum; the
     // remainder (n_tot % 4 elements) is added one by one
+#pragma unroll 1
     for (int g = tid; g < (n_tot >> 2); g += ATT_THREADS) {
         const float4 v = reinterpret_cast<const float4 *>(sc)[g];
         gs[g] = __fadd_rn(__fadd_rn(v.x, v.y), __fadd_rn(v.z, v.w));
@@ -251,17 +254,21 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
         float sum = 0.f;
         const int ng = n_tot >> 2;
         int g = 0;
+#pragma unroll 1
         for (; g + 4 <= ng; g += 4) {
             const float4 v = *reinterpret_cast<const float4 *>(gs + g);
             sum = __fadd_rn(sum, v.x); sum = __fadd_rn(sum, v.y); sum = __fadd_rn(sum, v.z); sum = __fadd_rn(sum, v.w);
         }
+#pragma unroll 1
         for (; g < ng; ++g) { sum = __fadd_rn(sum, gs[g]); }
+#pragma unroll 1
         for (int j = ng << 2; j < n_tot; ++j) { sum = __fadd_rn(sum, sc[j]); }
         bcast = __fdiv_rn(1.0f, sum);
     }
     __syncthreads();
     const float inv = bcast;
     // probabilities, rounded to fp16 as the PV MatMul does with its f32 operand
+#pragma unroll 1
     for (int j = tid; j < n_vis; j += ATT_THREADS) { sc[j] = __half2float(__float2half_rn(__fmul_rn(sc[j], inv))); }
     __syncthreads();
 
@@ -336,8 +343,10 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
         }
         if (half == 0) { p.out[(int64_t)t * (p.out_stride ? p.out_stride : p.dl) + (int64_t)h * ATT_HD + e] = __fadd_rn(tail, simd); }
     }
-    tp_publish(p.tp, p.T);
-    if (p.stamps != nullptr) { __syncthreads(); stamp(p.stamps, 3, true); }
+    if (!LEAN) {
+        tp_publish(p.tp, p.T);
+        if (p.stamps != nullptr) { __syncthreads(); stamp(p.stamps, 3, true); }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1243,7 +1252,8 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
     const size_t smem = (n_pad + n_pad / 4 + ATT_HD) * sizeof(float) + 16;
     if (smem > 200 * 1024) { return cudaErrorInvalidValue; }
     const bool many = (int64_t)p.n_head * p.T > device_sms();
-    const void *kernel = reinterpret_cast<const void *>(many ? attention_kernel<false, ATT_MANY> : p.early && p.T == 1 && p.seq_stride == 0 ? attention_kernel<true, 1> : attention_kernel<false, 1>);
+    const void *kernel = reinterpret_cast<const void *>(many ? attention_kernel<false, ATT_MANY, false> : !(p.early && p.T == 1 && p.seq_stride == 0) ? attention_kernel<false, 1, false>
+                                                          : p.stamps == nullptr && p.tp.counter == nullptr ? attention_kernel<true, 1, true> : attention_kernel<true, 1, false>);
     cudaError_t err = allow_dynamic_smem(kernel, smem);
     if (err != cudaSuccess) { return err; }
     return launch_with_pdl(kernel, dim3(p.n_head, p.T, 1), dim3(ATT_THREADS), smem, p, cfg);
