@@ -59,6 +59,15 @@ __device__ __forceinline__ void unpack8(const uint4 v, float f[8]) {
     f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
 }
 
+// a * b + c of the f16 values in the low halves of a and b: the fmaf of the widened values (their product is exact in f32) without widening
+// them; it issues as fast as fmaf, and half the bytes of its operands come out of shared memory
+__device__ __forceinline__ float fma_f16(uint32_t a, uint32_t b, float c) {
+    float d;
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"((uint16_t)a), "h"((uint16_t)b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t half_of(const uint32_t *w, int i) { return w[i >> 1] >> (16 * (i & 1)); }
+
 // EARLY: a step that reads cache rows ahead of its wait (a kernel of its own: 7B steps 0.6 % slower with both in one)
 // CTAS > 1: for launches of more CTAs than SMs, so many of them side by side on one: a K row and the V^T values are read when they are needed instead
 // of being held ahead in 248 registers, with which one CTA fills an SM. us a step of four layers, one CTA an SM / 2 / 3 / 4: 40 heads x 32 sequences at
@@ -84,9 +93,10 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
     // the sum and where Dot<FP16,FP16> switches from its vector loop to the scalar tail.
     auto row_length = [&](int base, int known) { return batch ? base + 1 : known > 0 ? known : base + p.T; };
     const int n_pad = (p.n_ctx + 3) & ~3;
-    float *qf = att_smem;                        // [hd] Q as f32 (exact widening of the fp16 values)
-    float *sc = qf + ATT_HD;                     // [n_pad] scores, then probabilities
+    float *sc = att_smem;                        // [n_pad] scores, then exponentials
     float *gs = sc + n_pad;                      // [n_pad / 4] four-wide partial sums of std::reduce
+    __half *qh = reinterpret_cast<__half *>(gs + ((n_pad >> 2) + 3) / 4 * 4);   // [hd] Q, on 16 bytes
+    __half *ph = qh + ATT_HD;                    // [n_pad] probabilities
 
     // Everything this thread will need from global memory is requested up front, so that Q, the first K row and
     // the V^T values of the PV product share one memory round trip instead of three: the PV thread pair of element
@@ -151,14 +161,14 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
         for (int c = 0; c < 8; ++c) { v_tail[c] = make_uint2(0u, 0u); }
         request(0, n_vis, n_main, true);
     }
-    if (tid < ATT_HD) { qf[tid] = __half2float(q_mine); }
+    if (tid < ATT_HD) { qh[tid] = q_mine; }
     __syncthreads();
 
     // ---- scores of the visible positions: one thread per position
 #pragma unroll 1
     for (int j = tid; j < n_vis; j += ATT_THREADS) {
         const uint4  *krow = reinterpret_cast<const uint4 *>(k_cache + (int64_t)j * p.dl + (int64_t)h * ATT_HD);
-        const float4 *q4   = reinterpret_cast<const float4 *>(qf);
+        const uint2  *q2   = reinterpret_cast<const uint2 *>(qh);
         float acc[4][8];
         if (AHEAD && j != tid) {
 #pragma unroll
@@ -181,11 +191,11 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
             part(step);
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                float kf[8]; unpack8(kv[AHEAD ? 4 * step + a : a], kf);
-                const float4 qa = q4[(4 * step + a) * 2], qb = q4[(4 * step + a) * 2 + 1];
-                const float  qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+                const uint4 kw = kv[AHEAD ? 4 * step + a : a];
+                const uint2 qa = q2[(4 * step + a) * 2], qb = q2[(4 * step + a) * 2 + 1];
+                const uint32_t kh[4] = {kw.x, kw.y, kw.z, kw.w}, qv[4] = {qa.x, qa.y, qb.x, qb.y};
 #pragma unroll
-                for (int e = 0; e < 8; ++e) { acc[a][e] = fmaf(kf[e], qv[e], acc[a][e]); }
+                for (int e = 0; e < 8; ++e) { acc[a][e] = fma_f16(half_of(kh, e), half_of(qv, e), acc[a][e]); }
             }
         }
         float u[4];
@@ -200,11 +210,11 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
         part(3);
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            float kf[8]; unpack8(kv[AHEAD ? 12 + a : a], kf);
-            const float4 qa = q4[(12 + a) * 2], qb = q4[(12 + a) * 2 + 1];
-            const float  qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+            const uint4 kw = kv[AHEAD ? 12 + a : a];
+            const uint2 qa = q2[(12 + a) * 2], qb = q2[(12 + a) * 2 + 1];
+            const uint32_t kh[4] = {kw.x, kw.y, kw.z, kw.w}, qv[4] = {qa.x, qa.y, qb.x, qb.y};
 #pragma unroll
-            for (int e = 0; e < 8; ++e) { tail = fmaf(kf[e], qv[e], tail); }
+            for (int e = 0; e < 8; ++e) { tail = fma_f16(half_of(kh, e), half_of(qv, e), tail); }
         }
         sc[j] = __fadd_rn(tail, simd);
     }
@@ -269,7 +279,7 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
     const float inv = bcast;
     // probabilities, rounded to fp16 as the PV MatMul does with its f32 operand
 #pragma unroll 1
-    for (int j = tid; j < n_vis; j += ATT_THREADS) { sc[j] = __half2float(__float2half_rn(__fmul_rn(sc[j], inv))); }
+    for (int j = tid; j < n_vis; j += ATT_THREADS) { ph[j] = __float2half_rn(__fmul_rn(sc[j], inv)); }
     __syncthreads();
 
     // ---- out[e] = Dot<FP16,FP16>(V_t[e][0..n_tot), probs): a thread pair per element, thread `half` holding
@@ -287,12 +297,11 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
                 const int    j  = j0 + 8 * a + 4 * half;
-                const float4 pr = *reinterpret_cast<const float4 *>(sc + j);
-                const float2 v01 = __half22float2(*reinterpret_cast<const __half2 *>(&vv[a].x)), v23 = __half22float2(*reinterpret_cast<const __half2 *>(&vv[a].y));
-                if (j + 0 < n_vis) { acc[a][0] = fmaf(v01.x, pr.x, acc[a][0]); }
-                if (j + 1 < n_vis) { acc[a][1] = fmaf(v01.y, pr.y, acc[a][1]); }
-                if (j + 2 < n_vis) { acc[a][2] = fmaf(v23.x, pr.z, acc[a][2]); }
-                if (j + 3 < n_vis) { acc[a][3] = fmaf(v23.y, pr.w, acc[a][3]); }
+                const uint2  pr = *reinterpret_cast<const uint2 *>(ph + j);
+                if (j + 0 < n_vis) { acc[a][0] = fma_f16(vv[a].x, pr.x, acc[a][0]); }
+                if (j + 1 < n_vis) { acc[a][1] = fma_f16(vv[a].x >> 16, pr.x >> 16, acc[a][1]); }
+                if (j + 2 < n_vis) { acc[a][2] = fma_f16(vv[a].y, pr.y, acc[a][2]); }
+                if (j + 3 < n_vis) { acc[a][3] = fma_f16(vv[a].y >> 16, pr.y >> 16, acc[a][3]); }
             }
         };
         if (0 < n_main) { pv_step(v_first, 0); }
@@ -333,12 +342,11 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
         for (int c = 0; c < 8; ++c) {
             const int j = n_main + 4 * c;
             if (j < n_vis) {
-                const float4 pr = *reinterpret_cast<const float4 *>(sc + j);
-                const float2 v01 = __half22float2(*reinterpret_cast<const __half2 *>(&v_tail[c].x)), v23 = __half22float2(*reinterpret_cast<const __half2 *>(&v_tail[c].y));
-                tail = fmaf(v01.x, pr.x, tail);
-                if (j + 1 < n_vis) { tail = fmaf(v01.y, pr.y, tail); }
-                if (j + 2 < n_vis) { tail = fmaf(v23.x, pr.z, tail); }
-                if (j + 3 < n_vis) { tail = fmaf(v23.y, pr.w, tail); }
+                const uint2 pr = *reinterpret_cast<const uint2 *>(ph + j);
+                tail = fma_f16(v_tail[c].x, pr.x, tail);
+                if (j + 1 < n_vis) { tail = fma_f16(v_tail[c].x >> 16, pr.x >> 16, tail); }
+                if (j + 2 < n_vis) { tail = fma_f16(v_tail[c].y, pr.y, tail); }
+                if (j + 3 < n_vis) { tail = fma_f16(v_tail[c].y >> 16, pr.y >> 16, tail); }
             }
         }
         if (half == 0) { p.out[(int64_t)t * (p.out_stride ? p.out_stride : p.dl) + (int64_t)h * ATT_HD + e] = __fadd_rn(tail, simd); }
@@ -433,15 +441,6 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(const AttnParams p) {
     }
     p.scratch[((int64_t)t * p.n_head + h) * n_pad + j] = score_dot(kv, reinterpret_cast<const float4 *>(qf));
 }
-
-// a * b + c of the f16 values in the low halves of a and b: the fmaf of the widened values (their product is exact in f32) without widening
-// them; it issues as fast as fmaf, and half the bytes of its operands come out of shared memory
-__device__ __forceinline__ float fma_f16(uint32_t a, uint32_t b, float c) {
-    float d;
-    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"((uint16_t)a), "h"((uint16_t)b), "f"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t half_of(const uint32_t *w, int i) { return w[i >> 1] >> (16 * (i & 1)); }
 
 // The same for a prompt, register-tiled: a CTA takes ATT_SG times ATT_ST tokens x ATT_SP positions of a head, a lane 4 tokens x 8
 // positions at a time. The 32 accumulators of a dot product are walked element by element of the CPU's eight-wide vectors: element e of
@@ -1211,7 +1210,7 @@ int attention_early(int n_head, int n_ctx, bool kq) { return !kq || n_head <= 8 
 // of 8-layer models with little beside the attention, us a layer: 2 heads 248: 17.7 / 18.2, 280: 18.7 / 18.4; 8 heads 248: 20.6 / 21.4, 280: 21.5 / 21.5;
 // 16 heads 216: 24.9 / 24.7, 248: 25.5 / 24.7; 24 heads 248: 29.0 / 29.1, 280: 29.9 / 29.3; 32 heads 248: 32.0 / 32.5, 280: 33.1 / 32.7; 40 heads 248:
 // 41.7 / 42.2, 280: 42.7 / 42.5. They meet between 210 (16 heads) and 280: 240 is off by at most 4 % of such a layer.
-constexpr int ATT_CLUSTER_POS = 240, ATT_ONE_CTA_CTX = 8192;   // (the score row of the longest context: 40 KB)
+constexpr int ATT_CLUSTER_POS = 240, ATT_ONE_CTA_CTX = 8192;   // (the rows of the longest context: 57 KB)
 int attention_form(const AttnParams &p, const LaunchCfg &cfg, int pos) {
     if (p.T != 1 || p.seq_stride != 0 || p.n_ctx > ATT_ONE_CTA_CTX || !atl_fits(p, cfg)) { return ATT_BY_CONTEXT; }
     return pos < ATT_CLUSTER_POS ? ATT_ONE_CTA : ATT_CLUSTER;
@@ -1249,7 +1248,7 @@ cudaError_t launch_attention(const AttnParams &p, const LaunchCfg &cfg) {
         if (err != cudaSuccess) { return err; }
         return launch_with_pdl(reinterpret_cast<const void *>(attn_pv_kernel), dim3(p.n_head * (ATT_HD / ATT_PV_WARPS), p.T), dim3(ATT_PV_WARPS * WARP), pv_smem, p, cfg);
     }
-    const size_t smem = (n_pad + n_pad / 4 + ATT_HD) * sizeof(float) + 16;
+    const size_t smem = (n_pad + (n_pad / 4 + 3) / 4 * 4) * sizeof(float) + (n_pad + ATT_HD) * sizeof(__half) + 16;   // (contexts of up to ATT_ONE_CTA_CTX positions; longer ones have a scratch)
     if (smem > 200 * 1024) { return cudaErrorInvalidValue; }
     const bool many = (int64_t)p.n_head * p.T > device_sms();
     const void *kernel = reinterpret_cast<const void *>(many ? attention_kernel<false, ATT_MANY, false> : !(p.early && p.T == 1 && p.seq_stride == 0) ? attention_kernel<false, 1, false>

@@ -772,7 +772,7 @@ def test_fused_attention_long_rows(be, oracle, pos0, t, n_total, n_ctx):
     assert np.array_equal(bits(got), bits(want))
 
 
-@pytest.mark.parametrize("pos0,t,n_total,n_ctx", [(0, 5, 0, 64), (20, 7, 0, 128), (31, 6, 40, 64), (60, 5, 70, 128), (255, 6, 300, 512), (700, 5, 0, 1024), (1019, 5, 0, 1024)])
+@pytest.mark.parametrize("pos0,t,n_total,n_ctx", [(0, 5, 0, 64), (20, 7, 0, 132), (31, 6, 40, 60), (60, 5, 70, 128), (255, 6, 300, 516), (700, 5, 0, 1024), (1015, 5, 0, 1020)])
 def test_fused_attention_of_more_ctas_than_sms(be, oracle, pos0, t, n_total, n_ctx):
     """More (head, token) pairs than the chip has SMs: the kernel of which an SM holds two CTAs, across the same boundaries."""
     rng = np.random.default_rng(pos0 + n_ctx + t)
