@@ -369,59 +369,38 @@ __global__ void __launch_bounds__(ATT_THREADS, CTAS) attention_kernel(const Attn
 // HBM-bound: the K rows and the V^T rows of the visible positions are read once (2 * n_kv * 128 * 2 bytes per head).
 constexpr int ATT_LONG_MIN = 1024;
 
-// Dot<FP16,FP16>(K row, Q) with the K row in registers (16 x 8 fp16) and Q as 128 floats in shared memory: 4 x 8
-// accumulators over elements 0..95, the reduction tree, the scalar chain over elements 96..127, tail + simd
-__device__ __forceinline__ float score_dot(const uint4 (&kv)[16], const float4 *q4) {
-    // the 4 x 8 accumulators as 4 x 4 packed f32x2 pairs (elements 2 p, 2 p + 1 of an accumulator step): one fma.rn.f32x2 is two
-    // of the scalar FMAs, bit for bit
-    uint64_t acc2[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { acc2[a][e] = 0ull; }
-    }
-#pragma unroll
-    for (int step = 0; step < 3; ++step) {       // elements 0..95: accumulator a takes elements 32 * step + 8a .. + 7
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const uint4 kw = kv[4 * step + a];
-            const float2 k0 = __half22float2(*reinterpret_cast<const __half2 *>(&kw.x)), k1 = __half22float2(*reinterpret_cast<const __half2 *>(&kw.y));
-            const float2 k2 = __half22float2(*reinterpret_cast<const __half2 *>(&kw.z)), k3 = __half22float2(*reinterpret_cast<const __half2 *>(&kw.w));
-            const float4 qa = q4[(4 * step + a) * 2], qb = q4[(4 * step + a) * 2 + 1];
-            acc2[a][0] = f2_fma(f2_pack(k0.x, k0.y), f2_pack(qa.x, qa.y), acc2[a][0]);
-            acc2[a][1] = f2_fma(f2_pack(k1.x, k1.y), f2_pack(qa.z, qa.w), acc2[a][1]);
-            acc2[a][2] = f2_fma(f2_pack(k2.x, k2.y), f2_pack(qb.x, qb.y), acc2[a][2]);
-            acc2[a][3] = f2_fma(f2_pack(k3.x, k3.y), f2_pack(qb.z, qb.w), acc2[a][3]);
-        }
-    }
+// Dot<FP16,FP16>(K row, Q): kv(a) is the row's 16-byte piece a, q_s the address of Q as f16 in shared memory. 4 x 8 accumulators over
+// elements 0..95, the reduction tree, the scalar chain over elements 96..127, tail + simd
+template <class KV>
+__device__ __forceinline__ float score_dot(KV kv, uint32_t q_s) {
     float acc[4][8];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
+    for (int a = 0; a < 16; ++a) {               // elements 0..95: accumulator a % 4 takes elements 8 a .. 8 a + 7
+        uint32_t kw[4], qw[4];
+        *reinterpret_cast<uint4 *>(kw) = kv(a); *reinterpret_cast<uint4 *>(qw) = lds128(q_s + 16 * a);
+        if (a < 12) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { f2_unpack(acc2[a][e], acc[a][2 * e], acc[a][2 * e + 1]); }
+            for (int e = 0; e < 8; ++e) { acc[a & 3][e] = fma_f16(half_of(kw, e), half_of(qw, e), a < 4 ? 0.f : acc[a & 3][e]); }
+            continue;
+        }
+        if (a == 12) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float lo = __fadd_rn(__fadd_rn(acc[0][e], acc[2][e]), __fadd_rn(acc[1][e], acc[3][e]));
+                const float hi = __fadd_rn(__fadd_rn(acc[0][e + 4], acc[2][e + 4]), __fadd_rn(acc[1][e + 4], acc[3][e + 4]));
+                acc[0][e] = __fadd_rn(lo, hi);
+            }
+            acc[0][0] = __fadd_rn(__fadd_rn(acc[0][0], acc[0][1]), __fadd_rn(acc[0][2], acc[0][3]));
+            acc[1][0] = 0.f;                     // elements 96..127: scalar chain
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { acc[1][0] = fma_f16(half_of(kw, e), half_of(qw, e), acc[1][0]); }
     }
-    float u[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const float lo = __fadd_rn(__fadd_rn(acc[0][e], acc[2][e]), __fadd_rn(acc[1][e], acc[3][e]));
-        const float hi = __fadd_rn(__fadd_rn(acc[0][e + 4], acc[2][e + 4]), __fadd_rn(acc[1][e + 4], acc[3][e + 4]));
-        u[e] = __fadd_rn(lo, hi);
-    }
-    const float simd = __fadd_rn(__fadd_rn(u[0], u[1]), __fadd_rn(u[2], u[3]));
-    float tail = 0.f;                             // elements 96..127: scalar chain
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        float kf[8]; unpack8(kv[12 + a], kf);
-        const float4 qa = q4[(12 + a) * 2], qb = q4[(12 + a) * 2 + 1];
-        const float  qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-#pragma unroll
-        for (int e = 0; e < 8; ++e) { tail = fmaf(kf[e], qv[e], tail); }
-    }
-    return __fadd_rn(tail, simd);
+    return __fadd_rn(acc[1][0], acc[0][0]);
 }
 
 __global__ void __launch_bounds__(256) attn_scores_kernel(const AttnParams p) {
-    __shared__ __align__(16) float qf[ATT_HD];
+    __shared__ __align__(16) __half qh[ATT_HD];
     const int h = blockIdx.y, t = blockIdx.z, tid = threadIdx.x;
     pdl_launch_dependents();
     pdl_wait();
@@ -429,7 +408,7 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(const AttnParams p) {
     const int n_vis = p.pos_base[0] + (batch ? 0 : t) + 1;
     if ((int)blockIdx.x * 256 >= n_vis) { return; }
     const int n_pad = (p.n_ctx + 3) & ~3;
-    if (tid < ATT_HD) { qf[tid] = __half2float(p.q[(int64_t)t * p.dl + (int64_t)h * ATT_HD + tid]); }
+    if (tid < ATT_HD) { qh[tid] = p.q[(int64_t)t * p.dl + (int64_t)h * ATT_HD + tid]; }
     __syncthreads();
     const int j = blockIdx.x * 256 + tid;
     if (j >= n_vis) { return; }
@@ -439,7 +418,7 @@ __global__ void __launch_bounds__(256) attn_scores_kernel(const AttnParams p) {
 #pragma unroll
         for (int a = 0; a < 16; ++a) { kv[a] = krow[a]; }
     }
-    p.scratch[((int64_t)t * p.n_head + h) * n_pad + j] = score_dot(kv, reinterpret_cast<const float4 *>(qf));
+    p.scratch[((int64_t)t * p.n_head + h) * n_pad + j] = score_dot([&](int a) { return kv[a]; }, smem_u32(qh));
 }
 
 // The same for a prompt, register-tiled: a CTA takes ATT_SG times ATT_ST tokens x ATT_SP positions of a head, a lane 4 tokens x 8
@@ -798,7 +777,7 @@ struct AtlSmem { size_t ex, gs, rs, red, bars, ring; };   // gs: the sums of fou
 __host__ __device__ static inline AtlSmem atl_smem(int n_ctx) {   // offsets in bytes; q lies in front
     const size_t n32 = ((size_t)n_ctx + 31) & ~(size_t)31;
     AtlSmem L;
-    L.ex = ATT_HD * 4; L.gs = L.ex + n32 * 4; L.rs = L.gs + 2 * n32; L.red = L.rs + rs_scratch_words(4) * 4; L.bars = L.red + (ATL_C * ATL_WARPS + 4) * 4;
+    L.ex = ATT_HD * 2; L.gs = L.ex + n32 * 4; L.rs = L.gs + 2 * n32; L.red = L.rs + rs_scratch_words(4) * 4; L.bars = L.red + (ATL_C * ATL_WARPS + 4) * 4;
     L.ring = (L.bars + (2 * ATL_MAX_STAGES + 2) * 8 + 127) / 128 * 128;
     return L;
 }
@@ -810,10 +789,12 @@ __device__ __forceinline__ void atl_wait(uint32_t bar, uint32_t parity, uint64_t
     if (limit_ns == 0 || !mbar_wait_prompt(bar, parity, limit_ns)) { limit_ns = 0; }
 }
 
-__global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const AttnParams p, const int NS) {
+__global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const AttnParams p, const int ns_log) {
+    const int NS = 1 << ns_log;
     extern __shared__ __align__(128) uint8_t atl_raw[];
     const AtlSmem L = atl_smem(p.n_ctx);
-    float *qf = reinterpret_cast<float *>(atl_raw), *ex = reinterpret_cast<float *>(atl_raw + L.ex), *gs = reinterpret_cast<float *>(atl_raw + L.gs);
+    __half *qh = reinterpret_cast<__half *>(atl_raw);
+    float *ex = reinterpret_cast<float *>(atl_raw + L.ex), *gs = reinterpret_cast<float *>(atl_raw + L.gs);
     float *rs = reinterpret_cast<float *>(atl_raw + L.rs), *red = reinterpret_cast<float *>(atl_raw + L.red);
     const uint32_t ring_s = smem_u32(atl_raw + L.ring), full_s = smem_u32(atl_raw + L.bars), empty_s = full_s + 8 * ATL_MAX_STAGES;
     const uint32_t max_s = empty_s + 8 * ATL_MAX_STAGES, exp_s = max_s + 8;
@@ -838,8 +819,8 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
         const __half *V = p.v_cache + (batch ? (int64_t)t * p.seq_stride : 0) + ((int64_t)h * ATT_HD + rank * (ATT_HD / ATL_C)) * p.n_ctx;
         const int total = nK + 4 * nC;
         for (int g = warp - ATL_WARPS; g < total; g += ATL_COPY_WARPS) {   // (atl_copy_warp)
-            const int slot = g % NS;
-            if (g >= NS) { atl_wait(empty_s + 8 * slot, (uint32_t)(g / NS - 1) & 1u, limit); }
+            const int slot = g & (NS - 1);
+            if (g >= NS) { atl_wait(empty_s + 8 * slot, (uint32_t)((g >> ns_log) - 1) & 1u, limit); }
             if (!__all_sync(0xffffffffu, limit != 0)) { break; }
             const uint32_t bar = full_s + 8 * slot, dst = ring_s + slot * ATL_STAGE;
             if (g < nK) {
@@ -858,19 +839,16 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
         }
         asm volatile("cp.async.wait_all;" ::: "memory");   // no copy is in flight when the CTA ends, also when its readers gave up
     } else {
-        if (tid < ATT_HD) { qf[tid] = __half2float(p.q[(int64_t)t * p.dl + (int64_t)h * ATT_HD + tid]); }
+        if (tid < ATT_HD) { qh[tid] = p.q[(int64_t)t * p.dl + (int64_t)h * ATT_HD + tid]; }
         asm volatile("bar.sync 2, 256;" ::: "memory");
         // scores of this CTA's positions, a tile of 32 per warp, a position per lane
         float m = -CUDART_INF_F;
         const int n_score = atl_score_warps(NS);
         for (int k = warp; warp < n_score && k < nK; k += n_score) {   // (atl_reader)
-            const int slot = k % NS;
-            atl_wait(full_s + 8 * slot, (uint32_t)(k / NS) & 1u, limit);
-            uint4 kv[16];
+            const int slot = k & (NS - 1);
+            atl_wait(full_s + 8 * slot, (uint32_t)(k >> ns_log) & 1u, limit);
             const uint32_t src = ring_s + slot * ATL_STAGE + lane * ATL_KPITCH;
-#pragma unroll
-            for (int a = 0; a < 16; ++a) { kv[a] = lds128(src + 16 * a); }
-            const float s = score_dot(kv, reinterpret_cast<const float4 *>(qf));
+            const float s = score_dot([=](int a) { return lds128(src + 16 * a); }, smem_u32(qh));
             __syncwarp();
             if (lane == 0) { mbar_arrive(empty_s + 8 * slot); }
             const int  j = 32 * k + lane;
@@ -887,6 +865,10 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
         cluster_wait(max_s, 0u, limit);
         m = warp_max(red[lane]);
         // exponentials and their sums of four, to all CTAs of the cluster
+        uint32_t there[ATL_C];   // the rows `ex` of the CTAs
+#pragma unroll
+        for (int r = 0; r < ATL_C; ++r) { there[r] = cluster_map(smem_u32(ex), r); }
+#pragma unroll 1
         for (int k0 = warp; k0 < nK; k0 += 4 * ATL_WARPS) {
             float e[4];
 #pragma unroll
@@ -899,11 +881,11 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
                 const int k = k0 + i * ATL_WARPS, j = 32 * k + lane;
                 if (k < nK) {   // uniform in the warp
                     const float two = __fadd_rn(e[i], __shfl_xor_sync(0xffffffffu, e[i], 1)), four = __fadd_rn(two, __shfl_xor_sync(0xffffffffu, two, 2));
-                    const uint32_t to = smem_u32(ex + start + j), to4 = smem_u32(gs + ((start + j) >> 2));
+                    const uint32_t to = 4u * (start + j), to4 = (uint32_t)(L.gs - L.ex) + start + j;   // (4 bytes per four values)
 #pragma unroll
                     for (int r = 0; r < ATL_C; ++r) {
-                        cluster_store(cluster_map(to, r), e[i]);
-                        if ((lane & 3) == 0) { cluster_store(cluster_map(to4, r), four); }
+                        cluster_store(there[r] + to, e[i]);
+                        if ((lane & 3) == 0) { cluster_store(there[r] + to4, four); }
                     }
                 }
             }
@@ -943,8 +925,8 @@ __global__ void __launch_bounds__(ATL_THREADS, 2) attn_cluster_kernel(const Attn
                 for (int i = 0; i < 8; ++i) { if (i < valid) { acc[i] = fma_f16(vw[i >> 1] >> (16 * (i & 1)), pw[i >> 1] >> (16 * (i & 1)), acc[i]); } }
             };
             for (int c = 0; c < nC; ++c) {
-                const int g = nK + 4 * c + warp, slot = g % NS;
-                atl_wait(full_s + 8 * slot, (uint32_t)(g / NS) & 1u, limit);
+                const int g = nK + 4 * c + warp, slot = g & (NS - 1);
+                atl_wait(full_s + 8 * slot, (uint32_t)(g >> ns_log) & 1u, limit);
                 const uint32_t row = ring_s + slot * ATL_STAGE + (lane >> 2) * ATL_VPITCH;
                 const int p0 = c * ATL_VCH, steps = min(ATL_VCH / 32, n_full - c * (ATL_VCH / 32));
 #pragma unroll 4
@@ -1187,7 +1169,8 @@ static cudaError_t launch_attn_cluster(const AttnParams &p, const LaunchCfg &cfg
     lc.attrs = attr; lc.numAttrs = cfg.pdl ? 2 : 1;
     AttnParams q = p;
     if (q.error_flag == nullptr) { q.error_flag = cfg.error_flag; }
-    void *args[] = {&q, &ns};
+    int ns_log = ns == 16 ? 4 : ns == 8 ? 3 : 2;   // (atl_stage_count: 4, 8 or 16)
+    void *args[] = {&q, &ns_log};
     return cudaLaunchKernelExC(&lc, reinterpret_cast<const void *>(attn_cluster_kernel), args);
 }
 
