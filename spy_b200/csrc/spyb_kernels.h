@@ -67,10 +67,8 @@ struct KqSeg {
     int64_t row_bytes = 0;
 };
 
-constexpr int MV_NARROW = 3072;   // widest d_model of a narrow model
 struct MatvecParams {
     int   stages_early = 64;          // single column, kernels built for one prologue: stages of each warp's ring whose copies are issued ahead of x (set at the launch)
-    int   narrow = 0;                 // the matrix of a narrow model (MV_NARROW): single columns on the kernel that serves all of a layer's
     DevMatrix A;
     DevMatrix B;               // second matrix when pair_mode == 1 (same shape as A)
     int       pair_mode = 0;   // 1: a warp's tile is rows 4u..4u+3 of A together with the same rows of B (FFN up and gate)

@@ -550,12 +550,12 @@ cudaError_t launch_matvec_kq(const MatvecParams &p, const LaunchCfg &cfg) {
             {matvec_kq_kernel<1, 12, KQP_PLAIN_LONG>, matvec_kq_kernel<1, 14, KQP_PLAIN_LONG>, matvec_kq_kernel<1, 0, KQP_PLAIN_LONG>}};
         const int64_t n4 = p.A.k >> 2;
         const bool norm = p.pro == PRO_NORM_QUANT;
-        // (narrow models: a layer's matrices of both types on one kernel, whose instructions the next launch finds in the caches; four layers of
-        // Q4_K / Q6_K with d = 512, ff 1536: 125.2 -> 105.7 us a step; 1024, 2816: 129.3 -> 109.8; 2048, 5632: 137.0 -> 133.8; 3072, 8192: 188.2 ->
-        // 186.9; but 4096, 11008: 227.2 -> 235.9)
+        // (One kernel for all of a layer's matrices, whose instructions the next launch finds in the caches, was the faster one below d = 3072 while
+        // each held the code of every epilogue. Eight layers of Q4_K / Q6_K, that kernel / these: d = 512, ff 1024: 197.8 / 188.5 us a step; 1536, 3072:
+        // 223.6 / 203.7; 2560, 5120: 320.4 / 285.2; 3072, 6144: 341.0 / 299.5.)
         const int pro = n4 <= 2 * KQ_THREADS ? (norm ? KQP_NORM : KQP_PLAIN) : norm && n4 <= 3 * KQ_THREADS ? KQP_NORM_MID : n4 <= 2 * KQ_PRO_GROUPS * KQ_THREADS ? (norm ? KQP_NORM_LONG : KQP_PLAIN_LONG) : KQP_ANY;
-        kernel = p.narrow ? one[KQP_ANY][2] : one[pro][ty];
-        if (!p.narrow && p.tp.counter == nullptr && p.tp.flag_in == nullptr && (p.epi == EPI_SILU_MUL || p.epi == EPI_QKV_ROPE || p.kq_n == 1)) {
+        kernel = one[pro][ty];
+        if (p.tp.counter == nullptr && p.tp.flag_in == nullptr && (p.epi == EPI_SILU_MUL || p.epi == EPI_QKV_ROPE || p.kq_n == 1)) {
             auto of_type = [&](auto pr, auto ep) -> Kernel {
                 constexpr int P = decltype(pr)::value, E = decltype(ep)::value;
                 return ty == 0 ? matvec_kq_kernel<1, 12, P, E> : ty == 1 ? matvec_kq_kernel<1, 14, P, E> : matvec_kq_kernel<1, 0, P, E>;

@@ -125,12 +125,12 @@ cudaError_t allow_dynamic_smem(const void *kernel, size_t bytes) {
 // (Eight values a thread: a 256-bit load each, half the shuffles and lane bookkeeping of groups of four. Behind the last read of 11008 values:
 // 2.1 us with groups of four, two quotients each and the conversion unit, 1.3 now; a 7B Q4_0 layer 45.9 -> 44.8 us.)
 constexpr int PRO_GROUPS = 3;
-// SUM: how the sum of squares is formed. SUM_FEW: by one thread in few registers (kernels with other paths to serve); SUM_CHAIN: by one thread
-// that reads ahead; SUM_WIDE (kernels of their own per prologue): the sum of squares runs on four warps and the
+// SUM: how the sum of squares is formed. SUM_FEW: by one thread in few registers (kernels with other paths to serve);
+// SUM_WIDE (kernels of their own per prologue): the sum of squares runs on four warps and the
 // norm weights of rows of at most NORM_EARLY * 4096 values are read at the start of the kernel, in front of the weight copies: behind a ring
 // full of them on every SM they arrive after the sum of squares is done.
 constexpr int NORM_EARLY = 2;
-enum { SUM_FEW, SUM_CHAIN, SUM_WIDE };
+enum { SUM_FEW, SUM_WIDE };
 template <int PG>
 __device__ __forceinline__ void norm_weights_early(const MatvecParams &p, float (&w)[PG][8]) {
     const int n8 = (int)(p.A.k >> 3);
@@ -214,7 +214,7 @@ __device__ __forceinline__ void matvec_prologue_1col(const MatvecParams &p, ActP
         __shared__ __align__(16) float rs_scratch[EARLY ? rs_scratch_words(CQ) : 4];
         float sum = 0.f;
         if (EARLY && n4 >= RS_MIN) { if (tid < RS_THREADS) { sum = running_sum_chunks<EARLY ? CQ : 2>(smem_u32(v3), n4, smem_u32(rs_scratch), tid, 1); } }
-        else if (tid == 0) { sum = EARLY ? running_sum_cold(smem_u32(v3), n4) : SUM == SUM_CHAIN ? running_sum_serial(smem_u32(v3), n4) : running_sum_small(v3, n4); }
+        else if (tid == 0) { sum = EARLY ? running_sum_cold(smem_u32(v3), n4) : running_sum_small(v3, n4); }
         if (tid == 0) {
             const float mean = __fdiv_rn(sum, (float)p.A.k);
             scales[0] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
@@ -524,10 +524,10 @@ __global__ void __launch_bounds__(MV_THREADS, (TM == 1) ? 2 : 1) matvec_kernel(c
 // number of columns.
 // (One kernel with all of them takes 121 registers instead of 79 and its loop is scheduled worse. A Q4_0 layer of a 7B step, with the
 // evict-first copies, the early norm weights and the late ring: 49.1 -> 43.7 us.)
-// MVP_ONE: any single column, for narrow models: a layer's four matrices on one kernel. There a launch is short, and the next one finding its
-// instructions in the caches is worth more than a better loop (four layers of d = 512, ff 5632, Q4_0: 102.3 -> 94.1 us a step; 1024, 2816:
-// 99.6 -> 93.5; 2048, 5632: 121.4 -> 117.7; 3072, 8192: 158.1 -> 153.8; but 4096, 11008: 188.2 -> 190.9).
-enum { MVP_ANY, MVP_NORM, MVP_NORM_MID, MVP_PLAIN, MVP_NORM_LONG, MVP_PLAIN_LONG, MVP_ONE };
+// (One kernel for all four matrices of a layer, whose instructions the next launch finds in the caches, was the faster one below d = 3072 while
+// each held the code of every epilogue. Eight layers, that kernel / these with their own epilogue, Q4_0: d = 512, ff 1024: 142.6 / 135.5 us a step;
+// 1536, 3072: 185.0 / 177.2; 2560, 5120: 233.7 / 219.4; 3072, 6144: 257.1 / 237.6; Q8_0: 144.3 / 136.4, 189.7 / 181.5, 248.2 / 234.2, 278.8 / 263.3.)
+enum { MVP_ANY, MVP_NORM, MVP_NORM_MID, MVP_PLAIN, MVP_NORM_LONG, MVP_PLAIN_LONG };
 template <int WT, int TM, int LPR, int PRO, int EPI = -1>
 __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const MatvecParams p, const int ring_bytes, const int S, const int wact) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -600,14 +600,6 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_rows_kernel(const Matvec
     {
         float *v3 = reinterpret_cast<float *>(smem_raw);
         if constexpr (PRO == MVP_ANY) { matvec_prologue<TM, true>(p, act, v3, norm_scales); }
-        else if constexpr (PRO == MVP_ONE) {
-            const bool norm = p.pro == PRO_NORM_QUANT;
-            if (nbp * 8 <= 2 * MV_THREADS) {
-                if (norm) { matvec_prologue_1col<1, true, SUM_CHAIN, true, true>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<1, false, SUM_FEW, true, true>(p, act, v3, norm_scales, nullptr, rest); }
-            } else {
-                if (norm) { matvec_prologue_1col<PRO_GROUPS, true, SUM_CHAIN, true, true>(p, act, v3, norm_scales, nullptr, rest); } else { matvec_prologue_1col<PRO_GROUPS, false, SUM_FEW, true, true>(p, act, v3, norm_scales, nullptr, rest); }
-            }
-        }
         else {
             constexpr bool NORM = PRO == MVP_NORM || PRO == MVP_NORM_MID || PRO == MVP_NORM_LONG;
             constexpr int  PG = (PRO == MVP_NORM || PRO == MVP_PLAIN) ? 1 : PRO == MVP_NORM_MID ? 2 : PRO_GROUPS;
@@ -957,8 +949,7 @@ static cudaError_t launch_matvec_rows_t(const MatvecParams &p, const LaunchCfg &
             constexpr int P = decltype(pro)::value;
             return lean && p.epi == EPI_RESID ? matvec_rows_kernel<WT, 1, LPR, P, EPI_RESID> : matvec_rows_kernel<WT, 1, LPR, P>;
         };
-        if (p.narrow && n4p <= 2 * PRO_GROUPS * MV_THREADS) { kernel = matvec_rows_kernel<WT, 1, LPR, MVP_ONE>; }
-        else if (n4p <= 2 * MV_THREADS) { kernel = norm ? normed(std::integral_constant<int, MVP_NORM>{}) : plain(std::integral_constant<int, MVP_PLAIN>{}); }
+        if (n4p <= 2 * MV_THREADS) { kernel = norm ? normed(std::integral_constant<int, MVP_NORM>{}) : plain(std::integral_constant<int, MVP_PLAIN>{}); }
         else if (norm && n4p <= 3 * MV_THREADS) { kernel = normed(std::integral_constant<int, MVP_NORM_MID>{}); }
         else if (n4p <= 2 * PRO_GROUPS * MV_THREADS) { kernel = norm ? normed(std::integral_constant<int, MVP_NORM_LONG>{}) : plain(std::integral_constant<int, MVP_PLAIN_LONG>{}); }
     }

@@ -395,7 +395,6 @@ spyb_status run_step(spyb_model *m, bool tap, int64_t *launches) {
 // the weights of one mat-vec of the step plan: kind 0 = Wq|Wk|Wv, 1 = Wo, 2 = up|gate, 3 = down, 4 = output head
 void set_weights(const spyb_model *m, const Layer *ly, int kind, MatvecParams &p) {
     const int d = m->info.d_model;
-    p.narrow = d <= MV_NARROW;
     if (m->kq) {
         DevMatrix A;   // only the shape is used
         A.type = SPYB_Q4_K; A.k = (kind == 3) ? m->info.n_ff : d; A.nb = (int)(A.k / 32); A.nbp = A.nb;
