@@ -762,6 +762,8 @@ __global__ void __launch_bounds__(ATT_PV_WARPS * WARP) attn_pv_kernel(const Attn
 // both through one ring of stages (32 K rows of 256 bytes, or 512 positions of eight V^T rows) without regard to the phases: while the
 // softmax is formed, V^T fills the ring. (cp.async, 512 bytes an instruction: bulk copies of a row each cost the warp 50 cycles, 54 us in all.) A stage is filled for one warp: no CTA-wide waits on the way.
 // 32 heads over 4000 positions, three kernels (scores, softmax, PV) before: 41 us, now about 22; the reads take 10.3.
+// (Q as f16 and products of f16 values by one instruction, stages counted by shifts, the other CTAs' rows mapped once: steps of eight layers, Q8_0 at 3968
+// positions 520.4 -> 518.4 us, Q4_0 at 250 335.3 -> 333.4, at 900 355.9 -> 353.7.)
 constexpr int ATL_C = 4, ATL_WARPS = 8, ATL_COPY_WARPS = 4, ATL_THREADS = (ATL_WARPS + ATL_COPY_WARPS) * WARP;
 constexpr int ATL_KPITCH = 272, ATL_VCH = 512, ATL_VROWS = 8, ATL_VPITCH = 2 * ATL_VCH + 64, ATL_STAGE = 32 * ATL_KPITCH;   // pitches without bank conflicts
 static_assert(ATL_VROWS * ATL_VPITCH == ATL_STAGE && ATL_C * 4 * ATL_VROWS == ATT_HD, "both kinds of stages fill the slot; four warps take a CTA's elements");
@@ -1185,7 +1187,8 @@ size_t attention_scratch_floats(int n_ctx, int n_head, int T) {   // 0: the sing
 // the early ones save. Steps of 4 layers, us, reads behind the wait / early, behind 20, 60, 220 positions. A context of 844: Q4_K_M 8 heads 104.7 /
 // 103.2, 106.5 / 103.4, 113.1 / 107.5; 12 heads 110.8 / 112.1, 113.1 / 114.7, 122.3 / 130.0; 20 heads 158.7 / 159.2, 160.7 / 161.8, 170.2 / 176.9; 32 heads 192.5 /
 // 191.7, 194.0 / 192.5, 203.8 / 201.5; Q4_0 12 heads 99.3 / 98.3, 101.1 / 99.6, 107.2 / 107.8. A context of 512: Q4_K_M 12 heads 111.6 / 111.1, 113.6 / 111.9, 123.6 /
-// 128.3; 24 heads 170.2 / 167.9, 172.3 / 168.9, 184.1 / 185.3.
+// 128.3; 24 heads 170.2 / 167.9, 172.3 / 168.9, 184.1 / 185.3. (With the kernels as they are, 8 layers, a context of 844, behind 10, 150 and 215: 10 heads
+// 185.2 / 184.0, 199.8 / 202.7, 209.1 / 217.8; 16 heads 206.8 / 206.9, 222.1 / 222.1, 231.2 / 237.4; 24 heads 293.4 / 292.3, 311.4 / 311.4, 324.9 / 330.9.)
 int attention_early(int n_head, int n_ctx, bool kq) { return !kq || n_head <= 8 || n_head > 24 || n_ctx % 64 == 0 ? 1 : 0; }
 
 // The form for a single token at position pos, where both kernels take the context. A layer's attention, us, one CTA a head / a cluster of four, 32
@@ -1193,6 +1196,8 @@ int attention_early(int n_head, int n_ctx, bool kq) { return !kq || n_head <= 8 
 // of 8-layer models with little beside the attention, us a layer: 2 heads 248: 17.7 / 18.2, 280: 18.7 / 18.4; 8 heads 248: 20.6 / 21.4, 280: 21.5 / 21.5;
 // 16 heads 216: 24.9 / 24.7, 248: 25.5 / 24.7; 24 heads 248: 29.0 / 29.1, 280: 29.9 / 29.3; 32 heads 248: 32.0 / 32.5, 280: 33.1 / 32.7; 40 heads 248:
 // 41.7 / 42.2, 280: 42.7 / 42.5. They meet between 210 (16 heads) and 280: 240 is off by at most 4 % of such a layer.
+// (With the kernels as they are, steps of 8 layers at 220: Q4_0 8 heads 161.5 / 169.9, 16 209.3 / 207.8, 24 249.8 / 254.5, 32 302.4 / 307.6, 40 403.4 / 407.1;
+// Q4_K_M 204.5 / 201.2, 235.4 / 225.4, 327.4 / 320.5, 361.1 / 361.6, 507.3 / 494.9; at 190 one CTA is ahead or level everywhere.)
 constexpr int ATT_CLUSTER_POS = 240, ATT_ONE_CTA_CTX = 8192;   // (the rows of the longest context: 57 KB)
 int attention_form(const AttnParams &p, const LaunchCfg &cfg, int pos) {
     if (p.T != 1 || p.seq_stride != 0 || p.n_ctx > ATT_ONE_CTA_CTX || !atl_fits(p, cfg)) { return ATT_BY_CONTEXT; }

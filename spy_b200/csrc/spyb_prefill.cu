@@ -46,11 +46,11 @@ constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF
 //
 // Bound: issue slots. A step is 32 packed FMAs (two slots each: a packed FMA measures no faster than 2.5 cycles per scheduler) and 4 packed
 // multiplies per epilogue warp, i.e. 290 slots per scheduler, and everything else around them another 165; the loop is written for few
-// instructions (waits of one test and one branch, D buffers as constants of the unrolled code, one arrival per step), and measures 570
-// cycles per step: 4096 x 4096 x 448 tokens 138 us, 22016 rows 644 us (the e4m3 form: 216 and 1017 us). Tiles of 32 tokens halve the
-// weight bytes per FMA but need 110 registers: spills, 265 us. Eight epilogue warps with 216 registers each: 186-208 us. (The epilogue's
-// registers are all taken: the same source with signed tile numbers, or with the expansion's two offsets computed for S = 2 in both forms,
-// is allocated differently and measures 709 or 668 us on the 22016 rows.)
+// instructions (waits of one test and one branch, D buffers as constants of the unrolled code, one arrival per step), and measures 564
+// cycles per step: 4096 x 4096 x 448 tokens 126 us (138 with whole tiles only), 22016 rows 640 us (the e4m3 form: 216 and 1017 us). Tiles of
+// 32 tokens halve the weight bytes per FMA but need 110 registers: spills, 265 us. Eight epilogue warps with 216 registers each: 186-208 us. (The
+// epilogue's registers are all taken, which is why its loop is written as PTX, pf_fold_steps: the compiler's own order of the same loop measured
+// between 640 and 709 us on the 22016 rows, depending on code beside it.)
 //
 // S = 2: few tokens of a matrix of few rows are fewer tiles than SMs, and a CTA takes no more than some 55 GB/s of weights. A cluster of two
 // CTAs then shares a tile by the halves of its blocks: the eight accumulators of an output are independent chains until the row's end, four
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
 // KQ false (Q4_0 / Q8_0 weights): [token][32 values as f16], the scales. KQ true: the f16 B operand itself (16 bytes of eight values of a token at
 // (value / 8) * 16 TOKT + 16 token), the scales, the blocks' integer sums as floats.
 // SILU: a token's row is [K up | K gate] as the stacked GEMM leaves it, and what is quantized is up * silu(gate) (model/src/llm/plugin/ffn.cpp:28-35),
-// which goes to act only where somebody wants it. (As two kernels, 512 x 11008: 27 + 14 us, 90 MB; this 21 us, 46 MB.)
+// which goes to act only where somebody wants it. (As two kernels, 512 x 11008: 27 + 14 us, 90 MB; this 22-27 us, 46 MB.)
 template <bool NORM, bool KQ, int PG, bool SILU>
 __global__ void __launch_bounds__(PF_QUANT_THREADS, PG <= 2 ? 2 : 1) prefill_quant_kernel(const float *x, int64_t x_stride, int K, const float *norm_w, float eps, uint8_t *yq,
                                                                          int TOKT, int part_len, int64_t part_stride, uint8_t *tap, const float *silu_table, float *act) {
@@ -644,7 +644,7 @@ __global__ void prefill_retile_kernel(const uint8_t *raw, int64_t row_stride, in
 // backend/host/operator/non-linear.cpp:270-371, view.cpp:163-191). The first qk_blocks blocks rotate, a thread per pair of neighbouring elements of a
 // token; the others turn 64 elements x 32 tokens of V over in shared memory, because the cache holds a row per element: a warp then writes
 // 32 neighbouring positions of a row, 64 bytes, where a thread per element wrote two bytes into a line of its own (512 tokens x 12288: 31.5 us,
-// 7 now; 38 MB). A batch in lockstep (seq_stride > 0: token t is sequence t, with its own cache) has nothing to turn over: a thread per element.
+// 16-17 now; 38 MB). A batch in lockstep (seq_stride > 0: token t is sequence t, with its own cache) has nothing to turn over: a thread per element.
 constexpr int PF_POST_THREADS = 256, PF_POST_E = 64, PF_POST_T = 32;
 __global__ void __launch_bounds__(PF_POST_THREADS) prefill_qkv_post_kernel(const float *qkv, int T, int dl, int hd, const int *pos_base, const float2 *rope, __half *q_out, __half *k_cache,
                                         __half *v_cache, int n_ctx, int64_t seq_stride, int qk_blocks) {
