@@ -217,6 +217,9 @@ spyb_status spyb_prefill_form(int64_t n_rows, int64_t k, int64_t n_cols, int32_t
  * its codes (4 = a shared-memory stage, 5 = operands or a free accumulator buffer, 6 = a tensor-core result; also
  * written to *error_code_out); the record is cleared again, so the backend stays usable. No reference counterpart. */
 spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *backend, uint64_t limit_ns, int32_t *error_code_out);
+/* The same for tiles that one CTA begins and another finishes: accumulators are handed over later than `limit_ns` allows. Succeeds when the
+ * kernel returned by itself with code 7 (the accumulators of another CTA) and left nothing behind for the next launch. */
+spyb_status spyb_prefill_selftest_handoff_timeout(spyb_backend *backend, uint64_t limit_ns, int32_t *error_code_out);
 
 /* ---- whole-model path: the graph LLAMAModel::build_graph emits (model/src/llm/model/llama.cpp:86-264)
  * executed as a fixed plan of fused kernels. */

@@ -113,6 +113,7 @@ def lib():
         "spyb_prefill_matmul_form": (i32, [vp, i32, vp, i64, i64, vp, i64, vp, C.c_float, i32, i32, vp]),
         "spyb_prefill_form": (i32, [i64, i64, i64, i32, C.POINTER(i32), C.POINTER(i32)]),
         "spyb_prefill_selftest_wait_timeout": (i32, [vp, u64, C.POINTER(i32)]),
+        "spyb_prefill_selftest_handoff_timeout": (i32, [vp, u64, C.POINTER(i32)]),
         "spyb_model_tp_export": (i32, [vp, vp]),
         "spyb_model_tp_import": (i32, [vp, vp]),
         "spyb_model_read_timeline": (i32, [vp, vp, i32]),
@@ -312,6 +313,12 @@ class B200Backend:
         """Runs the prompt kernel with one batch withheld; returns the code of the wait that gave up (4, 5 or 6)."""
         code = C.c_int32(0)
         self._check(self._l.spyb_prefill_selftest_wait_timeout(self.h, limit_ns, C.byref(code)))
+        return int(code.value)
+
+    def prefill_selftest_handoff_timeout(self, limit_ns: int) -> int:
+        """Runs the prompt kernel with accumulators handed over too late; returns the code of the wait that gave up (7)."""
+        code = C.c_int32(0)
+        self._check(self._l.spyb_prefill_selftest_handoff_timeout(self.h, limit_ns, C.byref(code)))
         return int(code.value)
 
     def attention(self, q16: np.ndarray, k_cache16: np.ndarray, v_cache_t16: np.ndarray, pos0: int, n_head: int, head_dim: int, n_ctx: int,

@@ -500,14 +500,55 @@ spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *be, uint64_t limit_
         g.error_flag = be->d_error_flag; g.wait_limit_ns = limit_ns; g.selftest_skip_step = 1;
         err = launch_prefill_gemm(g, be->stream);
         if (err == cudaSuccess) { err = cudaStreamSynchronize(be->stream); }   // returns: the kernel ended by itself
-        code = *reinterpret_cast<volatile int *>(be->h_error_flag);
-        *reinterpret_cast<volatile int *>(be->h_error_flag) = 0;   // the check leaves the backend usable
+        code = be->clear_device_error();   // the check leaves the backend usable
         if (code < 4 || code > 6) { break; }
     }
     release();
     if (err != cudaSuccess) { be->set_error("prefill selftest: %s", cudaGetErrorString(err)); return SPYB_FAIL; }
     if (error_code_out != nullptr) { *error_code_out = code; }
     if (code < 4 || code > 6) { be->set_error("prefill selftest: expected a wait of the prompt kernel to give up (codes 4-6), got %d", code); return SPYB_FAIL; }
+    return SPYB_SUCCESS;
+}
+
+// Failure-path check of the accumulators that one CTA begins and another finishes, which faults nothing: launches by one CTA a tile and by clusters of two, and
+// of a K-quant matrix, whose last tiles are shared and handed over three limits late. The walkers that wait for them give up (code 7) and clear words that are
+// set afterwards; the words are cleared with the record of the error, or the next shared launch would take accumulators that are not its own.
+spyb_status spyb_prefill_selftest_handoff_timeout(spyb_backend *be, uint64_t limit_ns, int32_t *error_code_out) {
+    if (be == nullptr || limit_ns == 0) { return SPYB_FAIL; }
+    cudaSetDevice(be->config.device_id);
+    SPYB_CUDA(be, cudaStreamSynchronize(be->stream));
+    if (be->device_error()) { return SPYB_FAIL; }
+    if (be->pf_handoff == nullptr) { be->set_error("prefill selftest: no memory for accumulators handed over, all tiles are whole"); return SPYB_UNSUPPORTED; }
+    constexpr int nb = 16;
+    const int T = 16 * (be->num_sms_total + be->num_sms_total / 4);   // tiles of 16 tokens: one round and a quarter by single CTAs, two and a half by clusters
+    const size_t wbytes = std::max(prefill_weight_bytes(SPYB_Q8_0, PF_ROWS, nb), prefill_weight_bytes(SPYB_Q4_K, PF_ROWS, nb)), ybytes = prefill_act_bytes(T, nb);
+    uint8_t *w = nullptr, *yq = nullptr; float *out = nullptr;
+    auto release = [&]() { cudaFree(w); cudaFree(yq); cudaFree(out); };
+    cudaError_t err = cudaMalloc(&w, wbytes);
+    if (err == cudaSuccess) { err = cudaMalloc(&yq, ybytes); }
+    if (err == cudaSuccess) { err = cudaMalloc(&out, (size_t)T * PF_ROWS * 4); }
+    if (err == cudaSuccess) { err = cudaMemsetAsync(w, 0, wbytes, be->stream); }
+    if (err == cudaSuccess) { err = cudaMemsetAsync(yq, 0, ybytes, be->stream); }
+    int code = 0, left = 0;
+    std::vector<unsigned> words(be->handoff_flag_bytes() / sizeof(unsigned));
+    for (const int form : {1, 2, 3}) {   // CTAs a tile; 3: K-quant
+        if (err != cudaSuccess) { break; }
+        PrefillGemm g;
+        g.w = w; g.type = form == 3 ? SPYB_Q4_K : SPYB_Q8_0; g.n_rows = PF_ROWS; g.nb = nb; g.yq = yq; g.tile_tok = PF_TOK; g.split = form == 3 ? 0 : form; g.T = T; g.out = out; g.out_stride = PF_ROWS;
+        be->prefill_shared(g);
+        g.tiles = 2; g.wait_limit_ns = limit_ns; g.selftest_late_ns = 3 * limit_ns;
+        err = launch_prefill_gemm(g, be->stream);
+        if (err == cudaSuccess) { err = cudaStreamSynchronize(be->stream); }   // returns: the kernel ended by itself
+        code = be->clear_device_error();
+        if (err == cudaSuccess) { err = cudaMemcpyAsync(words.data(), be->handoff_flags(), be->handoff_flag_bytes(), cudaMemcpyDeviceToHost, be->stream); }
+        if (err == cudaSuccess) { err = cudaStreamSynchronize(be->stream); }
+        for (const unsigned v : words) { left += v != 0; }
+        if (code != 7 || left != 0) { break; }
+    }
+    release();
+    if (err != cudaSuccess) { be->set_error("prefill selftest: %s", cudaGetErrorString(err)); return SPYB_FAIL; }
+    if (error_code_out != nullptr) { *error_code_out = code; }
+    if (code != 7 || left != 0) { be->set_error("prefill selftest: expected the wait for another CTA's accumulators to give up (code 7) and no word set after it, got %d and %d", code, left); return SPYB_FAIL; }
     return SPYB_SUCCESS;
 }
 

@@ -111,16 +111,27 @@ struct spyb_backend {
         if (h_error_flag != nullptr && *reinterpret_cast<volatile int *>(h_error_flag) != 0) {
             const int code = *reinterpret_cast<volatile int *>(h_error_flag);
             if (code == 1) { set_error("a kernel gave up waiting for a bulk copy into shared memory (device error flag 1); the backend must be re-created"); }
-            else if (code >= 4 && code <= 6) { set_error("the prompt GEMM gave up waiting for %s (device error flag %d); the backend must be re-created", code == 4 ? "a shared-memory stage" : code == 5 ? "its operands or a free accumulator buffer" : "a tensor-core result", code); }
+            else if (code >= 4 && code <= 7) {
+                const char *what[] = {"a shared-memory stage", "its operands or a free accumulator buffer", "a tensor-core result", "the accumulators of another CTA"};
+                set_error("the prompt GEMM gave up waiting for %s (device error flag %d); the backend must be re-created", what[code - 4], code);
+            }
             else { set_error("a kernel gave up waiting at a barrier or for another rank's partial result (device error flag %d); the backend must be re-created", code); }
             return true;
         }
         return false;
     }
+    size_t handoff_flag_bytes() const { return (size_t)num_sms_total * spyb::PF_HANDOFF_FLAGS * sizeof(unsigned); }
+    unsigned *handoff_flags() const { return pf_handoff == nullptr ? nullptr : reinterpret_cast<unsigned *>(static_cast<uint8_t *>(pf_handoff) + (size_t)num_sms_total * spyb::PF_HANDOFF_BYTES); }
+    // After a failure-path check, on an idle stream: no error recorded, and nothing handed over that nobody fetched. Returns the code that was recorded.
+    int clear_device_error() {
+        const int code = *reinterpret_cast<volatile int *>(h_error_flag);
+        *reinterpret_cast<volatile int *>(h_error_flag) = 0;
+        if (pf_handoff != nullptr && cudaMemsetAsync(handoff_flags(), 0, handoff_flag_bytes(), stream) != cudaSuccess) { cudaGetLastError(); }
+        return code;
+    }
     void prefill_shared(spyb::PrefillGemm &g) const {   // what every prompt GEMM on this backend's stream has in common
         g.error_flag = d_error_flag; g.wait_limit_ns = wait_limit_ns;
-        g.handoff = pf_handoff;
-        if (pf_handoff != nullptr) { g.handoff_flags = reinterpret_cast<unsigned *>(static_cast<uint8_t *>(pf_handoff) + (size_t)num_sms_total * spyb::PF_HANDOFF_BYTES); }
+        g.handoff = pf_handoff; g.handoff_flags = handoff_flags();
     }
     spyb::LaunchCfg launch_cfg(bool pdl) const {
         spyb::LaunchCfg c; c.stream = stream; c.pdl = pdl; c.num_sms = num_sms; c.mv_ctas_per_sm = mv_ctas_per_sm;

@@ -1382,9 +1382,8 @@ spyb_status spyb_model_selftest_wait_timeout(spyb_model *m, uint64_t limit_ns, i
     SPYB_CUDA(be, cudaMemsetAsync(m->d_step_sync, 0, 32, be->stream));
     SPYB_CUDA(be, launch_step(p, m->step_grid, m->step_ns, m->step_coop, be->stream));
     SPYB_CUDA(be, cudaStreamSynchronize(be->stream));   // returns: the kernel ended by itself
-    const int code = *reinterpret_cast<volatile int *>(be->h_error_flag);
+    const int code = be->clear_device_error();          // the check leaves the backend usable
     if (error_code_out != nullptr) { *error_code_out = code; }
-    *reinterpret_cast<volatile int *>(be->h_error_flag) = 0;   // the check leaves the backend usable
     if (code != 2) { be->set_error("selftest: expected the barrier wait to give up with code 2, got %d", code); return SPYB_FAIL; }
     return SPYB_SUCCESS;
 }

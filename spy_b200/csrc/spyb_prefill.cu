@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             const int tile = it.tile;
             if constexpr (SHARE) if (it.from > 0) {   // another walker's accumulators
                 const int64_t at = (int64_t)((int)blockIdx.x - S) * PF_GEMM_EPI_WARPS + warp;
-                handoff_wait(g.handoff_flags + at, left_ns);
+                handoff_wait(g.handoff_flags + at, left_ns, g.error_flag);
 #pragma unroll
                 for (int n = 0; n < 4 * HS * PW; ++n) { acc[n / (4 * HS)][n % (4 * HS)] = __ldcg(reinterpret_cast<const unsigned long long *>(g.handoff) + (at * 16 + n) * 32 + lane); }
                 __syncwarp();
@@ -415,7 +415,8 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                     a = 0ull;
                 }
                 __syncwarp();
-                if (lane == 0) { handoff_publish(g.handoff_flags + at); }
+                if (lane == 0) { handoff_publish(g.handoff_flags + at, g.selftest_late_ns); }
+                __syncwarp();
                 continue;
             }
             // hsum_float_8 (vec_util.h:74-81): accumulator n of a half is CPU accumulator 4 + n / n (Q4_0: low / high nibbles) or n / 4 + n
@@ -745,7 +746,7 @@ int device_sms() {
 // quantizer, one CTA / two: 4096 x 4096 x 8 tokens 18.1 / 15.2, 4096 x 11008 x 16 54.7 / 34.9; and 1680 x 2208 x 79 tokens 13.3 / 16.2, 22016 x 4096 x 448
 // 655 / 826; whole / shared tiles: 14968 x 1088 x 22 19.5 / 21.8, and the sizes above.
 struct PfForm { int tok, split; double launch_ns, tile_ns, block_ns, rows_ns, handoff_ns, slower; };
-static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int split, int sms, bool *share) {   // tok, split 0: any
+static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int split, int how, int sms, bool *share) {   // tok, split, how (PrefillGemm::tiles) 0: any
     static constexpr PfForm FORMS[4] = {{16, 1, 4240, 730, 149.9, 28.3, 5720, -0.025}, {8, 1, 3210, 0, 119.2, 87.6, 2510, 0.019},
                                         {16, 2, 5790, 1740, 84.5, 22.0, 5320, 0.065}, {8, 2, 5250, 1070, 65.1, 68.1, 3790, 0.020}};
     PfForm best = {};
@@ -756,9 +757,9 @@ static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int split, int s
         const double once = f.launch_ns + (double)row_tiles / sms * nb * f.rows_ns;
         double ns = once + (double)((tiles + walkers - 1) / walkers) * (f.tile_ns + nb * f.block_ns);
         bool shared = false;
-        if (tiles > walkers && tiles % walkers != 0) {
+        if (how != 1 && tiles > walkers && (how == 2 || tiles % walkers != 0)) {
             const double ns_shared = 1000.0 + 1.02 * (once + f.handoff_ns + (double)tiles / walkers * (f.tile_ns + nb * f.block_ns * (1.0 + f.slower)));
-            if (ns_shared < ns) { ns = ns_shared; shared = true; }
+            if (how == 2 || ns_shared < ns) { ns = ns_shared; shared = true; }
         }
         if (best.tok == 0 || ns < best_ns) { best = f; best_ns = ns; *share = shared; }
     }
@@ -766,7 +767,7 @@ static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int split, int s
 }
 void prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split) {
     bool share;
-    const PfForm f = best_form(n_rows, nb, T, 0, 0, sms, &share);
+    const PfForm f = best_form(n_rows, nb, T, 0, 0, 0, sms, &share);
     *tile_tok = f.tok; *split = f.split;
 }
 // host-only check of the shared tiles: every step of every tile is some walker's exactly once, and a tile's first steps are the lower neighbour's of the
@@ -797,8 +798,8 @@ int prefill_share_selftest() {
 }
 int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T) {
     bool share;
-    if (type == 12 || type == 14) { return prefill_kq_tile_tokens(n_rows, nb, T, 0, device_sms(), &share); }
-    return best_form(n_rows, nb, T, 0, 0, device_sms(), &share).tok;
+    if (type == 12 || type == 14) { return prefill_kq_tile_tokens(n_rows, nb, T, 0, 0, device_sms(), &share); }
+    return best_form(n_rows, nb, T, 0, 0, 0, device_sms(), &share).tok;
 }
 
 size_t prefill_weight_bytes(int type, int64_t n_rows, int nb) {
@@ -852,7 +853,7 @@ cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool 
     if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
     if ((g.tile_tok != 16 && g.tile_tok != 8) || g.split < 0 || g.split > 2) { return cudaErrorInvalidValue; }
     bool share = false;
-    const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok, g.split, device_sms(), &share).split == 2;
+    const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok, g.split, g.tiles, device_sms(), &share).split == 2;
     share = share && g.handoff != nullptr;
     // Many tokens (MANY): the epilogue is the bound and the weights come out of L2; copies of half a block are in its way for less long.
     // 22016 x 4096 x 448 tokens 659 us with one copy a step, 649 by blocks, 642 by halves, 646 by quarters. Where the weights' way

@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(KQ_GEMM_THREADS, 1) prefill_kq_gemm_kernel(Pre
             const int tile = it.tile;
             if constexpr (SHARE) if (it.from > 0) {   // the sums of the super-blocks in front are another CTA's
                 const int64_t at = (int64_t)((int)blockIdx.x - 1) * KQ_EPI_WARPS + warp;
-                handoff_wait(g.handoff_flags + at, left_ns);
+                handoff_wait(g.handoff_flags + at, left_ns, g.error_flag);
 #pragma unroll
                 for (int u = 0; u < PW; ++u) { tot[u] = __ldcg(reinterpret_cast<const unsigned long long *>(g.handoff) + (at * 16 + u) * 32 + lane); }
                 __syncwarp();
@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(KQ_GEMM_THREADS, 1) prefill_kq_gemm_kernel(Pre
 #pragma unroll
                 for (int u = 0; u < PW; ++u) { __stcg(reinterpret_cast<unsigned long long *>(g.handoff) + (at * 16 + u) * 32 + lane, (unsigned long long)tot[u]); tot[u] = 0ull; }
                 __syncwarp();
-                if (lane == 0) { handoff_publish(g.handoff_flags + at); }
+                if (lane == 0) { handoff_publish(g.handoff_flags + at, g.selftest_late_ns); }
+                __syncwarp();
                 continue;
             }
             const int64_t orow = (int64_t)(tile / n_tok) * PF_M + row;
@@ -350,7 +351,7 @@ cudaError_t launch_kq_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
 // that the matrices of a layer that read the same activations agree on a width. Fitted to 411 sizes of both (1024 x 1024 to 32000 x 14336, 8 to 512 tokens): 4.9 %
 // faster on average than the widths by whole rounds alone, 0.1 % behind the fastest choice, more than 3 % at 6 of them (Q4_K 8696 x 1536 x 82 9 %). us, whole
 // tiles / shared: Q4_K 11008 x 4096 x 64 41.7 / 31.9, 5120 x 5120 x 512 127.8 / 107.8, 4096 x 4096 x 512 78.7 / 72.2; Q6_K 4096 x 11008 x 512 193.9 / 174.4.
-int prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int sms, bool *share) {
+int prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int how, int sms, bool *share) {
     static constexpr struct { int tok; double launch_ns, tile_ns, block_ns, rows_ns, handoff_ns, slower; } WIDTHS[3] = {
         {16, 4230, 100, 102.6, 49.7, 3770, 0.0}, {32, 4810, 280, 139.9, 33.1, 3780, -0.009}, {64, 4540, 880, 274.4, 4.3, 5230, -0.018}};
     int best = 0;
@@ -361,9 +362,9 @@ int prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int sms, bool
         const double once = w.launch_ns + (double)row_tiles / sms * nb * w.rows_ns;
         double ns = once + (double)((tiles + sms - 1) / sms) * (w.tile_ns + nb * w.block_ns);
         bool shared = false;
-        if (tiles > sms && tiles % sms != 0 && nb >= 16) {
+        if (how != 1 && tiles > sms && (how == 2 || tiles % sms != 0) && nb >= 16) {
             const double ns_shared = 500.0 + 1.01 * (once + w.handoff_ns + (double)tiles / sms * (w.tile_ns + nb * w.block_ns * (1.0 + w.slower)));
-            if (ns_shared < ns) { ns = ns_shared; shared = true; }
+            if (how == 2 || ns_shared < ns) { ns = ns_shared; shared = true; }
         }
         if (best == 0 || ns < best_ns) { best = w.tok; best_ns = ns; *share = shared; }
     }
@@ -373,7 +374,7 @@ int prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int sms, bool
 cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     if (g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 8 || (g.nb & 7) || g.n_rows < 1 || (g.type != 12 && g.type != 14)) { return cudaErrorInvalidValue; }
     bool share = false;
-    prefill_kq_tile_tokens(g.n_rows, g.nb, g.T, g.tile_tok, device_sms(), &share);
+    prefill_kq_tile_tokens(g.n_rows, g.nb, g.T, g.tile_tok, g.tiles, device_sms(), &share);
     auto of_width = [&](auto tt) {
         constexpr int TT = decltype(tt)::value;
         if (share && g.handoff != nullptr) { return g.type == 12 ? launch_kq_t<12, TT, true>(g, stream, pdl) : launch_kq_t<14, TT, true>(g, stream, pdl); }

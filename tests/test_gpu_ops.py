@@ -300,6 +300,22 @@ def test_prefill_kernel_wait_runs_out_and_is_reported():
     b.close()
 
 
+def test_prefill_kernel_handover_too_late_is_reported_and_leaves_nothing(oracle):
+    """Accumulators that come after their walker gave up: the kernels return by themselves, the status names that wait, and the words that were set
+    too late are cleared, so that shared launches afterwards give the oracle's bits."""
+    b = B.B200Backend(0)
+    assert b.prefill_selftest_handoff_timeout(2_000_000) == 7
+    n, k, t = 9604, 4128, 32
+    rng = np.random.default_rng(3)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), quants.Q8_0)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    rows = np.arange(0, n, 97)
+    want = oracle.matmul(quants.Q8_0, np.ascontiguousarray(w[rows]), k, len(rows), x)
+    for form in [(16, 1), (16, 2)]:
+        assert np.array_equal(b.prefill_matmul(quants.Q8_0, w, n, k, x, form=form)[:, rows].view(np.uint32), want.view(np.uint32)), form
+    b.close()
+
+
 def test_prefill_matmul_rejects_what_does_not_fit(be):
     w = np.zeros(100 * 18, dtype=np.uint8)
     x = np.zeros((2, 48), dtype=np.float32)
