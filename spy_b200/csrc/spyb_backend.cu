@@ -218,7 +218,7 @@ spyb_status spyb_create(const spyb_config *config, spyb_backend **out) {
     if (!ok) { spyb_destroy(be); return SPYB_FAIL; }
     const size_t handoff = (size_t)be->num_sms_total * (PF_HANDOFF_BYTES + PF_HANDOFF_FLAGS * sizeof(unsigned));
     if (cudaMalloc(&be->pf_handoff, handoff) != cudaSuccess) { cudaGetLastError(); be->pf_handoff = nullptr; }   // (the GEMMs go without)
-    else if (cudaMemset(be->pf_handoff, 0, handoff) != cudaSuccess) { spyb_destroy(be); return SPYB_FAIL; }
+    else if (cudaMemsetAsync(be->pf_handoff, 0, handoff, be->stream) != cudaSuccess) { spyb_destroy(be); return SPYB_FAIL; }   // (in front of all that reads it)
     be->cb_thread = std::thread(callback_worker, be);
     *out = be;
     return SPYB_SUCCESS;
