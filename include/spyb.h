@@ -209,8 +209,17 @@ spyb_status spyb_prefill_matmul_form(spyb_backend *backend, int32_t weight_type,
                                      const float *x_host, int64_t n_cols, const float *norm_w_host, float eps, int32_t tile_tokens, int32_t tile_ctas,
                                      float *out_host);
 
+/* ... and with its last tiles whole (1) or shared between neighbouring CTAs or clusters (2, where there are more tiles than those; 0: by the sizes). */
+spyb_status spyb_prefill_matmul_tiles(spyb_backend *backend, int32_t weight_type, const void *w_rows_host, int64_t n_rows, int64_t k,
+                                      const float *x_host, int64_t n_cols, const float *norm_w_host, float eps, int32_t tile_tokens, int32_t tile_ctas,
+                                      int32_t last_tiles, float *out_host);
+
 /* The form that a Q4_0 / Q8_0 MatMul of these sizes takes on a device of n_sms SMs (host arithmetic only, no GPU needed). */
 spyb_status spyb_prefill_form(int64_t n_rows, int64_t k, int64_t n_cols, int32_t n_sms, int32_t *tile_tokens, int32_t *tile_ctas);
+/* The same for all weight types and with what becomes of the last tiles: what is zero of *tile_tokens, *tile_ctas and *last_tiles is filled in, what is not
+ * is asked for. *last_tiles comes back as 1 (whole, also where 2 was asked for and there is nothing to share) or 2. */
+spyb_status spyb_prefill_plan(int32_t weight_type, int64_t n_rows, int64_t k, int64_t n_cols, int32_t n_sms, int32_t *tile_tokens, int32_t *tile_ctas,
+                              int32_t *last_tiles);
 
 /* Failure-path check of the prompt kernel that faults nothing: a small launch whose second batch of blocks is never
  * copied, by one CTA and then by a cluster of two, with `limit_ns` as the bound of every wait. Succeeds when the kernel returned by itself and recorded one of

@@ -112,6 +112,8 @@ def lib():
         "spyb_prefill_matmul": (i32, [vp, i32, vp, i64, i64, vp, i64, vp, C.c_float, vp]),
         "spyb_prefill_matmul_form": (i32, [vp, i32, vp, i64, i64, vp, i64, vp, C.c_float, i32, i32, vp]),
         "spyb_prefill_form": (i32, [i64, i64, i64, i32, C.POINTER(i32), C.POINTER(i32)]),
+        "spyb_prefill_matmul_tiles": (i32, [vp, i32, vp, i64, i64, vp, i64, vp, C.c_float, i32, i32, i32, vp]),
+        "spyb_prefill_plan": (i32, [i32, i64, i64, i64, i32, C.POINTER(i32), C.POINTER(i32), C.POINTER(i32)]),
         "spyb_prefill_selftest_wait_timeout": (i32, [vp, u64, C.POINTER(i32)]),
         "spyb_prefill_selftest_handoff_timeout": (i32, [vp, u64, C.POINTER(i32)]),
         "spyb_model_tp_export": (i32, [vp, vp]),
@@ -161,6 +163,15 @@ def make_tensor(data_ptr, number_type: int, ne, nb=None, node_type: int = NODE_D
         t.elements[i], t.bytes[i] = ne[i], nb[i]
     t.data = data_ptr
     return t
+
+
+def prefill_plan(weight_type: int, n_rows: int, k: int, n_cols: int, form=(0, 0, 0), n_sms: int = 148) -> tuple:
+    """The form of the prompt GEMM for these sizes (no GPU needed): tokens a tile, CTAs a tile, last tiles whole (1) or shared (2). What is zero of
+    `form` is by the sizes."""
+    v = [C.c_int32(f) for f in form]
+    if lib().spyb_prefill_plan(weight_type, n_rows, k, n_cols, n_sms, *(C.byref(x) for x in v)) != SUCCESS:
+        raise SpybError(FAIL, f"no prompt GEMM of type {weight_type} with {n_rows} x {k}, {n_cols} columns, form {form}")
+    return tuple(int(x.value) for x in v)
 
 
 class B200Backend:
@@ -299,14 +310,15 @@ class B200Backend:
     def prefill_matmul(self, weight_type: int, w_rows: np.ndarray, n_rows: int, k: int, x: np.ndarray, norm_w=None, eps: float = 0.0,
                        form=(0, 0)) -> np.ndarray:
         """MatMul of raw-layout quantized rows (host bytes) with the columns x [T, k] on the tensor-core prompt kernel; returns f32 [T, n_rows].
-        form: tokens a tile and CTAs a tile (0: by the sizes)."""
+        form: tokens a tile, CTAs a tile and the last tiles whole (1) or shared (2); 0 or left out: by the sizes."""
         x = np.ascontiguousarray(x, dtype=np.float32)
         w_rows = np.ascontiguousarray(w_rows)
         t = x.shape[0]
         out = np.empty((t, n_rows), dtype=np.float32)
         nw = None if norm_w is None else np.ascontiguousarray(norm_w, dtype=np.float32)
-        self._check(self._l.spyb_prefill_matmul_form(self.h, weight_type, _np_ptr(w_rows), n_rows, k, _np_ptr(x), t, None if nw is None else _np_ptr(nw),
-                                                     C.c_float(eps), form[0], form[1], _np_ptr(out)))
+        tok, ctas, tiles = (*form, 0)[:3]
+        self._check(self._l.spyb_prefill_matmul_tiles(self.h, weight_type, _np_ptr(w_rows), n_rows, k, _np_ptr(x), t, None if nw is None else _np_ptr(nw),
+                                                      C.c_float(eps), tok, ctas, tiles, _np_ptr(out)))
         return out
 
     def prefill_selftest_wait_timeout(self, limit_ns: int) -> int:

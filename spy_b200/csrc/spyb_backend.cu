@@ -425,6 +425,10 @@ spyb_status spyb_prefill_matmul(spyb_backend *be, int32_t weight_type, const voi
 }
 spyb_status spyb_prefill_matmul_form(spyb_backend *be, int32_t weight_type, const void *w_rows_host, int64_t n_rows, int64_t k, const float *x_host,
                                      int64_t n_cols, const float *norm_w_host, float eps, int32_t tile_tokens, int32_t tile_ctas, float *out_host) {
+    return spyb_prefill_matmul_tiles(be, weight_type, w_rows_host, n_rows, k, x_host, n_cols, norm_w_host, eps, tile_tokens, tile_ctas, 0, out_host);
+}
+spyb_status spyb_prefill_matmul_tiles(spyb_backend *be, int32_t weight_type, const void *w_rows_host, int64_t n_rows, int64_t k, const float *x_host,
+                                      int64_t n_cols, const float *norm_w_host, float eps, int32_t tile_tokens, int32_t tile_ctas, int32_t last_tiles, float *out_host) {
     if (be == nullptr) { return SPYB_FAIL; }
     const bool kq = weight_type == SPYB_Q4_K || weight_type == SPYB_Q6_K;
     if (weight_type != SPYB_Q4_0 && weight_type != SPYB_Q8_0 && !kq) { be->set_error("prefill_matmul: weight type %d", weight_type); return SPYB_UNSUPPORTED; }
@@ -435,6 +439,7 @@ spyb_status spyb_prefill_matmul_form(spyb_backend *be, int32_t weight_type, cons
     }
     const bool width_ok = kq ? tile_tokens == 16 || tile_tokens == 32 || tile_tokens == 64 : tile_tokens == 8 || tile_tokens == 16;
     if ((tile_tokens != 0 && !width_ok) || tile_ctas < 0 || tile_ctas > (kq ? 1 : 2)) { be->set_error("prefill_matmul: no form with tiles of %d tokens by %d CTAs", tile_tokens, tile_ctas); return SPYB_UNSUPPORTED; }
+    if (last_tiles < 0 || last_tiles > 2) { be->set_error("prefill_matmul: last tiles %d", last_tiles); return SPYB_UNSUPPORTED; }
     cudaSetDevice(be->config.device_id);
     const int nb = (int)(k / QK), T = (int)n_cols, tile_tok = tile_tokens != 0 ? tile_tokens : prefill_tile_tokens(weight_type, n_rows, nb, T);
     const int64_t rb = kq ? (k / 256) * (weight_type == SPYB_Q4_K ? 144 : 210) : (int64_t)nb * (weight_type == SPYB_Q4_0 ? 18 : 34);
@@ -456,7 +461,7 @@ spyb_status spyb_prefill_matmul_form(spyb_backend *be, int32_t weight_type, cons
     if (err == cudaSuccess) { err = launch_prefill_quant(x, k, T, (int)k, nw, eps, yq, be->stream, weight_type, tile_tok); }
     if (err == cudaSuccess) {
         PrefillGemm g;
-        g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.tile_tok = tile_tok; g.split = tile_ctas; g.T = T; g.out = out; g.out_stride = n_rows;
+        g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.tile_tok = tile_tok; g.split = tile_ctas; g.tiles = last_tiles; g.T = T; g.out = out; g.out_stride = n_rows;
         be->prefill_shared(g);
         err = launch_prefill_gemm(g, be->stream);
     }
@@ -471,6 +476,15 @@ spyb_status spyb_prefill_matmul_form(spyb_backend *be, int32_t weight_type, cons
 spyb_status spyb_prefill_form(int64_t n_rows, int64_t k, int64_t n_cols, int32_t n_sms, int32_t *tile_tokens, int32_t *tile_ctas) {
     if (n_rows < 1 || k < QK || k % QK != 0 || k > PF_MAX_K || n_cols < 1 || n_cols > 4096 || n_sms < 2 || tile_tokens == nullptr || tile_ctas == nullptr) { return SPYB_FAIL; }
     prefill_form(n_rows, (int)(k / QK), (int)n_cols, n_sms, tile_tokens, tile_ctas);
+    return SPYB_SUCCESS;
+}
+spyb_status spyb_prefill_plan(int32_t weight_type, int64_t n_rows, int64_t k, int64_t n_cols, int32_t n_sms, int32_t *tile_tokens, int32_t *tile_ctas, int32_t *last_tiles) {
+    const bool kq = weight_type == SPYB_Q4_K || weight_type == SPYB_Q6_K;
+    if ((!kq && weight_type != SPYB_Q4_0 && weight_type != SPYB_Q8_0) || tile_tokens == nullptr || tile_ctas == nullptr || last_tiles == nullptr) { return SPYB_FAIL; }
+    if (n_rows < 1 || k < QK || k % (kq ? 256 : QK) != 0 || k > PF_MAX_K || n_cols < 1 || n_cols > 4096 || n_sms < 2) { return SPYB_FAIL; }
+    const bool width_ok = kq ? *tile_tokens == 16 || *tile_tokens == 32 || *tile_tokens == 64 : *tile_tokens == 8 || *tile_tokens == 16;
+    if ((*tile_tokens != 0 && !width_ok) || *tile_ctas < 0 || *tile_ctas > (kq ? 1 : 2) || *last_tiles < 0 || *last_tiles > 2) { return SPYB_FAIL; }
+    prefill_plan(weight_type, n_rows, (int)(k / QK), (int)n_cols, n_sms, tile_tokens, tile_ctas, last_tiles);
     return SPYB_SUCCESS;
 }
 

@@ -142,6 +142,7 @@ struct PrefillGemm {
 int         device_sms();         // SMs of the current device
 int         prefill_tile_tokens(int type, int64_t n_rows, int nb, int T);   // width of the token tiles for this matrix and number of tokens
 void        prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split);   // host-only: the Q4_0 / Q8_0 kernel's form on a device of so many SMs
+void        prefill_plan(int type, int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split, int *tiles);   // host-only: all of a kernel's form, what is zero of it by the sizes (PrefillGemm::tiles: 1 or 2)
 int         prefill_share_selftest();   // host-only: the cuts of shared tiles; 0 when they hold
 size_t      prefill_weight_bytes(int type, int64_t n_rows, int nb);
 size_t      prefill_act_bytes(int T, int nb);

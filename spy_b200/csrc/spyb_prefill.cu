@@ -770,13 +770,18 @@ void prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *sp
     const PfForm f = best_form(n_rows, nb, T, 0, 0, 0, sms, &share);
     *tile_tok = f.tok; *split = f.split;
 }
+void prefill_plan(int type, int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split, int *tiles) {
+    bool share = false;
+    if (type == 12 || type == 14) { *tile_tok = prefill_kq_tile_tokens(n_rows, nb, T, *tile_tok, *tiles, sms, &share); *split = 1; }
+    else { const PfForm f = best_form(n_rows, nb, T, *tile_tok, *split, *tiles, sms, &share); *tile_tok = f.tok; *split = f.split; }
+    *tiles = share ? 2 : 1;
+}
 // host-only check of the shared tiles: every step of every tile is some walker's exactly once, and a tile's first steps are the lower neighbour's of the
 // walker that goes on with it, and done by the time it does
 int prefill_share_selftest() {
     for (int walkers : {2, 3, 74, 148}) {
         for (int n_step : {1, 2, 3, 7, 64, 65, 172, 448}) {
             for (int n_tile = walkers + 1; n_tile < 4 * walkers; n_tile += 1 + walkers / 20) {
-                if (n_tile % walkers == 0) { continue; }
                 const PfShare h = pf_share(n_tile, n_step, walkers);
                 std::vector<int> begun(n_tile, 0), begun_by(n_tile, -1), begun_at(n_tile, 0), done(n_tile, 0);
                 for (int w = 0; w < walkers; ++w) {
