@@ -171,8 +171,13 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
+    // How the expanding and multiplying warps walk: items and their steps, or (COUNTED) one count over all of them; and who releases the stage before a step's: the
+    // thread that issues its MMAs, or (EARLY_FREE) lane 0 beforehand. Whole tiles, 8 to 30 sizes each, per cent of the time with one count throughout and lane 0 for
+    // two CTAs only, as it was: 16 tokens by one CTA as here -2.1 to -3.3 (lane 0: -0.5 to -1.5), 8 tokens by one CTA -1.3 to -1.9 (the issuing thread: -0.6), 8 by two
+    // -0.3 to -0.5; 16 by two by items +0.7.
+    constexpr bool COUNTED = TT == 16 && S == 2, EARLY_FREE = TT == 8 || S == 2;
     const int walker = (int)blockIdx.x / S;
-    const int total_steps = SHARE ? g.share.rounds * n_step + g.share.len + ((int)gridDim.x / S - 1 - walker < g.share.rem ? 1 : 0) : (g.share.rounds + (walker < g.share.rem ? 1 : 0)) * n_step;
+    [[maybe_unused]] const int total_steps = SHARE ? g.share.rounds * n_step + g.share.len + ((int)gridDim.x / S - 1 - walker < g.share.rem ? 1 : 0) : (g.share.rounds + (walker < g.share.rem ? 1 : 0)) * n_step;
     auto first_item = [&]() -> PfItem {
         if constexpr (SHARE) { return pf_share_item(g.share, n_tile, n_step, (int)blockIdx.x / S, (int)gridDim.x / S, 0); }
         return {(int)blockIdx.x / S, 0, n_step, 0};
@@ -180,6 +185,16 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
     auto next_item = [&](PfItem &it) {
         if constexpr (SHARE) { it = pf_share_item(g.share, n_tile, n_step, (int)blockIdx.x / S, (int)gridDim.x / S, it.q + 1); }
         else { it.tile += gridDim.x / S; }
+    };
+    // calls step(i, count) for the walker's steps, i the step of its tile (COUNTED: of none), until one returns false
+    auto each_step = [&](auto step) {
+        if constexpr (COUNTED) { for (int k = 0; k < total_steps; ++k) { if (!step(0, k)) { return; } } }
+        else {
+            int k = 0;
+            for (PfItem it = first_item(); it.tile < n_tile; next_item(it)) {
+                for (int i = it.from; i < it.to; ++i, ++k) { if (!step(i, k)) { return; } }
+            }
+        }
     };
 
     // CTAs that run together take neighbouring token tiles of the same rows: a weight tile crosses HBM once
@@ -258,9 +273,9 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             const int h = S == 2 ? 0 : (lane >> 1) & 1, np = lane & 1, t0 = S == 2 ? lane >> 1 : lane >> 2;
             const uint32_t dst_lane = (uint32_t)((S == 2 ? (t0 / TT) * 128 * TT : 0) + h * 128 * TT + np * (64 * TT + 64) + ((S == 2 ? t0 % TT : t0) >> 1) * 128 + (t0 & 1) * 16);
             const uint32_t src_lane = (uint32_t)(S == 2 ? (t0 / TT) * YB + (t0 % TT) * 64 + rank * 32 + np * 16 : lane * 16);
-            for (int k = 0; k < total_steps; ++k) {
+            each_step([&](int, int) {
                 mbar_wait_lean(raw_full(st), par, left_ns);
-                if (left_ns == 0) { break; }
+                if (left_ns == 0) { return false; }
                 const uint32_t base = sbase + (uint32_t)st * G::STAGE, src = base + NB * WB + src_lane, dst = base + G::RAW + dst_lane;
                 uint4 v[4];
 #pragma unroll
@@ -275,30 +290,31 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                 __syncwarp();
                 if (lane == 0) { mbar_arrive(ops_full(st)); }
                 if (++st == NS) { st = 0; par ^= 1u; }
-            }
+                return true;
+            });
             if (left_ns == 0 && lane == 0) { pf_report(g.error_flag, 4); }
         } else {
             // ---- MMAs: per block and half of 16 elements one 128 x 4 TT x 16 product; warp m takes the steps of D buffer m (issuing a step's
             // MMAs and their commit takes one warp up to 400 cycles)
             const int m = warp - (PF_GEMM_EPI_WARPS + 2);
             const uint32_t d0 = tmem + (uint32_t)m * 256u;
-            int st = 0, k = 0, mine = 0;
+            int st = 0, mine = 0;
             uint32_t par = 0;
-            for (; k < total_steps; ++k) {
+            each_step([&](int i, int k) {
                 if ((k & 1) == m) {
                     mbar_wait_lean(ops_full(st), par, left_ns);
                     mbar_wait_lean(d_free(m), (uint32_t)mine & 1u, left_ns);
-                    if (left_ns == 0) { break; }
-                    // (the step before on this buffer has been read. One CTA a tile: by the thread that issues, which is the quicker way to the MMAs and makes
-                    // 448 tokens 5 % faster; with two CTAs, which wait for their weights, 2 % are the other way)
-                    if (S == 2 && mine > 0 && lane == 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }
+                    if (left_ns == 0) { return false; }
+                    if (EARLY_FREE && mine > 0 && lane == 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }   // (the step before on this buffer has been read)
                     tc_fence_after();
                     const uint32_t base = sbase + (uint32_t)st * G::STAGE;
                     const uint64_t a0 = operand_desc(base + (uint32_t)rank * 512u, 2048u, 128u), b0 = operand_desc(base + G::RAW, 64u * TT, 128u);
+                    [[maybe_unused]] const int n = min(NB, nb - i * NB);
                     if (elect_one()) {
-                        if (S == 1 && mine > 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }
+                        if (!EARLY_FREE && mine > 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }   // (the step before on this buffer has been read)
 #pragma unroll
-                        for (int j = 0; j < NB; ++j) {   // (blocks past the end of a row are multiplied too, whatever lies there: nobody folds them)
+                        for (int j = 0; j < NB; ++j) {
+                            if (!COUNTED && j >= n) { continue; }   // (COUNTED: blocks past the end of a row are multiplied too, whatever lies there: nobody folds them)
 #pragma unroll
                             for (int h = 0; h < HS; ++h) {
                                 mma_f16_ss(d0 + (uint32_t)((j * HS + h) * 4 * TT), a0 + (uint64_t)((j * WB + h * (PF_HALF + 512)) >> 4), b0 + (uint64_t)(((j * HS + h) * 128 * TT) >> 4),
@@ -311,7 +327,8 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                     ++mine;
                 }
                 if (++st == NS) { st = 0; par ^= 1u; }
-            }
+                return true;
+            });
             if (left_ns == 0 && lane == 0) { pf_report(g.error_flag, 5); }
             // every MMA has completed (it reads shared memory and writes tensor memory) before the CTA leaves
             if (mine > 0 && !mbar_wait_relaxed(d_full(m), (uint32_t)(mine - 1) & 1u, limit)) { if (lane == 0) { pf_report(g.error_flag, 5); } }
