@@ -223,11 +223,11 @@ spyb_status spyb_prefill_plan(int32_t weight_type, int64_t n_rows, int64_t k, in
 
 /* Failure-path check of the prompt kernel that faults nothing: a small launch whose second batch of blocks is never
  * copied, by one CTA and then by a cluster of two, with `limit_ns` as the bound of every wait. Succeeds when the kernel returned by itself and recorded one of
- * its codes (4 = a shared-memory stage, 5 = operands or a free accumulator buffer, 6 = a tensor-core result; also
+ * its codes (4 = a shared-memory stage, 5 = operands or a free accumulator buffer, 6 = a tensor-core result or another CTA's accumulators; also
  * written to *error_code_out); the record is cleared again, so the backend stays usable. No reference counterpart. */
 spyb_status spyb_prefill_selftest_wait_timeout(spyb_backend *backend, uint64_t limit_ns, int32_t *error_code_out);
 /* The same for tiles that one CTA begins and another finishes: accumulators are handed over later than `limit_ns` allows. Succeeds when the
- * kernel returned by itself with code 7 (the accumulators of another CTA) and left nothing behind for the next launch. */
+ * kernels returned by themselves with such a code, accumulators came after their CTA had given up, and nothing of them is left for the next launch. */
 spyb_status spyb_prefill_selftest_handoff_timeout(spyb_backend *backend, uint64_t limit_ns, int32_t *error_code_out);
 
 /* ---- whole-model path: the graph LLAMAModel::build_graph emits (model/src/llm/model/llama.cpp:86-264)

@@ -328,7 +328,7 @@ class B200Backend:
         return int(code.value)
 
     def prefill_selftest_handoff_timeout(self, limit_ns: int) -> int:
-        """Runs the prompt kernel with accumulators handed over too late; returns the code of the wait that gave up (7)."""
+        """Runs the prompt kernel with accumulators handed over too late; returns the code of a wait that gave up (4, 5 or 6)."""
         code = C.c_int32(0)
         self._check(self._l.spyb_prefill_selftest_handoff_timeout(self.h, limit_ns, C.byref(code)))
         return int(code.value)

@@ -137,7 +137,7 @@ struct PrefillGemm {
     int           *error_flag = nullptr;
     uint64_t       wait_limit_ns = 1000000000ull;
     int            selftest_skip_step = -1;   // failure-path check: the copy warp leaves this step out, so the waits for it run out
-    uint64_t       selftest_late_ns = 0;      // failure-path check: accumulators are handed over so much later
+    bool           selftest_late = false;     // failure-path check (shared tiles of 16 tokens, Q4_0 / Q8_0 / Q4_K): accumulators are handed over three limits late
 };
 int         device_sms();         // SMs of the current device
 int         prefill_tile_tokens(int type, int64_t n_rows, int nb, int T);   // width of the token tiles for this matrix and number of tokens

@@ -124,7 +124,7 @@ __device__ __forceinline__ void pf_fold_steps(uint64_t (&acc)[2][8], int turns, 
 #undef PF_STEP
 
 // SHARE: the last tiles are cut among the CTAs or clusters (PfItem in spyb_tc.cuh)
-template <int TT, int S, bool MANY, bool SHARE>
+template <int TT, int S, bool MANY, bool SHARE, bool LATE>
 __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(PrefillGemm g) {
     using G = PfGeom<TT, S, MANY>;
     constexpr int NB = G::NB, NS = G::NS, PW = G::PW, PC = G::PC, YB = G::YB, HS = G::HS, WB = G::WB;
@@ -172,10 +172,10 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
     const uint32_t tmem = *tmem_slot;
 
     // How the expanding and multiplying warps walk: items and their steps, or (COUNTED) one count over all of them; and who releases the stage before a step's: the
-    // thread that issues its MMAs, or (EARLY_FREE) lane 0 beforehand. Whole tiles, 8 to 30 sizes each, per cent of the time with one count throughout and lane 0 for
-    // two CTAs only, as it was: 16 tokens by one CTA as here -2.1 to -3.3 (lane 0: -0.5 to -1.5), 8 tokens by one CTA -1.3 to -1.9 (the issuing thread: -0.6), 8 by two
-    // -0.3 to -0.5; 16 by two by items +0.7.
-    constexpr bool COUNTED = TT == 16 && S == 2, EARLY_FREE = TT == 8 || S == 2;
+    // thread that issues its MMAs, or (EARLY_FREE) lane 0 beforehand. Measured over 8 to 30 sizes a form, against one count throughout and lane 0 for two CTAs only: whole
+    // tiles of 16 tokens by one CTA -3 to -4 % of the time (lane 0: -0.5 to -1.5), their shared ones of up to 64 tokens -2 %, above +0.6 %; 8 tokens by one CTA -1.3 to
+    // -1.9 % (the issuing thread: -0.6), by two -0.3 to -0.5; 16 by two +0.7. Without the blocks past a row's end, tiles of 16 tokens +0.7 to +1.3 %, of 8 -0.5.
+    constexpr bool COUNTED = TT == 16 && (S == 2 || (SHARE && MANY)), EARLY_FREE = TT == 8 || S == 2;
     const int walker = (int)blockIdx.x / S;
     [[maybe_unused]] const int total_steps = SHARE ? g.share.rounds * n_step + g.share.len + ((int)gridDim.x / S - 1 - walker < g.share.rem ? 1 : 0) : (g.share.rounds + (walker < g.share.rem ? 1 : 0)) * n_step;
     auto first_item = [&]() -> PfItem {
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                         if (!EARLY_FREE && mine > 0) { mbar_arrive(st_free(st >= 2 ? st - 2 : st + NS - 2)); }   // (the step before on this buffer has been read)
 #pragma unroll
                         for (int j = 0; j < NB; ++j) {
-                            if (!COUNTED && j >= n) { continue; }   // (COUNTED: blocks past the end of a row are multiplied too, whatever lies there: nobody folds them)
+                            if (TT == 8 && j >= n) { continue; }   // (TT = 16: blocks past the end of a row are multiplied too, whatever lies there: nobody folds them)
 #pragma unroll
                             for (int h = 0; h < HS; ++h) {
                                 mma_f16_ss(d0 + (uint32_t)((j * HS + h) * 4 * TT), a0 + (uint64_t)((j * WB + h * (PF_HALF + 512)) >> 4), b0 + (uint64_t)(((j * HS + h) * 128 * TT) >> 4),
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
             const int tile = it.tile;
             if constexpr (SHARE) if (it.from > 0) {   // another walker's accumulators
                 const int64_t at = (int64_t)((int)blockIdx.x - S) * PF_GEMM_EPI_WARPS + warp;
-                handoff_wait(g.handoff_flags + at, left_ns, g.error_flag);
+                handoff_wait(g.handoff_flags + at, left_ns);
 #pragma unroll
                 for (int n = 0; n < 4 * HS * PW; ++n) { acc[n / (4 * HS)][n % (4 * HS)] = __ldcg(reinterpret_cast<const unsigned long long *>(g.handoff) + (at * 16 + n) * 32 + lane); }
                 __syncwarp();
@@ -431,9 +431,9 @@ __global__ void __launch_bounds__(PF_GEMM_THREADS, 1) prefill_gemm_kernel(Prefil
                     __stcg(reinterpret_cast<unsigned long long *>(g.handoff) + (at * 16 + n) * 32 + lane, (unsigned long long)a);
                     a = 0ull;
                 }
+                if constexpr (LATE) { const uint64_t t0 = global_timer_ns(); while (global_timer_ns() - t0 < 3 * limit) {} }   // (failure-path check)
                 __syncwarp();
-                if (lane == 0) { handoff_publish(g.handoff_flags + at, g.selftest_late_ns); }
-                __syncwarp();
+                if (lane == 0) { handoff_publish(g.handoff_flags + at); }
                 continue;
             }
             // hsum_float_8 (vec_util.h:74-81): accumulator n of a half is CPU accumulator 4 + n / n (Q4_0: low / high nibbles) or n / 4 + n
@@ -717,9 +717,9 @@ __global__ void prefill_silu_mul_kernel(const float *upgate, int T, int F, const
     act[i] = __fmul_rn(up, silu_table[f2h(gate)]);
 }
 
-template <int TT, int S, bool MANY = false, bool SHARE = false>
+template <int TT, int S, bool MANY = false, bool SHARE = false, bool LATE = false>
 cudaError_t launch_gemm_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
-    const void *kernel = reinterpret_cast<const void *>(prefill_gemm_kernel<TT, S, MANY, SHARE>);
+    const void *kernel = reinterpret_cast<const void *>(prefill_gemm_kernel<TT, S, MANY, SHARE, LATE>);
     const size_t smem = PfGeom<TT, S, MANY>::SMEM;
     cudaError_t err = allow_dynamic_smem(kernel, smem);
     if (err != cudaSuccess) { return err; }
@@ -877,6 +877,7 @@ cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool 
     bool share = false;
     const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok, g.split, g.tiles, device_sms(), &share).split == 2;
     share = share && g.handoff != nullptr;
+    if (g.selftest_late) { return !share || g.T <= 64 || g.tile_tok != 16 ? cudaErrorInvalidValue : pair ? launch_gemm_t<16, 2, false, true, true>(g, stream, pdl) : launch_gemm_t<16, 1, true, true, true>(g, stream, pdl); }
     // Many tokens (MANY): the epilogue is the bound and the weights come out of L2; copies of half a block are in its way for less long.
     // 22016 x 4096 x 448 tokens 659 us with one copy a step, 649 by blocks, 642 by halves, 646 by quarters. Where the weights' way
     // through HBM is the bound one copy is better: 4096 x 11008 x 64 tokens 55.8 us, by halves 56.2.

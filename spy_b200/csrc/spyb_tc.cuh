@@ -88,7 +88,7 @@ __device__ __forceinline__ void mbar_wait_lean(uint32_t bar, uint32_t parity, ui
                  : "+l"(limit_ns) : "r"(bar), "r"(parity) : "memory");
 }
 __device__ __forceinline__ void pf_report(int *error_flag, int code) {
-    if (error_flag != nullptr) { atomicMax(error_flag, code); }   // (who waits for whom: the highest code is the nearest to the cause)
+    if (error_flag != nullptr) { atomicExch(error_flag, code); }
 }
 
 // Shared tiles: where the tiles are no whole number of rounds, what is left after all rounds but one - one to two tiles a walker (CTA or cluster) - is laid end
@@ -116,21 +116,14 @@ inline PfShare pf_share(int n_tile, int n_step, int walkers) {   // n_tile > wal
 }
 // The word that says that a warp's accumulators lie in the handoff buffer; only the walker they are meant for clears it again. One that gave up may clear it
 // before it is set: after any reported error the words are the host's to clear (spyb_backend::clear_device_error).
-__device__ __forceinline__ void handoff_publish(unsigned *flag, uint64_t late_ns) {   // (late_ns: failure-path check)
-    if (late_ns != 0) { const uint64_t t0 = global_timer_ns(); while (global_timer_ns() - t0 < late_ns) {} }
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory");
-}
-__device__ __forceinline__ void handoff_wait(const unsigned *flag, uint64_t &limit_ns, int *error_flag) {
+__device__ __forceinline__ void handoff_publish(unsigned *flag) { asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory"); }
+__device__ __forceinline__ void handoff_wait(const unsigned *flag, uint64_t &limit_ns) {
     const uint64_t t0 = global_timer_ns();
     for (;;) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
         if (__all_sync(0xffffffffu, v != 0u)) { return; }
-        if (__any_sync(0xffffffffu, global_timer_ns() - t0 >= limit_ns)) {
-            if (limit_ns != 0 && (threadIdx.x & 31) == 0) { pf_report(error_flag, 7); }   // (not where an earlier wait had run out)
-            limit_ns = 0;
-            return;
-        }
+        if (__any_sync(0xffffffffu, global_timer_ns() - t0 >= limit_ns)) { limit_ns = 0; return; }
     }
 }
 
