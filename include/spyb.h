@@ -214,7 +214,7 @@ spyb_status spyb_prefill_matmul_tiles(spyb_backend *backend, int32_t weight_type
                                       const float *x_host, int64_t n_cols, const float *norm_w_host, float eps, int32_t tile_tokens, int32_t tile_ctas,
                                       int32_t last_tiles, float *out_host);
 
-/* The form that a Q4_0 / Q8_0 MatMul of these sizes takes on a device of n_sms SMs (host arithmetic only, no GPU needed). */
+/* The form that a Q4_0 / Q8_0 MatMul operator of these sizes takes on a device of n_sms SMs (host arithmetic only, no GPU needed). */
 spyb_status spyb_prefill_form(int64_t n_rows, int64_t k, int64_t n_cols, int32_t n_sms, int32_t *tile_tokens, int32_t *tile_ctas);
 /* The same for all weight types and with what becomes of the last tiles: what is zero of *tile_tokens, *tile_ctas and *last_tiles is filled in, what is not
  * is asked for. *last_tiles comes back as 1 (whole, also where 2 was asked for and there is nothing to share) or 2. */

@@ -441,7 +441,7 @@ spyb_status spyb_prefill_matmul_tiles(spyb_backend *be, int32_t weight_type, con
     if ((tile_tokens != 0 && !width_ok) || tile_ctas < 0 || tile_ctas > (kq ? 1 : 2)) { be->set_error("prefill_matmul: no form with tiles of %d tokens by %d CTAs", tile_tokens, tile_ctas); return SPYB_UNSUPPORTED; }
     if (last_tiles < 0 || last_tiles > 2) { be->set_error("prefill_matmul: last tiles %d", last_tiles); return SPYB_UNSUPPORTED; }
     cudaSetDevice(be->config.device_id);
-    const int nb = (int)(k / QK), T = (int)n_cols, tile_tok = tile_tokens != 0 ? tile_tokens : prefill_tile_tokens(weight_type, n_rows, nb, T);
+    const int nb = (int)(k / QK), T = (int)n_cols, tile_tok = tile_tokens != 0 ? tile_tokens : prefill_tile_tokens(weight_type, n_rows, nb, T, true);
     const int64_t rb = kq ? (k / 256) * (weight_type == SPYB_Q4_K ? 144 : 210) : (int64_t)nb * (weight_type == SPYB_Q4_0 ? 18 : 34);
     const size_t wbytes = prefill_weight_bytes(weight_type, n_rows, nb), ybytes = prefill_act_bytes(T, nb);
     uint8_t *raw = nullptr, *w = nullptr, *yq = nullptr; float *x = nullptr, *nw = nullptr, *out = nullptr;
@@ -461,7 +461,7 @@ spyb_status spyb_prefill_matmul_tiles(spyb_backend *be, int32_t weight_type, con
     if (err == cudaSuccess) { err = launch_prefill_quant(x, k, T, (int)k, nw, eps, yq, be->stream, weight_type, tile_tok); }
     if (err == cudaSuccess) {
         PrefillGemm g;
-        g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.tile_tok = tile_tok; g.split = tile_ctas; g.tiles = last_tiles; g.T = T; g.out = out; g.out_stride = n_rows;
+        g.w = w; g.type = weight_type; g.n_rows = n_rows; g.nb = nb; g.yq = yq; g.tile_tok = tile_tok; g.split = tile_ctas; g.tiles = last_tiles; g.beside = true; g.T = T; g.out = out; g.out_stride = n_rows;
         be->prefill_shared(g);
         err = launch_prefill_gemm(g, be->stream);
     }
@@ -661,7 +661,7 @@ spyb_status run_matmul_gemm(spyb_backend *be, const spyb_tensor &w, const spyb_t
         const int Tc = (int)std::min(chunk, T - t0);
         const bool pdl = be->config.use_pdl != 0;   // (columns that pad the last tile hold whatever the buffer held: their results are not stored)
         PrefillGemm g;
-        g.tile_tok = prefill_tile_tokens(type, n_rows, nb, Tc);
+        g.tile_tok = prefill_tile_tokens(type, n_rows, nb, Tc, true); g.beside = true;
         SPYB_CUDA(be, launch_prefill_quant(static_cast<const float *>(x.data) + t0 * k, k, Tc, (int)k, nullptr, 0.f, static_cast<uint8_t *>(yq), be->stream, type, g.tile_tok, 0, 0, pdl));
         g.w = tiles; g.type = type; g.n_rows = n_rows; g.nb = nb; g.yq = static_cast<uint8_t *>(yq); g.T = Tc;
         g.out = static_cast<float *>(out_dev) + t0 * n_rows; g.out_stride = n_rows;

@@ -131,6 +131,7 @@ struct PrefillGemm {
     int64_t        out_stride = 0;
     const float   *resid = nullptr;   // optional [T][out_stride]: out = W x + resid (may alias out)
     int            tiles = 0;                 // the last tiles: 1 whole, 2 shared (where there are more of them than CTAs or clusters), 0 by the sizes
+    bool           beside = false;            // an operator, beside which those of other backends may run
     PfShare        share = {};                // set by the launch
     void          *handoff = nullptr;         // PF_HANDOFF_BYTES per SM for accumulators that one CTA begins and another finishes; null: every tile is one CTA's
     unsigned      *handoff_flags = nullptr;   // sixteen words per SM, zero between launches that report no error
@@ -140,7 +141,7 @@ struct PrefillGemm {
     bool           selftest_late = false;     // failure-path check (shared tiles of 16 tokens, Q4_0 / Q8_0 / Q4_K): accumulators are handed over three limits late
 };
 int         device_sms();         // SMs of the current device
-int         prefill_tile_tokens(int type, int64_t n_rows, int nb, int T);   // width of the token tiles for this matrix and number of tokens
+int         prefill_tile_tokens(int type, int64_t n_rows, int nb, int T, bool beside);   // width of the token tiles for this matrix and number of tokens (beside: PrefillGemm)
 void        prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split);   // host-only: the Q4_0 / Q8_0 kernel's form on a device of so many SMs
 void        prefill_plan(int type, int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split, int *tiles);   // host-only: all of a kernel's form, what is zero of it by the sizes (PrefillGemm::tiles: 1 or 2)
 int         prefill_share_selftest();   // host-only: the cuts of shared tiles; 0 when they hold
@@ -154,7 +155,7 @@ cudaError_t launch_prefill_quant(const float *x, int64_t x_stride, int T, int K,
                                  int part_len = 0, int64_t part_stride = 0, bool pdl = false, uint8_t *tap = nullptr);   // tap: Q8_0 blocks of token 0, reference layout
 // up * silu(gate) of [T][2 F] and its Q8_0 blocks in one kernel; act [T][F]: also in f32 (null: not wanted)
 cudaError_t launch_prefill_silu_quant(const float *upgate, int T, int F, const float *silu_table, float *act, uint8_t *yq, cudaStream_t stream, int weight_type, int tile_tok, bool pdl);
-int         prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int how, int sms, bool *share);   // host-only: the K-quant kernel's width, and whether its last tiles are shared (how: PrefillGemm::tiles)
+int         prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int how, bool beside, int sms, bool *share);   // host-only: the K-quant kernel's width, and whether its last tiles are shared (how, beside: PrefillGemm::tiles, beside)
 cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream, bool pdl);   // type 12 = Q4_K, 14 = Q6_K (spyb_prefill_kq.cu)
 cudaError_t launch_prefill_retile_kq(int type, const uint8_t *raw, int64_t row_stride, int64_t n_rows, int nb, uint8_t *base, int64_t dst_row0, cudaStream_t stream);
 cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool pdl = false);

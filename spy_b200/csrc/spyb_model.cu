@@ -545,9 +545,9 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
     // the quantized activations are laid out for the type of the matrix they meet and for its token tile: quant() makes them for the
     // first matrix of a group, gemm() makes them again when a later matrix of the group wants another form
     struct { const float *x; int part_len; const float *norm_w; int K; int64_t part_stride; int type, tile_tok; } yq_src = {};
-    auto layout_of = [&](const PfMat &W, int K) { return ((W.type == SPYB_Q4_K || W.type == SPYB_Q6_K) ? 1000 : 0) + prefill_tile_tokens(W.type, W.n_rows, K / 32, T); };
+    auto layout_of = [&](const PfMat &W, int K) { return ((W.type == SPYB_Q4_K || W.type == SPYB_Q6_K) ? 1000 : 0) + prefill_tile_tokens(W.type, W.n_rows, K / 32, T, false); };
     auto quant = [&](const float *x, int part_len, int K, const float *norm_w, const PfMat &W, int64_t part_stride, uint8_t *tap_xq = nullptr) {
-        yq_src = {x, part_len, norm_w, K, part_stride, W.type, prefill_tile_tokens(W.type, W.n_rows, K / 32, T)};
+        yq_src = {x, part_len, norm_w, K, part_stride, W.type, prefill_tile_tokens(W.type, W.n_rows, K / 32, T, false)};
         return launch_prefill_quant(x, part_len, T, K, norm_w, norm_w != nullptr ? m->info.rms_eps : 0.f, m->pf_yq, s, W.type, yq_src.tile_tok, part_len, part_stride, pdl, tap_xq);
     };
     auto gemm = [&](const PfMat &W, int K, float *out, int64_t out_stride, const float *resid) {
@@ -612,7 +612,7 @@ spyb_status run_prefill_layers(spyb_model *m, int T, int64_t *launches, bool bat
         SPYB_CUDA(be, gemm(ly.pf_ug, d, m->pf_ug, 2 * (int64_t)fl, nullptr));
         if (m->kq) { SPYB_CUDA(be, gemm(ly.pf_gate, d, m->pf_ug + fl, 2 * (int64_t)fl, nullptr)); ++*launches; }
         if (tp == 1) {
-            const int tile_tok = prefill_tile_tokens(ly.pf_down.type, ly.pf_down.n_rows, ff / 32, T);
+            const int tile_tok = prefill_tile_tokens(ly.pf_down.type, ly.pf_down.n_rows, ff / 32, T, false);
             yq_src = {nullptr, ff, nullptr, ff, 0, ly.pf_down.type, tile_tok};
             SPYB_CUDA(be, launch_prefill_silu_quant(m->pf_ug, T, ff, be->d_silu_table, keep_act && &ly == &m->layers.back() ? m->pf_act : nullptr, m->pf_yq, s, ly.pf_down.type, tile_tok, pdl));
             --*launches;
@@ -1465,7 +1465,7 @@ spyb_status spyb_model_decode_batch(spyb_model *m, const int32_t *first_tokens, 
             if (m->pf_head.w != nullptr) {   // the logits of all sequences from one GEMM
                 const bool pdl = be->config.use_pdl != 0;
                 PrefillGemm g;
-                g.w = m->pf_head.w; g.type = m->pf_head.type; g.n_rows = V; g.nb = d / 32; g.yq = m->pf_yq; g.tile_tok = prefill_tile_tokens(g.type, V, d / 32, n_seq);
+                g.w = m->pf_head.w; g.type = m->pf_head.type; g.n_rows = V; g.nb = d / 32; g.yq = m->pf_yq; g.tile_tok = prefill_tile_tokens(g.type, V, d / 32, n_seq, false);
                 g.T = n_seq; g.out = m->logits_batch; g.out_stride = V; be->prefill_shared(g);
                 SPYB_CUDA(be, launch_prefill_quant(m->pf_x, dp, n_seq, d, m->output_norm, m->info.rms_eps, m->pf_yq, be->stream, g.type, g.tile_tok, dp, (int64_t)n_seq * dp, pdl));
                 SPYB_CUDA(be, launch_prefill_gemm(g, be->stream, pdl));

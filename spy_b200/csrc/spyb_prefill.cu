@@ -752,45 +752,39 @@ int device_sms() {
     return sms[dev];
 }
 
-// The form of the Q4_0 / Q8_0 kernel for a matrix and a number of tokens: tiles of 16 or of 8 tokens, by one CTA each or by a cluster of
-// two, the last ones whole or shared; the one whose cost is least. CTAs or clusters walk the tiles in rounds: a launch costs what fills its
-// pipelines, a round what a tile does once (its drain, and for two CTAs the joining of the halves) and a time for each block of the row (less
-// for narrow tiles, whose weights bound them, and about half for two CTAs), and every block of the matrix some time for its bytes, in
-// proportion to the chip. Shared tiles make the rounds a fraction, for the handing over and, for two CTAs, slower blocks; they are taken for a gain of
-// 2 % and 1 us, because the SMs that a last whole round leaves idle already copy the next GEMM's first weights (32000 x 4096 x 16, one submit after the other:
-// whole 44.5 us, shared 48.7). Fitted to 488 sizes, ten matrices of models and 70 drawn ones from 1024 x 1024 to 32000 x 14336, with 5 to 512 tokens: the rule's
-// choice is 0.3 % behind the fastest on average, more than 3 % behind it at 19 of them (3900 x 7136 x 38 tokens 10 %, 7980 x 2208 x 11 8 %). us with the activations'
-// quantizer, one CTA / two: 4096 x 4096 x 8 tokens 18.1 / 15.2, 4096 x 11008 x 16 54.7 / 34.9; and 1680 x 2208 x 79 tokens 13.3 / 16.2, 22016 x 4096 x 448
-// 655 / 826; whole / shared tiles: 14968 x 1088 x 22 19.5 / 21.8, and the sizes above.
-struct PfForm { int tok, split; double launch_ns, tile_ns, block_ns, rows_ns, handoff_ns, slower; };
-static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int split, int how, int sms, bool *share) {   // tok, split, how (PrefillGemm::tiles) 0: any
-    static constexpr PfForm FORMS[4] = {{16, 1, 4240, 730, 149.9, 28.3, 5720, -0.025}, {8, 1, 3210, 0, 119.2, 87.6, 2510, 0.019},
-                                        {16, 2, 5790, 1740, 84.5, 22.0, 5320, 0.065}, {8, 2, 5250, 1070, 65.1, 68.1, 3790, 0.020}};
+// The form of the Q4_0 / Q8_0 kernel for a matrix and a number of tokens: tiles of 16 or of 8 tokens, by one CTA each or by a cluster of two, the last ones whole or
+// shared; the one whose cost (pf_cost) is least. Fitted to 1068 sizes, fifteen matrices of models and 160 drawn ones from 1024 x 1536 to 32000 x 11264, with 5 to 512
+// tokens, every form timed with the submits of one backend and with those of three in turn. At 636 other sizes a model's choice is 0.25 % behind the fastest on average,
+// more than 3 % at 21 (28620 x 1728 x 8 tokens 10 %). An operator's, against a rule of whole tiles by rounds alone: one backend 5.9 % faster on average (more
+// than 3 % slower at 2 of 587), three 3.6 % (at 24); with a model's rule 6.7 % and 1.7 % (at 76). us a submit from one backend / three, with the quantizer,
+// 16 tokens a tile by one CTA, 8 by one, 16 by two, 8 by two: 4096 x 4096 x 8 tokens 24.0 / 9.9, 19.0 / 10.3, 19.0 / 14.2, 15.7 / 13.9; 4096 x 11008 x 16 57.4 /
+// 20.3, 54.9 / 25.9, 39.3 / 19.7, 35.9 / 30.0; 22016 x 4096 x 448 628 / 617, 998 / 974, 820 / 809, 1199 / 1190. The first and third with shared tiles: 12288 x 4096
+// x 32 whole 45.6 / 29.8, 46.2 / 39.3, shared 37.1 / 34.0, 47.6 / 44.3; 5120 x 13824 x 32 whole 70.9 / 40.4, 86.8 / 50.7, the third shared 57.8 / 54.2.
+struct PfForm { int tok, split; PfCost cost; };
+static PfForm best_form(int64_t n_rows, int nb, int T, int tok, int split, int how, bool beside, int sms, bool *share) {   // tok, split, how 0: any
+    static constexpr PfForm FORMS[4] = {{16, 1, {4320, 790, 143.9, 27.1, 5490, 0.044, 1850}}, {8, 1, {2430, 0, 118.7, 100.1, 4060, -0.019, 870}},
+                                        {16, 2, {6920, 1830, 87.9, 23.3, 4550, 0.079, 1420}}, {8, 2, {4890, 650, 63.3, 89.7, 6320, 0.004, 2300}}};
+    static constexpr PfRule RULE = {0.83, 0.46, 2340};
     PfForm best = {};
     double best_ns = 0.0;
     for (const PfForm &f : FORMS) {
         if ((tok != 0 && tok != f.tok) || (split != 0 && split != f.split)) { continue; }
-        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, tiles = row_tiles * ((T + f.tok - 1) / f.tok), walkers = std::max(1, sms / f.split);
-        const double once = f.launch_ns + (double)row_tiles / sms * nb * f.rows_ns;
-        double ns = once + (double)((tiles + walkers - 1) / walkers) * (f.tile_ns + nb * f.block_ns);
-        bool shared = false;
-        if (how != 1 && tiles > walkers && (how == 2 || tiles % walkers != 0)) {
-            const double ns_shared = 1000.0 + 1.02 * (once + f.handoff_ns + (double)tiles / walkers * (f.tile_ns + nb * f.block_ns * (1.0 + f.slower)));
-            if (how == 2 || ns_shared < ns) { ns = ns_shared; shared = true; }
-        }
+        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M;
+        bool shared;
+        const double ns = pf_cost(f.cost, RULE, row_tiles, row_tiles * ((T + f.tok - 1) / f.tok), std::max(1, sms / f.split), nb, sms, how, true, beside, &shared);
         if (best.tok == 0 || ns < best_ns) { best = f; best_ns = ns; *share = shared; }
     }
     return best;
 }
 void prefill_form(int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split) {
     bool share;
-    const PfForm f = best_form(n_rows, nb, T, 0, 0, 0, sms, &share);
+    const PfForm f = best_form(n_rows, nb, T, 0, 0, 0, true, sms, &share);
     *tile_tok = f.tok; *split = f.split;
 }
 void prefill_plan(int type, int64_t n_rows, int nb, int T, int sms, int *tile_tok, int *split, int *tiles) {
     bool share = false;
-    if (type == 12 || type == 14) { *tile_tok = prefill_kq_tile_tokens(n_rows, nb, T, *tile_tok, *tiles, sms, &share); *split = 1; }
-    else { const PfForm f = best_form(n_rows, nb, T, *tile_tok, *split, *tiles, sms, &share); *tile_tok = f.tok; *split = f.split; }
+    if (type == 12 || type == 14) { *tile_tok = prefill_kq_tile_tokens(n_rows, nb, T, *tile_tok, *tiles, true, sms, &share); *split = 1; }
+    else { const PfForm f = best_form(n_rows, nb, T, *tile_tok, *split, *tiles, true, sms, &share); *tile_tok = f.tok; *split = f.split; }
     *tiles = share ? 2 : 1;
 }
 // host-only check of the shared tiles: every step of every tile is some walker's exactly once, and a tile's first steps are the lower neighbour's of the
@@ -818,10 +812,10 @@ int prefill_share_selftest() {
     }
     return 0;
 }
-int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T) {
+int prefill_tile_tokens(int type, int64_t n_rows, int nb, int T, bool beside) {
     bool share;
-    if (type == 12 || type == 14) { return prefill_kq_tile_tokens(n_rows, nb, T, 0, 0, device_sms(), &share); }
-    return best_form(n_rows, nb, T, 0, 0, 0, device_sms(), &share).tok;
+    if (type == 12 || type == 14) { return prefill_kq_tile_tokens(n_rows, nb, T, 0, 0, beside, device_sms(), &share); }
+    return best_form(n_rows, nb, T, 0, 0, 0, beside, device_sms(), &share).tok;
 }
 
 size_t prefill_weight_bytes(int type, int64_t n_rows, int nb) {
@@ -875,7 +869,7 @@ cudaError_t launch_prefill_gemm(const PrefillGemm &g, cudaStream_t stream, bool 
     if ((g.type != 2 && g.type != 8) || g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 1 || g.n_rows < 1) { return cudaErrorInvalidValue; }
     if ((g.tile_tok != 16 && g.tile_tok != 8) || g.split < 0 || g.split > 2) { return cudaErrorInvalidValue; }
     bool share = false;
-    const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok, g.split, g.tiles, device_sms(), &share).split == 2;
+    const bool pair = best_form(g.n_rows, g.nb, g.T, g.tile_tok, g.split, g.tiles, g.beside, device_sms(), &share).split == 2;
     share = share && g.handoff != nullptr;
     if (g.selftest_late) { return !share || g.T <= 64 || g.tile_tok != 16 ? cudaErrorInvalidValue : pair ? launch_gemm_t<16, 2, false, true, true>(g, stream, pdl) : launch_gemm_t<16, 1, true, true, true>(g, stream, pdl); }
     // Many tokens (MANY): the epilogue is the bound and the weights come out of L2; copies of half a block are in its way for less long.

@@ -347,25 +347,23 @@ cudaError_t launch_kq_t(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
 
 }  // namespace
 
-// Tokens a tile: 16, 32 or 64 (tok 0: any), and whether the last tiles are shared; by a cost as in best_form of the Q4_0 / Q8_0 kernel, one for both types, so
-// that the matrices of a layer that read the same activations agree on a width. Fitted to 411 sizes of both (1024 x 1024 to 32000 x 14336, 8 to 512 tokens): 4.9 %
-// faster on average than the widths by whole rounds alone, 0.1 % behind the fastest choice, more than 3 % at 6 of them (Q4_K 8696 x 1536 x 82 9 %). us, whole
-// tiles / shared: Q4_K 11008 x 4096 x 64 41.7 / 31.9, 5120 x 5120 x 512 127.8 / 107.8, 4096 x 4096 x 512 78.7 / 72.2; Q6_K 4096 x 11008 x 512 193.9 / 174.4.
-int prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int how, int sms, bool *share) {
-    static constexpr struct { int tok; double launch_ns, tile_ns, block_ns, rows_ns, handoff_ns, slower; } WIDTHS[3] = {
-        {16, 4230, 100, 102.6, 49.7, 3770, 0.0}, {32, 4810, 280, 139.9, 33.1, 3780, -0.009}, {64, 4540, 880, 274.4, 4.3, 5230, -0.018}};
+// Tokens a tile: 16, 32 or 64 (tok 0: any), and whether the last tiles are shared; by the cost of pf_cost, one for both types, so that the matrices of a layer that read the
+// same activations agree on a width. Fitted to 1353 sizes of both (1024 x 1536 to 32000 x 11264, 5 to 512 tokens), timed with the submits of one backend and with those of three
+// in turn. At 626 other sizes a model's choice is 0.13 % behind the fastest on average, more than 3 % at 8 (Q6_K 12232 x 8192 x 83 7.5 %). An operator's, against
+// widths by whole rounds alone: one backend 3.7 % faster on average (more than 3 % slower at 4 of 476), three 1.1 % (at 40); with a model's rule 4.2 % and 0 % (at 72).
+// us a submit from one backend / three, whole and shared tiles: Q4_K 11008 x 4096 x 64, 32 tokens a tile 45.4 / 28.5 and 32.5 / 29.7; 64 tokens a tile: Q4_K
+// 5120 x 5120 x 512 141.8 / 110.2 and 108.4 / 105.1, 4096 x 4096 x 512 79.0 / 73.7 and 72.9 / 70.3; Q6_K 4096 x 11008 x 512 196.7 / 171.5 and 175.0 / 169.7.
+int prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int how, bool beside, int sms, bool *share) {
+    static constexpr struct { int tok; PfCost cost; } WIDTHS[3] = {
+        {16, {3420, 100, 98.6, 78.2, 4010, 0.003, 250}}, {32, {4370, 230, 137.6, 61.1, 3310, -0.026, 1560}}, {64, {4610, 800, 271.1, 2.6, 5760, -0.052, 1260}}};
+    static constexpr PfRule RULE = {0.91, 1.22, 430};
     int best = 0;
     double best_ns = 0.0;
     for (const auto &w : WIDTHS) {
         if (tok != 0 && tok != w.tok) { continue; }
-        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M, tiles = row_tiles * ((T + w.tok - 1) / w.tok);
-        const double once = w.launch_ns + (double)row_tiles / sms * nb * w.rows_ns;
-        double ns = once + (double)((tiles + sms - 1) / sms) * (w.tile_ns + nb * w.block_ns);
-        bool shared = false;
-        if (how != 1 && tiles > sms && (how == 2 || tiles % sms != 0) && nb >= 16) {
-            const double ns_shared = 500.0 + 1.01 * (once + w.handoff_ns + (double)tiles / sms * (w.tile_ns + nb * w.block_ns * (1.0 + w.slower)));
-            if (how == 2 || ns_shared < ns) { ns = ns_shared; shared = true; }
-        }
+        const int64_t row_tiles = (n_rows + PF_M - 1) / PF_M;
+        bool shared;
+        const double ns = pf_cost(w.cost, RULE, row_tiles, row_tiles * ((T + w.tok - 1) / w.tok), sms, nb, sms, how, nb >= 16, beside, &shared);
         if (best == 0 || ns < best_ns) { best = w.tok; best_ns = ns; *share = shared; }
     }
     return best;
@@ -374,7 +372,7 @@ int prefill_kq_tile_tokens(int64_t n_rows, int nb, int T, int tok, int how, int 
 cudaError_t launch_prefill_gemm_kq(const PrefillGemm &g, cudaStream_t stream, bool pdl) {
     if (g.w == nullptr || g.yq == nullptr || g.out == nullptr || g.T < 1 || g.nb < 8 || (g.nb & 7) || g.n_rows < 1 || (g.type != 12 && g.type != 14)) { return cudaErrorInvalidValue; }
     bool share = false;
-    prefill_kq_tile_tokens(g.n_rows, g.nb, g.T, g.tile_tok, g.tiles, device_sms(), &share);
+    prefill_kq_tile_tokens(g.n_rows, g.nb, g.T, g.tile_tok, g.tiles, g.beside, device_sms(), &share);
     auto of_width = [&](auto tt) {
         constexpr int TT = decltype(tt)::value;
         if (share && g.handoff != nullptr) { return g.type == 12 ? launch_kq_t<12, TT, true>(g, stream, pdl) : launch_kq_t<14, TT, true>(g, stream, pdl); }

@@ -2,6 +2,8 @@
 // shared-memory and mbarrier accessors, operand descriptors, the MMA / commit / tensor-memory instructions, bounded waits.
 #pragma once
 
+#include <algorithm>
+
 #include "spyb_common.cuh"
 #include "spyb_kernels.h"
 
@@ -97,7 +99,7 @@ __device__ __forceinline__ void pf_report(int *error_flag, int code) {
 // its own. Whoever waits thus waits for a CTA that was started before itself, and for steps that were done by then if all walk at one pace
 // (a stretch is at least a tile long). Whole rounds come first, in step: walkers that are beside each other then read the same weights at the same time.
 // Whole tiles / shared, us with the quantizer: 4096 x 4096 x 448 tokens (6.05 rounds) 142.5 / 126, 5120 x 13824 x 32 (1.08 rounds of clusters) 73.3 / 54, 12288
-// x 4096 x 32 (1.30 rounds) 45.8 / 37; 488 sizes: 6 % on average. What a cut costs, 2.5 to 5.7 us, is in best_form. Whole rounds keep a kernel of their own,
+// x 4096 x 32 (1.30 rounds) 45.8 / 37. What a cut costs, 2.5 to 6.3 us, is in pf_cost. Whole rounds keep a kernel of their own,
 // whose registers do not suffer from the handing over.
 struct PfItem { int tile, from, to, q; };   // steps (K-quants: super-blocks) [from, to) of a tile: a walker's item q
 __host__ __device__ __forceinline__ PfItem pf_share_item(const PfShare &h, int n_tile, int n_step, int walker, int walkers, int q) {
@@ -113,6 +115,26 @@ __host__ __device__ __forceinline__ PfItem pf_share_item(const PfShare &h, int n
 inline PfShare pf_share(int n_tile, int n_step, int walkers) {   // n_tile > walkers
     const int rounds = n_tile / walkers - 1, steps = (n_tile - rounds * walkers) * n_step;
     return {rounds, steps / walkers, steps % walkers, (0x100000000ull + n_step - 1) / n_step};
+}
+// What a launch costs, in ns, with its last tiles whole or shared, whichever is less (how: PrefillGemm::tiles). What fills its pipelines; for every block of the
+// matrix some time for its bytes, in proportion to the chip; then rounds of tiles: what a tile does once (its drain, and for two CTAs the joining of the
+// halves) and a time for each block of the row (less for narrow tiles, whose weights bound them, and about half for two CTAs). A last round that is full beyond
+// `full_from` costs up to full_ns more: what it leaves idle, the next launch begins on. Shared tiles make the rounds a fraction, for the handing over and somewhat slower
+// blocks. That is a launch with nothing beside it but its successor, a model's prompt. An operator (beside) also pays for the SMs' time that its tiles take, `idle`
+// times, and `margin_ns` for sharing: other backends' operators run on the SMs that a whole last round leaves, and shared tiles leave none. Three backends' submits in turn /
+// one's, us a submit, whole and shared: Q4_0 10024 x 3328 x 27 tokens 21.7 and 25.4 / 38.2 and 27.9; Q6_K 6520 x 6144 x 39 21.9 and 26.8 / 33.3 and 31.9.
+struct PfCost { double launch_ns, tile_ns, block_ns, rows_ns, handoff_ns, slower, full_ns; };
+struct PfRule { double full_from, idle, margin_ns; };
+inline double pf_cost(const PfCost &c, const PfRule &r, int64_t row_tiles, int64_t tiles, int64_t walkers, int nb, int sms, int how, bool sharable, bool beside, bool *shared) {
+    const double once = c.launch_ns + (double)row_tiles / sms * nb * c.rows_ns, busy = (double)tiles / walkers * (c.tile_ns + nb * c.block_ns);
+    const double fill = (double)((tiles - 1) % walkers + 1) / walkers;   // of the last round
+    const double whole = once + (double)((tiles + walkers - 1) / walkers) * (c.tile_ns + nb * c.block_ns) + c.full_ns * std::max(0.0, (fill - r.full_from) / (1.0 - r.full_from)) + (beside ? r.idle * busy : 0.0);
+    *shared = false;
+    if (how == 1 || !sharable || tiles <= walkers || (how != 2 && tiles % walkers == 0)) { return whole; }
+    const double cut = (double)tiles / walkers * (c.tile_ns + nb * c.block_ns * (1.0 + c.slower));
+    const double share = once + c.handoff_ns + cut + (beside ? r.margin_ns + r.idle * (cut + c.handoff_ns) : 0.0);
+    *shared = how == 2 || share < whole;
+    return *shared ? share : whole;
 }
 // The word that says that a warp's accumulators lie in the handoff buffer; only the walker they are meant for clears it again. One that gave up may clear it
 // before it is set: after any reported error the words are the host's to clear (spyb_backend::clear_device_error).

@@ -4,7 +4,7 @@ import os
 
 import pytest
 
-from spy_b200 import backend
+from spy_b200 import backend, quants
 
 
 def test_library_exports_every_declared_symbol():
@@ -64,3 +64,16 @@ def test_prompt_gemm_takes_the_form_that_measures_fastest(rows, k, tokens, form)
     tok, ctas = C.c_int32(0), C.c_int32(0)
     assert backend.lib().spyb_prefill_form(rows, k, tokens, 148, C.byref(tok), C.byref(ctas)) == backend.SUCCESS
     assert (tok.value, ctas.value) == form
+
+
+@pytest.mark.parametrize("qt,rows,k,tokens,shared", [
+    # measured on 148 SMs, us a submit with whole / shared last tiles, from one backend and from three in turn
+    (quants.Q4_0, 12288, 4096, 21, True),      # 45.9 / 37.2, 37.6 / 34.2
+    (quants.Q4_0, 32000, 4096, 16, False),     # 52.5 / 52.7, 45.2 / 49.8
+    (quants.Q4_0, 5120, 13824, 32, False),     # 70.9 / 57.7, 40.4 / 54.2
+    (quants.Q6_K, 6520, 6144, 39, False),      # 32.6 / 31.9, 21.8 / 26.8
+    (quants.Q4_K, 11008, 4096, 64, True),      # 45.4 / 32.5, 28.5 / 29.7
+    (quants.Q4_K, 4096, 4096, 512, True),      # 79.0 / 72.9, 73.7 / 70.3
+])
+def test_operators_share_tiles_where_that_pays_beside_others_too(qt, rows, k, tokens, shared):
+    assert (backend.prefill_plan(qt, rows, k, tokens)[2] == 2) == shared
