@@ -464,7 +464,7 @@ def test_matmul_without_room_for_the_tile_copy(oracle, qt):
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
-@pytest.mark.parametrize("n,k,t", [(4800, 256, 1), (4796, 1280, 3), (2, 256, 4), (300, 8448, 2), (292, 11008, 4), (9000, 768, 1)])
+@pytest.mark.parametrize("n,k,t", [(4800, 256, 1), (4796, 1280, 3), (2, 256, 4), (300, 8448, 2), (292, 11008, 4), (9000, 768, 1), (604, 3840, 2), (604, 2304, 2), (604, 1792, 2)])
 def test_k_quant_mat_vec_units_and_rounds(be, oracle, qt, n, k, t):
     """The K-quant mat-vec kernel on units of one, two and four row pairs, rows of 1 to 43 super-blocks (rounds of 32 that end inside a row
     and inside a unit), more units than warps and fewer, 1 to 4 columns; bit-identical to the restatement."""
