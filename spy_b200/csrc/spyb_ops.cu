@@ -53,12 +53,6 @@ constexpr int ATT_WARPS   = ATT_THREADS / WARP;
 constexpr int ATT_HD      = 128;
 constexpr int ATT_MANY    = 2;      // CTAs an SM holds of a launch that has more of them than the chip has SMs
 
-__device__ __forceinline__ void unpack8(const uint4 v, float f[8]) {
-    const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2 *>(&v.y));
-    const float2 c = __half22float2(*reinterpret_cast<const __half2 *>(&v.z)), d = __half22float2(*reinterpret_cast<const __half2 *>(&v.w));
-    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-}
-
 // a * b + c of the f16 values in the low halves of a and b: the fmaf of the widened values (their product is exact in f32) without widening
 // them; it issues as fast as fmaf, and half the bytes of its operands come out of shared memory
 __device__ __forceinline__ float fma_f16(uint32_t a, uint32_t b, float c) {
