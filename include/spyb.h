@@ -328,7 +328,8 @@ spyb_status spyb_model_tap_xq(spyb_model *model, void *blocks_host);
  * its predecessor finished, its activations quantized, last CTA finished, then the latest CTA's start,
  * predecessor-finished and activations-quantized times, and one unused word. Copies up to max_kernels records of
  * eight stamps (layer-major: QKV, attention, attention-out, FFN up/gate, FFN down; then the head) and
- * returns their number (0 when the timeline is off). */
+ * returns their number (0 when the timeline is off). The kernels that hold stamps are instances of their own, slower than those of
+ * other steps (7B Q4_0: 42.1 us a layer against 36.5): the stamps show what a kernel's time is made of, not how a step's is split. */
 int32_t spyb_model_read_timeline(spyb_model *model, uint64_t *stamps_host, int32_t max_kernels);
 /* The same for single-token steps that run as one persistent kernel: pairs (CTA 0's time, the latest CTA's time) at
  * every check point of the step - kernel entry, then per layer: barrier passed / activations quantized / mat-vec done for

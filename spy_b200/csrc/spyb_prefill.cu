@@ -44,10 +44,11 @@ constexpr int PF_QUANT_GROUPS  = (PF_MAX_K + 8 * PF_QUANT_THREADS - 1) / (8 * PF
 //   warps 18-19 issue the MMAs of alternate steps and one commit each
 // The pipeline does not drain between tiles: copies, expansion and MMAs run on into the next tile while a tile's rows are stored.
 //
-// Bound: issue slots. A step is 32 packed FMAs (two slots each: a packed FMA measures no faster than 2.5 cycles per scheduler) and 4 packed
-// multiplies per epilogue warp, i.e. 290 slots per scheduler, and everything else around them another 165; the loop is written for few
-// instructions (waits of one test and one branch, D buffers as constants of the unrolled code, one arrival per step), and measures 564
-// cycles per step: 4096 x 4096 x 448 tokens 126 us (138 with whole tiles only), 22016 rows 640 us (the e4m3 form: 216 and 1017 us). Tiles of
+// Bound: no unit is full. A step is 32 packed FMAs and 4 packed multiplies per epilogue warp, 144 a scheduler, each measured at 2.2-2.4 cycles, and 157 other
+// instructions a scheduler; the loop is written for few of them (waits of one test and one branch, D buffers as constants of the unrolled code, one
+// arrival per step) and measures 548 cycles per step, the FMA pipes 56 % busy, the issue slots 55 %, the tensor pipe 23 %: the folds wait for what they read from
+// tensor and shared memory, four warps a scheduler hide part of that, and no register is left to ask for it earlier. 4096 x 4096 x 448 tokens 127 us (138
+// with whole tiles only), 22016 rows 628 us (the e4m3 form: 216 and 1017 us). Tiles of
 // 32 tokens halve the weight bytes per FMA but need 110 registers: spills, 265 us. Eight epilogue warps with 216 registers each: 186-208 us. (The
 // epilogue's registers are all taken, which is why its loop is written as PTX, pf_fold_steps: the compiler's own order of the same loop measured
 // between 640 and 709 us on the 22016 rows, depending on code beside it.)
