@@ -4,7 +4,8 @@ import os
 
 import pytest
 
-from spy_b200 import backend, quants
+from spy_b200 import backend
+from spy_b200 import quants
 
 
 def test_library_exports_every_declared_symbol():

@@ -177,11 +177,26 @@ def test_prefill_matmul_shared_by_two_ctas(be, oracle, qt, n, k, t):
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
-@pytest.mark.parametrize("n,k,t", [(9604, 4128, 32), (2564, 4128, 118), (6148, 2080, 130), (19204, 1568, 36), (18944, 672, 32), (19204, 96, 24)])
+@pytest.mark.parametrize("n,k,t", [(9604, 4128, 32), (2564, 4128, 118), (6148, 2080, 130), (19204, 1568, 36)])
 def test_prefill_matmul_shares_its_last_tiles(be, oracle, qt, n, k, t):
-    """More tiles than walkers in every form, up to eleven rounds, and each form with its last tiles shared beside whole: they are cut between neighbours at odd and
-    even steps (in whole rounds also at a tile's end), rows end inside a step or have two steps, and calls follow one another (what one leaves in the buffer of
-    the handing over, the next one does not find)."""
+    """One to four rounds and a fraction of tiles in every form: the last tiles are cut between neighbours at odd and even steps, rows end inside a step, and
+    calls follow one another (what one leaves in the buffer of the handing over, the next one does not find)."""
+    rng = np.random.default_rng(n + k + t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    rows = np.unique(np.r_[np.arange(0, n, 128), n - 1, rng.integers(0, n, 60)])
+    want = oracle.matmul(qt, np.ascontiguousarray(w[rows]), k, len(rows), x)
+    for form in [(16, 1), (8, 1), (16, 2), (8, 2), (0, 0), (16, 1)]:
+        got = be.prefill_matmul(qt, w, n, k, x, form=form)
+        assert np.array_equal(got[:, rows].view(np.uint32), want.view(np.uint32)), form
+
+
+@pytest.mark.parametrize("qt", [quants.Q4_0, quants.Q8_0])
+@pytest.mark.parametrize("n,k,t", [(9604, 4128, 32), (2564, 4128, 118), (6148, 2080, 130), (19204, 1568, 36), (18944, 672, 32), (19204, 96, 24)])
+def test_prefill_matmul_with_last_tiles_shared_and_whole(be, oracle, qt, n, k, t):
+    """More tiles than walkers in every form, up to eleven rounds, and each form with its last tiles shared beside whole, whatever the sizes' own choice:
+    they are cut between neighbours at odd and even steps (in whole rounds also at a tile's end), rows end inside a step or have two steps, and calls follow
+    one another (what one leaves in the buffer of the handing over, the next one does not find)."""
     rng = np.random.default_rng(n + k + t + qt)
     w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
     x = rng.standard_normal((t, k)).astype(np.float32)
@@ -224,9 +239,24 @@ def test_prefill_matmul_k_quants_walk_tiles_of_all_widths(be, oracle, qt, n, k, 
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
-@pytest.mark.parametrize("n,k,t", [(2564, 2304, 490), (9604, 4352, 129), (19204, 2560, 9), (1028, 5632, 1100), (18944, 512, 128)])
+@pytest.mark.parametrize("n,k,t", [(2564, 2304, 490), (9604, 4352, 63), (19204, 2560, 9), (1028, 5632, 600)])
 def test_prefill_matmul_k_quants_share_their_last_tiles(be, oracle, qt, n, k, t):
-    """More tiles than CTAs in every width, up to four rounds, each with its last tiles shared, cut between neighbours at super-blocks, beside whole; calls follow one another."""
+    """One to four rounds and a fraction of tiles in every width, cut between neighbours at super-blocks; calls follow one another."""
+    rng = np.random.default_rng(n + k + t + qt)
+    w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
+    x = rng.standard_normal((t, k)).astype(np.float32)
+    rows, cols = np.unique(np.r_[np.arange(0, n, 128), n - 1, rng.integers(0, n, 20)]), np.unique(np.r_[np.arange(0, t, 16), t - 1])
+    want = oracle.matmul(qt, np.ascontiguousarray(w[rows]), k, len(rows), x[cols])
+    for form in [(64, 1), (32, 1), (16, 1), (0, 0), (64, 1)]:
+        got = be.prefill_matmul(qt, w, n, k, x, form=form)
+        assert np.array_equal(got[np.ix_(cols, rows)].view(np.uint32), want.view(np.uint32)), form
+
+
+@pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
+@pytest.mark.parametrize("n,k,t", [(2564, 2304, 490), (9604, 4352, 129), (19204, 2560, 9), (1028, 5632, 1100), (18944, 512, 128)])
+def test_prefill_matmul_k_quants_with_last_tiles_shared_and_whole(be, oracle, qt, n, k, t):
+    """Tiles of every width (where there are more of them than CTAs) with the last ones shared, cut between neighbours at super-blocks, beside whole,
+    whatever the sizes' own choice; calls follow one another."""
     rng = np.random.default_rng(n + k + t + qt)
     w = quants.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), qt)
     x = rng.standard_normal((t, k)).astype(np.float32)
@@ -464,7 +494,7 @@ def test_matmul_without_room_for_the_tile_copy(oracle, qt):
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
-@pytest.mark.parametrize("n,k,t", [(4800, 256, 1), (4796, 1280, 3), (2, 256, 4), (300, 8448, 2), (292, 11008, 4), (9000, 768, 1), (604, 3840, 2), (604, 2304, 2), (604, 1792, 2)])
+@pytest.mark.parametrize("n,k,t", [(4800, 256, 1), (4796, 1280, 3), (2, 256, 4), (300, 8448, 2), (292, 11008, 4), (9000, 768, 1)])
 def test_k_quant_mat_vec_units_and_rounds(be, oracle, qt, n, k, t):
     """The K-quant mat-vec kernel on units of one, two and four row pairs, rows of 1 to 43 super-blocks (rounds of 32 that end inside a row
     and inside a unit), more units than warps and fewer, 1 to 4 columns; bit-identical to the restatement."""
@@ -480,6 +510,13 @@ def test_k_quant_mat_vec_units_and_rounds(be, oracle, qt, n, k, t):
     be.submit(d); be.sync()
     got = be.download(po, (t, n), np.float32)
     assert np.array_equal(bits(got), bits(oracle.matmul(qt, w, k, n, x)))
+
+
+@pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])
+@pytest.mark.parametrize("k", [1792, 2304, 3840])
+def test_k_quant_mat_vec_of_two_columns_sums_the_end_of_a_row(be, oracle, qt, k):
+    """Two columns of rows of seven, nine and fifteen super-blocks: what is left of a row behind its groups of eight, up to seven values."""
+    test_k_quant_mat_vec_units_and_rounds(be, oracle, qt, 604, k, 2)
 
 
 @pytest.mark.parametrize("qt", [quants.Q4_K, quants.Q6_K])

@@ -26,3 +26,17 @@ def test_tensor_parallel_matches_single_gpu(world, nccl_only, model, tmp_path):
     r = subprocess.run(cmd, env=env, capture_output=True, text=True, timeout=900)
     print(r.stdout[-2000:], r.stderr[-2000:])
     assert r.returncode == 0 and "OK" in r.stdout
+
+
+@pytest.mark.parametrize("world", [2])
+def test_tensor_parallel_prompt_shares_tiles(world, tmp_path):
+    """A prompt whose GEMMs on a rank's slices share their last tiles between CTAs (waits inside a launch beside the exchange)."""
+    import torch
+    if torch.cuda.device_count() < world:
+        pytest.skip(f"needs {world} GPUs")
+    worker = os.path.join(os.path.dirname(__file__), "tp_prompt_worker.py")
+    cmd = [sys.executable, "-m", "torch.distributed.run", "--nnodes=1", f"--nproc-per-node={world}", "--master-addr", "127.0.0.1",
+           "--master-port", "29543", worker, str(tmp_path / "tp.gguf")]
+    r = subprocess.run(cmd, env=dict(os.environ, NCCL_NVLS_ENABLE="0"), capture_output=True, text=True, timeout=900)
+    print(r.stdout[-2000:], r.stderr[-2000:])
+    assert r.returncode == 0 and "OK" in r.stdout

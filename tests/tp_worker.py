@@ -32,8 +32,7 @@ def main():
     prompt = np.random.default_rng(3).integers(3, cfg.n_vocab, size=9)
 
     be = B.B200Backend(local, tp_size=world, tp_rank=rank)
-    n_ctx = 320 if deep else 64
-    m = B.LlamaModel(be, path, n_ctx=n_ctx)
+    m = B.LlamaModel(be, path, n_ctx=64)
     uid = [B.nccl_unique_id() if rank == 0 else None]
     dist.broadcast_object_list(uid, src=0)
     m.init_tp(uid[0])
@@ -46,9 +45,6 @@ def main():
     # output and the FFN activation are all-gathered once per layer
     long_prompt = np.random.default_rng(4).integers(3, cfg.n_vocab, size=41)
     long_logits = m.eval(long_prompt, 0).copy()
-    # ... and, on the deep model, one of so many tokens that the last tiles of a rank's slice of W_down (512 x 2816) are shared between CTAs
-    wide_prompt = np.random.default_rng(6).integers(3, cfg.n_vocab, size=300) if deep else long_prompt
-    wide_logits = m.eval(wide_prompt, 0).copy()
     # batches of sequences on the sharded model (every step one pass of the GEMM path, the sequences as its tokens): 3 and 18
     # sequences, each with its own 9-token prompt, decoded in lockstep
     batches = {}
@@ -64,21 +60,20 @@ def main():
     ok = True
     if rank == 0:
         b1 = B.B200Backend(local)
-        m1 = B.LlamaModel(b1, path, n_ctx=n_ctx)
+        m1 = B.LlamaModel(b1, path, n_ctx=64)
         ids1, logits1 = m1.generate(prompt, 12)
         err = float(np.abs(logits - logits1).max())
         same_bits = bool(np.array_equal(np.asarray(logits, dtype=np.float32).view(np.uint32), np.asarray(logits1, dtype=np.float32).view(np.uint32)))
         long_same = bool(np.array_equal(long_logits.view(np.uint32), m1.eval(long_prompt, 0).view(np.uint32)))
-        wide_same = bool(np.array_equal(wide_logits.view(np.uint32), m1.eval(wide_prompt, 0).view(np.uint32)))
         batch_same = True
         for nb, (prompts, firsts, b_ids, b_logits) in batches.items():
             for c in range(nb):
                 i1, l1 = m1.generate(prompts[c], 6)
                 batch_same = batch_same and int(i1[0]) == firsts[c] and bool(np.array_equal(i1[1:], b_ids[:, c]))
                 batch_same = batch_same and bool(np.array_equal(l1[1:].view(np.uint32), b_logits[:, c].view(np.uint32)))
-        ok = bool(np.array_equal(ids, ids1)) and same_bits and long_same and wide_same and batch_same
+        ok = bool(np.array_equal(ids, ids1)) and same_bits and long_same and batch_same
         print(f"TP{world} vs TP1 ({'deep' if deep else 'small'} model): max|dlogit| = {err:.3e}, bits identical = {same_bits}, "
-              f"ids identical = {np.array_equal(ids, ids1)}, 41-token prompt bits identical = {long_same}, {len(wide_prompt)}-token prompt {wide_same}, batches of 3 and 18 sequences bits identical = {batch_same} -> {'OK' if ok else 'FAIL'}", flush=True)
+              f"ids identical = {np.array_equal(ids, ids1)}, 41-token prompt bits identical = {long_same}, batches of 3 and 18 sequences bits identical = {batch_same} -> {'OK' if ok else 'FAIL'}", flush=True)
         m1.close(); b1.close()
     m.close(); be.close()
     flag = torch.tensor([0 if ok else 1])
