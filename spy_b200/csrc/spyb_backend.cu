@@ -213,8 +213,8 @@ spyb_status spyb_create(const spyb_config *config, spyb_backend **out) {
     }
     bool ok = cudaMalloc(reinterpret_cast<void **>(&be->d_silu_table), 65536 * 4) == cudaSuccess &&
               cudaMalloc(reinterpret_cast<void **>(&be->d_exp_table), 65536 * 4) == cudaSuccess &&
-              cudaMemcpy(be->d_silu_table, silu.data(), 65536 * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
-              cudaMemcpy(be->d_exp_table, ex.data(), 65536 * 4, cudaMemcpyHostToDevice) == cudaSuccess;
+              upload(be->d_silu_table, silu.data(), 65536 * 4) == cudaSuccess &&
+              upload(be->d_exp_table, ex.data(), 65536 * 4) == cudaSuccess;
     if (!ok) { spyb_destroy(be); return SPYB_FAIL; }
     const size_t handoff = (size_t)be->num_sms_total * (PF_HANDOFF_BYTES + PF_HANDOFF_FLAGS * sizeof(unsigned));
     if (cudaMalloc(&be->pf_handoff, handoff) != cudaSuccess) { cudaGetLastError(); be->pf_handoff = nullptr; }   // (the GEMMs go without)
@@ -292,7 +292,7 @@ void *spyb_upload_constant(spyb_backend *be, const char *name, const void *host_
     void *raw = nullptr;
     if (cudaMalloc(&raw, bytes + 64) != cudaSuccess) { be->set_error("cudaMalloc(%llu) failed for constant %s", (unsigned long long)bytes, name); return nullptr; }
     be->owned.push_back(raw);
-    if (cudaMemcpy(raw, host_ptr, bytes, cudaMemcpyHostToDevice) != cudaSuccess) { be->set_error("upload of %s failed", name); return nullptr; }
+    if (upload(raw, host_ptr, bytes) != cudaSuccess) { be->set_error("upload of %s failed", name); return nullptr; }
     if ((number_type == SPYB_Q4_0 || number_type == SPYB_Q8_0) && elements != nullptr) {
         // matrices also get the plane layout the mat-vec kernels stream; the raw copy stays for GetRow and parity checks
         const int64_t k = elements[0], rows = elements[1] * elements[2] * elements[3];

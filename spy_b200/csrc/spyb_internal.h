@@ -58,6 +58,13 @@ struct RopeTable {
     std::vector<uint8_t> have;
 };
 
+// Host memory to the device, arrived when it returns: a plain cudaMemcpy from pageable memory may return before its last piece has, and a backend's stream
+// does not wait for the legacy one. (Not a copy on the backend's stream: another thread may be capturing a step there.)
+inline cudaError_t upload(void *dst, const void *src, size_t bytes) {
+    const cudaError_t err = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return err != cudaSuccess ? err : cudaStreamSynchronize(cudaStreamLegacy);
+}
+
 }  // namespace spyb
 
 struct spyb_backend {

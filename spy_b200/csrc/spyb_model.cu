@@ -351,7 +351,7 @@ spyb_status build_step_plan(spyb_model *m) {
     }
     StepLayer *d_layers = nullptr;
     if (dev_alloc(m, &d_layers, hl.size()) != SPYB_SUCCESS) { return SPYB_FAIL; }
-    SPYB_CUDA(be, cudaMemcpy(d_layers, hl.data(), hl.size() * sizeof(StepLayer), cudaMemcpyHostToDevice));
+    SPYB_CUDA(be, upload(d_layers, hl.data(), hl.size() * sizeof(StepLayer)));
     int8_t *att_q = nullptr; float *att_d = nullptr;
     if (dev_alloc(m, &att_q, (size_t)m->info.d_model) != SPYB_SUCCESS || dev_alloc(m, &att_d, (size_t)m->info.d_model / 32) != SPYB_SUCCESS ||
         dev_alloc(m, &m->d_step_sync, 8) != SPYB_SUCCESS) { return SPYB_FAIL; }
@@ -757,7 +757,7 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
         if (!tensor(name, &t, &data)) { return SPYB_FAIL; }
         if (t->type != SPYB_FP32 || t->ne[0] != n) { be->set_error("GGUF: %s must be f32[%lld]", name.c_str(), (long long)n); return SPYB_FAIL; }
         if (dev_alloc(m, dst, (size_t)n) != SPYB_SUCCESS) { return SPYB_FAIL; }
-        SPYB_CUDA(be, cudaMemcpy(*dst, data, (size_t)n * 4, cudaMemcpyHostToDevice));
+        SPYB_CUDA(be, upload(*dst, data, (size_t)n * 4));
         return SPYB_SUCCESS;
     };
     // rows [row0, row0 + n_rows) and blocks [blk0, blk0 + nb) of a [k_full, rows_full] matrix -> planes (optionally into `into` at row dst_row)
@@ -787,7 +787,7 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
         uint8_t *dev = nullptr;
         if (dev_alloc(m, &dev, (size_t)n_rows * rb_dev) != SPYB_SUCCESS) { return SPYB_FAIL; }
         if (t->type == SPYB_Q4_K) {
-            SPYB_CUDA(be, cudaMemcpy(dev, data + row0 * rb_file, (size_t)n_rows * rb_file, cudaMemcpyHostToDevice));
+            SPYB_CUDA(be, upload(dev, data + row0 * rb_file, (size_t)n_rows * rb_file));
         } else {   // Q6_K: 210-byte super-blocks -> 16-byte-aligned pieces
             void *stage = nullptr;
             SPYB_CUDA(be, cudaMalloc(&stage, (size_t)n_rows * rb_file + 64));
@@ -851,7 +851,7 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
         }
         const size_t bytes = (size_t)GgufFile::row_bytes(t->type, d) * t->ne[1];
         if (dev_alloc(m, &m->embd, bytes) != SPYB_SUCCESS) { return fail(SPYB_FAIL); }
-        if (cudaMemcpy(m->embd, data, bytes, cudaMemcpyHostToDevice) != cudaSuccess) { be->set_error("embedding upload failed"); return fail(SPYB_FAIL); }
+        if (upload(m->embd, data, bytes) != cudaSuccess) { be->set_error("embedding upload failed"); return fail(SPYB_FAIL); }
     }
     spyb_status st = upload_f32("output_norm.weight", d, &m->output_norm);
     if (st != SPYB_SUCCESS) { return fail(st); }
@@ -972,11 +972,11 @@ spyb_status spyb_model_load_gguf(spyb_backend *be, const char *path, int32_t n_c
             for (int i = 0; i < hd / 2; ++i) { tab[(size_t)pos * (hd / 2) + i] = make_float2(std::cos(theta) * 1.0f, std::sin(theta) * 1.0f); theta *= theta_scale; }
         }
         if (dev_alloc(m, &m->rope_table, tab.size()) != SPYB_SUCCESS) { return fail(SPYB_FAIL); }
-        if (cudaMemcpy(m->rope_table, tab.data(), tab.size() * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess) { be->set_error("rope table upload failed"); return fail(SPYB_FAIL); }
+        if (upload(m->rope_table, tab.data(), tab.size() * sizeof(float2)) != cudaSuccess) { be->set_error("rope table upload failed"); return fail(SPYB_FAIL); }
     }
     {   // the exchange buffer: gathered attention output and FFN activation, flag words, counters (one plain cudaMalloc: it is exported)
         void *raw = nullptr;
-        if (cudaMalloc(&raw, tp_buffer_bytes(m)) != cudaSuccess || cudaMemset(raw, 0, tp_buffer_bytes(m)) != cudaSuccess) { be->set_error("exchange buffer allocation failed"); return fail(SPYB_FAIL); }
+        if (cudaMalloc(&raw, tp_buffer_bytes(m)) != cudaSuccess || cudaMemset(raw, 0, tp_buffer_bytes(m)) != cudaSuccess || cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) { be->set_error("exchange buffer allocation failed"); return fail(SPYB_FAIL); }
         m->owned.push_back(raw);
         m->tp_local = static_cast<uint8_t *>(raw);
         m->tp_peer[I.tp_rank] = m->tp_local;

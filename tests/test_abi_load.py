@@ -78,3 +78,16 @@ def test_prompt_gemm_takes_the_form_that_measures_fastest(rows, k, tokens, form)
 ])
 def test_operators_share_tiles_where_that_pays_beside_others_too(qt, rows, k, tokens, shared):
     assert (backend.prefill_plan(qt, rows, k, tokens)[2] == 2) == shared
+
+
+def test_uploads_have_arrived_when_they_return():
+    """A plain cudaMemcpy from pageable memory may return before its last piece has arrived, and a non-blocking stream does not wait for the legacy one: what
+    the legacy stream copies or clears is waited for beside the call."""
+    csrc = os.path.join(os.path.dirname(backend.__file__), "csrc")
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith((".cu", ".cuh", ".h")):
+            with open(os.path.join(csrc, name)) as f:
+                lines = f.read().split("\n")
+            for i, line in enumerate(lines):
+                if "cudaMemset(" in line or ("cudaMemcpy(" in line and "HostToDevice" in line):
+                    assert "cudaStreamSynchronize(cudaStreamLegacy)" in line + lines[i + 1], (name, line)
